@@ -2,7 +2,7 @@
 // state-space-duality form (a state matrix per head), and the gate and grouped norm that follows the latter.
 //
 //   selective scan   per channel c and state n, token by token:
-//                      dt = softplus(dtz[c] + dt_bias[c]) (made once per token and channel by a kernel ahead of the scan);
+//                      dt = softplus(dtz[c] + dt_bias[c]);
 //                      S[c][n] = exp(dt * A[c][n]) * S[c][n] + dt * x[c] * B[n];
 //                      y[c] = sum_n S[c][n] * C[n] + D[c] * x[c];  out[c] = y[c] * silu(z[c])
 //   duality form     per head h (group g = h / (heads / groups)) with S [N][V], token by token:
@@ -17,7 +17,7 @@
 // a token's result depends only on the tokens before it, never on what else is in the batch.
 // Everything here is float32 in both engine precisions; only the result leaves in the compute dtype.
 //
-// The portion-parallel forms cut a portion into segments that run side by side: every segment first runs from a zero
+// The portion-parallel form of the duality recurrence cuts a portion into segments that run side by side: every segment first runs from a zero
 // state and records the product of its decays and its end state; the segments' starting states then follow one from
 // another; a second pass repeats the segment from its true starting state and writes the results.
 #include "common.cuh"
@@ -41,113 +41,219 @@ struct Segments {
     int nseg;           // the most segments one portion has (grid z); request s's segments start at q_start[s] / seg_len + s
 };
 
-// dtz[t][c] <- softplus(dtz[t][c] + bias[c]): the step sizes, once per token and channel, ahead of the scan.
-__global__ void __launch_bounds__(256)
-step_sizes_kernel(float* __restrict__ dtz, long lddt, const void* __restrict__ bias, int pdt, int T, int inner) {
-    const int t = blockIdx.y, c = blockIdx.x * 256 + threadIdx.x;
-    if (c < inner) dtz[(size_t)t * lddt + c] = ssm_softplus(dtz[(size_t)t * lddt + c] + load_dyn(bias, pdt, c));
-}
-
+// ---- the selective scan
 // LANES neighbouring lanes share one channel: lane ln keeps the CH state values n = ln * CH .. ln * CH + CH - 1 in
-// registers (N <= LANES * CH) and the partial sums of y meet by shuffles.  U tokens are fetched ahead of their arithmetic.
-// The rows U tokens bring to one lane of the selective scan.
-template <int U, int CH>
-struct ScanRows {
-    float dt[U], x[U], z[U], b[U][CH], c[U][CH];
-    __device__ __forceinline__ void fetch(const float* __restrict__ xs, long ldx, const float* __restrict__ dtv, long lddt,
-                                          const float* __restrict__ zs, long ldz, const float* __restrict__ bc, long ldbc, int b_off,
-                                          int c_off, int ch, int n0, int N, int t, int t1, bool wants_z) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int tt = t + u < t1 ? t + u : t1 - 1;            // beyond the portion's end the last token's rows are read again
-            dt[u] = dtv[(size_t)tt * lddt + ch];
-            x[u] = xs[(size_t)tt * ldx + ch];
-            z[u] = wants_z ? zs[(size_t)tt * ldz + ch] : 0.f;
-            const float* br = bc + (size_t)tt * ldbc + b_off + n0;
-            const float* cr = bc + (size_t)tt * ldbc + c_off + n0;
-#pragma unroll
-            for (int i = 0; i < CH; ++i) { const bool in = n0 + i < N; b[u][i] = in ? br[i] : 0.f; c[u][i] = in ? cr[i] : 0.f; }
-        }
-    }
+// registers (N <= LANES * CH) and walks the portion's tokens in order.  One request has few walkers (4,096 channels with
+// 8 lanes are two warps a scheduler), so what bounds a walk is the length of a token's dependent instructions, then their
+// number (at the limit one exponential per token and state value, 16 a clock and SM).  Hence:
+//   * the rows of a stage of tokens arrive in shared memory by cp.async while the stage before is worked on;
+//   * all that does not depend on the state is made for the whole stage before and after its walk, by all threads: the
+//     step size (softplus) and its product with x before, the sum over a channel's lanes, the skip and the gate after;
+//   * inside the walk, eight tokens at a time, only one multiply-add a state value depends on the token before.
+// Tokens behind the portion's end have step size 0 and rows of zeros: they leave the state as it is.
+// 2,048 tokens of 4,096 channels with 16 states each, one request, B200: 764 us, and 26 us for the step sizes, with the
+// rows fetched into registers four tokens ahead; 137 us so
+// (31 instructions a token and warp, of which half a dozen in the prologue and epilogue of a stage; 16 lanes: 180 us, 4: 267 us).
+template <int LANES, int CH>
+struct ScanCfg {
+    static constexpr int NP = LANES * CH;
+    static constexpr int TOKENS = NP > 32 ? 16 : 32;                    // of a stage; two stages and the sums fit in 48 KB
+    static constexpr int CPB = SSM_THREADS / LANES;                     // channels of a CTA
+    static constexpr int ROWS = TOKENS * CPB;                           // one of dt, x, z
+    static constexpr int STAGE = 3 * ROWS + TOKENS * 2 * NP;            // dt | x | z | (B | C) per token
 };
 
-// exp for the decays: full precision where the result leaves in float32; through the special-function unit (relative
-// error near 2^-21) where it leaves in bfloat16, whose own rounding is a hundred times coarser.
-template <typename TO> __device__ __forceinline__ float decay_exp(float v);
-template <> __device__ __forceinline__ float decay_exp<float>(float v) { return expf(v); }
-template <> __device__ __forceinline__ float decay_exp<__nv_bfloat16>(float v) { return __expf(v); }
+__device__ __forceinline__ void scan_cp(float* dst, const float* src, bool wide, bool in) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
 
-template <int LANES, int CH, int U, typename TO>
-__global__ void __launch_bounds__(SSM_THREADS)
-selective_scan_kernel(const float* __restrict__ x, long ldx, const float* __restrict__ dtv, long lddt,
-                      const float* __restrict__ bc, long ldbc, int b_off, int c_off, const float* __restrict__ z, long ldz,
-                      const float* __restrict__ A, const void* __restrict__ D, int pdt,
-                      float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots,
-                      const int* __restrict__ q_start, const int* __restrict__ positions,
-                      TO* __restrict__ out, long ldo, int inner, int N, Segments sg) {
-    const int s = blockIdx.y, gid = blockIdx.x * SSM_THREADS + threadIdx.x;
-    const bool live = gid / LANES < inner;
-    const int c = live ? gid / LANES : inner - 1, ln = gid % LANES, n0 = ln * CH;   // lanes beyond the last channel repeat it and write nothing
-    int t0 = q_start[s];
-    int t1 = q_start[s + 1];
-    const bool fresh = positions[t0] == 0;
-    const int seg = sg.mode == 0 ? 0 : blockIdx.z;
-    const size_t seg0 = sg.mode == 0 ? 0 : (size_t)(t0 / sg.seg_len + s);          // the request's first segment in the scratch
-    if (sg.mode != 0) {
-        t0 += seg * sg.seg_len;
-        if (t0 + sg.seg_len < t1) t1 = t0 + sg.seg_len;                            // a segment beyond the portion's end walks no token
+struct ScanRowsIn {
+    const float* x; long ldx; const float* dtz; long lddt; const float* bc; long ldbc; int b_off, c_off; const float* z; long ldz;
+    bool wide, wide_bc;
+};
+
+// The rows of tokens t .. t + TOKENS - 1 of channels c0 .. c0 + CPB - 1, in pieces of UNIT (dt, x, z) and UBC (B, C)
+// numbers; zeros behind t1 and behind the last channel.
+template <int LANES, int CH, int UNIT, int UBC>
+__device__ __forceinline__ void scan_fetch_units(float* __restrict__ buf, const ScanRowsIn& in, int c0, int inner, int N, int t, int t1) {
+    using C = ScanCfg<LANES, CH>;
+    constexpr int per = C::CPB / UNIT, pb = C::NP / UBC;
+    const float* src[3] = {in.dtz, in.x, in.z};
+    const long ld[3] = {in.lddt, in.ldx, in.ldz};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll 1
+        for (int i = threadIdx.x; i < C::TOKENS * per; i += SSM_THREADS) {
+            const int tok = i / per, c = i % per * UNIT;
+            const bool ok = t + tok < t1 && c0 + c < inner;
+            scan_cp(buf + a * C::ROWS + tok * C::CPB + c, ok ? src[a] + (t + tok) * ld[a] + c0 + c : src[a], UNIT == 4, ok);
+        }
+    float* rows = buf + 3 * C::ROWS;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < C::TOKENS * 2 * pb; i += SSM_THREADS) {
+        const int tok = i / (2 * pb), r = i % (2 * pb), which = r >= pb, n = (r - which * pb) * UBC;
+        const bool ok = t + tok < t1 && n < N;
+        scan_cp(rows + tok * 2 * C::NP + which * C::NP + n, ok ? in.bc + (t + tok) * in.ldbc + (which ? in.c_off : in.b_off) + n : in.bc, UBC == 4, ok);
     }
-    const bool mine = t0 < t1 || sg.mode == 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int LANES, int CH>
+__device__ __forceinline__ void scan_fetch(float* __restrict__ buf, const ScanRowsIn& in, int c0, int inner, int N, int t, int t1) {
+    if (in.wide && in.wide_bc) scan_fetch_units<LANES, CH, 4, 4>(buf, in, c0, inner, N, t, t1);
+    else if (in.wide_bc) scan_fetch_units<LANES, CH, 1, 4>(buf, in, c0, inner, N, t, t1);
+    else scan_fetch_units<LANES, CH, 1, 1>(buf, in, c0, inner, N, t, t1);
+}
+
+// exp for the decays: full precision where the result leaves in float32; through the special-function unit (relative
+// error near 2^-21) where it leaves in bfloat16, whose own rounding is a hundred times coarser.  There the rate comes
+// times log2(e).
+template <typename TO> __device__ __forceinline__ float decay_rate(float a) { return a; }
+template <> __device__ __forceinline__ float decay_rate<__nv_bfloat16>(float a) { return a * 1.4426950408889634f; }
+template <typename TO> __device__ __forceinline__ float decay_exp(float v) { return expf(v); }
+template <> __device__ __forceinline__ float decay_exp<__nv_bfloat16>(float v) {
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v));
+    return e;
+}
+
+// the gate's silu, likewise
+template <typename TO> __device__ __forceinline__ float scan_gate(float z) { return ssm_silu(z); }
+template <> __device__ __forceinline__ float scan_gate<__nv_bfloat16>(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+
+template <int LANES, int CH, typename TO>
+__global__ void __launch_bounds__(SSM_THREADS)
+selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
+                      float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots,
+                      const int* __restrict__ q_start, const int* __restrict__ positions, TO* __restrict__ out, long ldo, int inner, int N) {
+    using C = ScanCfg<LANES, CH>;
+    constexpr int U = 8;
+    __shared__ __align__(16) float bufs[2][C::STAGE];
+    __shared__ __align__(16) float2 steps[C::ROWS];                    // (dt, dt * x) per token and channel
+    __shared__ __align__(16) float sums[C::TOKENS * SSM_THREADS];      // a lane's part of y per token
+    const int s = blockIdx.y, t0 = q_start[s], t1 = q_start[s + 1];
+    if (t1 <= t0) return;
+    const int cl = threadIdx.x / LANES, ln = threadIdx.x % LANES, n0 = ln * CH;
+    const int c0 = blockIdx.x * C::CPB, c = c0 + cl < inner ? c0 + cl : inner - 1;      // lanes beyond the last channel write nothing
+    const bool live = c0 + cl < inner;
+    scan_fetch<LANES, CH>(bufs[0], in, c0, inner, N, t0, t1);
     float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)c * N + n0;
-    const size_t lanes = (size_t)inner * N;
-    const size_t so = (seg0 + seg) * lanes + (size_t)c * N + n0;
-    const float* init = sg.mode == 2 ? (seg > 0 ? sg.end + so - lanes : sg.decay + so) : st;      // see segment_combine_kernel
-    const bool zero = !mine || sg.mode == 1 || (sg.mode == 0 && fresh);
-    float S[CH], a[CH], P[CH];
+    const bool zero = positions[t0] == 0;
+    float S[CH], a[CH];
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
-        const bool in = n0 + i < N;
-        a[i] = in ? A[(size_t)c * N + n0 + i] : 0.f;
-        P[i] = 1.f;
-        S[i] = (in && !zero) ? init[i] : 0.f;
+        const bool in_n = n0 + i < N;
+        a[i] = in_n ? decay_rate<TO>(A[(size_t)c * N + n0 + i]) : 0.f;
+        S[i] = (in_n && !zero) ? st[i] : 0.f;
     }
-    const float dskip = load_dyn(D, pdt, c);
-    const bool wants_z = ln == 0 && sg.mode != 1;
-    // The rows of U tokens are fetched while the U tokens before them are worked on (two sets of registers): at the few
-    // warps a scheduler has here, a fetch that started only after the arithmetic would be waited for in full.
-    ScanRows<U, CH> cur, nxt;
-    if (t0 < t1) cur.fetch(x, ldx, dtv, lddt, z, ldz, bc, ldbc, b_off, c_off, c, n0, N, t0, t1, wants_z);
-    for (int t = t0; t < t1; t += U) {
-        if (t + U < t1) nxt.fetch(x, ldx, dtv, lddt, z, ldz, bc, ldbc, b_off, c_off, c, n0, N, t + U, t1, wants_z);
+    // outside the walk a thread serves channel threadIdx.x % CPB of every LANES-th token
+    const int ec = threadIdx.x % C::CPB, e0 = threadIdx.x / C::CPB;
+    const int eg = c0 + ec < inner ? c0 + ec : inner - 1;
+    const float dskip = load_dyn(D, pdt, eg), bias = load_dyn(dt_bias, pdt, eg);
+    int b = 0;
+    for (int t = t0; t < t1; t += C::TOKENS, b ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (t + C::TOKENS < t1) scan_fetch<LANES, CH>(bufs[b ^ 1], in, c0, inner, N, t + C::TOKENS, t1);
+        const int n_tok = t1 - t < C::TOKENS ? t1 - t : C::TOKENS;
+        const float* rows = bufs[b];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (t + u < t1) {
-                const float dt = cur.dt[u], dx = dt * cur.x[u];
-                float y = 0.f;
+        for (int k = 0; k < C::TOKENS / LANES; ++k) {
+            const int tok = e0 + k * LANES, i = tok * C::CPB + ec;
+            const float dt = tok < n_tok ? ssm_softplus(rows[i] + bias) : 0.f;
+            steps[i] = make_float2(dt, dt * rows[C::ROWS + i]);
+        }
+        __syncthreads();
+        const float* sbc = rows + 3 * C::ROWS + n0;
+        for (int g = 0; g < n_tok; g += U) {
+            float y[U];
 #pragma unroll
-                for (int i = 0; i < CH; ++i) {
-                    const float e = decay_exp<TO>(dt * a[i]);
-                    S[i] = fmaf(e, S[i], dx * cur.b[u][i]);
-                    if (sg.mode == 1) P[i] *= e;
-                    y = fmaf(S[i], cur.c[u][i], y);
-                }
-                if (sg.mode != 1) {
+            for (int u = 0; u < U; ++u) {
+                const float2 dd = steps[(g + u) * C::CPB + cl];
+                const float* br = sbc + (g + u) * 2 * C::NP;
+                if (CH % 2 == 0) {
+                    float2 ys = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-                    if (ln == 0 && live) out[(size_t)(t + u) * ldo + c] = from_f<TO>(fmaf(dskip, cur.x[u], y) * ssm_silu(cur.z[u]));
+                    for (int i = 0; i < CH; i += 2) {
+                        const float2 b2 = *reinterpret_cast<const float2*>(br + i), c2 = *reinterpret_cast<const float2*>(br + C::NP + i);
+                        const float2 e = make_float2(decay_exp<TO>(dd.x * a[i]), decay_exp<TO>(dd.x * a[(i + 1) % CH]));
+                        const float2 S2 = __ffma2_rn(e, make_float2(S[i], S[(i + 1) % CH]), __fmul2_rn(make_float2(dd.y, dd.y), b2));
+                        S[i] = S2.x; S[(i + 1) % CH] = S2.y;
+                        ys = __ffma2_rn(S2, c2, ys);
+                    }
+                    y[u] = ys.x + ys.y;
+                } else {
+                    y[u] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < CH; ++i) {
+                        S[i] = fmaf(decay_exp<TO>(dd.x * a[i]), S[i], dd.y * br[i]);
+                        y[u] = fmaf(S[i], br[C::NP + i], y[u]);
+                    }
                 }
             }
-        }
-        cur = nxt;
-    }
-    if (!live || !mine) return;
-    if (sg.mode == 1) {
 #pragma unroll
-        for (int i = 0; i < CH; ++i) if (n0 + i < N) { sg.decay[so + i] = P[i]; sg.end[so + i] = S[i]; }
-    } else if (sg.mode == 0) {
+            for (int u = 0; u < U; ++u) sums[(g + u) * SSM_THREADS + threadIdx.x] = y[u];
+        }
+        __syncthreads();
+        if (c0 + ec < inner) {
+#pragma unroll
+            for (int k = 0; k < C::TOKENS / LANES; ++k) {
+                const int tok = e0 + k * LANES, i = tok * C::CPB + ec;
+                const float4* p = reinterpret_cast<const float4*>(sums + tok * SSM_THREADS + ec * LANES);
+                float y = 0.f;
+#pragma unroll
+                for (int j = 0; j < LANES / 4; ++j) { const float4 v = p[j]; y += (v.x + v.y) + (v.z + v.w); }
+                if (tok < n_tok) out[(size_t)(t + tok) * ldo + c0 + ec] = from_f<TO>(fmaf(dskip, rows[C::ROWS + i], y) * scan_gate<TO>(rows[2 * C::ROWS + i]));
+            }
+        }
+    }
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) if (n0 + i < N) st[i] = S[i];
+}
+
+// One token a request: a thread group lives for one token, so what counts is how many are resident and how much each
+// moves.  Four (sixteen) lanes a channel, no shared memory; 64 requests x 4,096 channels x 16 states (33.5 MB of
+// state read and written): 13.9 us, against 17.5 us with the step sizes in a launch of their own and 52 us for the walk's kernel.
+template <int LANES, int CH, typename TO>
+__global__ void __launch_bounds__(SSM_THREADS)
+selective_scan_token_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
+                            float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots,
+                            const int* __restrict__ q_start, const int* __restrict__ positions, TO* __restrict__ out, long ldo, int inner, int N) {
+    const int s = blockIdx.y, t = q_start[s], gid = blockIdx.x * SSM_THREADS + threadIdx.x;
+    if (q_start[s + 1] <= t) return;
+    const bool live = gid / LANES < inner;
+    const int c = live ? gid / LANES : inner - 1, ln = gid % LANES, n0 = ln * CH;   // lanes beyond the last channel repeat it and write nothing
+    float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)c * N + n0;
+    const bool zero = positions[t] == 0;
+    const float* br = in.bc + t * in.ldbc + in.b_off + n0;
+    const float* cr = in.bc + t * in.ldbc + in.c_off + n0;
+    float S[CH], a[CH], bv[CH], cv[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+        const bool ok = n0 + i < N;
+        S[i] = (ok && !zero) ? st[i] : 0.f;
+        a[i] = ok ? decay_rate<TO>(A[(size_t)c * N + n0 + i]) : 0.f;
+        bv[i] = ok ? br[i] : 0.f;
+        cv[i] = ok ? cr[i] : 0.f;
+    }
+    const float x = in.x[t * in.ldx + c], z = in.z[t * in.ldz + c];
+    const float dt = ssm_softplus(in.dtz[t * in.lddt + c] + load_dyn(dt_bias, pdt, c)), dx = dt * x;
+    float y = 0.f;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+        S[i] = fmaf(decay_exp<TO>(dt * a[i]), S[i], dx * bv[i]);
+        y = fmaf(S[i], cv[i], y);
+    }
+    if (live) {
 #pragma unroll
         for (int i = 0; i < CH; ++i) if (n0 + i < N) st[i] = S[i];
     }
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (ln == 0 && live) out[t * ldo + c] = from_f<TO>(fmaf(load_dyn(D, pdt, c), x, y) * scan_gate<TO>(z));
 }
 
 // Between the two passes: end[k] becomes the state at the end of segment k with the true start, one after another;
@@ -317,72 +423,62 @@ using namespace aien;
 AIEN_API long aien_ssm_segments_scratch(int T, int S, int seg_len, long lanes) { return 2L * (T / seg_len + S) * lanes; }
 
 struct ScanArgs {
-    const float* x; long ldx; float* dtz; long lddt; const float* bc; long ldbc; int b_off, c_off; const float* z; long ldz;
-    const float* A; const void* dt_bias; const void* D; int p_dt; float* state; size_t state_stride, s_off; const int* slots;
-    const int* q_start; const int* positions; void* out; long ldo; int T, S, inner, N; Segments sg; cudaStream_t stream;
+    ScanRowsIn in; const float* A; const void* dt_bias; const void* D; int p_dt; float* state; size_t state_stride, s_off; const int* slots;
+    const int* q_start; const int* positions; void* out; long ldo; int T, S, inner, N; cudaStream_t stream;
 };
 
-template <int LANES, int CH, int U, typename TO>
+template <int LANES, int CH, typename TO>
 static void launch_selective_scan(const ScanArgs& a) {
-    auto kern = selective_scan_kernel<LANES, CH, U, TO>;
-    const unsigned gx = (unsigned)(((long)a.inner * LANES + SSM_THREADS - 1) / SSM_THREADS);
-    Segments sg = a.sg;
-    const dim3 grid(gx, a.S, sg.mode == 0 ? 1 : sg.nseg);
-    step_sizes_kernel<<<dim3((a.inner + 255) / 256, a.T), 256, 0, a.stream>>>(a.dtz, a.lddt, a.dt_bias, a.p_dt, a.T, a.inner);
-    kern<<<grid, SSM_THREADS, 0, a.stream>>>(a.x, a.ldx, a.dtz, a.lddt, a.bc, a.ldbc, a.b_off, a.c_off, a.z, a.ldz, a.A, a.D, a.p_dt,
-                                             a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
-    if (sg.mode == 0) return;
-    const size_t lanes = (size_t)a.inner * a.N;
-    segment_combine_kernel<<<dim3((unsigned)((lanes + 255) / 256), a.S), 256, 0, a.stream>>>(a.state, a.state_stride, a.s_off, a.slots, a.q_start,
-                                                                                             a.positions, sg, lanes);
-    sg.mode = 2;
-    kern<<<grid, SSM_THREADS, 0, a.stream>>>(a.x, a.ldx, a.dtz, a.lddt, a.bc, a.ldbc, a.b_off, a.c_off, a.z, a.ldz, a.A, a.D, a.p_dt,
-                                             a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+    using C = ScanCfg<LANES, CH>;
+    selective_scan_kernel<LANES, CH, TO><<<dim3((unsigned)((a.inner + C::CPB - 1) / C::CPB), a.S), SSM_THREADS, 0, a.stream>>>(
+        a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N);
 }
 
+template <int LANES, int CH, typename TO>
+static void launch_selective_scan_token(const ScanArgs& a) {
+    const unsigned gx = (unsigned)(((long)a.inner * LANES + SSM_THREADS - 1) / SSM_THREADS);
+    selective_scan_token_kernel<LANES, CH, TO><<<dim3(gx, a.S), SSM_THREADS, 0, a.stream>>>(
+        a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N);
+}
+
+// Eight lanes a channel; with fewer than 2,048 channels in the step, whose walkers would leave SM schedulers without a
+// warp, and with many state values, sixteen.
 template <typename TO>
 static int dispatch_selective_scan(const ScanArgs& a) {
     const int N = a.N;
+    const bool few = (long)a.inner * a.S < 2048;
     if (N > 128) return AIEN_E_SHAPE;
     if (a.T == a.S) {
-        // single tokens: a CTA lives for one token, so what counts is how many are resident and how much each moves:
-        // four lanes a channel, no rows fetched ahead (fewer registers)
-        if (N <= 4) launch_selective_scan<4, 1, 1, TO>(a);
-        else if (N <= 8) launch_selective_scan<4, 2, 1, TO>(a);
-        else if (N <= 16) launch_selective_scan<4, 4, 1, TO>(a);
-        else if (N <= 32) launch_selective_scan<4, 8, 1, TO>(a);
-        else if (N <= 64) launch_selective_scan<16, 4, 1, TO>(a);
-        else launch_selective_scan<16, 8, 1, TO>(a);
+        if (N <= 4) launch_selective_scan_token<4, 1, TO>(a);
+        else if (N <= 8) launch_selective_scan_token<4, 2, TO>(a);
+        else if (N <= 16) launch_selective_scan_token<4, 4, TO>(a);
+        else if (N <= 32) launch_selective_scan_token<4, 8, TO>(a);
+        else if (N <= 64) launch_selective_scan_token<16, 4, TO>(a);
+        else launch_selective_scan_token<16, 8, TO>(a);
         return 0;
     }
-    if (N <= 2) launch_selective_scan<1, 2, 4, TO>(a);
-    else if (N <= 8) launch_selective_scan<4, 2, 4, TO>(a);
-    else if (N <= 16) launch_selective_scan<16, 1, 4, TO>(a);
-    else if (N <= 32) launch_selective_scan<16, 2, 4, TO>(a);
-    else if (N <= 64) launch_selective_scan<16, 4, 4, TO>(a);
-    else launch_selective_scan<16, 8, 2, TO>(a);
+    if (N <= 8) launch_selective_scan<8, 1, TO>(a);
+    else if (N <= 16) { if (few) launch_selective_scan<16, 1, TO>(a); else launch_selective_scan<8, 2, TO>(a); }
+    else if (N <= 32) { if (few) launch_selective_scan<16, 2, TO>(a); else launch_selective_scan<8, 4, TO>(a); }
+    else if (N <= 64) launch_selective_scan<16, 4, TO>(a);
+    else launch_selective_scan<16, 8, TO>(a);
     return 0;
 }
 
-// x [T, ldx] (after convolution and silu), dtz [T, lddt] = W_dt dt before its bias (overwritten with the step sizes
-// softplus(dtz + dt_bias)), bc [T, ldbc] with B at b_off and C at c_off (N numbers each, N <= 128), z [T, ldz] the gate's
-// input, A float32 [inner, N] (negative rates), dt_bias and D [inner] in p_dt.  seg_len > 0: portions are cut into nseg
-// segments of seg_len tokens that run side by side (scratch float32, aien_ssm_segments_scratch(T, S, seg_len, inner * N)
-// numbers); nseg * seg_len must cover the longest portion; T is the number of tokens in the step.
-AIEN_API int aien_selective_scan(const float* x, long ldx, float* dtz, long lddt, const float* bc, long ldbc, int b_off, int c_off,
+// x [T, ldx] (after convolution and silu), dtz [T, lddt] = W_dt dt before its bias, bc [T, ldbc] with B at b_off and C at
+// c_off (N numbers each, N <= 128), z [T, ldz] the gate's input, A float32 [inner, N] (negative rates), dt_bias and D
+// [inner] in p_dt.  T is the number of tokens in the step.
+AIEN_API int aien_selective_scan(const float* x, long ldx, const float* dtz, long lddt, const float* bc, long ldbc, int b_off, int c_off,
                                  const float* z, long ldz, const float* A, const void* dt_bias, const void* D, int p_dt,
                                  float* state, size_t state_stride, size_t s_off, const int* slots, const int* q_start,
-                                 const int* positions, void* out, int o_dt, long ldo, int T, int S, int inner, int N,
-                                 int seg_len, int nseg, float* scratch, cudaStream_t stream) {
+                                 const int* positions, void* out, int o_dt, long ldo, int T, int S, int inner, int N, cudaStream_t stream) {
     if (S <= 0 || T <= 0) return 0;
-    if (inner <= 0 || N <= 0 || S > 65535 || T > 65535 || nseg > 65535) return AIEN_E_SHAPE;
-    Segments sg{0, 0, nullptr, nullptr, 1};
-    if (seg_len > 0 && nseg > 1) {
-        if (scratch == nullptr) return AIEN_E_SHAPE;
-        sg = Segments{1, seg_len, scratch, scratch + (size_t)(T / seg_len + S) * (size_t)inner * N, nseg};
-    }
-    const ScanArgs a{x, ldx, dtz, lddt, bc, ldbc, b_off, c_off, z, ldz, A, dt_bias, D, p_dt, state, state_stride, s_off, slots, q_start,
-                     positions, out, ldo, T, S, inner, N, sg, stream};
+    if (inner <= 0 || N <= 0 || S > 65535) return AIEN_E_SHAPE;
+    const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dtz) | reinterpret_cast<uintptr_t>(z)) & 15) == 0 &&
+                      ((ldx | lddt | ldz | inner) & 3) == 0;
+    const bool wide_bc = (reinterpret_cast<uintptr_t>(bc) & 15) == 0 && ((ldbc | b_off | c_off | N) & 3) == 0;
+    const ScanArgs a{{x, ldx, dtz, lddt, bc, ldbc, b_off, c_off, z, ldz, wide, wide_bc}, A, dt_bias, D, p_dt, state, state_stride, s_off, slots,
+                     q_start, positions, out, ldo, T, S, inner, N, stream};
     int rc = 0;
     AIEN_DISPATCH_DTYPE(o_dt, TO, (rc = dispatch_selective_scan<TO>(a)));
     if (rc != 0) return rc;

@@ -191,7 +191,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "aien_paged_attention_decode_fused": [P, L, P, L, P, L, P, P, I, F, P, P, I, P, P, P, P, I, P, P, L, P, P, P,
                                               I, I, I, I, I, F, I, I, P],
         "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
-        "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, I, I, P, P],
+        "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, P],
         "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, P],
         "aien_gate_group_norm": [P, L, P, L, P, I, F, F, P, I, L, I, I, I, P],
         "aien_scaled_add_rmsnorm": [P, P, I, I, c_size_t, P, P, P, I, F, P, I, I, I, P],
@@ -1889,23 +1889,18 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
                    scratch: Optional[torch.Tensor] = None) -> None:
     """The selective scan over every request's portion: per channel c and state n, token by token,
     dt = softplus(dtz[c] + dt_bias[c]); S[c, n] = exp(dt * A[c, n]) * S[c, n] + dt * x[c] * B[n]; y[c] = sum_n S[c, n] * C[n]
-    + D[c] * x[c]; out[c] = y[c] * silu(z[c]).  x, dtz, z float32 [T, inner] (row strides free; dtz is overwritten with the
-    step sizes); B and C are the N numbers
-    from columns ``b_off`` / ``c_off`` of the float32 rows ``bc``; A float32 [inner, N]; S lives in the request's state row
-    from ``s_off`` on ([inner, N]) and starts from zeros where a portion's first token has position 0."""
+    + D[c] * x[c]; out[c] = y[c] * silu(z[c]).  x, dtz, z float32 [T, inner] (row strides free); B and C are the N numbers from columns ``b_off`` / ``c_off`` of the float32 rows ``bc``; A float32 [inner, N]; S lives in the request's state row
+    from ``s_off`` on ([inner, N]) and starts from zeros where a portion's first token has position 0.  Every portion is
+    walked in one piece: ``seg_len``, ``nseg`` and ``scratch`` (see :func:`scan_segments`) may be given and change nothing."""
     _dev(x, dtz, bc, z, A, dt_bias, D, state, slot_map, q_start, positions, out, scratch)
     T, inner = x.shape
     for t in (x, dtz, bc, z):
         assert t.dtype == torch.float32 and t.stride(1) == 1
     assert A.dtype == torch.float32 and A.is_contiguous() and tuple(A.shape) == (inner, N) and dt_bias.dtype == D.dtype
     assert dt_bias.is_contiguous() and D.is_contiguous() and state.dtype == torch.float32 and state.stride(-1) == 1 and out.stride(1) == 1
-    if seg_len and nseg > 1:
-        assert scratch is not None and scratch.numel() >= 2 * (T // seg_len + num_seqs) * inner * N
     _check(lib().aien_selective_scan(_p(x), x.stride(0), _p(dtz), dtz.stride(0), _p(bc), bc.stride(0), int(b_off), int(c_off), _p(z), z.stride(0),
                                      _p(A), _p(dt_bias), _p(D), dt(D), _p(state), state.stride(0), int(s_off), _p(slot_map), _p(q_start),
-                                     _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), int(seg_len), int(nseg),
-                                     _p(scratch), _stream()), "selective_scan")
-    add_launches(3 if (seg_len and nseg > 1) else 1)
+                                     _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), _stream()), "selective_scan")
 
 
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,

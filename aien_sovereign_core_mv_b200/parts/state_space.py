@@ -106,7 +106,7 @@ class SelectiveScan(Mixer):
     def workspace_bytes(self, lim):
         I, N, R = self.inner, self.state, self.dt_rank
         return lim.max_tokens * ((2 * I + I + (R + 2 * N) + I) * 4 + 2 * I * lim.itemsize + self.hidden_size * 4) + 16384 \
-            + 2 * K.PARTIALS_MAX_BYTES + 4 * K.scan_scratch_floats(lim.max_tokens, lim.max_seqs, I * N, I * min(N, 16))
+            + 2 * K.PARTIALS_MAX_BYTES
 
     def forward(self, ctx: StepContext, h: torch.Tensor, run: RunBinding):
         T, I, N, R = ctx.num_tokens, self.inner, self.state, self.dt_rank
@@ -122,9 +122,8 @@ class SelectiveScan(Mixer):
         xp = linear(ctx, xa, self.w_x, out_dtype=torch.float32)                         # dt | B | C
         dtz = linear(ctx, xp[:, :R], self.w_dt, out_dtype=torch.float32)                # float32 step sizes into the softplus
         y = ws.take((T, I), ctx.dtype)
-        seg, nseg, scratch = _segments(ctx, I * N, I * min(N, 16))
         K.selective_scan(x, dtz, xp, R, R + N, proj[:, I:], self.A, self.dt_b, self.D, state, self.conv_floats, group.slot_map,
-                         ctx.q_start, ctx.positions, y, ctx.num_seqs, N, seg, nseg, scratch)
+                         ctx.q_start, ctx.positions, y, ctx.num_seqs, N)
         return linear(ctx, y, self.w_o, out_dtype=torch.float32, may_defer_sum=True)
 
 

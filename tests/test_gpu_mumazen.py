@@ -281,6 +281,34 @@ def test_selective_scan_cut_any_way(inner, N):
         assert float((state[:, :s_off] - 7.0).abs().max()) == 0.0 and float((state[0] - 7.0).abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("inner,N,lens", [(2052, 16, [70, 33, 1]), (2049, 15, [9]), (1030, 32, [31, 2, 65]), (4100, 8, [40]), (2052, 16, [1, 1, 1]),
+                                          (2050, 70, [1, 1])])
+def test_selective_scan_many_channels_16_bit_results(inner, N, lens):
+    """The walk with eight lanes a channel (2,048 channels and more), rows that 16-byte copies take and rows they do not,
+    and the single-token form, with results in bfloat16: half a unit in the last place (2^-9) of the largest, twice."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(inner + N)
+    T, S, R = sum(lens), len(lens), 4
+    A = -torch.exp(torch.rand(inner, N, generator=g) * 4.0 - 3.0)
+    D, bias = torch.rand(inner, generator=g) + 0.5, torch.rand(inner, generator=g) * 2.0 - 3.0
+    x, dtz, z, bc = (torch.randn(T, n, generator=g) for n in (inner, inner, inner, R + 2 * N))
+    first = torch.randn(S, inner, N, generator=g)
+    state = torch.zeros(S + 1, inner * N)
+    state[1:] = first.reshape(S, -1)
+    state = state.cuda()
+    q = [sum(lens[:i]) for i in range(S + 1)]
+    out = torch.zeros(T, inner, dtype=torch.bfloat16).cuda()
+    K.selective_scan(x.cuda(), dtz.cuda(), bc.cuda(), R, R + N, z.cuda(), A.cuda(), bias.cuda(), D.cuda(), state, 0, i32([s + 1 for s in range(S)]),
+                     i32(q), i32([5 + p for n in lens for p in range(n)]), out, S, N)
+    for s in range(S):
+        r = slice(q[s], q[s + 1])
+        y, last = pz.selective_scan(f64(x[r]), pz.softplus(f64(dtz[r]) + f64(bias)), f64(A), f64(bc[r][:, R:R + N]), f64(bc[r][:, R + N:]), f64(D),
+                                    f64(first[s]))
+        H.assert_close(out[r].float().cpu().numpy(), y * pz.silu(f64(z[r])), 4e-3, f"request {s}")
+        H.assert_close(state[s + 1].view(inner, N).cpu().numpy(), last, 1e-5, f"state of request {s}")
+    assert float(state[0].abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("heads,V,G,N", [(3, 8, 1, 5), (4, 16, 2, 24), (6, 24, 3, 40), (2, 64, 1, 128), (1, 40, 1, 200)])
 def test_state_space_duality_cut_any_way(heads, V, G, N):
     from aien_sovereign_core_mv_b200 import kernels as K
