@@ -413,6 +413,35 @@ def test_convolution_norms_and_cache_rows_of_the_attention(dtype, taps, heads, k
         H.assert_close(k_, want_k[0], tol, "cached keys, portions"); H.assert_close(v_, want_v[0], tol, "cached values, portions")
 
 
+@pytest.mark.parametrize("taps,qk,dim,heads,vdim,lens", [(4, 8, 128, 16, 128, [1, 2, 3, 5, 130, 7, 152]), (3, 1, 64, 3, 20, [4, 1, 9]), (2, 2, 8, 2, 12, [1, 1])])
+def test_delta_preparation_in_runs_is_the_same(taps, qk, dim, heads, vdim, lens):
+    """Four channels a thread over runs of tokens against one channel a thread (the same rows one column further on):
+    values, gates and slots to the bit; unit vectors up to the order of their sums (2^-22 relative)."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    g = torch.Generator().manual_seed(taps * 1000 + dim)
+    T, S, QK, C = sum(lens), len(lens), qk * dim, 2 * qk * dim + heads * vdim
+    n = C + 2 * heads
+    u = torch.randn(T, n, generator=g).cuda()
+    ws = [torch.randn(c, taps, generator=g).to(torch.bfloat16).cuda() for c in (QK, QK, heads * vdim)]
+    a_log, dt_bias = torch.randn(heads, generator=g).cuda(), torch.randn(heads, generator=g).cuda()
+    q = [sum(lens[:i]) for i in range(S + 1)]
+    pos = [p + (0 if s % 3 == 1 else 9) for s, m in enumerate(lens) for p in range(m)]
+    sot = [s for s, m in enumerate(lens) for _ in range(m)]
+    kept = torch.randn(S + 2, ((taps - 1) * C + 7) // 4 * 4, generator=g).cuda()
+    got = []
+    for off in (0, 1):
+        rows = torch.zeros(T, (n + 8) // 4 * 4).cuda()
+        rows[:, off:off + n] = u
+        state, out, gb = kept.clone(), torch.zeros(T, C).cuda(), torch.zeros(T, 2 * heads).cuda()
+        K.delta_conv_prepare(rows, off, off + QK, off + 2 * QK, off + C, off + C + heads, qk, dim, heads, vdim, *ws, taps, a_log, dt_bias, state,
+                             i32([S - s for s in range(S)]), i32(sot), i32(q), i32(pos), out, gb)
+        got.append((out, gb, state))
+    (o0, g0, s0), (o1, g1, s1) = got
+    assert torch.equal(o0[:, 2 * QK:], o1[:, 2 * QK:]) and torch.equal(g0, g1) and torch.equal(s0, s1)
+    assert float((o0 - o1).abs().max()) <= 2.0 ** -22 and float(o0[:, :2 * QK].abs().max()) <= 1.001
+
+
 @pytest.mark.parametrize("taps,heads,qk,dim,vdim,slow", [(4, 3, 1, 20, 12, False), (1, 2, 2, 16, 40, True), (3, 4, 2, 64, 64, True), (2, 1, 1, 130, 8, False),
                                                          (3, 6, 3, 32, 64, False), (5, 4, 1, 6, 10, True)])
 def test_delta_rule_in_one_step_in_pieces_and_token_by_token(taps, heads, qk, dim, vdim, slow):

@@ -239,6 +239,32 @@ def test_convolution_with_bias_across_portions_and_slots(taps, channels):
     H.assert_close(out.cpu().numpy(), want[1], 3e-6, "a used slot")
 
 
+@pytest.mark.parametrize("taps,channels,lens", [(2, 2048, [1, 1, 1]), (3, 512, [5, 1, 2, 40]), (4, 4096, [1, 2, 3, 5, 130, 7, 252]), (4, 260, [3, 9]), (4, 512, [1])])
+def test_convolution_in_runs_is_the_same_to_the_bit(taps, channels, lens):
+    """Four channels a thread over runs of tokens (16-byte rows) against one channel a thread (the same rows one column
+    further on): portions shorter than the taps, runs that begin inside a portion's first tokens, slots that are
+    rewritten; float32 and bfloat16 results, new requests and old ones."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(taps * 1000 + channels)
+    T, S = sum(lens), len(lens)
+    u = torch.randn(T, channels + 8, generator=g).cuda()
+    w, b = torch.randn(channels, taps, generator=g).to(torch.bfloat16).cuda(), torch.randn(channels, generator=g).cuda()
+    q = [sum(lens[:i]) for i in range(S + 1)]
+    pos = [p + (0 if s % 3 == 1 else 9) for s, n in enumerate(lens) for p in range(n)]
+    sot = [s for s, n in enumerate(lens) for _ in range(n)]
+    kept = torch.randn(S + 2, (taps - 1) * channels + 4, generator=g).cuda()
+    got = []
+    for off in (4, 5):
+        rows = torch.zeros(T, channels + 8).cuda()
+        rows[:, off:off + channels] = u[:, 4:4 + channels]
+        state = kept.clone()
+        out, out16 = torch.zeros(T, channels).cuda(), torch.zeros(T, channels, dtype=torch.bfloat16).cuda()
+        K.conv_act(rows, off, channels, w, b, taps, "silu", state, i32([S - s for s in range(S)]), i32(sot), i32(q), i32(pos), out, out16)
+        got.append((out, out16, state))
+    for a, c, what in zip(got[0], got[1], ("float32", "bfloat16", "state")):
+        assert torch.equal(a, c), what
+
+
 @pytest.mark.parametrize("inner,N", [(37, 5), (64, 16), (130, 24), (48, 40), (20, 100)])
 def test_selective_scan_cut_any_way(inner, N):
     """Whole, in portions down to one token, and in side-by-side segments: the same numbers.  One channel decays so slowly
