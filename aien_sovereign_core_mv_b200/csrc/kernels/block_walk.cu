@@ -1,0 +1,436 @@
+// Portions of prompts through recurrences with a state matrix and one decay per head and token, sixteen tokens at a time.
+//
+//   S <- g S + k u^T ,  o = S^T q        u = v (linear attention; state-space duality with k = B, q = C, v = dt x), or
+//                                        u = beta (v - (g S)^T k) (the delta rule)
+//
+// Written out over a block of 16 tokens that finds the state S0, with G_i the product of the decays up to token i and
+// G_i/G_j the product of those behind j up to i:
+//   p_i = S0^T k_i ,  r_i = S0^T q_i
+//   u_i = beta_i (v_i - G_i p_i - sum_{j<i} G_i/G_j (k_i.k_j) u_j)   that is   u = M (v - G p)
+//   o_i = G_i r_i + sum_{j<=i} G_i/G_j (q_i.k_j) u_j                 that is   o = G r + A u
+//   S   = G_16 S0 + sum_j G_16/G_j k_j u_j^T
+// A, M (16 x 16, lower triangular), G and G_16/G_j depend on the rows alone.  A first kernel makes them for every block
+// and head side by side (M by forward substitution in float32); a second one walks a request's blocks in order with a CTA
+// for 16 columns of a head's state.  There S0^T [q | k] and the update are matrix products over the 16 columns, and what
+// a token waits for is one sixteenth of a block's chain instead of a chain of its own.
+//
+// The products run on the tensor cores (mma.sync tf32) with every float32 operand cut in two: x = hi + lo, hi the nearest
+// number of 11 bits, lo the rest, and x y = hi hi + hi lo + lo hi; what is dropped is 2^-22 of a product and has no sign
+// of its own.  tcgen05 would have to find the state in shared memory for every block's product; here the eight warps share
+// its rows and each keeps its own as accumulators: [16 columns] x [8 rows] fragments whose register order is the order of
+// the left operand once the rows of a fragment are counted 0 2 4 6 1 3 5 7 on both sides.  The update is accumulated from
+// zero and added to the decayed state by one float32 multiply-add, so the state is rounded once per block.
+//
+// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 186 us and 16 for the coefficients (603 token by
+// token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 113 and 6 us (540).
+#include "common.cuh"
+#include <math.h>
+
+namespace aien {
+
+constexpr int BW_B = 16;                       // tokens of a block
+constexpr int BW_COLS = 16;                    // state columns of a CTA
+constexpr int BW_WARPS = 8;
+constexpr int BW_THREADS = 32 * BW_WARPS;
+constexpr int BW_LD = 20;                      // floats between rows of A, M and of the partial sums: no bank twice in a quarter warp
+constexpr int BW_LDV = 24;                     // floats between rows of v and u
+constexpr int BW_COEF = 2 * BW_B * BW_B + 2 * BW_B;      // A | M | G | G_16 / G_j per block and head
+
+__device__ __forceinline__ void bw_split(float x, uint32_t& hi, uint32_t& lo) {
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi));
+}
+
+__device__ __forceinline__ void bw_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// c += a b, the small products first
+__device__ __forceinline__ void bw_mma3(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[2], const uint32_t (&bl)[2]) {
+    bw_mma(c, al, bh);
+    bw_mma(c, ah, bl);
+    bw_mma(c, ah, bh);
+}
+
+__device__ __forceinline__ void bw_cp16(float* dst, const float* src, bool in) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+struct BlockWalk {
+    const float* rows; long ld; int q_off, k_off, v_off;        // q, k: G heads of N numbers; v: `heads` heads of V
+    const float* gates; long ldg; int g_off, w_off;             // decay of head h in column g_off + h; its weight (beta, or the step size) in w_off + h (w_off < 0: 1)
+    const float* decay;                                         // or one decay per head for all tokens
+    float* act_rows; long ld_act;                               // with `act`: silu of q | k | v goes here first and is read from here
+    int act, delta;
+    float* coef;
+    const void* skip_any; int skip_dt;       // o += skip[h] * v (null: no such term)
+    float* state; size_t state_stride, s_off; int state_vn;     // state_vn: a head's state is [V][N], else [N][V]
+    const int* slots; const int* q_start; const int* positions;
+    float* out; long ldo;
+    int T, S, heads, G, N, V;
+};
+
+// the request whose blocks include block slot b; request s's blocks start at q_start[s] / 16 + s
+__device__ __forceinline__ int bw_first_block(const int* q_start, int s) { return q_start[s] / BW_B + s; }
+
+__device__ __forceinline__ float bw_silu(float z) { return z / (1.0f + expf(-z)); }
+
+// One CTA per (block, q/k head): its dot products once, then A, M and the decays of every head that shares the q/k head.
+__global__ void __launch_bounds__(256)
+block_coef_kernel(const BlockWalk a) {
+    extern __shared__ __align__(16) float bw_smem[];
+    __shared__ float dots[2][BW_B * BW_B];                      // q_i . k_j and k_i . k_j
+    const int slot = blockIdx.x, kvh = blockIdx.y;
+    int lo = 0, hi = a.S - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (bw_first_block(a.q_start, mid) <= slot) lo = mid; else hi = mid - 1;
+    }
+    const int s = lo, t0 = a.q_start[s] + (slot - bw_first_block(a.q_start, s)) * BW_B, end = a.q_start[s + 1];
+    const int n = end - t0 < BW_B ? end - t0 : BW_B;
+    if (n <= 0) return;
+    const int per = a.heads / a.G, N = a.N, LDN = N + 4;
+    float* sq = bw_smem;                                        // [16][N + 4]
+    float* sk = sq + BW_B * LDN;
+    float* sg = sk + BW_B * LDN;                                // [16][per] decays, then [16][per] weights
+    float* sw = sg + BW_B * per;
+    float* sl = sw + BW_B * per;                                // [per][16][16] the strictly lower part of I + L (the delta rule)
+    const int tid = threadIdx.x;
+    for (int i = tid; i < BW_B * (N / 4); i += 256) {
+        const int t = i / (N / 4), c = (i - t * (N / 4)) * 4;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
+        if (t < n) {
+            const float* r = a.rows + (size_t)(t0 + t) * a.ld + (size_t)kvh * N + c;
+            q = __ldcg(reinterpret_cast<const float4*>(r + a.q_off));
+            k = __ldcg(reinterpret_cast<const float4*>(r + a.k_off));
+            if (a.act) {
+                q = make_float4(bw_silu(q.x), bw_silu(q.y), bw_silu(q.z), bw_silu(q.w));
+                k = make_float4(bw_silu(k.x), bw_silu(k.y), bw_silu(k.z), bw_silu(k.w));
+                float* w = a.act_rows + (size_t)(t0 + t) * a.ld_act + (size_t)kvh * N + c;
+                *reinterpret_cast<float4*>(w) = q;
+                *reinterpret_cast<float4*>(w + a.G * N) = k;
+            }
+        }
+        *reinterpret_cast<float4*>(sq + t * LDN + c) = q;
+        *reinterpret_cast<float4*>(sk + t * LDN + c) = k;
+    }
+    if (a.act) {
+        const int cols = per * a.V / 4;
+        for (int i = tid; i < n * cols; i += 256) {
+            const int t = i / cols, c = kvh * per * a.V + (i - t * cols) * 4;
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(a.rows + (size_t)(t0 + t) * a.ld + a.v_off + c));
+            *reinterpret_cast<float4*>(a.act_rows + (size_t)(t0 + t) * a.ld_act + 2 * a.G * N + c) =
+                make_float4(bw_silu(v.x), bw_silu(v.y), bw_silu(v.z), bw_silu(v.w));
+        }
+    }
+    for (int i = tid; i < BW_B * per; i += 256) {
+        const int t = i / per, h = kvh * per + i - t * per;
+        float g = 1.f, w = 0.f;
+        if (t < n) {
+            g = a.gates != nullptr ? a.gates[(size_t)(t0 + t) * a.ldg + a.g_off + h] : a.decay[h];
+            w = a.w_off >= 0 ? a.gates[(size_t)(t0 + t) * a.ldg + a.w_off + h] : 1.f;
+        }
+        sg[i] = g;
+        sw[i] = w;
+    }
+    __syncthreads();
+    {
+        const int i = tid >> 4, j = tid & 15;
+        const float4* q4 = reinterpret_cast<const float4*>(sq + i * LDN);
+        const float4* ki4 = reinterpret_cast<const float4*>(sk + i * LDN);
+        const float4* kj4 = reinterpret_cast<const float4*>(sk + j * LDN);
+        float x0 = 0.f, x1 = 0.f, y0 = 0.f, y1 = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < N / 4; ++c) {
+            const float4 q = q4[c], b = kj4[c];
+            x0 = fmaf(q.x, b.x, x0); x1 = fmaf(q.y, b.y, x1); x0 = fmaf(q.z, b.z, x0); x1 = fmaf(q.w, b.w, x1);
+            if (a.delta) {
+                const float4 k = ki4[c];
+                y0 = fmaf(k.x, b.x, y0); y1 = fmaf(k.y, b.y, y1); y0 = fmaf(k.z, b.z, y0); y1 = fmaf(k.w, b.w, y1);
+            }
+        }
+        dots[0][tid] = x0 + x1;
+        dots[1][tid] = y0 + y1;
+    }
+    __syncthreads();
+    // a thread owns column j of one head's matrices: the product of the decays grows by one factor a row
+    for (int u = tid; u < per * BW_B; u += 256) {
+        const int hh = u >> 4, j = u & 15;
+        float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF;
+        const float wj = a.delta ? 1.f : sw[j * per + hh], g0 = sg[hh];
+        float ratio = 1.f;
+#pragma unroll
+        for (int i = 0; i < BW_B; ++i) {
+            if (i > j) ratio *= sg[i * per + hh];
+            c[i * 16 + j] = i >= j ? ratio * dots[0][i * 16 + j] * wj : 0.f;
+            if (a.delta) sl[hh * 256 + i * 16 + j] = i > j ? sw[i * per + hh] * ratio * dots[1][i * 16 + j] : 0.f;
+            if (j == 0) c[512 + i] = g0 * ratio;
+        }
+        c[512 + 16 + j] = ratio * wj;
+    }
+    if (!a.delta) return;
+    __syncthreads();
+    // (I + L)^-1 column by column: a thread owns one column of one head
+    for (int u = tid; u < per * BW_B; u += 256) {
+        const int hh = u >> 4, col = u & 15;
+        const float* L = sl + hh * 256;
+        const float beta = sw[col * per + hh];
+        float x[BW_B];
+#pragma unroll
+        for (int r = 0; r < BW_B; ++r) {
+            float v = r == col ? 1.f : 0.f;
+#pragma unroll
+            for (int m = 0; m < r; ++m) v = fmaf(-L[r * 16 + m], x[m], v);
+            x[r] = v;
+        }
+        float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF + 256;
+#pragma unroll
+        for (int r = 0; r < BW_B; ++r) c[r * 16 + col] = x[r] * beta;
+    }
+}
+
+// NT: fragments of 8 rows that a warp owns; N <= 64 NT.
+template <int NT>
+struct BwSmem {
+    static constexpr int LDN = 64 * NT + 8;                     // floats between rows of q and k: a half warp's 8-byte reads meet no bank twice
+    static constexpr int QK = BW_B * LDN;
+    static constexpr int STAGE = 2 * QK + BW_B * BW_LDV + 2 * BW_B * BW_LD + 2 * BW_B;     // q | k | v | A | M | G | G_16 / G_j
+    static constexpr int PART = BW_WARPS * BW_B * BW_LD;
+    static constexpr int TOTAL = 2 * STAGE + 2 * PART + BW_B * BW_LDV;                     // two stages, partial sums of p and r, u
+};
+
+template <int NT, bool DELTA>
+__device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWalk& a, const float* rows, long ld, int q_col, int k_col, int v_col,
+                                         int cols, const float* coef, int t, int t1) {
+    using C = BwSmem<NT>;
+    const int tid = threadIdx.x, pieces = 16 * NT;              // 16-byte pieces of a padded row
+#pragma unroll
+    for (int i = tid; i < BW_B * pieces; i += BW_THREADS) {
+        const int tok = i / pieces, c = i % pieces * 4;
+        const bool in = t + tok < t1 && c < a.N;
+        const float* r = in ? rows + (size_t)(t + tok) * ld + c : rows;
+        bw_cp16(buf + tok * C::LDN + c, r + (in ? q_col : 0), in);
+        bw_cp16(buf + C::QK + tok * C::LDN + c, r + (in ? k_col : 0), in);
+    }
+    if (tid < 64) {
+        const int tok = tid >> 2, c = (tid & 3) * 4;
+        const bool in = t + tok < t1 && c < cols;
+        bw_cp16(buf + 2 * C::QK + tok * BW_LDV + c, in ? rows + (size_t)(t + tok) * ld + v_col + c : rows, in);
+    } else if (tid < 128) {
+        const int e = tid - 64;
+        bw_cp16(buf + 2 * C::QK + BW_B * BW_LDV + (e >> 2) * BW_LD + (e & 3) * 4, coef + e * 4, true);
+    } else if (tid < 192) {
+        const int e = tid - 128;
+        if (DELTA) bw_cp16(buf + 2 * C::QK + BW_B * BW_LDV + BW_B * BW_LD + (e >> 2) * BW_LD + (e & 3) * 4, coef + 256 + e * 4, true);
+    } else if (tid < 200) {
+        const int e = tid - 192;
+        bw_cp16(buf + 2 * C::QK + BW_B * BW_LDV + 2 * BW_B * BW_LD + e * 4, coef + 512 + e * 4, true);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// partial products S0^T x of a warp's rows, x the q or k rows of a block: [16 columns] x [16 tokens] into part[token][column]
+template <int NT>
+__device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const uint32_t (&sh)[NT][4], const uint32_t (&sl)[NT][4],
+                                            float* __restrict__ part, int row0, int g, int t) {
+    using C = BwSmem<NT>;
+    float acc[2][4] = {};
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const float2 v = *reinterpret_cast<const float2*>(x + (half * 8 + g) * C::LDN + row0 + nt * 8 + 2 * t);
+            uint32_t bh[2], bl[2];
+            bw_split(v.x, bh[0], bl[0]);
+            bw_split(v.y, bh[1], bl[1]);
+            bw_mma3(acc[half], sh[nt], sl[nt], bh, bl);
+        }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float* p = part + (half * 8 + 2 * t) * BW_LD + g;
+        p[0] = acc[half][0];
+        p[BW_LD] = acc[half][1];
+        p[8] = acc[half][2];
+        p[BW_LD + 8] = acc[half][3];
+    }
+}
+
+__device__ __forceinline__ float bw_sum_parts(const float* __restrict__ part, int tok, int col) {
+    float v[BW_WARPS];
+#pragma unroll
+    for (int w = 0; w < BW_WARPS; ++w) v[w] = part[w * BW_B * BW_LD + tok * BW_LD + col];
+    return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+}
+
+template <int NT, bool DELTA>
+__global__ void __launch_bounds__(BW_THREADS)
+block_walk_kernel(const BlockWalk a) {
+    using C = BwSmem<NT>;
+    extern __shared__ __align__(16) float bw_smem[];
+    float* part_p = bw_smem + 2 * C::STAGE;
+    float* part_r = part_p + C::PART;
+    float* su = part_r + C::PART;
+    const int s = blockIdx.z, h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
+    if (t1 <= t0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const int col0 = blockIdx.x * BW_COLS, cols = a.V - col0 < BW_COLS ? a.V - col0 : BW_COLS, row0 = warp * 8 * NT;
+    const float* rows = a.act ? a.act_rows : a.rows;
+    const long ld = a.act ? a.ld_act : a.ld;
+    const int q_col = (a.act ? 0 : a.q_off) + kvh * a.N, k_col = (a.act ? a.G * a.N : a.k_off) + kvh * a.N;
+    const int v_col = (a.act ? 2 * a.G * a.N : a.v_off) + h * a.V + col0;
+    const float* coef = a.coef + ((size_t)bw_first_block(a.q_start, s) * a.heads + h) * BW_COEF;
+    const size_t coef_step = (size_t)a.heads * BW_COEF;
+    bw_fetch<NT, DELTA>(bw_smem, a, rows, ld, q_col, k_col, v_col, cols, coef, t0, t1);
+
+    // the state: thread (g, tq) of a warp holds columns g and g + 8, rows 2 tq and 2 tq + 1 of every fragment
+    float* st = a.state + (size_t)a.slots[s] * a.state_stride + a.s_off + (size_t)h * a.N * a.V;
+    const long sr = a.state_vn ? 1 : a.V, sc = a.state_vn ? a.N : 1;
+    const bool fresh = a.positions[t0] == 0;
+    float S[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int row = row0 + nt * 8 + 2 * tq + (e & 1), col = g + (e >> 1) * 8;
+            S[nt][e] = (!fresh && row < a.N && col < cols) ? st[row * sr + (col0 + col) * sc] : 0.f;
+        }
+    const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
+
+    int b = 0;
+    for (int t = t0; t < t1; t += BW_B, b ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                        // the block's rows are here, and everyone has left the block before
+        coef += coef_step;
+        if (t + BW_B < t1) bw_fetch<NT, DELTA>(bw_smem + (b ^ 1) * C::STAGE, a, rows, ld, q_col, k_col, v_col, cols, coef, t + BW_B, t1);
+        const float* sq = bw_smem + b * C::STAGE;
+        const float* sk = sq + C::QK;
+        const float* sv = sk + C::QK;
+        const float* sA = sv + BW_B * BW_LDV;
+        const float* sM = sA + BW_B * BW_LD;
+        const float* gam = sM + BW_B * BW_LD;
+        const float* suf = gam + BW_B;
+        uint32_t sh[NT][4], sl[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {                       // rows 2 tq are the operand's k index tq, rows 2 tq + 1 its tq + 4
+            bw_split(S[nt][0], sh[nt][0], sl[nt][0]);
+            bw_split(S[nt][2], sh[nt][1], sl[nt][1]);
+            bw_split(S[nt][1], sh[nt][2], sl[nt][2]);
+            bw_split(S[nt][3], sh[nt][3], sl[nt][3]);
+        }
+        const float* u = sv;
+        if (DELTA) {
+            bw_read_out<NT>(sk, sh, sl, part_p + warp * BW_B * BW_LD, row0, g, tq);
+            __syncthreads();
+            // thread: token lane % 16 of column tid / 16; the 16 tokens of a column meet in half a warp
+            const int tok = lane & 15, col = tid >> 4;
+            const float e = sv[tok * BW_LDV + col] - gam[tok] * bw_sum_parts(part_p, tok, col);
+            const float4* m4 = reinterpret_cast<const float4*>(sM + tok * BW_LD);
+            float u0 = 0.f, u1 = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 m = m4[j];
+                u0 = fmaf(m.x, __shfl_sync(0xffffffffu, e, 4 * j, 16), u0);
+                u1 = fmaf(m.y, __shfl_sync(0xffffffffu, e, 4 * j + 1, 16), u1);
+                u0 = fmaf(m.z, __shfl_sync(0xffffffffu, e, 4 * j + 2, 16), u0);
+                u1 = fmaf(m.w, __shfl_sync(0xffffffffu, e, 4 * j + 3, 16), u1);
+            }
+            su[tok * BW_LDV + col] = u0 + u1;
+            u = su;
+        }
+        bw_read_out<NT>(sq, sh, sl, part_r + warp * BW_B * BW_LD, row0, g, tq);
+        __syncthreads();                                        // u and the partial sums of r are there
+        float up[NT][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            const int ta = ks * 8 + tq;
+            const float w0 = suf[ta], w1 = suf[ta + 4];
+            uint32_t ah[4], al[4];
+            bw_split(u[ta * BW_LDV + g] * w0, ah[0], al[0]);
+            bw_split(u[ta * BW_LDV + g + 8] * w0, ah[1], al[1]);
+            bw_split(u[(ta + 4) * BW_LDV + g] * w1, ah[2], al[2]);
+            bw_split(u[(ta + 4) * BW_LDV + g + 8] * w1, ah[3], al[3]);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                uint32_t bh[2], bl[2];
+                bw_split(sk[ta * C::LDN + row0 + nt * 8 + g], bh[0], bl[0]);
+                bw_split(sk[(ta + 4) * C::LDN + row0 + nt * 8 + g], bh[1], bl[1]);
+                bw_mma3(up[nt], ah, al, bh, bl);
+            }
+        }
+        {
+            // the results: thread = column tid % 16 of token tid / 16
+            const int col = tid & 15, tok = tid >> 4;
+            const float4* a4 = reinterpret_cast<const float4*>(sA + tok * BW_LD);
+            float o0 = gam[tok] * bw_sum_parts(part_r, tok, col), o1 = skip * sv[tok * BW_LDV + col];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 m = a4[j];
+                o0 = fmaf(m.x, u[(4 * j) * BW_LDV + col], o0);
+                o1 = fmaf(m.y, u[(4 * j + 1) * BW_LDV + col], o1);
+                o0 = fmaf(m.z, u[(4 * j + 2) * BW_LDV + col], o0);
+                o1 = fmaf(m.w, u[(4 * j + 3) * BW_LDV + col], o1);
+            }
+            if (t + tok < t1 && col < cols) a.out[(size_t)(t + tok) * a.ldo + (size_t)h * a.V + col0 + col] = o0 + o1;
+        }
+        const float total = gam[BW_B - 1];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[nt][e] = fmaf(total, S[nt][e], up[nt][e]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int row = row0 + nt * 8 + 2 * tq + (e & 1), col = g + (e >> 1) * 8;
+            if (row < a.N && col < cols) st[row * sr + (col0 + col) * sc] = S[nt][e];
+        }
+}
+
+template <int NT, bool DELTA>
+static int launch_block_walk(const BlockWalk& a, cudaStream_t stream) {
+    constexpr int bytes = BwSmem<NT>::TOTAL * 4;
+    auto kern = block_walk_kernel<NT, DELTA>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
+    kern<<<dim3((a.V + BW_COLS - 1) / BW_COLS, a.heads, a.S), BW_THREADS, bytes, stream>>>(a);
+    return launch_status();
+}
+
+}  // namespace aien
+
+using namespace aien;
+
+// Whether the walk takes these sizes; the rows besides have to start on 16-byte boundaries (aien_block_walk refuses others).
+AIEN_API int aien_block_walk_supports(int heads, int G, int N, int V) {
+    if (heads <= 0 || G <= 0 || heads % G || N <= 0 || N > 128 || N % 4 || V <= 0 || V % 4 || heads > 65535) return 0;
+    const long smem = 2L * BW_B * (N + 4) + 2L * BW_B * (heads / G) + 256L * (heads / G);
+    return smem * 4 <= 160 * 1024;
+}
+
+// rows float32 [T, ld] with q (G heads of N numbers) at q_off, k at k_off, v (`heads` heads of V) at v_off; act: they pass
+// silu first.  gates float32 [T, ldg]: decay of head h at g_off + h and (w_off >= 0) its weight at w_off + h: beta with
+// delta, else a factor on v; gates null: decay[heads] for every token.  skip (in skip_dt, or null): o += skip[h] v.
+// state: rows of state_stride floats, a head's matrix at s_off + h N V, [V][N] with state_vn, else [N][V].  Request s (tokens
+// q_start[s] .. q_start[s+1]) continues from slot slots[s], from zeros where its first position is 0.  out float32 [T, ldo].
+// scratch: float32, (T / 16 + S) * heads * 544 numbers (the blocks' coefficients) and with act T * (2 G N + heads V) more.
+AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, int v_off, int act, const float* gates, long ldg, int g_off,
+                             int w_off, const float* decay, int delta, const void* skip, int skip_dt, float* state, size_t state_stride,
+                             size_t s_off, int state_vn, const int* slots, const int* q_start, const int* positions, float* out, long ldo,
+                             int T, int S, int heads, int G, int N, int V, float* scratch, cudaStream_t stream) {
+    if (S <= 0 || T <= 0) return 0;
+    if (!aien_block_walk_supports(heads, G, N, V) || S > 65535 || G > 65535 || scratch == nullptr || (gates == nullptr && decay == nullptr)) return AIEN_E_SHAPE;
+    if ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(scratch)) & 15 || (ld | q_off | k_off | v_off) & 3) return AIEN_E_ALIGN;
+    const long blocks = T / BW_B + S, coefs = blocks * heads * BW_COEF;
+    BlockWalk a{rows, ld, q_off, k_off, v_off, gates, ldg, g_off, w_off, decay, scratch + coefs, 2L * G * N + (long)heads * V, act, delta, scratch,
+                skip, skip_dt, state, state_stride, s_off, state_vn, slots, q_start, positions, out, ldo, T, S, heads, G, N, V};
+    const int per = heads / G, smem = 4 * (2 * BW_B * (N + 4) + 2 * BW_B * per + (delta ? 256 * per : 0));
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(block_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AIEN_E_STATE;
+    block_coef_kernel<<<dim3((unsigned)blocks, G), 256, smem, stream>>>(a);
+    const int rc = launch_status();
+    if (rc != 0) return rc;
+    if (N <= 64) return delta ? launch_block_walk<1, true>(a, stream) : launch_block_walk<1, false>(a, stream);
+    return delta ? launch_block_walk<2, true>(a, stream) : launch_block_walk<2, false>(a, stream);
+}

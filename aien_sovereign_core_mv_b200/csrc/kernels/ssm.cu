@@ -485,6 +485,14 @@ AIEN_API int aien_selective_scan(const float* x, long ldx, const float* dtz, lon
     return launch_status();
 }
 
+// steps [T][2 * heads]: the step sizes softplus(dtr + dt_bias) and the decays exp(-A * that) of a step's tokens.
+AIEN_API int aien_ssd_steps(const float* dtr, long lddt, const float* A, const void* dt_bias, int p_dt, float* steps, int T, int heads,
+                            cudaStream_t stream) {
+    if (T <= 0 || heads <= 0) return T == 0 ? 0 : AIEN_E_SHAPE;
+    ssd_steps_kernel<<<(unsigned)(((long)T * heads + 255) / 256), 256, 0, stream>>>(dtr, lddt, A, dt_bias, p_dt, steps, T, heads);
+    return launch_status();
+}
+
 struct SsdArgs {
     const float* xbc; long ld; int x_off, b_off, c_off; const float* dtr; long lddt; const float* A; const void* dt_bias; const void* D;
     int p_dt; float* state; size_t state_stride, s_off; const int* slots; const int* q_start; const int* positions; float* y; long ldy;

@@ -192,6 +192,8 @@ def _declare(l: ctypes.CDLL) -> None:
                                               I, I, I, I, I, F, I, I, P],
         "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
         "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, P],
+        "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
+        "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, P, P],
         "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, P],
         "aien_gate_group_norm": [P, L, P, L, P, I, F, F, P, I, L, I, I, I, P],
         "aien_scaled_add_rmsnorm": [P, P, I, I, c_size_t, P, P, P, I, F, P, I, I, I, P],
@@ -1752,14 +1754,19 @@ def delta_conv_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b
 
 def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gb: torch.Tensor, state: torch.Tensor, s_off: int,
                slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, o: torch.Tensor, num_seqs: int, heads: int,
-               qk_heads: int, dim: int, vdim: int) -> None:
+               qk_heads: int, dim: int, vdim: int, blocks: Optional[torch.Tensor] = None) -> None:
     """Per value head, token by token: S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, all float32.  ``qkv``
     float32 [T, *] holds the prepared q, k (qk_heads x dim) and v (heads x vdim), ``gb`` [T, 2 * heads] the decay g and
-    beta.  S [heads, dim, vdim] of request s lies ``s_off`` numbers into slot slot_map[s] of ``state`` (float32 [slots, n])."""
+    beta.  S [heads, dim, vdim] of request s lies ``s_off`` numbers into slot slot_map[s] of ``state`` (float32 [slots, n]).
+    ``blocks`` (``block_walk_scratch(T, num_seqs, heads, qk_heads, dim, vdim)`` float32 numbers): the portions are walked
+    sixteen tokens at a time (:func:`block_walk`)."""
     _dev(qkv, gb, state, slot_map, q_start, positions, o)
     assert qkv.dtype == torch.float32 and qkv.stride(1) == 1 and gb.dtype == torch.float32 and gb.stride(1) == 1
     assert o.dtype == torch.float32 and o.stride(1) == 1 and o.shape[1] == heads * vdim
     assert state.dtype == torch.float32 and state.is_contiguous() and state.dim() == 2 and state.shape[1] >= s_off + heads * dim * vdim
+    if blocks is not None and block_walk(qkv, q_off, k_off, v_off, gb, 0, heads, None, state, s_off, slot_map, q_start, positions, o, num_seqs, heads,
+                                         qk_heads, dim, vdim, blocks, delta=True):
+        return
     _check(lib().aien_delta_rule(_p(qkv), qkv.stride(0), int(q_off), int(k_off), int(v_off), _p(gb), gb.stride(0), _p(state), state.shape[1],
                                  int(s_off), _p(slot_map), _p(q_start), _p(positions), _p(o), o.stride(0), int(num_seqs), int(heads),
                                  int(qk_heads), int(dim), int(vdim), _stream()), "delta_rule")
@@ -1852,6 +1859,53 @@ def conv_act(proj: torch.Tensor, off: int, channels: int, w: torch.Tensor, bias:
                                out16.stride(0) if out16 is not None else 0, T, _stream()), "conv_act")
 
 
+# ---------------------------------------------------------------------------- recurrences sixteen tokens at a time
+def block_walk_takes(dtype: torch.dtype, num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int) -> bool:
+    """Whether a step's recurrence with one decay per head goes through :func:`block_walk`: a bfloat16 engine's portions of
+    prompts (a float32 engine keeps to plain float32 products) over state matrices of up to 128 rows, with tokens enough
+    beside each request's first that blocks of 16 are worth their coefficients' launch."""
+    per = heads // max(qk_heads, 1)
+    return (dtype == torch.bfloat16 and num_tokens - num_seqs >= BLOCK_WALK_MIN_TOKENS and 0 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
+            and 32 * (dim + 4) + 288 * per <= 40 * 1024)
+
+
+BLOCK_WALK_MIN_TOKENS = 32
+
+
+def block_walk_scratch(num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, act: bool = False) -> int:
+    """float32 numbers of scratch :func:`block_walk` needs: 544 a block and head, and with ``act`` the rows after it."""
+    return (num_tokens // 16 + num_seqs) * heads * 544 + (num_tokens * (2 * qk_heads * dim + heads * vdim) if act else 0)
+
+
+def block_walk(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: Optional[torch.Tensor], g_off: int, w_off: int,
+               decay: Optional[torch.Tensor], state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor,
+               positions: torch.Tensor, out: torch.Tensor, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, scratch: torch.Tensor,
+               delta: bool = False, act: bool = False, skip: Optional[torch.Tensor] = None, state_vn: bool = False) -> bool:
+    """Per head, token by token, S <- g S + k u^T; o = S^T q (+ skip[h] v), over every request's portion: u = w v, or with
+    ``delta`` u = w (v - (g S)^T k).  ``rows`` float32 [T, *] holds q and k (qk_heads x dim) and v (heads x vdim), with
+    ``act`` before their silu; ``gates`` float32 [T, *] the decay g of head h in column g_off + h and w in w_off + h
+    (w_off < 0: 1), or ``decay`` one per head.  S of request s lies ``s_off`` numbers into row slot_map[s] of ``state``, per
+    head [dim, vdim], or with ``state_vn`` [vdim, dim].  False, and nothing done, where the rows do not start on 16-byte boundaries."""
+    _dev(rows, gates, decay, state, slot_map, q_start, positions, out, scratch, skip)
+    T = rows.shape[0]
+    assert rows.dtype == torch.float32 and rows.stride(1) == 1 and out.dtype == torch.float32 and out.stride(1) == 1
+    assert tuple(out.shape) == (T, heads * vdim) and heads % qk_heads == 0 and (gates is None) != (decay is None)
+    assert gates is None or (gates.dtype == torch.float32 and gates.stride(1) == 1 and gates.shape[0] == T)
+    assert decay is None or (decay.dtype == torch.float32 and decay.is_contiguous() and decay.numel() == heads and w_off < 0)
+    assert state.dtype == torch.float32 and state.is_contiguous() and state[0].numel() >= s_off + heads * dim * vdim
+    assert skip is None or (skip.is_contiguous() and skip.numel() == heads)
+    assert scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.numel() >= block_walk_scratch(T, num_seqs, heads, qk_heads, dim, vdim, act)
+    if rows.data_ptr() % 16 or scratch.data_ptr() % 16 or (rows.stride(0) | q_off | k_off | v_off) % 4:
+        return False
+    _check(lib().aien_block_walk(
+        _p(rows), rows.stride(0), int(q_off), int(k_off), int(v_off), int(act), _p(gates), gates.stride(0) if gates is not None else 0, int(g_off),
+        int(w_off), _p(decay), int(delta), _p(skip), dt(skip) if skip is not None else F32, _p(state), state.stride(0), int(s_off), int(state_vn),
+        _p(slot_map), _p(q_start), _p(positions), _p(out), out.stride(0), T, int(num_seqs), int(heads), int(qk_heads), int(dim), int(vdim),
+        _p(scratch), _stream()), "block_walk")
+    add_launches(1)
+    return True
+
+
 SCAN_SEGMENT_MIN_TOKENS = 128        # steps with fewer tokens walk every portion in one piece
 # with this many lanes at work a portion is walked whole; with fewer it is cut until there are about as many
 # (AIEN_B200_SCAN_LANES pins another number for measurements)
@@ -1906,12 +1960,13 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
              state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, y: torch.Tensor,
              num_seqs: int, heads: int, V: int, G: int, N: int, seg_len: int = 0, nseg: int = 1, scratch: Optional[torch.Tensor] = None,
-             steps: Optional[torch.Tensor] = None) -> None:
+             steps: Optional[torch.Tensor] = None, blocks: Optional[torch.Tensor] = None) -> None:
     """The state-space-duality recurrence over every request's portion: per head h (group g = h // (heads // G)), token by
     token, dt = softplus(dtr[h] + dt_bias[h]); S = exp(-A[h] * dt) * S + dt * B[g] x[h]^T (S is N x V); y[h] = S^T C[g] +
     D[h] * x[h].  x, B, C are column blocks of the float32 rows ``xbc``; dtr float32 [T, heads] (row stride free); A float32
     [heads]; S lives in the request's state row from ``s_off`` on (as [heads, V, N]); y float32 [T, heads * V].  ``steps``:
-    float32 scratch of T * 2 * heads numbers (made here when not given)."""
+    float32 scratch of T * 2 * heads numbers (made here when not given).  ``blocks`` (``block_walk_scratch(T, num_seqs, heads,
+    G, N, V)`` float32 numbers): the portions are walked sixteen tokens at a time (:func:`block_walk`)."""
     _dev(xbc, dtr, A, dt_bias, D, state, slot_map, q_start, positions, y, scratch, steps)
     T = xbc.shape[0]
     if steps is None:
@@ -1920,6 +1975,11 @@ def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.T
     assert xbc.dtype == torch.float32 and xbc.stride(1) == 1 and dtr.dtype == torch.float32 and dtr.stride(1) == 1
     assert A.dtype == torch.float32 and A.numel() == heads and dt_bias.dtype == D.dtype and dt_bias.is_contiguous() and D.is_contiguous()
     assert state.dtype == torch.float32 and state.stride(-1) == 1 and y.dtype == torch.float32 and y.stride(1) == 1
+    if blocks is not None:
+        _check(lib().aien_ssd_steps(_p(dtr), dtr.stride(0), _p(A), _p(dt_bias), dt(dt_bias), _p(steps), T, int(heads), _stream()), "ssd_steps")
+        if block_walk(xbc, c_off, b_off, x_off, steps[:T * 2 * heads].view(T, 2 * heads), heads, 0, None, state, s_off, slot_map, q_start, positions, y,
+                      num_seqs, heads, G, N, V, blocks, skip=D, state_vn=True):
+            return
     if seg_len and nseg > 1:
         assert scratch is not None and scratch.numel() >= 2 * (T // seg_len + num_seqs) * heads * N * V
     _check(lib().aien_ssd_scan(_p(xbc), xbc.stride(0), int(x_off), int(b_off), int(c_off), _p(dtr), dtr.stride(0), _p(A), _p(dt_bias), _p(D),

@@ -170,7 +170,8 @@ class GatedDeltaRule(Mixer):
     def workspace_bytes(self, lim):
         n = 2 * self.qk_dim + 2 * self.v_dim + 2 * self.num_heads
         return lim.max_tokens * ((n + self.channels + 2 * self.num_heads + self.v_dim) * 4 + self.v_dim * lim.itemsize + self.hidden_size * 4) \
-            + 8192 + K.PARTIALS_MAX_BYTES
+            + 8192 + K.PARTIALS_MAX_BYTES \
+            + 4 * K.block_walk_scratch(lim.max_tokens, lim.max_seqs, self.num_heads, self.num_qk_heads, self.head_dim, self.value_dim)
 
     def forward(self, ctx: StepContext, h: torch.Tensor, run: RunBinding):
         T, n = ctx.num_tokens, self.num_heads
@@ -185,8 +186,12 @@ class GatedDeltaRule(Mixer):
                              self.conv["q"], self.conv["k"], self.conv["v"], self.taps, self.a_log, self.dt_bias, state, group.slot_map,
                              ctx.seq_of_token, ctx.q_start, ctx.positions, qkv, gb)
         o = ctx.workspace.take((T, self.v_dim), torch.float32)
+        sizes = (n, self.num_qk_heads, self.head_dim, self.value_dim)
+        blocks = None
+        if K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes) and not ctx.decode_only:
+            blocks = ctx.workspace.take((K.block_walk_scratch(T, ctx.num_seqs, *sizes),), torch.float32)
         K.delta_rule(qkv, 0, self.qk_dim, 2 * self.qk_dim, gb, state, self.conv_floats, group.slot_map, ctx.q_start, ctx.positions, o,
-                     ctx.num_seqs, n, self.num_qk_heads, self.head_dim, self.value_dim)
+                     ctx.num_seqs, *sizes, blocks)
         y = ctx.workspace.take((T, self.v_dim), ctx.dtype)
         K.grouped_gated_rmsnorm(o, proj[:, g_off:g_off + self.v_dim], self.norm_w, self.norm_eps, y, self.value_dim, "silu")
         return linear(ctx, y, self.w_o, out_dtype=torch.float32, may_defer_sum=True)

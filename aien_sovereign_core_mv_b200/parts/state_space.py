@@ -190,7 +190,8 @@ class StateSpaceDuality(BranchMixer):
 
     def core_workspace_bytes(self, lim):
         return lim.max_tokens * (self.channels + self.inner + 2 * self.num_heads) * 4 + 2048 \
-            + 4 * K.scan_scratch_floats(lim.max_tokens, lim.max_seqs, self.num_heads * self.state * self.value_dim, self.inner * min(self.state, 32))
+            + 4 * max(K.scan_scratch_floats(lim.max_tokens, lim.max_seqs, self.num_heads * self.state * self.value_dim, self.inner * min(self.state, 32)),
+                      K.block_walk_scratch(lim.max_tokens, lim.max_seqs, self.num_heads, self.groups, self.state, self.value_dim))
 
     def core(self, ctx, proj, col0, store, out, out_col0, mult):
         T, I, GN = ctx.num_tokens, self.inner, self.groups * self.state
@@ -200,11 +201,16 @@ class StateSpaceDuality(BranchMixer):
         K.conv_act(proj, col0 + I, self.channels, self.conv, self.conv_b, self.taps, "silu", state, slots, ctx.seq_of_token, ctx.q_start,
                    ctx.positions, xbc)
         y = ws.take((T, I), torch.float32)
-        seg, nseg, scratch = _segments(ctx, self.num_heads * self.state * self.value_dim, I * min(self.state, 32))
+        seg, nseg, scratch, blocks = 0, 1, None, None
+        if K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, self.num_heads, self.groups, self.state, self.value_dim) and not ctx.decode_only \
+                and self.channels % 4 == 0 and I % 4 == 0:
+            blocks = ws.take((K.block_walk_scratch(T, ctx.num_seqs, self.num_heads, self.groups, self.state, self.value_dim),), torch.float32)
+        else:
+            seg, nseg, scratch = _segments(ctx, self.num_heads * self.state * self.value_dim, I * min(self.state, 32))
         steps = ws.take((T * 2 * self.num_heads,), torch.float32)
         dt0 = col0 + 2 * I + 2 * GN
         K.ssd_scan(xbc, 0, I, I + GN, proj[:, dt0:dt0 + self.num_heads], self.A, self.dt_b, self.D, state, self.conv_floats, slots,
-                   ctx.q_start, ctx.positions, y, ctx.num_seqs, self.num_heads, self.value_dim, self.groups, self.state, seg, nseg, scratch, steps)
+                   ctx.q_start, ctx.positions, y, ctx.num_seqs, self.num_heads, self.value_dim, self.groups, self.state, seg, nseg, scratch, steps, blocks)
         K.gate_group_norm(y, proj[:, col0:col0 + I], self.norm_w, self.norm_eps, mult, out[:, out_col0:out_col0 + I], self.norm_groups)
 
 

@@ -1,0 +1,85 @@
+"""Recurrences with one decay per head walked sixteen tokens at a time (``kernels.block_walk``) against the recurrences
+themselves, token by token in 64 bits."""
+import numpy as np
+import pytest
+import torch
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+def _recurrence(q, k, v, g, w, S, delta, skip):
+    """q, k [T, heads, N], v [T, heads, V], g and w [T, heads], S [heads, N, V], all float64."""
+    out = []
+    for t in range(q.shape[0]):
+        S = g[t][:, None, None] * S
+        u = w[t][:, None] * (v[t] - (np.einsum("hnv,hn->hv", S, k[t]) if delta else 0.0))
+        S = S + k[t][:, :, None] * u[:, None, :]
+        out.append(np.einsum("hnv,hn->hv", S, q[t]) + skip[:, None] * v[t])
+    return np.stack(out), S
+
+
+@pytest.mark.parametrize("heads,G,N,V,lens,slow", [
+    (2, 1, 128, 128, [100, 1, 16, 33, 2], True), (4, 4, 64, 64, [17, 48], False), (3, 1, 20, 12, [64, 5], True), (6, 2, 68, 36, [40, 15, 1, 1], False),
+    (1, 1, 4, 4, [33], False), (32, 1, 128, 64, [50], True)])
+@pytest.mark.parametrize("form", ["delta", "weights", "decay"])
+def test_block_walk_follows_the_recurrence(form, heads, G, N, V, lens, slow):
+    """Blocks that end inside a portion, single tokens beside portions, sizes that fill no fragment, a q/k head shared by
+    several heads, decays that hardly decay, new requests and old ones, both layouts of the state.  A product of two
+    float32 numbers loses 3 * 2^-22 at most and a block rounds its state once: 1e-5 of the largest value covers 100
+    tokens of it."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    f64 = lambda a: a.double().cpu().numpy()
+    g_ = torch.Generator().manual_seed(heads * 1000 + N + V)
+    T, S, delta, act, state_vn = sum(lens), len(lens), form == "delta", form == "decay", form == "weights"
+    GN, s_off, extra = G * N, 5, 3
+    rows = torch.randn(T, 4 + 2 * GN + heads * V + 4, generator=g_)
+    k = rows[:, 4 + GN:4 + 2 * GN]
+    if delta:                                              # unit keys, as the delta rule has them
+        k /= k.reshape(T, G, N).norm(dim=-1).repeat_interleave(N, dim=1)
+    gates = torch.rand(T, 2 * heads + 1, generator=g_)
+    gates[:, :heads] = 1.0 - gates[:, :heads] * (1e-4 if slow else 0.9)
+    decay = 1.0 - torch.rand(heads, generator=g_) * (1e-4 if slow else 0.5)
+    skip = torch.randn(heads, generator=g_)
+    state = torch.randn(S + 2, s_off + heads * N * V + extra, generator=g_)
+    slots = [S - s for s in range(S)]
+    fresh = [s % 2 == 1 for s in range(S)]
+    q0 = [sum(lens[:s]) for s in range(S + 1)]
+    dev = state.clone().cuda()
+    out = torch.full((T, heads * V), 9.0).cuda()
+    blocks = torch.full((K.block_walk_scratch(T, S, heads, G, N, V, act),), float("nan")).cuda()
+    took = K.block_walk(rows.cuda(), 4, 4 + GN, 4 + 2 * GN, None if act else gates.cuda(), 0, -1 if act else heads, decay.cuda() if act else None,
+                        dev, s_off, i32(slots), i32(q0), i32([(0 if fresh[s] else 7) + p for s, n in enumerate(lens) for p in range(n)]), out, S, heads,
+                        G, N, V, blocks, delta=delta, act=act, skip=skip.cuda() if state_vn else None, state_vn=state_vn)
+    assert took
+    a = f64(rows)
+    if act:
+        a = a / (1.0 + np.exp(-a))
+    for s in range(S):
+        r = slice(q0[s], q0[s + 1])
+        qk = lambda off: np.repeat(a[r, off:off + GN].reshape(-1, G, N), heads // G, axis=1)
+        v = a[r, 4 + 2 * GN:4 + 2 * GN + heads * V].reshape(-1, heads, V)
+        S0 = f64(state[slots[s], s_off:s_off + heads * N * V]).reshape((heads, V, N) if state_vn else (heads, N, V))
+        S0 = S0.transpose(0, 2, 1) if state_vn else S0
+        n = lens[s]
+        g, w = (np.tile(f64(decay), (n, 1)), np.ones((n, heads))) if act else (f64(gates[r, :heads]), f64(gates[r, heads:2 * heads]))
+        want, last = _recurrence(qk(4), qk(4 + GN), v, g, w, S0 * 0.0 if fresh[s] else S0, delta, f64(skip) if state_vn else np.zeros(heads))
+        H.assert_close(out[r].cpu().numpy().reshape(n, heads, V), want, 1e-5, f"request {s}")
+        got = dev[slots[s], s_off:s_off + heads * N * V].cpu().numpy().reshape((heads, V, N) if state_vn else (heads, N, V))
+        H.assert_close(got.transpose(0, 2, 1) if state_vn else got, last, 1e-5, f"state of request {s}")
+    keep = [i for i in range(S + 2) if i not in slots]
+    assert torch.equal(dev[keep].cpu(), state[keep]) and torch.equal(dev[:, :s_off].cpu(), state[:, :s_off]) and torch.equal(dev[:, -extra:].cpu(), state[:, -extra:])
+
+
+def test_block_walk_declines_rows_off_the_boundary():
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    rows, out, state = torch.zeros(40, 26).cuda(), torch.full((40, 8), 3.0).cuda(), torch.ones(2, 64).cuda()
+    blocks = torch.empty(K.block_walk_scratch(40, 1, 1, 1, 8, 8)).cuda()
+    assert not K.block_walk(rows, 0, 8, 16, None, 0, -1, torch.ones(1).cuda(), state, 0, i32([0]), i32([0, 40]), i32(list(range(40))), out, 1, 1, 1, 8, 8,
+                            blocks)
+    assert float((out - 3.0).abs().max()) == 0.0 and float((state - 1.0).abs().max()) == 0.0
+    assert not K.block_walk_takes(torch.float32, 4096, 1, 4, 2, 64, 64) and not K.block_walk_takes(torch.bfloat16, 64, 64, 4, 2, 64, 64)
+    assert not K.block_walk_takes(torch.bfloat16, 4096, 1, 4, 2, 130, 64) and K.block_walk_takes(torch.bfloat16, 4096, 1, 4, 2, 128, 64)
