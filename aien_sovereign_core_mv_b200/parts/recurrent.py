@@ -49,7 +49,8 @@ class DecayLinearAttention(Mixer):
         return CacheNeed("state", state_shape=(self.num_heads, self.head_dim, self.value_dim), state_dtype="float32")
 
     def workspace_bytes(self, lim):
-        chunks = K.decay_linear_attention_scratch(lim.max_tokens, lim.max_seqs, self.num_heads, self.head_dim, self.value_dim) * 4
+        chunks = 4 * max(K.decay_linear_attention_scratch(lim.max_tokens, lim.max_seqs, self.num_heads, self.head_dim, self.value_dim),
+                         K.block_walk_scratch(lim.max_tokens, lim.max_seqs, self.num_heads, self.num_heads, self.head_dim, self.value_dim, act=True))
         return lim.max_tokens * ((2 * self.qk_dim + 2 * self.v_dim) * 4 + self.v_dim * (4 + lim.itemsize) + self.hidden_size * 4) + 8192 + chunks + K.PARTIALS_MAX_BYTES
 
     def forward(self, ctx: StepContext, h: torch.Tensor, run: RunBinding):
@@ -58,12 +59,19 @@ class DecayLinearAttention(Mixer):
         state = group.storage["state"][run.slot]
         proj = linear(ctx, h, self.w_in, out_dtype=torch.float32)
         o = ctx.workspace.take((T, self.v_dim), torch.float32)
-        scratch = None
-        if not ctx.decode_only:                                         # portions of prompts: their chunks side by side
-            n = K.decay_linear_attention_scratch(T, ctx.num_seqs, self.num_heads, self.head_dim, self.value_dim)
-            scratch = ctx.workspace.take((n,), torch.float32)
-        K.decay_linear_attention(proj, 0, self.qk_dim, 2 * self.qk_dim, self.decay, state, group.slot_map, ctx.q_start, ctx.positions,
-                                 o, ctx.num_seqs, self.num_heads, self.head_dim, self.value_dim, scratch, single_tokens=ctx.decode_only)
+        sizes = (self.num_heads, self.num_heads, self.head_dim, self.value_dim)
+        walked = False
+        if not ctx.decode_only and K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes) and proj.shape[1] % 4 == 0:
+            blocks = ctx.workspace.take((K.block_walk_scratch(T, ctx.num_seqs, *sizes, act=True),), torch.float32)
+            walked = K.block_walk(proj, 0, self.qk_dim, 2 * self.qk_dim, None, 0, -1, self.decay, state.view(state.shape[0], -1), 0, group.slot_map,
+                                  ctx.q_start, ctx.positions, o, ctx.num_seqs, *sizes, blocks, act=True)
+        if not walked:
+            scratch = None
+            if not ctx.decode_only:                                     # portions of prompts: their chunks side by side
+                n = K.decay_linear_attention_scratch(T, ctx.num_seqs, self.num_heads, self.head_dim, self.value_dim)
+                scratch = ctx.workspace.take((n,), torch.float32)
+            K.decay_linear_attention(proj, 0, self.qk_dim, 2 * self.qk_dim, self.decay, state, group.slot_map, ctx.q_start, ctx.positions,
+                                     o, ctx.num_seqs, self.num_heads, self.head_dim, self.value_dim, scratch, single_tokens=ctx.decode_only)
         y = ctx.workspace.take((T, self.v_dim), ctx.dtype)
         K.gated_rmsnorm(o, proj[:, 2 * self.qk_dim + self.v_dim:], self.norm_w, self.norm_eps, y)
         return linear(ctx, y, self.w_o, out_dtype=torch.float32, may_defer_sum=True)     # the branch norm adds partial products
