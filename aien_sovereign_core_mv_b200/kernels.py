@@ -192,6 +192,7 @@ def _declare(l: ctypes.CDLL) -> None:
                                               I, I, I, I, I, F, I, I, P],
         "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
         "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, P],
+        "aien_split_rows": [P, L, P, I, I, P],
         "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
         "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, P, P],
         "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, P],
@@ -1959,6 +1960,14 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
 
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
              state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, y: torch.Tensor,
+def split_rows(x: torch.Tensor, out: torch.Tensor) -> None:
+    """x float32 [T, n] as the sum of three bfloat16 rows side by side, out [T, 3 n] (up to 2^-25 of x): the left operand of
+    a tensor-core product that must not round its float32 rows, with the weights three times side by side."""
+    _dev(x, out)
+    assert x.dtype == torch.float32 and x.stride(1) == 1 and out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == (x.shape[0], 3 * x.shape[1])
+    _check(lib().aien_split_rows(_p(x), x.stride(0), _p(out), x.shape[0], x.shape[1], _stream()), "split_rows")
+
+
              num_seqs: int, heads: int, V: int, G: int, N: int, seg_len: int = 0, nseg: int = 1, scratch: Optional[torch.Tensor] = None,
              steps: Optional[torch.Tensor] = None, blocks: Optional[torch.Tensor] = None) -> None:
     """The state-space-duality recurrence over every request's portion: per head h (group g = h // (heads // G)), token by

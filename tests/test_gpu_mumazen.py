@@ -335,6 +335,24 @@ def test_selective_scan_many_channels_16_bit_results(inner, N, lens):
     assert float(state[0].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("T,n,N", [(1, 8, 16), (5, 24, 40), (130, 64, 72)])
+def test_product_of_float32_rows_in_three_parts(T, n, N):
+    """The three parts add up to the row (2^-25 of it: each leaves at most half a unit of 8 bits), and the tensor-core
+    product over them beside the weights three times is the product of the float32 rows: n float32 additions."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(T + n)
+    x = (torch.randn(T, n + 4, generator=g) * torch.exp(torch.randn(T, n + 4, generator=g) * 3.0)).cuda()
+    w = torch.randn(N, n, generator=g).to(torch.bfloat16).cuda()
+    parts = torch.zeros(T, 3 * n, dtype=torch.bfloat16).cuda()
+    K.split_rows(x[:, 4:], parts)
+    back = parts.double().view(T, 3, n).sum(1)
+    assert float(((back - x[:, 4:].double()).abs() / x[:, 4:].double().abs()).max()) <= 2.0 ** -25
+    out = torch.zeros(T, N).cuda()
+    K.gemm_tc(parts, torch.cat([w] * 3, dim=1).contiguous(), out)
+    want = x[:, 4:].double() @ w.double().T
+    assert float((out - want).abs().max()) <= 3 * n * 2.0 ** -23 * float((x[:, 4:].double().abs() @ w.double().abs().T).max())
+
+
 @pytest.mark.parametrize("heads,V,G,N", [(3, 8, 1, 5), (4, 16, 2, 24), (6, 24, 3, 40), (2, 64, 1, 128), (1, 40, 1, 200)])
 def test_state_space_duality_cut_any_way(heads, V, G, N):
     from aien_sovereign_core_mv_b200 import kernels as K
