@@ -3,7 +3,8 @@
 // Same job and same arguments as the mma.sync prefill kernel (portions of prompts of any length
 // at any offset, causal, grouped-query, optional window; the host lists tiles of 128 query tokens),
 // for head sizes 64 and 128 and pages of 8..128 tokens that divide 128.  Keys and values may have sizes of
-// their own, any multiples of 8 up to 128: a tile is then padded to 64 or 128 columns by the copies themselves,
+// their own, any multiples of 8 up to 128 (keys up to 192, which leaves room for one head a CTA only): a tile is then
+// padded to 64, 128 or 192 columns by the copies themselves,
 // which see every head as a matrix of its own and fill zeros beyond its columns.  A value head may serve
 // several neighbouring key heads (v_share: attention maps over the same values), and the result may
 // leave in float32.
@@ -79,7 +80,7 @@ template <int HD, int HDV> struct PtShape {
     static constexpr int SLOTS_FIT = (PT_SMEM_MAX - FIXED) / SLOT_BYTES;
     static constexpr int SLOTS = SLOTS_FIT > 6 ? 6 : SLOTS_FIT;
     static constexpr int SMEM = FIXED + SLOTS * SLOT_BYTES;
-    static_assert(SLOTS >= 3, "the K/V ring needs three slots");
+    static_assert(SLOTS >= (HD > 128 ? 2 : 3), "the K/V ring needs three slots; one head alone has one more");
 };
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -616,6 +617,7 @@ static int launch_prefill_tc(const CUtensorMap& mq, const PtMaps& mk, const PtMa
                              void* scratch, long scratch_bytes, int max_ctx, int force_splits, int chunk, const float* sinks,
                              const HeadTerms& ht, const PtSizes& sz, cudaStream_t stream) {
     auto kern = prefill_tc_kernel<HD, HDV>;
+    if (HD > 128 && force_splits > 1) return AIEN_E_SHAPE;
     // a chunk bounds the keys of a tile, and the merge of key ranges knows neither a sink nor a gate
     if (chunk > 0 || sinks != nullptr || ht.head_scale != nullptr || ht.slopes != nullptr || ht.gate != nullptr) {
         if (force_splits > 1) return AIEN_E_SHAPE;
@@ -645,14 +647,14 @@ static int launch_prefill_tc(const CUtensorMap& mq, const PtMaps& mk, const PtMa
     const long single = (long)num_tiles * nkv * group, paired = (long)num_tiles * nkv * ((group + 1) / 2);
     auto waves = [&](long ctas) { return (ctas + sms - 1) / sms; };
     const long blocks = max_ctx > 0 ? (max_ctx + PT_BN - 1) / PT_BN : 0;          // of the longest tile, at most
-    int heads_per_cta = (group >= 2 && 18 * waves(single) > 25 * waves(paired)) ? 2 : 1;
+    int heads_per_cta = (HD <= 128 && group >= 2 && 18 * waves(single) > 25 * waves(paired)) ? 2 : 1;
     int nsplit = 1;
     const long part_rows = (long)num_tiles * PT_BM * nq;
     auto fits = [&](int n) { return scratch != nullptr && part_rows * n * (HDV + 2) * 4 <= scratch_bytes; };
     if (force_splits > 0) {
         nsplit = force_splits;
         if (!fits(nsplit)) return AIEN_E_SHAPE;
-    } else if (group >= 2 && blocks > 0) {
+    } else if (HD <= 128 && group >= 2 && blocks > 0) {
         long best = heads_per_cta == 2 ? waves(paired) * (blocks * 3550 + 6000) : waves(single) * (blocks * 2870 + 6000);
         for (int n = 2; n <= PT_MAX_SPLITS && fits(n); ++n) {
             const long t = waves(paired * n) * ((blocks + n - 1) / n * 3550 + 6000) + 40000;
@@ -690,6 +692,13 @@ AIEN_API int aien_paged_attention_prefill_tc_values_supports(int hd, int hdv, in
             (page_size & 7) == 0 && 128 % page_size == 0) ? 1 : 0;
 }
 
+// And with keys of up to 192 numbers, one head a CTA: portions over keys that a step makes per head (latent attention with
+// a rotated part).  2,048 tokens, 16 heads of 192 / 128, window 1,024: 43 us, against 449 us over the latent itself; with
+// the product that makes the keys (23 us) and without those that carry query and result (54 us).
+AIEN_API int aien_paged_attention_prefill_tc_portions_supports(int hd, int hdv, int page_size) {
+    return aien_paged_attention_prefill_tc_values_supports(hd > 128 && hd <= 192 && (hd & 7) == 0 ? 128 : hd, hdv, page_size);
+}
+
 // q [q_rows, nq*hd] (leading dimension q_stride), k_cache/v_cache [cache_rows, nkv*hd] contiguous;
 // the other arguments as aien_paged_attention_prefill.
 // scratch (may be null), scratch_bytes: room for the partial results of key ranges, num_tiles * 128 * nq *
@@ -701,7 +710,8 @@ AIEN_API int aien_paged_attention_prefill_tc_values_supports(int hd, int hdv, in
 // (0: none): see HeadTerms.
 // k_ld, v_ld: numbers between rows of the caches (0: the rows are contiguous); egate, ldeg: see PtSizes (bfloat16 results only).
 // hdv, v_share, out_f32: values of hdv numbers, one value head for every v_share neighbouring key heads (v_cache
-// [cache_rows, nkv / v_share * hdv], out [tokens, nq * hdv]), float32 results; hd and hdv are multiples of 8 up to 128.
+// [cache_rows, nkv / v_share * hdv], out [tokens, nq * hdv]), float32 results; hd and hdv are multiples of 8,
+// hd up to 192, hdv up to 128.
 AIEN_API int aien_paged_attention_prefill_tc_values(
     const void* q, long q_stride, int q_rows, const void* k_cache, const void* v_cache, int cache_rows, const int* block_table,
     int max_blocks, const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_q0, int num_tiles, void* out,
@@ -711,7 +721,7 @@ AIEN_API int aien_paged_attention_prefill_tc_values(
     const HeadTerms ht{head_scale, slopes, gate, ldg, softcap > 0.f ? softcap : 0.f};
     if (num_tiles <= 0) return 0;
     if (chunk < 0) return AIEN_E_SHAPE;
-    if (!aien_paged_attention_prefill_tc_values_supports(hd, hdv, page_size) || nkv <= 0 || nq % nkv != 0 || q_rows <= 0 || cache_rows <= 0 ||
+    if (!aien_paged_attention_prefill_tc_portions_supports(hd, hdv, page_size) || nkv <= 0 || nq % nkv != 0 || q_rows <= 0 || cache_rows <= 0 ||
         v_share <= 0 || nkv % v_share != 0)
         return AIEN_E_SHAPE;
     if ((q_stride & 7) || (out_stride & 7) || ((uintptr_t)q & 15) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15) ||
@@ -751,6 +761,7 @@ AIEN_API int aien_paged_attention_prefill_tc_values(
                                          out_stride, nq, nkv, page_size, window, scale, cache_rows, scratch, scratch_bytes, max_ctx,       \
                                          force_splits, chunk, sinks, ht, sz, stream)
     if (hd <= 64) { if (hdv <= 64) PT_CASE(64, 64); else PT_CASE(64, 128); }
+    if (hd > 128) { if (hdv <= 64) PT_CASE(192, 64); else PT_CASE(192, 128); }
     if (hdv <= 64) PT_CASE(128, 64); else PT_CASE(128, 128);
 #undef PT_CASE
 }

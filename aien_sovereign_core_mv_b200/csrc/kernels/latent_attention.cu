@@ -64,22 +64,24 @@ latent_prepare_kernel(const TD* __restrict__ d, long ld, int q_rank, const void*
 // The rotated part of every query head, moved behind the head's latent query:
 // out[t, h, 0:rot_dim] = rotate(q[t, h, 0:rot_dim]) (first rot_dims numbers in pairs), the rotation in float32.
 template <typename TQ, typename TO>
-__global__ void rotate_pairs_rows_kernel(const TQ* __restrict__ q, long ldq, long q_head, TO* __restrict__ out, long ldo,
+__global__ void rotate_pairs_rows_kernel(const TQ* q, long ldq, long q_head, TO* out, long ldo,
                                          long o_head, int H, int rot_dim, int rot_dims, const float* __restrict__ cos_t,
                                          const float* __restrict__ sin_t) {
     const size_t t = blockIdx.x;
     const int half = rot_dims >> 1;
-    for (int idx = threadIdx.x; idx < H * rot_dim; idx += blockDim.x) {
-        const int h = idx / rot_dim, i = idx % rot_dim;
-        const TQ* src = q + t * ldq + (size_t)h * q_head;
-        float v = to_f(src[i]);
+    const int pairs = (rot_dim + 1) >> 1;
+    for (int idx = threadIdx.x; idx < H * pairs; idx += blockDim.x) {          // a thread owns a pair, so the rows may be turned where they lie
+        const int h = idx / pairs, p = idx % pairs, i = 2 * p;
+        const TQ* src = q + t * ldq + (size_t)h * q_head + i;
+        TO* dst = out + t * ldo + (size_t)h * o_head + i;
+        float a = to_f(src[0]), b = i + 1 < rot_dim ? to_f(src[1]) : 0.f;
         if (i < rot_dims) {
-            const int p = i >> 1;
-            const float c = cos_t[t * half + p], s = sin_t[t * half + p];
-            const float other = to_f(src[i ^ 1]);
-            v = (i & 1) ? v * c + other * s : v * c - other * s;
+            const float c = cos_t[t * half + p], s = sin_t[t * half + p], a0 = a;
+            a = a0 * c - b * s;
+            b = b * c + a0 * s;
         }
-        out[t * ldo + (size_t)h * o_head + i] = from_f<TO>(v);
+        dst[0] = from_f<TO>(a);
+        if (i + 1 < rot_dim) dst[1] = from_f<TO>(b);
     }
 }
 

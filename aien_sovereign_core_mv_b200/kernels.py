@@ -217,6 +217,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "aien_paged_attention_decode_values": [P, L, P, P, P, I, P, P, P, P, L, P, P, P, I, I, I, I, I, F, I, I, I, F, I, I, I, I, P],
         "aien_paged_attention_prefill_tc_values": [P, L, I, P, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, P, L, I, I, I, P, P, P, P, L, F, I, I, I, L, L, P, L, P],
         "aien_paged_attention_prefill_tc_values_supports": [I, I, I],
+        "aien_paged_attention_prefill_tc_portions_supports": [I, I, I],
     }
     for name, args in sigs.items():
         fn = getattr(l, name)
@@ -1446,7 +1447,7 @@ def latent_prepare(d: torch.Tensor, q_rank: int, wq: Optional[torch.Tensor], eps
 def rotate_pairs_rows(q: torch.Tensor, q_head: int, col0: int, out: torch.Tensor, o_head: int, ocol0: int, heads: int, rot_dim: int,
                       rot_dims: int, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor]) -> None:
     """out[t, h*o_head + ocol0 + i] = q[t, h*q_head + col0 + i], i < rot_dim, the first ``rot_dims`` of them rotated in
-    neighbouring pairs by the token's angle (the rotation itself in float32)."""
+    neighbouring pairs by the token's angle (the rotation itself in float32).  ``out`` may be ``q`` itself."""
     _dev(q, out, cos, sin)
     T = q.shape[0]
     assert q.stride(1) == 1 and out.stride(1) == 1
@@ -1560,7 +1561,7 @@ def latent_attention_tc_small_tiles(decode_only: bool, kv_rank: int) -> bool:
 def latent_attention_tc_ksplit(num_tokens: int, num_seqs: int, heads: int, max_ctx: int, window: int, small_tiles: bool = False) -> int:
     """Into how many CTAs the key blocks of a tile are dealt: enough to occupy the GPU (148 SMs, two rounds of CTAs)
     when the step has few tiles, never more than a tile has blocks.  Depends on the step's sizes only."""
-    tiles = (num_tokens * heads) // (16 if small_tiles else LATENT_TC_TILE) + num_seqs
+    tiles = num_tokens * ((heads + 15) // 16) if small_tiles else (num_tokens * heads) // LATENT_TC_TILE + num_seqs
     span = min(window, max_ctx) if window > 0 else max_ctx
     blocks = max(1, (span + LATENT_TC_TILE - 1) // LATENT_TC_TILE + 1)
     return max(1, min(blocks, 296 // tiles)) if tiles <= 148 else 1
@@ -1577,29 +1578,30 @@ def latent_expand_rows(max_ctx: int, portions: int) -> int:
     return portions * ((max_ctx + 127) // 128) * 128
 
 
-def latent_expand_takes(num_tokens: int, portions: int, max_ctx: int, heads: int, head_dim: int, value_dim: int, kv_rank: int) -> bool:
+def latent_expand_takes(num_tokens: int, portions: int, max_ctx: int, heads: int, key_dim: int, value_dim: int, kv_rank: int, rot_dim: int = 0,
+                        window: int = 0) -> bool:
     """Whether the portions of a step take the expanded form: where it is possible, where it fits, and where it is the
-    faster one.  The estimate counts flops at the rates the kernels reach on one B200 (TFLOP/s: products 900, tcgen05
-    attention 300, attention over the latent 115, products per head 80) and 15 us for the two more launches; the choice
-    depends on the step's sizes alone."""
+    faster one.  ``key_dim``: a head's key, rotated part and all.  The estimate counts flops at the rates the kernels reach on
+    one B200 (TFLOP/s: products 900, tcgen05 attention 300, attention over the latent 115, products per head 80) and 15 us
+    for the two more launches; the choice depends on the step's sizes alone."""
     rows = latent_expand_rows(max_ctx, portions)
     if (LATENT_PORTIONS == "absorb" or portions <= 0 or _PREFILL_IMPL != "tc" or _FORCE_ATTN == "generic" or _LATENT_IMPL == "plain"
-            or rows * heads * (head_dim + value_dim) * 2 > LATENT_EXPAND_MAX_BYTES
-            or not lib().aien_paged_attention_prefill_tc_values_supports(head_dim, value_dim, 128)):
+            or rows * heads * (key_dim + value_dim) * 2 > LATENT_EXPAND_MAX_BYTES
+            or not lib().aien_paged_attention_prefill_tc_portions_supports(key_dim, value_dim, 128)):
         return False
     if LATENT_PORTIONS == "expand":
         return True
-    pairs = num_tokens * max_ctx * 0.75 * heads
-    both = 2 * (head_dim + value_dim)
-    expand = rows * heads * both * kv_rank / 900e6 + pairs * both / 300e6 + 15.0
-    absorb = pairs * 4 * kv_rank / 115e6 + num_tokens * heads * both * kv_rank / 80e6
+    pairs = num_tokens * (min(max_ctx * 0.75, window) if window > 0 else max_ctx * 0.75) * heads
+    both = 2 * (key_dim + value_dim)
+    expand = rows * heads * both * (kv_rank + rot_dim) / 900e6 + pairs * both / 300e6 + 15.0
+    absorb = pairs * (4 * kv_rank + 2 * rot_dim) / 115e6 + num_tokens * heads * (both - 2 * rot_dim) * kv_rank / 80e6
     return expand < absorb
 
 
 def latent_gather(cache: torch.Tensor, group, q_start: torch.Tensor, ctx_len: torch.Tensor, num_seqs: int, portions: int, length: int,
                   out: torch.Tensor, table: torch.Tensor) -> None:
-    """The cached latents of the requests that bring several tokens, one after the other in ``out`` [portions * length,
-    kv_rank] (rows beyond a context are zeros); ``table`` int32 [num_seqs, length / 128]: the 128-row pages of a request's rows."""
+    """The cached rows of the requests that bring several tokens, one after the other in ``out`` [portions * length,
+    kv_rank + rot_dim] (rows beyond a context are zeros); ``table`` int32 [num_seqs, length / 128]: the 128-row pages of a request's rows."""
     _dev(cache, group.block_table, q_start, ctx_len, out, table)
     assert cache.dtype == torch.bfloat16 and cache.is_contiguous() and out.is_contiguous() and tuple(out.shape) == (portions * length, cache.shape[-1])
     assert length % 128 == 0 and table.dtype == torch.int32 and tuple(table.shape) == (num_seqs, length // 128)
@@ -1958,8 +1960,6 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
                                      _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), _stream()), "selective_scan")
 
 
-def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
-             state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, y: torch.Tensor,
 def split_rows(x: torch.Tensor, out: torch.Tensor) -> None:
     """x float32 [T, n] as the sum of three bfloat16 rows side by side, out [T, 3 n] (up to 2^-25 of x): the left operand of
     a tensor-core product that must not round its float32 rows, with the weights three times side by side."""
@@ -1969,6 +1969,8 @@ def split_rows(x: torch.Tensor, out: torch.Tensor) -> None:
 
 
              num_seqs: int, heads: int, V: int, G: int, N: int, seg_len: int = 0, nseg: int = 1, scratch: Optional[torch.Tensor] = None,
+def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
+             state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, y: torch.Tensor,
              steps: Optional[torch.Tensor] = None, blocks: Optional[torch.Tensor] = None) -> None:
     """The state-space-duality recurrence over every request's portion: per head h (group g = h // (heads // G)), token by
     token, dt = softplus(dtr[h] + dt_bias[h]); S = exp(-A[h] * dt) * S + dt * B[g] x[h]^T (S is N x V); y[h] = S^T C[g] +

@@ -25,8 +25,8 @@ class LatentAttention(Mixer):
     The cache keeps one row [c | k_rot] per token and nothing per head.  Two forms of the same sums read it.  *Absorbed*:
     no head's keys or values are built; W_uk is applied to the query (q_lat = W_uk,h^T q_unrot) and W_uv to the weighted
     sum of latents, so a cached row serves every head as key and as value.  *Expanded* (portions of prompts in a bfloat16
-    engine, without a rotated part): the contexts' keys and values are made per head by one product for the length of the
-    step, which costs less than carrying every score and sum at the latent's size as soon as a portion has more than
+    engine, keys of up to 192 numbers): the contexts' keys and values are made per head by one product for the length of the
+    step (its matrix copies the rotated part through for every head), which costs less than carrying every score and sum at the latent's size as soon as a portion has more than
     a few dozen tokens (``kernels.latent_expand_takes``); single tokens beside them take the absorbed form.  ``own_cache`` False: the layer has no W_dkv and attends over the rows
     another layer wrote (its run binding names that layer's planes).  ``cache_window``: how many positions the cache
     must keep, when layers that share it have different windows (default: ``window``)."""
@@ -60,8 +60,8 @@ class LatentAttention(Mixer):
         self.side_rows, self.riders = self.gate_rows, 0                  # and those behind them: gates, riders
         self.row = self.kv_rank + self.rot_dim
         # the expanded form of portions (a bfloat16 engine's)
-        self._expandable = self.rot_dim == 0 and self.kv_rank % 8 == 0 and self.head_dim % 8 == 0 and self.value_dim % 8 == 0 \
-            and max(self.head_dim, self.value_dim) <= 128
+        self._expandable = all(d % 8 == 0 for d in (self.rot_dim, self.kv_rank, self.head_dim, self.value_dim)) \
+            and self.q_head <= 192 and self.value_dim <= 128
         self.w_kv = None
         self.w_down = self.w_uq = self.w_uk_t = self.w_uv = self.w_o = self.dq_norm = self.dkv_norm = self.sinks = None
 
@@ -105,7 +105,14 @@ class LatentAttention(Mixer):
         self.w_uk_t = tensors["uk_proj"].view(n, self.head_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = tensors["uv_proj"].view(n, self.value_dim, self.kv_rank).contiguous()
         if self._expandable and tensors["uk_proj"].dtype == torch.bfloat16 == tensors["uv_proj"].dtype:
-            self.w_kv = torch.cat([tensors["uk_proj"], tensors["uv_proj"]], dim=0).contiguous()      # all heads' keys | all heads' values
+            # all heads' keys (unrotated | rotated part, the latter copied through by ones) | all heads' values, from whole cached rows
+            w = torch.zeros((n * (self.q_head + self.value_dim), self.row), dtype=torch.bfloat16, device=tensors["uk_proj"].device)
+            k = w[:n * self.q_head].view(n, self.q_head, self.row)
+            k[:, :self.head_dim, :self.kv_rank] = tensors["uk_proj"].view(n, self.head_dim, self.kv_rank)
+            if self.rot_dim:
+                k[:, self.head_dim:, self.kv_rank:] = torch.eye(self.rot_dim, dtype=torch.bfloat16, device=w.device)
+            w[n * self.q_head:, :self.kv_rank] = tensors["uv_proj"]
+            self.w_kv = w
         self.dq_norm = tensors["dq_norm"].contiguous() if self.q_rank else None
         if self.own_cache:
             self.dkv_norm = tensors["dkv_norm"].contiguous()
@@ -128,24 +135,28 @@ class LatentAttention(Mixer):
         expand = 0
         if self._expandable and lim.itemsize == 2:
             rows = K.latent_expand_rows(lim.max_context, lim.max_seqs)
-            per_row = n * (self.head_dim + self.value_dim) * 2
+            per_row = n * (self.q_head + self.value_dim) * 2
             rows = min(rows, K.LATENT_EXPAND_MAX_BYTES // per_row + 128)
-            expand = rows * (per_row + self.kv_rank * 2) + lim.max_seqs * (lim.max_context // 128 + 2) * 4 + 4096
+            expand = rows * (per_row + self.row * 2) + lim.max_seqs * (lim.max_context // 128 + 2) * 4 + 4096
         return lim.max_tokens * per_token + 16384 + split + K.PARTIALS_MAX_BYTES + expand
 
     # ---- one step
-    def _expanded(self, ctx, q, cache, group, portions, gate, o):
-        """The portions' rows of ``o``: keys and values per head for the length of the step."""
+    def _expanded(self, ctx, q, cache, group, portions, gate, o, rot):
+        """The portions' rows of ``o``: keys and values per head for the length of the step.  Turns the rotated part of
+        ``q`` where it lies."""
         n, ws = self.num_heads, ctx.workspace
+        if self.rotary_dim:
+            cos, sin, rdims = rot
+            K.rotate_pairs_rows(q, self.q_head, self.head_dim, q, self.q_head, self.head_dim, n, self.rot_dim, rdims, cos, sin)
         length = K.latent_expand_rows(ctx.max_ctx_len, 1)
-        lat = ws.take((portions * length, self.kv_rank), torch.bfloat16)
+        lat = ws.take((portions * length, self.row), torch.bfloat16)
         table = ws.take((ctx.num_seqs, length // 128), torch.int32)
         K.latent_gather(cache, group, ctx.q_start, ctx.ctx_len, ctx.num_seqs, portions, length, lat, table)
         kv = linear(ctx, lat, self.w_kv)
-        k, v = kv[:, :n * self.head_dim], kv[:, n * self.head_dim:]
+        k, v = kv[:, :n * self.q_head], kv[:, n * self.q_head:]
         by_head = gate if self.head_gate else None
         element = gate if self.out_gate else None
-        K.portion_attention(ctx, q, k, v, table, o, n, self.head_dim, self.value_dim, self.window, self.scale, self.sinks, by_head, element)
+        K.portion_attention(ctx, q, k, v, table, o, n, self.q_head, self.value_dim, self.window, self.scale, self.sinks, by_head, element)
 
     def _absorbed(self, ctx, q, cache, group, tc, gate, o, rot, singles, n_single):
         """Rows of ``o`` over the latent itself: all of the step's, or those of ``singles`` (tokens that come alone)."""
@@ -197,11 +208,11 @@ class LatentAttention(Mixer):
         gate_suits = gate is None or (gate.dtype == torch.float32 if self.head_gate else
                                       gate.dtype == torch.bfloat16 and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)
         expand = tc and self.w_kv is not None and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and gate_suits and \
-            K.latent_expand_takes(T - n_single, portions, ctx.max_ctx_len, n, self.head_dim, self.value_dim, self.kv_rank)
-        if expand:
-            self._expanded(ctx, q[:, :n * self.q_head], cache, group, portions, gate, o)
-        if not expand or n_single > 0:
+            K.latent_expand_takes(T - n_single, portions, ctx.max_ctx_len, n, self.q_head, self.value_dim, self.kv_rank, self.rot_dim, self.window)
+        if not expand or n_single > 0:                                  # first: it reads the query before its rotation
             self._absorbed(ctx, q, cache, group, tc, gate, o, rot, singles if expand else None, n_single if expand else 0)
+        if expand:
+            self._expanded(ctx, q[:, :n * self.q_head], cache, group, portions, gate, o, rot)
         y = linear(ctx, o, self.w_o, out_dtype=torch.float32, may_defer_sum=True)        # the consumer's norm adds partial products
         if not self.riders:
             return y

@@ -684,3 +684,82 @@ def test_configurations_drawn_at_random(seed, tmp_path):
             check(H.run_steps(eng, steps(mode)), want, tol, f"seed {seed} {dtype} {mode}")
             assert eng.cache_state()["check"] == "" and eng.cache_state()["requests"] == 0
 
+
+
+@pytest.mark.parametrize("dim,rot,vdim,heads,q_rank,window,sink", [(128, 64, 128, 3, 48, 200, True), (64, 32, 64, 4, 0, 0, False), (72, 64, 40, 2, 64, 130, True),
+                                                                  (16, 8, 64, 5, 0, 50, True), (128, 8, 24, 1, 32, 0, False)])
+def test_latent_portions_with_a_rotated_part_expanded_and_absorbed(dim, rot, vdim, heads, q_rank, window, sink):
+    """A mixed step (portions that fill no tile, single tokens, a window that has moved on, pages in any order) in both forms
+    against 64 bits.  Four roundings to bfloat16 lie on the way of a result (2^-9 each of numbers its own size, a key's under
+    the softmax): 3e-2 of the largest."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    from aien_sovereign_core_mv_b200.parts import GroupView, RunBinding, StepContext, StepLimits, Workspace
+    from aien_sovereign_core_mv_b200.registry import make_part
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(dim + rot)
+    width, r, page = 96, 64, 16
+    part = make_part("mixer", "latent_attention", hidden_size=width, num_heads=heads, head_dim=dim, rot_dim=rot, value_dim=vdim, kv_rank=r, q_rank=q_rank,
+                     window=window, sink=sink, norm_eps=1e-5,
+                     position=make_part("position", "rotary", head_dim=rot, theta=10000.0, pairing="interleaved"))
+    W = {n: (torch.randn(shape, generator=g, device="cuda") * (shape[-1] ** -0.5 if kind == "matrix" else 1.0)).to(torch.bfloat16)
+         for n, (shape, kind) in part.param_shapes().items()}
+    part.bind(W)
+    bring, held = [150, 1, 40, 1, 2], [37, 260, 300, 0, 11]
+    S, T = len(bring), sum(bring)
+    h = torch.randn(T, width, generator=g, device="cuda").to(torch.bfloat16)
+    q0 = [sum(bring[:s]) for s in range(S + 1)]
+    pages = [(a + b + page - 1) // page for a, b in zip(bring, held)]
+    order = torch.randperm(sum(pages) + 2, generator=g, device="cuda").to(torch.int32)
+    table = torch.full((S, max(pages) + 1), -1, dtype=torch.int32, device="cuda")
+    slot = lambda s, p: table[s, p // page].long() * page + p % page
+    first = torch.zeros(1, (sum(pages) + 2) * page, r + rot, dtype=torch.bfloat16, device="cuda")
+    slots = []
+    for s in range(S):
+        table[s, :pages[s]] = order[sum(pages[:s]):sum(pages[:s + 1])]
+        p = torch.arange(held[s] + bring[s], device="cuda")
+        first[0, slot(s, p[:held[s]])] = torch.randn(held[s], r + rot, generator=g, device="cuda").to(torch.bfloat16)
+        slots.append(slot(s, p[held[s]:]))
+    norm = lambda x, w: x / torch.sqrt(x.square().mean(-1, keepdim=True) + 1e-5) * w
+
+    def turned(x, pos):
+        a = pos.double().view(-1, *([1] * (x.dim() - 1))) * 10000.0 ** (-torch.arange(0, rot, 2, device="cuda").double() / rot)
+        return torch.stack([x[..., 0::2] * a.cos() - x[..., 1::2] * a.sin(), x[..., 1::2] * a.cos() + x[..., 0::2] * a.sin()], -1).flatten(-2)
+
+    D = {n: t.double() for n, t in W.items()}
+    want = []
+    for s in range(S):
+        x, pos = h[q0[s]:q0[s + 1]].double(), torch.arange(held[s], held[s] + bring[s], device="cuda")
+        q = (norm(x @ D["dq_proj"].T, D["dq_norm"]) @ D["uq_proj"].T if q_rank else x @ D["q_proj"].T).view(-1, heads, dim + rot)
+        q = torch.cat([q[..., :dim], turned(q[..., dim:], pos)], -1)
+        d = x @ D["dkv_proj"].T
+        rows = torch.cat([first[0, slot(s, torch.arange(held[s], device="cuda"))].double(), torch.cat([norm(d[:, :r], D["dkv_norm"]), turned(d[:, r:], pos)], -1)])
+        k = torch.cat([(rows[:, :r] @ D["uk_proj"].T).view(-1, heads, dim), rows[:, None, r:].expand(-1, heads, -1)], -1)
+        z = torch.einsum("tnd,mnd->ntm", q, k) * (dim + rot) ** -0.5
+        j = torch.arange(rows.shape[0], device="cuda")
+        z = z.masked_fill((j > pos[:, None]) | (j <= pos[:, None] - (window or 1 << 30)), -float("inf"))
+        if sink:
+            z = torch.cat([z, D["sink"][:, None, None].expand(-1, z.shape[1], 1)], -1)
+        o = torch.einsum("ntm,mnv->tnv", z.softmax(-1)[..., :rows.shape[0]], (rows[:, :r] @ D["uv_proj"].T).view(-1, heads, vdim))
+        want.append(o.flatten(1) @ D["o_proj"].T)
+    want = torch.cat(want).cpu().numpy()
+    need = part.cache_need()
+    tiles = [(s, q) for s in range(S) for q in range(0, bring[s], 128) if bring[s] > 1]
+    lim = StepLimits(max_tokens=T, max_seqs=S, max_context=max(a + b for a, b in zip(bring, held)), itemsize=2)
+    saved = K.LATENT_PORTIONS
+    try:
+        for form in ("absorb", "expand"):
+            K.LATENT_PORTIONS = form
+            store = first.clone()
+            ws = Workspace(1 << 20, part.workspace_bytes(lim) + (1 << 16), torch.device("cuda"))
+            ws.begin_layer()
+            ctx = StepContext(dtype=torch.bfloat16, num_tokens=T, num_seqs=S, token_ids=i32([0] * T),
+                              positions=i32([held[s] + i for s in range(S) for i in range(bring[s])]), seq_of_token=i32([s for s in range(S) for _ in range(bring[s])]),
+                              q_start=i32(q0), ctx_len=i32([a + b for a, b in zip(bring, held)]),
+                              groups=[GroupView(need.kind, page, need.window, table.shape[1], table, torch.cat(slots).to(torch.int32), {"latent": store})],
+                              workspace=ws, max_q_len=max(bring), max_ctx_len=lim.max_context, decode_only=False,
+                              prefill_tiles=(i32([s for s, _ in tiles]), i32([q for _, q in tiles]), len(tiles)), single_tokens=(i32([q0[1], q0[3]]), 2))
+            y = part.forward(ctx, h, RunBinding(0, 0, True))
+            y = (y.float().sum(0) if y.dim() == 3 else y.float()).cpu().numpy()
+            H.assert_close(y, want, 3e-2, form)
+    finally:
+        K.LATENT_PORTIONS = saved
