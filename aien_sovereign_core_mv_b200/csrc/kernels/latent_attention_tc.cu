@@ -16,7 +16,7 @@
 
 namespace aien {
 
-constexpr int LX_BM = 64, LX_BN = 64, LX_PSTR = LX_BN + 8;
+constexpr int LX_BM = 64, LX_BN = 64;
 
 // Numbers a row of D numbers takes in shared memory (without its padding): whole k-steps of 16, and all R columns of the sum.
 __host__ __device__ __forceinline__ int lx_row_width(int R, int D) { return (D + 15) / 16 * 16 > R ? (D + 15) / 16 * 16 : R; }
@@ -50,6 +50,16 @@ __device__ __forceinline__ uint32_t lx_pack(float lo, float hi) {
 // a request has only its heads as rows).  The WARPS / SLABS warps of a slab deal out the keys of a block for the scores and
 // the channels for the weighted sum (tiles of 64 rows run 16 warps: four to a slab, so that a warp's share of the weighted
 // sum, 16 rows x a quarter of the latent, leaves registers for loads in flight).
+//
+// Tiles of 16 rows are bound by the reading of their keys.  They take them in blocks of 32 through two stages, the next one
+// requested before the products of this one, by CTAs of four warps that fit an SM twice (85 KB at a latent of 512); where a key's
+// row lies is looked up a block further ahead, by one thread a key, and a warp then copies whole rows.  With a block of 64
+// looked up, copied and waited for in turn (every 16-byte piece with its own look-up), 64 requests at 1,500 tokens of
+// context took 126 us for 98 MB; 50 us so, with four CTAs a token instead of two (a token's 16 heads are one tile).
+template <int SLABS> struct LxBlock {
+    static constexpr int BN = SLABS == 1 ? 32 : 64, STAGES = SLABS == 1 ? 2 : 1, PSTR = BN + 8;
+};
+
 template <int R, int SLABS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, SLABS == 1 ? 2 : 1)
 latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
@@ -57,32 +67,42 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
                            const int* __restrict__ positions, int S, __nv_bfloat16* __restrict__ out,
                            int H, int r_lat, int rd, int page_size, int window, float scale_log2e, const float* __restrict__ sinks,
                            int ksplit, float* __restrict__ part_o, float* __restrict__ part_ml, int single_only) {
-    constexpr int BM = SLABS * 16, PARTS = WARPS / SLABS, KP = LX_BN / PARTS, NJ = KP / 8, CHP = R / PARTS, THREADS = WARPS * 32;
+    constexpr int LX_BN = LxBlock<SLABS>::BN, STAGES = LxBlock<SLABS>::STAGES, LX_PSTR = LxBlock<SLABS>::PSTR;
+    constexpr int BM = SLABS * 16, PARTS = WARPS / SLABS, KP = LX_BN / PARTS, NJ = KP / 8, CHP = R / PARTS;
     constexpr int DT = CHP / 8;                  // n8 tiles of this warp's share of the channels
     static_assert(DT >= 2 && DT % 2 == 0, "a warp's share of the latent must be whole pairs of n8 tiles");
     // r_lat <= R: the latent's own size; a row's D numbers are read, the rest of its width in shared memory is zeros
     const int D = r_lat + rd, CH = D / 8, KS = (D + 15) / 16, W = lx_row_width(R, D), CHW = W / 8, STR = W + 8;
     extern __shared__ __align__(16) uint8_t lx_smem[];
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(lx_smem);          // [BM][STR]
-    __nv_bfloat16* Ks = Qs + BM * STR;                                      // [64][STR]
-    __nv_bfloat16* Ps = Ks + LX_BN * STR;                                   // [BM][LX_PSTR]
+    __nv_bfloat16* Ks = Qs + BM * STR;                                      // [STAGES][BN][STR]
+    __nv_bfloat16* Ps = Ks + STAGES * LX_BN * STR;                          // [BM][PSTR]
     float* stat = reinterpret_cast<float*>(Ps + BM * LX_PSTR);              // [PARTS][BM]
-    __shared__ int key_there[LX_BN];                                        // whether the block's key is in the cache and needed
-    const uint32_t Qs_u = (uint32_t)__cvta_generic_to_shared(Qs), Ks_u = (uint32_t)__cvta_generic_to_shared(Ks);
+    __shared__ int key_row[2][LX_BN];                                       // the cache row of a block's key, -1: not there or not needed
+    const uint32_t Qs_u = (uint32_t)__cvta_generic_to_shared(Qs), Ks0_u = (uint32_t)__cvta_generic_to_shared(Ks);
     const uint32_t Ps_u = (uint32_t)__cvta_generic_to_shared(Ps);
 
-    // which request, which rows
-    int s = -1, row0 = 0, acc = 0, unit = 0;             // unit: how many served tokens come before a single one
-    for (int i = 0; i < S; ++i) {
-        const int n = q_start[i + 1] - q_start[i];
+    // which request, which rows: the lanes count 32 requests' tiles at a time
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int s = -1, row0 = 0, unit = 0;                      // unit: how many served tokens come before a single one
+    for (int base = 0, acc = 0; base < S; base += 32) {
+        const int i = base + lane, n = i < S ? q_start[i + 1] - q_start[i] : 0;
         const int tiles = single_only && n != 1 ? 0 : (n * H + BM - 1) / BM;         // single_only: portions are served elsewhere
-        if ((int)blockIdx.x < acc + tiles) {
-            s = i;
-            row0 = ((int)blockIdx.x - acc) * BM;
-            unit = acc / tiles;
+        int upto = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const uint32_t here = __ballot_sync(0xffffffffu, acc + upto > (int)blockIdx.x);
+        if (here != 0) {
+            const int l = __ffs(here) - 1, before = acc + __shfl_sync(0xffffffffu, upto - tiles, l);
+            s = base + l;
+            row0 = ((int)blockIdx.x - before) * BM;
+            unit = before / __shfl_sync(0xffffffffu, tiles, l);
             break;
         }
-        acc += tiles;
+        acc += __shfl_sync(0xffffffffu, upto, 31);
     }
     if (s < 0) return;
     const int qs = q_start[s], len = q_start[s + 1] - qs;
@@ -92,18 +112,15 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
     const int first = (window > 0 && pos_lo - window + 1 > 0) ? pos_lo - window + 1 : 0;
     const int* bt = block_table + (size_t)s * max_blocks;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int slab = warp % SLABS, half = warp / SLABS;                     // half: which share of the keys / channels
     const int g = lane >> 2, c = lane & 3;
 
     const __nv_bfloat16* qbase = q + ((size_t)qs * H + row0) * D;
-    for (int idx = tid; idx < BM * CHW; idx += THREADS) {
-        const int r = idx / CHW, ch = idx - r * CHW;
-        const bool valid = r < nrows && ch < CH;
-        lx_cp_async16(Qs_u + (uint32_t)(r * STR + ch * 8) * 2, qbase + (valid ? (size_t)r * D + ch * 8 : 0), valid);
-    }
-    lx_cp_async_commit();
-
+    for (int r = warp; r < BM; r += WARPS)
+        for (int ch = lane; ch < CHW; ch += 32) {
+            const bool valid = r < nrows && ch < CH;
+            lx_cp_async16(Qs_u + (uint32_t)(r * STR + ch * 8) * 2, qbase + (valid ? (size_t)r * D + ch * 8 : 0), valid);
+        }
     const uint32_t q_frag_u = Qs_u + (uint32_t)((slab * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * STR + (lane >> 4) * 8) * 2;
     const uint32_t p_frag_u = Ps_u + (uint32_t)((slab * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * LX_PSTR + (lane >> 4) * 8) * 2;
 
@@ -116,31 +133,52 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
     const int wlo0 = window > 0 ? qpos0 - window + 1 : 0, wlo1 = window > 0 ? qpos1 - window + 1 : 0;
     const bool active = slab * 16 < nrows;
 
-    const int kb_begin = first / LX_BN, kb_end = pos_hi / LX_BN;
-    if (ksplit > 1) {                                                      // Q must have landed even if this CTA gets no block
+    const int kb_begin = first / LX_BN, kb_end = pos_hi / LX_BN, kb0 = kb_begin + (int)blockIdx.y;
+    // where the keys of block kb lie (one thread a key), and the copies of its rows (a warp a row)
+    auto look_up = [&](int kb, int* rows) {
+        if (tid < LX_BN) {
+            const int key = kb * LX_BN + tid;
+            const int page = kb <= kb_end && key >= first && key <= pos_hi ? bt[key / page_size] : -1;
+            rows[tid] = page >= 0 ? page * page_size + key % page_size : -1;
+        }
+    };
+    auto copy_rows = [&](const int* rows, uint32_t dst) {
+#pragma unroll 2
+        for (int r = warp; r < LX_BN; r += WARPS) {
+            const int slot = rows[r];
+            const __nv_bfloat16* src = cache + (slot >= 0 ? (size_t)slot * D : 0);
+            for (int ch = lane; ch < CHW; ch += 32) {
+                const bool copy = slot >= 0 && ch < CH;
+                lx_cp_async16(dst + (uint32_t)(r * STR + ch * 8) * 2, src + (copy ? ch * 8 : 0), copy);
+            }
+        }
+    };
+    look_up(kb0, key_row[0]);
+    look_up(kb0 + ksplit, key_row[1]);
+    __syncthreads();
+    if (STAGES == 2 && kb0 <= kb_end) copy_rows(key_row[0], Ks0_u);
+    lx_cp_async_commit();
+    if (ksplit > 1 && kb0 > kb_end) {                                      // Q must have landed even if this CTA gets no block
         lx_cp_async_wait_all();
         __syncthreads();
     }
-    for (int kb = kb_begin + (int)blockIdx.y; kb <= kb_end; kb += ksplit) {
-        for (int idx = tid; idx < LX_BN * CHW; idx += THREADS) {
-            const int r = idx / CHW, ch = idx - r * CHW;
-            const int key = kb * LX_BN + r;
-            bool valid = key >= first && key <= pos_hi;
-            long slot = 0;
-            if (valid) {
-                const int page = bt[key / page_size];
-                valid = page >= 0;
-                slot = (long)page * page_size + key % page_size;
-            }
-            const bool copy = valid && ch < CH;
-            lx_cp_async16(Ks_u + (uint32_t)(r * STR + ch * 8) * 2, cache + (copy ? (size_t)slot * D + ch * 8 : 0), copy);
-            if (ch == 0) key_there[r] = valid ? 1 : 0;
+    for (int kb = kb0, it = 0; kb <= kb_end; kb += ksplit, ++it) {
+        const int* rows = key_row[it & 1];
+        uint32_t Ks_u = Ks0_u;
+        if (STAGES == 1) {
+            copy_rows(rows, Ks0_u);
+            lx_cp_async_commit();
+            lx_cp_async_wait_all();
+            __syncthreads();                                               // the block's rows (and, first time, Q) have landed
+        } else {
+            Ks_u += (uint32_t)((it & 1) * LX_BN * STR) * 2;
+            lx_cp_async_wait_all();
+            __syncthreads();                                               // likewise, and everyone is done with the other stage
+            if (kb + ksplit <= kb_end) copy_rows(key_row[(it + 1) & 1], Ks0_u + (uint32_t)(((it + 1) & 1) * LX_BN * STR) * 2);
+            lx_cp_async_commit();
         }
-        lx_cp_async_commit();
-        lx_cp_async_wait_all();
-        __syncthreads();                                                   // the block's rows (and, first time, Q) have landed
 
-        float sc[NJ][4];
+        float sc[NJ][4], sc2[4] = {0.f, 0.f, 0.f, 0.f};                    // sc2: every other k-step's sums where a warp has one tile of keys
 #pragma unroll
         for (int j = 0; j < NJ; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
         if (active) {
@@ -152,7 +190,7 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
                     const int row = half * KP + (lane & 7), col = kk * 16 + ((lane >> 3) & 1) * 8;
                     uint32_t b0, b1;
                     lx_ldmatrix_x2(Ks_u + (uint32_t)(row * STR + col) * 2, b0, b1);
-                    lx_mma(sc[0], q0r, q1r, q2r, q3r, b0, b1);
+                    lx_mma((kk & 1) ? sc2 : sc[0], q0r, q1r, q2r, q3r, b0, b1);
                 } else {
 #pragma unroll
                     for (int j = 0; j < NJ; j += 2) {
@@ -166,6 +204,10 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
                 }
             }
         }
+        if constexpr (NJ == 1) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sc[0][e] += sc2[e];
+        }
         // masks and this half's row maxima (scores in log2 units)
         float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
@@ -173,7 +215,7 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int kl = half * KP + j * 8 + 2 * c + e, key = kb * LX_BN + kl;
-                const bool there = key_there[kl] != 0;
+                const bool there = rows[kl] >= 0;
                 const bool ok0 = there && key <= qpos0 && key >= wlo0, ok1 = there && key <= qpos1 && key >= wlo1;
                 sc[j][e] = ok0 ? sc[j][e] * scale_log2e : -INFINITY;
                 sc[j][2 + e] = ok1 ? sc[j][2 + e] * scale_log2e : -INFINITY;
@@ -230,6 +272,8 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
                 }
             }
         }
+        // (block kb's places have been read for the last time before the barrier above)
+        look_up(kb + 2 * ksplit, key_row[it & 1]);
         __syncthreads();                                                   // every warp is done with this block
     }
 
@@ -348,12 +392,12 @@ static int launch_latent_tc(const void* q, const void* cache, const int* bt, int
                             int ksplit, float* part_o, float* part_ml, const int* tokens, int num_tokens, cudaStream_t stream) {
     const int D = r_lat + rd;
     constexpr int BM = SLABS * 16;
-    const size_t smem = (size_t)(BM + LX_BN) * (lx_row_width(R, D) + 8) * 2 + (size_t)BM * LX_PSTR * 2 + (size_t)WARPS * 16 * sizeof(float);
+    const size_t smem = (size_t)(BM + LxBlock<SLABS>::STAGES * LxBlock<SLABS>::BN) * (lx_row_width(R, D) + 8) * 2 + (size_t)BM * LxBlock<SLABS>::PSTR * 2 + (size_t)WARPS * 16 * sizeof(float);
     if (smem > 227 * 1024) return AIEN_E_SHAPE;
     auto kern = latent_attention_tc_kernel<R, SLABS, WARPS>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return AIEN_E_STATE;
     // tokens: only these, each a request's one token of the step
-    const long tiles = tokens != nullptr ? (long)num_tokens * ((H + BM - 1) / BM) : ((long)T * H) / BM + S;
+    const long tiles = tokens != nullptr || T == S ? (long)(tokens != nullptr ? num_tokens : T) * ((H + BM - 1) / BM) : ((long)T * H) / BM + S;
     kern<<<dim3((unsigned)tiles, ksplit), WARPS * 32, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start,
                                                                      positions, S, (__nv_bfloat16*)out, H, r_lat, rd, page_size, window,
                                                                      scale * 1.4426950408889634f, sinks, ksplit, part_o, part_ml, tokens != nullptr ? 1 : 0);
@@ -506,7 +550,7 @@ static int lx_padded_rank(int kv_rank) { return kv_rank <= 64 ? 64 : (kv_rank <=
 
 AIEN_API int aien_latent_attention_tc_supports(int kv_rank, int rot_dim) {
     if (kv_rank <= 0 || kv_rank > 512 || (kv_rank & 7) || rot_dim < 0 || (rot_dim & 7)) return 0;
-    const size_t smem = (size_t)(LX_BM + LX_BN) * (lx_row_width(lx_padded_rank(kv_rank), kv_rank + rot_dim) + 8) * 2 + (size_t)LX_BM * LX_PSTR * 2 + 16 * 16 * sizeof(float);
+    const size_t smem = (size_t)(LX_BM + LX_BN) * (lx_row_width(lx_padded_rank(kv_rank), kv_rank + rot_dim) + 8) * 2 + (size_t)LX_BM * LxBlock<4>::PSTR * 2 + 16 * 16 * sizeof(float);
     return smem <= 227 * 1024 ? 1 : 0;
 }
 
@@ -527,7 +571,7 @@ AIEN_API int aien_latent_attention_tc(const void* q, const void* cache, const in
     const int padded = lx_padded_rank(kv_rank);
 #define LX_CASE(RV, SL)                                                                                                          \
     if (padded == RV)                                                                                                            \
-        return launch_latent_tc<RV, SL, (SL == 4 ? 16 : 8)>(q, cache, block_table, max_blocks, q_start, positions, T, S, out, H, kv_rank, rot_dim, page_size,  \
+        return launch_latent_tc<RV, SL, (SL == 4 ? 16 : 4)>(q, cache, block_table, max_blocks, q_start, positions, T, S, out, H, kv_rank, rot_dim, page_size,  \
                                         window, scale, sinks, ksplit, part_o, part_ml, tokens, num_tokens, stream);
     if (small_tiles && padded >= 128) {                    // tiles of 16 rows: a latent of 64 would leave a warp half a pair of n8 tiles
         LX_CASE(128, 1) LX_CASE(256, 1) LX_CASE(512, 1)

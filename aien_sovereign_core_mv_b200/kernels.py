@@ -1563,7 +1563,8 @@ def latent_attention_tc_ksplit(num_tokens: int, num_seqs: int, heads: int, max_c
     when the step has few tiles, never more than a tile has blocks.  Depends on the step's sizes only."""
     tiles = num_tokens * ((heads + 15) // 16) if small_tiles else (num_tokens * heads) // LATENT_TC_TILE + num_seqs
     span = min(window, max_ctx) if window > 0 else max_ctx
-    blocks = max(1, (span + LATENT_TC_TILE - 1) // LATENT_TC_TILE + 1)
+    block = 32 if small_tiles else LATENT_TC_TILE
+    blocks = max(1, (span + block - 1) // block + 1)
     return max(1, min(blocks, 296 // tiles)) if tiles <= 148 else 1
 
 
@@ -1968,9 +1969,9 @@ def split_rows(x: torch.Tensor, out: torch.Tensor) -> None:
     _check(lib().aien_split_rows(_p(x), x.stride(0), _p(out), x.shape[0], x.shape[1], _stream()), "split_rows")
 
 
-             num_seqs: int, heads: int, V: int, G: int, N: int, seg_len: int = 0, nseg: int = 1, scratch: Optional[torch.Tensor] = None,
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
              state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, y: torch.Tensor,
+             num_seqs: int, heads: int, V: int, G: int, N: int, seg_len: int = 0, nseg: int = 1, scratch: Optional[torch.Tensor] = None,
              steps: Optional[torch.Tensor] = None, blocks: Optional[torch.Tensor] = None) -> None:
     """The state-space-duality recurrence over every request's portion: per head h (group g = h // (heads // G)), token by
     token, dt = softplus(dtr[h] + dt_bias[h]); S = exp(-A[h] * dt) * S + dt * B[g] x[h]^T (S is N x V); y[h] = S^T C[g] +
