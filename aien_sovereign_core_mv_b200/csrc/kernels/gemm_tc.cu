@@ -215,6 +215,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
 }
 
+// a chunk's values through the activation that a grouped product applies ahead of its store
+template <int EPI>
+__device__ __forceinline__ void tc_activate(uint32_t (&r)[32]) {
+    if (EPI == 2) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(tc_gelu_erf(__uint_as_float(r[j])));
+    } else if (EPI == 3) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(tc_gelu_tanh(__uint_as_float(r[j])));
+    } else if (EPI == 4) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(tc_relu2(__uint_as_float(r[j])));
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // The grouped form, for routed experts: the rows of A are sorted by group (expert), every group's
 // run of rows starts at a multiple of 128, and W holds the groups' matrices one below the other
@@ -318,16 +333,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
                 for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * rs);
             }
-            if (EPI == 2) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(tc_gelu_erf(__uint_as_float(r[j])));
-            } else if (EPI == 3) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(tc_gelu_tanh(__uint_as_float(r[j])));
-            } else if (EPI == 4) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(tc_relu2(__uint_as_float(r[j])));
-            }
+            tc_activate<EPI>(r);
             if (row_dest != nullptr && row_scale != nullptr) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * rs);
@@ -502,6 +508,170 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)P::TMEM_COLS) : "memory");
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The grouped product (gemm_tc_grouped_kernel: A's rows sorted by group, runs of whole 128-row tiles, tile_group[m] the
+// group of row tile m, negative for the tiles behind the last run) in the persistent form with tiles of 128 x 256.  What
+// bounds the 128 x 128 tiles, two CTAs an SM, is shared memory (see above), and every tile waits for its own first k-blocks
+// and its own epilogue; here both run under the next tile's products.  Units are ordered column tiles fastest, as
+// there, so a row tile of A and one expert's W come from HBM once.  2,048 tokens x 6 of 64 experts (12,288 rows), up
+// 768 x 2,048 / down 2,048 x 768: 88 and 97 us in 128 x 128 tiles, 71 and 76 so.  (Asking for W's boxes in L2 eight
+// k-blocks ahead of the ring made them 77 and 90.)
+template <int EPI, typename TC>
+__global__ void __launch_bounds__(192, 1)
+gemm_tc_grouped_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                                  TC* __restrict__ out, long ldc, const int* __restrict__ tile_group, int m_tiles, const int* __restrict__ row_dest,
+                                  const float* __restrict__ row_scale, int N, int K) {
+    constexpr int BN = 256;
+    using P = TcP<BN>;
+    constexpr int STAGES = P::STAGES;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t sA = base, sB = base + STAGES * P::STAGE_A;
+    const uint32_t bars = sB + STAGES * P::STAGE_B;
+    const uint32_t full0 = bars, empty0 = bars + 8 * STAGES, tfull0 = bars + 16 * STAGES, tempty0 = tfull0 + 16;
+    const uint32_t tmem_slot = tempty0 + 16;
+    uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen + (tmem_slot - base));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_tiles = (N + BN - 1) / BN, total = m_tiles * n_tiles;
+    const int num_kb = (K + TC_BK - 1) / TC_BK;
+
+    griddep_launch();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)P::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_acc = *tmem_slot_ptr;
+    griddep_wait();                                       // the rows and the tile map are the kernels' ahead
+    // every role walks the same units: u = (row tile, column tile), up to the first row tile without a group
+    auto group_of = [&](int u) { return u < total ? __ldcg(tile_group + u / n_tiles) : -1; };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            for (int u = blockIdx.x, group = group_of(u); group >= 0; u += gridDim.x, group = group_of(u)) {
+                const int m0 = (u / n_tiles) * TC_BM, w0 = group * N + (u % n_tiles) * BN;
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (it >= (uint32_t)STAGES) mbar_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1, 1);
+                    mbar_expect_tx(full0 + 8 * s, P::STAGE_A + P::STAGE_B);
+                    tma_load_2d(sA + s * P::STAGE_A, &map_a, full0 + 8 * s, kb * TC_BK, m0);
+                    tma_load_2d(sB + s * P::STAGE_B, &map_w, full0 + 8 * s, kb * TC_BK, w0);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = umma_idesc_bf16(TC_BM, BN, false);
+            uint32_t it = 0;
+            int i = 0;
+            for (int u = blockIdx.x, group = group_of(u); group >= 0; u += gridDim.x, group = group_of(u), ++i) {
+                const int acc = i & 1;
+                if (i >= 2) mbar_wait(tempty0 + 8 * acc, ((i >> 1) - 1) & 1, 4);      // the epilogue has drained this accumulator
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    mbar_wait(full0 + 8 * s, (it / STAGES) & 1, 2);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t da = make_desc_sw128(sA + s * P::STAGE_A), db = make_desc_sw128(sB + s * P::STAGE_B);
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; ++k)
+                        umma_bf16(tmem_acc + acc * (P::TMEM_COLS / 2), da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(empty0 + 8 * s);
+                }
+                umma_commit(tfull0 + 8 * acc);
+            }
+        }
+    } else {
+        const int quarter = warp & 3;
+        const bool scale_first = row_dest == nullptr && row_scale != nullptr;
+        int i = 0;
+        for (int u = blockIdx.x, group = group_of(u); group >= 0; u += gridDim.x, group = group_of(u), ++i) {
+            const int acc = i & 1;
+            const int row = (u / n_tiles) * TC_BM + quarter * 32 + lane, n0 = (u % n_tiles) * BN;
+            int dest = row;
+            float rs = 1.0f;
+            if (row_dest != nullptr) dest = __ldcg(row_dest + row);
+            if (row_scale != nullptr) rs = __ldcg(row_scale + row);
+            mbar_wait(tfull0 + 8 * acc, (i >> 1) & 1, 3);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN && n0 + c0 < N; c0 += 32) {
+                uint32_t r[32];
+                tmem_ld32(tmem_acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * (P::TMEM_COLS / 2) + c0), r);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (scale_first) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * rs);
+                }
+                tc_activate<EPI>(r);
+                if (row_dest != nullptr && row_scale != nullptr) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * rs);
+                }
+                if (dest >= 0) tc_store_chunk<(EPI == 1 ? 1 : 0), TC>(r, out, ldc, dest, n0, c0, N);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)P::TMEM_COLS) : "memory");
+    }
+}
+
+static int tc_num_sms();
+
+// Row tiles with work are known on the device only; a step of `pairs` rows spread evenly has groups * ceil(pairs / groups /
+// 128) of them.  By the cycles a k-block takes (128 x 256: 760; 128 x 128: 600 alone, 1,024 for two CTAs of an SM), the
+// epilogue that nothing hides (9,000 and 5,000) and the waves either way: 300 tokens x 4 of 16 experts, 1,024 x 512 down,
+// take 12.5 us in 128 x 128 tiles and 16 in the others.
+static bool tc_grouped_persistent(int tiles, int groups, int N, int K) {
+    static const char* e = getenv("AIEN_B200_GEMM_GROUPED");               // "tile" / "persistent" pin the form
+    if (e != nullptr && (e[0] == 't' || e[0] == 'p')) return e[0] == 'p';
+    const long sms = tc_num_sms(), kb = (K + TC_BK - 1) / TC_BK;
+    const long real = tiles > groups ? tiles - groups : 1;                 // `tiles` is pairs / 128 + groups: what must be there
+    const long used = real > groups ? real + groups / 2 : groups;
+    const long small = used * ((N + 127) / 128);
+    const long wide = ((used * ((N + 255) / 256) + sms - 1) / sms) * (kb * 760) + 9000;
+    const long narrow = ((small + 2 * sms - 1) / (2 * sms)) * (kb * (small > sms ? 1024 : 600) + 5000);
+    return wide < narrow;
+}
+
+template <int EPI, typename TC>
+static int launch_tc_grouped_persistent(const void* A, long lda, int rows_a, const void* W, long ldw, int groups, void* out, long ldc,
+                                        const int* tile_group, int tiles, const int* row_dest, const float* row_scale, int N, int K,
+                                        cudaStream_t stream) {
+    using P = TcP<256>;
+    CUtensorMap ma, mw;
+    if (!make_map(&ma, A, (uint64_t)rows_a, (uint64_t)K, (uint64_t)lda, TC_BK, 128u) ||
+        !make_map(&mw, W, (uint64_t)groups * (uint64_t)N, (uint64_t)K, (uint64_t)ldw, TC_BK, 256u))
+        return AIEN_E_STATE;
+    auto kern = gemm_tc_grouped_persistent_kernel<EPI, TC>;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM) != cudaSuccess) return AIEN_E_STATE;
+        configured = true;
+    }
+    const long units = (long)tiles * ((N + 255) / 256);
+    const unsigned grid = (unsigned)(units < tc_num_sms() ? units : tc_num_sms());
+    launch_chain(kern, dim3(grid), dim3(192), (size_t)P::SMEM, stream, ma, mw, (TC*)out, ldc, tile_group, tiles, row_dest, row_scale, N, K);
+    return launch_status();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -914,7 +1084,9 @@ AIEN_API int aien_gemm_tc_grouped(const void* A, long lda, const void* W, long l
     if ((lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return AIEN_E_ALIGN;
     if ((long)tiles * ((N + 127) / 128) > 2147483647L || (long)groups * N > 2147483647L) return AIEN_E_SHAPE;
     const int rows_a = tiles * 128;
-#define TCG_CASE(EPIV, T) return launch_tc_grouped<EPIV, T>(A, lda, rows_a, W, ldw, groups, out, ldc, tile_group, tiles, row_dest, row_scale, N, K, stream)
+    const bool persistent = tc_grouped_persistent(tiles, groups, N, K);
+#define TCG_CASE(EPIV, T) return persistent ? launch_tc_grouped_persistent<EPIV, T>(A, lda, rows_a, W, ldw, groups, out, ldc, tile_group, tiles, row_dest, row_scale, N, K, stream) \
+                                            : launch_tc_grouped<EPIV, T>(A, lda, rows_a, W, ldw, groups, out, ldc, tile_group, tiles, row_dest, row_scale, N, K, stream)
     if (c_dt == AIEN_DT_BF16) {
         if (epilogue == 0) TCG_CASE(0, __nv_bfloat16);
         if (epilogue == 1) TCG_CASE(1, __nv_bfloat16);

@@ -1203,3 +1203,50 @@ def test_cache_housekeeping_kernels(K):
     assert (buf[3:990] == 0).all() and (buf[:3] == 7).all() and (buf[990:] == 7).all()
     big = torch.full((1 << 20,), 3.0, device="cuda")
     assert (K.zero_fill(big) == 0).all()
+
+
+@pytest.mark.parametrize("N,K,counts", [(768, 136, [130, 0, 1, 256]), (264, 64, [5, 128, 129]), (8, 1032, [0, 77]), (2048, 24, [400] * 40), (256, 72, [128] * 200)])
+@pytest.mark.parametrize("form", ["gelu", "gated", "scattered", "weight_first"])
+def test_grouped_product_in_both_tile_forms(form, N, K, counts):
+    """Rows sorted by group in runs of whole 128-row tiles, groups without rows, tiles behind the last run, more units than
+    SMs (several tiles a CTA) and fewer, columns that fill no tile: against float64 from the same bfloat16 numbers.  K
+    products are added in float32 and the result is rounded to bfloat16 once: half a unit of 8 bits, at most 2^-8 of the value."""
+    from aien_sovereign_core_mv_b200 import kernels as K_
+    if form == "gated" and N % 16:
+        pytest.skip("gate and up rows come in runs of 8")
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    E, used = len(counts), [(c + 127) // 128 for c in counts]
+    tiles = (sum(counts) + 127) // 128 + E
+    rows = tiles * 128
+    a = torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(E, N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    group = [e for e in range(E) for _ in range(used[e])]
+    tile_group = torch.tensor(group + [-1] * (tiles - len(group)), dtype=torch.int32, device="cuda")
+    live = torch.cat([torch.arange(128 * sum(used[:e]), 128 * sum(used[:e]) + counts[e]) for e in range(E)]).cuda()
+    scale = torch.rand(rows, generator=g, device="cuda") + 0.5
+    dest = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    dest[live] = torch.randperm(live.numel(), generator=g, device="cuda").to(torch.int32)
+    cols = N // 2 if form == "gated" else N
+    out = torch.full((live.numel() if form == "scattered" else rows, cols), 7.0, dtype=torch.bfloat16, device="cuda")
+    epi = {"gelu": 2, "gated": 1, "scattered": 0, "weight_first": 3}[form]
+    rc = K_.lib().aien_gemm_tc_grouped(a.data_ptr(), K, w.data_ptr(), K, E, out.data_ptr(), K_.BF16, cols, tile_group.data_ptr(), tiles,
+                                       dest.data_ptr() if form == "scattered" else 0, scale.data_ptr() if form in ("scattered", "weight_first") else 0,
+                                       N, K, epi, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and K_.gemm_tc_error() == 0
+    of = torch.tensor(group, device="cuda").repeat_interleave(128)
+    for e in range(E):
+        r = live[of[live] == e]
+        if r.numel() == 0:
+            continue
+        z = a[r].double() @ w[e].double().T
+        if form == "gelu":
+            z = torch.nn.functional.gelu(z)
+        elif form == "gated":
+            z = z.view(-1, N // 16, 2, 8)
+            z = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).flatten(1)
+        elif form == "scattered":
+            z = z * scale[r, None].double()
+        else:
+            z = torch.nn.functional.gelu(z * scale[r, None].double(), approximate="tanh")
+        got = out[dest[r].long()] if form == "scattered" else out[r]
+        H.assert_close(got.float().cpu().numpy(), z.cpu().numpy(), 4.2e-3, f"group {e}")
