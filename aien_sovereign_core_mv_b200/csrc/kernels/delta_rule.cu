@@ -19,6 +19,7 @@
 // grouped_gated_rmsnorm: out = o / sqrt(mean_group(o^2) + eps) * w[c mod group] * act(gate), the norm taken over
 // every group of `group` neighbouring columns (one head) with one weight vector shared by the groups.
 #include "common.cuh"
+#include "gated_rows.cuh"
 #include <math.h>
 
 namespace aien {
@@ -229,6 +230,44 @@ grouped_gated_rmsnorm_kernel(const float* __restrict__ o, long ldo, const TP* __
     }
 }
 
+// The same with four neighbouring numbers a lane, read once: groups of up to 256 numbers, multiples of 4, rows that
+// four-number accesses take.  2,048 tokens, 16 groups of 128 (42 MB), B200: 21 us a number at a time, 12 so.
+template <typename TP, typename TO>
+__global__ void __launch_bounds__(256)
+grouped_gated_rmsnorm_vec_kernel(const float* __restrict__ o, long ldo, const TP* __restrict__ gate, long ldg, const void* __restrict__ w,
+                                 int wdt, float eps, TO* __restrict__ out, long ldout, int T, int groups, int group, int act) {
+    const size_t unit = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= (size_t)T * groups) return;
+    const int lane = threadIdx.x & 31;
+    const size_t t = unit / groups;
+    const int c0 = (int)(unit - t * groups) * group;
+    float v[2][4], z[2][4];
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int d = (lane + 32 * k) * 4;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (d < group) {
+            a = ld_act4(o + t * ldo + c0 + d);
+            b = ld_act4(gate + t * ldg + c0 + d);
+        }
+        v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+        z[k][0] = b.x; z[k][1] = b.y; z[k][2] = b.z; z[k][3] = b.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss = fmaf(v[k][e], v[k][e], ss);
+    }
+    const float scale = 1.0f / sqrtf(warp_sum(ss) / (float)group + eps);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int d = (lane + 32 * k) * 4;
+        if (d >= group) break;
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = v[k][e] * scale * load_dyn(w, wdt, d + e) * gate_act(z[k][e], act);
+        store4(out + t * ldout + c0 + d, y);
+    }
+}
+
 }  // namespace aien
 
 using namespace aien;
@@ -270,6 +309,14 @@ AIEN_API int aien_grouped_gated_rmsnorm(const float* o, long ldo, const void* ga
     if (groups <= 0 || group <= 0) return AIEN_E_SHAPE;
     const size_t units = (size_t)T * groups;
     const unsigned blocks = (unsigned)((units + 7) / 8);
+    const bool four = group % 4 == 0 && group <= 256 && ((ldo | ldg | ldout) & 3) == 0 && (reinterpret_cast<uintptr_t>(o) & 15) == 0 &&
+                      reinterpret_cast<uintptr_t>(gate) % (g_dt == AIEN_DT_F32 ? 16 : 8) == 0 && reinterpret_cast<uintptr_t>(out) % (o_dt == AIEN_DT_F32 ? 16 : 8) == 0;
+    if (four) {
+        AIEN_DISPATCH_DTYPE(g_dt, TP, AIEN_DISPATCH_DTYPE(o_dt, TO,
+            (grouped_gated_rmsnorm_vec_kernel<TP, TO><<<blocks, 256, 0, stream>>>(o, ldo, (const TP*)gate, ldg, w, w_dt, eps, (TO*)out, ldout, T,
+                                                                                 groups, group, act))));
+        return launch_status();
+    }
     AIEN_DISPATCH_DTYPE(g_dt, TP, AIEN_DISPATCH_DTYPE(o_dt, TO,
         (grouped_gated_rmsnorm_kernel<TP, TO><<<blocks, 256, 0, stream>>>(o, ldo, (const TP*)gate, ldg, w, w_dt, eps, (TO*)out, ldout, T,
                                                                          groups, group, act))));

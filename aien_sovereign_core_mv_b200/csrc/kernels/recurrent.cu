@@ -8,6 +8,7 @@
 // position 0 starts from a zero state whatever the slot held.  A launch depends on the number of
 // requests and on the sizes only, so a step can be captured or recorded.
 #include "common.cuh"
+#include "gated_rows.cuh"
 #include <math.h>
 
 namespace aien {
@@ -628,7 +629,10 @@ AIEN_API int aien_gated_rmsnorm(const float* o, long ldo, const void* gate, int 
     if (T <= 0) return 0;
     if (N <= 0) return AIEN_E_SHAPE;
     AIEN_DISPATCH_DTYPE(g_dt, TP, AIEN_DISPATCH_DTYPE(o_dt, TO,
-        (gated_rmsnorm_kernel<TP, TO><<<T, 256, 0, stream>>>(o, ldo, (const TP*)gate, ldg, w, w_dt, eps, (TO*)out, ldout, N))));
+        if (gated_rows_take(o, ldo, (const TP*)gate, ldg, (const TO*)out, ldout, N))
+            launch_gated_rows<false>(o, ldo, (const TP*)gate, ldg, w, w_dt, eps, 1.0f, (TO*)out, ldout, T, 1, N, stream);
+        else
+            (gated_rmsnorm_kernel<TP, TO><<<T, 256, 0, stream>>>(o, ldo, (const TP*)gate, ldg, w, w_dt, eps, (TO*)out, ldout, N))));
     return launch_status();
 }
 

@@ -21,6 +21,7 @@
 // state and records the product of its decays and its end state; the segments' starting states then follow one from
 // another; a second pass repeats the segment from its true starting state and writes the results.
 #include "common.cuh"
+#include "gated_rows.cuh"
 #include <math.h>
 
 namespace aien {
@@ -590,7 +591,11 @@ AIEN_API int aien_gate_group_norm(const float* y, long ldy, const float* z, long
                                   void* out, int o_dt, long ldo, int T, int width, int groups, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (groups <= 0 || width <= 0 || width % groups || groups > 65535) return AIEN_E_SHAPE;
+    const int part = width / groups;
     AIEN_DISPATCH_DTYPE(o_dt, TO,
-        (gate_group_norm_kernel<TO><<<dim3(T, groups), 256, 0, stream>>>(y, ldy, z, ldz, w, w_dt, eps, mult, (TO*)out, ldo, width / groups)));
+        if (gated_rows_take(y, ldy, z, ldz, (const TO*)out, ldo, part))
+            launch_gated_rows<true>(y, ldy, z, ldz, w, w_dt, eps, mult, (TO*)out, ldo, T, groups, part, stream);
+        else
+            (gate_group_norm_kernel<TO><<<dim3(T, groups), 256, 0, stream>>>(y, ldy, z, ldz, w, w_dt, eps, mult, (TO*)out, ldo, part)));
     return launch_status();
 }

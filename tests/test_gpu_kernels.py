@@ -1250,3 +1250,56 @@ def test_grouped_product_in_both_tile_forms(form, N, K, counts):
             z = torch.nn.functional.gelu(z * scale[r, None].double(), approximate="tanh")
         got = out[dest[r].long()] if form == "scattered" else out[r]
         H.assert_close(got.float().cpu().numpy(), z.cpu().numpy(), 4.2e-3, f"group {e}")
+
+
+@pytest.mark.parametrize("T,H,parts,dtype", [(3, 1024, 6, torch.bfloat16), (130, 260, 5, torch.float32), (2, 4, 1, torch.bfloat16)])
+def test_routed_combine_four_channels_at_a_time_is_the_same(T, H, parts, dtype):
+    """Rows that four-channel accesses take against the same rows where they may not (an odd distance between the parts):
+    the additions come in the same order, so the bits agree."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(T + H)
+    p, sh = torch.randn(parts, T, H, generator=g).to(dtype).cuda(), torch.randn(T, H, generator=g).to(dtype).cuda()
+    h, w, zs = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda(), torch.rand(T, generator=g).cuda(), torch.randn(T, 3, generator=g).cuda()
+    store = torch.zeros(parts * T * H + parts, dtype=dtype).cuda()
+    odd = store.as_strided((parts, T, H), (T * H + 1, H, 1))
+    odd.copy_(p)
+    for gate in (zs[:, 1], None):
+        for same in (w, None):
+            got = []
+            for src, stride in ((p, T * H), (odd, T * H + 1)):
+                out = torch.zeros(T, H).cuda()
+                rc = K.lib().aien_routed_combine(src.data_ptr(), K.dt(src), parts, stride, h.data_ptr() if same is not None else 0, K.BF16, H,
+                                                 same.data_ptr() if same is not None else 0, sh.data_ptr(), K.dt(sh), 1, 0,
+                                                 gate.data_ptr() if gate is not None else 0, 3, out.data_ptr(), T, H, torch.cuda.current_stream().cuda_stream)
+                assert rc == 0
+                got.append(out)
+            assert torch.equal(*got) and float(got[0].abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("form", ["gate_group_norm", "gated_rmsnorm", "grouped_gated_rmsnorm"])
+@pytest.mark.parametrize("T,groups,part,dtype", [(5, 1, 2048, torch.bfloat16), (3, 2, 1028, torch.float32), (2, 1, 4096, torch.bfloat16), (7, 3, 256, torch.float32),
+                                                 (9, 5, 64, torch.bfloat16), (4, 2, 132, torch.float32)])
+def test_gated_norms_of_rows_that_wide_loads_take(form, T, groups, part, dtype):
+    """Parts of one to four groups of numbers a thread, against 64 bits: a mean of `part` float32 squares, and for bfloat16
+    results half a unit of 8 bits (2^-8)."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(part + groups)
+    if form == "gated_rmsnorm":
+        groups, part = 1, groups * part
+    N = groups * part
+    o, z = torch.randn(T, N + 4, generator=g).cuda()[:, 4:], torch.randn(T, N + 8, generator=g).cuda()[:, :N]
+    w = (torch.rand(part if form == "grouped_gated_rmsnorm" else N, generator=g) + 0.5).cuda()
+    out = torch.zeros(T, N + 4, dtype=dtype).cuda()
+    od, zd, wd = o.double().view(T, groups, part), z.double().view(T, groups, part), w.double().view(-1, part)
+    rms = lambda v: v / torch.sqrt(v.square().mean(-1, keepdim=True) + 1e-5)
+    if form == "gate_group_norm":
+        K.gate_group_norm(o, z, w, 1e-5, 0.7, out[:, :N], groups)
+        want = rms(od * zd * torch.sigmoid(zd)) * wd * 0.7
+    elif form == "gated_rmsnorm":
+        K.gated_rmsnorm(o, z, w, 1e-5, out[:, :N])
+        want = rms(od) * wd * torch.sigmoid(zd)
+    else:
+        K.grouped_gated_rmsnorm(o, z, w, 1e-5, out[:, :N], part, "silu")
+        want = rms(od) * wd * zd * torch.sigmoid(zd)
+    H.assert_close(out[:, :N].float().cpu().numpy(), want.view(T, N).cpu().numpy(), 4.2e-3 if dtype == torch.bfloat16 else 3e-6, form)
+    assert float(out[:, N:].float().abs().max()) == 0.0
