@@ -1303,3 +1303,25 @@ def test_gated_norms_of_rows_that_wide_loads_take(form, T, groups, part, dtype):
         want = rms(od) * wd * zd * torch.sigmoid(zd)
     H.assert_close(out[:, :N].float().cpu().numpy(), want.view(T, N).cpu().numpy(), 4.2e-3 if dtype == torch.bfloat16 else 3e-6, form)
     assert float(out[:, N:].float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("M,N,Kd,splits", [(2085, 2052, 128, 1), (4100, 4108, 192, 1), (130, 300, 1024, 2), (333, 1026, 512, 3), (70, 256, 64, 1), (2048, 8192, 64, 1)])
+def test_float32_results_stored_in_boxes_are_the_same(K, M, N, Kd, splits):
+    """Results that leave by TMA (rows on 16-byte boundaries) against the same product stored from registers (one number
+    further on): the sums are the same, so are the bits; rows, columns and parts beyond the result stay as they were."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, Kd, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, Kd, generator=g, device="cuda").to(torch.bfloat16)
+    parts = K.gemm_tc_ranges(Kd, splits)
+    ld = N + 8 - N % 4 if parts == 1 else N                       # partial products are contiguous
+    got = []
+    for at in (4, 5):
+        store = torch.full((at + (parts * M + 2) * ld + 8,), 7.0, device="cuda")
+        out = store.as_strided((parts, M, N), (M * ld, ld, 1), at)
+        K.gemm_tc(a, w, out if parts > 1 else out[0])
+        got.append(out.clone())
+        out.fill_(7.0)
+        assert float((store - 7.0).abs().max()) == 0.0
+    assert torch.equal(*got) and K.gemm_tc_error() == 0
+    want = a.double() @ w.double().T
+    assert float((got[0].double().sum(0) - want).abs().max()) <= Kd * 2.0 ** -22 * float((a.double().abs() @ w.double().abs().T).max())
