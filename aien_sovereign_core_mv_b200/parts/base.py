@@ -156,7 +156,6 @@ class Workspace:
         self.step_bytes = (int(step_bytes) + 255) & ~255
         self.layer_bytes = (int(layer_bytes) + 255) & ~255
         self.buf = torch.empty(self.step_bytes + 2 * self.layer_bytes, dtype=torch.uint8, device=device)
-        self._typed: Dict[torch.dtype, torch.Tensor] = {}
         self._base = [0, self.step_bytes, self.step_bytes + self.layer_bytes]
         self._size = [self.step_bytes, self.layer_bytes, self.layer_bytes]
         self._off = [0, 0, 0]
@@ -175,25 +174,19 @@ class Workspace:
         self.begin_layer()
 
     def _take(self, region: int, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
-        n, strides = 1, []
-        for s in reversed(shape):
-            strides.append(n)
+        n = 1
+        for s in shape:
             n *= int(s)
-        size = _ELEMENT_SIZE[dtype]
+        nbytes = n * _ELEMENT_SIZE[dtype]
         start = (self._off[region] + 255) & ~255
-        end = start + n * size
-        if end > self._size[region]:
+        if start + nbytes > self._size[region]:
             which = "step" if region == 0 else "layer"
             raise RuntimeError(
-                f"{which} workspace too small: need {end} bytes, have {self._size[region]} "
+                f"{which} workspace too small: need {start + nbytes} bytes, have {self._size[region]} "
                 f"(the step brings more tokens than max_batch_tokens allows)")
-        self._off[region] = end
-        # one call on a view of the whole buffer in this type, not a slice, a change of type and a change of shape
-        whole = self._typed.get(dtype)
-        if whole is None:
-            whole = self._typed[dtype] = self.buf.view(dtype)
-        strides.reverse()
-        return whole.as_strided(shape, strides, (self._base[region] + start) // size)
+        self._off[region] = start + nbytes
+        lo = self._base[region] + start
+        return self.buf[lo:lo + nbytes].view(dtype).view(*shape)
 
     def take(self, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         return self._take(self._cur, shape, dtype)
