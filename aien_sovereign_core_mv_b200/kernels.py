@@ -73,13 +73,14 @@ class _Library:
         return wrapped
 
 
-def lib() -> "_Library":
+def lib():
+    """The loaded library; while launches are being written down, with its launching entry points wrapped."""
     global _lib, _proxy
     if _proxy is None:
         _lib = _build.load_kernels()
         _declare(_lib)
         _proxy = _Library(_lib)
-    return _proxy
+    return _lib if _RECORD is None else _proxy
 
 
 def begin_recording() -> None:
@@ -779,6 +780,32 @@ def gemv_takes_activation(K_: int) -> bool:
 def gemv_stream_error() -> int:
     """Error code left by a bounded wait inside the streamed decode product (0: none); clears it."""
     return int(lib().aien_gemv_stream_error())
+
+
+def product_operands(a: torch.Tensor, w: torch.Tensor) -> Optional[tuple]:
+    """(M, N, K, a's address and row stride, w's address and row stride) of a product that the bfloat16 kernels take (what
+    :func:`gemm_tc_supports` and :func:`gemv_supports` ask of the operands), looked up once for the launch; None: they do not."""
+    if a.dtype is not torch.bfloat16 or w.dtype is not torch.bfloat16:
+        return None
+    (M, K_), (lda, ia), (ldw, iw) = a.shape, a.stride(), w.stride()
+    pa, pw = a.data_ptr(), w.data_ptr()
+    if ia != 1 or iw != 1 or (lda | ldw | K_) & 7 or (pa | pw) & 15 or w.shape[1] != K_:
+        return None
+    return M, w.shape[0], K_, pa, lda, pw, ldw
+
+
+def launch_product(ops: tuple, out: torch.Tensor, few: bool, epilogue: int = 0) -> None:
+    """The product of :func:`product_operands` into ``out``: [M, columns], or [P, M, N] float32 for P partial products over
+    ranges of K.  ``few``: by the streamed decode kernels (:func:`gemv`), else on the tensor cores (:func:`gemm_tc`); the
+    epilogues are theirs."""
+    M, N, K_, pa, lda, pw, ldw = ops
+    splits, part_stride = (out.shape[0], M * N) if out.dim() == 3 else (1, 0)
+    if few:
+        fn = lib().aien_gemv_stream_bf16 if (GEMV_IMPL == "stream" and K_ % 64 == 0) else lib().aien_gemv_bf16
+    else:
+        fn = lib().aien_gemm_tc
+    _check(fn(pa, lda, pw, ldw, out.data_ptr(), _DT[out.dtype], out.stride(-2), M, N, K_, epilogue, splits, part_stride, _stream()),
+           "gemv_bf16" if few else "gemm_tc")
 
 
 def gemm_tc_supports(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:

@@ -143,6 +143,20 @@ class StepLimits:
 _ELEMENT_SIZE = {torch.float32: 4, torch.bfloat16: 2, torch.float16: 2, torch.int32: 4, torch.int64: 8, torch.uint8: 1, torch.float64: 8}
 
 
+_LAYOUTS: Dict[tuple, Tuple[int, tuple]] = {}          # shape -> (numbers, strides), of the shapes asked for lately
+
+
+def _layout_of(shape) -> Tuple[int, tuple]:
+    n, strides = 1, []
+    for s in reversed(shape):
+        strides.append(n)
+        n *= int(s)
+    if len(_LAYOUTS) >= 4096:
+        _LAYOUTS.clear()
+    _LAYOUTS[tuple(shape)] = out = (n, tuple(reversed(strides)))
+    return out
+
+
 class Workspace:
     """Scratch for one step, carved from one device buffer so that a step allocates nothing
     and its addresses repeat (which a captured CUDA graph needs).
@@ -156,6 +170,7 @@ class Workspace:
         self.step_bytes = (int(step_bytes) + 255) & ~255
         self.layer_bytes = (int(layer_bytes) + 255) & ~255
         self.buf = torch.empty(self.step_bytes + 2 * self.layer_bytes, dtype=torch.uint8, device=device)
+        self._typed: Dict[torch.dtype, torch.Tensor] = {}
         self._base = [0, self.step_bytes, self.step_bytes + self.layer_bytes]
         self._size = [self.step_bytes, self.layer_bytes, self.layer_bytes]
         self._off = [0, 0, 0]
@@ -174,19 +189,25 @@ class Workspace:
         self.begin_layer()
 
     def _take(self, region: int, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
-        n = 1
-        for s in shape:
-            n *= int(s)
-        nbytes = n * _ELEMENT_SIZE[dtype]
+        if type(shape) is not tuple:
+            shape = tuple(shape)
+        layout = _LAYOUTS.get(shape)
+        if layout is None:
+            layout = _layout_of(shape)
+        size = _ELEMENT_SIZE[dtype]
         start = (self._off[region] + 255) & ~255
-        if start + nbytes > self._size[region]:
+        end = start + layout[0] * size
+        if end > self._size[region]:
             which = "step" if region == 0 else "layer"
             raise RuntimeError(
-                f"{which} workspace too small: need {start + nbytes} bytes, have {self._size[region]} "
+                f"{which} workspace too small: need {end} bytes, have {self._size[region]} "
                 f"(the step brings more tokens than max_batch_tokens allows)")
-        self._off[region] = start + nbytes
-        lo = self._base[region] + start
-        return self.buf[lo:lo + nbytes].view(dtype).view(*shape)
+        self._off[region] = end
+        # one call on a view of the whole buffer in this type, not a slice, a change of type and a change of shape
+        whole = self._typed.get(dtype)
+        if whole is None:
+            whole = self._typed[dtype] = self.buf.view(dtype)
+        return whole.as_strided(shape, layout[1], (self._base[region] + start) // size)
 
     def take(self, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         return self._take(self._cur, shape, dtype)

@@ -29,31 +29,45 @@ def linear(ctx: StepContext, a: torch.Tensor, w: torch.Tensor, out_dtype: Option
     ``may_defer_sum``: the caller's consumer can add partial products, so the decode kernel may
     cut K across CTAs and return float32 partials [P, M, N] instead (the norm kernel, the q/k
     kernel and the row gather add them in order)."""
+    if _FORCE:
+        return _pinned(ctx, a, w, out_dtype, out, act)
     M, N = a.shape[0], w.shape[0]
-    if out is None and may_defer_sum and not _FORCE and M <= K.GEMV_ROUTE_ROWS and a.dtype == torch.bfloat16 \
-            and w.dtype == torch.bfloat16:
-        splits = K.gemv_splits(N, a.shape[1])
+    ops = K.product_operands(a, w)
+    few = ops is not None and M <= K.GEMV_ROUTE_ROWS
+    if ops is not None and out is None and may_defer_sum:
+        splits = K.gemv_splits(N, ops[2]) if few else K.gemm_tc_splits(M, N, ops[2])
         if splits > 1:
             parts = ctx.workspace.take((splits, M, N), torch.float32)
-            if K.gemv_supports(a, w, parts):
-                K.gemv(a, w, parts)
-                return parts
-    if out is None and may_defer_sum and not _FORCE and M > K.GEMV_ROUTE_ROWS and a.dtype == torch.bfloat16 \
-            and w.dtype == torch.bfloat16:
-        splits = K.gemm_tc_splits(M, N, a.shape[1])
-        if splits > 1:
-            parts = ctx.workspace.take((splits, M, N), torch.float32)
-            if K.gemm_tc_supports(a, w, parts[0]):
-                K.gemm_tc(a, w, parts)
-                return parts
+            K._dev(a, w, parts)
+            K.launch_product(ops, parts, few)
+            return parts
     if out is None:
         out = ctx.workspace.take((M, N), out_dtype or a.dtype)
-    choice = _FORCE or _choose(a, w, out, M)
+    else:
+        assert tuple(out.shape) == (M, N)
+    fused = False
+    if ops is not None and out.stride(-1) == 1 and (few or out.dtype in (torch.bfloat16, torch.float32)):
+        if act is not None:
+            fused = act in K.ACT_IN_PRODUCT and out.dtype == torch.bfloat16 and out.is_contiguous() and (not few or K.gemv_takes_activation(ops[2]))
+        K._dev(a, w, out)
+        K.launch_product(ops, out, few, (act + (3 if few else 2)) if fused else 0)
+    else:
+        K.gemm_simple(a, w, out)
+    if act is not None and not fused:
+        K.act_rows(out, act)
+    return out
+
+
+def _pinned(ctx: StepContext, a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype], out: Optional[torch.Tensor],
+            act: Optional[int]) -> torch.Tensor:
+    """linear() with the kernel that ``AIEN_B200_GEMM`` names, without partial products."""
+    if out is None:
+        out = ctx.workspace.take((a.shape[0], w.shape[0]), out_dtype or a.dtype)
     fused = act is not None and act in K.ACT_IN_PRODUCT and out.dtype == torch.bfloat16 and out.is_contiguous()
-    if choice == "gemv":
+    if _FORCE == "gemv":
         fused = fused and K.gemv_takes_activation(a.shape[1])
         K.gemv(a, w, out, epilogue=3 + act if fused else 0)
-    elif choice == "tc":
+    elif _FORCE == "tc":
         K.gemm_tc(a, w, out, epilogue=2 + act if fused else 0)
     else:
         fused = False
@@ -72,16 +86,6 @@ def stack_rows(rows, multiple: int = 1) -> torch.Tensor:
     if pad:
         rows = list(rows) + [rows[0].new_zeros((pad, rows[0].shape[1]))]
     return torch.cat(list(rows), dim=0).contiguous()
-
-
-def _choose(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int) -> str:
-    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
-        return "simple"
-    if M <= K.GEMV_ROUTE_ROWS and K.gemv_supports(a, w, out):
-        return "gemv"
-    if K.gemm_tc_supports(a, w, out):
-        return "tc"
-    return "simple"
 
 
 def linear_prenormed(ctx: StepContext, h: Prenormed, w: torch.Tensor, epilogue: int = 0) -> Optional[torch.Tensor]:
