@@ -21,7 +21,7 @@
 // the left operand once the rows of a fragment are counted 0 2 4 6 1 3 5 7 on both sides.  The update is accumulated from
 // zero and added to the decayed state by one float32 multiply-add, so the state is rounded once per block.
 //
-// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 186 us and 16 for the coefficients (603 token by
+// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 153 us and 16 for the coefficients (603 token by
 // token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 113 and 6 us (540).
 #include "common.cuh"
 #include <math.h>
@@ -193,20 +193,23 @@ block_coef_kernel(const BlockWalk a) {
 }
 
 // NT: fragments of 8 rows that a warp owns; N <= 64 NT.
-template <int NT>
+// HELP: with helper warps (see block_walk_kernel).
+template <int NT, bool HELP>
 struct BwSmem {
+    static constexpr int STAGES = HELP ? 3 : 2, TURNS = HELP ? 2 : 1;                      // sums of r and u for so many blocks
     static constexpr int LDN = 64 * NT + 8;                     // floats between rows of q and k: a half warp's 8-byte reads meet no bank twice
     static constexpr int QK = BW_B * LDN;
     static constexpr int STAGE = 2 * QK + BW_B * BW_LDV + 2 * BW_B * BW_LD + 2 * BW_B;     // q | k | v | A | M | G | G_16 / G_j
     static constexpr int PART = BW_WARPS * BW_B * BW_LD;
-    static constexpr int TOTAL = 2 * STAGE + 2 * PART + BW_B * BW_LDV;                     // two stages, partial sums of p and r, u
+    static constexpr int U = BW_B * BW_LDV;
+    static constexpr int TOTAL = STAGES * STAGE + (1 + TURNS) * PART + TURNS * U;          // partial sums of p, and of r, and u
 };
 
-template <int NT, bool DELTA>
+template <int NT, bool DELTA, bool HELP>
 __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWalk& a, const float* rows, long ld, int q_col, int k_col, int v_col,
-                                         int cols, const float* coef, int t, int t1) {
-    using C = BwSmem<NT>;
-    const int tid = threadIdx.x, pieces = 16 * NT;              // 16-byte pieces of a padded row
+                                         int cols, const float* coef, int t, int t1, int tid) {
+    using C = BwSmem<NT, HELP>;
+    constexpr int pieces = 16 * NT;                             // 16-byte pieces of a padded row
 #pragma unroll
     for (int i = tid; i < BW_B * pieces; i += BW_THREADS) {
         const int tok = i / pieces, c = i % pieces * 4;
@@ -236,7 +239,7 @@ __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWal
 template <int NT>
 __device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const uint32_t (&sh)[NT][4], const uint32_t (&sl)[NT][4],
                                             float* __restrict__ part, int row0, int g, int t) {
-    using C = BwSmem<NT>;
+    using C = BwSmem<NT, false>;
     float acc[2][4] = {};
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
@@ -265,27 +268,94 @@ __device__ __forceinline__ float bw_sum_parts(const float* __restrict__ part, in
     return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
 }
 
-template <int NT, bool DELTA>
-__global__ void __launch_bounds__(BW_THREADS)
+// Barriers of part of a CTA: `sync` waits, `arrive` does not.
+__device__ __forceinline__ void bw_sync(int id, int threads) { asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bw_arrive(int id, int threads) { asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+constexpr int BW_BAR_STATE = 1, BW_BAR_FULL = 2, BW_BAR_DONE = 5;              // FULL + stage, DONE + block & 1
+
+// Eight warps hold the state, bring the blocks and make the results.  With HELP eight more bring the blocks and turn a
+// block's partial sums into results while the state warps, which then do only what the next block waits for, are at the next
+// one.  A helper passes DONE of block i before it refills the stage of block i - 1 (whose update came before) with block
+// i + 2, makes block i's results and then reports block i + 2 FULL, so the state warps write block i + 2's sums over block
+// i's only after these were read.  That shortens the delta rule's long chain where a CTA has its SM to itself (185 -> 153 us
+// for 2,048 tokens of 16 heads); with two CTAs on an SM, and without the delta rule, the extra warps only get in the
+// way (linear attention, 1,900 tokens of two requests: 88 -> 107 us).
+template <int NT, bool DELTA, bool HELP>
+__global__ void __launch_bounds__((HELP ? 2 : 1) * BW_THREADS)
 block_walk_kernel(const BlockWalk a) {
-    using C = BwSmem<NT>;
+    using C = BwSmem<NT, HELP>;
     extern __shared__ __align__(16) float bw_smem[];
-    float* part_p = bw_smem + 2 * C::STAGE;
-    float* part_r = part_p + C::PART;
-    float* su = part_r + C::PART;
+    float* part_p = bw_smem + C::STAGES * C::STAGE;
+    float* parts_r = part_p + C::PART;
+    float* us = parts_r + C::TURNS * C::PART;
     const int s = blockIdx.z, h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
     if (t1 <= t0) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
-    const int col0 = blockIdx.x * BW_COLS, cols = a.V - col0 < BW_COLS ? a.V - col0 : BW_COLS, row0 = warp * 8 * NT;
+    const int tid = threadIdx.x & (BW_THREADS - 1), warp = tid >> 5, lane = tid & 31;
+    const int col0 = blockIdx.x * BW_COLS, cols = a.V - col0 < BW_COLS ? a.V - col0 : BW_COLS;
+
     const float* rows = a.act ? a.act_rows : a.rows;
     const long ld = a.act ? a.ld_act : a.ld;
     const int q_col = (a.act ? 0 : a.q_off) + kvh * a.N, k_col = (a.act ? a.G * a.N : a.k_off) + kvh * a.N;
     const int v_col = (a.act ? 2 * a.G * a.N : a.v_off) + h * a.V + col0;
     const float* coef = a.coef + ((size_t)bw_first_block(a.q_start, s) * a.heads + h) * BW_COEF;
     const size_t coef_step = (size_t)a.heads * BW_COEF;
-    bw_fetch<NT, DELTA>(bw_smem, a, rows, ld, q_col, k_col, v_col, cols, coef, t0, t1);
+    auto fetch = [&](int t, int stage) {                        // the next block in order, which starts at token t
+        bw_fetch<NT, DELTA, HELP>(bw_smem + stage * C::STAGE, a, rows, ld, q_col, k_col, v_col, cols, coef, t, t1, tid);
+        coef += coef_step;
+    };
+    const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
+    auto results = [&](int t, int stage, int turn) {            // thread = column tid % 16 of token tid / 16
+        const int col = tid & 15, tok = tid >> 4;
+        const float* sv = bw_smem + stage * C::STAGE + 2 * C::QK;
+        const float* sA = sv + BW_B * BW_LDV;
+        const float* gam = sA + 2 * BW_B * BW_LD;
+        const float* u = DELTA ? us + turn * C::U : sv;
+        const float4* a4 = reinterpret_cast<const float4*>(sA + tok * BW_LD);
+        float o0 = gam[tok] * bw_sum_parts(parts_r + turn * C::PART, tok, col), o1 = skip * sv[tok * BW_LDV + col];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 m = a4[j];
+            o0 = fmaf(m.x, u[(4 * j) * BW_LDV + col], o0);
+            o1 = fmaf(m.y, u[(4 * j + 1) * BW_LDV + col], o1);
+            o0 = fmaf(m.z, u[(4 * j + 2) * BW_LDV + col], o0);
+            o1 = fmaf(m.w, u[(4 * j + 3) * BW_LDV + col], o1);
+        }
+        if (t + tok < t1 && col < cols) a.out[(size_t)(t + tok) * a.ldo + (size_t)h * a.V + col0 + col] = o0 + o1;
+    };
 
-    // the state: thread (g, tq) of a warp holds columns g and g + 8, rows 2 tq and 2 tq + 1 of every fragment
+    if (HELP && threadIdx.x >= BW_THREADS) {
+        const bool more = t0 + BW_B < t1;
+        fetch(t0, 0);
+        if (more) {
+            fetch(t0 + BW_B, 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        bw_arrive(BW_BAR_FULL, 2 * BW_THREADS);
+        if (more) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            bw_arrive(BW_BAR_FULL + 1, 2 * BW_THREADS);
+        }
+        int b = 0, turn = 0;
+        for (int t = t0; t < t1; t += BW_B, turn ^= 1) {
+            const int ahead = b == 0 ? 2 : b - 1;               // the stage of the block before, for the one two blocks on
+            bw_sync(BW_BAR_DONE + turn, 2 * BW_THREADS);
+            if (t + 2 * BW_B < t1) fetch(t + 2 * BW_B, ahead);
+            results(t, b, turn);
+            if (t + 2 * BW_B < t1) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                bw_arrive(BW_BAR_FULL + ahead, 2 * BW_THREADS);
+            }
+            b = b == 2 ? 0 : b + 1;
+        }
+        return;
+    }
+
+    // ---------------------------------------------------------------------- the state
+    // thread (g, tq) of a warp holds columns g and g + 8, rows 2 tq and 2 tq + 1 of every fragment
+    if (!HELP) fetch(t0, 0);
+    const int g = lane >> 2, tq = lane & 3, row0 = warp * 8 * NT;
     float* st = a.state + (size_t)a.slots[s] * a.state_stride + a.s_off + (size_t)h * a.N * a.V;
     const long sr = a.state_vn ? 1 : a.V, sc = a.state_vn ? a.N : 1;
     const bool fresh = a.positions[t0] == 0;
@@ -297,19 +367,19 @@ block_walk_kernel(const BlockWalk a) {
             const int row = row0 + nt * 8 + 2 * tq + (e & 1), col = g + (e >> 1) * 8;
             S[nt][e] = (!fresh && row < a.N && col < cols) ? st[row * sr + (col0 + col) * sc] : 0.f;
         }
-    const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
-
-    int b = 0;
-    for (int t = t0; t < t1; t += BW_B, b ^= 1) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                                        // the block's rows are here, and everyone has left the block before
-        coef += coef_step;
-        if (t + BW_B < t1) bw_fetch<NT, DELTA>(bw_smem + (b ^ 1) * C::STAGE, a, rows, ld, q_col, k_col, v_col, cols, coef, t + BW_B, t1);
+    int b = 0, turn = 0;
+    for (int t = t0; t < t1; t += BW_B) {
+        if (HELP) {
+            bw_sync(BW_BAR_FULL + b, 2 * BW_THREADS);
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();                                    // the block's rows are here, and everyone has left the block before
+            if (t + BW_B < t1) fetch(t + BW_B, b ^ 1);
+        }
         const float* sq = bw_smem + b * C::STAGE;
         const float* sk = sq + C::QK;
         const float* sv = sk + C::QK;
-        const float* sA = sv + BW_B * BW_LDV;
-        const float* sM = sA + BW_B * BW_LD;
+        const float* sM = sv + BW_B * BW_LDV + BW_B * BW_LD;
         const float* gam = sM + BW_B * BW_LD;
         const float* suf = gam + BW_B;
         uint32_t sh[NT][4], sl[NT][4];
@@ -322,8 +392,9 @@ block_walk_kernel(const BlockWalk a) {
         }
         const float* u = sv;
         if (DELTA) {
+            float* su = us + turn * C::U;
             bw_read_out<NT>(sk, sh, sl, part_p + warp * BW_B * BW_LD, row0, g, tq);
-            __syncthreads();
+            HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();
             // thread: token lane % 16 of column tid / 16; the 16 tokens of a column meet in half a warp
             const int tok = lane & 15, col = tid >> 4;
             const float e = sv[tok * BW_LDV + col] - gam[tok] * bw_sum_parts(part_p, tok, col);
@@ -340,8 +411,9 @@ block_walk_kernel(const BlockWalk a) {
             su[tok * BW_LDV + col] = u0 + u1;
             u = su;
         }
-        bw_read_out<NT>(sq, sh, sl, part_r + warp * BW_B * BW_LD, row0, g, tq);
-        __syncthreads();                                        // u and the partial sums of r are there
+        bw_read_out<NT>(sq, sh, sl, parts_r + turn * C::PART + warp * BW_B * BW_LD, row0, g, tq);
+        HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();     // u and the partial sums of r are there
+        if (HELP) bw_arrive(BW_BAR_DONE + turn, 2 * BW_THREADS);
         float up[NT][4] = {};
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
@@ -360,26 +432,18 @@ block_walk_kernel(const BlockWalk a) {
                 bw_mma3(up[nt], ah, al, bh, bl);
             }
         }
-        {
-            // the results: thread = column tid % 16 of token tid / 16
-            const int col = tid & 15, tok = tid >> 4;
-            const float4* a4 = reinterpret_cast<const float4*>(sA + tok * BW_LD);
-            float o0 = gam[tok] * bw_sum_parts(part_r, tok, col), o1 = skip * sv[tok * BW_LDV + col];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 m = a4[j];
-                o0 = fmaf(m.x, u[(4 * j) * BW_LDV + col], o0);
-                o1 = fmaf(m.y, u[(4 * j + 1) * BW_LDV + col], o1);
-                o0 = fmaf(m.z, u[(4 * j + 2) * BW_LDV + col], o0);
-                o1 = fmaf(m.w, u[(4 * j + 3) * BW_LDV + col], o1);
-            }
-            if (t + tok < t1 && col < cols) a.out[(size_t)(t + tok) * a.ldo + (size_t)h * a.V + col0 + col] = o0 + o1;
-        }
+        if (!HELP) results(t, b, 0);
         const float total = gam[BW_B - 1];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) S[nt][e] = fmaf(total, S[nt][e], up[nt][e]);
+        if (HELP) {
+            b = b == 2 ? 0 : b + 1;
+            turn ^= 1;
+        } else {
+            b ^= 1;
+        }
     }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
@@ -390,13 +454,22 @@ block_walk_kernel(const BlockWalk a) {
         }
 }
 
-template <int NT, bool DELTA>
+template <int NT, bool DELTA, bool HELP>
 static int launch_block_walk(const BlockWalk& a, cudaStream_t stream) {
-    constexpr int bytes = BwSmem<NT>::TOTAL * 4;
-    auto kern = block_walk_kernel<NT, DELTA>;
+    constexpr int bytes = BwSmem<NT, HELP>::TOTAL * 4;
+    auto kern = block_walk_kernel<NT, DELTA, HELP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
-    kern<<<dim3((a.V + BW_COLS - 1) / BW_COLS, a.heads, a.S), BW_THREADS, bytes, stream>>>(a);
+    kern<<<dim3((a.V + BW_COLS - 1) / BW_COLS, a.heads, a.S), (HELP ? 2 : 1) * BW_THREADS, bytes, stream>>>(a);
     return launch_status();
+}
+
+template <int NT>
+static int dispatch_block_walk(const BlockWalk& a, cudaStream_t stream) {
+    if (!a.delta) return launch_block_walk<NT, false, false>(a, stream);
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    const long ctas = (long)((a.V + BW_COLS - 1) / BW_COLS) * a.heads * a.S;
+    return ctas <= sms ? launch_block_walk<NT, true, true>(a, stream) : launch_block_walk<NT, true, false>(a, stream);
 }
 
 }  // namespace aien
@@ -431,6 +504,5 @@ AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, i
     block_coef_kernel<<<dim3((unsigned)blocks, G), 256, smem, stream>>>(a);
     const int rc = launch_status();
     if (rc != 0) return rc;
-    if (N <= 64) return delta ? launch_block_walk<1, true>(a, stream) : launch_block_walk<1, false>(a, stream);
-    return delta ? launch_block_walk<2, true>(a, stream) : launch_block_walk<2, false>(a, stream);
+    return N <= 64 ? dispatch_block_walk<1>(a, stream) : dispatch_block_walk<2>(a, stream);
 }
