@@ -21,19 +21,17 @@
 // the left operand once the rows of a fragment are counted 0 2 4 6 1 3 5 7 on both sides.  The update is accumulated from
 // zero and added to the decayed state by one float32 multiply-add, so the state is rounded once per block.
 //
-// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 153 us and 16 for the coefficients (603 token by
-// token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 113 and 6 us (540).
+// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 148 us and 16 for the coefficients (603 token by
+// token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 110 and 6 us (540).
 #include "common.cuh"
 #include <math.h>
 
 namespace aien {
 
 constexpr int BW_B = 16;                       // tokens of a block
-constexpr int BW_COLS = 16;                    // state columns of a CTA
 constexpr int BW_WARPS = 8;
 constexpr int BW_THREADS = 32 * BW_WARPS;
-constexpr int BW_LD = 20;                      // floats between rows of A, M and of the partial sums: no bank twice in a quarter warp
-constexpr int BW_LDV = 24;                     // floats between rows of v and u
+constexpr int BW_LD = 20;                      // floats between rows of A and M: no bank twice in a quarter warp
 constexpr int BW_COEF = 2 * BW_B * BW_B + 2 * BW_B;      // A | M | G | G_16 / G_j per block and head
 
 __device__ __forceinline__ void bw_split(float x, uint32_t& hi, uint32_t& lo) {
@@ -192,23 +190,24 @@ block_coef_kernel(const BlockWalk a) {
     }
 }
 
-// NT: fragments of 8 rows that a warp owns; N <= 64 NT.
+// NT: fragments of 8 rows that a warp owns; N <= 64 NT.  MT: a CTA has 16 MT columns of the state.
 // HELP: with helper warps (see block_walk_kernel).
-template <int NT, bool HELP>
+template <int NT, int MT, bool HELP>
 struct BwSmem {
     static constexpr int STAGES = HELP ? 3 : 2, TURNS = HELP ? 2 : 1;                      // sums of r and u for so many blocks
     static constexpr int LDN = 64 * NT + 8;                     // floats between rows of q and k: a half warp's 8-byte reads meet no bank twice
+    static constexpr int LDV = 16 * MT + 8, LDP = 16 * MT + 4;  // floats between rows of v and u, and of the partial sums
     static constexpr int QK = BW_B * LDN;
-    static constexpr int STAGE = 2 * QK + BW_B * BW_LDV + 2 * BW_B * BW_LD + 2 * BW_B;     // q | k | v | A | M | G | G_16 / G_j
-    static constexpr int PART = BW_WARPS * BW_B * BW_LD;
-    static constexpr int U = BW_B * BW_LDV;
+    static constexpr int STAGE = 2 * QK + BW_B * LDV + 2 * BW_B * BW_LD + 2 * BW_B;     // q | k | v | A | M | G | G_16 / G_j
+    static constexpr int PART = BW_WARPS * BW_B * LDP;
+    static constexpr int U = BW_B * LDV;
     static constexpr int TOTAL = STAGES * STAGE + (1 + TURNS) * PART + TURNS * U;          // partial sums of p, and of r, and u
 };
 
-template <int NT, bool DELTA, bool HELP>
+template <int NT, int MT, bool DELTA, bool HELP>
 __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWalk& a, const float* rows, long ld, int q_col, int k_col, int v_col,
                                          int cols, const float* coef, int t, int t1, int tid) {
-    using C = BwSmem<NT, HELP>;
+    using C = BwSmem<NT, MT, HELP>;
     constexpr int pieces = 16 * NT;                             // 16-byte pieces of a padded row
 #pragma unroll
     for (int i = tid; i < BW_B * pieces; i += BW_THREADS) {
@@ -218,29 +217,28 @@ __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWal
         bw_cp16(buf + tok * C::LDN + c, r + (in ? q_col : 0), in);
         bw_cp16(buf + C::QK + tok * C::LDN + c, r + (in ? k_col : 0), in);
     }
-    if (tid < 64) {
-        const int tok = tid >> 2, c = (tid & 3) * 4;
+    float* sA = buf + 2 * C::QK + BW_B * C::LDV;
+    if (tid < 64 * MT) {
+        const int tok = tid / (4 * MT), c = tid % (4 * MT) * 4;
         const bool in = t + tok < t1 && c < cols;
-        bw_cp16(buf + 2 * C::QK + tok * BW_LDV + c, in ? rows + (size_t)(t + tok) * ld + v_col + c : rows, in);
-    } else if (tid < 128) {
-        const int e = tid - 64;
-        bw_cp16(buf + 2 * C::QK + BW_B * BW_LDV + (e >> 2) * BW_LD + (e & 3) * 4, coef + e * 4, true);
-    } else if (tid < 192) {
-        const int e = tid - 128;
-        if (DELTA) bw_cp16(buf + 2 * C::QK + BW_B * BW_LDV + BW_B * BW_LD + (e >> 2) * BW_LD + (e & 3) * 4, coef + 256 + e * 4, true);
-    } else if (tid < 200) {
-        const int e = tid - 192;
-        bw_cp16(buf + 2 * C::QK + BW_B * BW_LDV + 2 * BW_B * BW_LD + e * 4, coef + 512 + e * 4, true);
+        bw_cp16(buf + 2 * C::QK + tok * C::LDV + c, in ? rows + (size_t)(t + tok) * ld + v_col + c : rows, in);
+    } else if (tid < 64 * MT + 64) {
+        const int e = tid - 64 * MT;
+        bw_cp16(sA + (e >> 2) * BW_LD + (e & 3) * 4, coef + e * 4, true);
+    } else if (DELTA && tid < 64 * MT + 128) {
+        const int e = tid - 64 * MT - 64;
+        bw_cp16(sA + BW_B * BW_LD + (e >> 2) * BW_LD + (e & 3) * 4, coef + 256 + e * 4, true);
     }
+    if (tid < 8) bw_cp16(sA + 2 * BW_B * BW_LD + tid * 4, coef + 512 + tid * 4, true);
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// partial products S0^T x of a warp's rows, x the q or k rows of a block: [16 columns] x [16 tokens] into part[token][column]
-template <int NT>
-__device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const uint32_t (&sh)[NT][4], const uint32_t (&sl)[NT][4],
+// partial products S0^T x of a warp's rows, x the q or k rows of a block: [16 MT columns] x [16 tokens] into part[token][column]
+template <int NT, int MT>
+__device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const uint32_t (&sh)[MT][NT][4], const uint32_t (&sl)[MT][NT][4],
                                             float* __restrict__ part, int row0, int g, int t) {
-    using C = BwSmem<NT, false>;
-    float acc[2][4] = {};
+    using C = BwSmem<NT, MT, false>;
+    float acc[MT][2][4] = {};
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -249,22 +247,26 @@ __device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const u
             uint32_t bh[2], bl[2];
             bw_split(v.x, bh[0], bl[0]);
             bw_split(v.y, bh[1], bl[1]);
-            bw_mma3(acc[half], sh[nt], sl[nt], bh, bl);
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) bw_mma3(acc[mt][half], sh[mt][nt], sl[mt][nt], bh, bl);
         }
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        float* p = part + (half * 8 + 2 * t) * BW_LD + g;
-        p[0] = acc[half][0];
-        p[BW_LD] = acc[half][1];
-        p[8] = acc[half][2];
-        p[BW_LD + 8] = acc[half][3];
-    }
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float* p = part + (half * 8 + 2 * t) * C::LDP + mt * 16 + g;
+            p[0] = acc[mt][half][0];
+            p[C::LDP] = acc[mt][half][1];
+            p[8] = acc[mt][half][2];
+            p[C::LDP + 8] = acc[mt][half][3];
+        }
 }
 
+template <int LDP>
 __device__ __forceinline__ float bw_sum_parts(const float* __restrict__ part, int tok, int col) {
     float v[BW_WARPS];
 #pragma unroll
-    for (int w = 0; w < BW_WARPS; ++w) v[w] = part[w * BW_B * BW_LD + tok * BW_LD + col];
+    for (int w = 0; w < BW_WARPS; ++w) v[w] = part[(w * BW_B + tok) * LDP + col];
     return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
 }
 
@@ -277,13 +279,15 @@ constexpr int BW_BAR_STATE = 1, BW_BAR_FULL = 2, BW_BAR_DONE = 5;              /
 // block's partial sums into results while the state warps, which then do only what the next block waits for, are at the next
 // one.  A helper passes DONE of block i before it refills the stage of block i - 1 (whose update came before) with block
 // i + 2, makes block i's results and then reports block i + 2 FULL, so the state warps write block i + 2's sums over block
-// i's only after these were read.  That shortens the delta rule's long chain where a CTA has its SM to itself (185 -> 153 us
+// i's only after these were read.  That shortens the delta rule's long chain where a CTA has its SM to itself (185 -> 148 us
 // for 2,048 tokens of 16 heads); with two CTAs on an SM, and without the delta rule, the extra warps only get in the
-// way (linear attention, 1,900 tokens of two requests: 88 -> 107 us).
-template <int NT, bool DELTA, bool HELP>
-__global__ void __launch_bounds__((HELP ? 2 : 1) * BW_THREADS)
+// way (linear attention, 1,900 tokens of two requests: 88 -> 107 us).  The least number of CTAs an SM keeps the compiler from
+// saving registers: with 80 a thread and three CTAs on an SM the same walk took 100 us, with 126 it takes 86.
+template <int NT, int MT, bool DELTA, bool HELP>
+__global__ void __launch_bounds__((HELP ? 2 : 1) * BW_THREADS, HELP ? 1 : 2)
 block_walk_kernel(const BlockWalk a) {
-    using C = BwSmem<NT, HELP>;
+    using C = BwSmem<NT, MT, HELP>;
+    constexpr int COLS = 16 * MT;
     extern __shared__ __align__(16) float bw_smem[];
     float* part_p = bw_smem + C::STAGES * C::STAGE;
     float* parts_r = part_p + C::PART;
@@ -291,7 +295,7 @@ block_walk_kernel(const BlockWalk a) {
     const int s = blockIdx.z, h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
     if (t1 <= t0) return;
     const int tid = threadIdx.x & (BW_THREADS - 1), warp = tid >> 5, lane = tid & 31;
-    const int col0 = blockIdx.x * BW_COLS, cols = a.V - col0 < BW_COLS ? a.V - col0 : BW_COLS;
+    const int col0 = blockIdx.x * COLS, cols = a.V - col0 < COLS ? a.V - col0 : COLS;
 
     const float* rows = a.act ? a.act_rows : a.rows;
     const long ld = a.act ? a.ld_act : a.ld;
@@ -300,27 +304,37 @@ block_walk_kernel(const BlockWalk a) {
     const float* coef = a.coef + ((size_t)bw_first_block(a.q_start, s) * a.heads + h) * BW_COEF;
     const size_t coef_step = (size_t)a.heads * BW_COEF;
     auto fetch = [&](int t, int stage) {                        // the next block in order, which starts at token t
-        bw_fetch<NT, DELTA, HELP>(bw_smem + stage * C::STAGE, a, rows, ld, q_col, k_col, v_col, cols, coef, t, t1, tid);
+        bw_fetch<NT, MT, DELTA, HELP>(bw_smem + stage * C::STAGE, a, rows, ld, q_col, k_col, v_col, cols, coef, t, t1, tid);
         coef += coef_step;
     };
     const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
-    auto results = [&](int t, int stage, int turn) {            // thread = column tid % 16 of token tid / 16
-        const int col = tid & 15, tok = tid >> 4;
+    auto results = [&](int t, int stage, int turn) {            // thread = column tid % COLS of token tid / COLS and, with MT, eight on
+        const int col = tid % COLS, tok = tid / COLS;
         const float* sv = bw_smem + stage * C::STAGE + 2 * C::QK;
-        const float* sA = sv + BW_B * BW_LDV;
+        const float* sA = sv + BW_B * C::LDV;
         const float* gam = sA + 2 * BW_B * BW_LD;
-        const float* u = DELTA ? us + turn * C::U : sv;
-        const float4* a4 = reinterpret_cast<const float4*>(sA + tok * BW_LD);
-        float o0 = gam[tok] * bw_sum_parts(parts_r + turn * C::PART, tok, col), o1 = skip * sv[tok * BW_LDV + col];
+        const float* u = (DELTA ? us + turn * C::U : sv) + col;
+        float o0[MT], o1[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            o0[m] = gam[tok + 8 * m] * bw_sum_parts<C::LDP>(parts_r + turn * C::PART, tok + 8 * m, col);
+            o1[m] = skip * sv[(tok + 8 * m) * C::LDV + col];
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float4 m = a4[j];
-            o0 = fmaf(m.x, u[(4 * j) * BW_LDV + col], o0);
-            o1 = fmaf(m.y, u[(4 * j + 1) * BW_LDV + col], o1);
-            o0 = fmaf(m.z, u[(4 * j + 2) * BW_LDV + col], o0);
-            o1 = fmaf(m.w, u[(4 * j + 3) * BW_LDV + col], o1);
+            const float u0 = u[(4 * j) * C::LDV], u1 = u[(4 * j + 1) * C::LDV], u2 = u[(4 * j + 2) * C::LDV], u3 = u[(4 * j + 3) * C::LDV];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float4 w = *reinterpret_cast<const float4*>(sA + (tok + 8 * m) * BW_LD + 4 * j);
+                o0[m] = fmaf(w.x, u0, o0[m]);
+                o1[m] = fmaf(w.y, u1, o1[m]);
+                o0[m] = fmaf(w.z, u2, o0[m]);
+                o1[m] = fmaf(w.w, u3, o1[m]);
+            }
         }
-        if (t + tok < t1 && col < cols) a.out[(size_t)(t + tok) * a.ldo + (size_t)h * a.V + col0 + col] = o0 + o1;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+            if (t + tok + 8 * m < t1 && col < cols) a.out[(size_t)(t + tok + 8 * m) * a.ldo + (size_t)h * a.V + col0 + col] = o0[m] + o1[m];
     };
 
     if (HELP && threadIdx.x >= BW_THREADS) {
@@ -353,19 +367,19 @@ block_walk_kernel(const BlockWalk a) {
     }
 
     // ---------------------------------------------------------------------- the state
-    // thread (g, tq) of a warp holds columns g and g + 8, rows 2 tq and 2 tq + 1 of every fragment
+    // thread (g, tq) of a warp holds columns g and g + 8 of every 16, rows 2 tq and 2 tq + 1 of every fragment
     if (!HELP) fetch(t0, 0);
     const int g = lane >> 2, tq = lane & 3, row0 = warp * 8 * NT;
     float* st = a.state + (size_t)a.slots[s] * a.state_stride + a.s_off + (size_t)h * a.N * a.V;
     const long sr = a.state_vn ? 1 : a.V, sc = a.state_vn ? a.N : 1;
     const bool fresh = a.positions[t0] == 0;
-    float S[NT][4];
+    float S[MT][NT][4];
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int f = 0; f < MT * NT; ++f)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int row = row0 + nt * 8 + 2 * tq + (e & 1), col = g + (e >> 1) * 8;
-            S[nt][e] = (!fresh && row < a.N && col < cols) ? st[row * sr + (col0 + col) * sc] : 0.f;
+            const int row = row0 + f % NT * 8 + 2 * tq + (e & 1), col = f / NT * 16 + g + (e >> 1) * 8;
+            S[f / NT][f % NT][e] = (!fresh && row < a.N && col < cols) ? st[row * sr + (col0 + col) * sc] : 0.f;
         }
     int b = 0, turn = 0;
     for (int t = t0; t < t1; t += BW_B) {
@@ -379,65 +393,75 @@ block_walk_kernel(const BlockWalk a) {
         const float* sq = bw_smem + b * C::STAGE;
         const float* sk = sq + C::QK;
         const float* sv = sk + C::QK;
-        const float* sM = sv + BW_B * BW_LDV + BW_B * BW_LD;
+        const float* sM = sv + BW_B * C::LDV + BW_B * BW_LD;
         const float* gam = sM + BW_B * BW_LD;
         const float* suf = gam + BW_B;
-        uint32_t sh[NT][4], sl[NT][4];
+        uint32_t sh[MT][NT][4], sl[MT][NT][4];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {                       // rows 2 tq are the operand's k index tq, rows 2 tq + 1 its tq + 4
-            bw_split(S[nt][0], sh[nt][0], sl[nt][0]);
-            bw_split(S[nt][2], sh[nt][1], sl[nt][1]);
-            bw_split(S[nt][1], sh[nt][2], sl[nt][2]);
-            bw_split(S[nt][3], sh[nt][3], sl[nt][3]);
+        for (int f = 0; f < MT * NT; ++f) {                     // rows 2 tq are the operand's k index tq, rows 2 tq + 1 its tq + 4
+            const float(&x)[4] = S[f / NT][f % NT];
+            uint32_t(&xh)[4] = sh[f / NT][f % NT], (&xl)[4] = sl[f / NT][f % NT];
+            bw_split(x[0], xh[0], xl[0]);
+            bw_split(x[2], xh[1], xl[1]);
+            bw_split(x[1], xh[2], xl[2]);
+            bw_split(x[3], xh[3], xl[3]);
         }
         const float* u = sv;
         if (DELTA) {
             float* su = us + turn * C::U;
-            bw_read_out<NT>(sk, sh, sl, part_p + warp * BW_B * BW_LD, row0, g, tq);
+            bw_read_out<NT, MT>(sk, sh, sl, part_p + warp * BW_B * C::LDP, row0, g, tq);
             HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();
-            // thread: token lane % 16 of column tid / 16; the 16 tokens of a column meet in half a warp
-            const int tok = lane & 15, col = tid >> 4;
-            const float e = sv[tok * BW_LDV + col] - gam[tok] * bw_sum_parts(part_p, tok, col);
+            // thread: token lane % 16 of column tid / 16 of every 16; the 16 tokens of a column meet in half a warp
+            const int tok = lane & 15;
             const float4* m4 = reinterpret_cast<const float4*>(sM + tok * BW_LD);
-            float u0 = 0.f, u1 = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 m = m4[j];
-                u0 = fmaf(m.x, __shfl_sync(0xffffffffu, e, 4 * j, 16), u0);
-                u1 = fmaf(m.y, __shfl_sync(0xffffffffu, e, 4 * j + 1, 16), u1);
-                u0 = fmaf(m.z, __shfl_sync(0xffffffffu, e, 4 * j + 2, 16), u0);
-                u1 = fmaf(m.w, __shfl_sync(0xffffffffu, e, 4 * j + 3, 16), u1);
+            for (int mt = 0; mt < MT; ++mt) {
+                const int col = mt * 16 + (tid >> 4);
+                const float e = sv[tok * C::LDV + col] - gam[tok] * bw_sum_parts<C::LDP>(part_p, tok, col);
+                float u0 = 0.f, u1 = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 m = m4[j];
+                    u0 = fmaf(m.x, __shfl_sync(0xffffffffu, e, 4 * j, 16), u0);
+                    u1 = fmaf(m.y, __shfl_sync(0xffffffffu, e, 4 * j + 1, 16), u1);
+                    u0 = fmaf(m.z, __shfl_sync(0xffffffffu, e, 4 * j + 2, 16), u0);
+                    u1 = fmaf(m.w, __shfl_sync(0xffffffffu, e, 4 * j + 3, 16), u1);
+                }
+                su[tok * C::LDV + col] = u0 + u1;
             }
-            su[tok * BW_LDV + col] = u0 + u1;
             u = su;
         }
-        bw_read_out<NT>(sq, sh, sl, parts_r + turn * C::PART + warp * BW_B * BW_LD, row0, g, tq);
+        bw_read_out<NT, MT>(sq, sh, sl, parts_r + turn * C::PART + warp * BW_B * C::LDP, row0, g, tq);
         HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();     // u and the partial sums of r are there
         if (HELP) bw_arrive(BW_BAR_DONE + turn, 2 * BW_THREADS);
-        float up[NT][4] = {};
+        float up[MT][NT][4] = {};
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
             const int ta = ks * 8 + tq;
             const float w0 = suf[ta], w1 = suf[ta + 4];
-            uint32_t ah[4], al[4];
-            bw_split(u[ta * BW_LDV + g] * w0, ah[0], al[0]);
-            bw_split(u[ta * BW_LDV + g + 8] * w0, ah[1], al[1]);
-            bw_split(u[(ta + 4) * BW_LDV + g] * w1, ah[2], al[2]);
-            bw_split(u[(ta + 4) * BW_LDV + g + 8] * w1, ah[3], al[3]);
+            uint32_t ah[MT][4], al[MT][4];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                bw_split(u[ta * C::LDV + mt * 16 + g] * w0, ah[mt][0], al[mt][0]);
+                bw_split(u[ta * C::LDV + mt * 16 + g + 8] * w0, ah[mt][1], al[mt][1]);
+                bw_split(u[(ta + 4) * C::LDV + mt * 16 + g] * w1, ah[mt][2], al[mt][2]);
+                bw_split(u[(ta + 4) * C::LDV + mt * 16 + g + 8] * w1, ah[mt][3], al[mt][3]);
+            }
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 uint32_t bh[2], bl[2];
                 bw_split(sk[ta * C::LDN + row0 + nt * 8 + g], bh[0], bl[0]);
                 bw_split(sk[(ta + 4) * C::LDN + row0 + nt * 8 + g], bh[1], bl[1]);
-                bw_mma3(up[nt], ah, al, bh, bl);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) bw_mma3(up[mt][nt], ah[mt], al[mt], bh, bl);
             }
         }
         if (!HELP) results(t, b, 0);
         const float total = gam[BW_B - 1];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
+        for (int f = 0; f < MT * NT; ++f)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S[nt][e] = fmaf(total, S[nt][e], up[nt][e]);
+            for (int e = 0; e < 4; ++e) S[f / NT][f % NT][e] = fmaf(total, S[f / NT][f % NT][e], up[f / NT][f % NT][e]);
         if (HELP) {
             b = b == 2 ? 0 : b + 1;
             turn ^= 1;
@@ -446,30 +470,35 @@ block_walk_kernel(const BlockWalk a) {
         }
     }
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int f = 0; f < MT * NT; ++f)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int row = row0 + nt * 8 + 2 * tq + (e & 1), col = g + (e >> 1) * 8;
-            if (row < a.N && col < cols) st[row * sr + (col0 + col) * sc] = S[nt][e];
+            const int row = row0 + f % NT * 8 + 2 * tq + (e & 1), col = f / NT * 16 + g + (e >> 1) * 8;
+            if (row < a.N && col < cols) st[row * sr + (col0 + col) * sc] = S[f / NT][f % NT][e];
         }
 }
 
-template <int NT, bool DELTA, bool HELP>
+template <int NT, int MT, bool DELTA, bool HELP>
 static int launch_block_walk(const BlockWalk& a, cudaStream_t stream) {
-    constexpr int bytes = BwSmem<NT, HELP>::TOTAL * 4;
-    auto kern = block_walk_kernel<NT, DELTA, HELP>;
+    constexpr int bytes = BwSmem<NT, MT, HELP>::TOTAL * 4;
+    auto kern = block_walk_kernel<NT, MT, DELTA, HELP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
-    kern<<<dim3((a.V + BW_COLS - 1) / BW_COLS, a.heads, a.S), (HELP ? 2 : 1) * BW_THREADS, bytes, stream>>>(a);
+    kern<<<dim3((a.V + 16 * MT - 1) / (16 * MT), a.heads, a.S), (HELP ? 2 : 1) * BW_THREADS, bytes, stream>>>(a);
     return launch_status();
 }
 
+// Without the delta rule 16 columns a CTA are the faster whatever the load (2,000 tokens of three requests, 32 heads of 128 x
+// 64: 110 us, with 32 columns 139; 1,900 of two, 16 heads of 128 x 128: 86 and 102): a CTA's chain is the longer with 32.  The
+// delta rule has twice the work per block on the rows of q and k, which 32 columns share: where more CTAs than SMs walk
+// anyway, a layer of 1,239 tokens of two requests, 32 heads of 128 x 128, takes 356 us with 32 columns and 388 with 16 (1,186
+// of five requests, 16 heads: 173 and 182).  With fewer, a CTA of 16 columns and helpers has an SM to itself.
 template <int NT>
 static int dispatch_block_walk(const BlockWalk& a, cudaStream_t stream) {
-    if (!a.delta) return launch_block_walk<NT, false, false>(a, stream);
     int sms = 148, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    const long ctas = (long)((a.V + BW_COLS - 1) / BW_COLS) * a.heads * a.S;
-    return ctas <= sms ? launch_block_walk<NT, true, true>(a, stream) : launch_block_walk<NT, true, false>(a, stream);
+    if (!a.delta) return launch_block_walk<NT, 1, false, false>(a, stream);
+    if ((long)((a.V + 15) / 16) * a.heads * a.S <= sms) return launch_block_walk<NT, 1, true, true>(a, stream);
+    return a.V <= 16 ? launch_block_walk<NT, 1, true, false>(a, stream) : launch_block_walk<NT, 2, true, false>(a, stream);
 }
 
 }  // namespace aien

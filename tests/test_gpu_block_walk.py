@@ -21,7 +21,8 @@ def _recurrence(q, k, v, g, w, S, delta, skip):
 
 
 @pytest.mark.parametrize("heads,G,N,V,lens,slow", [
-    (2, 1, 128, 128, [100, 1, 16, 33, 2], True), (24, 8, 72, 64, [50, 3, 16], False), (4, 4, 64, 64, [17, 48], False), (3, 1, 20, 12, [64, 5], True), (6, 2, 68, 36, [40, 15, 1, 1], False),
+    (2, 1, 128, 128, [100, 1, 16, 33, 2], True), (24, 8, 72, 64, [50, 3, 16], False),
+    (60, 20, 64, 36, [17, 31, 1], False), (150, 50, 12, 12, [33], False), (4, 4, 64, 64, [17, 48], False), (3, 1, 20, 12, [64, 5], True), (6, 2, 68, 36, [40, 15, 1, 1], False),
     (1, 1, 4, 4, [33], False), (32, 1, 128, 64, [50], True)])
 @pytest.mark.parametrize("form", ["delta", "weights", "decay"])
 def test_block_walk_follows_the_recurrence(form, heads, G, N, V, lens, slow):
