@@ -400,13 +400,27 @@ ssd_scan_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, in
 // out[t] = the three bfloat16 parts of x[t]'s numbers, part by part: x = p0 + p1 + p2 up to 2^-25 of x (each part rounds
 // what the ones before leave).  With the weights three times side by side a product on the tensor cores then has float32
 // rows on the left: the step sizes' product of 2,048 tokens, 4,096 x 128 bfloat16 weights, took 101 us on the CUDA cores
-// and takes 23 with this launch (2.6 of it).
+// and takes 23 with this launch (2.6 of it).  x may come as partial products over ranges of K: the product that makes it has
+// few columns (160 over 4,096: 32 tiles at 2,048 tokens, 28 us) and is cut over the whole GPU (14 us, and 1.7 more here).
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const float* __restrict__ x, long ldx, __nv_bfloat16* __restrict__ out, int T, int n) {
+split_rows_kernel(const float* __restrict__ x, long ldx, int P, size_t part_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ rest,
+                  int T, int n, int m) {
     const long i = (long)blockIdx.x * 256 + threadIdx.x;
-    if (i >= (long)T * n) return;
-    const int t = (int)(i / n), c = (int)(i - (long)t * n);
-    const float v = x[t * ldx + c];
+    if (i >= (long)T * (n + m)) return;
+    const int t = (int)(i / (n + m)), c = (int)(i - (long)t * (n + m));
+    const float* xc = x + t * ldx + c;
+    float v = xc[0];
+    for (int p0 = 1; p0 < P; p0 += 4) {                         // partial products in order, four loads in flight
+        float w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = p0 + j < P ? xc[(p0 + j) * part_stride] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v += w[j];
+    }
+    if (c >= n) {
+        rest[(size_t)t * m + c - n] = v;
+        return;
+    }
     const __nv_bfloat16 p0 = __float2bfloat16_rn(v);
     const float r0 = v - __bfloat162float(p0);
     const __nv_bfloat16 p1 = __float2bfloat16_rn(r0);
@@ -577,11 +591,12 @@ AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int 
     return launch_status();
 }
 
-// x float32 [T, ldx], n columns; out bfloat16 [T, 3 n].
-AIEN_API int aien_split_rows(const float* x, long ldx, void* out, int T, int n, cudaStream_t stream) {
+// x float32 [T, ldx] (or P partial products of it, part_stride numbers apart); out bfloat16 [T, 3 n] of the first n columns,
+// rest float32 [T, m] (may be null with m = 0) the m columns behind them.
+AIEN_API int aien_split_rows(const float* x, long ldx, int P, size_t part_stride, void* out, float* rest, int T, int n, int m, cudaStream_t stream) {
     if (T <= 0) return 0;
-    if (n <= 0) return AIEN_E_SHAPE;
-    split_rows_kernel<<<(unsigned)(((long)T * n + 255) / 256), 256, 0, stream>>>(x, ldx, (__nv_bfloat16*)out, T, n);
+    if (n <= 0 || m < 0 || P < 1 || (m > 0 && rest == nullptr) || ((long)T * (n + m) + 255) / 256 > 2147483647L) return AIEN_E_SHAPE;
+    split_rows_kernel<<<(unsigned)(((long)T * (n + m) + 255) / 256), 256, 0, stream>>>(x, ldx, P, part_stride, (__nv_bfloat16*)out, rest, T, n, m);
     return launch_status();
 }
 

@@ -193,7 +193,7 @@ def _declare(l: ctypes.CDLL) -> None:
                                               I, I, I, I, I, F, I, I, P],
         "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
         "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, P],
-        "aien_split_rows": [P, L, P, I, I, P],
+        "aien_split_rows": [P, L, I, c_size_t, P, P, I, I, I, P],
         "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
         "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, P, P],
         "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, P],
@@ -1988,12 +1988,17 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
                                      _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), _stream()), "selective_scan")
 
 
-def split_rows(x: torch.Tensor, out: torch.Tensor) -> None:
+def split_rows(x: torch.Tensor, out: torch.Tensor, rest: Optional[torch.Tensor] = None) -> None:
     """x float32 [T, n] as the sum of three bfloat16 rows side by side, out [T, 3 n] (up to 2^-25 of x): the left operand of
-    a tensor-core product that must not round its float32 rows, with the weights three times side by side."""
-    _dev(x, out)
-    assert x.dtype == torch.float32 and x.stride(1) == 1 and out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == (x.shape[0], 3 * x.shape[1])
-    _check(lib().aien_split_rows(_p(x), x.stride(0), _p(out), x.shape[0], x.shape[1], _stream()), "split_rows")
+    a tensor-core product that must not round its float32 rows, with the weights three times side by side.  x may also be
+    float32 partial products [P, T, *], added first; ``rest`` float32 [T, m]: the m columns behind the n, as they are."""
+    _dev(x, out, rest)
+    T, n, m = x.shape[-2], out.shape[1] // 3, 0 if rest is None else rest.shape[1]
+    parts, part_stride = (x.shape[0], x.stride(0)) if x.dim() == 3 else (1, 0)
+    assert x.dtype == torch.float32 and x.stride(-1) == 1 and x.shape[-1] == n + m
+    assert out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == (T, 3 * n)
+    assert rest is None or (rest.dtype == torch.float32 and rest.is_contiguous() and rest.shape[0] == T)
+    _check(lib().aien_split_rows(_p(x), x.stride(-2), parts, part_stride, _p(out), _p(rest), T, n, m, _stream()), "split_rows")
 
 
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,

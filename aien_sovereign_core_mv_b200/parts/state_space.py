@@ -107,7 +107,7 @@ class SelectiveScan(Mixer):
 
     def workspace_bytes(self, lim):
         I, N, R = self.inner, self.state, self.dt_rank
-        return lim.max_tokens * ((2 * I + I + (R + 2 * N) + I) * 4 + (2 * I + 3 * R) * lim.itemsize + self.hidden_size * 4) + 16384 \
+        return lim.max_tokens * ((2 * I + I + (R + 4 * N) + I) * 4 + (2 * I + 3 * R) * lim.itemsize + self.hidden_size * 4) + 16384 \
             + 2 * K.PARTIALS_MAX_BYTES
 
     def forward(self, ctx: StepContext, h: torch.Tensor, run: RunBinding):
@@ -121,15 +121,22 @@ class SelectiveScan(Mixer):
         xa = ws.take((T, I), ctx.dtype) if ctx.dtype != torch.float32 else x
         K.conv_act(proj, 0, I, self.conv, self.conv_b, self.taps, "silu", state, group.slot_map, ctx.seq_of_token, ctx.q_start,
                    ctx.positions, x, xa if xa is not x else None)
-        xp = linear(ctx, xa, self.w_x, out_dtype=torch.float32)                         # dt | B | C
-        if ctx.dtype == torch.bfloat16 and self.w_dt3 is not None:                      # float32 step sizes into the softplus
+        # dt | B | C: few columns over a long K, so in ranges of K where tiles alone leave SMs idle; split_rows adds them
+        in_three = ctx.dtype == torch.bfloat16 and self.w_dt3 is not None
+        xp = linear(ctx, xa, self.w_x, out_dtype=torch.float32, may_defer_sum=in_three)
+        bc, b_off = xp, R
+        if in_three:                                                                    # float32 step sizes into the softplus
             parts = ws.take((T, 3 * R), torch.bfloat16)
-            K.split_rows(xp[:, :R], parts)
+            if xp.dim() == 3:
+                bc, b_off = ws.take((T, 2 * N), torch.float32), 0
+                K.split_rows(xp, parts, bc)
+            else:
+                K.split_rows(xp[:, :R], parts)
             dtz = linear(ctx, parts, self.w_dt3, out_dtype=torch.float32)
         else:
             dtz = linear(ctx, xp[:, :R], self.w_dt, out_dtype=torch.float32)
         y = ws.take((T, I), ctx.dtype)
-        K.selective_scan(x, dtz, xp, R, R + N, proj[:, I:], self.A, self.dt_b, self.D, state, self.conv_floats, group.slot_map,
+        K.selective_scan(x, dtz, bc, b_off, b_off + N, proj[:, I:], self.A, self.dt_b, self.D, state, self.conv_floats, group.slot_map,
                          ctx.q_start, ctx.positions, y, ctx.num_seqs, N)
         return linear(ctx, y, self.w_o, out_dtype=torch.float32, may_defer_sum=True)
 

@@ -353,6 +353,22 @@ def test_product_of_float32_rows_in_three_parts(T, n, N):
     assert float((out - want).abs().max()) <= 3 * n * 2.0 ** -23 * float((x[:, 4:].double().abs() @ w.double().abs().T).max())
 
 
+@pytest.mark.parametrize("P,T,n,m", [(1, 3, 8, 2), (2, 5, 4, 6), (5, 130, 64, 32), (8, 33, 24, 10)])
+def test_partial_products_added_while_cut_in_three(P, T, n, m):
+    """Partial products are added in order and the columns behind the cut ones leave as they are: the same bits as the sum
+    made first."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    x = torch.randn(P, T, n + m, generator=torch.Generator().manual_seed(P + T)).cuda()
+    whole = x[0].clone()
+    for p in range(1, P):
+        whole += x[p]
+    parts, rest = torch.empty(T, 3 * n, dtype=torch.bfloat16).cuda(), torch.empty(T, m).cuda()
+    want = torch.empty_like(parts)
+    K.split_rows(x, parts, rest)
+    K.split_rows(whole[:, :n], want)
+    assert torch.equal(parts, want) and torch.equal(rest, whole[:, n:])
+
+
 @pytest.mark.parametrize("heads,V,G,N", [(3, 8, 1, 5), (4, 16, 2, 24), (6, 24, 3, 40), (2, 64, 1, 128), (1, 40, 1, 200)])
 def test_state_space_duality_cut_any_way(heads, V, G, N):
     from aien_sovereign_core_mv_b200 import kernels as K
