@@ -77,10 +77,14 @@ __device__ __forceinline__ int bw_first_block(const int* q_start, int s) { retur
 __device__ __forceinline__ float bw_silu(float z) { return z / (1.0f + expf(-z)); }
 
 // One CTA per (block, q/k head): its dot products once, then A, M and the decays of every head that shares the q/k head.
-__global__ void __launch_bounds__(256)
+// Its life is one chain (loads, silu, dot products, coefficients), so other CTAs have to fill it: without the delta rule,
+// whose solve takes 64 registers, six to an SM and, with few heads a q/k head, all threads on the coefficients: linear
+// attention with the silu of all rows, 1,900 tokens, 16 heads of 128 x 128: 35 us with four and half a warp, 28.5 so.
+template <bool DELTA>
+__global__ void __launch_bounds__(256, DELTA ? 4 : 6)
 block_coef_kernel(const BlockWalk a) {
     extern __shared__ __align__(16) float bw_smem[];
-    __shared__ float dots[2][BW_B * BW_B];                      // q_i . k_j and k_i . k_j
+    __shared__ float dots[DELTA ? 2 : 1][BW_B * BW_B];                      // q_i . k_j and k_i . k_j
     const int slot = blockIdx.x, kvh = blockIdx.y;
     int lo = 0, hi = a.S - 1;
     while (lo < hi) {
@@ -145,31 +149,44 @@ block_coef_kernel(const BlockWalk a) {
         for (int c = 0; c < N / 4; ++c) {
             const float4 q = q4[c], b = kj4[c];
             x0 = fmaf(q.x, b.x, x0); x1 = fmaf(q.y, b.y, x1); x0 = fmaf(q.z, b.z, x0); x1 = fmaf(q.w, b.w, x1);
-            if (a.delta) {
+            if (DELTA) {
                 const float4 k = ki4[c];
                 y0 = fmaf(k.x, b.x, y0); y1 = fmaf(k.y, b.y, y1); y0 = fmaf(k.z, b.z, y0); y1 = fmaf(k.w, b.w, y1);
             }
         }
         dots[0][tid] = x0 + x1;
-        dots[1][tid] = y0 + y1;
+        if (DELTA) dots[DELTA ? 1 : 0][tid] = y0 + y1;
     }
     __syncthreads();
-    // a thread owns column j of one head's matrices: the product of the decays grows by one factor a row
-    for (int u = tid; u < per * BW_B; u += 256) {
-        const int hh = u >> 4, j = u & 15;
-        float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF;
-        const float wj = a.delta ? 1.f : sw[j * per + hh], g0 = sg[hh];
-        float ratio = 1.f;
-#pragma unroll
-        for (int i = 0; i < BW_B; ++i) {
-            if (i > j) ratio *= sg[i * per + hh];
+    if (per * BW_B * 4 <= 256) {                                // few heads: a thread owns numbers (i, j), and its product of decays
+        for (int u = tid; u < per * BW_B * BW_B; u += 256) {
+            const int hh = u >> 8, i = (u >> 4) & 15, j = u & 15;
+            float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF;
+            const float wj = DELTA ? 1.f : sw[j * per + hh];
+            float ratio = 1.f;
+            for (int r = j + 1; r <= i; ++r) ratio *= sg[r * per + hh];
             c[i * 16 + j] = i >= j ? ratio * dots[0][i * 16 + j] * wj : 0.f;
-            if (a.delta) sl[hh * 256 + i * 16 + j] = i > j ? sw[i * per + hh] * ratio * dots[1][i * 16 + j] : 0.f;
-            if (j == 0) c[512 + i] = g0 * ratio;
+            if (DELTA) sl[u] = i > j ? sw[i * per + hh] * ratio * dots[DELTA ? 1 : 0][i * 16 + j] : 0.f;
+            if (j == 0) c[512 + i] = sg[hh] * ratio;
+            if (i == BW_B - 1) c[512 + 16 + j] = ratio * wj;
         }
-        c[512 + 16 + j] = ratio * wj;
+    } else {                                                    // a thread owns column j of one head's matrices: the product of the decays grows by one factor a row
+        for (int u = tid; u < per * BW_B; u += 256) {
+            const int hh = u >> 4, j = u & 15;
+            float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF;
+            const float wj = DELTA ? 1.f : sw[j * per + hh], g0 = sg[hh];
+            float ratio = 1.f;
+#pragma unroll
+            for (int i = 0; i < BW_B; ++i) {
+                if (i > j) ratio *= sg[i * per + hh];
+                c[i * 16 + j] = i >= j ? ratio * dots[0][i * 16 + j] * wj : 0.f;
+                if (DELTA) sl[hh * 256 + i * 16 + j] = i > j ? sw[i * per + hh] * ratio * dots[DELTA ? 1 : 0][i * 16 + j] : 0.f;
+                if (j == 0) c[512 + i] = g0 * ratio;
+            }
+            c[512 + 16 + j] = ratio * wj;
+        }
     }
-    if (!a.delta) return;
+    if (!DELTA) return;
     __syncthreads();
     // (I + L)^-1 column by column: a thread owns one column of one head
     for (int u = tid; u < per * BW_B; u += 256) {
@@ -529,8 +546,9 @@ AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, i
     BlockWalk a{rows, ld, q_off, k_off, v_off, gates, ldg, g_off, w_off, decay, scratch + coefs, 2L * G * N + (long)heads * V, act, delta, scratch,
                 skip, skip_dt, state, state_stride, s_off, state_vn, slots, q_start, positions, out, ldo, T, S, heads, G, N, V};
     const int per = heads / G, smem = 4 * (2 * BW_B * (N + 4) + 2 * BW_B * per + (delta ? 256 * per : 0));
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(block_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AIEN_E_STATE;
-    block_coef_kernel<<<dim3((unsigned)blocks, G), 256, smem, stream>>>(a);
+    auto coef = delta ? block_coef_kernel<true> : block_coef_kernel<false>;
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(coef, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AIEN_E_STATE;
+    coef<<<dim3((unsigned)blocks, G), 256, smem, stream>>>(a);
     const int rc = launch_status();
     if (rc != 0) return rc;
     return N <= 64 ? dispatch_block_walk<1>(a, stream) : dispatch_block_walk<2>(a, stream);
