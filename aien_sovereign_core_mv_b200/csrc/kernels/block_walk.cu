@@ -292,6 +292,64 @@ __device__ __forceinline__ void bw_sync(int id, int threads) { asm volatile("bar
 __device__ __forceinline__ void bw_arrive(int id, int threads) { asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 constexpr int BW_BAR_STATE = 1, BW_BAR_FULL = 2, BW_BAR_DONE = 5;              // FULL + stage, DONE + block & 1
 
+// Columns col0 .. col0 + cols - 1 of a head's state through a portion token by token in plain float32, from the slot's state as
+// the portion found it; a warp a column, its lanes the rows.  A block multiplies all its tokens with zeros above the
+// diagonal and adds products of halves, which holds for finite numbers only: an infinity or NaN would reach the block's
+// earlier tokens, and an infinity become NaN.  One anywhere in a CTA's rows, gates or state shows in a result or in the
+// last state, so the CTA then walks its columns again here, where a token's number reaches what follows it and nothing else.
+template <bool DELTA>
+__device__ __noinline__ void bw_walk_tokens(const BlockWalk& a, const float* rows, long ld, int q_col, int k_col, int v_col, int s, int h, int col0, int cols) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = a.q_start[s], t1 = a.q_start[s + 1];
+    const long sr = a.state_vn ? 1 : a.V, sc = a.state_vn ? a.N : 1;
+    const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
+    const bool fresh = a.positions[t0] == 0;
+    for (int c = warp; c < cols; c += blockDim.x >> 5) {
+        float* st = a.state + (size_t)a.slots[s] * a.state_stride + a.s_off + (size_t)h * a.N * a.V + (col0 + c) * sc;
+        float S[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[i] = !fresh && lane + 32 * i < a.N ? st[(lane + 32 * i) * sr] : 0.f;
+        for (int t = t0; t < t1; ++t) {
+            const float* r = rows + (size_t)t * ld;
+            const float v = r[v_col + c], g = a.gates != nullptr ? a.gates[(size_t)t * a.ldg + a.g_off + h] : a.decay[h];
+            const float w = a.w_off >= 0 ? a.gates[(size_t)t * a.ldg + a.w_off + h] : 1.f;
+            float k[4], q[4], sk = 0.f, sq = 0.f, kq = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool in = lane + 32 * i < a.N;
+                k[i] = in ? r[k_col + lane + 32 * i] : 0.f;
+                q[i] = in ? r[q_col + lane + 32 * i] : 0.f;
+                if (DELTA) {
+                    sk = fmaf(S[i], k[i], sk);
+                    sq = fmaf(S[i], q[i], sq);
+                    kq = fmaf(k[i], q[i], kq);
+                }
+            }
+            float o;
+            if (DELTA) {
+                const float u = w * (v - g * warp_sum(sk));
+                o = fmaf(warp_sum(kq), u, g * warp_sum(sq));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (lane + 32 * i < a.N) S[i] = fmaf(k[i], u, g * S[i]);
+            } else {
+                const float u = w * v;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (lane + 32 * i < a.N) {
+                        S[i] = fmaf(g, S[i], u * k[i]);
+                        sq = fmaf(S[i], q[i], sq);
+                    }
+                o = warp_sum(sq);
+            }
+            if (a.skip_any != nullptr) o = fmaf(skip, v, o);
+            if (lane == 0) a.out[(size_t)t * a.ldo + (size_t)h * a.V + col0 + c] = o;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) if (lane + 32 * i < a.N) st[(lane + 32 * i) * sr] = S[i];
+    }
+}
+
+__device__ __forceinline__ bool bw_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
 // Eight warps hold the state, bring the blocks and make the results.  With HELP eight more bring the blocks and turn a
 // block's partial sums into results while the state warps, which then do only what the next block waits for, are at the next
 // one.  A helper passes DONE of block i before it refills the stage of block i - 1 (whose update came before) with block
@@ -302,7 +360,7 @@ constexpr int BW_BAR_STATE = 1, BW_BAR_FULL = 2, BW_BAR_DONE = 5;              /
 // saving registers: with 80 a thread and three CTAs on an SM the same walk took 100 us, with 126 it takes 86.
 template <int NT, int MT, bool DELTA, bool HELP>
 __global__ void __launch_bounds__((HELP ? 2 : 1) * BW_THREADS, HELP ? 1 : 2)
-block_walk_kernel(const BlockWalk a) {
+block_walk_kernel(const __grid_constant__ BlockWalk a) {
     using C = BwSmem<NT, MT, HELP>;
     constexpr int COLS = 16 * MT;
     extern __shared__ __align__(16) float bw_smem[];
@@ -325,6 +383,7 @@ block_walk_kernel(const BlockWalk a) {
         coef += coef_step;
     };
     const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
+    bool odd = false;                                           // a number that is not finite has been seen
     auto results = [&](int t, int stage, int turn) {            // thread = column tid % COLS of token tid / COLS and, with MT, eight on
         const int col = tid % COLS, tok = tid / COLS;
         const float* sv = bw_smem + stage * C::STAGE + 2 * C::QK;
@@ -351,7 +410,11 @@ block_walk_kernel(const BlockWalk a) {
         }
 #pragma unroll
         for (int m = 0; m < MT; ++m)
-            if (t + tok + 8 * m < t1 && col < cols) a.out[(size_t)(t + tok + 8 * m) * a.ldo + (size_t)h * a.V + col0 + col] = o0[m] + o1[m];
+            if (t + tok + 8 * m < t1 && col < cols) {
+                const float o = o0[m] + o1[m];
+                odd |= !bw_finite(o);
+                a.out[(size_t)(t + tok + 8 * m) * a.ldo + (size_t)h * a.V + col0 + col] = o;
+            }
     };
 
     if (HELP && threadIdx.x >= BW_THREADS) {
@@ -380,6 +443,7 @@ block_walk_kernel(const BlockWalk a) {
             }
             b = b == 2 ? 0 : b + 1;
         }
+        if (__syncthreads_or(odd)) bw_walk_tokens<DELTA>(a, rows, ld, q_col, k_col, v_col, s, h, col0, cols);
         return;
     }
 
@@ -485,6 +549,14 @@ block_walk_kernel(const BlockWalk a) {
         } else {
             b ^= 1;
         }
+    }
+#pragma unroll
+    for (int f = 0; f < MT * NT; ++f)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) odd |= !bw_finite(S[f / NT][f % NT][e]);
+    if (__syncthreads_or(odd)) {
+        bw_walk_tokens<DELTA>(a, rows, ld, q_col, k_col, v_col, s, h, col0, cols);
+        return;
     }
 #pragma unroll
     for (int f = 0; f < MT * NT; ++f)

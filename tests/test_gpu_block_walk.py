@@ -84,3 +84,62 @@ def test_block_walk_declines_rows_off_the_boundary():
     assert float((out - 3.0).abs().max()) == 0.0 and float((state - 1.0).abs().max()) == 0.0
     assert not K.block_walk_takes(torch.float32, 4096, 1, 4, 2, 64, 64) and not K.block_walk_takes(torch.bfloat16, 64, 64, 4, 2, 64, 64)
     assert not K.block_walk_takes(torch.bfloat16, 4096, 1, 4, 2, 130, 64) and K.block_walk_takes(torch.bfloat16, 4096, 1, 4, 2, 128, 64)
+
+
+@pytest.mark.parametrize("heads,G,N,V", [(2, 1, 128, 32), (4, 2, 64, 20), (150, 50, 12, 36), (1, 1, 36, 16)])
+@pytest.mark.parametrize("form", ["delta", "weights", "decay"])
+@pytest.mark.parametrize("where", ["value", "key", "gate", "state"])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan")])
+def test_a_number_that_is_not_finite_reaches_what_follows_it(odd, where, form, heads, G, N, V):
+    """An infinity or NaN in one token's value, key or gate, or in a request's state: every number that the recurrence, token
+    by token, leaves finite is the one it would be without blocks (the tokens before it in its block, the other columns,
+    heads and requests), and where the recurrence is not, neither is this.  Without the delta rule nothing but sums of one
+    infinity is made of an infinite state: it stays one."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    if where == "gate" and form == "decay":
+        pytest.skip("one decay for all tokens")
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    g_ = torch.Generator().manual_seed(heads + N)
+    lens, at = [41, 20], 21                                   # the sixth token of the second block
+    T, S, GN, delta, act, vn = sum(lens), 2, G * N, form == "delta", form == "decay", form == "weights"
+    rows = torch.randn(T, 2 * GN + heads * V, generator=g_)
+    if delta:
+        rows[:, GN:2 * GN] /= rows[:, GN:2 * GN].reshape(T, G, N).norm(dim=-1).repeat_interleave(N, dim=1)
+    gates = 1.0 - 0.9 * torch.rand(T, 2 * heads, generator=g_)
+    decay, skip = 1.0 - 0.5 * torch.rand(heads, generator=g_), torch.randn(heads, generator=g_)
+    state = torch.randn(S, heads * N * V, generator=g_)
+    h = heads - 1
+    if where == "value":
+        rows[at, 2 * GN + h * V + V - 1] = odd
+    elif where == "key":
+        rows[at, 2 * GN - 1] = odd
+    elif where == "gate":
+        gates[at, h] = odd
+    else:
+        state[0, h * N * V + 3] = odd
+    dev, out = state.clone().cuda(), torch.zeros(T, heads * V).cuda()
+    blocks = torch.empty(K.block_walk_scratch(T, S, heads, G, N, V, act)).cuda()
+    assert K.block_walk(rows.cuda(), 0, GN, 2 * GN, None if act else gates.cuda(), 0, -1 if act else heads, decay.cuda() if act else None, dev, 0,
+                        i32([0, 1]), i32([0, lens[0], T]), i32(list(range(5, 5 + lens[0])) + list(range(9, 9 + lens[1]))), out, S, heads, G, N, V,
+                        blocks, delta=delta, act=act, skip=skip.cuda() if vn else None, state_vn=vn)
+    a = rows.double().numpy()
+    with np.errstate(all="ignore"):
+        if act:
+            a = a / (1.0 + np.exp(-a))
+        for s, r in ((0, slice(0, lens[0])), (1, slice(lens[0], T))):
+            qk = lambda off: np.repeat(a[r, off:off + GN].reshape(-1, G, N), heads // G, axis=1)
+            S0 = state[s].double().numpy().reshape((heads, V, N) if vn else (heads, N, V))
+            S0 = S0.transpose(0, 2, 1) if vn else S0
+            g, w = (np.tile(decay.double().numpy(), (lens[s], 1)), np.ones((lens[s], heads))) if act else (gates[r, :heads].double().numpy(), gates[r, heads:].double().numpy())
+            want, last = _recurrence(qk(0), qk(GN), a[r, 2 * GN:].reshape(-1, heads, V), g, w, S0, delta, skip.double().numpy() if vn else np.zeros(heads))
+            got = out[r].cpu().double().numpy().reshape(want.shape)
+            end = dev[s].cpu().double().numpy().reshape((heads, V, N) if vn else (heads, N, V))
+            end = end.transpose(0, 2, 1) if vn else end
+            for x, y, what in ((got, want, "results"), (end, last, "state")):
+                assert np.array_equal(np.isfinite(x), np.isfinite(y)), f"{what} of request {s}"
+                ok = np.isfinite(y)
+                assert np.abs((x - y)[ok]).max(initial=0.0) <= 1e-5 * np.abs(y[ok]).max(initial=0.0), f"{what} of request {s}"
+            assert s == 1 or not np.isfinite(last).all()
+            if s == 0 and where == "state" and not delta and np.isinf(odd):
+                assert np.isinf(end).sum() == 1 and np.isinf(got).sum() == lens[0]
+    assert np.isfinite(out.cpu().numpy()[:at if where != "state" else 0]).all()
