@@ -120,10 +120,6 @@ template <> __device__ __forceinline__ float decay_exp<__nv_bfloat16>(float v) {
     return e;
 }
 
-// the gate's silu, likewise
-template <typename TO> __device__ __forceinline__ float scan_gate(float z) { return ssm_silu(z); }
-template <> __device__ __forceinline__ float scan_gate<__nv_bfloat16>(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-
 template <int LANES, int CH, typename TO>
 __global__ void __launch_bounds__(SSM_THREADS)
 selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
@@ -206,7 +202,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
                 float y = 0.f;
 #pragma unroll
                 for (int j = 0; j < LANES / 4; ++j) { const float4 v = p[j]; y += (v.x + v.y) + (v.z + v.w); }
-                if (tok < n_tok) out[(size_t)(t + tok) * ldo + c0 + ec] = from_f<TO>(fmaf(dskip, rows[C::ROWS + i], y) * scan_gate<TO>(rows[2 * C::ROWS + i]));
+                if (tok < n_tok) out[(size_t)(t + tok) * ldo + c0 + ec] = from_f<TO>(fmaf(dskip, rows[C::ROWS + i], y) * ssm_silu(rows[2 * C::ROWS + i]));
             }
         }
     }
@@ -254,7 +250,7 @@ selective_scan_token_kernel(ScanRowsIn in, const float* __restrict__ A, const vo
     }
 #pragma unroll
     for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    if (ln == 0 && live) out[t * ldo + c] = from_f<TO>(fmaf(load_dyn(D, pdt, c), x, y) * scan_gate<TO>(z));
+    if (ln == 0 && live) out[t * ldo + c] = from_f<TO>(fmaf(load_dyn(D, pdt, c), x, y) * ssm_silu(z));
 }
 
 // Between the two passes: end[k] becomes the state at the end of segment k with the true start, one after another;

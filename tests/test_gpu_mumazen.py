@@ -335,6 +335,47 @@ def test_selective_scan_many_channels_16_bit_results(inner, N, lens):
     assert float(state[0].abs().max()) == 0.0
 
 
+def _scan_beside_64_bits(K, inner, N, lens, seed, dtype, segments=None, **given):
+    """(results, states) of a scan of used slots on the GPU, and the same in 64 bits; ``given`` replaces inputs."""
+    g = torch.Generator().manual_seed(seed)
+    T, S = sum(lens), len(lens)
+    p = dict(A=-torch.exp(torch.rand(inner, N, generator=g) * 4.0 - 3.0), D=torch.rand(inner, generator=g) + 0.5,
+             bias=torch.rand(inner, generator=g) * 2.0 - 3.0, x=torch.randn(T, inner, generator=g), dtz=torch.randn(T, inner, generator=g),
+             z=torch.randn(T, inner, generator=g), bc=torch.randn(T, 2 * N, generator=g), first=torch.randn(S, inner, N, generator=g))
+    p.update(given)
+    state, out = p["first"].reshape(S, -1).clone().cuda(), torch.zeros(T, inner, dtype=dtype).cuda()
+    q = [sum(lens[:i]) for i in range(S + 1)]
+    seg, nseg = segments or (0, 1)
+    scratch = torch.full((2 * (T // seg + S) * inner * N,), float("nan")).cuda() if seg else None
+    c = {n: t.cuda() for n, t in p.items()}
+    K.selective_scan(c["x"], c["dtz"], c["bc"], 0, N, c["z"], c["A"], c["bias"], c["D"], state, 0, i32(list(range(S))), i32(q),
+                     i32([5 + i for n in lens for i in range(n)] or [0]), out, S, N, seg, nseg, scratch)
+    ys, lasts = [], []
+    for s in range(S):
+        r = slice(q[s], q[s + 1])
+        if not lens[s]:
+            lasts.append(f64(p["first"][s]))
+            continue
+        with np.errstate(all="ignore"):
+            y, last = pz.selective_scan(f64(p["x"][r]), pz.softplus(f64(p["dtz"][r]) + f64(p["bias"])), f64(p["A"]), f64(p["bc"][r][:, :N]), f64(p["bc"][r][:, N:]),
+                                        f64(p["D"]), f64(p["first"][s]))
+            ys.append(y * pz.silu(f64(p["z"][r])))
+        lasts.append(last)
+    return out.float().cpu().numpy(), state.view(S, inner, N).cpu().numpy(), np.concatenate(ys), np.stack(lasts)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", [[1, 1, 1], [40]])
+def test_selective_scan_gates_that_nearly_close(lens, dtype):
+    """silu(-88) is -5e-37, not zero: large results keep it in either type."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    T = sum(lens)
+    z = torch.linspace(-88.4, -87.5, T * 64).view(T, 64)
+    y, _, want, _ = _scan_beside_64_bits(K, 64, 16, lens, 5, dtype, z=z, x=torch.randn(T, 64, generator=torch.Generator().manual_seed(1)) * 1e30)
+    assert float(np.abs(want).max()) > 1e-8
+    H.assert_close(y, want, 3e-5 if dtype == torch.float32 else 4.2e-3, "results")          # 88.4 * 2^-24 in the exponent: 5e-6
+
+
 @pytest.mark.parametrize("T,n,N", [(1, 8, 16), (5, 24, 40), (130, 64, 72)])
 def test_product_of_float32_rows_in_three_parts(T, n, N):
     """The three parts add up to the row (2^-25 of it: each leaves at most half a unit of 8 bits), and the tensor-core
