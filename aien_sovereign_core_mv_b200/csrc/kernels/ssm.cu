@@ -211,7 +211,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
     for (int i = 0; i < CH; ++i) if (n0 + i < N) st[i] = S[i];
 }
 
-// One token a request: a thread group lives for one token, so what counts is how many are resident and how much each
+// One token a request (as many tokens as requests): a thread group lives for one token, so what counts is how many are resident and how much each
 // moves.  Four (sixteen) lanes a channel, no shared memory; 64 requests x 4,096 channels x 16 states (33.5 MB of
 // state read and written): 13.9 us, against 17.5 us with the step sizes in a launch of their own and 52 us for the walk's kernel.
 template <int LANES, int CH, typename TO>
@@ -219,38 +219,46 @@ __global__ void __launch_bounds__(SSM_THREADS)
 selective_scan_token_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
                             float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots,
                             const int* __restrict__ q_start, const int* __restrict__ positions, TO* __restrict__ out, long ldo, int inner, int N) {
-    const int s = blockIdx.y, t = q_start[s], gid = blockIdx.x * SSM_THREADS + threadIdx.x;
-    if (q_start[s + 1] <= t) return;
+    const int s = blockIdx.y, t0 = q_start[s], t1 = q_start[s + 1], gid = blockIdx.x * SSM_THREADS + threadIdx.x;
+    if (t1 <= t0) return;
     const bool live = gid / LANES < inner;
     const int c = live ? gid / LANES : inner - 1, ln = gid % LANES, n0 = ln * CH;   // lanes beyond the last channel repeat it and write nothing
     float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)c * N + n0;
-    const bool zero = positions[t] == 0;
-    const float* br = in.bc + t * in.ldbc + in.b_off + n0;
-    const float* cr = in.bc + t * in.ldbc + in.c_off + n0;
-    float S[CH], a[CH], bv[CH], cv[CH];
+    const bool zero = positions[t0] == 0;
+    float S[CH], a[CH];
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
         const bool ok = n0 + i < N;
         S[i] = (ok && !zero) ? st[i] : 0.f;
         a[i] = ok ? decay_rate<TO>(A[(size_t)c * N + n0 + i]) : 0.f;
-        bv[i] = ok ? br[i] : 0.f;
-        cv[i] = ok ? cr[i] : 0.f;
     }
-    const float x = in.x[t * in.ldx + c], z = in.z[t * in.ldz + c];
-    const float dt = ssm_softplus(in.dtz[t * in.lddt + c] + load_dyn(dt_bias, pdt, c)), dx = dt * x;
-    float y = 0.f;
+    int t = t0;
+    do {                                            // once, unless a step of as many tokens as requests has an empty request beside a portion
+        const float* br = in.bc + t * in.ldbc + in.b_off + n0;
+        const float* cr = in.bc + t * in.ldbc + in.c_off + n0;
+        float bv[CH], cv[CH];
 #pragma unroll
-    for (int i = 0; i < CH; ++i) {
-        S[i] = fmaf(decay_exp<TO>(dt * a[i]), S[i], dx * bv[i]);
-        y = fmaf(S[i], cv[i], y);
-    }
+        for (int i = 0; i < CH; ++i) {
+            const bool ok = n0 + i < N;
+            bv[i] = ok ? br[i] : 0.f;
+            cv[i] = ok ? cr[i] : 0.f;
+        }
+        const float x = in.x[t * in.ldx + c], z = in.z[t * in.ldz + c];
+        const float dt = ssm_softplus(in.dtz[t * in.lddt + c] + load_dyn(dt_bias, pdt, c)), dx = dt * x;
+        float y = 0.f;
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            S[i] = fmaf(decay_exp<TO>(dt * a[i]), S[i], dx * bv[i]);
+            y = fmaf(S[i], cv[i], y);
+        }
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        if (ln == 0 && live) out[t * ldo + c] = from_f<TO>(fmaf(load_dyn(D, pdt, c), x, y) * ssm_silu(z));
+    } while (++t < t1);
     if (live) {
 #pragma unroll
         for (int i = 0; i < CH; ++i) if (n0 + i < N) st[i] = S[i];
     }
-#pragma unroll
-    for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    if (ln == 0 && live) out[t * ldo + c] = from_f<TO>(fmaf(load_dyn(D, pdt, c), x, y) * ssm_silu(z));
 }
 
 // Between the two passes: end[k] becomes the state at the end of segment k with the true start, one after another;

@@ -376,6 +376,16 @@ def test_selective_scan_gates_that_nearly_close(lens, dtype):
     H.assert_close(y, want, 3e-5 if dtype == torch.float32 else 4.2e-3, "results")          # 88.4 * 2^-24 in the exponent: 5e-6
 
 
+@pytest.mark.parametrize("lens", [[0, 2], [3, 0, 0], [1, 0, 2, 1]])
+def test_selective_scan_of_as_many_tokens_as_requests_with_an_empty_one(lens):
+    """As many tokens as requests need not be one each."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    for inner, N in ((40, 16), (130, 40)):
+        y, S, want, last = _scan_beside_64_bits(K, inner, N, lens, 6, torch.float32)
+        H.assert_close(y, want, 3e-5, "results")
+        H.assert_close(S, last, 1e-5, "states")
+
+
 @pytest.mark.parametrize("T,n,N", [(1, 8, 16), (5, 24, 40), (130, 64, 72)])
 def test_product_of_float32_rows_in_three_parts(T, n, N):
     """The three parts add up to the row (2^-25 of it: each leaves at most half a unit of 8 bits), and the tensor-core
