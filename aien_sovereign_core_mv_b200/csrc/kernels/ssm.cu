@@ -17,7 +17,7 @@
 // a token's result depends only on the tokens before it, never on what else is in the batch.
 // Everything here is float32 in both engine precisions; only the result leaves in the compute dtype.
 //
-// The portion-parallel form of the duality recurrence cuts a portion into segments that run side by side: every segment first runs from a zero
+// The portion-parallel forms cut a portion into segments that run side by side: every segment first runs from a zero
 // state and records the product of its decays and its end state; the segments' starting states then follow one from
 // another; a second pass repeats the segment from its true starting state and writes the results.
 #include "common.cuh"
@@ -120,30 +120,42 @@ template <> __device__ __forceinline__ float decay_exp<__nv_bfloat16>(float v) {
     return e;
 }
 
-template <int LANES, int CH, typename TO>
+// FIRST: the first pass over segments (Segments, mode 1): no results, and a channel's decay over the segment is one exponential
+// a state value of the sum of its step sizes.
+template <int LANES, int CH, bool FIRST, typename TO>
 __global__ void __launch_bounds__(SSM_THREADS)
 selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
                       float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots,
-                      const int* __restrict__ q_start, const int* __restrict__ positions, TO* __restrict__ out, long ldo, int inner, int N) {
+                      const int* __restrict__ q_start, const int* __restrict__ positions, TO* __restrict__ out, long ldo, int inner, int N, Segments sg) {
     using C = ScanCfg<LANES, CH>;
     constexpr int U = 8;
     __shared__ __align__(16) float bufs[2][C::STAGE];
     __shared__ __align__(16) float2 steps[C::ROWS];                    // (dt, dt * x) per token and channel
     __shared__ __align__(16) float sums[C::TOKENS * SSM_THREADS];      // a lane's part of y per token
-    const int s = blockIdx.y, t0 = q_start[s], t1 = q_start[s + 1];
+    const int s = blockIdx.y, seg = sg.mode == 0 ? 0 : blockIdx.z;
+    int t0 = q_start[s], t1 = q_start[s + 1];
     if (t1 <= t0) return;
+    const bool fresh = positions[t0] == 0;
+    const size_t seg0 = sg.mode == 0 ? 0 : (size_t)(t0 / sg.seg_len + s);         // the request's first segment in the scratch
+    if (sg.mode != 0) {
+        t0 += seg * sg.seg_len;
+        if (t0 >= t1) return;                                           // a segment beyond the portion's end
+        if (t0 + sg.seg_len < t1) t1 = t0 + sg.seg_len;
+    }
     const int cl = threadIdx.x / LANES, ln = threadIdx.x % LANES, n0 = ln * CH;
     const int c0 = blockIdx.x * C::CPB, c = c0 + cl < inner ? c0 + cl : inner - 1;      // lanes beyond the last channel write nothing
     const bool live = c0 + cl < inner;
     scan_fetch<LANES, CH>(bufs[0], in, c0, inner, N, t0, t1);
     float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)c * N + n0;
-    const bool zero = positions[t0] == 0;
-    float S[CH], a[CH];
+    const size_t so = ((seg0 + seg) * inner + c) * N + n0;
+    const float* init = sg.mode == 2 ? (seg > 0 ? sg.end + so - (size_t)inner * N : sg.decay + so) : st;      // see segment_combine_kernel
+    const bool zero = FIRST || (sg.mode == 0 && fresh);
+    float S[CH], a[CH], dts = 0.f;
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
         const bool in_n = n0 + i < N;
         a[i] = in_n ? decay_rate<TO>(A[(size_t)c * N + n0 + i]) : 0.f;
-        S[i] = (in_n && !zero) ? st[i] : 0.f;
+        S[i] = (in_n && !zero) ? init[i] : 0.f;
     }
     // outside the walk a thread serves channel threadIdx.x % CPB of every LANES-th token
     const int ec = threadIdx.x % C::CPB, e0 = threadIdx.x / C::CPB;
@@ -170,6 +182,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
             for (int u = 0; u < U; ++u) {
                 const float2 dd = steps[(g + u) * C::CPB + cl];
                 const float* br = sbc + (g + u) * 2 * C::NP;
+                if (FIRST) dts += dd.x;
                 if (CH % 2 == 0) {
                     float2 ys = make_float2(0.f, 0.f);
 #pragma unroll
@@ -191,8 +204,9 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
                 }
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) sums[(g + u) * SSM_THREADS + threadIdx.x] = y[u];
+            for (int u = 0; u < U; ++u) if (!FIRST) sums[(g + u) * SSM_THREADS + threadIdx.x] = y[u];
         }
+        if (FIRST) continue;
         __syncthreads();
         if (c0 + ec < inner) {
 #pragma unroll
@@ -206,9 +220,13 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
             }
         }
     }
-    if (!live) return;
+    if (!live || sg.mode == 2) return;
 #pragma unroll
-    for (int i = 0; i < CH; ++i) if (n0 + i < N) st[i] = S[i];
+    for (int i = 0; i < CH; ++i)
+        if (n0 + i < N) {
+            if (FIRST) { sg.decay[so + i] = decay_exp<TO>(dts * a[i]); sg.end[so + i] = S[i]; }
+            else st[i] = S[i];
+        }
 }
 
 // One token a request (as many tokens as requests): a thread group lives for one token, so what counts is how many are resident and how much each
@@ -462,14 +480,24 @@ AIEN_API long aien_ssm_segments_scratch(int T, int S, int seg_len, long lanes) {
 
 struct ScanArgs {
     ScanRowsIn in; const float* A; const void* dt_bias; const void* D; int p_dt; float* state; size_t state_stride, s_off; const int* slots;
-    const int* q_start; const int* positions; void* out; long ldo; int T, S, inner, N; cudaStream_t stream;
+    const int* q_start; const int* positions; void* out; long ldo; int T, S, inner, N; Segments sg; cudaStream_t stream;
 };
 
 template <int LANES, int CH, typename TO>
 static void launch_selective_scan(const ScanArgs& a) {
     using C = ScanCfg<LANES, CH>;
-    selective_scan_kernel<LANES, CH, TO><<<dim3((unsigned)((a.inner + C::CPB - 1) / C::CPB), a.S), SSM_THREADS, 0, a.stream>>>(
-        a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N);
+    Segments sg = a.sg;
+    const dim3 grid((unsigned)((a.inner + C::CPB - 1) / C::CPB), a.S, sg.mode == 0 ? 1 : sg.nseg);
+    if (sg.mode != 0) {
+        const size_t lanes = (size_t)a.inner * a.N;
+        selective_scan_kernel<LANES, CH, true, TO><<<grid, SSM_THREADS, 0, a.stream>>>(
+            a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+        segment_combine_kernel<<<dim3((unsigned)((lanes + 255) / 256), a.S), 256, 0, a.stream>>>(a.state, a.state_stride, a.s_off, a.slots, a.q_start,
+                                                                                                 a.positions, sg, lanes);
+        sg.mode = 2;
+    }
+    selective_scan_kernel<LANES, CH, false, TO><<<grid, SSM_THREADS, 0, a.stream>>>(
+        a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
 }
 
 template <int LANES, int CH, typename TO>
@@ -505,18 +533,26 @@ static int dispatch_selective_scan(const ScanArgs& a) {
 
 // x [T, ldx] (after convolution and silu), dtz [T, lddt] = W_dt dt before its bias, bc [T, ldbc] with B at b_off and C at
 // c_off (N numbers each, N <= 128), z [T, ldz] the gate's input, A float32 [inner, N] (negative rates), dt_bias and D
-// [inner] in p_dt.  T is the number of tokens in the step.
+// [inner] in p_dt.  T is the number of tokens in the step.  seg_len > 0: portions are cut into nseg segments of seg_len tokens
+// that run side by side (scratch float32, aien_ssm_segments_scratch(T, S, seg_len, inner * N) numbers); nseg * seg_len must cover
+// the longest portion.
 AIEN_API int aien_selective_scan(const float* x, long ldx, const float* dtz, long lddt, const float* bc, long ldbc, int b_off, int c_off,
                                  const float* z, long ldz, const float* A, const void* dt_bias, const void* D, int p_dt,
                                  float* state, size_t state_stride, size_t s_off, const int* slots, const int* q_start,
-                                 const int* positions, void* out, int o_dt, long ldo, int T, int S, int inner, int N, cudaStream_t stream) {
+                                 const int* positions, void* out, int o_dt, long ldo, int T, int S, int inner, int N,
+                                 int seg_len, int nseg, float* scratch, cudaStream_t stream) {
     if (S <= 0 || T <= 0) return 0;
-    if (inner <= 0 || N <= 0 || S > 65535) return AIEN_E_SHAPE;
+    if (inner <= 0 || N <= 0 || S > 65535 || nseg > 65535) return AIEN_E_SHAPE;
+    Segments sg{0, 0, nullptr, nullptr, 1};
+    if (seg_len > 0 && nseg > 1) {
+        if (scratch == nullptr) return AIEN_E_SHAPE;
+        sg = Segments{1, seg_len, scratch, scratch + (size_t)(T / seg_len + S) * (size_t)inner * N, nseg};
+    }
     const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dtz) | reinterpret_cast<uintptr_t>(z)) & 15) == 0 &&
                       ((ldx | lddt | ldz | inner) & 3) == 0;
     const bool wide_bc = (reinterpret_cast<uintptr_t>(bc) & 15) == 0 && ((ldbc | b_off | c_off | N) & 3) == 0;
     const ScanArgs a{{x, ldx, dtz, lddt, bc, ldbc, b_off, c_off, z, ldz, wide, wide_bc}, A, dt_bias, D, p_dt, state, state_stride, s_off, slots,
-                     q_start, positions, out, ldo, T, S, inner, N, stream};
+                     q_start, positions, out, ldo, T, S, inner, N, sg, stream};
     int rc = 0;
     AIEN_DISPATCH_DTYPE(o_dt, TO, (rc = dispatch_selective_scan<TO>(a)));
     if (rc != 0) return rc;

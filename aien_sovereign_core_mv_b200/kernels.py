@@ -192,7 +192,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "aien_paged_attention_decode_fused": [P, L, P, L, P, L, P, P, I, F, P, P, I, P, P, P, P, I, P, P, L, P, P, P,
                                               I, I, I, I, I, F, I, I, P],
         "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
-        "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, P],
+        "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, I, I, P, P],
         "aien_split_rows": [P, L, I, c_size_t, P, P, I, I, I, P],
         "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
         "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, P, P],
@@ -1968,6 +1968,25 @@ def scan_scratch_floats(max_tokens: int, max_seqs: int, lanes: int, parallel: in
     return 2 * (want + 1 + max_seqs) * lanes
 
 
+def selective_scan_segments(num_tokens: int, num_seqs: int, decode_only: bool, inner: int) -> tuple:
+    """(segment length, most segments a portion has) for :func:`selective_scan` in a step; (0, 1): every portion in one piece.
+    A whole walk takes 50 ns a token and more however few channels walk, and a CTA has 8 of them; two passes over segments take
+    as long as their length twice, once the GPU has room for the CTAs.  2,048 tokens of one request, 16 states, B200, whole
+    and in segments of 128: 256 channels 101 and 31 us, 1,024 channels 101 and 72, 4,096 channels 152 and 159; 256 tokens in
+    segments of 64: 64 channels 17 and 15 us, 512 channels 17 and 17, 1,024 channels 17 and 19.  It depends on the step's token and
+    request counts and the layer's channels alone."""
+    average = num_tokens // max(num_seqs, 1)
+    if decode_only or inner * num_seqs > (1024 if average >= 1024 else 512) or average < 256:
+        return 0, 1
+    seg = 128 if average >= 1024 else 64
+    return seg, -(-num_tokens // seg)
+
+
+def selective_scan_scratch(max_tokens: int, max_seqs: int, inner: int, N: int) -> int:
+    """Upper bound of the float32 scratch that steps in segments take (2 numbers a state value and segment)."""
+    return 2 * (max_tokens // 64 + min(max_seqs, 1024 // inner)) * inner * N if inner <= 1024 else 0
+
+
 def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: int, c_off: int, z: torch.Tensor, A: torch.Tensor,
                    dt_bias: torch.Tensor, D: torch.Tensor, state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor,
                    positions: torch.Tensor, out: torch.Tensor, num_seqs: int, N: int, seg_len: int = 0, nseg: int = 1,
@@ -1975,17 +1994,22 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
     """The selective scan over every request's portion: per channel c and state n, token by token,
     dt = softplus(dtz[c] + dt_bias[c]); S[c, n] = exp(dt * A[c, n]) * S[c, n] + dt * x[c] * B[n]; y[c] = sum_n S[c, n] * C[n]
     + D[c] * x[c]; out[c] = y[c] * silu(z[c]).  x, dtz, z float32 [T, inner] (row strides free); B and C are the N numbers from columns ``b_off`` / ``c_off`` of the float32 rows ``bc``; A float32 [inner, N]; S lives in the request's state row
-    from ``s_off`` on ([inner, N]) and starts from zeros where a portion's first token has position 0.  Every portion is
-    walked in one piece: ``seg_len``, ``nseg`` and ``scratch`` (see :func:`scan_segments`) may be given and change nothing."""
+    from ``s_off`` on ([inner, N]) and starts from zeros where a portion's first token has position 0.  ``seg_len`` > 0: portions
+    are cut into at most ``nseg`` segments of so many tokens that run side by side (``scratch``: 2 * (T // seg_len + num_seqs) *
+    inner * N float32 numbers; see :func:`selective_scan_segments`)."""
     _dev(x, dtz, bc, z, A, dt_bias, D, state, slot_map, q_start, positions, out, scratch)
     T, inner = x.shape
     for t in (x, dtz, bc, z):
         assert t.dtype == torch.float32 and t.stride(1) == 1
     assert A.dtype == torch.float32 and A.is_contiguous() and tuple(A.shape) == (inner, N) and dt_bias.dtype == D.dtype
     assert dt_bias.is_contiguous() and D.is_contiguous() and state.dtype == torch.float32 and state.stride(-1) == 1 and out.stride(1) == 1
+    if seg_len and nseg > 1:
+        assert scratch is not None and scratch.numel() >= 2 * (T // seg_len + num_seqs) * inner * N
     _check(lib().aien_selective_scan(_p(x), x.stride(0), _p(dtz), dtz.stride(0), _p(bc), bc.stride(0), int(b_off), int(c_off), _p(z), z.stride(0),
                                      _p(A), _p(dt_bias), _p(D), dt(D), _p(state), state.stride(0), int(s_off), _p(slot_map), _p(q_start),
-                                     _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), _stream()), "selective_scan")
+                                     _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), int(seg_len), int(nseg),
+                                     _p(scratch), _stream()), "selective_scan")
+    add_launches(2 if (seg_len and nseg > 1) else 0)
 
 
 def split_rows(x: torch.Tensor, out: torch.Tensor, rest: Optional[torch.Tensor] = None) -> None:

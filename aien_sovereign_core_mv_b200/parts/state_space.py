@@ -108,7 +108,7 @@ class SelectiveScan(Mixer):
     def workspace_bytes(self, lim):
         I, N, R = self.inner, self.state, self.dt_rank
         return lim.max_tokens * ((2 * I + I + (R + 4 * N) + I) * 4 + (2 * I + 3 * R) * lim.itemsize + self.hidden_size * 4) + 16384 \
-            + 2 * K.PARTIALS_MAX_BYTES
+            + 2 * K.PARTIALS_MAX_BYTES + 4 * K.selective_scan_scratch(lim.max_tokens, lim.max_seqs, I, N)
 
     def forward(self, ctx: StepContext, h: torch.Tensor, run: RunBinding):
         T, I, N, R = ctx.num_tokens, self.inner, self.state, self.dt_rank
@@ -136,8 +136,10 @@ class SelectiveScan(Mixer):
         else:
             dtz = linear(ctx, xp[:, :R], self.w_dt, out_dtype=torch.float32)
         y = ws.take((T, I), ctx.dtype)
+        seg, nseg = K.selective_scan_segments(T, ctx.num_seqs, ctx.decode_only, I)
+        scratch = ws.take((2 * (T // seg + ctx.num_seqs) * I * N,), torch.float32) if seg else None
         K.selective_scan(x, dtz, bc, b_off, b_off + N, proj[:, I:], self.A, self.dt_b, self.D, state, self.conv_floats, group.slot_map,
-                         ctx.q_start, ctx.positions, y, ctx.num_seqs, N)
+                         ctx.q_start, ctx.positions, y, ctx.num_seqs, N, seg, nseg, scratch)
         return linear(ctx, y, self.w_o, out_dtype=torch.float32, may_defer_sum=True)
 
 

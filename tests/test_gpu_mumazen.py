@@ -386,6 +386,18 @@ def test_selective_scan_of_as_many_tokens_as_requests_with_an_empty_one(lens):
         H.assert_close(S, last, 1e-5, "states")
 
 
+@pytest.mark.parametrize("inner,N,lens", [(64, 16, [300]), (36, 8, [511, 257]), (128, 64, [260, 1, 700]), (1024, 16, [1100]), (37, 5, [2, 900])])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_selective_scan_in_the_segments_of_few_channels(inner, N, lens, dtype):
+    """Steps that the rule cuts: last segments of every length, requests shorter than a segment, 16-byte rows and others."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    cut = K.selective_scan_segments(sum(lens), len(lens), False, inner)
+    assert cut[0] > 0 and 2 * (sum(lens) // cut[0] + len(lens)) * inner * N <= K.selective_scan_scratch(sum(lens), len(lens), inner, N)
+    y, S, want, last = _scan_beside_64_bits(K, inner, N, lens, 8, dtype, cut)
+    H.assert_close(y, want, 3e-5 if dtype == torch.float32 else 4.2e-3, "results")
+    H.assert_close(S, last, 1e-5, "states")
+
+
 @pytest.mark.parametrize("T,n,N", [(1, 8, 16), (5, 24, 40), (130, 64, 72)])
 def test_product_of_float32_rows_in_three_parts(T, n, N):
     """The three parts add up to the row (2^-25 of it: each leaves at most half a unit of 8 bits), and the tensor-core
