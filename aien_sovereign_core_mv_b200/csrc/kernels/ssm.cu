@@ -51,7 +51,6 @@ struct Segments {
 //   * all that does not depend on the state is made for the whole stage before and after its walk, by all threads: the
 //     step size (softplus) and its product with x before, the sum over a channel's lanes, the skip and the gate after;
 //   * inside the walk, eight tokens at a time, only one multiply-add a state value depends on the token before.
-// Tokens behind the portion's end have step size 0 and rows of zeros: they leave the state as it is.
 // 2,048 tokens of 4,096 channels with 16 states each, one request, B200: 764 us, and 26 us for the step sizes, with the
 // rows fetched into registers four tokens ahead; 137 us so
 // (31 instructions a token and warp, of which half a dozen in the prologue and epilogue of a stage; 16 lanes: 180 us, 4: 267 us).
@@ -176,35 +175,43 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
         }
         __syncthreads();
         const float* sbc = rows + 3 * C::ROWS + n0;
-        for (int g = 0; g < n_tok; g += U) {
+        auto token = [&](int tok) {                                     // the lane's part of y
+            const float2 dd = steps[tok * C::CPB + cl];
+            const float* br = sbc + tok * 2 * C::NP;
+            if (FIRST) dts += dd.x;
+            if (CH % 2 == 0) {
+                float2 ys = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < CH; i += 2) {
+                    const float2 b2 = *reinterpret_cast<const float2*>(br + i), c2 = *reinterpret_cast<const float2*>(br + C::NP + i);
+                    const float2 e = make_float2(decay_exp<TO>(dd.x * a[i]), decay_exp<TO>(dd.x * a[(i + 1) % CH]));
+                    const float2 S2 = __ffma2_rn(e, make_float2(S[i], S[(i + 1) % CH]), __fmul2_rn(make_float2(dd.y, dd.y), b2));
+                    S[i] = S2.x; S[(i + 1) % CH] = S2.y;
+                    ys = __ffma2_rn(S2, c2, ys);
+                }
+                return ys.x + ys.y;
+            }
+            float y = 0.f;
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                S[i] = fmaf(decay_exp<TO>(dd.x * a[i]), S[i], dd.y * br[i]);
+                y = fmaf(S[i], br[C::NP + i], y);
+            }
+            return y;
+        };
+        int g = 0;
+        for (; g + U <= n_tok; g += U) {
             float y[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const float2 dd = steps[(g + u) * C::CPB + cl];
-                const float* br = sbc + (g + u) * 2 * C::NP;
-                if (FIRST) dts += dd.x;
-                if (CH % 2 == 0) {
-                    float2 ys = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int i = 0; i < CH; i += 2) {
-                        const float2 b2 = *reinterpret_cast<const float2*>(br + i), c2 = *reinterpret_cast<const float2*>(br + C::NP + i);
-                        const float2 e = make_float2(decay_exp<TO>(dd.x * a[i]), decay_exp<TO>(dd.x * a[(i + 1) % CH]));
-                        const float2 S2 = __ffma2_rn(e, make_float2(S[i], S[(i + 1) % CH]), __fmul2_rn(make_float2(dd.y, dd.y), b2));
-                        S[i] = S2.x; S[(i + 1) % CH] = S2.y;
-                        ys = __ffma2_rn(S2, c2, ys);
-                    }
-                    y[u] = ys.x + ys.y;
-                } else {
-                    y[u] = 0.f;
-#pragma unroll
-                    for (int i = 0; i < CH; ++i) {
-                        S[i] = fmaf(decay_exp<TO>(dd.x * a[i]), S[i], dd.y * br[i]);
-                        y[u] = fmaf(S[i], br[C::NP + i], y[u]);
-                    }
-                }
-            }
+            for (int u = 0; u < U; ++u) y[u] = token(g + u);
 #pragma unroll
             for (int u = 0; u < U; ++u) if (!FIRST) sums[(g + u) * SSM_THREADS + threadIdx.x] = y[u];
+        }
+        // the rest of a portion; the tokens behind its end have no step: 0 times an infinite rate is no decay
+#pragma unroll 1
+        for (; g < n_tok; ++g) {
+            const float y = token(g);
+            if (!FIRST) sums[g * SSM_THREADS + threadIdx.x] = y;
         }
         if (FIRST) continue;
         __syncthreads();

@@ -365,6 +365,21 @@ def _scan_beside_64_bits(K, inner, N, lens, seed, dtype, segments=None, **given)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner", [48, 2048])
+def test_selective_scan_with_an_infinite_rate(inner, dtype):
+    """A state whose rate is minus infinity forgets everything before the token; a portion that ends inside a group of tokens
+    leaves it as finite as one that does not."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    for n in (8, 9, 33):
+        A = -torch.exp(torch.rand(inner, 16, generator=torch.Generator().manual_seed(3)) * 4.0 - 3.0)
+        A[::3, 5] = -float("inf")
+        y, S, want, last = _scan_beside_64_bits(K, inner, 16, [n], 4, dtype, A=A)
+        assert np.isfinite(S).all()
+        H.assert_close(S, last, 1e-5, f"state, {n} tokens")
+        H.assert_close(y, want, 3e-5 if dtype == torch.float32 else 4.2e-3, f"results, {n} tokens")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("lens", [[1, 1, 1], [40]])
 def test_selective_scan_gates_that_nearly_close(lens, dtype):
     """silu(-88) is -5e-37, not zero: large results keep it in either type."""
