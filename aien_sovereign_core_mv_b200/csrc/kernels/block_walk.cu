@@ -595,9 +595,9 @@ static int dispatch_block_walk(const BlockWalk& a, cudaStream_t stream) {
 using namespace aien;
 
 // Whether the walk takes these sizes; the rows besides have to start on 16-byte boundaries (aien_block_walk refuses others).
-AIEN_API int aien_block_walk_supports(int heads, int G, int N, int V) {
+AIEN_API int aien_block_walk_supports(int heads, int G, int N, int V, int delta) {
     if (heads <= 0 || G <= 0 || heads % G || N <= 0 || N > 128 || N % 4 || V <= 0 || V % 4 || heads > 65535) return 0;
-    const long smem = 2L * BW_B * (N + 4) + 2L * BW_B * (heads / G) + 256L * (heads / G);
+    const long smem = 2L * BW_B * (N + 4) + (2L * BW_B + (delta ? 256 : 0)) * (heads / G);       // as the launch of block_coef_kernel counts
     return smem * 4 <= 160 * 1024;
 }
 
@@ -612,7 +612,7 @@ AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, i
                              size_t s_off, int state_vn, const int* slots, const int* q_start, const int* positions, float* out, long ldo,
                              int T, int S, int heads, int G, int N, int V, float* scratch, cudaStream_t stream) {
     if (S <= 0 || T <= 0) return 0;
-    if (!aien_block_walk_supports(heads, G, N, V) || S > 65535 || G > 65535 || scratch == nullptr || (gates == nullptr && decay == nullptr)) return AIEN_E_SHAPE;
+    if (!aien_block_walk_supports(heads, G, N, V, delta) || S > 65535 || G > 65535 || scratch == nullptr || (gates == nullptr && decay == nullptr)) return AIEN_E_SHAPE;
     if ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(scratch)) & 15 || (ld | q_off | k_off | v_off) & 3) return AIEN_E_ALIGN;
     const long blocks = T / BW_B + S, coefs = blocks * heads * BW_COEF;
     BlockWalk a{rows, ld, q_off, k_off, v_off, gates, ldg, g_off, w_off, decay, scratch + coefs, 2L * G * N + (long)heads * V, act, delta, scratch,

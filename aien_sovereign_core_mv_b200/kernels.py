@@ -1891,13 +1891,14 @@ def conv_act(proj: torch.Tensor, off: int, channels: int, w: torch.Tensor, bias:
 
 
 # ---------------------------------------------------------------------------- recurrences sixteen tokens at a time
-def block_walk_takes(dtype: torch.dtype, num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int) -> bool:
+def block_walk_takes(dtype: torch.dtype, num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, delta: bool = False) -> bool:
     """Whether a step's recurrence with one decay per head goes through :func:`block_walk`: a bfloat16 engine's portions of
     prompts (a float32 engine keeps to plain float32 products) over state matrices of up to 128 rows, with tokens enough
-    beside each request's first that blocks of 16 are worth their coefficients' launch."""
+    beside each request's first that blocks of 16 are worth their coefficients' launch, and heads whose coefficients fit a
+    CTA's shared memory (the delta rule solves a 16 x 16 system a head there)."""
     per = heads // max(qk_heads, 1)
     return (dtype == torch.bfloat16 and num_tokens - num_seqs >= BLOCK_WALK_MIN_TOKENS and 0 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
-            and 32 * (dim + 4) + 288 * per <= 40 * 1024)
+            and 32 * (dim + 4) + (288 if delta else 32) * per <= 40 * 1024)
 
 
 BLOCK_WALK_MIN_TOKENS = 32

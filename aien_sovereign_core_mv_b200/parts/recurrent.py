@@ -196,7 +196,7 @@ class GatedDeltaRule(Mixer):
         o = ctx.workspace.take((T, self.v_dim), torch.float32)
         sizes = (n, self.num_qk_heads, self.head_dim, self.value_dim)
         blocks = None
-        if K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes) and not ctx.decode_only:
+        if K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes, delta=True) and not ctx.decode_only:
             blocks = ctx.workspace.take((K.block_walk_scratch(T, ctx.num_seqs, *sizes),), torch.float32)
         K.delta_rule(qkv, 0, self.qk_dim, 2 * self.qk_dim, gb, state, self.conv_floats, group.slot_map, ctx.q_start, ctx.positions, o,
                      ctx.num_seqs, *sizes, blocks)

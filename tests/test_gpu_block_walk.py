@@ -74,6 +74,27 @@ def test_block_walk_follows_the_recurrence(form, heads, G, N, V, lens, slow):
     assert torch.equal(dev[keep].cpu(), state[keep]) and torch.equal(dev[:, :s_off].cpu(), state[:, :s_off]) and torch.equal(dev[:, -extra:].cpu(), state[:, -extra:])
 
 
+def test_many_heads_over_one_group_walk_by_blocks():
+    """The duality form needs no 16 x 16 system a head, so heads that are too many for the delta rule are not for it."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    T, heads, G, N, V = 40, 128, 1, 128, 4
+    assert K.block_walk_takes(torch.bfloat16, 2048, 1, heads, G, N, 64) and not K.block_walk_takes(torch.bfloat16, 2048, 1, heads, G, N, 64, delta=True)
+    g_ = torch.Generator().manual_seed(1)
+    rows, gates = torch.randn(T, 2 * N + heads * V, generator=g_), 1.0 - 0.9 * torch.rand(T, 2 * heads, generator=g_)
+    state, out = torch.zeros(1, heads * N * V).cuda(), torch.zeros(T, heads * V).cuda()
+    run = lambda delta: K.block_walk(rows.cuda(), 0, N, 2 * N, gates.cuda(), 0, heads, None, state, 0, i32([0]), i32([0, T]), i32(list(range(T))), out, 1,
+                                     heads, G, N, V, torch.empty(K.block_walk_scratch(T, 1, heads, G, N, V)).cuda(), delta=delta, state_vn=True)
+    with pytest.raises(K.KernelError):
+        run(True)
+    assert run(False)
+    a, ga = rows.double().numpy(), gates.double().numpy()
+    qk = lambda off: np.repeat(a[:, off:off + N].reshape(T, 1, N), heads, axis=1)
+    want, last = _recurrence(qk(0), qk(N), a[:, 2 * N:].reshape(T, heads, V), ga[:, :heads], ga[:, heads:], np.zeros((heads, N, V)), False, np.zeros(heads))
+    H.assert_close(out.cpu().numpy().reshape(T, heads, V), want, 1e-5, "results")
+    H.assert_close(state.cpu().numpy().reshape(heads, V, N).transpose(0, 2, 1), last, 1e-5, "state")
+
+
 def test_block_walk_declines_rows_off_the_boundary():
     from aien_sovereign_core_mv_b200 import kernels as K
     i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
