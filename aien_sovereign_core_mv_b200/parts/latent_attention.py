@@ -65,6 +65,13 @@ class LatentAttention(Mixer):
         self.w_kv = None
         self.w_down = self.w_uq = self.w_uk_t = self.w_uv = self.w_o = self.dq_norm = self.dkv_norm = self.sinks = None
 
+    def _may_expand(self) -> bool:
+        """Whether the expanded form can be taken at all.  It needs a second copy of the up-projections (``w_kv``) and
+        workspace for the step's keys and values (up to ``kernels.LATENT_EXPAND_MAX_BYTES`` and the gathered rows, twice:
+        the workspace has two layer regions); a program that wants this memory for something else sets
+        AIEN_B200_LATENT_PORTIONS=absorb before it loads the model, and neither is made."""
+        return self._expandable and K.LATENT_PORTIONS != "absorb"
+
     # ---- tensors
     def param_shapes(self):
         H, n = self.hidden_size, self.num_heads
@@ -104,7 +111,7 @@ class LatentAttention(Mixer):
         # per head [kv_rank, head_dim]: the matrix that takes a head's unrotated query to the latent
         self.w_uk_t = tensors["uk_proj"].view(n, self.head_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = tensors["uv_proj"].view(n, self.value_dim, self.kv_rank).contiguous()
-        if self._expandable and tensors["uk_proj"].dtype == torch.bfloat16 == tensors["uv_proj"].dtype:
+        if self._may_expand() and tensors["uk_proj"].dtype == torch.bfloat16 == tensors["uv_proj"].dtype:
             # all heads' keys (unrotated | rotated part, the latter copied through by ones) | all heads' values, from whole cached rows
             w = torch.zeros((n * (self.q_head + self.value_dim), self.row), dtype=torch.bfloat16, device=tensors["uk_proj"].device)
             k = w[:n * self.q_head].view(n, self.q_head, self.row)
@@ -133,7 +140,7 @@ class LatentAttention(Mixer):
         # below 296 tiles' worth of 64 rows
         split = 296 * K.LATENT_TC_TILE * (self.kv_rank + 2) * 4
         expand = 0
-        if self._expandable and lim.itemsize == 2:
+        if self._may_expand() and lim.itemsize == 2:
             rows = K.latent_expand_rows(lim.max_context, lim.max_seqs)
             per_row = n * (self.q_head + self.value_dim) * 2
             rows = min(rows, K.LATENT_EXPAND_MAX_BYTES // per_row + 128)

@@ -78,3 +78,22 @@ def test_config_errors_name_the_field():
     bad = copy.deepcopy(CONFIG); del bad["norm"]
     with pytest.raises(ConfigError, match="norm"):
         model_spec_for(bad)
+
+
+def test_no_room_is_kept_for_expanded_portions_that_are_pinned_away(monkeypatch):
+    """The second copy of the up-projections and the workspace of the expanded form, up to 256 MiB of keys and values, are
+    there only where the form can be taken."""
+    import torch
+    from aien_sovereign_core_mv_b200 import kernels as K
+    from aien_sovereign_core_mv_b200.parts import StepLimits
+    from aien_sovereign_core_mv_b200.registry import make_part
+    lim = StepLimits(max_tokens=2048, max_seqs=64, max_context=8192, itemsize=2)
+    room, kept = {}, {}
+    for pin in ("", "absorb"):
+        monkeypatch.setattr(K, "LATENT_PORTIONS", pin)
+        part = make_part("mixer", "latent_attention", hidden_size=64, num_heads=16, head_dim=128, rot_dim=64, value_dim=128, kv_rank=64, q_rank=0,
+                         window=1024, sink=True, position=make_part("position", "rotary", head_dim=64, theta=10000.0, pairing="interleaved"))
+        part.bind({n: torch.zeros(shape, dtype=torch.bfloat16) for n, (shape, _) in part.param_shapes().items()})
+        room[pin], kept[pin] = part.workspace_bytes(lim), part.w_kv
+    assert kept["absorb"] is None and tuple(kept[""].shape) == (16 * (192 + 128), 128)
+    assert room[""] - room["absorb"] > K.LATENT_EXPAND_MAX_BYTES - (1 << 20)
