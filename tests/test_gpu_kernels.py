@@ -1205,11 +1205,14 @@ def test_cache_housekeeping_kernels(K):
     assert (K.zero_fill(big) == 0).all()
 
 
-@pytest.mark.parametrize("N,K,counts", [(768, 136, [130, 0, 1, 256]), (264, 64, [5, 128, 129]), (8, 1032, [0, 77]), (2048, 24, [400] * 40), (256, 72, [128] * 200)])
+@pytest.mark.parametrize("N,K,counts", [(768, 136, [130, 0, 1, 256]), (264, 64, [5, 128, 129]), (8, 1032, [0, 77]), (2048, 24, [400] * 40), (256, 72, [128] * 200),
+                                        (264, 328, [2000, 0, 77, 0, 35000, 128, 0]), (784, 328, [0, 5000, 129, 0, 7000, 1, 640, 0])])
 @pytest.mark.parametrize("form", ["gelu", "gated", "scattered", "weight_first"])
 def test_grouped_product_in_both_tile_forms(form, N, K, counts):
     """Rows sorted by group in runs of whole 128-row tiles, groups without rows, tiles behind the last run, more units than
-    SMs (several tiles a CTA) and fewer, columns that fill no tile: against float64 from the same bfloat16 numbers.  K
+    SMs (several tiles a CTA) and fewer, columns that fill no tile; by the rule on 148 SMs the first three take tiles of 128 x
+    128, the others the persistent form, the last two with column tiles that run into the next group's rows, empty groups
+    between and behind, and more k-blocks than the ring has stages, the last one not whole: against float64 from the same bfloat16 numbers.  K
     products are added in float32 and the result is rounded to bfloat16 once: half a unit of 8 bits, at most 2^-8 of the value."""
     from aien_sovereign_core_mv_b200 import kernels as K_
     if form == "gated" and N % 16:
