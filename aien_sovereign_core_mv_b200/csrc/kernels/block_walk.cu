@@ -16,10 +16,22 @@
 //
 // The products run on the tensor cores (mma.sync tf32) with every float32 operand cut in two: x = hi + lo, hi the nearest
 // number of 11 bits, lo the rest, and x y = hi hi + hi lo + lo hi; what is dropped is 2^-22 of a product and has no sign
-// of its own.  tcgen05 would have to find the state in shared memory for every block's product; here the eight warps share
-// its rows and each keeps its own as accumulators: [16 columns] x [8 rows] fragments whose register order is the order of
-// the left operand once the rows of a fragment are counted 0 2 4 6 1 3 5 7 on both sides.  The update is accumulated from
-// zero and added to the decayed state by one float32 multiply-add, so the state is rounded once per block.
+// of its own.  The two small products have accumulators of their own: the tensor cores cut off what does not fit 24 bits
+// where a multiply-add rounds, which adds up where everything is of one sign (see bw_total).  tcgen05 would have to find the state in
+// shared memory for every block's product; here the eight warps share its rows and each keeps its own as accumulators:
+// [16 columns] x [8 rows] fragments whose register order is the order of the left operand once the rows of a fragment are
+// counted 0 2 4 6 1 3 5 7 on both sides.  The update is accumulated from zero and added to the decayed state by float32
+// multiply-adds, so the state is rounded once per block.  The decays' products are sums of two numbers until they are
+// written, and G_16 stays one: rounded, it would be off by the same factor in every block where the decay is constant.
+//
+// Relative error (2-norm) of the results and the last states against 64 bits, 2,048 tokens, and in brackets that of the
+// float32 kernels that go token by token or, for one decay per head, by chunks of 64:
+//   one decay per head, 1 - 2^-5 .. 1 - 2^-8          0.8e-7 and 0.8e-7  (1.7e-7 and 1.3e-7)
+//   one decay per head, 1 - 1e-4                      0.9e-7 and 1.7e-7  (2.7e-7 and 3.2e-7)
+//   duality, rows of silu, drawn step sizes           0.9e-7 and 1.0e-7  (0.9e-7 and 3.0e-7)
+//   delta rule, rows of silu, drawn decays            1.4e-7 and 1.4e-7  (2.1e-7 and 3.1e-7)
+//   delta rule, rows of either sign, decays 0.74 .. 1 1.3e-7 and 1.1e-7  (1.1e-7 and 0.8e-7)
+// With one accumulator, nothing added back and rounded products of decays the first two were 6.8e-7 and 2.3e-6.
 //
 // 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 148 us and 16 for the coefficients (603 token by
 // token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 110 and 6 us (540).
@@ -32,7 +44,8 @@ constexpr int BW_B = 16;                       // tokens of a block
 constexpr int BW_WARPS = 8;
 constexpr int BW_THREADS = 32 * BW_WARPS;
 constexpr int BW_LD = 20;                      // floats between rows of A and M: no bank twice in a quarter warp
-constexpr int BW_COEF = 2 * BW_B * BW_B + 2 * BW_B;      // A | M | G | G_16 / G_j per block and head
+constexpr int BW_TAIL = 2 * BW_B + 4;                     // G | G_16 / G_j | what G_16 lacks, padded
+constexpr int BW_COEF = 2 * BW_B * BW_B + BW_TAIL;       // A | M and the tail per block and head
 
 __device__ __forceinline__ void bw_split(float x, uint32_t& hi, uint32_t& lo) {
     hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
@@ -45,12 +58,24 @@ __device__ __forceinline__ void bw_mma(float (&c)[4], const uint32_t (&a)[4], co
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// c += a b, the small products first
-__device__ __forceinline__ void bw_mma3(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[2], const uint32_t (&bl)[2]) {
-    bw_mma(c, al, bh);
-    bw_mma(c, ah, bl);
+// c + d += a b, the small products in d
+__device__ __forceinline__ void bw_mma3(float (&c)[4], float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[2],
+                                        const uint32_t (&bl)[2]) {
+    bw_mma(d, al, bh);
+    bw_mma(d, ah, bl);
     bw_mma(c, ah, bh);
 }
+
+// a product of decays as the sum of two numbers
+struct BwDecay {
+    float h = 1.f, l = 0.f;
+    __device__ __forceinline__ void by(float g) {
+        const float p = h * g;
+        l = fmaf(l, g, fmaf(h, g, -p));
+        h = p;
+    }
+    __device__ __forceinline__ float times(float x) const { return fmaf(h, x, l * x); }
+};
 
 __device__ __forceinline__ void bw_cp16(float* dst, const float* src, bool in) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -75,6 +100,14 @@ struct BlockWalk {
 __device__ __forceinline__ int bw_first_block(const int* q_start, int s) { return q_start[s] / BW_B + s; }
 
 __device__ __forceinline__ float bw_silu(float z) { return z / (1.0f + expf(-z)); }
+
+// G_i from the product of the decays behind the block's first token, and for the last what its rounding lacks
+__device__ __forceinline__ void bw_write_decay(float* c, int i, BwDecay d, float g0) {
+    d.by(g0);
+    const float g = d.h + d.l;
+    c[512 + i] = g;
+    if (i == BW_B - 1) c[512 + 2 * BW_B] = d.l - (g - d.h);
+}
 
 // One CTA per (block, q/k head): its dot products once, then A, M and the decays of every head that shares the q/k head.
 // Its life is one chain (loads, silu, dot products, coefficients), so other CTAs have to fill it: without the delta rule,
@@ -144,18 +177,18 @@ block_coef_kernel(const BlockWalk a) {
         const float4* q4 = reinterpret_cast<const float4*>(sq + i * LDN);
         const float4* ki4 = reinterpret_cast<const float4*>(sk + i * LDN);
         const float4* kj4 = reinterpret_cast<const float4*>(sk + j * LDN);
-        float x0 = 0.f, x1 = 0.f, y0 = 0.f, y1 = 0.f;
+        float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f, y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
 #pragma unroll 4
         for (int c = 0; c < N / 4; ++c) {
             const float4 q = q4[c], b = kj4[c];
-            x0 = fmaf(q.x, b.x, x0); x1 = fmaf(q.y, b.y, x1); x0 = fmaf(q.z, b.z, x0); x1 = fmaf(q.w, b.w, x1);
+            x0 = fmaf(q.x, b.x, x0); x1 = fmaf(q.y, b.y, x1); x2 = fmaf(q.z, b.z, x2); x3 = fmaf(q.w, b.w, x3);
             if (DELTA) {
                 const float4 k = ki4[c];
-                y0 = fmaf(k.x, b.x, y0); y1 = fmaf(k.y, b.y, y1); y0 = fmaf(k.z, b.z, y0); y1 = fmaf(k.w, b.w, y1);
+                y0 = fmaf(k.x, b.x, y0); y1 = fmaf(k.y, b.y, y1); y2 = fmaf(k.z, b.z, y2); y3 = fmaf(k.w, b.w, y3);
             }
         }
-        dots[0][tid] = x0 + x1;
-        if (DELTA) dots[DELTA ? 1 : 0][tid] = y0 + y1;
+        dots[0][tid] = (x0 + x1) + (x2 + x3);
+        if (DELTA) dots[DELTA ? 1 : 0][tid] = (y0 + y1) + (y2 + y3);
     }
     __syncthreads();
     if (per * BW_B * 4 <= 256) {                                // few heads: a thread owns numbers (i, j), and its product of decays
@@ -163,27 +196,27 @@ block_coef_kernel(const BlockWalk a) {
             const int hh = u >> 8, i = (u >> 4) & 15, j = u & 15;
             float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF;
             const float wj = DELTA ? 1.f : sw[j * per + hh];
-            float ratio = 1.f;
-            for (int r = j + 1; r <= i; ++r) ratio *= sg[r * per + hh];
-            c[i * 16 + j] = i >= j ? ratio * dots[0][i * 16 + j] * wj : 0.f;
-            if (DELTA) sl[u] = i > j ? sw[i * per + hh] * ratio * dots[DELTA ? 1 : 0][i * 16 + j] : 0.f;
-            if (j == 0) c[512 + i] = sg[hh] * ratio;
-            if (i == BW_B - 1) c[512 + 16 + j] = ratio * wj;
+            BwDecay ratio;
+            for (int r = j + 1; r <= i; ++r) ratio.by(sg[r * per + hh]);
+            c[i * 16 + j] = i >= j ? ratio.times(dots[0][i * 16 + j]) * wj : 0.f;
+            if (DELTA) sl[u] = i > j ? ratio.times(dots[DELTA ? 1 : 0][i * 16 + j]) * sw[i * per + hh] : 0.f;
+            if (i == BW_B - 1) c[512 + 16 + j] = ratio.times(wj);
+            if (j == 0) bw_write_decay(c, i, ratio, sg[hh]);
         }
     } else {                                                    // a thread owns column j of one head's matrices: the product of the decays grows by one factor a row
         for (int u = tid; u < per * BW_B; u += 256) {
             const int hh = u >> 4, j = u & 15;
             float* c = a.coef + ((size_t)slot * a.heads + kvh * per + hh) * BW_COEF;
-            const float wj = DELTA ? 1.f : sw[j * per + hh], g0 = sg[hh];
-            float ratio = 1.f;
+            const float wj = DELTA ? 1.f : sw[j * per + hh];
+            BwDecay ratio;
 #pragma unroll
             for (int i = 0; i < BW_B; ++i) {
-                if (i > j) ratio *= sg[i * per + hh];
-                c[i * 16 + j] = i >= j ? ratio * dots[0][i * 16 + j] * wj : 0.f;
-                if (DELTA) sl[hh * 256 + i * 16 + j] = i > j ? sw[i * per + hh] * ratio * dots[DELTA ? 1 : 0][i * 16 + j] : 0.f;
-                if (j == 0) c[512 + i] = g0 * ratio;
+                if (i > j) ratio.by(sg[i * per + hh]);
+                c[i * 16 + j] = i >= j ? ratio.times(dots[0][i * 16 + j]) * wj : 0.f;
+                if (DELTA) sl[hh * 256 + i * 16 + j] = i > j ? ratio.times(dots[DELTA ? 1 : 0][i * 16 + j]) * sw[i * per + hh] : 0.f;
+                if (j == 0) bw_write_decay(c, i, ratio, sg[hh]);
             }
-            c[512 + 16 + j] = ratio * wj;
+            c[512 + 16 + j] = ratio.times(wj);
         }
     }
     if (!DELTA) return;
@@ -215,7 +248,7 @@ struct BwSmem {
     static constexpr int LDN = 64 * NT + 8;                     // floats between rows of q and k: a half warp's 8-byte reads meet no bank twice
     static constexpr int LDV = 16 * MT + 8, LDP = 16 * MT + 4;  // floats between rows of v and u, and of the partial sums
     static constexpr int QK = BW_B * LDN;
-    static constexpr int STAGE = 2 * QK + BW_B * LDV + 2 * BW_B * BW_LD + 2 * BW_B;     // q | k | v | A | M | G | G_16 / G_j
+    static constexpr int STAGE = 2 * QK + BW_B * LDV + 2 * BW_B * BW_LD + BW_TAIL;      // q | k | v | A | M | G | G_16 / G_j, what G_16 lacks
     static constexpr int PART = BW_WARPS * BW_B * LDP;
     static constexpr int U = BW_B * LDV;
     static constexpr int TOTAL = STAGES * STAGE + (1 + TURNS) * PART + TURNS * U;          // partial sums of p, and of r, and u
@@ -246,8 +279,16 @@ __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWal
         const int e = tid - 64 * MT - 64;
         bw_cp16(sA + BW_B * BW_LD + (e >> 2) * BW_LD + (e & 3) * 4, coef + 256 + e * 4, true);
     }
-    if (tid < 8) bw_cp16(sA + 2 * BW_B * BW_LD + tid * 4, coef + 512 + tid * 4, true);
+    if (tid < BW_TAIL / 4) bw_cp16(sA + 2 * BW_B * BW_LD + tid * 4, coef + 512 + tid * 4, true);
     asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// What the tensor cores cut off a sum lies between nothing and one unit of its 24 bits: on the average over mantissas 0.36 x
+// 2^-23 of it, and 0.54 x 2^-23 where the sum takes two steps, the first of half the size.  The mean is added back with the
+// small products; what is left has no sign.
+template <int STEPS>
+__device__ __forceinline__ float bw_total(float c, float d) {
+    return c + fmaf(c, (STEPS == 2 ? 0.54f : 0.36f) * 1.1920929e-7f, d);
 }
 
 // partial products S0^T x of a warp's rows, x the q or k rows of a block: [16 MT columns] x [16 tokens] into part[token][column]
@@ -255,28 +296,32 @@ template <int NT, int MT>
 __device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const uint32_t (&sh)[MT][NT][4], const uint32_t (&sl)[MT][NT][4],
                                             float* __restrict__ part, int row0, int g, int t) {
     using C = BwSmem<NT, MT, false>;
-    float acc[MT][2][4] = {};
+    constexpr int HALVES = 2 / MT;                              // of the tokens at a time: as many accumulators with 32 columns as with 16
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int h0 = 0; h0 < 2; h0 += HALVES) {
+        float acc[MT][HALVES][4] = {}, low[MT][HALVES][4] = {};
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const float2 v = *reinterpret_cast<const float2*>(x + (half * 8 + g) * C::LDN + row0 + nt * 8 + 2 * t);
-            uint32_t bh[2], bl[2];
-            bw_split(v.x, bh[0], bl[0]);
-            bw_split(v.y, bh[1], bl[1]);
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) bw_mma3(acc[mt][half], sh[mt][nt], sl[mt][nt], bh, bl);
-        }
+            for (int h = 0; h < HALVES; ++h) {
+                const float2 v = *reinterpret_cast<const float2*>(x + ((h0 + h) * 8 + g) * C::LDN + row0 + nt * 8 + 2 * t);
+                uint32_t bh[2], bl[2];
+                bw_split(v.x, bh[0], bl[0]);
+                bw_split(v.y, bh[1], bl[1]);
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+                for (int mt = 0; mt < MT; ++mt) bw_mma3(acc[mt][h], low[mt][h], sh[mt][nt], sl[mt][nt], bh, bl);
+            }
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float* p = part + (half * 8 + 2 * t) * C::LDP + mt * 16 + g;
-            p[0] = acc[mt][half][0];
-            p[C::LDP] = acc[mt][half][1];
-            p[8] = acc[mt][half][2];
-            p[C::LDP + 8] = acc[mt][half][3];
-        }
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h) {
+                float* p = part + ((h0 + h) * 8 + 2 * t) * C::LDP + mt * 16 + g;
+                p[0] = bw_total<NT>(acc[mt][h][0], low[mt][h][0]);
+                p[C::LDP] = bw_total<NT>(acc[mt][h][1], low[mt][h][1]);
+                p[8] = bw_total<NT>(acc[mt][h][2], low[mt][h][2]);
+                p[C::LDP + 8] = bw_total<NT>(acc[mt][h][3], low[mt][h][3]);
+            }
+    }
 }
 
 template <int LDP>
@@ -515,34 +560,37 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
         bw_read_out<NT, MT>(sq, sh, sl, parts_r + turn * C::PART + warp * BW_B * C::LDP, row0, g, tq);
         HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();     // u and the partial sums of r are there
         if (HELP) bw_arrive(BW_BAR_DONE + turn, 2 * BW_THREADS);
-        float up[MT][NT][4] = {};
+        uint32_t kh[2][NT][2], kl[2][NT][2];
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            const int ta = ks * 8 + tq;
-            const float w0 = suf[ta], w1 = suf[ta + 4];
-            uint32_t ah[MT][4], al[MT][4];
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                bw_split(u[ta * C::LDV + mt * 16 + g] * w0, ah[mt][0], al[mt][0]);
-                bw_split(u[ta * C::LDV + mt * 16 + g + 8] * w0, ah[mt][1], al[mt][1]);
-                bw_split(u[(ta + 4) * C::LDV + mt * 16 + g] * w1, ah[mt][2], al[mt][2]);
-                bw_split(u[(ta + 4) * C::LDV + mt * 16 + g + 8] * w1, ah[mt][3], al[mt][3]);
-            }
+        for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                uint32_t bh[2], bl[2];
-                bw_split(sk[ta * C::LDN + row0 + nt * 8 + g], bh[0], bl[0]);
-                bw_split(sk[(ta + 4) * C::LDN + row0 + nt * 8 + g], bh[1], bl[1]);
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt) bw_mma3(up[mt][nt], ah[mt], al[mt], bh, bl);
+                bw_split(sk[(ks * 8 + tq) * C::LDN + row0 + nt * 8 + g], kh[ks][nt][0], kl[ks][nt][0]);
+                bw_split(sk[(ks * 8 + tq + 4) * C::LDN + row0 + nt * 8 + g], kh[ks][nt][1], kl[ks][nt][1]);
             }
+        const float total = gam[BW_B - 1], rest = gam[2 * BW_B];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            float up[NT][4] = {}, low[NT][4] = {};
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const int ta = ks * 8 + tq;
+                const float w0 = suf[ta], w1 = suf[ta + 4];
+                const float* u0 = u + ta * C::LDV + mt * 16 + g;
+                uint32_t ah[4], al[4];
+                bw_split(u0[0] * w0, ah[0], al[0]);
+                bw_split(u0[8] * w0, ah[1], al[1]);
+                bw_split(u0[4 * C::LDV] * w1, ah[2], al[2]);
+                bw_split(u0[4 * C::LDV + 8] * w1, ah[3], al[3]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) bw_mma3(up[nt], low[nt], ah, al, kh[ks][nt], kl[ks][nt]);
+            }
+            if (!HELP && mt == MT - 1) results(t, b, 0);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[mt][nt][e] = fmaf(total, S[mt][nt][e], fmaf(rest, S[mt][nt][e], bw_total<2>(up[nt][e], low[nt][e])));
         }
-        if (!HELP) results(t, b, 0);
-        const float total = gam[BW_B - 1];
-#pragma unroll
-        for (int f = 0; f < MT * NT; ++f)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) S[f / NT][f % NT][e] = fmaf(total, S[f / NT][f % NT][e], up[f / NT][f % NT][e]);
         if (HELP) {
             b = b == 2 ? 0 : b + 1;
             turn ^= 1;
@@ -606,7 +654,7 @@ AIEN_API int aien_block_walk_supports(int heads, int G, int N, int V, int delta)
 // delta, else a factor on v; gates null: decay[heads] for every token.  skip (in skip_dt, or null): o += skip[h] v.
 // state: rows of state_stride floats, a head's matrix at s_off + h N V, [V][N] with state_vn, else [N][V].  Request s (tokens
 // q_start[s] .. q_start[s+1]) continues from slot slots[s], from zeros where its first position is 0.  out float32 [T, ldo].
-// scratch: float32, (T / 16 + S) * heads * 544 numbers (the blocks' coefficients) and with act T * (2 G N + heads V) more.
+// scratch: float32, (T / 16 + S) * heads * 548 numbers (the blocks' coefficients) and with act T * (2 G N + heads V) more.
 AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, int v_off, int act, const float* gates, long ldg, int g_off,
                              int w_off, const float* decay, int delta, const void* skip, int skip_dt, float* state, size_t state_stride,
                              size_t s_off, int state_vn, const int* slots, const int* q_start, const int* positions, float* out, long ldo,

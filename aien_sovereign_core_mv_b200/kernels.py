@@ -1905,8 +1905,8 @@ BLOCK_WALK_MIN_TOKENS = 32
 
 
 def block_walk_scratch(num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, act: bool = False) -> int:
-    """float32 numbers of scratch :func:`block_walk` needs: 544 a block and head, and with ``act`` the rows after it."""
-    return (num_tokens // 16 + num_seqs) * heads * 544 + (num_tokens * (2 * qk_heads * dim + heads * vdim) if act else 0)
+    """float32 numbers of scratch :func:`block_walk` needs: 548 a block and head, and with ``act`` the rows after it."""
+    return (num_tokens // 16 + num_seqs) * heads * 548 + (num_tokens * (2 * qk_heads * dim + heads * vdim) if act else 0)
 
 
 def block_walk(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: Optional[torch.Tensor], g_off: int, w_off: int,

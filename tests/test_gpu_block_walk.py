@@ -74,6 +74,47 @@ def test_block_walk_follows_the_recurrence(form, heads, G, N, V, lens, slow):
     assert torch.equal(dev[keep].cpu(), state[keep]) and torch.equal(dev[:, :s_off].cpu(), state[:, :s_off]) and torch.equal(dev[:, -extra:].cpu(), state[:, -extra:])
 
 
+@pytest.mark.parametrize("form", ["linear", "duality", "delta"])
+@pytest.mark.parametrize("slow", [False, True])
+def test_long_portions_lose_no_more_than_token_by_token(form, slow):
+    """2,048 tokens whose keys, queries and values are mostly of one sign, so that a rounding that always cuts off would add
+    up, under decays that hardly decay (one for all tokens, whose products are the same in every block) and ordinary ones:
+    the state is rounded once a block, 128 times, at 2^-25 on the average and either way (3.4e-7 together), and no more
+    than as much again comes from what is added to it; relative 2-norms."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    g_ = torch.Generator(device="cuda").manual_seed(7)
+    T, heads, G, N, V = 2048, 4, {"linear": 4, "duality": 1, "delta": 2}[form], 128, 64
+    silu = lambda x: x * torch.sigmoid(x)
+    GN = G * N
+    rows = torch.randn(T, 2 * GN + heads * V, generator=g_, device="cuda")
+    if form != "linear":
+        rows = silu(rows)
+    if form == "delta":
+        for at in (0, GN):
+            part = rows[:, at:at + GN].view(T, G, N)
+            rows[:, at:at + GN] = (part / part.norm(dim=-1, keepdim=True)).reshape(T, GN)
+    span = 1e-4 if slow else 0.1
+    gates = torch.cat([1.0 - span * torch.rand(T, heads, generator=g_, device="cuda"), torch.rand(T, heads, generator=g_, device="cuda")], 1)
+    decay = 1.0 - span * (0.1 + 0.9 * torch.rand(heads, generator=g_, device="cuda"))
+    act = form == "linear"
+    state, out = torch.zeros(1, heads * N * V).cuda(), torch.zeros(T, heads * V).cuda()
+    blocks = torch.empty(K.block_walk_scratch(T, 1, heads, G, N, V, act)).cuda()
+    assert K.block_walk(rows, 0, GN, 2 * GN, None if act else gates, 0, -1 if act else heads, decay if act else None, state, 0, i32([0]), i32([0, T]),
+                        i32(list(range(T))), out, 1, heads, G, N, V, blocks, delta=form == "delta", act=act)
+    a = silu(rows.double()) if act else rows.double()
+    q, k = (a[:, at:at + GN].view(T, G, N).repeat_interleave(heads // G, dim=1) for at in (0, GN))
+    v = a[:, 2 * GN:].view(T, heads, V)
+    S, want = torch.zeros(heads, N, V, dtype=torch.float64, device="cuda"), []
+    for t in range(T):
+        S = (decay if act else gates[t, :heads]).double()[:, None, None] * S
+        u = v[t] - torch.einsum("hnv,hn->hv", S, k[t]) if form == "delta" else v[t]
+        S = S + k[t][:, :, None] * (u if act else gates[t, heads:].double()[:, None] * u)[:, None]
+        want.append(torch.einsum("hnv,hn->hv", S, q[t]))
+    rel = lambda x, y: float((x.double().flatten() - y.flatten()).norm() / y.norm())
+    assert rel(out, torch.stack(want)) <= 7e-7 and rel(state, S) <= 7e-7
+
+
 def test_many_heads_over_one_group_walk_by_blocks():
     """The duality form needs no 16 x 16 system a head, so heads that are too many for the delta rule are not for it."""
     from aien_sovereign_core_mv_b200 import kernels as K
