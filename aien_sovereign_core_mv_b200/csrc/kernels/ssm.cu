@@ -428,8 +428,7 @@ ssd_scan_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, in
 
 // out[t] = the three bfloat16 parts of x[t]'s numbers, part by part: x = p0 + p1 + p2 up to 2^-25 of x (each part rounds
 // what the ones before leave).  With the weights three times side by side a product on the tensor cores then has float32
-// rows on the left: the step sizes' product of 2,048 tokens, 4,096 x 128 bfloat16 weights, took 101 us on the CUDA cores
-// and takes 23 with this launch (2.6 of it).  x may come as partial products over ranges of K: the product that makes it has
+// rows on the left (parts_product.cu).  x may come as partial products over ranges of K: the product that makes it has
 // few columns (160 over 4,096: 32 tiles at 2,048 tokens, 28 us) and is cut over the whole GPU (14 us, and 1.7 more here).
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, long ldx, int P, size_t part_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ rest,

@@ -194,6 +194,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
         "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, I, I, P, P],
         "aien_split_rows": [P, L, I, c_size_t, P, P, I, I, I, P],
+        "aien_parts_product": [P, P, L, P, L, I, I, I, P],
         "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
         "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, P, P],
         "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, P],
@@ -2015,7 +2016,7 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
 
 def split_rows(x: torch.Tensor, out: torch.Tensor, rest: Optional[torch.Tensor] = None) -> None:
     """x float32 [T, n] as the sum of three bfloat16 rows side by side, out [T, 3 n] (up to 2^-25 of x): the left operand of
-    a tensor-core product that must not round its float32 rows, with the weights three times side by side.  x may also be
+    :func:`parts_product`, which does not round its float32 rows.  x may also be
     float32 partial products [P, T, *], added first; ``rest`` float32 [T, m]: the m columns behind the n, as they are."""
     _dev(x, out, rest)
     T, n, m = x.shape[-2], out.shape[1] // 3, 0 if rest is None else rest.shape[1]
@@ -2024,6 +2025,16 @@ def split_rows(x: torch.Tensor, out: torch.Tensor, rest: Optional[torch.Tensor] 
     assert out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == (T, 3 * n)
     assert rest is None or (rest.dtype == torch.float32 and rest.is_contiguous() and rest.shape[0] == T)
     _check(lib().aien_split_rows(_p(x), x.stride(-2), parts, part_stride, _p(out), _p(rest), T, n, m, _stream()), "split_rows")
+
+
+def parts_product(parts: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """out = x . w^T for float32 rows x in the three parts of :func:`split_rows`, w bfloat16 [N, n], n a multiple of 8: on the
+    tensor cores, with the rounding of float32 multiply-adds (out float32)."""
+    _dev(parts, w, out)
+    (T, n3), (N, n) = parts.shape, w.shape
+    assert parts.dtype == torch.bfloat16 and parts.is_contiguous() and n3 == 3 * n and w.dtype == torch.bfloat16 and w.stride(1) == 1
+    assert out.dtype == torch.float32 and out.stride(1) == 1 and tuple(out.shape) == (T, N)
+    _check(lib().aien_parts_product(_p(parts), _p(w), w.stride(0), _p(out), out.stride(0), T, N, n, _stream()), "parts_product")
 
 
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,

@@ -85,7 +85,7 @@ class SelectiveScan(Mixer):
         if self.inner <= 0 or self.dt_rank <= 0:
             raise ValueError("inner and dt_rank must be positive")
         self.conv_floats = (self.taps - 1) * self.inner
-        self.w_in = self.w_x = self.w_dt = self.w_dt3 = self.w_o = self.conv = self.conv_b = self.dt_b = self.A = self.D = None
+        self.w_in = self.w_x = self.w_dt = self.w_o = self.conv = self.conv_b = self.dt_b = self.A = self.D = None
 
     def param_shapes(self):
         H, I, N, R = self.hidden_size, self.inner, self.state, self.dt_rank
@@ -96,8 +96,6 @@ class SelectiveScan(Mixer):
     def bind(self, tensors):
         self.w_in, self.w_x = tensors["in_proj"].contiguous(), tensors["x_proj"].contiguous()
         self.w_dt, self.w_o = tensors["dt_proj"].contiguous(), tensors["o_proj"].contiguous()
-        if self.w_dt.dtype == torch.bfloat16 and self.dt_rank % 8 == 0:
-            self.w_dt3 = torch.cat([self.w_dt] * 3, dim=1).contiguous()          # beside float32 rows in three bfloat16 parts
         self.conv, self.conv_b = tensors["conv"].contiguous(), tensors["conv_bias"].float().contiguous()
         self.dt_b, self.D = tensors["dt_bias"].float().contiguous(), tensors["D"].float().contiguous()
         self.A = (-torch.exp(tensors["A_log"].float())).contiguous()
@@ -122,7 +120,7 @@ class SelectiveScan(Mixer):
         K.conv_act(proj, 0, I, self.conv, self.conv_b, self.taps, "silu", state, group.slot_map, ctx.seq_of_token, ctx.q_start,
                    ctx.positions, x, xa if xa is not x else None)
         # dt | B | C: few columns over a long K, so in ranges of K where tiles alone leave SMs idle; split_rows adds them
-        in_three = ctx.dtype == torch.bfloat16 and self.w_dt3 is not None
+        in_three = ctx.dtype == torch.bfloat16 == self.w_dt.dtype and R % 8 == 0 and self.w_dt.data_ptr() % 16 == 0
         xp = linear(ctx, xa, self.w_x, out_dtype=torch.float32, may_defer_sum=in_three)
         bc, b_off = xp, R
         if in_three:                                                                    # float32 step sizes into the softplus
@@ -132,7 +130,8 @@ class SelectiveScan(Mixer):
                 K.split_rows(xp, parts, bc)
             else:
                 K.split_rows(xp[:, :R], parts)
-            dtz = linear(ctx, parts, self.w_dt3, out_dtype=torch.float32)
+            dtz = ws.take((T, I), torch.float32)
+            K.parts_product(parts, self.w_dt, dtz)
         else:
             dtz = linear(ctx, xp[:, :R], self.w_dt, out_dtype=torch.float32)
         y = ws.take((T, I), ctx.dtype)

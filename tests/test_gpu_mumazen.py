@@ -413,6 +413,28 @@ def test_selective_scan_in_the_segments_of_few_channels(inner, N, lens, dtype):
     H.assert_close(S, last, 1e-5, "states")
 
 
+@pytest.mark.parametrize("T,n,N", [(1, 8, 1), (127, 24, 63), (128, 32, 64), (129, 40, 66), (300, 128, 130), (5, 136, 257), (2, 256, 64)])
+@pytest.mark.parametrize("one_sign", [False, True])
+def test_product_of_three_parts_rounds_like_float32(T, n, N, one_sign):
+    """Edges of the tiles and of the steps over K, strided weights and results.  An entry is n / 16 float32 additions of sums
+    cut off at 24 bits, and the parts' own 2^-25: (n / 16 + 2) units of 2^-23 of the sum of magnitudes at the most, and as a
+    relative 2-norm what the multiply-adds of the product on the CUDA cores lose, or half as much again."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(T + n + N)
+    x, w = torch.randn(T, n, generator=g).cuda(), torch.randn(N, n + 8, generator=g).to(torch.bfloat16).cuda()[:, 8:]
+    if one_sign:
+        x, w = x.abs(), torch.randn(N, n, generator=g).abs().to(torch.bfloat16).cuda()
+    parts, store, plain = torch.empty(T, 3 * n, dtype=torch.bfloat16).cuda(), torch.full((T + 1, N + 3), 7.0).cuda(), torch.empty(T, N).cuda()
+    K.split_rows(x, parts)
+    K.parts_product(parts, w, store[:T, :N])
+    K.gemm_simple(x, w, plain)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert float(((store[:T, :N] - want).abs() / size).max()) <= (n / 16 + 2) * 2.0 ** -23
+    assert float((store[:, N:] - 7.0).abs().max()) == 0.0 and float((store[T] - 7.0).abs().max()) == 0.0
+    rel = lambda y: float((y.double() - want).norm() / want.norm())
+    assert rel(store[:T, :N]) <= max(1.5 * rel(plain), 2.0 ** -23)
+
+
 @pytest.mark.parametrize("T,n,N", [(1, 8, 16), (5, 24, 40), (130, 64, 72)])
 def test_product_of_float32_rows_in_three_parts(T, n, N):
     """The three parts add up to the row (2^-25 of it: each leaves at most half a unit of 8 bits), and the tensor-core
