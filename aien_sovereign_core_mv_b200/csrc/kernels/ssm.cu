@@ -449,8 +449,9 @@ split_rows_kernel(const float* __restrict__ x, long ldx, int P, size_t part_stri
         rest[(size_t)t * m + c - n] = v;
         return;
     }
-    const __nv_bfloat16 p0 = __float2bfloat16_rn(v);
-    const float r0 = v - __bfloat162float(p0);
+    __nv_bfloat16 p0 = __float2bfloat16_rn(v);
+    if (fabsf(__bfloat162float(p0)) == INFINITY && fabsf(v) < INFINITY) p0 = __float2bfloat16_rz(v);        // the largest numbers round beyond the type
+    const float r0 = fabsf(v) < INFINITY ? v - __bfloat162float(p0) : 0.f;                                  // an infinity (or NaN) is whole in its first part
     const __nv_bfloat16 p1 = __float2bfloat16_rn(r0);
     __nv_bfloat16* o = out + (size_t)t * 3 * n + c;
     o[0] = p0;

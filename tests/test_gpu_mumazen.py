@@ -413,6 +413,26 @@ def test_selective_scan_in_the_segments_of_few_channels(inner, N, lens, dtype):
     H.assert_close(S, last, 1e-5, "states")
 
 
+def test_float32_rows_beyond_bfloat16_in_three_parts():
+    """Infinities stay what they are, in the parts and in the product over them; the largest numbers stay finite."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    x = torch.ones(40, 8)
+    x[1, 2], x[3, 4], x[5, 6], x[7, 0] = float("inf"), -float("inf"), float("nan"), 3.4028e38
+    parts = torch.zeros(40, 24, dtype=torch.bfloat16).cuda()
+    K.split_rows(x.cuda(), parts)
+    back = parts.double().cpu().view(40, 3, 8).sum(1)
+    odd = ~torch.isfinite(x)
+    assert torch.equal(back[odd].nan_to_num(nan=7.0), x.double()[odd].nan_to_num(nan=7.0))
+    assert float(((back - x.double()).abs() / x.double().abs())[~odd].max()) <= 2.0 ** -24
+    w = (0.01 * torch.rand(16, 8, generator=torch.Generator().manual_seed(2)) + 0.001).to(torch.bfloat16).cuda()
+    out = torch.zeros(40, 16).cuda()
+    K.parts_product(parts, w, out)
+    want = x.double().cuda() @ w.double().T
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+    ok = torch.isfinite(want)
+    assert float(((out - want).abs() / want.abs())[ok].max()) <= 4 * 2.0 ** -23              # no sums of two signs
+
+
 @pytest.mark.parametrize("T,n,N", [(1, 8, 1), (127, 24, 63), (128, 32, 64), (129, 40, 66), (300, 128, 130), (5, 136, 257), (2, 256, 64)])
 @pytest.mark.parametrize("one_sign", [False, True])
 def test_product_of_three_parts_rounds_like_float32(T, n, N, one_sign):
