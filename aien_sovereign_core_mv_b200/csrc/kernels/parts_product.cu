@@ -8,7 +8,10 @@
 // would have to pass every such piece through tensor memory; mma.sync leaves it in registers.
 //
 // A CTA makes 128 x 64 results, its eight warps 32 x 32 each, in steps of 32 columns of K through three stages of shared
-// memory; 128 registers and 105 KB, so two CTAs an SM take turns at waiting.
+// memory; 128 registers and 105 KB, so two CTAs an SM take turns at waiting.  What bounds it is the rate of mma.sync and the
+// additions beside it.  Relative error and time on a B200, in brackets of multiply-adds on the CUDA cores and of a tcgen05
+// accumulator: 2,048 x 4,096 x 128 0.62e-7, 31 us (0.93e-7, 101 us; 6.6e-7, 12 us); 2,048 x 8,192 x 256 0.80e-7, 107 us
+// (1.07e-7, 381 us; 12.8e-7, 31 us); one row of 4,096 x 128 6.3 us (10.4; 6.3).
 #include "common.cuh"
 
 namespace aien {

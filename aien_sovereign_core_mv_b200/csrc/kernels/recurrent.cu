@@ -1,7 +1,8 @@
 // Recurrent mixers whose state has a fixed size per request: linear attention with a per-head
 // decay, and a gated recurrence over channels.  The state is float32 and lives in a state slot
-// of the cache ([slots, ...]); everything that enters a recurrence (decay powers, gates,
-// candidates, the state itself, the products with it) is float32 in both engine precisions.
+// of the cache ([slots, ...]); everything that enters a recurrence here (decay powers, gates,
+// candidates, the state itself, the products with it) is float32 in both engine precisions.  (Linear
+// attention over portions in a bfloat16 engine goes through block_walk.cu.)
 //
 // The rules of a state slot, all of them on the device: the portion of request s of the step is
 // the tokens q_start[s] .. q_start[s+1]; its slot is slot_map[s]; a portion whose first token has
