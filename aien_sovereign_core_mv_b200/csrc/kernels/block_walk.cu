@@ -33,8 +33,10 @@
 //   delta rule, rows of either sign, decays 0.74 .. 1 1.3e-7 and 1.1e-7  (1.1e-7 and 0.8e-7)
 // With one accumulator, nothing added back and rounded products of decays the first two were 6.8e-7 and 2.3e-6.
 //
-// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 148 us and 16 for the coefficients (603 token by
-// token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 110 and 6 us (540).
+// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 152 us and 16 for the coefficients (603 token by
+// token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 122 and 6 us (540); linear attention, 1,900
+// tokens of two requests, 16 heads of 128 x 128: 95 and 29 us (237 by chunks).  What bounds the walk is a block's chain of loads,
+// products and barriers.  (The choices of a form below were measured at 148, 110 and 86 us, with one accumulator a sum.)
 #include "common.cuh"
 #include <math.h>
 
@@ -94,6 +96,7 @@ struct BlockWalk {
     const int* slots; const int* q_start; const int* positions;
     float* out; long ldo;
     int T, S, heads, G, N, V;
+    int alone;                               // requests of one token that are served elsewhere: left out here
 };
 
 // the request whose blocks include block slot b; request s's blocks start at q_start[s] / 16 + s
@@ -126,7 +129,7 @@ block_coef_kernel(const BlockWalk a) {
     }
     const int s = lo, t0 = a.q_start[s] + (slot - bw_first_block(a.q_start, s)) * BW_B, end = a.q_start[s + 1];
     const int n = end - t0 < BW_B ? end - t0 : BW_B;
-    if (n <= 0) return;
+    if (n <= 0 || (a.alone && end - a.q_start[s] == 1)) return;
     const int per = a.heads / a.G, N = a.N, LDN = N + 4;
     float* sq = bw_smem;                                        // [16][N + 4]
     float* sk = sq + BW_B * LDN;
@@ -413,7 +416,7 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
     float* parts_r = part_p + C::PART;
     float* us = parts_r + C::TURNS * C::PART;
     const int s = blockIdx.z, h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
-    if (t1 <= t0) return;
+    if (t1 <= t0 || (a.alone && t1 - t0 == 1)) return;
     const int tid = threadIdx.x & (BW_THREADS - 1), warp = tid >> 5, lane = tid & 31;
     const int col0 = blockIdx.x * COLS, cols = a.V - col0 < COLS ? a.V - col0 : COLS;
 
@@ -634,7 +637,7 @@ static int dispatch_block_walk(const BlockWalk& a, cudaStream_t stream) {
     int sms = 148, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     if (!a.delta) return launch_block_walk<NT, 1, false, false>(a, stream);
-    if ((long)((a.V + 15) / 16) * a.heads * a.S <= sms) return launch_block_walk<NT, 1, true, true>(a, stream);
+    if ((long)((a.V + 15) / 16) * a.heads * (a.S - a.alone) <= sms) return launch_block_walk<NT, 1, true, true>(a, stream);
     return a.V <= 16 ? launch_block_walk<NT, 1, true, false>(a, stream) : launch_block_walk<NT, 2, true, false>(a, stream);
 }
 
@@ -654,17 +657,18 @@ AIEN_API int aien_block_walk_supports(int heads, int G, int N, int V, int delta)
 // delta, else a factor on v; gates null: decay[heads] for every token.  skip (in skip_dt, or null): o += skip[h] v.
 // state: rows of state_stride floats, a head's matrix at s_off + h N V, [V][N] with state_vn, else [N][V].  Request s (tokens
 // q_start[s] .. q_start[s+1]) continues from slot slots[s], from zeros where its first position is 0.  out float32 [T, ldo].
+// alone: how many requests bring one token and are served elsewhere; 0: none is left out.
 // scratch: float32, (T / 16 + S) * heads * 548 numbers (the blocks' coefficients) and with act T * (2 G N + heads V) more.
 AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, int v_off, int act, const float* gates, long ldg, int g_off,
                              int w_off, const float* decay, int delta, const void* skip, int skip_dt, float* state, size_t state_stride,
                              size_t s_off, int state_vn, const int* slots, const int* q_start, const int* positions, float* out, long ldo,
-                             int T, int S, int heads, int G, int N, int V, float* scratch, cudaStream_t stream) {
+                             int T, int S, int heads, int G, int N, int V, int alone, float* scratch, cudaStream_t stream) {
     if (S <= 0 || T <= 0) return 0;
     if (!aien_block_walk_supports(heads, G, N, V, delta) || S > 65535 || G > 65535 || scratch == nullptr || (gates == nullptr && decay == nullptr)) return AIEN_E_SHAPE;
     if ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(scratch)) & 15 || (ld | q_off | k_off | v_off) & 3) return AIEN_E_ALIGN;
     const long blocks = T / BW_B + S, coefs = blocks * heads * BW_COEF;
     BlockWalk a{rows, ld, q_off, k_off, v_off, gates, ldg, g_off, w_off, decay, scratch + coefs, 2L * G * N + (long)heads * V, act, delta, scratch,
-                skip, skip_dt, state, state_stride, s_off, state_vn, slots, q_start, positions, out, ldo, T, S, heads, G, N, V};
+                skip, skip_dt, state, state_stride, s_off, state_vn, slots, q_start, positions, out, ldo, T, S, heads, G, N, V, alone};
     const int per = heads / G, smem = 4 * (2 * BW_B * (N + 4) + 2 * BW_B * per + (delta ? 256 * per : 0));
     auto coef = delta ? block_coef_kernel<true> : block_coef_kernel<false>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(coef, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AIEN_E_STATE;

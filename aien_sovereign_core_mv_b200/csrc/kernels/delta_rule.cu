@@ -117,13 +117,13 @@ __global__ void __launch_bounds__(DR_THREADS)
 delta_rule_kernel(const float* __restrict__ qkv, long ld, int q_off, int k_off, int v_off, const float* __restrict__ gb, long ldgb,
                   float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slot_map,
                   const int* __restrict__ q_start, const int* __restrict__ positions, float* __restrict__ o, long ldo,
-                  int heads, int G, int D, int V) {
+                  int heads, int G, int D, int V, int longest) {
     using C = DeltaCfg<DPT, RS>;
     constexpr int N4 = DPT / 4;
     __shared__ __align__(16) float bufs[2][C::TC * C::ROW];
     const int s = blockIdx.z, h = blockIdx.y, kvh = h / (heads / G);
     const int t0 = q_start[s], t1 = q_start[s + 1];
-    if (t1 <= t0) return;
+    if (t1 <= t0 || t1 - t0 > longest) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rs = lane / C::CW, cw = lane % C::CW;
     const int col0 = blockIdx.x * C::COLS, cl = warp * C::CW + cw, col = col0 + cl;
@@ -275,22 +275,24 @@ using namespace aien;
 template <int DPT, int RS>
 static void launch_delta_rule(cudaStream_t stream, const float* qkv, long ld, int q_off, int k_off, int v_off, const float* gb,
                               long ldgb, float* state, size_t state_stride, size_t s_off, const int* slot_map, const int* q_start,
-                              const int* positions, float* o, long ldo, int S, int heads, int G, int D, int V) {
+                              const int* positions, float* o, long ldo, int S, int heads, int G, int D, int V, int longest) {
     constexpr int COLS = DeltaCfg<DPT, RS>::COLS;
     dim3 grid((V + COLS - 1) / COLS, heads, S);
     delta_rule_kernel<DPT, RS><<<grid, DR_THREADS, 0, stream>>>(qkv, ld, q_off, k_off, v_off, gb, ldgb, state, state_stride, s_off,
-                                                                slot_map, q_start, positions, o, ldo, heads, G, D, V);
+                                                                slot_map, q_start, positions, o, ldo, heads, G, D, V, longest);
 }
 
 // qkv float32 [T, ld]: prepared q (G*D) at q_off, k (G*D) at k_off, v (heads*V) at v_off; gb float32 [T, ldgb]: decay
 // of head h at column h, beta at heads + h.  state: float32 rows of state_stride numbers per slot, S [heads][D][V] at
 // s_off.  Request s of the step (tokens q_start[s] .. q_start[s+1]) continues from slot slot_map[s].  o float32 [T, ldo].
+// longest > 0: requests that bring more tokens are served elsewhere and left alone here.
 AIEN_API int aien_delta_rule(const float* qkv, long ld, int q_off, int k_off, int v_off, const float* gb, long ldgb, float* state,
                              size_t state_stride, size_t s_off, const int* slot_map, const int* q_start, const int* positions,
-                             float* o, long ldo, int S, int heads, int G, int D, int V, cudaStream_t stream) {
+                             float* o, long ldo, int S, int heads, int G, int D, int V, int longest, cudaStream_t stream) {
     if (S <= 0) return 0;
+    if (longest <= 0) longest = 0x7fffffff;
     if (heads <= 0 || G <= 0 || heads % G || D <= 0 || D > 256 || V <= 0 || S > 65535 || heads > 65535) return AIEN_E_SHAPE;
-#define DR_CASE(N, R) launch_delta_rule<N, R>(stream, qkv, ld, q_off, k_off, v_off, gb, ldgb, state, state_stride, s_off, slot_map, q_start, positions, o, ldo, S, heads, G, D, V)
+#define DR_CASE(N, R) launch_delta_rule<N, R>(stream, qkv, ld, q_off, k_off, v_off, gb, ldgb, state, state_stride, s_off, slot_map, q_start, positions, o, ldo, S, heads, G, D, V, longest)
     if (D <= 16) DR_CASE(4, 4);
     else if (D <= 32) DR_CASE(8, 4);
     else if (D <= 64) DR_CASE(8, 8);

@@ -13,9 +13,12 @@
 //
 // The state of request s lives in row slot_map[s] of `state` (rows of state_stride floats, the recurrence's part from
 // s_off on); a portion whose first token has position 0 starts from zeros.  A few neighbouring lanes own a channel (or a
-// column of a head's state), keep its N state values in registers between them and walk the portion's tokens in order, so
-// a token's result depends only on the tokens before it, never on what else is in the batch.
-// Everything here is float32 in both engine precisions; only the result leaves in the compute dtype.
+// column of a head's state), keep its N state values in registers between them and walk the portion's tokens in order: a
+// token's result depends only on the tokens before it.  The order of the float32 additions in it may depend on the step: the
+// scan has eight or sixteen lanes a channel by the channels of all its requests, a step of single tokens four, and whether
+// portions are cut into segments goes by the step's size too.
+// Everything here is float32 in both engine precisions; only the result leaves in the compute dtype, and where that is
+// bfloat16 the scan's decays come from the special-function unit (see decay_exp).
 //
 // The portion-parallel forms cut a portion into segments that run side by side: every segment first runs from a zero
 // state and records the product of its decays and its end state; the segments' starting states then follow one from
@@ -52,8 +55,9 @@ struct Segments {
 //     step size (softplus) and its product with x before, the sum over a channel's lanes, the skip and the gate after;
 //   * inside the walk, eight tokens at a time, only one multiply-add a state value depends on the token before.
 // 2,048 tokens of 4,096 channels with 16 states each, one request, B200: 764 us, and 26 us for the step sizes, with the
-// rows fetched into registers four tokens ahead; 137 us so
+// rows fetched into registers four tokens ahead; 147 us so, 7 of them the gate's exponential and division
 // (31 instructions a token and warp, of which half a dozen in the prologue and epilogue of a stage; 16 lanes: 180 us, 4: 267 us).
+// With few channels a portion is cut into segments (see kernels.selective_scan_segments).
 template <int LANES, int CH>
 struct ScanCfg {
     static constexpr int NP = LANES * CH;
@@ -296,6 +300,7 @@ segment_combine_kernel(float* __restrict__ state, size_t state_stride, size_t s_
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= lanes) return;
     const int t0 = q_start[s], n_tok = q_start[s + 1] - t0;
+    if (n_tok <= 0) return;
     const int used = (n_tok + sg.seg_len - 1) / sg.seg_len;
     const size_t seg0 = (size_t)(t0 / sg.seg_len + s);
     float* slot = state + (size_t)slots[s] * state_stride + s_off + i;
@@ -333,7 +338,7 @@ __global__ void __launch_bounds__(SSD_THREADS)
 ssd_scan_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, int c_off,
                 const float* __restrict__ steps, const void* __restrict__ D, int pdt, float* __restrict__ state, size_t state_stride, size_t s_off,
                 const int* __restrict__ slots, const int* __restrict__ q_start, const int* __restrict__ positions,
-                float* __restrict__ y_out, long ldy, int heads, int V, int G, int N, Segments sg) {
+                float* __restrict__ y_out, long ldy, int heads, int V, int G, int N, Segments sg, int longest) {
     const int s = blockIdx.y, gid = blockIdx.x * SSD_THREADS + threadIdx.x;
     const int cols = heads * V;
     const bool live = gid / LANES < cols;
@@ -341,6 +346,7 @@ ssd_scan_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, in
     const int h = col / V, g = h / (heads / G), n0 = ln * CH;
     int t0 = q_start[s];
     int t1 = q_start[s + 1];
+    if (t1 <= t0 || t1 - t0 > longest) return;
     const bool fresh = positions[t0] == 0;
     const int seg = sg.mode == 0 ? 0 : blockIdx.z;
     const size_t seg0 = sg.mode == 0 ? 0 : (size_t)(t0 / sg.seg_len + s);
@@ -577,7 +583,7 @@ AIEN_API int aien_ssd_steps(const float* dtr, long lddt, const float* A, const v
 struct SsdArgs {
     const float* xbc; long ld; int x_off, b_off, c_off; const float* dtr; long lddt; const float* A; const void* dt_bias; const void* D;
     int p_dt; float* state; size_t state_stride, s_off; const int* slots; const int* q_start; const int* positions; float* y; long ldy;
-    int T, S, heads, V, G, N; Segments sg; float* steps; cudaStream_t stream;
+    int T, S, heads, V, G, N; Segments sg; int longest; float* steps; cudaStream_t stream;
 };
 
 template <int LANES, int CH, int U, bool VEC>
@@ -589,26 +595,27 @@ static void launch_ssd_scan(const SsdArgs& a) {
     const dim3 grid(gx, a.S, sg.mode == 0 ? 1 : sg.nseg);
     ssd_steps_kernel<<<(unsigned)(((long)a.T * a.heads + 255) / 256), 256, 0, a.stream>>>(a.dtr, a.lddt, a.A, a.dt_bias, a.p_dt, a.steps, a.T, a.heads);
     kern<<<grid, SSD_THREADS, 0, a.stream>>>(a.xbc, a.ld, a.x_off, a.b_off, a.c_off, a.steps, a.D, a.p_dt, a.state,
-                                             a.state_stride, a.s_off, a.slots, a.q_start, a.positions, a.y, a.ldy, a.heads, a.V, a.G, a.N, sg);
+                                             a.state_stride, a.s_off, a.slots, a.q_start, a.positions, a.y, a.ldy, a.heads, a.V, a.G, a.N, sg, a.longest);
     if (sg.mode == 0) return;
     const size_t lanes = (size_t)a.heads * a.N * a.V;
     segment_combine_kernel<<<dim3((unsigned)((lanes + 255) / 256), a.S), 256, 0, a.stream>>>(a.state, a.state_stride, a.s_off, a.slots, a.q_start,
                                                                                              a.positions, sg, lanes);
     sg.mode = 2;
     kern<<<grid, SSD_THREADS, 0, a.stream>>>(a.xbc, a.ld, a.x_off, a.b_off, a.c_off, a.steps, a.D, a.p_dt, a.state,
-                                             a.state_stride, a.s_off, a.slots, a.q_start, a.positions, a.y, a.ldy, a.heads, a.V, a.G, a.N, sg);
+                                             a.state_stride, a.s_off, a.slots, a.q_start, a.positions, a.y, a.ldy, a.heads, a.V, a.G, a.N, sg, a.longest);
 }
 
 // xbc [T, ld] (after convolution and silu): x (heads * V) at x_off, B (G * N) at b_off, C (G * N) at c_off; dtr [T, lddt]
 // the raw step sizes, one per head; A float32 [heads] (positive rates exp(A_log)); dt_bias and D [heads] in p_dt;
 // y float32 [T, ldy]; N <= 256; steps: float32 scratch of T * 2 * heads numbers (the step sizes and decays of the step's
 // tokens).  The slot holds S as [heads][V][N].  Segments as for aien_selective_scan, with heads * N * V state values per
-// request.
+// request.  longest > 0: requests that bring more tokens are served elsewhere and left alone here (but for their steps).
 AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int c_off, const float* dtr, long lddt, const float* A,
                            const void* dt_bias, const void* D, int p_dt, float* state, size_t state_stride, size_t s_off,
                            const int* slots, const int* q_start, const int* positions, float* y, long ldy, int T, int S, int heads, int V,
-                           int G, int N, int seg_len, int nseg, float* scratch, float* steps, cudaStream_t stream) {
+                           int G, int N, int seg_len, int nseg, float* scratch, float* steps, int longest, cudaStream_t stream) {
     if (S <= 0 || T <= 0) return 0;
+    if (longest <= 0) longest = 0x7fffffff;
     if (heads <= 0 || V <= 0 || G <= 0 || heads % G || N <= 0 || N > 256 || S > 65535 || nseg > 65535 || steps == nullptr) return AIEN_E_SHAPE;
     Segments sg{0, 0, nullptr, nullptr, 1};
     if (seg_len > 0 && nseg > 1) {
@@ -616,11 +623,11 @@ AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int 
         sg = Segments{1, seg_len, scratch, scratch + (size_t)(T / seg_len + S) * (size_t)heads * N * V, nseg};
     }
     const SsdArgs a{xbc, ld, x_off, b_off, c_off, dtr, lddt, A, dt_bias, D, p_dt, state, state_stride, s_off, slots, q_start, positions,
-                    y, ldy, T, S, heads, V, G, N, sg, steps, stream};
+                    y, ldy, T, S, heads, V, G, N, sg, longest, steps, stream};
     // float4 moves: every lane's first state value, B and C value on a 16-byte boundary, whole groups of four inside N
     const bool vec = N >= 128 && N % 4 == 0 && ld % 4 == 0 && b_off % 4 == 0 && c_off % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
                      ((uintptr_t)xbc & 15) == 0 && ((uintptr_t)state & 15) == 0 && (scratch == nullptr || ((uintptr_t)scratch & 15) == 0);
-    if (T == S) {                                     // single tokens: no rows fetched ahead (fewer registers, more CTAs resident)
+    if (T == S || longest == 1) {                     // single tokens: no rows fetched ahead (fewer registers, more CTAs resident)
         if (N <= 8) launch_ssd_scan<8, 1, 1, false>(a);
         else if (N <= 16) launch_ssd_scan<8, 2, 1, false>(a);
         else if (N <= 32) launch_ssd_scan<32, 1, 1, false>(a);

@@ -187,7 +187,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "aien_embed_gather_sinusoid": [P, I, P, P, P, P, I, I, I, F, P],
         "aien_attn_conv_prepare": [P, L, I, I, I, I, I, I, P, P, P, I, I, P, P, I, F, I, I, I, P, P, P, P, P, P, P, P, I, P, I, L, I, P],
         "aien_delta_conv_prepare": [P, L, I, I, I, I, I, I, I, I, I, P, P, P, I, I, P, P, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
-        "aien_delta_rule": [P, L, I, I, I, P, L, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, P],
+        "aien_delta_rule": [P, L, I, I, I, P, L, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, P],
         "aien_grouped_gated_rmsnorm": [P, L, P, I, L, P, I, F, P, I, L, I, I, I, I, P],
         "aien_paged_attention_decode_fused": [P, L, P, L, P, L, P, P, I, F, P, P, I, P, P, P, P, I, P, P, L, P, P, P,
                                               I, I, I, I, I, F, I, I, P],
@@ -196,8 +196,8 @@ def _declare(l: ctypes.CDLL) -> None:
         "aien_split_rows": [P, L, I, c_size_t, P, P, I, I, I, P],
         "aien_parts_product": [P, P, L, P, L, I, I, I, P],
         "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
-        "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, P, P],
-        "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, P],
+        "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, I, P, P],
+        "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, I, P],
         "aien_gate_group_norm": [P, L, P, L, P, I, F, F, P, I, L, I, I, I, P],
         "aien_scaled_add_rmsnorm": [P, P, I, I, c_size_t, P, P, P, I, F, P, I, I, I, P],
         "aien_pass_input": [P, P, P, I, I, I, P],
@@ -1786,22 +1786,25 @@ def delta_conv_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b
 
 def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gb: torch.Tensor, state: torch.Tensor, s_off: int,
                slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, o: torch.Tensor, num_seqs: int, heads: int,
-               qk_heads: int, dim: int, vdim: int, blocks: Optional[torch.Tensor] = None) -> None:
+               qk_heads: int, dim: int, vdim: int, blocks: Optional[torch.Tensor] = None, alone: int = 0) -> None:
     """Per value head, token by token: S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, all float32.  ``qkv``
     float32 [T, *] holds the prepared q, k (qk_heads x dim) and v (heads x vdim), ``gb`` [T, 2 * heads] the decay g and
     beta.  S [heads, dim, vdim] of request s lies ``s_off`` numbers into slot slot_map[s] of ``state`` (float32 [slots, n]).
     ``blocks`` (``block_walk_scratch(T, num_seqs, heads, qk_heads, dim, vdim)`` float32 numbers): the portions are walked
-    sixteen tokens at a time (:func:`block_walk`)."""
+    sixteen tokens at a time (:func:`block_walk`), and ``alone`` > 0: but for the so many requests of the step that bring one token."""
     _dev(qkv, gb, state, slot_map, q_start, positions, o)
     assert qkv.dtype == torch.float32 and qkv.stride(1) == 1 and gb.dtype == torch.float32 and gb.stride(1) == 1
     assert o.dtype == torch.float32 and o.stride(1) == 1 and o.shape[1] == heads * vdim
     assert state.dtype == torch.float32 and state.is_contiguous() and state.dim() == 2 and state.shape[1] >= s_off + heads * dim * vdim
     if blocks is not None and block_walk(qkv, q_off, k_off, v_off, gb, 0, heads, None, state, s_off, slot_map, q_start, positions, o, num_seqs, heads,
-                                         qk_heads, dim, vdim, blocks, delta=True):
-        return
+                                         qk_heads, dim, vdim, blocks, delta=True, alone=alone):
+        if not alone:
+            return
+    else:
+        alone = 0
     _check(lib().aien_delta_rule(_p(qkv), qkv.stride(0), int(q_off), int(k_off), int(v_off), _p(gb), gb.stride(0), _p(state), state.shape[1],
                                  int(s_off), _p(slot_map), _p(q_start), _p(positions), _p(o), o.stride(0), int(num_seqs), int(heads),
-                                 int(qk_heads), int(dim), int(vdim), _stream()), "delta_rule")
+                                 int(qk_heads), int(dim), int(vdim), 1 if alone else 0, _stream()), "delta_rule")
 
 
 GATE_ACTS = {"sigmoid": 0, "silu": 1}
@@ -1892,17 +1895,26 @@ def conv_act(proj: torch.Tensor, off: int, channels: int, w: torch.Tensor, bias:
 
 
 # ---------------------------------------------------------------------------- recurrences sixteen tokens at a time
-def block_walk_takes(dtype: torch.dtype, num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, delta: bool = False) -> bool:
+def block_walk_takes(dtype: torch.dtype, num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, delta: bool = False,
+                     singles: int = 0, least: int = 1) -> bool:
     """Whether a step's recurrence with one decay per head goes through :func:`block_walk`: a bfloat16 engine's portions of
     prompts (a float32 engine keeps to plain float32 products) over state matrices of up to 128 rows, with tokens enough
     beside each request's first that blocks of 16 are worth their coefficients' launch, and heads whose coefficients fit a
-    CTA's shared memory (the delta rule solves a 16 x 16 system a head there)."""
-    per = heads // max(qk_heads, 1)
+    CTA's shared memory (the delta rule solves a 16 x 16 system a head there).  ``singles``: how many of the step's requests
+    bring one token; the others must bring ``least`` tokens on the average.  The answer goes by the step's counts alone, so
+    that recorded steps of equal counts launch alike."""
+    per, portions = heads // max(qk_heads, 1), num_seqs - singles
+    if portions <= 0 or num_tokens - singles < least * portions:
+        return False
     return (dtype == torch.bfloat16 and num_tokens - num_seqs >= BLOCK_WALK_MIN_TOKENS and 0 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
             and 32 * (dim + 4) + (288 if delta else 32) * per <= 40 * 1024)
 
 
 BLOCK_WALK_MIN_TOKENS = 32
+# The delta rule and the duality form go token by token where portions are shorter than this on the average, and single
+# tokens beside portions always do: a block of 16 costs as much with one token in it.  Delta rule, a layer of 16 heads, 64
+# requests of two tokens: 72 us by blocks and 53 token by token (64 x 64), 141 and 121 (128 x 128); of five tokens 146 and 194.
+BLOCK_WALK_LEAST = 4
 
 
 def block_walk_scratch(num_tokens: int, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, act: bool = False) -> int:
@@ -1910,15 +1922,20 @@ def block_walk_scratch(num_tokens: int, num_seqs: int, heads: int, qk_heads: int
     return (num_tokens // 16 + num_seqs) * heads * 548 + (num_tokens * (2 * qk_heads * dim + heads * vdim) if act else 0)
 
 
+def _rows_walk(rows: torch.Tensor, scratch: torch.Tensor, *offs: int) -> bool:
+    return rows.data_ptr() % 16 == 0 and scratch.data_ptr() % 16 == 0 and all(n % 4 == 0 for n in (rows.stride(0),) + offs)
+
+
 def block_walk(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: Optional[torch.Tensor], g_off: int, w_off: int,
                decay: Optional[torch.Tensor], state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor,
                positions: torch.Tensor, out: torch.Tensor, num_seqs: int, heads: int, qk_heads: int, dim: int, vdim: int, scratch: torch.Tensor,
-               delta: bool = False, act: bool = False, skip: Optional[torch.Tensor] = None, state_vn: bool = False) -> bool:
+               delta: bool = False, act: bool = False, skip: Optional[torch.Tensor] = None, state_vn: bool = False, alone: int = 0) -> bool:
     """Per head, token by token, S <- g S + k u^T; o = S^T q (+ skip[h] v), over every request's portion: u = w v, or with
     ``delta`` u = w (v - (g S)^T k).  ``rows`` float32 [T, *] holds q and k (qk_heads x dim) and v (heads x vdim), with
     ``act`` before their silu; ``gates`` float32 [T, *] the decay g of head h in column g_off + h and w in w_off + h
     (w_off < 0: 1), or ``decay`` one per head.  S of request s lies ``s_off`` numbers into row slot_map[s] of ``state``, per
-    head [dim, vdim], or with ``state_vn`` [vdim, dim].  False, and nothing done, where the rows do not start on 16-byte boundaries."""
+    head [dim, vdim], or with ``state_vn`` [vdim, dim].  ``alone`` > 0: the so many requests that bring one token are left to
+    another kernel.  False, and nothing done, where the rows do not start on 16-byte boundaries."""
     _dev(rows, gates, decay, state, slot_map, q_start, positions, out, scratch, skip)
     T = rows.shape[0]
     assert rows.dtype == torch.float32 and rows.stride(1) == 1 and out.dtype == torch.float32 and out.stride(1) == 1
@@ -1928,13 +1945,13 @@ def block_walk(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: Op
     assert state.dtype == torch.float32 and state.is_contiguous() and state[0].numel() >= s_off + heads * dim * vdim
     assert skip is None or (skip.is_contiguous() and skip.numel() == heads)
     assert scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.numel() >= block_walk_scratch(T, num_seqs, heads, qk_heads, dim, vdim, act)
-    if rows.data_ptr() % 16 or scratch.data_ptr() % 16 or (rows.stride(0) | q_off | k_off | v_off) % 4:
+    if not _rows_walk(rows, scratch, q_off, k_off, v_off):
         return False
     _check(lib().aien_block_walk(
         _p(rows), rows.stride(0), int(q_off), int(k_off), int(v_off), int(act), _p(gates), gates.stride(0) if gates is not None else 0, int(g_off),
         int(w_off), _p(decay), int(delta), _p(skip), dt(skip) if skip is not None else F32, _p(state), state.stride(0), int(s_off), int(state_vn),
         _p(slot_map), _p(q_start), _p(positions), _p(out), out.stride(0), T, int(num_seqs), int(heads), int(qk_heads), int(dim), int(vdim),
-        _p(scratch), _stream()), "block_walk")
+        int(alone), _p(scratch), _stream()), "block_walk")
     add_launches(1)
     return True
 
@@ -2040,13 +2057,14 @@ def parts_product(parts: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
              state: torch.Tensor, s_off: int, slot_map: torch.Tensor, q_start: torch.Tensor, positions: torch.Tensor, y: torch.Tensor,
              num_seqs: int, heads: int, V: int, G: int, N: int, seg_len: int = 0, nseg: int = 1, scratch: Optional[torch.Tensor] = None,
-             steps: Optional[torch.Tensor] = None, blocks: Optional[torch.Tensor] = None) -> None:
+             steps: Optional[torch.Tensor] = None, blocks: Optional[torch.Tensor] = None, alone: int = 0) -> None:
     """The state-space-duality recurrence over every request's portion: per head h (group g = h // (heads // G)), token by
     token, dt = softplus(dtr[h] + dt_bias[h]); S = exp(-A[h] * dt) * S + dt * B[g] x[h]^T (S is N x V); y[h] = S^T C[g] +
     D[h] * x[h].  x, B, C are column blocks of the float32 rows ``xbc``; dtr float32 [T, heads] (row stride free); A float32
     [heads]; S lives in the request's state row from ``s_off`` on (as [heads, V, N]); y float32 [T, heads * V].  ``steps``:
     float32 scratch of T * 2 * heads numbers (made here when not given).  ``blocks`` (``block_walk_scratch(T, num_seqs, heads,
-    G, N, V)`` float32 numbers): the portions are walked sixteen tokens at a time (:func:`block_walk`)."""
+    G, N, V)`` float32 numbers): the portions are walked sixteen tokens at a time (:func:`block_walk`), and ``alone`` > 0: but for the
+    so many requests of the step that bring one token."""
     _dev(xbc, dtr, A, dt_bias, D, state, slot_map, q_start, positions, y, scratch, steps)
     T = xbc.shape[0]
     if steps is None:
@@ -2055,16 +2073,26 @@ def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.T
     assert xbc.dtype == torch.float32 and xbc.stride(1) == 1 and dtr.dtype == torch.float32 and dtr.stride(1) == 1
     assert A.dtype == torch.float32 and A.numel() == heads and dt_bias.dtype == D.dtype and dt_bias.is_contiguous() and D.is_contiguous()
     assert state.dtype == torch.float32 and state.stride(-1) == 1 and y.dtype == torch.float32 and y.stride(1) == 1
-    if blocks is not None:
+    walk = blocks is not None and _rows_walk(xbc, blocks, x_off, b_off, c_off)
+    if walk and not alone:
         _check(lib().aien_ssd_steps(_p(dtr), dtr.stride(0), _p(A), _p(dt_bias), dt(dt_bias), _p(steps), T, int(heads), _stream()), "ssd_steps")
-        if block_walk(xbc, c_off, b_off, x_off, steps[:T * 2 * heads].view(T, 2 * heads), heads, 0, None, state, s_off, slot_map, q_start, positions, y,
-                      num_seqs, heads, G, N, V, blocks, skip=D, state_vn=True):
-            return
+    else:
+        _ssd_tokens(xbc, x_off, b_off, c_off, dtr, A, dt_bias, D, state, s_off, slot_map, q_start, positions, y, num_seqs, heads, V, G, N, seg_len, nseg,
+                    scratch, steps, 1 if walk else 0)
+    if walk:
+        block_walk(xbc, c_off, b_off, x_off, steps[:T * 2 * heads].view(T, 2 * heads), heads, 0, None, state, s_off, slot_map, q_start, positions, y,
+                   num_seqs, heads, G, N, V, blocks, skip=D, state_vn=True, alone=alone)
+
+
+def _ssd_tokens(xbc, x_off, b_off, c_off, dtr, A, dt_bias, D, state, s_off, slot_map, q_start, positions, y, num_seqs, heads, V, G, N, seg_len, nseg,
+                scratch, steps, longest) -> None:
+    T = xbc.shape[0]
     if seg_len and nseg > 1:
         assert scratch is not None and scratch.numel() >= 2 * (T // seg_len + num_seqs) * heads * N * V
     _check(lib().aien_ssd_scan(_p(xbc), xbc.stride(0), int(x_off), int(b_off), int(c_off), _p(dtr), dtr.stride(0), _p(A), _p(dt_bias), _p(D),
                                dt(D), _p(state), state.stride(0), int(s_off), _p(slot_map), _p(q_start), _p(positions), _p(y), y.stride(0),
-                               T, int(num_seqs), int(heads), int(V), int(G), int(N), int(seg_len), int(nseg), _p(scratch), _p(steps), _stream()), "ssd_scan")
+                               T, int(num_seqs), int(heads), int(V), int(G), int(N), int(seg_len), int(nseg), _p(scratch), _p(steps), int(longest),
+                               _stream()), "ssd_scan")
     add_launches(3 if (seg_len and nseg > 1) else 1)
 
 

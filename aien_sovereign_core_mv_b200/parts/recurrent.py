@@ -17,7 +17,9 @@ class DecayLinearAttention(Mixer):
     (heads x ``value_dim``); per head S_t = decay_h S_(t-1) + k_t v_t^T and o_t = S_t^T q_t, with no other scale.  The
     heads together pass an RMS norm (plain weight ``norm``), are multiplied by sigmoid(W_g h) and projected by W_o.
     The state [heads, head_dim, value_dim] is float32, starts at zero and is carried in a state slot of the cache; the
-    recurrence, its decay powers and the norm are float32 in both engine precisions.  One product makes q | k | v | g."""
+    recurrence, its decay powers and the norm are float32 in both engine precisions, but for the products of portions in a
+    bfloat16 engine, which run on the tensor cores with float32 operands in two halves (``kernels.block_walk``: as near to 64
+    bits as the float32 kernels).  One product makes q | k | v | g."""
 
     def __init__(self, hidden_size: int, num_heads: int, head_dim: int, value_dim: int, decay: Sequence[float],
                  norm_eps: float = 1e-6, position=None):
@@ -133,7 +135,9 @@ class GatedDeltaRule(Mixer):
 
     One float32 state slot per request holds the last taps-1 projected rows of q | k | v followed by S
     [num_heads, head_dim, value_dim].  Convolution, activations, unit norms, decay, beta, the recurrence and the output
-    norm are float32 in both engine precisions.  One product makes q | k | v | g | b | a."""
+    norm are float32 in both engine precisions, but for the products of portions in a bfloat16 engine, which run on the
+    tensor cores with float32 operands in two halves (``kernels.block_walk``).  Which kernel a portion takes depends on the
+    step it is in, and with it the order of its float32 additions.  One product makes q | k | v | g | b | a."""
 
     def __init__(self, hidden_size: int, num_heads: int, num_qk_heads: int, head_dim: int, value_dim: int, taps: int = 1,
                  norm_eps: float = 1e-6, position=None):
@@ -196,10 +200,14 @@ class GatedDeltaRule(Mixer):
         o = ctx.workspace.take((T, self.v_dim), torch.float32)
         sizes = (n, self.num_qk_heads, self.head_dim, self.value_dim)
         blocks = None
-        if K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes, delta=True) and not ctx.decode_only:
+        alone = ctx.single_tokens[1] if ctx.single_tokens is not None else 0
+        # the walk token by token of a portion hides behind many single tokens: beside 200 of them one of 33 tokens takes a layer of
+        # 16 heads of 64 x 64 122 us by blocks, 106 without, beside 64 of them 68 and 66 (128 x 128: 150 and 158)
+        least = max(K.BLOCK_WALK_LEAST, alone // 2)
+        if not ctx.decode_only and K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes, delta=True, singles=alone, least=least):
             blocks = ctx.workspace.take((K.block_walk_scratch(T, ctx.num_seqs, *sizes),), torch.float32)
         K.delta_rule(qkv, 0, self.qk_dim, 2 * self.qk_dim, gb, state, self.conv_floats, group.slot_map, ctx.q_start, ctx.positions, o,
-                     ctx.num_seqs, *sizes, blocks)
+                     ctx.num_seqs, *sizes, blocks, alone)
         y = ctx.workspace.take((T, self.v_dim), ctx.dtype)
         K.grouped_gated_rmsnorm(o, proj[:, g_off:g_off + self.v_dim], self.norm_w, self.norm_eps, y, self.value_dim, "silu")
         return linear(ctx, y, self.w_o, out_dtype=torch.float32, may_defer_sum=True)

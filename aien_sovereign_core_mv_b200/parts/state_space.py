@@ -74,7 +74,9 @@ class SelectiveScan(Mixer):
     W_o (y * silu(z)).
 
     One float32 state slot per request holds the convolution's last taps - 1 inputs followed by S; it starts from zeros.
-    Step sizes, decays, the recurrence and the gate are float32 in both engine precisions."""
+    Step sizes, decays, the recurrence and the gate are float32 in both engine precisions.  In a bfloat16 engine the decays
+    come from the special-function unit (relative error near 2^-21), and the step sizes' product runs on the tensor cores over
+    its float32 rows in three bfloat16 parts, added like float32 (``kernels.parts_product``)."""
 
     def __init__(self, hidden_size: int, inner: int, state: int, dt_rank: int, taps: int = 4, position=None):
         self.hidden_size, self.inner, self.state, self.dt_rank, self.taps = int(hidden_size), int(inner), int(state), int(dt_rank), int(taps)
@@ -153,7 +155,10 @@ class StateSpaceDuality(BranchMixer):
     the root), multiplied by the weight ``norm`` and projected by W_o.
 
     One float32 state slot per request holds the convolution's last taps - 1 inputs followed by S as [heads, value_dim, N];
-    it starts from zeros.  Step sizes, decays, the recurrence, the gate and the norm are float32 in both precisions."""
+    it starts from zeros.  Step sizes, decays, the recurrence, the gate and the norm are float32 in both precisions, but for
+    the products of portions in a bfloat16 engine, which run on the tensor cores with float32 operands in two halves
+    (``kernels.block_walk``).  Which kernel a portion takes depends on the step it is in, and with it the order of its float32
+    additions."""
 
     def __init__(self, hidden_size: int, num_heads: int, value_dim: int, state: int, groups: int = 1, norm_groups: int = 1,
                  taps: int = 4, norm_eps: float = 1e-6, position=None):
@@ -217,15 +222,16 @@ class StateSpaceDuality(BranchMixer):
                    ctx.positions, xbc)
         y = ws.take((T, I), torch.float32)
         seg, nseg, scratch, blocks = 0, 1, None, None
-        if K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, self.num_heads, self.groups, self.state, self.value_dim) and not ctx.decode_only \
-                and self.channels % 4 == 0 and I % 4 == 0:
+        alone = ctx.single_tokens[1] if ctx.single_tokens is not None else 0
+        if not ctx.decode_only and K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, self.num_heads, self.groups, self.state, self.value_dim, singles=alone,
+                                                      least=K.BLOCK_WALK_LEAST) and self.channels % 4 == 0 and I % 4 == 0:
             blocks = ws.take((K.block_walk_scratch(T, ctx.num_seqs, self.num_heads, self.groups, self.state, self.value_dim),), torch.float32)
         else:
             seg, nseg, scratch = _segments(ctx, self.num_heads * self.state * self.value_dim, I * min(self.state, 32))
         steps = ws.take((T * 2 * self.num_heads,), torch.float32)
         dt0 = col0 + 2 * I + 2 * GN
         K.ssd_scan(xbc, 0, I, I + GN, proj[:, dt0:dt0 + self.num_heads], self.A, self.dt_b, self.D, state, self.conv_floats, slots,
-                   ctx.q_start, ctx.positions, y, ctx.num_seqs, self.num_heads, self.value_dim, self.groups, self.state, seg, nseg, scratch, steps, blocks)
+                   ctx.q_start, ctx.positions, y, ctx.num_seqs, self.num_heads, self.value_dim, self.groups, self.state, seg, nseg, scratch, steps, blocks, alone)
         K.gate_group_norm(y, proj[:, col0:col0 + I], self.norm_w, self.norm_eps, mult, out[:, out_col0:out_col0 + I], self.norm_groups)
 
 

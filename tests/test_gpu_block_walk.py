@@ -136,6 +136,58 @@ def test_many_heads_over_one_group_walk_by_blocks():
     H.assert_close(state.cpu().numpy().reshape(heads, V, N).transpose(0, 2, 1), last, 1e-5, "state")
 
 
+@pytest.mark.parametrize("form", ["delta", "duality"])
+@pytest.mark.parametrize("lens", [[1, 40, 1, 33, 1, 1], [2, 1, 17], [50, 1]])
+def test_single_tokens_beside_portions(form, lens):
+    """Requests of one token go token by token beside the walk of the others: every request against 64 bits, with the walk for
+    all of them and for the portions alone, where the single tokens have the bits of the token kernel."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    g_ = torch.Generator().manual_seed(len(lens))
+    T, S, heads, G, N, V = sum(lens), len(lens), 6, 2, 68, 36
+    GN, s_off, delta = G * N, 3, form == "delta"
+    rows = torch.randn(T, 2 * GN + heads * V, generator=g_)
+    rows[:, GN:2 * GN] /= rows[:, GN:2 * GN].reshape(T, G, N).norm(dim=-1).repeat_interleave(N, dim=1)
+    gb = torch.rand(T, 2 * heads, generator=g_) * 0.9 + 0.1
+    dtr, A, bias, D = torch.randn(T, heads, generator=g_), torch.rand(heads, generator=g_), torch.randn(heads, generator=g_) - 2.0, torch.randn(heads, generator=g_)
+    state = torch.randn(S, s_off + heads * N * V, generator=g_)
+    q0, pos = [sum(lens[:s]) for s in range(S + 1)], [p + (0 if s % 2 else 7) for s, n in enumerate(lens) for p in range(n)]
+    singles = [t for s, t in enumerate(q0[:-1]) if lens[s] == 1]
+    got = []
+    for blocks, alone in ((True, 0), (True, len(singles)), (False, 0)):
+        st, out = state.clone().cuda(), torch.zeros(T, heads * V).cuda()
+        scratch = torch.full((K.block_walk_scratch(T, S, heads, G, N, V),), float("nan")).cuda() if blocks else None
+        common = (st, s_off, i32(list(range(S))), i32(q0), i32(pos), out, S, heads)
+        if delta:
+            K.delta_rule(rows.cuda(), 0, GN, 2 * GN, gb.cuda(), *common, G, N, V, scratch, alone)
+        else:
+            K.ssd_scan(rows.cuda(), 2 * GN, GN, 0, dtr.cuda(), A.cuda(), bias.cuda(), D.cuda(), *common, V, G, N, blocks=scratch, alone=alone)
+        got.append((out.cpu(), st.cpu()))
+    assert torch.equal(got[1][0][singles], got[2][0][singles])
+    a = rows.double().numpy()
+    dt = np.logaddexp(0.0, (dtr + bias).double().numpy())
+    g, w = (gb[:, :heads].double().numpy(), gb[:, heads:].double().numpy()) if delta else (np.exp(-A.double().numpy() * dt), dt)
+    for s in range(S):
+        r = slice(q0[s], q0[s + 1])
+        qk = lambda off: np.repeat(a[r, off:off + GN].reshape(-1, G, N), heads // G, axis=1)
+        S0 = state[s, s_off:].double().numpy().reshape((heads, N, V) if delta else (heads, V, N))
+        S0 = (S0 if delta else S0.transpose(0, 2, 1)) * (0.0 if s % 2 else 1.0)
+        want, last = _recurrence(qk(0), qk(GN), a[r, 2 * GN:].reshape(-1, heads, V), g[r], w[r], S0, delta, np.zeros(heads) if delta else D.double().numpy())
+        for out, st in got:
+            H.assert_close(out[r].numpy().reshape(want.shape), want, 1e-5, f"request {s}")
+            end = st[s, s_off:].numpy().reshape((heads, N, V) if delta else (heads, V, N))
+            H.assert_close(end if delta else end.transpose(0, 2, 1), last, 1e-5, f"state of request {s}")
+
+
+def test_which_steps_walk_by_blocks():
+    """By counts alone: enough tokens behind each request's first, and portions that are not short on the average."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    takes = lambda T, S, singles: K.block_walk_takes(torch.bfloat16, T, S, 16, 8, 64, 64, singles=singles, least=K.BLOCK_WALK_LEAST)
+    assert takes(97, 65, 64) and takes(33, 1, 0) and takes(320, 64, 0) and takes(88, 56, 48)
+    assert not takes(128, 64, 0) and not takes(192, 64, 0) and not takes(112, 80, 64) and not takes(32, 1, 0) and not takes(64, 64, 64)
+    assert K.block_walk_takes(torch.bfloat16, 128, 64, 16, 16, 64, 64)                 # without a least: linear attention
+
+
 def test_block_walk_declines_rows_off_the_boundary():
     from aien_sovereign_core_mv_b200 import kernels as K
     i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
