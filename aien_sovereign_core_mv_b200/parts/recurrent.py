@@ -202,7 +202,7 @@ class GatedDeltaRule(Mixer):
         blocks = None
         alone = ctx.single_tokens[1] if ctx.single_tokens is not None else 0
         # the walk token by token of a portion hides behind many single tokens: beside 200 of them one of 33 tokens takes a layer of
-        # 16 heads of 64 x 64 122 us by blocks, 106 without, beside 64 of them 68 and 66 (128 x 128: 150 and 158)
+        # 16 heads of 64 x 64 122 us by blocks and 90 without; beside 64 of them, 16 heads of 128 x 128, 150 and 158
         least = max(K.BLOCK_WALK_LEAST, alone // 2)
         if not ctx.decode_only and K.block_walk_takes(ctx.dtype, T, ctx.num_seqs, *sizes, delta=True, singles=alone, least=least):
             blocks = ctx.workspace.take((K.block_walk_scratch(T, ctx.num_seqs, *sizes),), torch.float32)
