@@ -194,13 +194,15 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
                 emit_run(zt, kvh, seg * per_seg, per_seg);
             }
         } else {
-            // More (token, kv head) pairs than CTAs (T <= 256): the chunks of all pairs, in pair order,
-            // are cut into gridDim.x equal ranges, so a CTA takes the tail of one pair, whole pairs and
-            // the head of another, and contexts of different lengths weigh what they hold.  Lane l keeps
-            // the chunk counts of tokens l, l + 32, ... and how many chunks lie before each.
+            // Ranges (T <= 256): the chunks of all pairs, in pair order, are cut into gridDim.x equal ranges, so a
+            // CTA takes the tail of one pair, whole pairs and the head of another, and contexts of different
+            // lengths weigh what they hold.  Lane l keeps the chunk counts of tokens l, l + 32, ... and how many
+            // chunks lie before each.  All of it is 32-bit: fewer than 2^31 chunks (see launch_decode_stream).
             int nch[8], pre[8], all = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
+                nch[j] = 0; pre[j] = 0;
+                if (j * 32 >= T) continue;
                 const int zt = j * 32 + lane;
                 int n = 0;
                 if (zt < T) {
@@ -217,14 +219,16 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
                 nch[j] = n; pre[j] = all + incl - n;
                 all += __shfl_sync(0xffffffffu, incl, 31);
             }
-            const long chunks = (long)all * nkv;
-            long at = chunks * blockIdx.x / gridDim.x;
-            const long end = chunks * (blockIdx.x + 1) / gridDim.x;
+            // the first `longer` ranges hold one chunk more
+            const unsigned chunks = (unsigned)(all * nkv), each = chunks / gridDim.x, longer = chunks - each * gridDim.x;
+            int at = (int)(each * blockIdx.x + min(blockIdx.x, longer));
+            const int end = at + (int)each + (blockIdx.x < longer ? 1 : 0);
             while (at < end) {
                 int zt = -1, before = 0, n = 0;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const bool mine = nch[j] > 0 && (long)nkv * pre[j] <= at && at < (long)nkv * (pre[j] + nch[j]);
+                    if (j * 32 >= T) continue;
+                    const bool mine = nch[j] > 0 && nkv * pre[j] <= at && at < nkv * (pre[j] + nch[j]);
                     const unsigned m = __ballot_sync(0xffffffffu, mine);
                     if (m != 0u) {
                         const int src = __ffs(m) - 1;
@@ -234,9 +238,9 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
                     }
                 }
                 if (zt < 0) break;                                 // cannot happen: every chunk index belongs to a token
-                const int rem = (int)(at - (long)nkv * before);
+                const int rem = at - nkv * before;
                 const int kvh = rem / n, rel = rem - kvh * n;
-                const int count = (int)min((long)(n - rel), end - at);
+                const int count = min(n - rel, end - at);
                 emit_run(zt, kvh, rel, count);
                 at += count;
             }
@@ -460,16 +464,25 @@ static int launch_decode_stream(const CUtensorMap& mk, const CUtensorMap& mv, co
     const bool outside = ds_merge_outside(max_splits);
     int segs = ds_segments_per_pair((long)T * nkv, max_splits, slots);
     if (const char* e = getenv("AIEN_B200_DECODE_SEGMENTS")) { const int v = atoi(e); if (v > 0 && v <= max_splits) segs = v; }
-    // more pairs than CTAs: equal ranges of chunks instead of whole pairs (segs = 0 tells the kernel); AIEN_B200_DECODE_BALANCED=0: off
+    // Equal ranges of chunks instead of whole segments (segs = 0 tells the kernel); AIEN_B200_DECODE_BALANCED=0: never, 2: always.
+    // A range shares pairs with its neighbours, and every shared pair is a ticket and a merge more, but contexts of different
+    // lengths weigh what they hold.  32q/8kv x 128, the kernel alone, whole segments -> ranges, us:
+    //   * more pairs than CTAs, where whole pairs would leave a fifth of the CTA rounds empty, or take three rounds or more (1,030
+    //     keys: batch 48 the same, 64 54.3 -> 53.5, 96 81.2 -> 76.9, 128 108.0 -> 99.0; inside a decode step of 36 layers: batch 48
+    //     5.26 -> 5.03 ms, 64 5.69 -> 5.73 ms, 96 7.09 -> 7.02 ms, 128 8.37 -> 8.25 ms);
+    //   * one or two segments a pair that would leave a fifth (two: a tenth) of the CTAs without one, from eight chunks a token
+    //     on; contexts of 1,600 keys, and in brackets spread 1 to 1.7: batch 13 21.4 -> 20.0 (22.8 -> 20.6), 16 23.2 -> 23.4 (26.5 ->
+    //     23.6), 19 32.7 -> 28.5 (37.4 -> 27.6), 24 34.0 -> 32.3 (38.4 -> 32.5), 28 36.2 -> 36.0 (39.9 -> 36.0).  Batch 32, whose
+    //     pairs are 0.86 of the CTAs, loses with even contexts (39.3 -> 40.6), batch 8 with its four segments too (14.6 ->
+    //     15.9), and so do four chunks a token (batch 24, 480 keys: 13.4 -> 14.4).
     static int balanced = -1;
-    if (balanced < 0) { const char* e = getenv("AIEN_B200_DECODE_BALANCED"); balanced = (e && e[0] == '0') ? 0 : 1; }
-    // (measured, 32q/8kv x 128 at 1,030 keys, whole pairs -> ranges, the kernel alone: batch 48 the same, 64 54.3 -> 53.5 us,
-    // 96 81.2 -> 76.9 us, 128 108.0 -> 99.0 us; inside a decode step of 36 layers: batch 48 5.26 -> 5.03 ms, 64 5.69 -> 5.73 ms,
-    // 96 7.09 -> 7.02 ms, 128 8.37 -> 8.25 ms.  A range shares pairs with its neighbours, and every shared pair is a ticket
-    // and a merge more: so only when whole pairs would leave a fifth of the CTA rounds empty, or take three rounds or more.)
+    if (balanced < 0) { const char* e = getenv("AIEN_B200_DECODE_BALANCED"); balanced = e == nullptr ? 1 : e[0] == '0' ? 0 : e[0] == '2' ? 2 : 1; }
     const long pairs = (long)T * nkv, rounds = (pairs + slots - 1) / slots;
-    if (balanced && segs == 1 && pairs > slots && (pairs * 10 < slots * rounds * 8 || rounds >= 3) && T <= 256 &&
-        getenv("AIEN_B200_DECODE_SEGMENTS") == nullptr) segs = 0;
+    bool ranges = segs == 1 && pairs > slots && (pairs * 10 < slots * rounds * 8 || rounds >= 3);
+    const int most = window > 0 && window / DS_CHUNK + 2 < max_splits ? window / DS_CHUNK + 2 : max_splits;      // chunks a token can see
+    ranges |= pairs <= slots && segs <= 2 && segs * pairs * 10 < slots * (segs == 1 ? 8 : 9) && most >= 8;
+    ranges |= balanced == 2;
+    if (ranges && balanced != 0 && T <= 256 && pairs * max_splits < (1L << 31) && getenv("AIEN_B200_DECODE_SEGMENTS") == nullptr) segs = 0;
     const long total = segs > 0 ? (long)segs * T * nkv : slots;
     const unsigned grid = (unsigned)(total < slots ? total : slots);
     launch_chain(kern, dim3(grid), dim3(DS_THREADS), smem, stream, mk, mv, (const __nv_bfloat16*)q, q_stride, bt, max_blocks, seq_of_token,

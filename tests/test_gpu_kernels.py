@@ -459,6 +459,38 @@ def test_paged_attention_decode_stream_gives_the_same_bits(K, nq, nkv, hd, page,
     assert K.attention_decode_stream_error() == 0
 
 
+@pytest.mark.parametrize("nq,nkv,hd,window,n_req", [(32, 8, 128, 0, 13), (16, 8, 64, 0, 19), (32, 8, 128, 0, 29), (32, 8, 128, 0, 30),
+                                                    (32, 8, 128, 900, 20), (8, 2, 128, 0, 80), (3, 1, 128, 0, 256)])
+def test_paged_attention_decode_stream_in_ranges(K, nq, nkv, hd, window, n_req):
+    """Fewer (token, kv head) pairs than CTAs, but too many for whole segments to keep the CTAs busy: equal ranges of chunks
+    (and, at 30 requests, one pair more than the rule takes).  Contexts from one key on; the same bits as the
+    one-CTA-per-chunk kernel, twice, and for a list of the tokens."""
+    rng = np.random.default_rng(n_req)
+    seq_lens = [1, 2200, 128, 129] + [int(x) for x in rng.integers(1, 1500, size=n_req - 4)]
+    kc, vc, bt, mb, _ = paged_setup(rng, seq_lens, nkv, hd, 16, torch.bfloat16, sum((n + 15) // 16 for n in seq_lens) + 8)
+    positions = torch.tensor([n - 1 for n in seq_lens], dtype=torch.int32).cuda()
+    q = torch.tensor(rng.standard_normal((n_req, nq * hd)), dtype=torch.float32).to(torch.bfloat16).cuda()
+    splits = (max(seq_lens) + 127) // 128
+    part_out = torch.empty(n_req * nq * splits * hd, device="cuda"); part_ml = torch.empty(n_req * nq * splits * 2, device="cuda")
+
+    def attend(impl, tokens=None):
+        out = torch.full((n_req, nq * hd), 5.0, dtype=torch.bfloat16, device="cuda")
+        K.paged_attention_decode(q, kc, vc, bt, mb, torch.arange(n_req, dtype=torch.int32).cuda(), positions, out, part_out, part_ml, nq, nkv, hd, 16, window,
+                                 hd ** -0.5, splits, impl=impl, token_list=None if tokens is None else torch.tensor(tokens, dtype=torch.int32).cuda(),
+                                 num_tokens=None if tokens is None else len(tokens))
+        torch.cuda.synchronize()
+        assert K.attention_decode_stream_error() == 0
+        return out
+
+    want = attend("direct")
+    for _ in range(2):                                        # twice: the ticket counters must come back to zero
+        assert torch.equal(attend("stream"), want)
+    some = list(range(n_req - 1, -1, -2))
+    sub = attend("stream", some)
+    rest = [i for i in range(n_req) if i not in some]
+    assert torch.equal(sub[some], want[some]) and (sub[rest] == 5.0).all()
+
+
 @pytest.mark.parametrize("nq,nkv,hd,page,window,lens", [(8, 2, 128, 16, 0, [20001, 9000, 130]), (4, 1, 64, 64, 12000, [16500, 1]),
                                                           (6, 2, 96, 16, 0, [8300, 700])])
 def test_decode_attention_over_long_contexts(K, nq, nkv, hd, page, window, lens):
