@@ -26,17 +26,20 @@
 //
 // Relative error (2-norm) of the results and the last states against 64 bits, 2,048 tokens, and in brackets that of the
 // float32 kernels that go token by token or, for one decay per head, by chunks of 64:
-//   one decay per head, 1 - 2^-5 .. 1 - 2^-8          0.8e-7 and 0.8e-7  (1.7e-7 and 1.3e-7)
-//   one decay per head, 1 - 1e-4                      0.9e-7 and 1.7e-7  (2.7e-7 and 3.2e-7)
-//   duality, rows of silu, drawn step sizes           0.9e-7 and 1.0e-7  (0.9e-7 and 3.0e-7)
+//   one decay per head, 1 - 2^-5 .. 1 - 2^-8          0.7e-7 and 0.8e-7  (1.7e-7 and 1.3e-7)
+//   one decay per head, 1 - 1e-4                      0.8e-7 and 1.7e-7  (2.7e-7 and 3.2e-7)
+//   duality, rows of silu, drawn step sizes           0.7e-7 and 1.0e-7  (0.9e-7 and 3.0e-7)
 //   delta rule, rows of silu, drawn decays            1.4e-7 and 1.4e-7  (2.1e-7 and 3.1e-7)
 //   delta rule, rows of either sign, decays 0.74 .. 1 1.3e-7 and 1.1e-7  (1.1e-7 and 0.8e-7)
 // With one accumulator, nothing added back and rounded products of decays the first two were 6.8e-7 and 2.3e-6.
 //
-// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 152 us and 16 for the coefficients (603 token by
-// token); 2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 122 and 6 us (540); linear attention, 1,900
-// tokens of two requests, 16 heads of 128 x 128: 95 and 29 us (237 by chunks).  What bounds the walk is a block's chain of loads,
-// products and barriers.  (The choices of a form below were measured at 148, 110 and 86 us, with one accumulator a sum.)
+// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 151 us and 16 for the coefficients (603 token by
+// token); linear attention 123 and 31.  2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 100 and 6 us (540;
+// 122 with the longest request's CTAs the last to start); linear attention, 1,900 tokens of two requests, 16 heads of 128 x 128: 92
+// and 29 us (237 by chunks).  What bounds the walk is a block's chain of dependent instructions (390 a warp, of which each
+// waits 4 to 5 cycles; issue slots 43 % used with one CTA on an SM, 53 % with two), not its barriers or its rows: fetched two
+// blocks ahead instead of one, with one barrier a block instead of two, and with products of different sums between dependent
+// ones it gains 4 us in 128.  (The choices of a form below were measured at 148, 110 and 86 us, with one accumulator a sum.)
 #include "common.cuh"
 #include <math.h>
 
@@ -55,7 +58,7 @@ __device__ __forceinline__ void bw_split(float x, uint32_t& hi, uint32_t& lo) {
 }
 
 __device__ __forceinline__ void bw_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
@@ -82,6 +85,11 @@ struct BwDecay {
 __device__ __forceinline__ void bw_cp16(float* dst, const float* src, bool in) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+__device__ __forceinline__ void bw_cp16(float* dst, const float* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
 struct BlockWalk {
@@ -245,22 +253,24 @@ block_coef_kernel(const BlockWalk a) {
 
 // NT: fragments of 8 rows that a warp owns; N <= 64 NT.  MT: a CTA has 16 MT columns of the state.
 // HELP: with helper warps (see block_walk_kernel).
-template <int NT, int MT, bool HELP>
+template <int NT, int MT, bool DELTA, bool HELP>
 struct BwSmem {
-    static constexpr int STAGES = HELP ? 3 : 2, TURNS = HELP ? 2 : 1;                      // sums of r and u for so many blocks
+    static constexpr int STAGES = DELTA ? 3 : 4, TURNS = HELP || !DELTA ? 2 : 1;  // TURNS: sums of r (and u) for so many blocks
     static constexpr int LDN = 64 * NT + 8;                     // floats between rows of q and k: a half warp's 8-byte reads meet no bank twice
     static constexpr int LDV = 16 * MT + 8, LDP = 16 * MT + 4;  // floats between rows of v and u, and of the partial sums
     static constexpr int QK = BW_B * LDN;
-    static constexpr int STAGE = 2 * QK + BW_B * LDV + 2 * BW_B * BW_LD + BW_TAIL;      // q | k | v | A | M | G | G_16 / G_j, what G_16 lacks
+    static constexpr int M_AT = 2 * QK + BW_B * LDV + BW_B * BW_LD, G_AT = M_AT + (DELTA ? BW_B * BW_LD : 0);
+    static constexpr int STAGE = G_AT + BW_TAIL;                // q | k | v | A | M (the delta rule) | G | G_16 / G_j, what G_16 lacks
     static constexpr int PART = BW_WARPS * BW_B * LDP;
-    static constexpr int U = BW_B * LDV;
-    static constexpr int TOTAL = STAGES * STAGE + (1 + TURNS) * PART + TURNS * U;          // partial sums of p, and of r, and u
+    static constexpr int SUMS = PART + (DELTA ? 0 : 2 * BW_B * LDP);                       // without the delta rule A u too, by halves of its tokens
+    static constexpr int U = DELTA ? BW_B * LDV : 0;
+    static constexpr int TOTAL = STAGES * STAGE + (DELTA ? PART : 0) + TURNS * (SUMS + U);            // partial sums of p, and of r, and u
 };
 
 template <int NT, int MT, bool DELTA, bool HELP>
 __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWalk& a, const float* rows, long ld, int q_col, int k_col, int v_col,
                                          int cols, const float* coef, int t, int t1, int tid) {
-    using C = BwSmem<NT, MT, HELP>;
+    using C = BwSmem<NT, MT, DELTA, HELP>;
     constexpr int pieces = 16 * NT;                             // 16-byte pieces of a padded row
 #pragma unroll
     for (int i = tid; i < BW_B * pieces; i += BW_THREADS) {
@@ -282,7 +292,7 @@ __device__ __forceinline__ void bw_fetch(float* __restrict__ buf, const BlockWal
         const int e = tid - 64 * MT - 64;
         bw_cp16(sA + BW_B * BW_LD + (e >> 2) * BW_LD + (e & 3) * 4, coef + 256 + e * 4, true);
     }
-    if (tid < BW_TAIL / 4) bw_cp16(sA + 2 * BW_B * BW_LD + tid * 4, coef + 512 + tid * 4, true);
+    if (tid < BW_TAIL / 4) bw_cp16(buf + C::G_AT + tid * 4, coef + 512 + tid * 4, true);
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
@@ -294,36 +304,52 @@ __device__ __forceinline__ float bw_total(float c, float d) {
     return c + fmaf(c, (STEPS == 2 ? 0.54f : 0.36f) * 1.1920929e-7f, d);
 }
 
-// partial products S0^T x of a warp's rows, x the q or k rows of a block: [16 MT columns] x [16 tokens] into part[token][column]
-template <int NT, int MT>
-__device__ __forceinline__ void bw_read_out(const float* __restrict__ x, const uint32_t (&sh)[MT][NT][4], const uint32_t (&sl)[MT][NT][4],
-                                            float* __restrict__ part, int row0, int g, int t) {
-    using C = BwSmem<NT, MT, false>;
+// Partial products S0^T x of a warp's rows, x the q or k rows of a block (IN of them): [16 MT columns] x [16 tokens] into
+// part[token][column].  A product whose sum the one before it adds to waits for that, so products of different sums stand between.
+template <int NT, int MT, int IN>
+__device__ __forceinline__ void bw_read_out(const float* const (&x)[IN], const uint32_t (&sh)[MT][NT][4], const uint32_t (&sl)[MT][NT][4],
+                                            float* const (&part)[IN], int row0, int g, int t) {
+    using C = BwSmem<NT, MT, true, false>;
     constexpr int HALVES = 2 / MT;                              // of the tokens at a time: as many accumulators with 32 columns as with 16
 #pragma unroll
     for (int h0 = 0; h0 < 2; h0 += HALVES) {
-        float acc[MT][HALVES][4] = {}, low[MT][HALVES][4] = {};
+        float acc[IN][MT][HALVES][4] = {}, low[IN][MT][HALVES][4] = {};
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < NT; ++nt) {
+            uint32_t bh[IN][HALVES][2], bl[IN][HALVES][2];
 #pragma unroll
-            for (int h = 0; h < HALVES; ++h) {
-                const float2 v = *reinterpret_cast<const float2*>(x + ((h0 + h) * 8 + g) * C::LDN + row0 + nt * 8 + 2 * t);
-                uint32_t bh[2], bl[2];
-                bw_split(v.x, bh[0], bl[0]);
-                bw_split(v.y, bh[1], bl[1]);
+            for (int i = 0; i < IN; ++i)
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) bw_mma3(acc[mt][h], low[mt][h], sh[mt][nt], sl[mt][nt], bh, bl);
-            }
+                for (int h = 0; h < HALVES; ++h) {
+                    const float2 v = *reinterpret_cast<const float2*>(x[i] + ((h0 + h) * 8 + g) * C::LDN + row0 + nt * 8 + 2 * t);
+                    bw_split(v.x, bh[i][h][0], bl[i][h][0]);
+                    bw_split(v.y, bh[i][h][1], bl[i][h][1]);
+                }
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+            for (int step = 0; step < 3; ++step)
 #pragma unroll
-            for (int h = 0; h < HALVES; ++h) {
-                float* p = part + ((h0 + h) * 8 + 2 * t) * C::LDP + mt * 16 + g;
-                p[0] = bw_total<NT>(acc[mt][h][0], low[mt][h][0]);
-                p[C::LDP] = bw_total<NT>(acc[mt][h][1], low[mt][h][1]);
-                p[8] = bw_total<NT>(acc[mt][h][2], low[mt][h][2]);
-                p[C::LDP + 8] = bw_total<NT>(acc[mt][h][3], low[mt][h][3]);
-            }
+                for (int i = 0; i < IN; ++i)
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                        for (int h = 0; h < HALVES; ++h) {
+                            if (step == 0) bw_mma(low[i][mt][h], sl[mt][nt], bh[i][h]);
+                            if (step == 1) bw_mma(acc[i][mt][h], sh[mt][nt], bh[i][h]);
+                            if (step == 2) bw_mma(low[i][mt][h], sh[mt][nt], bl[i][h]);
+                        }
+        }
+#pragma unroll
+        for (int i = 0; i < IN; ++i)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int h = 0; h < HALVES; ++h) {
+                    float* p = part[i] + ((h0 + h) * 8 + 2 * t) * C::LDP + mt * 16 + g;
+                    p[0] = bw_total<NT>(acc[i][mt][h][0], low[i][mt][h][0]);
+                    p[C::LDP] = bw_total<NT>(acc[i][mt][h][1], low[i][mt][h][1]);
+                    p[8] = bw_total<NT>(acc[i][mt][h][2], low[i][mt][h][2]);
+                    p[C::LDP + 8] = bw_total<NT>(acc[i][mt][h][3], low[i][mt][h][3]);
+                }
     }
 }
 
@@ -396,9 +422,24 @@ __device__ __noinline__ void bw_walk_tokens(const BlockWalk& a, const float* row
     }
 }
 
+// The request with the n-th longest portion (of equal ones the first counts as the longer), for up to 32 requests; beyond, the
+// n-th: CTAs start in this order, so a walk of many blocks does not begin when the short ones have ended.
+__device__ __forceinline__ int bw_nth_longest(const int* __restrict__ q_start, int S, int n) {
+    if (S == 1 || S > 32) return n;
+    const int lane = threadIdx.x & 31, len = lane < S ? q_start[lane + 1] - q_start[lane] : -1;
+    int rank = 0;
+    for (int j = 0; j < S; ++j) {
+        const int other = __shfl_sync(0xffffffffu, len, j);
+        rank += other > len || (other == len && j < lane);
+    }
+    return __ffs(__ballot_sync(0xffffffffu, lane < S && rank == n)) - 1;
+}
+
 __device__ __forceinline__ bool bw_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
-// Eight warps hold the state, bring the blocks and make the results.  With HELP eight more bring the blocks and turn a
+// Eight warps hold the state, bring the blocks and make the results.  Without the delta rule a block's u depends on no state, so
+// A u is a product on the tensor cores too (three fragments, by three warps) and the sums over the warps' rows are added up
+// beside the next block, behind its one barrier.  With HELP eight more bring the blocks and turn a
 // block's partial sums into results while the state warps, which then do only what the next block waits for, are at the next
 // one.  A helper passes DONE of block i before it refills the stage of block i - 1 (whose update came before) with block
 // i + 2, makes block i's results and then reports block i + 2 FULL, so the state warps write block i + 2's sums over block
@@ -409,13 +450,15 @@ __device__ __forceinline__ bool bw_finite(float x) { return fabsf(x) <= 3.402823
 template <int NT, int MT, bool DELTA, bool HELP>
 __global__ void __launch_bounds__((HELP ? 2 : 1) * BW_THREADS, HELP ? 1 : 2)
 block_walk_kernel(const __grid_constant__ BlockWalk a) {
-    using C = BwSmem<NT, MT, HELP>;
+    using C = BwSmem<NT, MT, DELTA, HELP>;
     constexpr int COLS = 16 * MT;
+    constexpr bool PIPE = !DELTA;                               // a block's results are made beside the next block
+    static_assert(!PIPE || (MT == 1 && !HELP), "without the delta rule 16 columns and no helpers");
     extern __shared__ __align__(16) float bw_smem[];
     float* part_p = bw_smem + C::STAGES * C::STAGE;
-    float* parts_r = part_p + C::PART;
-    float* us = parts_r + C::TURNS * C::PART;
-    const int s = blockIdx.z, h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
+    float* parts_r = part_p + (DELTA ? C::PART : 0);
+    float* us = parts_r + C::TURNS * C::SUMS;
+    const int s = bw_nth_longest(a.q_start, a.S, blockIdx.z), h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
     if (t1 <= t0 || (a.alone && t1 - t0 == 1)) return;
     const int tid = threadIdx.x & (BW_THREADS - 1), warp = tid >> 5, lane = tid & 31;
     const int col0 = blockIdx.x * COLS, cols = a.V - col0 < COLS ? a.V - col0 : COLS;
@@ -426,26 +469,61 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
     const int v_col = (a.act ? 2 * a.G * a.N : a.v_off) + h * a.V + col0;
     const float* coef = a.coef + ((size_t)bw_first_block(a.q_start, s) * a.heads + h) * BW_COEF;
     const size_t coef_step = (size_t)a.heads * BW_COEF;
+    // What a thread copies of a whole block lies in the same place of every block: one address a row piece and one of v, A or M,
+    // moved on by a block each time.  (Looked up block by block, the copies took a fifth of the walk's instructions.)
+    constexpr int PIECES = 16 * NT, ROWS = BW_THREADS / PIECES;  // 16-byte pieces of a row of q or k; rows at a time
+    const int mrow = tid / PIECES, mcol = tid % PIECES * 4, side = tid - 64 * MT;
+    const float* from = rows + (size_t)(t0 + mrow) * ld + q_col + mcol;
+    const float* from2 = side < 0 ? rows + (size_t)(t0 + tid / (4 * MT)) * ld + v_col + tid % (4 * MT) * 4 : coef + side * 4;
+    const bool has = mcol < a.N, has2 = side < 0 ? tid % (4 * MT) * 4 < cols : side < (DELTA ? 128 : 64);
+    const long from2_step = side < 0 ? BW_B * ld : (long)coef_step, k_minus_q = k_col - q_col;
+    const int to2 = side < 0 ? 2 * C::QK + tid / (4 * MT) * C::LDV + tid % (4 * MT) * 4
+                             : 2 * C::QK + BW_B * C::LDV + (side >> 2) * BW_LD + (side & 3) * 4;          // M's rows follow A's
     auto fetch = [&](int t, int stage) {                        // the next block in order, which starts at token t
-        bw_fetch<NT, MT, DELTA, HELP>(bw_smem + stage * C::STAGE, a, rows, ld, q_col, k_col, v_col, cols, coef, t, t1, tid);
+        float* buf = bw_smem + stage * C::STAGE;
+        if (t + BW_B <= t1) {
+            if (has) {
+                float* to = buf + mrow * C::LDN + mcol;
+#pragma unroll
+                for (int i = 0; i < BW_B / ROWS; ++i) {
+                    bw_cp16(to + i * ROWS * C::LDN, from + i * ROWS * ld);
+                    bw_cp16(to + C::QK + i * ROWS * C::LDN, from + k_minus_q + i * ROWS * ld);
+                }
+            }
+            if (has2) bw_cp16(buf + to2, from2);
+            if (tid < BW_TAIL / 4) bw_cp16(buf + C::G_AT + tid * 4, coef + 512 + tid * 4);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        } else {
+            bw_fetch<NT, MT, DELTA, HELP>(buf, a, rows, ld, q_col, k_col, v_col, cols, coef, t, t1, tid);
+        }
+        from += BW_B * ld;
+        from2 += from2_step;
         coef += coef_step;
     };
+    if (a.N < 64 * NT || cols < COLS) {                         // columns that no block brings
+        for (int i = threadIdx.x; i < C::STAGES * C::STAGE; i += (HELP ? 2 : 1) * BW_THREADS) bw_smem[i] = 0.f;
+        __syncthreads();
+    }
     const float skip = a.skip_any != nullptr ? load_dyn(a.skip_any, a.skip_dt, h) : 0.f;
     bool odd = false;                                           // a number that is not finite has been seen
     auto results = [&](int t, int stage, int turn) {            // thread = column tid % COLS of token tid / COLS and, with MT, eight on
         const int col = tid % COLS, tok = tid / COLS;
         const float* sv = bw_smem + stage * C::STAGE + 2 * C::QK;
         const float* sA = sv + BW_B * C::LDV;
-        const float* gam = sA + 2 * BW_B * BW_LD;
-        const float* u = (DELTA ? us + turn * C::U : sv) + col;
+        const float* gam = bw_smem + stage * C::STAGE + C::G_AT;
+        const float* u = us + turn * C::U + col;
         float o0[MT], o1[MT];
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-            o0[m] = gam[tok + 8 * m] * bw_sum_parts<C::LDP>(parts_r + turn * C::PART, tok + 8 * m, col);
+            o0[m] = gam[tok + 8 * m] * bw_sum_parts<C::LDP>(parts_r + turn * C::SUMS, tok + 8 * m, col);
             o1[m] = skip * sv[(tok + 8 * m) * C::LDV + col];
         }
+        if (PIPE) {                                             // A u was made on the tensor cores; the later tokens reach no earlier result
+            const float* au = parts_r + turn * C::SUMS + C::PART + tok * C::LDP + col;
+            o1[0] += tok < BW_B / 2 ? au[0] : au[0] + au[BW_B * C::LDP];
+        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < (PIPE ? 0 : 4); ++j) {
             const float u0 = u[(4 * j) * C::LDV], u1 = u[(4 * j + 1) * C::LDV], u2 = u[(4 * j + 2) * C::LDV], u3 = u[(4 * j + 3) * C::LDV];
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
@@ -497,7 +575,11 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
 
     // ---------------------------------------------------------------------- the state
     // thread (g, tq) of a warp holds columns g and g + 8 of every 16, rows 2 tq and 2 tq + 1 of every fragment
-    if (!HELP) fetch(t0, 0);
+    if (!HELP) {
+        fetch(t0, 0);
+        if (t0 + BW_B < t1) fetch(t0 + BW_B, 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     const int g = lane >> 2, tq = lane & 3, row0 = warp * 8 * NT;
     float* st = a.state + (size_t)a.slots[s] * a.state_stride + a.s_off + (size_t)h * a.N * a.V;
     const long sr = a.state_vn ? 1 : a.V, sc = a.state_vn ? a.N : 1;
@@ -515,15 +597,17 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
         if (HELP) {
             bw_sync(BW_BAR_FULL + b, 2 * BW_THREADS);
         } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();                                    // the block's rows are here, and everyone has left the block before
-            if (t + BW_B < t1) fetch(t + BW_B, b ^ 1);
+            const int ahead = b + 2 < C::STAGES ? b + 2 : b + 2 - C::STAGES;
+            if (t + 2 * BW_B < t1) fetch(t + 2 * BW_B, ahead);
+            else asm volatile("cp.async.commit_group;" ::: "memory");
         }
         const float* sq = bw_smem + b * C::STAGE;
         const float* sk = sq + C::QK;
         const float* sv = sk + C::QK;
-        const float* sM = sv + BW_B * C::LDV + BW_B * BW_LD;
-        const float* gam = sM + BW_B * BW_LD;
+        const float* sM = sq + C::M_AT;
+        const float* gam = sq + C::G_AT;
         const float* suf = gam + BW_B;
         uint32_t sh[MT][NT][4], sl[MT][NT][4];
 #pragma unroll
@@ -538,7 +622,9 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
         const float* u = sv;
         if (DELTA) {
             float* su = us + turn * C::U;
-            bw_read_out<NT, MT>(sk, sh, sl, part_p + warp * BW_B * C::LDP, row0, g, tq);
+            const float* const in[2] = {sk, sq};
+            float* const to[2] = {part_p + warp * BW_B * C::LDP, parts_r + turn * C::SUMS + warp * BW_B * C::LDP};
+            bw_read_out<NT, MT, 2>(in, sh, sl, to, row0, g, tq);
             HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();
             // thread: token lane % 16 of column tid / 16 of every 16; the 16 tokens of a column meet in half a warp
             const int tok = lane & 15;
@@ -560,8 +646,33 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
             }
             u = su;
         }
-        bw_read_out<NT, MT>(sq, sh, sl, parts_r + turn * C::PART + warp * BW_B * C::LDP, row0, g, tq);
-        HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();     // u and the partial sums of r are there
+        if (!DELTA) {
+            const float* const in[1] = {sq};
+            float* const to[1] = {parts_r + turn * C::SUMS + warp * BW_B * C::LDP};
+            bw_read_out<NT, MT, 1>(in, sh, sl, to, row0, g, tq);
+        }
+        if (PIPE && warp < 3) {                                 // A u: tokens 8 hh .. of the earlier (ks 0) and later (ks 1) half of the u
+            const int ks = warp >> 1, hh = warp > 0, j = ks * 8 + tq;
+            const float* A = sv + BW_B * C::LDV + (hh * 8 + g) * BW_LD + j;
+            const float* uj = sv + j * C::LDV + g;
+            uint32_t ah[4], al[4], bh[2], bl[2];
+            bw_split(uj[0], ah[0], al[0]);
+            bw_split(uj[8], ah[1], al[1]);
+            bw_split(uj[4 * C::LDV], ah[2], al[2]);
+            bw_split(uj[4 * C::LDV + 8], ah[3], al[3]);
+            bw_split(A[0], bh[0], bl[0]);
+            bw_split(A[4], bh[1], bl[1]);
+            float acc[4] = {}, low[4] = {};
+            bw_mma3(acc, low, ah, al, bh, bl);
+            float* p = parts_r + turn * C::SUMS + C::PART + (ks * BW_B + hh * 8 + 2 * tq) * C::LDP + g;
+            p[0] = bw_total<1>(acc[0], low[0]);
+            p[C::LDP] = bw_total<1>(acc[1], low[1]);
+            p[8] = bw_total<1>(acc[2], low[2]);
+            p[C::LDP + 8] = bw_total<1>(acc[3], low[3]);
+        }
+        if (HELP) bw_sync(BW_BAR_STATE, BW_THREADS);            // u and the partial sums of r are there
+        else if (!PIPE) __syncthreads();
+        else if (t > t0) results(t - BW_B, b == 0 ? C::STAGES - 1 : b - 1, turn ^ 1);
         if (HELP) bw_arrive(BW_BAR_DONE + turn, 2 * BW_THREADS);
         uint32_t kh[2][NT][2], kl[2][NT][2];
 #pragma unroll
@@ -586,20 +697,24 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
                 bw_split(u0[4 * C::LDV] * w1, ah[2], al[2]);
                 bw_split(u0[4 * C::LDV + 8] * w1, ah[3], al[3]);
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) bw_mma3(up[nt], low[nt], ah, al, kh[ks][nt], kl[ks][nt]);
+                for (int nt = 0; nt < NT; ++nt) bw_mma(low[nt], al, kh[ks][nt]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) bw_mma(up[nt], ah, kh[ks][nt]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) bw_mma(low[nt], ah, kl[ks][nt]);
             }
-            if (!HELP && mt == MT - 1) results(t, b, 0);
+            if (!HELP && !PIPE && mt == MT - 1) results(t, b, 0);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[mt][nt][e] = fmaf(total, S[mt][nt][e], fmaf(rest, S[mt][nt][e], bw_total<2>(up[nt][e], low[nt][e])));
         }
-        if (HELP) {
-            b = b == 2 ? 0 : b + 1;
-            turn ^= 1;
-        } else {
-            b ^= 1;
-        }
+        b = b == C::STAGES - 1 ? 0 : b + 1;
+        if (C::TURNS == 2) turn ^= 1;
+    }
+    if (PIPE) {
+        __syncthreads();                                        // the last block's partial sums are there
+        results(t0 + (t1 - t0 - 1) / BW_B * BW_B, b == 0 ? C::STAGES - 1 : b - 1, turn ^ 1);
     }
 #pragma unroll
     for (int f = 0; f < MT * NT; ++f)
@@ -620,7 +735,7 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
 
 template <int NT, int MT, bool DELTA, bool HELP>
 static int launch_block_walk(const BlockWalk& a, cudaStream_t stream) {
-    constexpr int bytes = BwSmem<NT, MT, HELP>::TOTAL * 4;
+    constexpr int bytes = BwSmem<NT, MT, DELTA, HELP>::TOTAL * 4;
     auto kern = block_walk_kernel<NT, MT, DELTA, HELP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
     kern<<<dim3((a.V + 16 * MT - 1) / (16 * MT), a.heads, a.S), (HELP ? 2 : 1) * BW_THREADS, bytes, stream>>>(a);
