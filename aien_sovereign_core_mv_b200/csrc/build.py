@@ -1,12 +1,14 @@
 """Compiles the engine's native code in-tree and loads it.
 
-Two artefacts, both under ``<package>/_build`` (or ``$AIEN_B200_BUILD_DIR``, or a per-user
+Three artefacts, all under ``<package>/_build`` (or ``$AIEN_B200_BUILD_DIR``, or a per-user
 folder in the temporary directory when the package folder is read-only):
 
 * ``libaien_kernels.so``: every ``csrc/kernels/*.cu`` compiled by ``nvcc`` for sm_100a
   (``-gencode arch=compute_100a,code=sm_100a``), loaded with ``ctypes``;
 * ``_aien_host*.so``: the C++ cache manager and scheduler (``csrc/host/*.cpp``) behind
-  pybind11, compiled by ``g++``.
+  pybind11, compiled by ``g++``;
+* ``_aien_launch*.so``: the callers of the kernels' entry points (``csrc/launch/launch.cpp`` and a
+  table made from ``csrc/signatures.py``), compiled by ``g++`` against torch's headers.
 
 Nothing is fetched and nothing outside the build folder is written, so the first call works in
 a fresh checkout for any user, with or without a home directory.  A content hash of the
@@ -33,6 +35,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 _PKG = os.path.dirname(_HERE)
 KERNEL_DIR = os.path.join(_HERE, "kernels")
 HOST_DIR = os.path.join(_HERE, "host")
+LAUNCH_DIR = os.path.join(_HERE, "launch")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
@@ -231,7 +234,55 @@ def build_host(force: bool = False) -> str:
     return lib
 
 
+def _launch_table() -> str:
+    """One caller per list of argument types: the C++ that ``launch.cpp`` includes."""
+    from .signatures import SIGNATURES
+    types = {"P": ("void*", "a[%d].p"), "I": ("int", "(int)a[%d].l"), "L": ("long", "a[%d].l"), "Z": ("size_t", "(size_t)a[%d].l"),
+             "F": ("float", "(float)a[%d].d"), "D": ("double", "a[%d].d")}
+    rows = []
+    for sig in sorted(set(SIGNATURES.values())):
+        rows.append('{"%s", [](void* f, const Arg* a) { return ((int (*)(%s))f)(%s); }},\n' % (
+            sig, ", ".join(types[c][0] for c in sig), ", ".join(types[c][1] % i for i, c in enumerate(sig))))
+    return "".join(rows)
+
+
+def build_launch(force: bool = False) -> str:
+    """Compile the callers of the kernels' entry points into a Python module; returns its path."""
+    import torch                                               # its headers, and the libraries that the module resolves against
+    out_dir = build_dir()
+    source = os.path.join(LAUNCH_DIR, "launch.cpp")
+    table = _launch_table()
+    lib = os.path.join(out_dir, "_aien_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    stamp = lib + ".stamp"
+    root = os.path.dirname(torch.__file__)
+    flags = [*CXX_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    digest = _hash_sources([source], flags + [torch.__version__, table])
+    if not force and os.path.exists(lib) and os.path.exists(stamp) and open(stamp).read().strip() == digest:
+        return lib
+    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        raise BuildError("no C++ compiler found (g++)")
+    _say(f"compiling the launch callers into {out_dir}")
+    made = os.path.join(out_dir, f"launch.{os.getpid()}")      # a folder of this process: the table is found as an include
+    os.makedirs(made, exist_ok=True)
+    with open(os.path.join(made, "signatures.inc"), "w") as f:
+        f.write(table)
+    tmp = lib + f".{os.getpid()}.tmp"
+    inc = os.path.join(root, "include")
+    cmd = [cxx, *flags, "-I", made, "-I", inc, "-I", os.path.join(inc, "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
+           source, "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-o", tmp]
+    try:
+        _run_parallel([cmd], "launch", jobs=1)
+    finally:
+        shutil.rmtree(made, ignore_errors=True)
+    os.replace(tmp, lib)
+    with open(stamp, "w") as f:
+        f.write(digest)
+    return lib
+
+
 _KERNELS: Optional[ctypes.CDLL] = None
+_LAUNCH = None
 _HOST = None
 
 
@@ -240,6 +291,18 @@ def load_kernels() -> ctypes.CDLL:
     if _KERNELS is None:
         _KERNELS = ctypes.CDLL(build_kernels())
     return _KERNELS
+
+
+def load_launch():
+    global _LAUNCH
+    if _LAUNCH is None:
+        path = build_launch()
+        import torch  # noqa: F401  (its libraries come first)
+        spec = importlib.util.spec_from_file_location("_aien_launch", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _LAUNCH = mod
+    return _LAUNCH
 
 
 def load_host():
@@ -255,6 +318,7 @@ def load_host():
 
 def build_all(force: bool = False) -> None:
     build_host(force)
+    build_launch(force)
     build_kernels(force)
 
 

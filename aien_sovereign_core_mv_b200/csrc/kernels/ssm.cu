@@ -61,7 +61,7 @@ struct Segments {
 template <int LANES, int CH>
 struct ScanCfg {
     static constexpr int NP = LANES * CH;
-    static constexpr int TOKENS = NP > 32 ? 16 : 32;                    // of a stage; two stages and the sums fit in 48 KB
+    static constexpr int TOKENS = NP > 32 || LANES == 4 ? 16 : 32;      // of a stage; two stages and the sums fit in 48 KB
     static constexpr int CPB = SSM_THREADS / LANES;                     // channels of a CTA
     static constexpr int ROWS = TOKENS * CPB;                           // one of dt, x, z
     static constexpr int STAGE = 3 * ROWS + TOKENS * 2 * NP;            // dt | x | z | (B | C) per token
@@ -79,15 +79,15 @@ struct ScanRowsIn {
 };
 
 // The rows of tokens t .. t + TOKENS - 1 of channels c0 .. c0 + CPB - 1, in pieces of UNIT (dt, x, z) and UBC (B, C)
-// numbers; zeros behind t1 and behind the last channel.
-template <int LANES, int CH, int UNIT, int UBC>
+// numbers; zeros behind t1 and behind the last channel.  FIRST: no z and no C, which only results need.
+template <int LANES, int CH, int UNIT, int UBC, bool FIRST>
 __device__ __forceinline__ void scan_fetch_units(float* __restrict__ buf, const ScanRowsIn& in, int c0, int inner, int N, int t, int t1) {
     using C = ScanCfg<LANES, CH>;
-    constexpr int per = C::CPB / UNIT, pb = C::NP / UBC;
+    constexpr int per = C::CPB / UNIT, pb = C::NP / UBC, pr = FIRST ? pb : 2 * pb;
     const float* src[3] = {in.dtz, in.x, in.z};
     const long ld[3] = {in.lddt, in.ldx, in.ldz};
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < (FIRST ? 2 : 3); ++a)
 #pragma unroll 1
         for (int i = threadIdx.x; i < C::TOKENS * per; i += SSM_THREADS) {
             const int tok = i / per, c = i % per * UNIT;
@@ -96,19 +96,19 @@ __device__ __forceinline__ void scan_fetch_units(float* __restrict__ buf, const 
         }
     float* rows = buf + 3 * C::ROWS;
 #pragma unroll 1
-    for (int i = threadIdx.x; i < C::TOKENS * 2 * pb; i += SSM_THREADS) {
-        const int tok = i / (2 * pb), r = i % (2 * pb), which = r >= pb, n = (r - which * pb) * UBC;
+    for (int i = threadIdx.x; i < C::TOKENS * pr; i += SSM_THREADS) {
+        const int tok = i / pr, r = i % pr, which = r >= pb, n = (r - which * pb) * UBC;
         const bool ok = t + tok < t1 && n < N;
         scan_cp(rows + tok * 2 * C::NP + which * C::NP + n, ok ? in.bc + (t + tok) * in.ldbc + (which ? in.c_off : in.b_off) + n : in.bc, UBC == 4, ok);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-template <int LANES, int CH>
+template <int LANES, int CH, bool FIRST>
 __device__ __forceinline__ void scan_fetch(float* __restrict__ buf, const ScanRowsIn& in, int c0, int inner, int N, int t, int t1) {
-    if (in.wide && in.wide_bc) scan_fetch_units<LANES, CH, 4, 4>(buf, in, c0, inner, N, t, t1);
-    else if (in.wide_bc) scan_fetch_units<LANES, CH, 1, 4>(buf, in, c0, inner, N, t, t1);
-    else scan_fetch_units<LANES, CH, 1, 1>(buf, in, c0, inner, N, t, t1);
+    if (in.wide && in.wide_bc) scan_fetch_units<LANES, CH, 4, 4, FIRST>(buf, in, c0, inner, N, t, t1);
+    else if (in.wide_bc) scan_fetch_units<LANES, CH, 1, 4, FIRST>(buf, in, c0, inner, N, t, t1);
+    else scan_fetch_units<LANES, CH, 1, 1, FIRST>(buf, in, c0, inner, N, t, t1);
 }
 
 // exp for the decays: full precision where the result leaves in float32; through the special-function unit (relative
@@ -148,7 +148,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
     const int cl = threadIdx.x / LANES, ln = threadIdx.x % LANES, n0 = ln * CH;
     const int c0 = blockIdx.x * C::CPB, c = c0 + cl < inner ? c0 + cl : inner - 1;      // lanes beyond the last channel write nothing
     const bool live = c0 + cl < inner;
-    scan_fetch<LANES, CH>(bufs[0], in, c0, inner, N, t0, t1);
+    scan_fetch<LANES, CH, FIRST>(bufs[0], in, c0, inner, N, t0, t1);
     float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)c * N + n0;
     const size_t so = ((seg0 + seg) * inner + c) * N + n0;
     const float* init = sg.mode == 2 ? (seg > 0 ? sg.end + so - (size_t)inner * N : sg.decay + so) : st;      // see segment_combine_kernel
@@ -168,7 +168,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
     for (int t = t0; t < t1; t += C::TOKENS, b ^= 1) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (t + C::TOKENS < t1) scan_fetch<LANES, CH>(bufs[b ^ 1], in, c0, inner, N, t + C::TOKENS, t1);
+        if (t + C::TOKENS < t1) scan_fetch<LANES, CH, FIRST>(bufs[b ^ 1], in, c0, inner, N, t + C::TOKENS, t1);
         const int n_tok = t1 - t < C::TOKENS ? t1 - t : C::TOKENS;
         const float* rows = bufs[b];
 #pragma unroll
@@ -185,13 +185,24 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
             if (FIRST) dts += dd.x;
             if (CH % 2 == 0) {
                 float2 ys = make_float2(0.f, 0.f);
+                float bv[CH], cv[CH];
+#pragma unroll
+                for (int i = 0; i < CH; i += CH % 4 == 0 ? 4 : 2) {
+                    if (CH % 4 == 0) {
+                        *reinterpret_cast<float4*>(bv + i) = *reinterpret_cast<const float4*>(br + i);
+                        if (!FIRST) *reinterpret_cast<float4*>(cv + i) = *reinterpret_cast<const float4*>(br + C::NP + i);
+                    } else {
+                        *reinterpret_cast<float2*>(bv + i) = *reinterpret_cast<const float2*>(br + i);
+                        if (!FIRST) *reinterpret_cast<float2*>(cv + i) = *reinterpret_cast<const float2*>(br + C::NP + i);
+                    }
+                }
 #pragma unroll
                 for (int i = 0; i < CH; i += 2) {
-                    const float2 b2 = *reinterpret_cast<const float2*>(br + i), c2 = *reinterpret_cast<const float2*>(br + C::NP + i);
+                    const float2 b2 = make_float2(bv[i], bv[(i + 1) % CH]), c2 = FIRST ? b2 : make_float2(cv[i], cv[(i + 1) % CH]);
                     const float2 e = make_float2(decay_exp<TO>(dd.x * a[i]), decay_exp<TO>(dd.x * a[(i + 1) % CH]));
                     const float2 S2 = __ffma2_rn(e, make_float2(S[i], S[(i + 1) % CH]), __fmul2_rn(make_float2(dd.y, dd.y), b2));
                     S[i] = S2.x; S[(i + 1) % CH] = S2.y;
-                    ys = __ffma2_rn(S2, c2, ys);
+                    if (!FIRST) ys = __ffma2_rn(S2, c2, ys);
                 }
                 return ys.x + ys.y;
             }
@@ -199,7 +210,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
                 S[i] = fmaf(decay_exp<TO>(dd.x * a[i]), S[i], dd.y * br[i]);
-                y = fmaf(S[i], br[C::NP + i], y);
+                if (!FIRST) y = fmaf(S[i], br[C::NP + i], y);
             }
             return y;
         };
@@ -537,7 +548,12 @@ static int dispatch_selective_scan(const ScanArgs& a) {
         return 0;
     }
     if (N <= 8) launch_selective_scan<8, 1, TO>(a);
-    else if (N <= 16) { if (few) launch_selective_scan<16, 1, TO>(a); else launch_selective_scan<8, 2, TO>(a); }
+    else if (N <= 16) {
+        const char* e = getenv("SCANL"); const int L = e ? atoi(e) : 0;
+        if (L == 4) launch_selective_scan<4, 4, TO>(a);
+        else if (L == 16 || (L == 0 && few)) launch_selective_scan<16, 1, TO>(a);
+        else launch_selective_scan<8, 2, TO>(a);
+    }
     else if (N <= 32) { if (few) launch_selective_scan<16, 2, TO>(a); else launch_selective_scan<8, 4, TO>(a); }
     else if (N <= 64) launch_selective_scan<16, 4, TO>(a);
     else launch_selective_scan<16, 8, TO>(a);

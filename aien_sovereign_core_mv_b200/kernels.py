@@ -1,4 +1,4 @@
-"""Python face of the CUDA kernel library (``csrc/kernels``), loaded with ctypes.
+"""Python face of the CUDA kernel library (``csrc/kernels``), loaded with ctypes and called through ``csrc/launch``.
 
 Every function here takes torch tensors that already live on the device, checks what the
 kernel cannot check for itself, and launches on the current CUDA stream.  Nothing falls back
@@ -7,12 +7,13 @@ to another implementation: a missing library, a refused size or a failed launch 
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_double, c_float, c_int, c_long, c_size_t, c_void_p
+from functools import partial
 from typing import Optional
 
 import torch
 
 from .csrc import build as _build
+from .csrc.signatures import SIGNATURES
 
 F32, BF16 = 0, 1
 _DT = {torch.float32: F32, torch.bfloat16: BF16}
@@ -30,15 +31,29 @@ class KernelError(RuntimeError):
     pass
 
 
-_lib: Optional[ctypes.CDLL] = None
+_lib: Optional["_Callers"] = None
 _proxy = None
 _RECORD: Optional[list] = None
 _QUERIES = ("_supports", "_ranges", "_grid", "_error")     # answer a question, launch nothing
 
 
+class _Callers:
+    """The entry points of ``csrc/signatures.py`` as native callers, which take tensors as they are (``csrc/launch/launch.cpp``);
+    any other symbol is the ctypes function."""
+
+    def __init__(self, cdll: ctypes.CDLL):
+        self._cdll = cdll
+        bind = _build.load_launch().bind
+        for name, types in SIGNATURES.items():
+            setattr(self, name, bind(ctypes.cast(getattr(cdll, name), ctypes.c_void_p).value, types, name))
+
+    def __getattr__(self, name: str):
+        return getattr(self._cdll, name)
+
+
 class _Entry:
-    """One launching entry point.  Calls go to the ctypes function and, while a recording is on,
-    into the list; every attribute (argtypes, restype, ...) is the ctypes function's own, so code
+    """One launching entry point.  Calls go to the function and, while a recording is on, into the list, with tensors as
+    their addresses; every attribute (of a ctypes function argtypes, restype, ...) is the function's own, so code
     that declares a signature on what :func:`lib` hands out declares it on the real thing."""
     __slots__ = ("_fn",)
 
@@ -48,7 +63,7 @@ class _Entry:
     def __call__(self, *args):
         rc = self._fn(*args)
         if _RECORD is not None:
-            _RECORD.append((self._fn, args))
+            _RECORD.append((self._fn, tuple(a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args)))
         return rc
 
     def __getattr__(self, key):
@@ -63,7 +78,7 @@ class _Library:
     launches can be written down as (function, arguments) and issued again by
     :func:`replay_launches` without the Python that chose the arguments."""
 
-    def __init__(self, cdll: ctypes.CDLL):
+    def __init__(self, cdll):
         self._cdll = cdll
 
     def __getattr__(self, name: str):
@@ -75,10 +90,10 @@ class _Library:
 
 def lib():
     """The loaded library; while launches are being written down, with its launching entry points wrapped."""
-    global _lib, _proxy
+    global _lib, _proxy, _dev
     if _proxy is None:
-        _lib = _build.load_kernels()
-        _declare(_lib)
+        _lib = _Callers(_build.load_kernels())
+        _dev = partial(_build.load_launch().on_device, KernelError)
         _proxy = _Library(_lib)
     return _lib if _RECORD is None else _proxy
 
@@ -106,136 +121,15 @@ def replay_launches(plan: list) -> None:
     _launches += len(plan)
 
 
-def _declare(l: ctypes.CDLL) -> None:
-    P, I, L, F = c_void_p, c_int, c_long, c_float
-    sigs = {
-        "aien_embed_gather": [P, I, P, P, I, I, I, P],
-        "aien_add_rmsnorm": [P, P, I, I, c_size_t, P, I, F, P, I, I, I, P],
-        "aien_add_layernorm": [P, P, I, I, c_size_t, P, I, F, P, I, I, I, P],
-        "aien_gather_add_rows": [P, P, I, I, c_size_t, P, P, I, I, P],
-        "aien_swiglu": [P, P, I, I, I, I, I, P],
-        "aien_add_residual": [P, P, I, I, c_size_t, I, I, P],
-        "aien_rope_table": [P, P, P, P, I, I, c_double, P],
-        "aien_qk_norm_rope_kv_write": [P, L, I, P, L, P, L, I, I, I, c_size_t, P, L, I, P, P, I, F, P, P, I, P, P, P, I, I, I, P],
-        "aien_convert": [P, I, P, I, c_size_t, P],
-        "aien_gemm_simple": [P, I, L, P, I, L, P, I, L, I, I, I, P],
-        "aien_paged_attention_generic": [P, L, P, P, P, I, P, P, P, L, I, I, I, I, I, F, I, I, I, I, P, I, P, P, P, P, L, F, I, I, P],
-        "aien_branch_norm_add": [P, P, I, I, c_size_t, P, I, I, c_size_t, P, I, F, P, I, I, I, P],
-        "aien_stream_norm_inplace": [P, P, I, F, P, I, I, I, I, P],
-        "aien_qk_rope_pairs_unit_kv_write": [P, L, I, P, L, P, L, I, I, I, c_size_t, P, L, I, I, I, F, P, P, I, P, P, P, I, I, I, P],
-        "aien_moe_route": [P, I, I, I, I, I, I, P, P, P, P],
-        "aien_moe_expert_up": [P, I, L, P, I, P, P, P, I, I, I, I, I, I, I, I, P],
-        "aien_moe_expert_down": [P, I, P, I, P, P, P, I, I, I, I, P],
-        "aien_act_rows": [P, I, c_size_t, I, P],
-        "aien_moe_plan_rows": [P, I, I, P, P, P, P],
-        "aien_moe_place_rows": [P, L, P, P, P, I, I, P, I, P, P, P],
-        "aien_moe_expert_rows_bf16": [I, P, L, P, P, P, P, I, I, I, I, I, I, P],
-        "aien_gemm_tc_grouped": [P, L, P, L, I, P, I, L, P, I, P, P, I, I, I, P],
-        "aien_argmax_rows": [P, I, I, P, P],
-        "aien_sample_rows": [P, I, I, P, P, P, P, P, P, P, P, P],
-        "aien_sample_rows_logprob": [P, I, I, P, P, P, P, P, P, P, P, P, P],
-        "aien_gemv_bf16": [P, L, P, L, P, I, L, I, I, I, I, I, c_size_t, P],
-        "aien_gemv_stream_bf16": [P, L, P, L, P, I, L, I, I, I, I, I, c_size_t, P],
-        "aien_gemv_stream_error": [],
-        "aien_gemm_tc": [P, L, P, L, P, I, L, I, I, I, I, I, c_size_t, P],
-        "aien_gemm_tc_ranges": [I, I],
-        "aien_gemm_tc_m256_supports": [I, I, I, I],
-        "aien_gemv_stream_scaled": [P, L, P, L, P, I, L, I, I, I, I, P, I, F, P],
-        "aien_gemv_stream_residual": [P, L, P, L, P, L, P, I, P, L, P, I, I, I, P],
-        "aien_gemv_stream_grid": [I],
-        "aien_feed_token_ids": [P, P, P, I, P],
-        "aien_copy_spans": [P, c_size_t, I, c_size_t, c_size_t, c_size_t, P],
-        "aien_zero_fill": [P, c_size_t, P],
-        "aien_scale_rows_ssq": [P, L, P, I, F, P, L, I, I, P],
-        "aien_gemm_tc_error": [],
-        "aien_attention_prefill_tc_error": [],
-        "aien_paged_attention_prefill": [P, L, P, P, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, I, P, P],
-        "aien_paged_attention_prefill_tc": [P, L, I, P, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, P],
-        "aien_paged_attention_prefill_tc_split": [P, L, I, P, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, P, L, I, I, P],
-        "aien_paged_attention_prefill_tc_supports": [I, I],
-        "aien_paged_attention_prefill_tc_masked": [P, L, I, P, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, P, L, I, I, I, P, P],
-        "aien_paged_attention_decode": [P, L, P, P, P, I, P, P, P, P, L, P, P, P, I, I, I, I, I, F, I, I, P],
-        "aien_paged_attention_decode_masked": [P, L, P, P, P, I, P, P, P, P, L, P, P, P, I, I, I, I, I, F, I, I, I, P, P],
-        "aien_paged_attention_decode_terms": [P, L, P, P, P, I, P, P, P, P, L, P, P, P, I, I, I, I, I, F, I, I, P, P, P, L, F, P],
-        "aien_paged_attention_prefill_tc_terms": [P, L, I, P, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, P, L, I, I, I, P, P, P, P, L, F, P],
-        "aien_paged_attention_decode_stream": [P, L, P, P, I, P, I, P, P, P, P, L, P, P, P, I, I, I, I, I, F, I, I, P],
-        "aien_paged_attention_decode_stream_supports": [I, I, I, I, I],
-        "aien_attention_decode_stream_error": [],
-        "aien_collect_wait_errors": [P, P],
-        "aien_decay_linear_attention": [P, I, L, I, I, I, P, P, P, P, P, P, L, I, I, I, I, I, P],
-        "aien_gated_rmsnorm": [P, L, P, I, L, P, I, F, P, I, L, I, I, P],
-        "aien_gated_recurrence": [P, I, L, I, I, I, P, P, I, P, P, P, P, P, I, L, I, I, I, P],
-        "aien_decay_linear_attention_chunked": [P, I, L, I, I, I, P, P, P, P, P, P, L, P, I, I, I, I, I, P],
-        "aien_latent_prepare": [P, I, L, I, P, P, I, F, P, I, L, I, I, I, I, P, P, P, P, I, I, P],
-        "aien_rotate_pairs_rows": [P, I, L, L, P, I, L, L, I, I, I, I, P, P, P],
-        "aien_latent_attention_tc": [P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, P, I, P, P, I, P, I, P],
-        "aien_paged_attention_decode_warps_supports": [I, I, I, I, I],
-        "aien_paged_attention_decode_warps": [P, L, P, P, P, I, P, P, P, P, L, I, P, P, I, I, I, I, I, I, I, I, F, F, I, I, I, F, F, F, P],
-        "aien_latent_gather": [P, I, P, I, I, P, P, I, I, I, P, P, P],
-        "aien_head_project_tc": [P, L, L, P, P, I, L, L, I, I, I, I, P, I, L, I, P, P],
-        "aien_latent_attention_tc_supports": [I, I],
-        "aien_head_project": [P, I, L, L, P, I, L, L, P, I, L, L, I, I, I, I, P, I, L, I, P],
-        "aien_latent_attention": [P, L, P, I, P, I, P, P, P, P, I, L, I, I, I, I, I, I, F, P, P],
-        "aien_post_norm_add": [P, P, I, I, c_size_t, P, I, F, F, P, I, F, P, I, I, I, P],
-        "aien_embed_gather_scaled": [P, I, P, P, I, I, I, F, P],
-        "aien_gelu_times_table": [P, I, L, P, I, L, I, P, I, P, I, L, I, I, P],
-        "aien_softcap": [P, c_size_t, F, F, P],
-        "aien_replicate_streams": [P, c_size_t, I, P],
-        "aien_hc_norm": [P, I, P, I, I, c_size_t, P, P, P, I, F, P, I, I, I, P, I, P, P, P, P],
-        "aien_token_shift": [P, P, I, P, P, P, P, P, P, I, I, I, P],
-        "aien_hc_sum_rows": [P, I, I, P, I, I, c_size_t, P, P, P, I, I, P],
-        "aien_embed_gather_sinusoid": [P, I, P, P, P, P, I, I, I, F, P],
-        "aien_attn_conv_prepare": [P, L, I, I, I, I, I, I, P, P, P, I, I, P, P, I, F, I, I, I, P, P, P, P, P, P, P, P, I, P, I, L, I, P],
-        "aien_delta_conv_prepare": [P, L, I, I, I, I, I, I, I, I, I, P, P, P, I, I, P, P, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
-        "aien_delta_rule": [P, L, I, I, I, P, L, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, P],
-        "aien_grouped_gated_rmsnorm": [P, L, P, I, L, P, I, F, P, I, L, I, I, I, I, P],
-        "aien_paged_attention_decode_fused": [P, L, P, L, P, L, P, P, I, F, P, P, I, P, P, P, P, I, P, P, L, P, P, P,
-                                              I, I, I, I, I, F, I, I, P],
-        "aien_conv_act": [P, L, I, I, P, I, P, I, I, I, P, c_size_t, P, P, P, P, P, L, P, L, I, P],
-        "aien_selective_scan": [P, L, P, L, P, L, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, I, L, I, I, I, I, I, I, P, P],
-        "aien_split_rows": [P, L, I, c_size_t, P, P, I, I, I, P],
-        "aien_parts_product": [P, P, L, P, L, I, I, I, P],
-        "aien_ssd_steps": [P, L, P, P, I, P, I, I, P],
-        "aien_block_walk": [P, L, I, I, I, I, P, L, I, I, P, I, P, I, P, c_size_t, c_size_t, I, P, P, P, P, L, I, I, I, I, I, I, I, P, P],
-        "aien_ssd_scan": [P, L, I, I, I, P, L, P, P, P, I, P, c_size_t, c_size_t, P, P, P, P, L, I, I, I, I, I, I, I, I, P, P, I, P],
-        "aien_gate_group_norm": [P, L, P, L, P, I, F, F, P, I, L, I, I, I, P],
-        "aien_scaled_add_rmsnorm": [P, P, I, I, c_size_t, P, P, P, I, F, P, I, I, I, P],
-        "aien_pass_input": [P, P, P, I, I, I, P],
-        "aien_clamped_glu": [P, I, L, I, I, P, P, I, F, F, P, I, L, I, I, P],
-        "aien_sigmoid_gate": [P, I, L, P, L, F, P, I, L, I, I, P],
-        "aien_routed_combine": [P, I, I, c_size_t, P, I, L, P, P, I, I, c_size_t, P, L, P, I, I, P],
-        "aien_moe_route_biased": [P, L, I, I, I, I, I, F, P, I, I, P, P, P, P, P],
-        "aien_sum_terms_rmsnorm": [P, I] + 3 * [P, I, I, c_size_t, P, L] + [P, I, I, P, I, F, P, I, I, I, P],
-        "aien_pass_rows": [P, I] + 3 * [P, I, I, c_size_t, P, L] + [P, P, I, I, I, P],
-        "aien_matrix_memory_gates": [P, L, I, I, P, P, F, P, c_size_t, c_size_t, P, P, P, P, I, I, I, P],
-        "aien_matrix_memory_walk": [P, I, L, I, I, I, F, P, P, c_size_t, P, P, P, P, P, I, I, I, I, P],
-        "aien_matrix_memory_finish": [P, P, P, P, I, L, P, I, F, F, P, I, L, I, I, I, P],
-        "aien_matrix_memory_token_supports": [I, I],
-        "aien_matrix_memory_chunks_supports": [I, I],
-        "aien_matrix_memory_chunked": [P, L, I, I, I, I, F, P, P, c_size_t, P, P, P, P, I, F, F, P, L, P, I, I, I, I, I, P],
-        "aien_matrix_memory_token": [P, I, L, I, I, I, I, F, P, L, I, I, P, P, F, P, c_size_t, P, P, P, P, I, F, F, P, I, L, I, I, I, I, P],
-        "aien_rope_halves_value_write": [P, I, L, I, c_size_t, P, I, I, I, I, I, I, I, I, P, P, I, P, P, I, L, P, P, I, I, P],
-        "aien_map_difference_norm": [P, L, P, I, L, I, I, I, I, F, F, F, P],
-        "aien_paged_attention_decode_values": [P, L, P, P, P, I, P, P, P, P, L, P, P, P, I, I, I, I, I, F, I, I, I, F, I, I, I, I, P],
-        "aien_paged_attention_prefill_tc_values": [P, L, I, P, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, I, F, P, L, I, I, I, P, P, P, P, L, F, I, I, I, L, L, P, L, P],
-        "aien_paged_attention_prefill_tc_values_supports": [I, I, I],
-        "aien_paged_attention_prefill_tc_portions_supports": [I, I, I],
-    }
-    for name, args in sigs.items():
-        fn = getattr(l, name)
-        fn.argtypes = args
-        fn.restype = c_int
-
-
 def declare_optional(name: str, args) -> bool:
     """Declare a symbol that later kernel files add; returns False when the library lacks it."""
     lib()
     try:
-        fn = getattr(_lib, name)
+        fn = getattr(_lib._cdll, name)
     except AttributeError:
         return False
     fn.argtypes = args
-    fn.restype = c_int
+    fn.restype = ctypes.c_int
     return True
 
 
@@ -285,10 +179,6 @@ def _stream() -> int:
     return _STREAM if _STREAM is not None else torch.cuda.current_stream().cuda_stream
 
 
-def _p(t: Optional[torch.Tensor]) -> int:
-    return 0 if t is None else t.data_ptr()
-
-
 def dt(t: torch.Tensor) -> int:
     try:
         return _DT[t.dtype]
@@ -297,6 +187,7 @@ def dt(t: torch.Tensor) -> int:
 
 
 def _dev(*ts: Optional[torch.Tensor]) -> None:
+    """Every tensor lives on the device (:func:`lib` puts the native check in this one's place)."""
     for t in ts:
         if t is not None and not t.is_cuda:
             raise KernelError("kernel arguments must live on the CUDA device (there is no CPU path)")
@@ -309,7 +200,7 @@ def embed_gather(table: torch.Tensor, ids: torch.Tensor, x: torch.Tensor) -> Non
     T, H = x.shape
     assert table.is_contiguous() and x.is_contiguous() and ids.dtype == torch.int32 and x.dtype == torch.float32
     assert table.shape[1] == H and ids.numel() >= T
-    _check(lib().aien_embed_gather(_p(table), dt(table), _p(ids), _p(x), T, H, table.shape[0], _stream()), "embed_gather")
+    _check(lib().aien_embed_gather(table, dt(table), ids, x, T, H, table.shape[0], _stream()), "embed_gather")
 
 
 def _parts_of(delta: Optional[torch.Tensor], shape) -> tuple:
@@ -331,8 +222,8 @@ def add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Te
     assert x.dtype == torch.float32 and x.is_contiguous() and out.is_contiguous() and out.shape == x.shape
     assert weight.numel() == H and weight.is_contiguous()
     nparts, stride = _parts_of(delta, x.shape)
-    _check(lib().aien_add_rmsnorm(_p(x), _p(delta), dt(delta) if delta is not None else F32, nparts, stride,
-                                  _p(weight), dt(weight), float(eps), _p(out), dt(out), T, H, _stream()), "add_rmsnorm")
+    _check(lib().aien_add_rmsnorm(x, delta, dt(delta) if delta is not None else F32, nparts, stride,
+                                  weight, dt(weight), float(eps), out, dt(out), T, H, _stream()), "add_rmsnorm")
 
 
 def add_layernorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor, eps: float, out: torch.Tensor) -> None:
@@ -342,8 +233,8 @@ def add_layernorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.
     assert x.dtype == torch.float32 and x.is_contiguous() and out.is_contiguous() and out.shape == x.shape
     assert weight.numel() == H and weight.is_contiguous()
     nparts, stride = _parts_of(delta, x.shape)
-    _check(lib().aien_add_layernorm(_p(x), _p(delta), dt(delta) if delta is not None else F32, nparts, stride,
-                                    _p(weight), dt(weight), float(eps), _p(out), dt(out), T, H, _stream()), "add_layernorm")
+    _check(lib().aien_add_layernorm(x, delta, dt(delta) if delta is not None else F32, nparts, stride,
+                                    weight, dt(weight), float(eps), out, dt(out), T, H, _stream()), "add_layernorm")
 
 
 def gather_add_rows(x: torch.Tensor, delta: Optional[torch.Tensor], rows: torch.Tensor, out: torch.Tensor) -> None:
@@ -353,8 +244,8 @@ def gather_add_rows(x: torch.Tensor, delta: Optional[torch.Tensor], rows: torch.
     assert x.dtype == torch.float32 and out.dtype == torch.float32 and rows.dtype == torch.int32
     assert x.is_contiguous() and out.is_contiguous() and x.shape[1] == H and rows.numel() >= R
     nparts, stride = _parts_of(delta, x.shape)
-    _check(lib().aien_gather_add_rows(_p(x), _p(delta), dt(delta) if delta is not None else F32, nparts, stride,
-                                      _p(rows), _p(out), R, H, _stream()), "gather_add_rows")
+    _check(lib().aien_gather_add_rows(x, delta, dt(delta) if delta is not None else F32, nparts, stride,
+                                      rows, out, R, H, _stream()), "gather_add_rows")
 
 
 def add_residual(x: torch.Tensor, delta: torch.Tensor) -> None:
@@ -363,7 +254,7 @@ def add_residual(x: torch.Tensor, delta: torch.Tensor) -> None:
     T, H = x.shape
     assert x.dtype == torch.float32 and x.is_contiguous()
     nparts, stride = _parts_of(delta, x.shape)
-    _check(lib().aien_add_residual(_p(x), _p(delta), dt(delta), nparts, stride, T, H, _stream()), "add_residual")
+    _check(lib().aien_add_residual(x, delta, dt(delta), nparts, stride, T, H, _stream()), "add_residual")
 
 
 GATED_ACTS = {"silu": 1, "gelu_tanh": 6}        # act(gate) * up: the products' epilogue that computes it
@@ -375,7 +266,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, group: int = 0, act: str = 
     _dev(gate_up, out)
     T, I = out.shape
     assert gate_up.shape == (T, 2 * I) and gate_up.is_contiguous() and out.is_contiguous() and gate_up.dtype == out.dtype
-    _check(lib().aien_swiglu(_p(gate_up), _p(out), dt(out), T, I, int(group), 1 if act == "gelu_tanh" else 0, _stream()), "swiglu")
+    _check(lib().aien_swiglu(gate_up, out, dt(out), T, I, int(group), 1 if act == "gelu_tanh" else 0, _stream()), "swiglu")
 
 
 def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, mult: float = 1.0) -> None:
@@ -384,7 +275,7 @@ def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, cos: torch.Tenso
     T, half = cos.shape
     assert positions.dtype == torch.int32 and inv_freq.dtype == torch.float64 and inv_freq.numel() == half
     assert cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
-    _check(lib().aien_rope_table(_p(positions), _p(inv_freq), _p(cos), _p(sin), T, half, float(mult), _stream()), "rope_table")
+    _check(lib().aien_rope_table(positions, inv_freq, cos, sin, T, half, float(mult), _stream()), "rope_table")
 
 
 def qk_norm_rope_kv_write(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Tensor], head_dim: int,
@@ -425,9 +316,9 @@ def qk_norm_rope_kv_write(q: torch.Tensor, k: Optional[torch.Tensor], v: Optiona
     if cos is not None:
         assert sin is not None and cos.shape == (T, rotary_dim // 2) and cos.is_contiguous() and sin.is_contiguous()
     _check(lib().aien_qk_norm_rope_kv_write(
-        _p(q), q.stride(-2), nq, _p(k), k.stride(-2) if k is not None else 0, _p(v), v.stride(-2) if v is not None else 0,
-        nkv, dt(q), nparts, part_stride, _p(q_out), q_out.stride(0), head_dim, _p(q_norm_w), _p(k_norm_w), wdt, float(eps),
-        _p(cos), _p(sin), rotary_dim if cos is not None else 0, _p(slot_map), _p(k_cache), _p(v_cache),
+        q, q.stride(-2), nq, k, k.stride(-2) if k is not None else 0, v, v.stride(-2) if v is not None else 0,
+        nkv, dt(q), nparts, part_stride, q_out, q_out.stride(0), head_dim, q_norm_w, k_norm_w, wdt, float(eps),
+        cos, sin, rotary_dim if cos is not None else 0, slot_map, k_cache, v_cache,
         dt(q_out), dt(k_cache) if k_cache is not None else dt(q_out), T, _stream()), "qk_norm_rope_kv_write")
 
 
@@ -438,9 +329,9 @@ def _source(t: Optional[torch.Tensor], shape) -> tuple:
     assert t.is_contiguous()
     if t.dim() == 3:                         # parts [P,T,H], float32 or (the weighted outputs of routed experts) bfloat16
         assert tuple(t.shape[1:]) == tuple(shape)
-        return _p(t), dt(t), t.shape[0], t.shape[1] * t.shape[2]
+        return t, dt(t), t.shape[0], t.shape[1] * t.shape[2]
     assert tuple(t.shape) == tuple(shape)
-    return _p(t), dt(t), 1, 0
+    return t, dt(t), 1, 0
 
 
 def branch_norm_add(x: torch.Tensor, a: torch.Tensor, weight: torch.Tensor, eps: float, b: Optional[torch.Tensor] = None,
@@ -455,8 +346,8 @@ def branch_norm_add(x: torch.Tensor, a: torch.Tensor, weight: torch.Tensor, eps:
         assert h.is_contiguous() and tuple(h.shape) == (T, H)
     pa, da, na, sa = _source(a, x.shape)
     pb, db, nb, sb = _source(b, x.shape)
-    _check(lib().aien_branch_norm_add(_p(x), pa, da, na, sa, pb, db, nb, sb, _p(weight), dt(weight), float(eps),
-                                      _p(h), dt(h) if h is not None else F32, T, H, _stream()), "branch_norm_add")
+    _check(lib().aien_branch_norm_add(x, pa, da, na, sa, pb, db, nb, sb, weight, dt(weight), float(eps),
+                                      h, dt(h) if h is not None else F32, T, H, _stream()), "branch_norm_add")
 
 
 def stream_norm_inplace(x: torch.Tensor, weight: torch.Tensor, eps: float, h: Optional[torch.Tensor] = None, center: bool = False) -> None:
@@ -466,7 +357,7 @@ def stream_norm_inplace(x: torch.Tensor, weight: torch.Tensor, eps: float, h: Op
     assert x.dtype == torch.float32 and x.is_contiguous() and weight.numel() == H and weight.is_contiguous()
     if h is not None:
         assert h.is_contiguous() and tuple(h.shape) == (T, H)
-    _check(lib().aien_stream_norm_inplace(_p(x), _p(weight), dt(weight), float(eps), _p(h), dt(h) if h is not None else F32,
+    _check(lib().aien_stream_norm_inplace(x, weight, dt(weight), float(eps), h, dt(h) if h is not None else F32,
                                           T, H, 1 if center else 0, _stream()), "stream_norm_inplace")
 
 
@@ -498,9 +389,9 @@ def qk_rope_pairs_unit_kv_write(q: torch.Tensor, k: Optional[torch.Tensor], v: O
     if cos is not None:
         assert sin is not None and cos.shape == (T, rotary_dim // 2) and cos.is_contiguous() and sin.is_contiguous()
     _check(lib().aien_qk_rope_pairs_unit_kv_write(
-        _p(q), q.stride(-2), nq, _p(k), k.stride(-2) if k is not None else 0, _p(v), v.stride(-2) if v is not None else 0, nkv,
-        dt(q), nparts, part_stride, _p(q_out), q_out.stride(0), head_dim, int(value_dim), 1 if unit else 0, float(eps),
-        _p(cos), _p(sin), rotary_dim if cos is not None else 0, _p(slot_map), _p(k_cache), _p(v_cache),
+        q, q.stride(-2), nq, k, k.stride(-2) if k is not None else 0, v, v.stride(-2) if v is not None else 0, nkv,
+        dt(q), nparts, part_stride, q_out, q_out.stride(0), head_dim, int(value_dim), 1 if unit else 0, float(eps),
+        cos, sin, rotary_dim if cos is not None else 0, slot_map, k_cache, v_cache,
         dt(q_out), dt(k_cache) if k_cache is not None else dt(q_out), T, _stream()), "qk_rope_pairs_unit_kv_write")
 
 
@@ -520,7 +411,7 @@ def moe_route(z: torch.Tensor, groups: int, keep: int, top: int, renorm: bool, i
     T, E = z.shape
     assert z.dtype == torch.float32 and z.is_contiguous() and ids.dtype == torch.int32 and wts.dtype == torch.float32
     assert ids.is_contiguous() and wts.is_contiguous() and ids.numel() >= T * top and wts.numel() >= T * top
-    _check(lib().aien_moe_route(_p(z), T, E, int(groups), int(keep), int(top), 1 if renorm else 0, _p(ids), _p(wts), _p(expert_count),
+    _check(lib().aien_moe_route(z, T, E, int(groups), int(keep), int(top), 1 if renorm else 0, ids, wts, expert_count,
                                 _stream()), "moe_route")
 
 
@@ -538,7 +429,7 @@ def moe_expert_up(h: torch.Tensor, w_up: torch.Tensor, ids: torch.Tensor, act: t
     Fd = Fd // 2 if gated else Fd
     assert D2 == D and h.stride(1) == 1 and w_up.is_contiguous() and act.is_contiguous() and tuple(act.shape) == (T * top, Fd)
     assert in_wts is None or (in_wts.dtype == torch.float32 and in_wts.is_contiguous() and in_wts.numel() >= T * top)
-    _check(lib().aien_moe_expert_up(_p(h), dt(h), h.stride(0), _p(w_up), dt(w_up), _p(ids), _p(in_wts), _p(act), dt(act), T, int(top), D, Fd,
+    _check(lib().aien_moe_expert_up(h, dt(h), h.stride(0), w_up, dt(w_up), ids, in_wts, act, dt(act), T, int(top), D, Fd,
                                     0 if gated else int(act_kind), 1 if gated else 0, int(group), _stream()), "moe_expert_up")
 
 
@@ -549,7 +440,7 @@ def moe_expert_down(act: torch.Tensor, w_down: torch.Tensor, ids: torch.Tensor, 
     T = act.shape[0] // top
     assert act.is_contiguous() and act.shape[1] == Fd and w_down.is_contiguous()
     assert parts.dtype == torch.float32 and parts.is_contiguous() and tuple(parts.shape) == (top, T, D)
-    _check(lib().aien_moe_expert_down(_p(act), dt(act), _p(w_down), dt(w_down), _p(ids), _p(wts), _p(parts), T, int(top), D, Fd,
+    _check(lib().aien_moe_expert_down(act, dt(act), w_down, dt(w_down), ids, wts, parts, T, int(top), D, Fd,
                                       _stream()), "moe_expert_down")
 
 
@@ -608,9 +499,9 @@ def moe_experts(ctx, h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, 
     parts = ws.take((top, T, D), torch.bfloat16 if grouped else torch.float32)
     if ok and not grouped:
         act = ws.take((T * top, Fd), torch.bfloat16)
-        _check(lib().aien_moe_expert_rows_bf16(2 if gated else 0, _p(h), h.stride(0), _p(w_up), _p(ids), _p(wts if on_input else None), _p(act), T,
+        _check(lib().aien_moe_expert_rows_bf16(2 if gated else 0, h, h.stride(0), w_up, ids, wts if on_input else None, act, T,
                                                top, Fd, D, 0 if gated else int(act_kind), int(group), _stream()), "moe_expert_rows(up)")
-        _check(lib().aien_moe_expert_rows_bf16(1, _p(act), Fd, _p(w_down), _p(ids), _p(None if on_input else wts), _p(parts), T, top, D, Fd,
+        _check(lib().aien_moe_expert_rows_bf16(1, act, Fd, w_down, ids, None if on_input else wts, parts, T, top, D, Fd,
                                                0, 0, _stream()), "moe_expert_rows(down)")
         return parts
     if grouped:
@@ -622,14 +513,14 @@ def moe_experts(ctx, h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, 
         row_scale = ws.take((rows,), torch.float32)
         a_sorted = ws.take((rows, D), torch.bfloat16)
         act = ws.take((rows, Fd), torch.bfloat16)
-        _check(lib().aien_moe_plan_rows(_p(expert_count), E, tiles, _p(cursor), _p(tile_group), _p(row_dest), _stream()), "moe_plan_rows")
-        _check(lib().aien_moe_place_rows(_p(h), h.stride(0), _p(ids), _p(wts), _p(cursor), T, top, _p(a_sorted), D, _p(row_dest),
-                                         _p(row_scale), _stream()), "moe_place_rows")
-        _check(lib().aien_gemm_tc_grouped(_p(a_sorted), D, _p(w_up), D, E, _p(act), BF16, Fd, _p(tile_group), tiles, None,
-                                          _p(row_scale) if on_input else None, w_up.shape[1], D, 1 if gated else 2 + int(act_kind), _stream()),
+        _check(lib().aien_moe_plan_rows(expert_count, E, tiles, cursor, tile_group, row_dest, _stream()), "moe_plan_rows")
+        _check(lib().aien_moe_place_rows(h, h.stride(0), ids, wts, cursor, T, top, a_sorted, D, row_dest,
+                                         row_scale, _stream()), "moe_place_rows")
+        _check(lib().aien_gemm_tc_grouped(a_sorted, D, w_up, D, E, act, BF16, Fd, tile_group, tiles, None,
+                                          row_scale if on_input else None, w_up.shape[1], D, 1 if gated else 2 + int(act_kind), _stream()),
                "gemm_tc_grouped(up)")
-        _check(lib().aien_gemm_tc_grouped(_p(act), Fd, _p(w_down), Fd, E, _p(parts), BF16, D, _p(tile_group), tiles, _p(row_dest),
-                                          None if on_input else _p(row_scale), D, Fd, 0, _stream()), "gemm_tc_grouped(down)")
+        _check(lib().aien_gemm_tc_grouped(act, Fd, w_down, Fd, E, parts, BF16, D, tile_group, tiles, row_dest,
+                                          None if on_input else row_scale, D, Fd, 0, _stream()), "gemm_tc_grouped(down)")
         return parts
     act = ws.take((T * top, Fd), ctx.dtype)
     moe_expert_up(h, w_up, ids, act, top, act_kind, wts if on_input else None, group)
@@ -641,13 +532,13 @@ def act_rows(a: torch.Tensor, act_kind: int) -> None:
     """a = f(a) in place: 0 the erf gelu, 1 the tanh gelu, 2 the square of relu."""
     _dev(a)
     assert a.is_contiguous()
-    _check(lib().aien_act_rows(_p(a), dt(a), a.numel(), int(act_kind), _stream()), "act_rows")
+    _check(lib().aien_act_rows(a, dt(a), a.numel(), int(act_kind), _stream()), "act_rows")
 
 
 def convert(src: torch.Tensor, dst: torch.Tensor) -> None:
     _dev(src, dst)
     assert src.is_contiguous() and dst.is_contiguous() and src.numel() == dst.numel()
-    _check(lib().aien_convert(_p(src), dt(src), _p(dst), dt(dst), src.numel(), _stream()), "convert")
+    _check(lib().aien_convert(src, dt(src), dst, dt(dst), src.numel(), _stream()), "convert")
 
 
 # ---------------------------------------------------------------------------- matrix products
@@ -658,7 +549,7 @@ def gemm_simple(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     N = w.shape[0]
     assert w.shape[1] == K and out.shape == (M, N)
     assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
-    _check(lib().aien_gemm_simple(_p(a), dt(a), a.stride(0), _p(w), dt(w), w.stride(0), _p(out), dt(out), out.stride(0),
+    _check(lib().aien_gemm_simple(a, dt(a), a.stride(0), w, dt(w), w.stride(0), out, dt(out), out.stride(0),
                                   M, N, K, _stream()), "gemm_simple")
 
 
@@ -692,9 +583,9 @@ def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     assert block_table.dtype == torch.int32 and seq_of_token.dtype == torch.int32 and positions.dtype == torch.int32
     assert token_list is None or (token_list.dtype == torch.int32 and token_list.numel() >= T)
     _check(lib().aien_paged_attention_generic(
-        _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(block_table), max_blocks, _p(seq_of_token), _p(positions),
-        _p(out), out.stride(0), num_q_heads, num_kv_heads, head_dim, page_size, window, float(scale),
-        dt(q), dt(k_cache), T, int(chunk), _p(sinks), int(value_dim), _p(token_list), _p(head_scale), _p(slopes), _p(gate),
+        q, q.stride(0), k_cache, v_cache, block_table, max_blocks, seq_of_token, positions,
+        out, out.stride(0), num_q_heads, num_kv_heads, head_dim, page_size, window, float(scale),
+        dt(q), dt(k_cache), T, int(chunk), sinks, int(value_dim), token_list, head_scale, slopes, gate,
         gate.stride(0) if gate is not None else 0, float(softcap or 0.0), int(v_share), dt(out), _stream()), "paged_attention_generic")
 
 
@@ -703,7 +594,7 @@ def argmax_rows(logits: torch.Tensor, out_ids: torch.Tensor) -> None:
     _dev(logits, out_ids)
     R, V = logits.shape
     assert logits.dtype == torch.float32 and logits.is_contiguous() and out_ids.dtype == torch.int32 and out_ids.numel() >= R
-    _check(lib().aien_argmax_rows(_p(logits), R, V, _p(out_ids), _stream()), "argmax_rows")
+    _check(lib().aien_argmax_rows(logits, R, V, out_ids, _stream()), "argmax_rows")
 
 
 def sample_rows(logits: torch.Tensor, temperature: torch.Tensor, top_p: torch.Tensor, top_k: torch.Tensor,
@@ -719,11 +610,11 @@ def sample_rows(logits: torch.Tensor, temperature: torch.Tensor, top_p: torch.Te
     assert scratch.dtype == torch.float32 and scratch.numel() >= R * V and out_ids.dtype == torch.int32
     if out_logprob is not None:
         assert out_logprob.dtype == torch.float32 and out_logprob.numel() >= R and out_logprob.is_contiguous()
-        _check(lib().aien_sample_rows_logprob(_p(logits), R, V, _p(temperature), _p(top_p), _p(top_k), _p(seeds), _p(request_ids),
-                                              _p(positions), _p(scratch), _p(out_ids), _p(out_logprob), _stream()), "sample_rows_logprob")
+        _check(lib().aien_sample_rows_logprob(logits, R, V, temperature, top_p, top_k, seeds, request_ids,
+                                              positions, scratch, out_ids, out_logprob, _stream()), "sample_rows_logprob")
         return
-    _check(lib().aien_sample_rows(_p(logits), R, V, _p(temperature), _p(top_p), _p(top_k), _p(seeds), _p(request_ids),
-                                  _p(positions), _p(scratch), _p(out_ids), _stream()), "sample_rows")
+    _check(lib().aien_sample_rows(logits, R, V, temperature, top_p, top_k, seeds, request_ids,
+                                  positions, scratch, out_ids, _stream()), "sample_rows")
 
 
 # ---------------------------------------------------------------------------- decode product
@@ -769,7 +660,7 @@ def gemv(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 0)
         assert w.shape[1] == K_ and out.shape == (M, N // 2 if epilogue in (1, 6) else N)
     assert epilogue in (0, 1, 6) or gemv_takes_activation(K_)
     fn = lib().aien_gemv_stream_bf16 if (GEMV_IMPL == "stream" and K_ % 64 == 0) else lib().aien_gemv_bf16
-    _check(fn(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), dt(out), out.stride(-2), M, N, K_,
+    _check(fn(a, a.stride(0), w, w.stride(0), out, dt(out), out.stride(-2), M, N, K_,
               epilogue, splits, part_stride, _stream()), "gemv_bf16")
 
 
@@ -831,7 +722,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int =
         splits, part_stride = out.shape[0], M * N
     else:
         assert w.shape[1] == K_ and out.shape == (M, N // 2 if epilogue in (1, 6) else N)
-    _check(lib().aien_gemm_tc(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), dt(out), out.stride(-2), M, N, K_,
+    _check(lib().aien_gemm_tc(a, a.stride(0), w, w.stride(0), out, dt(out), out.stride(-2), M, N, K_,
                               epilogue, splits, part_stride, _stream()), "gemm_tc")
 
 
@@ -923,8 +814,8 @@ def gemv_scaled(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ssq: torch.
     N = w.shape[0]
     assert gemv_stream_fusable(a, w) and ssq.dtype == torch.float32 and ssq.is_contiguous() and ssq.numel() >= parts * 16
     assert out.shape == (M, N // 2 if epilogue else N) and out.stride(1) == 1
-    _check(lib().aien_gemv_stream_scaled(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), dt(out), out.stride(0), M, N, Kd,
-                                         int(epilogue), _p(ssq), int(parts), float(eps), _stream()), "gemv_stream_scaled")
+    _check(lib().aien_gemv_stream_scaled(a, a.stride(0), w, w.stride(0), out, dt(out), out.stride(0), M, N, Kd,
+                                         int(epilogue), ssq, int(parts), float(eps), _stream()), "gemv_stream_scaled")
 
 
 def gemv_residual(a: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, norm_w: torch.Tensor, xw: torch.Tensor, ssq_out: torch.Tensor) -> int:
@@ -937,8 +828,8 @@ def gemv_residual(a: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, norm_w:
     assert gemv_stream_fusable(a, w) and resid.dtype == torch.float32 and resid.shape == (M, N) and resid.stride(1) == 1
     assert xw.dtype == torch.bfloat16 and xw.shape == (M, N) and xw.stride(1) == 1 and norm_w.numel() == N and norm_w.is_contiguous()
     assert ssq_out.dtype == torch.float32 and ssq_out.is_contiguous() and ssq_out.numel() >= parts * 16
-    _check(lib().aien_gemv_stream_residual(_p(a), a.stride(0), _p(w), w.stride(0), _p(resid), resid.stride(0), _p(norm_w), dt(norm_w),
-                                           _p(xw), xw.stride(0), _p(ssq_out), M, N, Kd, _stream()), "gemv_stream_residual")
+    _check(lib().aien_gemv_stream_residual(a, a.stride(0), w, w.stride(0), resid, resid.stride(0), norm_w, dt(norm_w),
+                                           xw, xw.stride(0), ssq_out, M, N, Kd, _stream()), "gemv_stream_residual")
     return parts
 
 
@@ -946,7 +837,7 @@ def feed_token_ids(token_ids: torch.Tensor, src: torch.Tensor, prev: torch.Tenso
     """token_ids[i] = prev[src[i]] where src[i] >= 0 (int32 device tensors)."""
     _dev(token_ids, src, prev)
     assert token_ids.dtype == torch.int32 and src.dtype == torch.int32 and prev.dtype == torch.int32 and src.numel() >= token_ids.numel()
-    _check(lib().aien_feed_token_ids(_p(token_ids), _p(src), _p(prev), token_ids.numel(), _stream()), "feed_token_ids")
+    _check(lib().aien_feed_token_ids(token_ids, src, prev, token_ids.numel(), _stream()), "feed_token_ids")
 
 
 def copy_rows(storage: torch.Tensor, src: int, dst: int, count: int = 1) -> None:
@@ -955,7 +846,7 @@ def copy_rows(storage: torch.Tensor, src: int, dst: int, count: int = 1) -> None
     _dev(storage)
     assert storage.is_contiguous() and storage.dim() >= 2
     row = storage[0, 0].numel() * storage.element_size()
-    _check(lib().aien_copy_spans(_p(storage), storage.shape[1] * row, storage.shape[0], src * row, dst * row, count * row, _stream()),
+    _check(lib().aien_copy_spans(storage, storage.shape[1] * row, storage.shape[0], src * row, dst * row, count * row, _stream()),
            "copy_spans")
 
 
@@ -963,7 +854,7 @@ def zero_fill(t: torch.Tensor) -> torch.Tensor:
     """Zeroes a contiguous device tensor in place (the cache pools at start: the paged kernels load whole pages)."""
     _dev(t)
     assert t.is_contiguous()
-    _check(lib().aien_zero_fill(_p(t), t.numel() * t.element_size(), _stream()), "zero_fill")
+    _check(lib().aien_zero_fill(t, t.numel() * t.element_size(), _stream()), "zero_fill")
     return t
 
 
@@ -972,7 +863,7 @@ def scale_rows_ssq(xw: torch.Tensor, ssq: torch.Tensor, parts: int, eps: float, 
     _dev(xw, ssq, out)
     T, H = xw.shape
     assert xw.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and out.shape == (T, H) and xw.stride(1) == 1 and out.stride(1) == 1
-    _check(lib().aien_scale_rows_ssq(_p(xw), xw.stride(0), _p(ssq), int(parts), float(eps), _p(out), out.stride(0), T, H, _stream()),
+    _check(lib().aien_scale_rows_ssq(xw, xw.stride(0), ssq, int(parts), float(eps), out, out.stride(0), T, H, _stream()),
            "scale_rows_ssq")
 
 
@@ -1033,27 +924,27 @@ def paged_attention_decode(q, k_cache, v_cache, block_table, max_blocks, seq_of_
         assert not chunk and sinks is None
         _check_head_terms(num_q_heads, head_scale, slopes, gate)
         _check(lib().aien_paged_attention_decode_terms(
-            _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(block_table), max_blocks, _p(seq_of_token), _p(positions),
-            _p(token_list), _p(out), out.stride(0), _p(part_out), _p(part_ml), _p(_ticket_counters), num_q_heads, num_kv_heads, head_dim,
-            page_size, window, float(scale), max_splits, T, _p(head_scale), _p(slopes), _p(gate),
+            q, q.stride(0), k_cache, v_cache, block_table, max_blocks, seq_of_token, positions,
+            token_list, out, out.stride(0), part_out, part_ml, _ticket_counters, num_q_heads, num_kv_heads, head_dim,
+            page_size, window, float(scale), max_splits, T, head_scale, slopes, gate,
             gate.stride(0) if gate is not None else 0, float(softcap or 0.0), _stream()), "paged_attention_decode_terms")
         return
     if chunk or sinks is not None:
         assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == num_q_heads)
         _check(lib().aien_paged_attention_decode_masked(
-            _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(block_table), max_blocks, _p(seq_of_token), _p(positions),
-            _p(token_list), _p(out), out.stride(0), _p(part_out), _p(part_ml), _p(_ticket_counters), num_q_heads, num_kv_heads, head_dim,
-            page_size, window, float(scale), max_splits, T, int(chunk), _p(sinks), _stream()), "paged_attention_decode_masked")
+            q, q.stride(0), k_cache, v_cache, block_table, max_blocks, seq_of_token, positions,
+            token_list, out, out.stride(0), part_out, part_ml, _ticket_counters, num_q_heads, num_kv_heads, head_dim,
+            page_size, window, float(scale), max_splits, T, int(chunk), sinks, _stream()), "paged_attention_decode_masked")
         return
     if impl == "stream" and decode_stream_supports(num_q_heads, num_kv_heads, head_dim, page_size, max_splits):
         _check(lib().aien_paged_attention_decode_stream(
-            _p(q), q.stride(0), _p(k_cache), _p(v_cache), k_cache.shape[0], _p(block_table), max_blocks, _p(seq_of_token),
-            _p(positions), _p(token_list), _p(out), out.stride(0), _p(part_out), _p(part_ml), _p(_ticket_counters), num_q_heads,
+            q, q.stride(0), k_cache, v_cache, k_cache.shape[0], block_table, max_blocks, seq_of_token,
+            positions, token_list, out, out.stride(0), part_out, part_ml, _ticket_counters, num_q_heads,
             num_kv_heads, head_dim, page_size, window, float(scale), max_splits, T, _stream()), "paged_attention_decode_stream")
         return
     _check(lib().aien_paged_attention_decode(
-        _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(block_table), max_blocks, _p(seq_of_token), _p(positions),
-        _p(token_list), _p(out), out.stride(0), _p(part_out), _p(part_ml), _p(_ticket_counters), num_q_heads, num_kv_heads, head_dim,
+        q, q.stride(0), k_cache, v_cache, block_table, max_blocks, seq_of_token, positions,
+        token_list, out, out.stride(0), part_out, part_ml, _ticket_counters, num_q_heads, num_kv_heads, head_dim,
         page_size, window, float(scale), max_splits, T, _stream()), "paged_attention_decode")
 
 
@@ -1093,9 +984,9 @@ def paged_attention_decode_fused(ctx, q, k, v, q_norm_w, k_norm_w, eps, cos, sin
     k2 = k_cache.view(-1, num_kv_heads, head_dim)
     v2 = v_cache.view(-1, num_kv_heads, head_dim)
     _check(lib().aien_paged_attention_decode_fused(
-        _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(q_norm_w), _p(k_norm_w), wdt, float(eps),
-        _p(cos), _p(sin), rotary_dim if cos is not None else 0, _p(group.slot_map), _p(k2), _p(v2), _p(group.block_table),
-        group.max_blocks, _p(ctx.positions), _p(out), out.stride(0), _p(part_out), _p(part_ml), _p(_ticket_counters),
+        q, q.stride(0), k, k.stride(0), v, v.stride(0), q_norm_w, k_norm_w, wdt, float(eps),
+        cos, sin, rotary_dim if cos is not None else 0, group.slot_map, k2, v2, group.block_table,
+        group.max_blocks, ctx.positions, out, out.stride(0), part_out, part_ml, _ticket_counters,
         num_q_heads, num_kv_heads, head_dim, group.page_size, window, float(scale), splits, T, _stream()),
         "paged_attention_decode_fused")
 
@@ -1276,19 +1167,19 @@ def paged_attention_prefill(q, k_cache, v_cache, block_table, max_blocks, q_star
             _dev(scratch)
             assert scratch.dtype == torch.float32 and scratch.is_contiguous()
         _check(lib().aien_paged_attention_prefill_tc_terms(
-            _p(q), q.stride(0), q.shape[0], _p(k_cache), _p(v_cache), k_cache.shape[0], _p(block_table), max_blocks, _p(q_start),
-            _p(ctx_len), _p(tile_seq), _p(tile_q0), num_tiles, _p(out), out.stride(0), num_q_heads, num_kv_heads, head_dim,
-            page_size, window, float(scale), _p(scratch) if scratch is not None else None,
-            scratch.numel() * 4 if scratch is not None else 0, int(max_ctx), int(splits), int(chunk), _p(sinks),
-            _p(head_scale), _p(slopes), _p(gate), gate.stride(0) if gate is not None else 0, float(softcap or 0.0), _stream()),
+            q, q.stride(0), q.shape[0], k_cache, v_cache, k_cache.shape[0], block_table, max_blocks, q_start,
+            ctx_len, tile_seq, tile_q0, num_tiles, out, out.stride(0), num_q_heads, num_kv_heads, head_dim,
+            page_size, window, float(scale), scratch if scratch is not None else None,
+            scratch.numel() * 4 if scratch is not None else 0, int(max_ctx), int(splits), int(chunk), sinks,
+            head_scale, slopes, gate, gate.stride(0) if gate is not None else 0, float(softcap or 0.0), _stream()),
             "paged_attention_prefill_tc")
         return
     if terms:
         raise KernelError("paged_attention_prefill: only the tcgen05 kernel takes terms per head")
     _check(lib().aien_paged_attention_prefill(
-        _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(block_table), max_blocks, _p(q_start), _p(ctx_len), _p(tile_seq),
-        _p(tile_q0), num_tiles, _p(out), out.stride(0), num_q_heads, num_kv_heads, head_dim, page_size, window,
-        float(scale), int(chunk), _p(sinks), _stream()), "paged_attention_prefill")
+        q, q.stride(0), k_cache, v_cache, block_table, max_blocks, q_start, ctx_len, tile_seq,
+        tile_q0, num_tiles, out, out.stride(0), num_q_heads, num_kv_heads, head_dim, page_size, window,
+        float(scale), int(chunk), sinks, _stream()), "paged_attention_prefill")
 
 
 def attention_prefill_tc_error() -> int:
@@ -1306,7 +1197,7 @@ def collect_wait_errors(out: torch.Tensor) -> None:
     whatever was launched before.  The words stay set until read_wait_errors() clears them."""
     _dev(out)
     assert out.dtype == torch.int32 and out.numel() >= 4 and out.is_contiguous()
-    _check(lib().aien_collect_wait_errors(_p(out), _stream()), "collect_wait_errors")
+    _check(lib().aien_collect_wait_errors(out, _stream()), "collect_wait_errors")
 
 
 def read_wait_errors() -> tuple:
@@ -1331,7 +1222,7 @@ def embed_gather_scaled(table: torch.Tensor, ids: torch.Tensor, x: torch.Tensor,
     T, H = x.shape
     assert table.is_contiguous() and x.is_contiguous() and ids.dtype == torch.int32 and x.dtype == torch.float32
     assert table.shape[1] == H and ids.numel() >= T
-    _check(lib().aien_embed_gather_scaled(_p(table), dt(table), _p(ids), _p(x), T, H, table.shape[0], float(scale), _stream()),
+    _check(lib().aien_embed_gather_scaled(table, dt(table), ids, x, T, H, table.shape[0], float(scale), _stream()),
            "embed_gather_scaled")
 
 
@@ -1346,8 +1237,8 @@ def post_norm_add(x: torch.Tensor, a: torch.Tensor, weight: torch.Tensor, eps: f
     assert next_weight is None or (next_weight.numel() == H and next_weight.is_contiguous() and h is not None)
     assert h is None or (h.is_contiguous() and tuple(h.shape) == (T, H))
     pa, da, na, sa = _source(a, x.shape)
-    _check(lib().aien_post_norm_add(_p(x), pa, da, na, sa, _p(weight), dt(weight), float(eps), float(mult), _p(next_weight),
-                                    dt(next_weight) if next_weight is not None else F32, float(next_eps), _p(h),
+    _check(lib().aien_post_norm_add(x, pa, da, na, sa, weight, dt(weight), float(eps), float(mult), next_weight,
+                                    dt(next_weight) if next_weight is not None else F32, float(next_eps), h,
                                     dt(h) if h is not None else F32, T, H, _stream()), "post_norm_add")
 
 
@@ -1357,15 +1248,15 @@ def gelu_times_table(z: torch.Tensor, table: torch.Tensor, col0: int, ids: torch
     T, n = out.shape
     assert z.shape == (T, n) and z.stride(1) == 1 and out.stride(1) == 1 and table.is_contiguous() and table.dim() == 2
     assert 0 <= col0 and col0 + n <= table.shape[1] and ids.dtype == torch.int32 and ids.numel() >= T
-    _check(lib().aien_gelu_times_table(_p(z), dt(z), z.stride(0), _p(table), dt(table), table.shape[1], int(col0), _p(ids),
-                                       table.shape[0], _p(out), dt(out), out.stride(0), T, n, _stream()), "gelu_times_table")
+    _check(lib().aien_gelu_times_table(z, dt(z), z.stride(0), table, dt(table), table.shape[1], int(col0), ids,
+                                       table.shape[0], out, dt(out), out.stride(0), T, n, _stream()), "gelu_times_table")
 
 
 def softcap(v: torch.Tensor, cap: float, mult: float = 1.0) -> None:
     """v = cap * tanh(v * mult / cap) in place (float32); cap 0: v = v * mult."""
     _dev(v)
     assert v.dtype == torch.float32 and v.is_contiguous()
-    _check(lib().aien_softcap(_p(v), v.numel(), float(cap), float(mult), _stream()), "softcap")
+    _check(lib().aien_softcap(v, v.numel(), float(cap), float(mult), _stream()), "softcap")
 
 
 # ---------------------------------------------------------------------------- mixers with a state of fixed size
@@ -1391,13 +1282,13 @@ def decay_linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: in
         T = proj.shape[0]
         assert scratch.dtype == torch.float32 and scratch.is_contiguous() and out.shape[0] == T
         assert scratch.numel() >= decay_linear_attention_scratch(T, num_seqs, heads, dim, vdim)
-        _check(lib().aien_decay_linear_attention_chunked(_p(proj), dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), _p(decay),
-                                                         _p(state), _p(slot_map), _p(q_start), _p(positions), _p(out), out.stride(0),
-                                                         _p(scratch), T, int(num_seqs), int(heads), int(dim), int(vdim), _stream()),
+        _check(lib().aien_decay_linear_attention_chunked(proj, dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), decay,
+                                                         state, slot_map, q_start, positions, out, out.stride(0),
+                                                         scratch, T, int(num_seqs), int(heads), int(dim), int(vdim), _stream()),
                "decay_linear_attention_chunked")
         return
-    _check(lib().aien_decay_linear_attention(_p(proj), dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), _p(decay),
-                                             _p(state), _p(slot_map), _p(q_start), _p(positions), _p(out), out.stride(0),
+    _check(lib().aien_decay_linear_attention(proj, dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), decay,
+                                             state, slot_map, q_start, positions, out, out.stride(0),
                                              int(num_seqs), int(heads), int(dim), int(vdim), 1 if single_tokens else 0, _stream()),
            "decay_linear_attention")
 
@@ -1413,8 +1304,8 @@ def gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps
     T, N = o.shape
     assert o.dtype == torch.float32 and o.stride(1) == 1 and gate.stride(1) == 1 and out.stride(1) == 1
     assert tuple(gate.shape) == (T, N) and tuple(out.shape) == (T, N) and weight.numel() == N and weight.is_contiguous()
-    _check(lib().aien_gated_rmsnorm(_p(o), o.stride(0), _p(gate), dt(gate), gate.stride(0), _p(weight), dt(weight), float(eps),
-                                    _p(out), dt(out), out.stride(0), T, N, _stream()), "gated_rmsnorm")
+    _check(lib().aien_gated_rmsnorm(o, o.stride(0), gate, dt(gate), gate.stride(0), weight, dt(weight), float(eps),
+                                    out, dt(out), out.stride(0), T, N, _stream()), "gated_rmsnorm")
 
 
 def gated_recurrence(proj: torch.Tensor, z_off: int, x_off: int, g_off: int, bz: Optional[torch.Tensor], bx: Optional[torch.Tensor],
@@ -1435,8 +1326,8 @@ def gated_recurrence(proj: torch.Tensor, z_off: int, x_off: int, g_off: int, bz:
     assert bz is None or bx is None or bz.dtype == bx.dtype
     for t in (slot_map, q_start, positions):
         assert t.dtype == torch.int32
-    _check(lib().aien_gated_recurrence(_p(proj), dt(proj), proj.stride(0), int(z_off), int(x_off), int(g_off), _p(bz), _p(bx), bdt,
-                                       _p(state), _p(slot_map), _p(q_start), _p(positions), _p(out), dt(out), out.stride(0),
+    _check(lib().aien_gated_recurrence(proj, dt(proj), proj.stride(0), int(z_off), int(x_off), int(g_off), bz, bx, bdt,
+                                       state, slot_map, q_start, positions, out, dt(out), out.stride(0),
                                        int(num_seqs), int(width), 1 if segments else 0, _stream()), "gated_recurrence")
 
 
@@ -1466,9 +1357,9 @@ def latent_prepare(d: torch.Tensor, q_rank: int, wq: Optional[torch.Tensor], eps
         assert kv_off + kv_rank + rot_dim <= d.shape[1]
         if rot_dims:
             assert cos is not None and tuple(cos.shape) == (T, rot_dims // 2) and cos.is_contiguous() and sin.is_contiguous()
-    _check(lib().aien_latent_prepare(_p(d), dt(d), d.stride(0), int(q_rank), _p(wq), _p(wkv), wdt, float(eps), _p(cq),
+    _check(lib().aien_latent_prepare(d, dt(d), d.stride(0), int(q_rank), wq, wkv, wdt, float(eps), cq,
                                      dt(cq) if cq is not None else F32, cq.stride(0) if cq is not None else 0, int(kv_off),
-                                     int(kv_rank), int(rot_dim), int(rot_dims), _p(cos), _p(sin), _p(slot_map), _p(cache),
+                                     int(kv_rank), int(rot_dim), int(rot_dims), cos, sin, slot_map, cache,
                                      dt(cache) if cache is not None else F32, T, _stream()), "latent_prepare")
 
 
@@ -1482,8 +1373,8 @@ def rotate_pairs_rows(q: torch.Tensor, q_head: int, col0: int, out: torch.Tensor
     if rot_dims:
         assert cos is not None and tuple(cos.shape) == (T, rot_dims // 2) and cos.is_contiguous() and sin.is_contiguous()
     qv, ov = q[:, col0:], out[:, ocol0:]
-    _check(lib().aien_rotate_pairs_rows(_p(qv), dt(q), q.stride(0), int(q_head), _p(ov), dt(out), out.stride(0), int(o_head), T, int(heads),
-                                        int(rot_dim), int(rot_dims), _p(cos), _p(sin), _stream()), "rotate_pairs_rows")
+    _check(lib().aien_rotate_pairs_rows(qv, dt(q), q.stride(0), int(q_head), ov, dt(out), out.stride(0), int(o_head), T, int(heads),
+                                        int(rot_dim), int(rot_dims), cos, sin, _stream()), "rotate_pairs_rows")
 
 
 def head_project(a: torch.Tensor, a_head: int, a_col0: int, w: torch.Tensor, out: torch.Tensor, o_head: int, o_col0: int,
@@ -1502,17 +1393,17 @@ def head_project(a: torch.Tensor, a_head: int, a_col0: int, w: torch.Tensor, out
     assert gate is None or (tuple(gate.shape) in ((M, heads), (M, heads * N)) and gate.stride(1) == 1)
     _dev(gate)
     gate_n = N if gate is not None and gate.shape[1] == heads * N and N > 1 else 0
-    gp, gdt, ldg = _p(gate), dt(gate) if gate is not None else F32, gate.stride(0) if gate is not None else 0
+    gp, gdt, ldg = gate, dt(gate) if gate is not None else F32, gate.stride(0) if gate is not None else 0
     av, ov = a[:, a_col0:], out[:, o_col0:]
     if (_LATENT_IMPL != "plain" and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K_ % 8 == 0 and a.stride(0) % 8 == 0
             and a_head % 8 == 0 and av.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
-        _check(lib().aien_head_project_tc(_p(av), a.stride(0), int(a_head), _p(w), _p(ov), dt(out), out.stride(0), int(o_head),
-                                          M if rows is None else int(num_rows), N, K_, heads, gp, gdt, ldg, gate_n, _p(rows), _stream()),
+        _check(lib().aien_head_project_tc(av, a.stride(0), int(a_head), w, ov, dt(out), out.stride(0), int(o_head),
+                                          M if rows is None else int(num_rows), N, K_, heads, gp, gdt, ldg, gate_n, rows, _stream()),
                "head_project_tc")
         return
     if rows is not None:
         raise KernelError("head_project: only the tensor-core form takes a list of rows")
-    _check(lib().aien_head_project(_p(av), dt(a), a.stride(0), int(a_head), _p(w), dt(w), K_, N * K_, _p(ov), dt(out), out.stride(0),
+    _check(lib().aien_head_project(av, dt(a), a.stride(0), int(a_head), w, dt(w), K_, N * K_, ov, dt(out), out.stride(0),
                                    int(o_head), M, N, K_, heads, gp, gdt, ldg, gate_n, _stream()), "head_project")
 
 
@@ -1529,9 +1420,9 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Te
     assert out.shape == (T, heads * kv_rank) and cache.is_contiguous() and cache.shape[-1] == D
     assert block_table.dtype == torch.int32 and seq_of_token.dtype == torch.int32 and positions.dtype == torch.int32
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == heads)
-    _check(lib().aien_latent_attention(_p(q), q.stride(0), _p(cache), dt(cache), _p(block_table), int(max_blocks), _p(seq_of_token),
-                                       _p(positions), None, _p(out), dt(out), out.stride(0), T, int(heads), int(kv_rank),
-                                       int(rot_dim), int(page_size), int(window), float(scale), _p(sinks), _stream()),
+    _check(lib().aien_latent_attention(q, q.stride(0), cache, dt(cache), block_table, int(max_blocks), seq_of_token,
+                                       positions, None, out, dt(out), out.stride(0), T, int(heads), int(kv_rank),
+                                       int(rot_dim), int(page_size), int(window), float(scale), sinks, _stream()),
            "latent_attention")
 
 
@@ -1568,9 +1459,9 @@ def latent_attention_tc(q: torch.Tensor, cache: torch.Tensor, block_table: torch
         assert scratch is not None and scratch.dtype == torch.float32 and scratch.is_contiguous()
         assert scratch.numel() >= latent_attention_tc_scratch(count, heads, kv_rank, ksplit)
         part_o, part_ml = scratch[:n_o], scratch[n_o:]
-    _check(lib().aien_latent_attention_tc(_p(q), _p(cache), _p(block_table), int(max_blocks), _p(q_start), _p(positions), _p(out), T,
+    _check(lib().aien_latent_attention_tc(q, cache, block_table, int(max_blocks), q_start, positions, out, T,
                                           int(num_seqs), int(heads), int(kv_rank), int(rot_dim), int(page_size), int(window),
-                                          float(scale), _p(sinks), int(ksplit), _p(part_o), _p(part_ml), 1 if small_tiles else 0, _p(tokens),
+                                          float(scale), sinks, int(ksplit), part_o, part_ml, 1 if small_tiles else 0, tokens,
                                           int(num_single), _stream()), "latent_attention_tc")
 
 
@@ -1634,8 +1525,8 @@ def latent_gather(cache: torch.Tensor, group, q_start: torch.Tensor, ctx_len: to
     _dev(cache, group.block_table, q_start, ctx_len, out, table)
     assert cache.dtype == torch.bfloat16 and cache.is_contiguous() and out.is_contiguous() and tuple(out.shape) == (portions * length, cache.shape[-1])
     assert length % 128 == 0 and table.dtype == torch.int32 and tuple(table.shape) == (num_seqs, length // 128)
-    _check(lib().aien_latent_gather(_p(cache), cache.shape[-1], _p(group.block_table), group.max_blocks, group.page_size, _p(q_start),
-                                    _p(ctx_len), int(num_seqs), int(portions), int(length), _p(out), _p(table), _stream()), "latent_gather")
+    _check(lib().aien_latent_gather(cache, cache.shape[-1], group.block_table, group.max_blocks, group.page_size, q_start,
+                                    ctx_len, int(num_seqs), int(portions), int(length), out, table, _stream()), "latent_gather")
 
 
 def portion_attention(ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, table: torch.Tensor, out: torch.Tensor, heads: int,
@@ -1652,10 +1543,10 @@ def portion_attention(ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ta
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] == heads * value_dim)
     _check_head_terms(heads, None, None, head_gate)
     _check(lib().aien_paged_attention_prefill_tc_values(
-        _p(q), q.stride(0), q.shape[0], _p(k), _p(v), k.shape[0], _p(table), table.shape[1], _p(ctx.q_start), _p(ctx.ctx_len), _p(tile_seq),
-        _p(tile_q0), n, _p(out), out.stride(0), heads, heads, head_dim, 128, window, float(scale), None, 0, int(ctx.max_ctx_len), 0, 0,
-        _p(sinks), None, None, _p(head_gate), head_gate.stride(0) if head_gate is not None else 0, 0.0, value_dim, 1, 0, k.stride(0),
-        v.stride(0), _p(gate), gate.stride(0) if gate is not None else 0, _stream()), "paged_attention_prefill_tc_values")
+        q, q.stride(0), q.shape[0], k, v, k.shape[0], table, table.shape[1], ctx.q_start, ctx.ctx_len, tile_seq,
+        tile_q0, n, out, out.stride(0), heads, heads, head_dim, 128, window, float(scale), None, 0, int(ctx.max_ctx_len), 0, 0,
+        sinks, None, None, head_gate, head_gate.stride(0) if head_gate is not None else 0, 0.0, value_dim, 1, 0, k.stride(0),
+        v.stride(0), gate, gate.stride(0) if gate is not None else 0, _stream()), "paged_attention_prefill_tc_values")
 
 
 # ---------------------------------------------------------------------------- several residual streams, token shift
@@ -1663,7 +1554,7 @@ def replicate_streams(x: torch.Tensor) -> None:
     """x float32 [n, T, H]: copies x[0] into x[1:]."""
     _dev(x)
     assert x.dtype == torch.float32 and x.is_contiguous() and x.dim() == 3
-    _check(lib().aien_replicate_streams(_p(x), x.shape[1] * x.shape[2], x.shape[0], _stream()), "replicate_streams")
+    _check(lib().aien_replicate_streams(x, x.shape[1] * x.shape[2], x.shape[0], _stream()), "replicate_streams")
 
 
 def _pending(y: Optional[torch.Tensor], T: int, H: int) -> tuple:
@@ -1672,9 +1563,9 @@ def _pending(y: Optional[torch.Tensor], T: int, H: int) -> tuple:
     assert y.is_contiguous()
     if y.dim() == 3:
         assert y.dtype == torch.float32 and tuple(y.shape[1:]) == (T, H)
-        return _p(y), F32, y.shape[0], T * H
+        return y, F32, y.shape[0], T * H
     assert tuple(y.shape) == (T, H)
-    return _p(y), dt(y), 1, 0
+    return y, dt(y), 1, 0
 
 
 def hc_norm(x: torch.Tensor, y: Optional[torch.Tensor], prev: Optional[torch.Tensor], cur: torch.Tensor, weight: torch.Tensor,
@@ -1695,8 +1586,8 @@ def hc_norm(x: torch.Tensor, y: Optional[torch.Tensor], prev: Optional[torch.Ten
         assert shift_w.numel() == H and shift_state.dtype == torch.float32 and shift_state.is_contiguous() and shift_state.shape[-1] == H
         assert slot_map.dtype == torch.int32 and positions.dtype == torch.int32
     yp, ydt, parts, stride = _pending(y, T, H)
-    _check(lib().aien_hc_norm(_p(x), n, yp, ydt, parts, stride, _p(prev), _p(cur), _p(weight), dt(weight), float(eps), _p(h), dt(h), T, H,
-                              _p(shift_w), dt(shift_w) if shift_w is not None else F32, _p(shift_state), _p(slot_map), _p(positions),
+    _check(lib().aien_hc_norm(x, n, yp, ydt, parts, stride, prev, cur, weight, dt(weight), float(eps), h, dt(h), T, H,
+                              shift_w, dt(shift_w) if shift_w is not None else F32, shift_state, slot_map, positions,
                               _stream()), "hc_norm")
 
 
@@ -1708,8 +1599,8 @@ def token_shift(hn: torch.Tensor, shift_w: torch.Tensor, state: torch.Tensor, sl
     T, H = hn.shape
     assert hn.dtype == torch.float32 and hn.is_contiguous() and h.is_contiguous() and tuple(h.shape) == (T, H)
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[-1] == H and shift_w.numel() == H
-    _check(lib().aien_token_shift(_p(hn), _p(shift_w), dt(shift_w), _p(state), _p(slot_map), _p(seq_of_token), _p(q_start), _p(positions),
-                                  _p(h), dt(h), T, H, _stream()), "token_shift")
+    _check(lib().aien_token_shift(hn, shift_w, dt(shift_w), state, slot_map, seq_of_token, q_start, positions,
+                                  h, dt(h), T, H, _stream()), "token_shift")
 
 
 def hc_sum_rows(x: torch.Tensor, y: Optional[torch.Tensor], prev: Optional[torch.Tensor], rows: torch.Tensor, out: torch.Tensor) -> None:
@@ -1720,7 +1611,7 @@ def hc_sum_rows(x: torch.Tensor, y: Optional[torch.Tensor], prev: Optional[torch
     assert x.dtype == torch.float32 and x.is_contiguous() and out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == H
     assert rows.dtype == torch.int32 and rows.numel() >= R
     yp, ydt, parts, stride = _pending(y, T, H)
-    _check(lib().aien_hc_sum_rows(_p(x), n, T, yp, ydt, parts, stride, _p(prev), _p(rows), _p(out), R, H, _stream()), "hc_sum_rows")
+    _check(lib().aien_hc_sum_rows(x, n, T, yp, ydt, parts, stride, prev, rows, out, R, H, _stream()), "hc_sum_rows")
 
 
 def embed_gather_sinusoid(table: torch.Tensor, ids: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tensor, x: torch.Tensor,
@@ -1730,7 +1621,7 @@ def embed_gather_sinusoid(table: torch.Tensor, ids: torch.Tensor, positions: tor
     T, H = x.shape
     assert table.is_contiguous() and x.is_contiguous() and x.dtype == torch.float32 and table.shape[1] == H
     assert ids.dtype == torch.int32 and positions.dtype == torch.int32 and inv_freq.dtype == torch.float64 and inv_freq.numel() >= (H + 1) // 2
-    _check(lib().aien_embed_gather_sinusoid(_p(table), dt(table), _p(ids), _p(positions), _p(inv_freq), _p(x), T, H, table.shape[0],
+    _check(lib().aien_embed_gather_sinusoid(table, dt(table), ids, positions, inv_freq, x, T, H, table.shape[0],
                                             float(scale), _stream()), "embed_gather_sinusoid")
 
 
@@ -1756,10 +1647,10 @@ def attn_conv_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, Cq
     if Ck > 0:
         assert k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.dtype == v_cache.dtype and kv_slots.dtype == torch.int32
     _check(lib().aien_attn_conv_prepare(
-        _p(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), int(Cq), int(Ck), int(Cv), _p(wq), _p(wk), _p(wv), dt(wq), int(taps),
-        _p(q_norm), _p(k_norm), dt(q_norm), float(eps), int(kv_heads), int(value_dim), 1 if value_norm else 0, _p(state), _p(state_slots),
-        _p(seq_of_token), _p(q_start), _p(positions), _p(kv_slots), _p(k_cache), _p(v_cache), dt(k_cache) if k_cache is not None else dt(q_out),
-        _p(q_out), dt(q_out), q_out.stride(0), T, _stream()), "attn_conv_prepare")
+        proj, proj.stride(0), int(q_off), int(k_off), int(v_off), int(Cq), int(Ck), int(Cv), wq, wk, wv, dt(wq), int(taps),
+        q_norm, k_norm, dt(q_norm), float(eps), int(kv_heads), int(value_dim), 1 if value_norm else 0, state, state_slots,
+        seq_of_token, q_start, positions, kv_slots, k_cache, v_cache, dt(k_cache) if k_cache is not None else dt(q_out),
+        q_out, dt(q_out), q_out.stride(0), T, _stream()), "attn_conv_prepare")
 
 
 def delta_conv_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b_off: int, a_off: int, qk_heads: int, dim: int, heads: int,
@@ -1779,9 +1670,9 @@ def delta_conv_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b
     assert a_log.dtype == dt_bias.dtype and a_log.numel() == heads and dt_bias.numel() == heads and a_log.is_contiguous() and dt_bias.is_contiguous()
     assert state.dtype == torch.float32 and state.is_contiguous() and state.dim() == 2 and state.shape[1] >= (taps - 1) * C
     _check(lib().aien_delta_conv_prepare(
-        _p(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), int(b_off), int(a_off), int(qk_heads), int(dim), int(heads), int(vdim),
-        _p(wq), _p(wk), _p(wv), dt(wq), int(taps), _p(a_log), _p(dt_bias), dt(a_log), _p(state), state.shape[1], _p(state_slots),
-        _p(seq_of_token), _p(q_start), _p(positions), _p(out), out.stride(0), _p(gb), gb.stride(0), T, _stream()), "delta_conv_prepare")
+        proj, proj.stride(0), int(q_off), int(k_off), int(v_off), int(b_off), int(a_off), int(qk_heads), int(dim), int(heads), int(vdim),
+        wq, wk, wv, dt(wq), int(taps), a_log, dt_bias, dt(a_log), state, state.shape[1], state_slots,
+        seq_of_token, q_start, positions, out, out.stride(0), gb, gb.stride(0), T, _stream()), "delta_conv_prepare")
 
 
 def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gb: torch.Tensor, state: torch.Tensor, s_off: int,
@@ -1802,8 +1693,8 @@ def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gb: torch.
             return
     else:
         alone = 0
-    _check(lib().aien_delta_rule(_p(qkv), qkv.stride(0), int(q_off), int(k_off), int(v_off), _p(gb), gb.stride(0), _p(state), state.shape[1],
-                                 int(s_off), _p(slot_map), _p(q_start), _p(positions), _p(o), o.stride(0), int(num_seqs), int(heads),
+    _check(lib().aien_delta_rule(qkv, qkv.stride(0), int(q_off), int(k_off), int(v_off), gb, gb.stride(0), state, state.shape[1],
+                                 int(s_off), slot_map, q_start, positions, o, o.stride(0), int(num_seqs), int(heads),
                                  int(qk_heads), int(dim), int(vdim), 1 if alone else 0, _stream()), "delta_rule")
 
 
@@ -1818,8 +1709,8 @@ def grouped_gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, weight: torch.Ten
     T, N = o.shape
     assert o.dtype == torch.float32 and o.stride(1) == 1 and gate.stride(1) == 1 and out.stride(1) == 1 and N % group == 0
     assert tuple(gate.shape) == (T, N) and tuple(out.shape) == (T, N) and weight.numel() == group and weight.is_contiguous()
-    _check(lib().aien_grouped_gated_rmsnorm(_p(o), o.stride(0), _p(gate), dt(gate), gate.stride(0), _p(weight), dt(weight), float(eps),
-                                            _p(out), dt(out), out.stride(0), T, N // group, int(group), GATE_ACTS[gate_act], _stream()),
+    _check(lib().aien_grouped_gated_rmsnorm(o, o.stride(0), gate, dt(gate), gate.stride(0), weight, dt(weight), float(eps),
+                                            out, dt(out), out.stride(0), T, N // group, int(group), GATE_ACTS[gate_act], _stream()),
            "grouped_gated_rmsnorm")
 
 
@@ -1888,9 +1779,9 @@ def conv_act(proj: torch.Tensor, off: int, channels: int, w: torch.Tensor, bias:
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and out.dtype == torch.float32 and out.stride(1) == 1
     assert w.is_contiguous() and tuple(w.shape) == (channels, taps) and (bias is None or (bias.is_contiguous() and bias.numel() == channels))
     assert taps == 1 or (state is not None and state.dtype == torch.float32 and state.stride(-1) == 1 and state.shape[-1] >= (taps - 1) * channels)
-    _check(lib().aien_conv_act(_p(proj), proj.stride(0), int(off), int(channels), _p(w), dt(w), _p(bias), dt(bias) if bias is not None else F32,
-                               int(taps), {"none": 0, "silu": 1}[act], _p(state), state.stride(0) if state is not None else 0, _p(slot_map),
-                               _p(seq_of_token), _p(q_start), _p(positions), _p(out), out.stride(0), _p(out16),
+    _check(lib().aien_conv_act(proj, proj.stride(0), int(off), int(channels), w, dt(w), bias, dt(bias) if bias is not None else F32,
+                               int(taps), {"none": 0, "silu": 1}[act], state, state.stride(0) if state is not None else 0, slot_map,
+                               seq_of_token, q_start, positions, out, out.stride(0), out16,
                                out16.stride(0) if out16 is not None else 0, T, _stream()), "conv_act")
 
 
@@ -1948,10 +1839,10 @@ def block_walk(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: Op
     if not _rows_walk(rows, scratch, q_off, k_off, v_off):
         return False
     _check(lib().aien_block_walk(
-        _p(rows), rows.stride(0), int(q_off), int(k_off), int(v_off), int(act), _p(gates), gates.stride(0) if gates is not None else 0, int(g_off),
-        int(w_off), _p(decay), int(delta), _p(skip), dt(skip) if skip is not None else F32, _p(state), state.stride(0), int(s_off), int(state_vn),
-        _p(slot_map), _p(q_start), _p(positions), _p(out), out.stride(0), T, int(num_seqs), int(heads), int(qk_heads), int(dim), int(vdim),
-        int(alone), _p(scratch), _stream()), "block_walk")
+        rows, rows.stride(0), int(q_off), int(k_off), int(v_off), int(act), gates, gates.stride(0) if gates is not None else 0, int(g_off),
+        int(w_off), decay, int(delta), skip, dt(skip) if skip is not None else F32, state, state.stride(0), int(s_off), int(state_vn),
+        slot_map, q_start, positions, out, out.stride(0), T, int(num_seqs), int(heads), int(qk_heads), int(dim), int(vdim),
+        int(alone), scratch, _stream()), "block_walk")
     add_launches(1)
     return True
 
@@ -2024,10 +1915,10 @@ def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: 
     assert dt_bias.is_contiguous() and D.is_contiguous() and state.dtype == torch.float32 and state.stride(-1) == 1 and out.stride(1) == 1
     if seg_len and nseg > 1:
         assert scratch is not None and scratch.numel() >= 2 * (T // seg_len + num_seqs) * inner * N
-    _check(lib().aien_selective_scan(_p(x), x.stride(0), _p(dtz), dtz.stride(0), _p(bc), bc.stride(0), int(b_off), int(c_off), _p(z), z.stride(0),
-                                     _p(A), _p(dt_bias), _p(D), dt(D), _p(state), state.stride(0), int(s_off), _p(slot_map), _p(q_start),
-                                     _p(positions), _p(out), dt(out), out.stride(0), T, int(num_seqs), inner, int(N), int(seg_len), int(nseg),
-                                     _p(scratch), _stream()), "selective_scan")
+    _check(lib().aien_selective_scan(x, x.stride(0), dtz, dtz.stride(0), bc, bc.stride(0), int(b_off), int(c_off), z, z.stride(0),
+                                     A, dt_bias, D, dt(D), state, state.stride(0), int(s_off), slot_map, q_start,
+                                     positions, out, dt(out), out.stride(0), T, int(num_seqs), inner, int(N), int(seg_len), int(nseg),
+                                     scratch, _stream()), "selective_scan")
     add_launches(2 if (seg_len and nseg > 1) else 0)
 
 
@@ -2041,7 +1932,7 @@ def split_rows(x: torch.Tensor, out: torch.Tensor, rest: Optional[torch.Tensor] 
     assert x.dtype == torch.float32 and x.stride(-1) == 1 and x.shape[-1] == n + m
     assert out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == (T, 3 * n)
     assert rest is None or (rest.dtype == torch.float32 and rest.is_contiguous() and rest.shape[0] == T)
-    _check(lib().aien_split_rows(_p(x), x.stride(-2), parts, part_stride, _p(out), _p(rest), T, n, m, _stream()), "split_rows")
+    _check(lib().aien_split_rows(x, x.stride(-2), parts, part_stride, out, rest, T, n, m, _stream()), "split_rows")
 
 
 def parts_product(parts: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
@@ -2051,7 +1942,7 @@ def parts_product(parts: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
     (T, n3), (N, n) = parts.shape, w.shape
     assert parts.dtype == torch.bfloat16 and parts.is_contiguous() and n3 == 3 * n and w.dtype == torch.bfloat16 and w.stride(1) == 1
     assert out.dtype == torch.float32 and out.stride(1) == 1 and tuple(out.shape) == (T, N)
-    _check(lib().aien_parts_product(_p(parts), _p(w), w.stride(0), _p(out), out.stride(0), T, N, n, _stream()), "parts_product")
+    _check(lib().aien_parts_product(parts, w, w.stride(0), out, out.stride(0), T, N, n, _stream()), "parts_product")
 
 
 def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.Tensor, A: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor,
@@ -2075,7 +1966,7 @@ def ssd_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dtr: torch.T
     assert state.dtype == torch.float32 and state.stride(-1) == 1 and y.dtype == torch.float32 and y.stride(1) == 1
     walk = blocks is not None and _rows_walk(xbc, blocks, x_off, b_off, c_off)
     if walk and not alone:
-        _check(lib().aien_ssd_steps(_p(dtr), dtr.stride(0), _p(A), _p(dt_bias), dt(dt_bias), _p(steps), T, int(heads), _stream()), "ssd_steps")
+        _check(lib().aien_ssd_steps(dtr, dtr.stride(0), A, dt_bias, dt(dt_bias), steps, T, int(heads), _stream()), "ssd_steps")
     else:
         _ssd_tokens(xbc, x_off, b_off, c_off, dtr, A, dt_bias, D, state, s_off, slot_map, q_start, positions, y, num_seqs, heads, V, G, N, seg_len, nseg,
                     scratch, steps, 1 if walk else 0)
@@ -2089,9 +1980,9 @@ def _ssd_tokens(xbc, x_off, b_off, c_off, dtr, A, dt_bias, D, state, s_off, slot
     T = xbc.shape[0]
     if seg_len and nseg > 1:
         assert scratch is not None and scratch.numel() >= 2 * (T // seg_len + num_seqs) * heads * N * V
-    _check(lib().aien_ssd_scan(_p(xbc), xbc.stride(0), int(x_off), int(b_off), int(c_off), _p(dtr), dtr.stride(0), _p(A), _p(dt_bias), _p(D),
-                               dt(D), _p(state), state.stride(0), int(s_off), _p(slot_map), _p(q_start), _p(positions), _p(y), y.stride(0),
-                               T, int(num_seqs), int(heads), int(V), int(G), int(N), int(seg_len), int(nseg), _p(scratch), _p(steps), int(longest),
+    _check(lib().aien_ssd_scan(xbc, xbc.stride(0), int(x_off), int(b_off), int(c_off), dtr, dtr.stride(0), A, dt_bias, D,
+                               dt(D), state, state.stride(0), int(s_off), slot_map, q_start, positions, y, y.stride(0),
+                               T, int(num_seqs), int(heads), int(V), int(G), int(N), int(seg_len), int(nseg), scratch, steps, int(longest),
                                _stream()), "ssd_scan")
     add_launches(3 if (seg_len and nseg > 1) else 1)
 
@@ -2103,7 +1994,7 @@ def gate_group_norm(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, eps:
     T, width = y.shape
     assert y.dtype == torch.float32 and z.dtype == torch.float32 and y.stride(1) == 1 and z.stride(1) == 1 and out.stride(1) == 1
     assert weight.is_contiguous() and weight.numel() == width and tuple(out.shape) == (T, width)
-    _check(lib().aien_gate_group_norm(_p(y), y.stride(0), _p(z), z.stride(0), _p(weight), dt(weight), float(eps), float(mult), _p(out), dt(out),
+    _check(lib().aien_gate_group_norm(y, y.stride(0), z, z.stride(0), weight, dt(weight), float(eps), float(mult), out, dt(out),
                                       out.stride(0), T, width, int(groups), _stream()), "gate_group_norm")
 
 
@@ -2119,8 +2010,8 @@ def scaled_add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], vec: Opti
         assert v is None or (v.dtype == torch.float32 and v.is_contiguous() and v.numel() == H)
     assert out is None or (out.is_contiguous() and out.shape == x.shape and weight is not None and weight.is_contiguous() and weight.numel() == H)
     nparts, stride = _parts_of(delta, x.shape)
-    _check(lib().aien_scaled_add_rmsnorm(_p(x), _p(delta), dt(delta) if delta is not None else F32, nparts, stride, _p(vec), _p(bias),
-                                         _p(weight), dt(weight) if weight is not None else F32, float(eps), _p(out),
+    _check(lib().aien_scaled_add_rmsnorm(x, delta, dt(delta) if delta is not None else F32, nparts, stride, vec, bias,
+                                         weight, dt(weight) if weight is not None else F32, float(eps), out,
                                          dt(out) if out is not None else F32, T, H, _stream()), "scaled_add_rmsnorm")
 
 
@@ -2130,7 +2021,7 @@ def pass_input(x: torch.Tensor, again: Optional[torch.Tensor], row: torch.Tensor
     T, H = x.shape
     assert x.dtype == torch.float32 and x.is_contiguous() and row.is_contiguous() and row.numel() == H
     assert again is None or (again.dtype == torch.float32 and again.is_contiguous() and again.shape == x.shape)
-    _check(lib().aien_pass_input(_p(x), _p(again), _p(row), dt(row), T, H, _stream()), "pass_input")
+    _check(lib().aien_pass_input(x, again, row, dt(row), T, H, _stream()), "pass_input")
 
 
 def clamped_glu(a: torch.Tensor, gate_off: int, up_off: int, F_: int, bias_gate: Optional[torch.Tensor], bias_up: Optional[torch.Tensor],
@@ -2146,8 +2037,8 @@ def clamped_glu(a: torch.Tensor, gate_off: int, up_off: int, F_: int, bias_gate:
             assert b.is_contiguous() and b.numel() == F_
             bdt = dt(b)
     assert bias_gate is None or bias_up is None or bias_gate.dtype == bias_up.dtype
-    _check(lib().aien_clamped_glu(_p(a), dt(a), a.stride(0), int(gate_off), int(up_off), _p(bias_gate), _p(bias_up), bdt, float(limit),
-                                  float(alpha), _p(out), dt(out), out.stride(0), T, int(F_), _stream()), "clamped_glu")
+    _check(lib().aien_clamped_glu(a, dt(a), a.stride(0), int(gate_off), int(up_off), bias_gate, bias_up, bdt, float(limit),
+                                  float(alpha), out, dt(out), out.stride(0), T, int(F_), _stream()), "clamped_glu")
 
 
 def sigmoid_gate(o: torch.Tensor, g: Optional[torch.Tensor], mult: float, out: torch.Tensor) -> None:
@@ -2156,7 +2047,7 @@ def sigmoid_gate(o: torch.Tensor, g: Optional[torch.Tensor], mult: float, out: t
     T, C = o.shape
     assert o.stride(1) == 1 and out.stride(1) == 1 and tuple(out.shape) == (T, C)
     assert g is None or (g.dtype == torch.float32 and g.stride(1) == 1 and tuple(g.shape) == (T, C))
-    _check(lib().aien_sigmoid_gate(_p(o), dt(o), o.stride(0), _p(g), g.stride(0) if g is not None else 0, float(mult), _p(out), dt(out),
+    _check(lib().aien_sigmoid_gate(o, dt(o), o.stride(0), g, g.stride(0) if g is not None else 0, float(mult), out, dt(out),
                                    out.stride(0), T, C, _stream()), "sigmoid_gate")
 
 
@@ -2223,9 +2114,9 @@ def paged_attention_decode_warps(ctx, q, k2, v2, group, out, num_q_heads: int, n
     part = ctx.workspace.take((n * nv * splits * (heads * value_dim + (2 * heads + 3) // 4 * 4),), torch.float32) if splits > 1 else None
     lam, eps, mult = diff if diff else (0.0, 0.0, 1.0)
     _check(lib().aien_paged_attention_decode_warps(
-        _p(q), q.stride(0), _p(k2), _p(v2), _p(group.block_table), group.max_blocks, None if tokens is None else _p(ctx.seq_of_token),
-        _p(ctx.positions), _p(tokens), _p(out), out.stride(0), 1 if out.dtype == torch.float32 else 0, _p(part),
-        _p(_tickets(q.device, n * nv)), num_q_heads, num_kv_heads, head_dim, value_dim, maps, group.page_size, window, int(chunk), float(scale),
+        q, q.stride(0), k2, v2, group.block_table, group.max_blocks, None if tokens is None else ctx.seq_of_token,
+        ctx.positions, tokens, out, out.stride(0), 1 if out.dtype == torch.float32 else 0, part,
+        _tickets(q.device, n * nv), num_q_heads, num_kv_heads, head_dim, value_dim, maps, group.page_size, window, int(chunk), float(scale),
         float(softcap or 0.0), splits, n, 1 if diff else 0, float(lam), float(eps), float(mult), _stream()), "paged_attention_decode_warps")
 
 
@@ -2273,8 +2164,8 @@ def capped_attention(ctx, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
         part_out = ctx.workspace.take((n * num_q_heads * splits * value_dim,), torch.float32)
         part_ml = ctx.workspace.take((n * num_q_heads * splits * 2,), torch.float32)
         _check(lib().aien_paged_attention_decode_values(
-            _p(q), q.stride(0), _p(k2), _p(v2), _p(group.block_table), group.max_blocks, None if tokens is None else _p(ctx.seq_of_token),
-            _p(ctx.positions), _p(tokens), _p(out), out.stride(0), _p(part_out), _p(part_ml), _p(_tickets(q.device, n * num_kv_heads)), num_q_heads,
+            q, q.stride(0), k2, v2, group.block_table, group.max_blocks, None if tokens is None else ctx.seq_of_token,
+            ctx.positions, tokens, out, out.stride(0), part_out, part_ml, _tickets(q.device, n * num_kv_heads), num_q_heads,
             num_kv_heads, head_dim, group.page_size, window, float(scale), splits, n, int(chunk), float(softcap or 0.0), value_dim,
             int(v_share), 1 if out.dtype == torch.float32 else 0, 1 if window > 0 or chunk > 0 else 0, _stream()),
             "paged_attention_decode_values")
@@ -2298,9 +2189,9 @@ def capped_attention(ctx, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
                 nbytes = prefill_split_scratch_bytes(n, num_q_heads, _tile_cols(value_dim), ctx.max_ctx_len)
                 scratch = ctx.workspace.take((nbytes // 4,), torch.float32) if nbytes else None
             _check(lib().aien_paged_attention_prefill_tc_values(
-                _p(q), q.stride(0), q.shape[0], _p(k2), _p(v2), k2.shape[0], _p(group.block_table), group.max_blocks, _p(ctx.q_start),
-                _p(ctx.ctx_len), _p(tile_seq), _p(tile_q0), n, _p(out), out.stride(0), num_q_heads, num_kv_heads, head_dim,
-                group.page_size, window, float(scale), _p(scratch), scratch.numel() * 4 if scratch is not None else 0,
+                q, q.stride(0), q.shape[0], k2, v2, k2.shape[0], group.block_table, group.max_blocks, ctx.q_start,
+                ctx.ctx_len, tile_seq, tile_q0, n, out, out.stride(0), num_q_heads, num_kv_heads, head_dim,
+                group.page_size, window, float(scale), scratch, scratch.numel() * 4 if scratch is not None else 0,
                 int(ctx.max_ctx_len), 0, int(chunk), None, None, None, None, 0, float(softcap or 0.0), value_dim, int(v_share),
                 1 if out.dtype == torch.float32 else 0, 0, 0, None, 0, _stream()), "paged_attention_prefill_tc_values")
         tokens, nd = ctx.single_tokens if ctx.single_tokens is not None else (None, 0)
@@ -2325,9 +2216,9 @@ def routed_combine(parts: torch.Tensor, h: Optional[torch.Tensor], w_same: Optio
         assert h.stride(1) == 1 and w_same.dtype == torch.float32 and w_same.is_contiguous() and w_same.numel() >= T
     sparts, sstride = _parts_of(shared, (T, H))
     assert zs is None or zs.dtype == torch.float32
-    _check(lib().aien_routed_combine(_p(parts), dt(parts), P_, T * H, _p(h), dt(h) if h is not None else F32, h.stride(0) if h is not None else 0,
-                                     _p(w_same), _p(shared), dt(shared) if shared is not None else F32, sparts, sstride, _p(zs),
-                                     zs.stride(0) if zs is not None else 0, _p(out), T, H, _stream()), "routed_combine")
+    _check(lib().aien_routed_combine(parts, dt(parts), P_, T * H, h, dt(h) if h is not None else F32, h.stride(0) if h is not None else 0,
+                                     w_same, shared, dt(shared) if shared is not None else F32, sparts, sstride, zs,
+                                     zs.stride(0) if zs is not None else 0, out, T, H, _stream()), "routed_combine")
 
 
 def moe_route_biased(z: torch.Tensor, num_experts: int, real: int, top: int, renorm: bool, renorm_eps: float,
@@ -2343,9 +2234,9 @@ def moe_route_biased(z: torch.Tensor, num_experts: int, real: int, top: int, ren
     assert ids.is_contiguous() and wts.is_contiguous() and ids.numel() >= T * top and wts.numel() >= T * top
     assert correction is None or (correction.is_contiguous() and correction.numel() == num_experts)
     assert w_same is None or (w_same.dtype == torch.float32 and w_same.is_contiguous() and w_same.numel() >= T)
-    _check(lib().aien_moe_route_biased(_p(z), z.stride(0), T, int(num_experts), int(real), int(top), 1 if renorm else 0, float(renorm_eps),
-                                       _p(correction), dt(correction) if correction is not None else F32, 1 if sigmoid else 0, _p(ids), _p(wts),
-                                       _p(w_same), _p(expert_count), _stream()), "moe_route_biased")
+    _check(lib().aien_moe_route_biased(z, z.stride(0), T, int(num_experts), int(real), int(top), 1 if renorm else 0, float(renorm_eps),
+                                       correction, dt(correction) if correction is not None else F32, 1 if sigmoid else 0, ids, wts,
+                                       w_same, expert_count, _stream()), "moe_route_biased")
 
 
 def rope_halves_value_write(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, nq: int, nkv: int, hd: int, hdv: int,
@@ -2369,9 +2260,9 @@ def rope_halves_value_write(proj: torch.Tensor, q_off: int, k_off: int, v_off: i
     assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() >= max(q_off + nq * hd, k_off + nkv * hd, v_off + nv * hdv))
     if rot:
         assert cos is not None and tuple(cos.shape) == (T, rot // 2) and cos.is_contiguous() and sin.is_contiguous()
-    _check(lib().aien_rope_halves_value_write(_p(proj), dt(proj), proj.stride(-2), nparts, stride, _p(bias), int(q_off), int(k_off), int(v_off),
-                                              int(nq), int(nkv), int(hd), nv, int(hdv), _p(cos), _p(sin), int(rot), _p(slot_map), _p(q_out),
-                                              dt(q_out), q_out.stride(0), _p(k_cache), _p(v_cache), dt(k_cache), T, _stream()),
+    _check(lib().aien_rope_halves_value_write(proj, dt(proj), proj.stride(-2), nparts, stride, bias, int(q_off), int(k_off), int(v_off),
+                                              int(nq), int(nkv), int(hd), nv, int(hdv), cos, sin, int(rot), slot_map, q_out,
+                                              dt(q_out), q_out.stride(0), k_cache, v_cache, dt(k_cache), T, _stream()),
            "rope_halves_value_write")
 
 
@@ -2382,7 +2273,7 @@ def map_difference_norm(a: torch.Tensor, out: torch.Tensor, heads: int, per_grou
     T = a.shape[0]
     assert a.dtype == torch.float32 and a.stride(1) == 1 and out.stride(1) == 1
     assert a.shape[1] == 2 * heads * value_dim and tuple(out.shape) == (T, heads * value_dim)
-    _check(lib().aien_map_difference_norm(_p(a), a.stride(0), _p(out), dt(out), out.stride(0), T, int(heads), int(per_group), int(value_dim),
+    _check(lib().aien_map_difference_norm(a, a.stride(0), out, dt(out), out.stride(0), T, int(heads), int(per_group), int(value_dim),
                                           float(lam), float(eps), float(mult), _stream()), "map_difference_norm")
 
 
@@ -2397,7 +2288,7 @@ def _term_args(terms, T: int, H: int) -> list:
         _dev(t, gate)
         assert t.is_contiguous() and tuple(t.shape[-2:]) == (T, H) and t.dim() in (2, 3)
         assert gate is None or (gate.dtype == torch.float32 and gate.numel() >= T)
-        args += [_p(t), dt(t), t.shape[0] if t.dim() == 3 else 1, T * H if t.dim() == 3 else 0, _p(gate), gate.stride(0) if gate is not None else 0]
+        args += [t, dt(t), t.shape[0] if t.dim() == 3 else 1, T * H if t.dim() == 3 else 0, gate, gate.stride(0) if gate is not None else 0]
     return args + [0, F32, 0, 0, 0, 0] * (MAX_SUM_TERMS - len(terms))
 
 
@@ -2409,8 +2300,8 @@ def sum_terms_rmsnorm(x: torch.Tensor, terms, bias: Optional[torch.Tensor], repl
     T, H = x.shape
     assert x.dtype == torch.float32 and x.is_contiguous() and (bias is None or (bias.numel() == H and bias.is_contiguous()))
     assert out is None or (out.is_contiguous() and out.shape == x.shape and weight.numel() == H and weight.is_contiguous())
-    _check(lib().aien_sum_terms_rmsnorm(_p(x), len(terms), *_term_args(terms, T, H), _p(bias), dt(bias) if bias is not None else F32, 1 if replace else 0,
-                                        _p(weight), dt(weight) if weight is not None else F32, float(eps), _p(out), dt(out) if out is not None else F32,
+    _check(lib().aien_sum_terms_rmsnorm(x, len(terms), *_term_args(terms, T, H), bias, dt(bias) if bias is not None else F32, 1 if replace else 0,
+                                        weight, dt(weight) if weight is not None else F32, float(eps), out, dt(out) if out is not None else F32,
                                         T, H, _stream()), "sum_terms_rmsnorm")
 
 
@@ -2421,7 +2312,7 @@ def pass_rows(x: torch.Tensor, terms, x0: torch.Tensor, out: torch.Tensor) -> No
     T, H = x.shape
     assert x.dtype == torch.float32 and x.is_contiguous() and x0.dtype == torch.float32 and x0.is_contiguous() and x0.shape == x.shape
     assert out.is_contiguous() and tuple(out.shape) == (T, (2 if out.dtype == torch.float32 else 3) * H)
-    _check(lib().aien_pass_rows(_p(x), len(terms), *_term_args(terms, T, H), _p(x0), _p(out), dt(out), T, H, _stream()), "pass_rows")
+    _check(lib().aien_pass_rows(x, len(terms), *_term_args(terms, T, H), x0, out, dt(out), T, H, _stream()), "pass_rows")
 
 
 # ---------------------------------------------------------------------------- matrix memory
@@ -2449,8 +2340,8 @@ def matrix_memory_gates(z: torch.Tensor, i_off: int, f_off: int, bi: torch.Tenso
     assert bi.dtype == torch.float32 and bf.dtype == torch.float32 and bi.numel() == heads and bf.numel() == heads
     assert gates.dtype == torch.float32 and gates.is_contiguous() and tuple(gates.shape) == (T, 3 * heads)
     assert state.shape[1] >= matrix_memory_state_floats(heads, dim, vdim)
-    _check(lib().aien_matrix_memory_gates(_p(z), z.stride(0), int(i_off), int(f_off), _p(bi), _p(bf), float(cap), _p(state), state.stride(0),
-                                          heads * (dim * vdim + dim), _p(slot_map), _p(q_start), _p(positions), _p(gates), T, int(num_seqs),
+    _check(lib().aien_matrix_memory_gates(z, z.stride(0), int(i_off), int(f_off), bi, bf, float(cap), state, state.stride(0),
+                                          heads * (dim * vdim + dim), slot_map, q_start, positions, gates, T, int(num_seqs),
                                           int(heads), _stream()), "matrix_memory_gates")
 
 
@@ -2465,8 +2356,8 @@ def matrix_memory_walk(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q
     assert proj.stride(1) == 1 and max(q_off, k_off) + heads * dim <= proj.shape[1] and v_off + heads * vdim <= proj.shape[1]
     assert gates.is_contiguous() and tuple(gates.shape) == (T, 3 * heads) and state.shape[1] >= matrix_memory_state_floats(heads, dim, vdim)
     assert num.dtype == torch.float32 and num.is_contiguous() and num.numel() == T * heads * vdim and nq.is_contiguous() and nq.numel() == T * heads
-    _check(lib().aien_matrix_memory_walk(_p(proj), dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), float(q_scale), _p(gates), _p(state),
-                                         state.stride(0), _p(slot_map), _p(q_start), _p(positions), _p(num), _p(nq), int(num_seqs), int(heads),
+    _check(lib().aien_matrix_memory_walk(proj, dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), float(q_scale), gates, state,
+                                         state.stride(0), slot_map, q_start, positions, num, nq, int(num_seqs), int(heads),
                                          int(dim), int(vdim), _stream()), "matrix_memory_walk")
 
 
@@ -2477,8 +2368,8 @@ def matrix_memory_finish(num: torch.Tensor, nq: torch.Tensor, gates: torch.Tenso
     T = num.shape[0]
     assert g.stride(1) == 1 and tuple(g.shape) == (T, heads * vdim) and out.stride(1) == 1 and tuple(out.shape) == (T, heads * vdim)
     assert weight.is_contiguous() and weight.numel() == heads * vdim
-    _check(lib().aien_matrix_memory_finish(_p(num), _p(nq), _p(gates), _p(g), dt(g), g.stride(0), _p(weight), dt(weight), float(eps), float(den_eps),
-                                           _p(out), dt(out), out.stride(0), T, int(heads), int(vdim), _stream()), "matrix_memory_finish")
+    _check(lib().aien_matrix_memory_finish(num, nq, gates, g, dt(g), g.stride(0), weight, dt(weight), float(eps), float(den_eps),
+                                           out, dt(out), out.stride(0), T, int(heads), int(vdim), _stream()), "matrix_memory_finish")
 
 
 def matrix_memory_token_supports(dim: int, vdim: int) -> bool:
@@ -2496,9 +2387,9 @@ def matrix_memory_token(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, 
     assert max(q_off, k_off) + heads * dim <= proj.shape[1] and max(v_off, g_off) + heads * vdim <= proj.shape[1]
     assert max(i_off, f_off) + heads <= z.shape[1] and bi.dtype == torch.float32 and bf.dtype == torch.float32
     assert state.shape[1] >= matrix_memory_state_floats(heads, dim, vdim) and weight.is_contiguous() and weight.numel() == heads * vdim
-    _check(lib().aien_matrix_memory_token(_p(proj), dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), int(g_off), float(q_scale), _p(z),
-                                          z.stride(0), int(i_off), int(f_off), _p(bi), _p(bf), float(cap), _p(state), state.stride(0), _p(slot_map),
-                                          _p(q_start), _p(positions), _p(weight), dt(weight), float(eps), float(den_eps), _p(out), dt(out),
+    _check(lib().aien_matrix_memory_token(proj, dt(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), int(g_off), float(q_scale), z,
+                                          z.stride(0), int(i_off), int(f_off), bi, bf, float(cap), state, state.stride(0), slot_map,
+                                          q_start, positions, weight, dt(weight), float(eps), float(den_eps), out, dt(out),
                                           out.stride(0), int(num_seqs), int(heads), int(dim), int(vdim), _stream()), "matrix_memory_token")
 
 
@@ -2527,7 +2418,7 @@ def matrix_memory_chunked(proj: torch.Tensor, q_off: int, k_off: int, v_off: int
     assert gates.is_contiguous() and tuple(gates.shape) == (T, 3 * heads) and state.shape[1] >= matrix_memory_state_floats(heads, dim, vdim)
     assert out.shape[0] == T and out.shape[1] == heads * vdim and weight.is_contiguous() and weight.numel() == heads * vdim
     assert scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.numel() >= matrix_memory_chunks_scratch(T, num_seqs, heads, dim, vdim)
-    _check(lib().aien_matrix_memory_chunked(_p(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), int(g_off), float(q_scale), _p(gates),
-                                            _p(state), state.stride(0), _p(slot_map), _p(q_start), _p(positions), _p(weight), dt(weight), float(eps),
-                                            float(den_eps), _p(out), out.stride(0), _p(scratch), T, int(num_seqs), int(heads), int(dim), int(vdim),
+    _check(lib().aien_matrix_memory_chunked(proj, proj.stride(0), int(q_off), int(k_off), int(v_off), int(g_off), float(q_scale), gates,
+                                            state, state.stride(0), slot_map, q_start, positions, weight, dt(weight), float(eps),
+                                            float(den_eps), out, out.stride(0), scratch, T, int(num_seqs), int(heads), int(dim), int(vdim),
                                             _stream()), "matrix_memory_chunked")

@@ -30,6 +30,8 @@ from typing import Any, Dict, List, Mapping, Optional, Tuple
 
 import torch
 
+from ..csrc import build as _build
+
 
 # ------------------------------------------------------------------ what a mixer keeps
 @dataclass(frozen=True)
@@ -171,6 +173,7 @@ class Workspace:
         self.layer_bytes = (int(layer_bytes) + 255) & ~255
         self.buf = torch.empty(self.step_bytes + 2 * self.layer_bytes, dtype=torch.uint8, device=device)
         self._typed: Dict[torch.dtype, torch.Tensor] = {}
+        self._strided = _build.load_launch().strided
         self._base = [0, self.step_bytes, self.step_bytes + self.layer_bytes]
         self._size = [self.step_bytes, self.layer_bytes, self.layer_bytes]
         self._off = [0, 0, 0]
@@ -203,11 +206,11 @@ class Workspace:
                 f"{which} workspace too small: need {end} bytes, have {self._size[region]} "
                 f"(the step brings more tokens than max_batch_tokens allows)")
         self._off[region] = end
-        # one call on a view of the whole buffer in this type, not a slice, a change of type and a change of shape
+        # one native call on a view of the whole buffer in this type, not a slice, a change of type and a change of shape
         whole = self._typed.get(dtype)
         if whole is None:
             whole = self._typed[dtype] = self.buf.view(dtype)
-        return whole.as_strided(shape, layout[1], (self._base[region] + start) // size)
+        return self._strided(whole, shape, layout[1], (self._base[region] + start) // size)
 
     def take(self, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         return self._take(self._cur, shape, dtype)
