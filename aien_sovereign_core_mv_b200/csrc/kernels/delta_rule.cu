@@ -13,6 +13,7 @@
 // the next chunk of tokens arrive through cp.async while the current one is walked, and the next token's are taken
 // into registers while the current one's sums are on their way.  Every operation is float32 and a token's are the
 // same whatever the cut of the prompt or the batch, so its output depends on the tokens before it only through S.
+// (Single tokens have a kernel of their own, which adds a column's products in another order.)
 //
 // The state lives in the request's slot between steps (a portion whose first token has position 0 starts from zero).
 //
@@ -205,6 +206,86 @@ delta_rule_kernel(const float* __restrict__ qkv, long ld, int q_off, int k_off, 
     }
 }
 
+// One token a request: what counts is the state, read and written once, and how much of it is on its way at a time.  A CTA has a
+// head's whole state in registers (V / 4 threads across a row, 16 rows or fewer a thread), all of it requested before the
+// token's rows arrive; the sums over a column meet in shared memory, once.  64 requests, 16 heads of 128 x 128 (134 MB
+// of state read and written), B200: 81 us by delta_rule_kernel, whose threads read 4 bytes of every row they own; 26 us so
+// (5.1 TB/s).
+constexpr int DT_THREADS = 256, DT_ROWS = 16;
+
+template <int LANES>
+__global__ void __launch_bounds__(DT_THREADS, 2)
+delta_token_kernel(const float* __restrict__ qkv, long ld, int q_off, int k_off, int v_off, const float* __restrict__ gb, long ldgb,
+                   float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slot_map,
+                   const int* __restrict__ q_start, const int* __restrict__ positions, float* __restrict__ o, long ldo,
+                   int heads, int G, int D, int longest) {
+    constexpr int RG = DT_THREADS / LANES, V = 4 * LANES, ROWS = 128 / RG < DT_ROWS ? 128 / RG : DT_ROWS;
+    __shared__ __align__(16) float rows[2][128];               // k, q
+    __shared__ __align__(16) float sums[2][RG][V];             // S^T k and S^T q, by row groups
+    __shared__ float dots[RG];
+    const int s = blockIdx.y, h = blockIdx.x, kvh = h / (heads / G), tid = threadIdx.x;
+    const int t0 = q_start[s], t1 = q_start[s + 1];
+    if (t1 <= t0 || t1 - t0 > longest) return;
+    const int rg = tid / LANES, c = tid % LANES * 4;
+    float* st = state + (size_t)slot_map[s] * state_stride + s_off + (size_t)h * D * V + c;
+    const bool fresh = positions[t0] == 0;
+    float4 S[ROWS];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+        const int d = rg + RG * j;
+        S[j] = (!fresh && d < D) ? *reinterpret_cast<const float4*>(st + (size_t)d * V) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int t = t0; t < t1; ++t) {                 // once, unless a step of as many tokens as requests has an empty request beside a portion
+        const float* row = qkv + (size_t)t * ld;
+        {
+            const int which = tid >> 7, d = tid & 127;
+            rows[which][d] = d < D ? row[(which ? q_off : k_off) + kvh * D + d] : 0.f;
+        }
+        const float4 v = *reinterpret_cast<const float4*>(row + v_off + (size_t)h * V + c);
+        const float g = gb[(size_t)t * ldgb + h], beta = gb[(size_t)t * ldgb + heads + h];
+        __syncthreads();
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        float kq = 0.f;
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            const float k = rows[0][rg + RG * j], q = rows[1][rg + RG * j];
+            a.x = fmaf(S[j].x, k, a.x); a.y = fmaf(S[j].y, k, a.y); a.z = fmaf(S[j].z, k, a.z); a.w = fmaf(S[j].w, k, a.w);
+            b.x = fmaf(S[j].x, q, b.x); b.y = fmaf(S[j].y, q, b.y); b.z = fmaf(S[j].z, q, b.z); b.w = fmaf(S[j].w, q, b.w);
+            kq = fmaf(k, q, kq);
+        }
+        *reinterpret_cast<float4*>(&sums[0][rg][c]) = a;
+        *reinterpret_cast<float4*>(&sums[1][rg][c]) = b;
+        if (c == 0) dots[rg] = kq;
+        __syncthreads();
+        a = b = make_float4(0.f, 0.f, 0.f, 0.f);
+        kq = 0.f;
+#pragma unroll
+        for (int r = 0; r < RG; ++r) {
+            const float4 x = *reinterpret_cast<const float4*>(&sums[0][r][c]), y = *reinterpret_cast<const float4*>(&sums[1][r][c]);
+            a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+            b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+            kq += dots[r];
+        }
+        const float4 u = make_float4(beta * (v.x - g * a.x), beta * (v.y - g * a.y), beta * (v.z - g * a.z), beta * (v.w - g * a.w));
+        if (rg == 0) {
+            float* dst = o + (size_t)t * ldo + (size_t)h * V + c;
+            dst[0] = fmaf(kq, u.x, g * b.x); dst[1] = fmaf(kq, u.y, g * b.y); dst[2] = fmaf(kq, u.z, g * b.z); dst[3] = fmaf(kq, u.w, g * b.w);
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            const float k = rows[0][rg + RG * j];
+            S[j].x = fmaf(k, u.x, g * S[j].x); S[j].y = fmaf(k, u.y, g * S[j].y);
+            S[j].z = fmaf(k, u.z, g * S[j].z); S[j].w = fmaf(k, u.w, g * S[j].w);
+        }
+        if (t + 1 < t1) __syncthreads();                        // the rows are read before the next token's arrive
+    }
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+        const int d = rg + RG * j;
+        if (d < D) *reinterpret_cast<float4*>(st + (size_t)d * V) = S[j];
+    }
+}
+
 __device__ __forceinline__ float gate_act(float z, int kind) {
     const float sg = 1.0f / (1.0f + expf(-z));
     return kind == 1 ? z * sg : sg;
@@ -284,14 +365,22 @@ static void launch_delta_rule(cudaStream_t stream, const float* qkv, long ld, in
 
 // qkv float32 [T, ld]: prepared q (G*D) at q_off, k (G*D) at k_off, v (heads*V) at v_off; gb float32 [T, ldgb]: decay
 // of head h at column h, beta at heads + h.  state: float32 rows of state_stride numbers per slot, S [heads][D][V] at
-// s_off.  Request s of the step (tokens q_start[s] .. q_start[s+1]) continues from slot slot_map[s].  o float32 [T, ldo].
+// s_off.  T: the step's tokens.  Request s of the step (tokens q_start[s] .. q_start[s+1]) continues from slot slot_map[s].  o float32 [T, ldo].
 // longest > 0: requests that bring more tokens are served elsewhere and left alone here.
 AIEN_API int aien_delta_rule(const float* qkv, long ld, int q_off, int k_off, int v_off, const float* gb, long ldgb, float* state,
                              size_t state_stride, size_t s_off, const int* slot_map, const int* q_start, const int* positions,
-                             float* o, long ldo, int S, int heads, int G, int D, int V, int longest, cudaStream_t stream) {
+                             float* o, long ldo, int T, int S, int heads, int G, int D, int V, int longest, cudaStream_t stream) {
     if (S <= 0) return 0;
     if (longest <= 0) longest = 0x7fffffff;
     if (heads <= 0 || G <= 0 || heads % G || D <= 0 || D > 256 || V <= 0 || S > 65535 || heads > 65535) return AIEN_E_SHAPE;
+    // single tokens, and states whose rows are 64 or 128 columns and start on 16-byte boundaries (D <= 128: a thread's share fits its registers)
+    if ((T == S || longest == 1) && (V == 128 || V == 64) && D <= 128 && ((ld | v_off) & 3) == 0 && ((state_stride | s_off) & 3) == 0 &&
+        ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(state)) & 15) == 0) {
+        const auto kern = V == 128 ? delta_token_kernel<32> : delta_token_kernel<16>;
+        kern<<<dim3(heads, S), DT_THREADS, 0, stream>>>(qkv, ld, q_off, k_off, v_off, gb, ldgb, state, state_stride, s_off, slot_map, q_start, positions,
+                                                        o, ldo, heads, G, D, longest);
+        return launch_status();
+    }
 #define DR_CASE(N, R) launch_delta_rule<N, R>(stream, qkv, ld, q_off, k_off, v_off, gb, ldgb, state, state_stride, s_off, slot_map, q_start, positions, o, ldo, S, heads, G, D, V, longest)
     if (D <= 16) DR_CASE(4, 4);
     else if (D <= 32) DR_CASE(8, 4);

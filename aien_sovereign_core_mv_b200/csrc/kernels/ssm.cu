@@ -253,8 +253,10 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
 
 // One token a request (as many tokens as requests): a thread group lives for one token, so what counts is how many are resident and how much each
 // moves.  Four (sixteen) lanes a channel, no shared memory; 64 requests x 4,096 channels x 16 states (33.5 MB of
-// state read and written): 13.9 us, against 17.5 us with the step sizes in a launch of their own and 52 us for the walk's kernel.
-template <int LANES, int CH, typename TO>
+// state read and written): 12.8 us with float4 moves and 15.9 without, against 17.5 us with the step sizes in a launch of their own and
+// 52 us for the walk's kernel.
+// VEC: a lane's state values, rates, B and C as float4 (they lie on 16-byte boundaries and N = LANES CH).
+template <int LANES, int CH, bool VEC, typename TO>
 __global__ void __launch_bounds__(SSM_THREADS)
 selective_scan_token_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
                             float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots,
@@ -265,23 +267,41 @@ selective_scan_token_kernel(ScanRowsIn in, const float* __restrict__ A, const vo
     const int c = live ? gid / LANES : inner - 1, ln = gid % LANES, n0 = ln * CH;   // lanes beyond the last channel repeat it and write nothing
     float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)c * N + n0;
     const bool zero = positions[t0] == 0;
-    float S[CH], a[CH];
+    __align__(16) float S[CH], a[CH];
+    if (VEC) {
 #pragma unroll
-    for (int i = 0; i < CH; ++i) {
-        const bool ok = n0 + i < N;
-        S[i] = (ok && !zero) ? st[i] : 0.f;
-        a[i] = ok ? decay_rate<TO>(A[(size_t)c * N + n0 + i]) : 0.f;
+        for (int i = 0; i < CH; i += 4) {
+            *reinterpret_cast<float4*>(S + i) = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(st + i);
+            *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(A + (size_t)c * N + n0 + i);
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) a[i] = decay_rate<TO>(a[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const bool ok = n0 + i < N;
+            S[i] = (ok && !zero) ? st[i] : 0.f;
+            a[i] = ok ? decay_rate<TO>(A[(size_t)c * N + n0 + i]) : 0.f;
+        }
     }
     int t = t0;
     do {                                            // once, unless a step of as many tokens as requests has an empty request beside a portion
         const float* br = in.bc + t * in.ldbc + in.b_off + n0;
         const float* cr = in.bc + t * in.ldbc + in.c_off + n0;
-        float bv[CH], cv[CH];
+        __align__(16) float bv[CH], cv[CH];
+        if (VEC) {
 #pragma unroll
-        for (int i = 0; i < CH; ++i) {
-            const bool ok = n0 + i < N;
-            bv[i] = ok ? br[i] : 0.f;
-            cv[i] = ok ? cr[i] : 0.f;
+            for (int i = 0; i < CH; i += 4) {
+                *reinterpret_cast<float4*>(bv + i) = *reinterpret_cast<const float4*>(br + i);
+                *reinterpret_cast<float4*>(cv + i) = *reinterpret_cast<const float4*>(cr + i);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                const bool ok = n0 + i < N;
+                bv[i] = ok ? br[i] : 0.f;
+                cv[i] = ok ? cr[i] : 0.f;
+            }
         }
         const float x = in.x[t * in.ldx + c], z = in.z[t * in.ldz + c];
         const float dt = ssm_softplus(in.dtz[t * in.lddt + c] + load_dyn(dt_bias, pdt, c)), dx = dt * x;
@@ -295,7 +315,11 @@ selective_scan_token_kernel(ScanRowsIn in, const float* __restrict__ A, const vo
         for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
         if (ln == 0 && live) out[t * ldo + c] = from_f<TO>(fmaf(load_dyn(D, pdt, c), x, y) * ssm_silu(z));
     } while (++t < t1);
-    if (live) {
+    if (!live) return;
+    if (VEC) {
+#pragma unroll
+        for (int i = 0; i < CH; i += 4) *reinterpret_cast<float4*>(st + i) = *reinterpret_cast<const float4*>(S + i);
+    } else {
 #pragma unroll
         for (int i = 0; i < CH; ++i) if (n0 + i < N) st[i] = S[i];
     }
@@ -446,6 +470,66 @@ ssd_scan_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, in
 // out[t] = the three bfloat16 parts of x[t]'s numbers, part by part: x = p0 + p1 + p2 up to 2^-25 of x (each part rounds
 // what the ones before leave).  With the weights three times side by side a product on the tensor cores then has float32
 // rows on the left (parts_product.cu).  x may come as partial products over ranges of K: the product that makes it has
+// The duality form where a request brings one token and a state column 128 numbers: what counts is the state, read and written
+// once, and how much of it is on its way at a time.  A warp has eight columns of a head, a float4 of each a lane, all requested
+// before the token's numbers, and makes the head's step size and decay itself; the eight sums over the lanes are folded
+// together (nine shuffles, added in the order of a butterfly a column).  64 requests x 32 heads of 64 x 128 (134 MB of
+// state read and written), B200: 51 us with one column a warp, and 2 for the steps
+// in a launch of their own; 24 us so (5.6 TB/s).
+constexpr int SSD_TOKEN_COLS = 8;
+
+__global__ void __launch_bounds__(SSD_THREADS)
+ssd_token_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, int c_off, const float* __restrict__ dtr, long lddt,
+                 const float* __restrict__ A, const void* __restrict__ dt_bias, const void* __restrict__ D, int pdt,
+                 float* __restrict__ state, size_t state_stride, size_t s_off, const int* __restrict__ slots, const int* __restrict__ q_start,
+                 const int* __restrict__ positions, float* __restrict__ y_out, long ldy, int heads, int V, int G, int longest) {
+    constexpr int COLS = SSD_TOKEN_COLS, N = 128;
+    const int s = blockIdx.y, lane = threadIdx.x & 31, col0 = (blockIdx.x * (SSD_THREADS / 32) + (threadIdx.x >> 5)) * COLS;
+    const int t0 = q_start[s], t1 = q_start[s + 1];
+    if (t1 <= t0 || t1 - t0 > longest || col0 >= heads * V) return;
+    const int h = col0 / V, g = h / (heads / G);
+    float* st = state + (size_t)slots[s] * state_stride + s_off + (size_t)col0 * N + lane * 4;
+    const bool fresh = positions[t0] == 0;
+    float4 S[COLS];
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) S[i] = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(st + i * N);
+    const float dskip = load_dyn(D, pdt, h), rate = -A[h], bias = load_dyn(dt_bias, pdt, h);
+    for (int t = t0; t < t1; ++t) {                 // once, unless a step of as many tokens as requests has an empty request beside a portion
+        const float* row = xbc + (size_t)t * ld;
+        const float4 b = *reinterpret_cast<const float4*>(row + b_off + (size_t)g * N + lane * 4);
+        const float4 c = *reinterpret_cast<const float4*>(row + c_off + (size_t)g * N + lane * 4);
+        const float x = row[x_off + col0 + (lane & (COLS - 1))];
+        const float dt = ssm_softplus(dtr[(size_t)t * lddt + h] + bias), e = expf(rate * dt);
+        float y[COLS];
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) {
+            const float dx = dt * __shfl_sync(0xffffffffu, x, i);
+            S[i].x = fmaf(e, S[i].x, dx * b.x);
+            S[i].y = fmaf(e, S[i].y, dx * b.y);
+            S[i].z = fmaf(e, S[i].z, dx * b.z);
+            S[i].w = fmaf(e, S[i].w, dx * b.w);
+            y[i] = fmaf(S[i].w, c.w, fmaf(S[i].z, c.z, fmaf(S[i].y, c.y, S[i].x * c.x)));
+        }
+        // lane bits 0, 1, 2 choose the column (4, 2, 1) that the lane goes on with
+#pragma unroll
+        for (int k = COLS / 2, bit = 1; k > 0; k >>= 1, bit <<= 1) {
+            const bool upper = lane & bit;
+#pragma unroll
+            for (int i = 0; i < k; ++i) {
+                const float mine = upper ? y[i + k] : y[i], other = upper ? y[i] : y[i + k];
+                y[i] = mine + __shfl_xor_sync(0xffffffffu, other, bit);
+            }
+        }
+        float sum = y[0] + __shfl_xor_sync(0xffffffffu, y[0], 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        const int col = (lane & 1) * 4 + (lane & 2) + ((lane >> 2) & 1);
+        const float xc = __shfl_sync(0xffffffffu, x, col);
+        if (lane < COLS) y_out[(size_t)t * ldy + col0 + col] = fmaf(dskip, xc, sum);
+    }
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) *reinterpret_cast<float4*>(st + i * N) = S[i];
+}
+
 // few columns (160 over 4,096: 32 tiles at 2,048 tokens, 28 us) and is cut over the whole GPU (14 us, and 1.7 more here).
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, long ldx, int P, size_t part_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ rest,
@@ -527,7 +611,10 @@ static void launch_selective_scan(const ScanArgs& a) {
 template <int LANES, int CH, typename TO>
 static void launch_selective_scan_token(const ScanArgs& a) {
     const unsigned gx = (unsigned)(((long)a.inner * LANES + SSM_THREADS - 1) / SSM_THREADS);
-    selective_scan_token_kernel<LANES, CH, TO><<<dim3(gx, a.S), SSM_THREADS, 0, a.stream>>>(
+    const bool vec = CH % 4 == 0 && a.N == LANES * CH && a.in.wide_bc && ((a.state_stride | a.s_off) & 3) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(a.state) | reinterpret_cast<uintptr_t>(a.A)) & 15) == 0;
+    const auto kern = vec ? selective_scan_token_kernel<LANES, CH, CH % 4 == 0, TO> : selective_scan_token_kernel<LANES, CH, false, TO>;
+    kern<<<dim3(gx, a.S), SSM_THREADS, 0, a.stream>>>(
         a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N);
 }
 
@@ -650,6 +737,13 @@ AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int 
         else if (N <= 64) launch_ssd_scan<32, 2, 1, false>(a);
         else if (N <= 128) { if (vec) launch_ssd_scan<32, 4, 1, true>(a); else launch_ssd_scan<32, 4, 1, false>(a); }
         else { if (vec && N % 8 == 0) launch_ssd_scan<32, 8, 1, true>(a); else launch_ssd_scan<32, 8, 1, false>(a); }
+    if ((T == S || longest == 1) && vec && N == 128 && V % SSD_TOKEN_COLS == 0) {
+        if (T != S) ssd_steps_kernel<<<(unsigned)(((long)T * heads + 255) / 256), 256, 0, stream>>>(dtr, lddt, A, dt_bias, p_dt, steps, T, heads);
+        const unsigned gx = (unsigned)(((long)heads * V / SSD_TOKEN_COLS + SSD_THREADS / 32 - 1) / (SSD_THREADS / 32));
+        ssd_token_kernel<<<dim3(gx, S), SSD_THREADS, 0, stream>>>(xbc, ld, x_off, b_off, c_off, dtr, lddt, A, dt_bias, D, p_dt, state, state_stride,
+                                                                  s_off, slots, q_start, positions, y, ldy, heads, V, G, longest);
+        return launch_status();
+    }
         return launch_status();
     }
     if (N <= 8) launch_ssd_scan<8, 1, 4, false>(a);

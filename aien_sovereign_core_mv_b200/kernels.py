@@ -1694,7 +1694,7 @@ def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gb: torch.
     else:
         alone = 0
     _check(lib().aien_delta_rule(qkv, qkv.stride(0), int(q_off), int(k_off), int(v_off), gb, gb.stride(0), state, state.shape[1],
-                                 int(s_off), slot_map, q_start, positions, o, o.stride(0), int(num_seqs), int(heads),
+                                 int(s_off), slot_map, q_start, positions, o, o.stride(0), qkv.shape[0], int(num_seqs), int(heads),
                                  int(qk_heads), int(dim), int(vdim), 1 if alone else 0, _stream()), "delta_rule")
 
 
