@@ -56,8 +56,10 @@ struct Segments {
 //   * inside the walk, eight tokens at a time, only one multiply-add a state value depends on the token before.
 // 2,048 tokens of 4,096 channels with 16 states each, one request, B200: 764 us, and 26 us for the step sizes, with the
 // rows fetched into registers four tokens ahead; 147 us so, 7 of them the gate's exponential and division
-// (31 instructions a token and warp, of which half a dozen in the prologue and epilogue of a stage; 16 lanes: 180 us, 4: 267 us).
-// With few channels a portion is cut into segments (see kernels.selective_scan_segments).
+// (31 instructions a token and warp, of which half a dozen in the prologue and epilogue of a stage; 16 lanes: 180 us, 4: 216 us).
+// With few channels a portion is cut into segments (see kernels.selective_scan_segments): 126 us with four lanes a channel, of
+// which the passes take 50 and 70; there 70 % of the issue slots are used (37 and 55 instructions a token and warp of eight
+// channels, a third of them the step sizes and the gate) and 50 to 60 % of the special-function unit.
 template <int LANES, int CH>
 struct ScanCfg {
     static constexpr int NP = LANES * CH;
@@ -199,7 +201,8 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
 #pragma unroll
                 for (int i = 0; i < CH; i += 2) {
                     const float2 b2 = make_float2(bv[i], bv[(i + 1) % CH]), c2 = FIRST ? b2 : make_float2(cv[i], cv[(i + 1) % CH]);
-                    const float2 e = make_float2(decay_exp<TO>(dd.x * a[i]), decay_exp<TO>(dd.x * a[(i + 1) % CH]));
+                    const float2 p = __fmul2_rn(make_float2(dd.x, dd.x), make_float2(a[i], a[(i + 1) % CH]));
+                    const float2 e = make_float2(decay_exp<TO>(p.x), decay_exp<TO>(p.y));
                     const float2 S2 = __ffma2_rn(e, make_float2(S[i], S[(i + 1) % CH]), __fmul2_rn(make_float2(dd.y, dd.y), b2));
                     S[i] = S2.x; S[(i + 1) % CH] = S2.y;
                     if (!FIRST) ys = __ffma2_rn(S2, c2, ys);
@@ -467,9 +470,6 @@ ssd_scan_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, in
     }
 }
 
-// out[t] = the three bfloat16 parts of x[t]'s numbers, part by part: x = p0 + p1 + p2 up to 2^-25 of x (each part rounds
-// what the ones before leave).  With the weights three times side by side a product on the tensor cores then has float32
-// rows on the left (parts_product.cu).  x may come as partial products over ranges of K: the product that makes it has
 // The duality form where a request brings one token and a state column 128 numbers: what counts is the state, read and written
 // once, and how much of it is on its way at a time.  A warp has eight columns of a head, a float4 of each a lane, all requested
 // before the token's numbers, and makes the head's step size and decay itself; the eight sums over the lanes are folded
@@ -530,6 +530,9 @@ ssd_token_kernel(const float* __restrict__ xbc, long ld, int x_off, int b_off, i
     for (int i = 0; i < COLS; ++i) *reinterpret_cast<float4*>(st + i * N) = S[i];
 }
 
+// out[t] = the three bfloat16 parts of x[t]'s numbers, part by part: x = p0 + p1 + p2 up to 2^-25 of x (each part rounds
+// what the ones before leave).  With the weights three times side by side a product on the tensor cores then has float32
+// rows on the left (parts_product.cu).  x may come as partial products over ranges of K: the product that makes it has
 // few columns (160 over 4,096: 32 tiles at 2,048 tokens, 28 us) and is cut over the whole GPU (14 us, and 1.7 more here).
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, long ldx, int P, size_t part_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ rest,
@@ -619,7 +622,10 @@ static void launch_selective_scan_token(const ScanArgs& a) {
 }
 
 // Eight lanes a channel; with fewer than 2,048 channels in the step, whose walkers would leave SM schedulers without a
-// warp, and with many state values, sixteen.
+// warp, and with many state values, sixteen.  Where walkers are many, four with four states each, whose instructions per
+// state are fewer: of 16 states in segments beyond 512 channels, and whole from 12,288 channels of the step's requests on (six of
+// 300 tokens, 4,096 channels each: 88 us with eight lanes, 75 with four; six of 80 tokens 27 and 22; four of 512 tokens, 2,048
+// channels each, 54 and 64).  In segments of up to 512 channels eight from 512 tokens on (1,024 tokens: 26 us with sixteen, 23).
 template <typename TO>
 static int dispatch_selective_scan(const ScanArgs& a) {
     const int N = a.N;
@@ -636,9 +642,10 @@ static int dispatch_selective_scan(const ScanArgs& a) {
     }
     if (N <= 8) launch_selective_scan<8, 1, TO>(a);
     else if (N <= 16) {
-        const char* e = getenv("SCANL"); const int L = e ? atoi(e) : 0;
-        if (L == 4) launch_selective_scan<4, 4, TO>(a);
-        else if (L == 16 || (L == 0 && few)) launch_selective_scan<16, 1, TO>(a);
+        const long channels = (long)a.inner * a.S;
+        const bool few_cut = channels <= 512 && a.T >= 512L * a.S;
+        if (a.sg.mode != 0 ? channels > 512 : channels >= 12288) launch_selective_scan<4, 4, TO>(a);
+        else if (few && !(a.sg.mode != 0 && few_cut)) launch_selective_scan<16, 1, TO>(a);
         else launch_selective_scan<8, 2, TO>(a);
     }
     else if (N <= 32) { if (few) launch_selective_scan<16, 2, TO>(a); else launch_selective_scan<8, 4, TO>(a); }
@@ -730,13 +737,6 @@ AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int 
     // float4 moves: every lane's first state value, B and C value on a 16-byte boundary, whole groups of four inside N
     const bool vec = N >= 128 && N % 4 == 0 && ld % 4 == 0 && b_off % 4 == 0 && c_off % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
                      ((uintptr_t)xbc & 15) == 0 && ((uintptr_t)state & 15) == 0 && (scratch == nullptr || ((uintptr_t)scratch & 15) == 0);
-    if (T == S || longest == 1) {                     // single tokens: no rows fetched ahead (fewer registers, more CTAs resident)
-        if (N <= 8) launch_ssd_scan<8, 1, 1, false>(a);
-        else if (N <= 16) launch_ssd_scan<8, 2, 1, false>(a);
-        else if (N <= 32) launch_ssd_scan<32, 1, 1, false>(a);
-        else if (N <= 64) launch_ssd_scan<32, 2, 1, false>(a);
-        else if (N <= 128) { if (vec) launch_ssd_scan<32, 4, 1, true>(a); else launch_ssd_scan<32, 4, 1, false>(a); }
-        else { if (vec && N % 8 == 0) launch_ssd_scan<32, 8, 1, true>(a); else launch_ssd_scan<32, 8, 1, false>(a); }
     if ((T == S || longest == 1) && vec && N == 128 && V % SSD_TOKEN_COLS == 0) {
         if (T != S) ssd_steps_kernel<<<(unsigned)(((long)T * heads + 255) / 256), 256, 0, stream>>>(dtr, lddt, A, dt_bias, p_dt, steps, T, heads);
         const unsigned gx = (unsigned)(((long)heads * V / SSD_TOKEN_COLS + SSD_THREADS / 32 - 1) / (SSD_THREADS / 32));
@@ -744,6 +744,13 @@ AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int 
                                                                   s_off, slots, q_start, positions, y, ldy, heads, V, G, longest);
         return launch_status();
     }
+    if (T == S || longest == 1) {                     // single tokens: no rows fetched ahead (fewer registers, more CTAs resident)
+        if (N <= 8) launch_ssd_scan<8, 1, 1, false>(a);
+        else if (N <= 16) launch_ssd_scan<8, 2, 1, false>(a);
+        else if (N <= 32) launch_ssd_scan<32, 1, 1, false>(a);
+        else if (N <= 64) launch_ssd_scan<32, 2, 1, false>(a);
+        else if (N <= 128) { if (vec) launch_ssd_scan<32, 4, 1, true>(a); else launch_ssd_scan<32, 4, 1, false>(a); }
+        else { if (vec && N % 8 == 0) launch_ssd_scan<32, 8, 1, true>(a); else launch_ssd_scan<32, 8, 1, false>(a); }
         return launch_status();
     }
     if (N <= 8) launch_ssd_scan<8, 1, 4, false>(a);

@@ -1878,23 +1878,45 @@ def scan_scratch_floats(max_tokens: int, max_seqs: int, lanes: int, parallel: in
     return 2 * (want + 1 + max_seqs) * lanes
 
 
-def selective_scan_segments(num_tokens: int, num_seqs: int, decode_only: bool, inner: int) -> tuple:
+def selective_scan_segments(num_tokens: int, num_seqs: int, decode_only: bool, inner: int, state: int = 16) -> tuple:
     """(segment length, most segments a portion has) for :func:`selective_scan` in a step; (0, 1): every portion in one piece.
-    A whole walk takes 50 ns a token and more however few channels walk, and a CTA has 8 of them; two passes over segments take
-    as long as their length twice, once the GPU has room for the CTAs.  2,048 tokens of one request, 16 states, B200, whole
-    and in segments of 128: 256 channels 101 and 31 us, 1,024 channels 101 and 72, 4,096 channels 152 and 159; 256 tokens in
-    segments of 64: 64 channels 17 and 15 us, 512 channels 17 and 17, 1,024 channels 17 and 19.  It depends on the step's token and
-    request counts and the layer's channels alone."""
-    average = num_tokens // max(num_seqs, 1)
-    if decode_only or inner * num_seqs > (1024 if average >= 1024 else 512) or average < 256:
+    A whole walk takes 50 ns a token and more however few channels walk; two passes over segments take as long as their length
+    twice, once the GPU has room for the CTAs, but every exponential twice.  16 states, one request, B200, us whole (eight or
+    sixteen lanes a channel) and in segments of the length chosen here (eight lanes up to 512 channels, four beyond):
+
+        channels       512 tokens     1,024          2,048
+        512            25 and 17      39 and 23      92 and 33
+        1,024          25 and 24      59 and 32      92 and 50
+        2,048          33 and 29      62 and 42      122 and 71
+        3,072          38 and 36      73 and 58      144 and 103
+        4,096          39 and 40      73 and 70      144 and 126
+        6,144          45 and 56      88 and 97      171 and 179
+
+    and 4,096 channels of requests of 1,500 and 500 tokens (2,048 channels each) 96 and 73.  With more than 16 states, or 8 and fewer, whose
+    forms have other lanes, only steps of few channels are cut.  It depends on the step's token and request counts and
+    the layer's sizes alone."""
+    average, channels = num_tokens // max(num_seqs, 1), inner * num_seqs
+    if 8 < state <= 16:
+        least = 256 if channels <= 512 else 512 if channels <= 3072 else 1000
+        limit = 4096
+    else:
+        least, limit = 256, 1024 if average >= 1024 else 512
+    if decode_only or channels > limit or average < least:
         return 0, 1
-    seg = 128 if average >= 1024 else 64
+    seg = 128 if average >= SCAN_LONG_PORTION else 64
     return seg, -(-num_tokens // seg)
+
+
+SCAN_LONG_PORTION = 1500             # tokens a request on the average, from which the scan's segments are 128 tokens long instead of 64
 
 
 def selective_scan_scratch(max_tokens: int, max_seqs: int, inner: int, N: int) -> int:
     """Upper bound of the float32 scratch that steps in segments take (2 numbers a state value and segment)."""
-    return 2 * (max_tokens // 64 + min(max_seqs, 1024 // inner)) * inner * N if inner <= 1024 else 0
+    seqs = min(max_seqs, (4096 if 8 < N <= 16 else 1024) // inner)        # a step of more requests is not cut
+    if seqs <= 0:
+        return 0
+    segments = max(max_tokens // 128, min(max_tokens, SCAN_LONG_PORTION * seqs) // 64)
+    return 2 * (segments + seqs) * inner * N
 
 
 def selective_scan(x: torch.Tensor, dtz: torch.Tensor, bc: torch.Tensor, b_off: int, c_off: int, z: torch.Tensor, A: torch.Tensor,

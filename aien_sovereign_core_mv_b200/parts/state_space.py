@@ -137,7 +137,7 @@ class SelectiveScan(Mixer):
         else:
             dtz = linear(ctx, xp[:, :R], self.w_dt, out_dtype=torch.float32)
         y = ws.take((T, I), ctx.dtype)
-        seg, nseg = K.selective_scan_segments(T, ctx.num_seqs, ctx.decode_only, I)
+        seg, nseg = K.selective_scan_segments(T, ctx.num_seqs, ctx.decode_only, I, self.state)
         scratch = ws.take((2 * (T // seg + ctx.num_seqs) * I * N,), torch.float32) if seg else None
         K.selective_scan(x, dtz, bc, b_off, b_off + N, proj[:, I:], self.A, self.dt_b, self.D, state, self.conv_floats, group.slot_map,
                          ctx.q_start, ctx.positions, y, ctx.num_seqs, N, seg, nseg, scratch)

@@ -413,6 +413,21 @@ def test_selective_scan_in_the_segments_of_few_channels(inner, N, lens, dtype):
     H.assert_close(S, last, 1e-5, "states")
 
 
+@pytest.mark.parametrize("inner,N,lens", [(700, 16, [600, 601]), (515, 9, [130, 900]), (4093, 12, [1030]), (513, 16, [3, 1600, 1]), (2061, 16, [5, 40, 33, 2, 17, 90]),
+                                          (4100, 13, [16, 1, 31]), (300, 16, [1100]), (512, 16, [511])])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_selective_scan_as_many_walkers_go(inner, N, lens, dtype):
+    """Four lanes a channel, in segments and (from 12,288 channels of the step on) whole, and the steps at the rule's edges; channels
+    that fill no CTA, tokens that fill no stage."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    cut = K.selective_scan_segments(sum(lens), len(lens), False, inner, N)
+    assert 2 * (sum(lens) // max(cut[0], 1) + len(lens)) * inner * N <= K.selective_scan_scratch(sum(lens), len(lens), inner, N) or cut[0] == 0
+    assert (cut[0] > 0) == (inner * len(lens) <= 4096 and sum(lens) // len(lens) >= (256 if inner * len(lens) <= 512 else 512 if inner * len(lens) <= 3072 else 1000))
+    y, S, want, last = _scan_beside_64_bits(K, inner, N, lens, 9, dtype, *([cut] if cut[0] else []))
+    H.assert_close(y, want, 3e-5 if dtype == torch.float32 else 4.2e-3, "results")
+    H.assert_close(S, last, 1e-5, "states")
+
+
 def test_float32_rows_beyond_bfloat16_in_three_parts():
     """Infinities stay what they are, in the parts and in the product over them; the largest numbers stay finite."""
     from aien_sovereign_core_mv_b200 import kernels as K
