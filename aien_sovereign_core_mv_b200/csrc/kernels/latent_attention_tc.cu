@@ -410,29 +410,34 @@ static int launch_latent_tc(const void* q, const void* cache, const int* bt, int
 
 // ---------------------------------------------------------------- one product per head, on the tensor cores
 // C[m, h, n] = sum_k A[m, h, k] * W[h, n, k], times sigmoid(gate[m, h]) when given (see head_project_kernel), for bfloat16 A and W: tiles of 64 x 64 per CTA of
-// four warps, k in steps of 64 through shared memory (cp.async), mma.sync.m16n8k16 with float32 accumulation.
-constexpr int HT_BM = 64, HT_BN = 64, HT_BK = 64, HT_STR = HT_BK + 8;
+// four warps, or 64 x 32 where those would leave SMs idle (16 heads of 64 rows x 128 columns: 64 CTAs, not 32), k in steps of 64 through shared memory
+// (cp.async), mma.sync.m16n8k16 with float32 accumulation.
+constexpr int HT_BM = 64, HT_BK = 64, HT_STR = HT_BK + 8;
 
-// Two stages of k-steps: the next one's pieces are requested before the products of this one.  rows (or null): A's and C's rows
+// What bounds a step of few tokens is a k-step's way through memory: three stages of 32 columns, two of them on their way, and the gate's
+// values are requested with the first.  64 rows, 16 heads, 512 -> 128 columns, B200: 8.2 us with two stages of 64 columns and 13.9
+// with a gate per element read behind the products; 7.5 and 10.4 so.  rows (or null): A's and C's rows
 // are those that it lists, M of them.
-template <typename TC>
+template <int HT_BN, typename TC>
 __global__ void __launch_bounds__(128)
 head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_head, const __nv_bfloat16* __restrict__ W, long w_head,
                        TC* __restrict__ C, long ldc, long c_head, int M, int N, int K, const void* __restrict__ gate, int gdt, long ldg, int gate_n,
                        const int* __restrict__ rows) {
-    __shared__ __align__(16) __nv_bfloat16 As[2][HT_BM * HT_STR];
-    __shared__ __align__(16) __nv_bfloat16 Ws[2][HT_BN * HT_STR];
+    constexpr int HT_STAGES = HT_BN == 32 ? 3 : 2;             // what 48 KB hold
+    __shared__ __align__(16) __nv_bfloat16 As[HT_STAGES][HT_BM * HT_STR];
+    __shared__ __align__(16) __nv_bfloat16 Ws[HT_STAGES][HT_BN * HT_STR];
+    constexpr int NJ = HT_BN / 16;                             // n8 tiles of a warp
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int mh = warp & 1, nh = warp >> 1, g = lane >> 2, c = lane & 3;
     const int m0 = blockIdx.y * HT_BM, n0 = blockIdx.x * HT_BN, h = blockIdx.z;
     A += (size_t)h * a_head;
     W += (size_t)h * w_head;
     C += (size_t)h * c_head;
-    float acc[2][4][4];
+    float acc[2][NJ][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+        for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
     auto fetch = [&](int k0, int st) {
         const uint32_t As_u = (uint32_t)__cvta_generic_to_shared(As[st]), Ws_u = (uint32_t)__cvta_generic_to_shared(Ws[st]);
         for (int idx = tid; idx < HT_BM * (HT_BK / 8); idx += 128) {
@@ -441,19 +446,37 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
             const bool va = kin && m0 + r < M, vw = kin && n0 + r < N;
             const size_t ar = va ? (size_t)(rows != nullptr ? rows[m0 + r] : m0 + r) : 0;
             lx_cp_async16(As_u + (uint32_t)(r * HT_STR + ch * 8) * 2, A + ar * lda + (va ? k0 + ch * 8 : 0), va);
-            lx_cp_async16(Ws_u + (uint32_t)(r * HT_STR + ch * 8) * 2, W + (size_t)(vw ? n0 + r : 0) * K + (vw ? k0 + ch * 8 : 0), vw);
+            if (r < HT_BN) lx_cp_async16(Ws_u + (uint32_t)(r * HT_STR + ch * 8) * 2, W + (size_t)(vw ? n0 + r : 0) * K + (vw ? k0 + ch * 8 : 0), vw);
         }
         lx_cp_async_commit();
     };
-    fetch(0, 0);
-    for (int k0 = 0, st = 0; k0 < K; k0 += HT_BK, st ^= 1) {
-        if (k0 + HT_BK < K) {
-            fetch(k0 + HT_BK, st ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            lx_cp_async_wait_all();
+    // the places of this thread's results, and with a gate an element its values for them
+    size_t at[2][2];
+    float gates[2][2][NJ][2];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int ml = m0 + mh * 32 + mt * 16 + g + r * 8;
+            at[mt][r] = ml < M ? (size_t)(rows != nullptr ? rows[ml] : ml) : 0;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int n = n0 + nh * (HT_BN / 2) + j * 8 + 2 * c + e;
+                    gates[mt][r][j][e] = gate_n > 0 && ml < M && n < N ? load_dyn(gate, gdt, at[mt][r] * ldg + (size_t)h * gate_n + n) : 0.f;
+                }
         }
-        __syncthreads();
+    const int steps = (K + HT_BK - 1) / HT_BK;
+    for (int i = 0; i < HT_STAGES - 1; ++i) {
+        if (i < steps) fetch(i * HT_BK, i);
+        else lx_cp_async_commit();
+    }
+    for (int i = 0, st = 0; i < steps; ++i, st = st + 1 == HT_STAGES ? 0 : st + 1) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(HT_STAGES - 2) : "memory");
+        __syncthreads();                                        // the step has landed, and everyone is done with the one before it
+        if (i + HT_STAGES - 1 < steps) fetch((i + HT_STAGES - 1) * HT_BK, st == 0 ? HT_STAGES - 1 : st - 1);
+        else lx_cp_async_commit();
         const uint32_t As_u = (uint32_t)__cvta_generic_to_shared(As[st]), Ws_u = (uint32_t)__cvta_generic_to_shared(Ws[st]);
 #pragma unroll
         for (int kk = 0; kk < HT_BK / 16; ++kk) {
@@ -463,10 +486,10 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
                 lx_ldmatrix_x4(As_u + (uint32_t)((mh * 32 + mt * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * HT_STR + kk * 16 + (lane >> 4) * 8) * 2,
                                a[mt][0], a[mt][1], a[mt][2], a[mt][3]);
 #pragma unroll
-            for (int j = 0; j < 4; j += 2) {
+            for (int j = 0; j < NJ; j += 2) {
                 const int mi = lane >> 3;
                 uint32_t b0, b1, b2, b3;
-                lx_ldmatrix_x4(Ws_u + (uint32_t)((nh * 32 + (j + (mi >> 1)) * 8 + (lane & 7)) * HT_STR + kk * 16 + (mi & 1) * 8) * 2, b0, b1, b2, b3);
+                lx_ldmatrix_x4(Ws_u + (uint32_t)((nh * (HT_BN / 2) + (j + (mi >> 1)) * 8 + (lane & 7)) * HT_STR + kk * 16 + (mi & 1) * 8) * 2, b0, b1, b2, b3);
 #pragma unroll
                 for (int mt = 0; mt < 2; ++mt) {
                     lx_mma(acc[mt][j], a[mt][0], a[mt][1], a[mt][2], a[mt][3], b0, b1);
@@ -474,7 +497,6 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
                 }
             }
         }
-        __syncthreads();
     }
     const bool pairs = ((N | ldc | c_head) & 1) == 0 && ((uintptr_t)C & (2 * sizeof(TC) - 1)) == 0;     // two neighbouring columns at a time
 #pragma unroll
@@ -483,16 +505,16 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
         for (int r = 0; r < 2; ++r) {
             const int ml = m0 + mh * 32 + mt * 16 + g + r * 8;
             if (ml >= M) continue;
-            const size_t m = (size_t)(rows != nullptr ? rows[ml] : ml);
+            const size_t m = at[mt][r];
             const float gs = (gate != nullptr && gate_n == 0) ? 1.0f / (1.0f + expf(-load_dyn(gate, gdt, m * ldg + h))) : 1.0f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int n = n0 + nh * 32 + j * 8 + 2 * c;
+            for (int j = 0; j < NJ; ++j) {
+                const int n = n0 + nh * (HT_BN / 2) + j * 8 + 2 * c;
                 float v[2] = {acc[mt][j][2 * r] * gs, acc[mt][j][2 * r + 1] * gs};
                 if (gate_n > 0) {
 #pragma unroll
                     for (int e = 0; e < 2; ++e)
-                        if (n + e < N) v[e] *= __fdividef(1.0f, 1.0f + __expf(-load_dyn(gate, gdt, m * ldg + (size_t)h * gate_n + n + e)));
+                        v[e] *= __fdividef(1.0f, 1.0f + __expf(-gates[mt][r][j][e]));
                 }
                 TC* dst = C + m * ldc + n;
                 if (pairs && n + 1 < N) {
@@ -589,10 +611,13 @@ AIEN_API int aien_head_project_tc(const void* A, long lda, long a_head, const vo
     if (M <= 0 || N <= 0 || heads <= 0) return 0;
     if (K <= 0 || heads > 65535 || gate_n < 0 || (gate_n > 0 && (gate == nullptr || gate_n != N))) return AIEN_E_SHAPE;
     if ((K & 7) || (lda & 7) || (a_head & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return AIEN_E_ALIGN;
-    dim3 grid((N + HT_BN - 1) / HT_BN, (M + HT_BM - 1) / HT_BM, heads);
-    if (grid.y > 65535) return AIEN_E_SHAPE;
-    AIEN_DISPATCH_DTYPE(c_dt, TC, (head_project_tc_kernel<TC><<<grid, 128, 0, stream>>>((const __nv_bfloat16*)A, lda, a_head, (const __nv_bfloat16*)W,
-                                                                                     (long)N * K, (TC*)C, ldc, c_head, M, N, K, gate, gate_dt, ldg, gate_n, rows)));
+    const long rows64 = (M + HT_BM - 1) / HT_BM;
+    if (rows64 > 65535) return AIEN_E_SHAPE;
+    const bool narrow = rows64 * ((N + 63) / 64) * heads <= 148;           // 64 columns would give every SM one CTA at most
+    const int bn = narrow ? 32 : 64;
+    const dim3 grid((N + bn - 1) / bn, (unsigned)rows64, heads);
+    AIEN_DISPATCH_DTYPE(c_dt, TC, ((narrow ? head_project_tc_kernel<32, TC> : head_project_tc_kernel<64, TC>)<<<grid, 128, 0, stream>>>(
+        (const __nv_bfloat16*)A, lda, a_head, (const __nv_bfloat16*)W, (long)N * K, (TC*)C, ldc, c_head, M, N, K, gate, gate_dt, ldg, gate_n, rows)));
     return launch_status();
 }
 
