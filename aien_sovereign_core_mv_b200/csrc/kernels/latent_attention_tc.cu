@@ -30,9 +30,6 @@ __device__ __forceinline__ void lx_cp_async_wait_all() { asm volatile("cp.async.
 __device__ __forceinline__ void lx_ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
-__device__ __forceinline__ void lx_ldmatrix_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
 __device__ __forceinline__ void lx_ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
@@ -46,40 +43,30 @@ __device__ __forceinline__ uint32_t lx_pack(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&p);
 }
 
-// SLABS: 16-row slabs of a tile (4: tiles of 64 rows, for portions; 1: tiles of 16 rows, for steps of single tokens, where
-// a request has only its heads as rows).  The WARPS / SLABS warps of a slab deal out the keys of a block for the scores and
-// the channels for the weighted sum (tiles of 64 rows run 16 warps: four to a slab, so that a warp's share of the weighted
-// sum, 16 rows x a quarter of the latent, leaves registers for loads in flight).
-//
-// Tiles of 16 rows are bound by the reading of their keys.  They take them in blocks of 32 through two stages, the next one
-// requested before the products of this one, by CTAs of four warps that fit an SM twice (85 KB at a latent of 512); where a key's
-// row lies is looked up a block further ahead, by one thread a key, and a warp then copies whole rows.  With a block of 64
-// looked up, copied and waited for in turn (every 16-byte piece with its own look-up), 64 requests at 1,500 tokens of
-// context took 126 us for 98 MB; 50 us so, with four CTAs a token instead of two (a token's 16 heads are one tile).
-template <int SLABS> struct LxBlock {
-    static constexpr int BN = SLABS == 1 ? 32 : 64, STAGES = SLABS == 1 ? 2 : 1, PSTR = BN + 8;
-};
+// A tile's 64 rows are four 16-row slabs; the four warps of a slab deal out the keys of a block for the scores and the channels
+// for the weighted sum, so that a warp's share of the weighted sum, 16 rows x a quarter of the latent, leaves registers for
+// loads in flight.  (Steps of single tokens have latent_token_kernel.)
+constexpr int LX_SLABS = LX_BM / 16, LX_WARPS = 16, LX_PSTR = LX_BN + 8;
 
-template <int R, int SLABS, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, SLABS == 1 ? 2 : 1)
+template <int R>
+__global__ void __launch_bounds__(LX_WARPS * 32, 1)
 latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                            const int* __restrict__ block_table, int max_blocks, const int* __restrict__ q_start,
                            const int* __restrict__ positions, int S, __nv_bfloat16* __restrict__ out,
                            int H, int r_lat, int rd, int page_size, int window, float scale_log2e, const float* __restrict__ sinks,
                            int ksplit, float* __restrict__ part_o, float* __restrict__ part_ml, int single_only) {
-    constexpr int LX_BN = LxBlock<SLABS>::BN, STAGES = LxBlock<SLABS>::STAGES, LX_PSTR = LxBlock<SLABS>::PSTR;
-    constexpr int BM = SLABS * 16, PARTS = WARPS / SLABS, KP = LX_BN / PARTS, NJ = KP / 8, CHP = R / PARTS;
+    constexpr int SLABS = LX_SLABS, WARPS = LX_WARPS, BM = LX_BM, PARTS = WARPS / SLABS, KP = LX_BN / PARTS, NJ = KP / 8, CHP = R / PARTS;
     constexpr int DT = CHP / 8;                  // n8 tiles of this warp's share of the channels
     static_assert(DT >= 2 && DT % 2 == 0, "a warp's share of the latent must be whole pairs of n8 tiles");
     // r_lat <= R: the latent's own size; a row's D numbers are read, the rest of its width in shared memory is zeros
     const int D = r_lat + rd, CH = D / 8, KS = (D + 15) / 16, W = lx_row_width(R, D), CHW = W / 8, STR = W + 8;
     extern __shared__ __align__(16) uint8_t lx_smem[];
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(lx_smem);          // [BM][STR]
-    __nv_bfloat16* Ks = Qs + BM * STR;                                      // [STAGES][BN][STR]
-    __nv_bfloat16* Ps = Ks + STAGES * LX_BN * STR;                          // [BM][PSTR]
+    __nv_bfloat16* Ks = Qs + BM * STR;                                      // [BN][STR]
+    __nv_bfloat16* Ps = Ks + LX_BN * STR;                                   // [BM][PSTR]
     float* stat = reinterpret_cast<float*>(Ps + BM * LX_PSTR);              // [PARTS][BM]
     __shared__ int key_row[2][LX_BN];                                       // the cache row of a block's key, -1: not there or not needed
-    const uint32_t Qs_u = (uint32_t)__cvta_generic_to_shared(Qs), Ks0_u = (uint32_t)__cvta_generic_to_shared(Ks);
+    const uint32_t Qs_u = (uint32_t)__cvta_generic_to_shared(Qs), Ks_u = (uint32_t)__cvta_generic_to_shared(Ks);
     const uint32_t Ps_u = (uint32_t)__cvta_generic_to_shared(Ps);
 
     // which request, which rows: the lanes count 32 requests' tiles at a time
@@ -155,30 +142,20 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
     };
     look_up(kb0, key_row[0]);
     look_up(kb0 + ksplit, key_row[1]);
-    __syncthreads();
-    if (STAGES == 2 && kb0 <= kb_end) copy_rows(key_row[0], Ks0_u);
     lx_cp_async_commit();
+    __syncthreads();
     if (ksplit > 1 && kb0 > kb_end) {                                      // Q must have landed even if this CTA gets no block
         lx_cp_async_wait_all();
         __syncthreads();
     }
     for (int kb = kb0, it = 0; kb <= kb_end; kb += ksplit, ++it) {
         const int* rows = key_row[it & 1];
-        uint32_t Ks_u = Ks0_u;
-        if (STAGES == 1) {
-            copy_rows(rows, Ks0_u);
-            lx_cp_async_commit();
-            lx_cp_async_wait_all();
-            __syncthreads();                                               // the block's rows (and, first time, Q) have landed
-        } else {
-            Ks_u += (uint32_t)((it & 1) * LX_BN * STR) * 2;
-            lx_cp_async_wait_all();
-            __syncthreads();                                               // likewise, and everyone is done with the other stage
-            if (kb + ksplit <= kb_end) copy_rows(key_row[(it + 1) & 1], Ks0_u + (uint32_t)(((it + 1) & 1) * LX_BN * STR) * 2);
-            lx_cp_async_commit();
-        }
+        copy_rows(rows, Ks_u);
+        lx_cp_async_commit();
+        lx_cp_async_wait_all();
+        __syncthreads();                                                   // the block's rows (and, first time, Q) have landed
 
-        float sc[NJ][4], sc2[4] = {0.f, 0.f, 0.f, 0.f};                    // sc2: every other k-step's sums where a warp has one tile of keys
+        float sc[NJ][4];
 #pragma unroll
         for (int j = 0; j < NJ; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
         if (active) {
@@ -186,27 +163,16 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
             for (int kk = 0; kk < KS; ++kk) {
                 uint32_t q0r, q1r, q2r, q3r;
                 lx_ldmatrix_x4(q_frag_u + kk * 32, q0r, q1r, q2r, q3r);
-                if constexpr (NJ == 1) {
-                    const int row = half * KP + (lane & 7), col = kk * 16 + ((lane >> 3) & 1) * 8;
-                    uint32_t b0, b1;
-                    lx_ldmatrix_x2(Ks_u + (uint32_t)(row * STR + col) * 2, b0, b1);
-                    lx_mma((kk & 1) ? sc2 : sc[0], q0r, q1r, q2r, q3r, b0, b1);
-                } else {
 #pragma unroll
-                    for (int j = 0; j < NJ; j += 2) {
-                        const int mi = lane >> 3;
-                        const int row = half * KP + (j + (mi >> 1)) * 8 + (lane & 7), col = kk * 16 + (mi & 1) * 8;
-                        uint32_t b0, b1, b2, b3;
-                        lx_ldmatrix_x4(Ks_u + (uint32_t)(row * STR + col) * 2, b0, b1, b2, b3);
-                        lx_mma(sc[j], q0r, q1r, q2r, q3r, b0, b1);
-                        lx_mma(sc[j + (NJ > 1 ? 1 : 0)], q0r, q1r, q2r, q3r, b2, b3);
-                    }
+                for (int j = 0; j < NJ; j += 2) {
+                    const int mi = lane >> 3;
+                    const int row = half * KP + (j + (mi >> 1)) * 8 + (lane & 7), col = kk * 16 + (mi & 1) * 8;
+                    uint32_t b0, b1, b2, b3;
+                    lx_ldmatrix_x4(Ks_u + (uint32_t)(row * STR + col) * 2, b0, b1, b2, b3);
+                    lx_mma(sc[j], q0r, q1r, q2r, q3r, b0, b1);
+                    lx_mma(sc[j + 1], q0r, q1r, q2r, q3r, b2, b3);
                 }
             }
-        }
-        if constexpr (NJ == 1) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) sc[0][e] += sc2[e];
         }
         // masks and this half's row maxima (scores in log2 units)
         float mx0 = -INFINITY, mx1 = -INFINITY;
@@ -342,6 +308,247 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
     }
 }
 
+// Steps of single tokens: a request has only its heads as rows, so a tile is 16 of them.  Eight warps take the keys in blocks of 32
+// through two stages (three where a latent is 256 or fewer numbers), the next requested before the products of this one and
+// its pages two blocks ahead; two CTAs fit an SM.  The warps share out the numbers of a row for the scores (every warp all 32 keys,
+// so that four sums run beside one another), add their parts up in shared memory, where sixteen threads a row make its
+// probabilities, and share out the channels for the weighted sum.  What bounds a block is its chain of phases and the number of
+// its instructions, not its bytes (contexts that lie in L2 take as long): 64 requests at 1,500 tokens (uneven, 98 MB), 16 heads, a
+// latent of 512, four CTAs a token, B200: 49 us with four warps, eight keys a warp and whole rows; 45 with eight warps that share the
+// row; 43 without waiting for a page's number in the block that asks for it; 39 with a warp's copies and products laid out at
+// compile time.  (CTAs dealt out to the tokens by their keys: 48, and 2 more in the merge: the SMs are full as it is.)
+constexpr int LT_BN = 32, LT_WARPS = 8, LT_BM = 16, LT_PSTR = LT_BN + 8, LT_SSTR = LT_BN + 4;
+template <int R> struct LtCfg { static constexpr int STAGES = R == 512 ? 2 : 3; };
+
+template <int R>
+static size_t lt_smem(int D) {
+    return (size_t)(LT_BM + LtCfg<R>::STAGES * LT_BN) * (lx_row_width(R, D) + 8) * 2 + (size_t)LT_BM * LT_PSTR * 2 + (size_t)LT_WARPS * LT_BM * LT_SSTR * 4;
+}
+
+template <int R>
+__global__ void __launch_bounds__(LT_WARPS * 32, 2)
+latent_token_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int max_blocks,
+                    const int* __restrict__ q_start, const int* __restrict__ positions, int S, __nv_bfloat16* __restrict__ out, int H, int r_lat, int rd,
+                    int page_size, int window, float scale_log2e, const float* __restrict__ sinks, int ksplit, float* __restrict__ part_o,
+                    float* __restrict__ part_ml, int single_only) {
+    constexpr int STAGES = LtCfg<R>::STAGES, CHP = R / LT_WARPS, DT = CHP / 8, TURNS = STAGES + 1;
+    const int D = r_lat + rd, CH = D / 8, KS = (D + 15) / 16, W = lx_row_width(R, D), CHW = W / 8, STR = W + 8;
+    extern __shared__ __align__(16) uint8_t lx_smem[];
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(lx_smem);          // [BM][STR]
+    __nv_bfloat16* Ks = Qs + LT_BM * STR;                                   // [STAGES][BN][STR]
+    __nv_bfloat16* Ps = Ks + STAGES * LT_BN * STR;                          // [BM][PSTR]
+    float* parts = reinterpret_cast<float*>(Ps + LT_BM * LT_PSTR);          // [WARPS][BM][SSTR]
+    __shared__ int key_row[TURNS][LT_BN];                                   // the cache row of a block's key, -1: not there or not needed
+    __shared__ float corrs[LT_BM], sums[LT_BM], tops[LT_BM];
+    const uint32_t Qs_u = (uint32_t)__cvta_generic_to_shared(Qs), Ks0_u = (uint32_t)__cvta_generic_to_shared(Ks);
+    const uint32_t Ps_u = (uint32_t)__cvta_generic_to_shared(Ps);
+
+    // which request, which rows: the lanes count 32 requests' tiles at a time
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int s = -1, row0 = 0, unit = 0;                      // unit: how many served tokens come before a single one
+    for (int base = 0, acc = 0; base < S; base += 32) {
+        const int i = base + lane, n = i < S ? q_start[i + 1] - q_start[i] : 0;
+        const int tiles = single_only && n != 1 ? 0 : (n * H + LT_BM - 1) / LT_BM;   // single_only: portions are served elsewhere
+        int upto = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const uint32_t here = __ballot_sync(0xffffffffu, acc + upto > (int)blockIdx.x);
+        if (here != 0) {
+            const int l = __ffs(here) - 1, before = acc + __shfl_sync(0xffffffffu, upto - tiles, l);
+            s = base + l;
+            row0 = ((int)blockIdx.x - before) * LT_BM;
+            unit = before / __shfl_sync(0xffffffffu, tiles, l);
+            break;
+        }
+        acc += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (s < 0) return;
+    const int qs = q_start[s], len = q_start[s + 1] - qs;
+    const int nrows = min(LT_BM, len * H - row0);
+    const int pos_first = positions[qs];
+    const int pos_lo = pos_first + row0 / H, pos_hi = pos_first + (row0 + nrows - 1) / H;
+    const int first = (window > 0 && pos_lo - window + 1 > 0) ? pos_lo - window + 1 : 0;
+    const int* bt = block_table + (size_t)s * max_blocks;
+    const int g = lane >> 2, c = lane & 3;
+
+    const int kb_begin = first / LT_BN, kb_end = pos_hi / LT_BN, kb0 = kb_begin + (int)blockIdx.y;
+    const int blocks = kb0 <= kb_end ? (kb_end - kb0) / ksplit + 1 : 0;
+    // where the keys of this CTA's n-th block lie (one thread a key), and the copies of its rows (a warp a row)
+    const int shift = (page_size & (page_size - 1)) == 0 ? __ffs(page_size) - 1 : -1;
+    auto page_of = [&](int n) {
+        const int key = (kb0 + n * ksplit) * LT_BN + tid;
+        return tid < LT_BN && n < blocks && key >= first && key <= pos_hi ? bt[shift >= 0 ? key >> shift : key / page_size] : -1;
+    };
+    auto place = [&](int n, int turn, int page) {
+        if (tid < LT_BN) {
+            const int key = (kb0 + n * ksplit) * LT_BN + tid;
+            key_row[turn][tid] = page >= 0 ? page * page_size + (shift >= 0 ? key & (page_size - 1) : key % page_size) : -1;
+        }
+    };
+    auto copy_rows = [&](int n, int turn, int stage) {
+        if (n < blocks) {
+            const uint32_t dst = Ks0_u + (uint32_t)((stage * LT_BN + warp) * STR + lane * 8) * 2;
+#pragma unroll
+            for (int i = 0; i < LT_BN / LT_WARPS; ++i) {
+                const int slot = key_row[turn][warp + i * LT_WARPS];
+                const __nv_bfloat16* src = cache + (slot >= 0 ? (size_t)slot * D : 0) + lane * 8;
+#pragma unroll
+                for (int k = 0; k < R / 256; ++k)                          // (R = 128: half a warp's pieces, in the loop below)
+                    lx_cp_async16(dst + (uint32_t)(i * LT_WARPS * STR + k * 256) * 2, src + k * 256, slot >= 0 && lane + 32 * k < CH);
+                for (int ch = lane + R / 256 * 32; ch < CHW; ch += 32) {
+                    const bool copy = slot >= 0 && ch < CH;
+                    lx_cp_async16(dst + (uint32_t)(i * LT_WARPS * STR + (ch - lane) * 8) * 2, copy ? src + (ch - lane) * 8 : cache, copy);
+                }
+            }
+        }
+        lx_cp_async_commit();
+    };
+    for (int n = 0; n < STAGES; ++n) place(n, n, page_of(n));
+    int page = page_of(STAGES);                                            // of the block whose places are written next
+    const __nv_bfloat16* qbase = q + ((size_t)qs * H + row0) * D;
+    for (int r = warp; r < LT_BM; r += LT_WARPS)
+        for (int ch = lane; ch < CHW; ch += 32) {
+            const bool valid = r < nrows && ch < CH;
+            lx_cp_async16(Qs_u + (uint32_t)(r * STR + ch * 8) * 2, qbase + (valid ? (size_t)r * D + ch * 8 : 0), valid);
+        }
+    __syncthreads();
+    for (int n = 0; n < STAGES - 1; ++n) copy_rows(n, n, n);
+
+    const uint32_t q_frag_u = Qs_u + (uint32_t)((((lane >> 3) & 1) * 8 + (lane & 7)) * STR + (lane >> 4) * 8) * 2;
+    const uint32_t p_frag_u = Ps_u + (uint32_t)((((lane >> 3) & 1) * 8 + (lane & 7)) * LT_PSTR + (lane >> 4) * 8) * 2;
+    const uint32_t k_frag = (uint32_t)(((lane >> 4) * 8 + (lane & 7)) * STR + ((lane >> 3) & 1) * 8) * 2;
+    float o[DT][4];
+#pragma unroll
+    for (int d = 0; d < DT; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
+    // TPR threads make a row's probabilities, KPT keys each
+    constexpr int TPR = LT_WARPS * 32 / LT_BM, KPT = LT_BN / TPR;
+    static_assert(KPT == 2, "two keys a thread");
+    const int srow = tid / TPR, skey = tid % TPR * KPT;
+    const int qpos = srow < nrows ? pos_first + (row0 + srow) / H : -1, wlo = window > 0 ? qpos - window + 1 : 0;
+    float m_run = -INFINITY, l_run = 0.f;
+
+    for (int n = 0, stage = 0, turn = 0; n < blocks; ++n) {                // block n lies in stage n % STAGES, its places in key_row[n % TURNS]
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                                                   // the block (and, first time, Q) has landed; everyone is done with the one before
+        const int before = turn == 0 ? TURNS - 1 : turn - 1;
+        copy_rows(n + STAGES - 1, before == 0 ? TURNS - 1 : before - 1, stage == 0 ? STAGES - 1 : stage - 1);
+        place(n + STAGES, before, page);                                   // the page was asked for an iteration ago
+        page = page_of(n + STAGES + 1);
+        const uint32_t Ks_u = Ks0_u + (uint32_t)(stage * LT_BN * STR) * 2;
+
+        float sc[LT_BN / 8][4];
+#pragma unroll
+        for (int j = 0; j < LT_BN / 8; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
+        auto score = [&](int kk) {
+            uint32_t a0, a1, a2, a3;
+            lx_ldmatrix_x4(q_frag_u + kk * 32, a0, a1, a2, a3);
+#pragma unroll
+            for (int j = 0; j < LT_BN / 8; j += 2) {
+                uint32_t b0, b1, b2, b3;
+                lx_ldmatrix_x4(Ks_u + k_frag + (uint32_t)(j * 8 * STR) * 2 + kk * 32, b0, b1, b2, b3);
+                lx_mma(sc[j], a0, a1, a2, a3, b0, b1);
+                lx_mma(sc[j + 1], a0, a1, a2, a3, b2, b3);
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < R / 16 / LT_WARPS; ++i) score(warp + i * LT_WARPS);       // rows are R numbers wide at least, zeros behind their own
+        for (int kk = R / 16 + warp; kk < KS; kk += LT_WARPS) score(kk);
+        float* part = parts + warp * LT_BM * LT_SSTR + g * LT_SSTR + 2 * c;
+#pragma unroll
+        for (int j = 0; j < LT_BN / 8; ++j) {
+            *reinterpret_cast<float2*>(part + j * 8) = make_float2(sc[j][0], sc[j][1]);
+            *reinterpret_cast<float2*>(part + 8 * LT_SSTR + j * 8) = make_float2(sc[j][2], sc[j][3]);
+        }
+        __syncthreads();                                                   // every warp's part of the scores is there
+        {
+            float z[KPT] = {0.f, 0.f}, mx = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < LT_WARPS; ++w) {
+                const float2 v = *reinterpret_cast<const float2*>(parts + (w * LT_BM + srow) * LT_SSTR + skey);
+                z[0] += v.x; z[1] += v.y;
+            }
+#pragma unroll
+            for (int e = 0; e < KPT; ++e) {
+                const int key = (kb0 + n * ksplit) * LT_BN + skey + e;
+                const bool ok = key_row[turn][skey + e] >= 0 && key <= qpos && key >= wlo;
+                z[e] = ok ? z[e] * scale_log2e : -INFINITY;                // scores in log2 units
+                mx = fmaxf(mx, z[e]);
+            }
+#pragma unroll
+            for (int x = 1; x < TPR; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+            const float mn = fmaxf(m_run, mx), base = mn == -INFINITY ? 0.f : mn;
+            const float corr = m_run == -INFINITY ? 0.f : exp2f(m_run - mn);
+            const float p0 = exp2f(z[0] - base), p1 = exp2f(z[1] - base);  // exp2(-inf) = 0 for masked keys
+            l_run = l_run * corr + (p0 + p1);
+            m_run = mn;
+            *reinterpret_cast<uint32_t*>(Ps + srow * LT_PSTR + skey) = lx_pack(p0, p1);
+            if (tid % TPR == 0) corrs[srow] = corr;
+        }
+        __syncthreads();                                                   // the probabilities are there
+        const float corr0 = corrs[g], corr1 = corrs[g + 8];
+        if (__any_sync(0xffffffffu, corr0 != 1.f || corr1 != 1.f)) {
+#pragma unroll
+            for (int d = 0; d < DT; ++d) { o[d][0] *= corr0; o[d][1] *= corr0; o[d][2] *= corr1; o[d][3] *= corr1; }
+        }
+#pragma unroll
+        for (int ks = 0; ks < LT_BN / 16; ++ks) {
+            uint32_t a0, a1, a2, a3;
+            lx_ldmatrix_x4(p_frag_u + ks * 32, a0, a1, a2, a3);
+#pragma unroll
+            for (int d = 0; d < DT; d += 2) {
+                const int row = ks * 16 + (lane & 15), col = warp * CHP + (d + (lane >> 4)) * 8;
+                uint32_t b0, b1, b2, b3;
+                lx_ldmatrix_x4_trans(Ks_u + (uint32_t)(row * STR + col) * 2, b0, b1, b2, b3);
+                lx_mma(o[d], a0, a1, a2, a3, b0, b1);
+                lx_mma(o[d + 1], a0, a1, a2, a3, b2, b3);
+            }
+        }
+        stage = stage + 1 == STAGES ? 0 : stage + 1;
+        turn = turn + 1 == TURNS ? 0 : turn + 1;
+    }
+    lx_cp_async_wait_all();                                                // nothing is left on its way, even where this CTA had no block
+#pragma unroll
+    for (int x = 1; x < TPR; x <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, x);
+    if (tid % TPR == 0) {
+        tops[srow] = m_run;
+        sums[srow] = l_run;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = g + 8 * r;
+        if (row >= nrows) continue;
+        float m = tops[row], l = sums[row], f = 1.f;
+        if (ksplit > 1) {
+            // this CTA saw only some of the key blocks: its maximum, its sum and its unnormalised weighted sum go to the scratch, and a
+            // second launch combines the CTAs of a row
+            const size_t slot = ((size_t)(single_only ? unit : qs) * H + row0 + row) * ksplit + blockIdx.y;
+            if (warp == 0 && c == 0) {
+                part_ml[slot * 2] = m;
+                part_ml[slot * 2 + 1] = l;
+            }
+            float* dst = part_o + slot * r_lat + warp * CHP;
+#pragma unroll
+            for (int d = 0; d < DT; ++d)
+                if (warp * CHP + d * 8 < r_lat) *reinterpret_cast<float2*>(dst + d * 8 + 2 * c) = make_float2(o[d][2 * r], o[d][2 * r + 1]);
+            continue;
+        }
+        if (sinks != nullptr) {                                            // the sink joins the denominator once (log2 units like the scores)
+            const float sk = sinks[(row0 + row) % H] * 1.4426950408889634f, mn = fmaxf(m, sk);
+            f = m == -INFINITY ? 0.f : exp2f(m - mn);
+            l = l * f + exp2f(sk - mn);
+        }
+        const float inv = l > 0.f ? f / l : 0.f;
+        __nv_bfloat16* dst = out + ((size_t)qs * H + row0 + row) * r_lat + warp * CHP;
+#pragma unroll
+        for (int d = 0; d < DT; ++d)
+            if (warp * CHP + d * 8 < r_lat) *reinterpret_cast<uint32_t*>(dst + d * 8 + 2 * c) = lx_pack(o[d][2 * r] * inv, o[d][2 * r + 1] * inv);
+    }
+}
+
 // out[row] = sum_s 2^(m_s - M) o_s / (sum_s 2^(m_s - M) l_s + 2^(sink - M)), M = max over the row's parts and the sink.
 // One CTA per (token, head) row; tokens (may be null): the tokens served.  The weights of the parts are made once, in shared
 // memory; the sums run over the parts in order, eight requested at a time.
@@ -386,21 +593,32 @@ latent_attention_merge_kernel(int R, const float* __restrict__ part_o, const flo
     }
 }
 
-template <int R, int SLABS, int WARPS>
+template <int R, bool SMALL>
 static int launch_latent_tc(const void* q, const void* cache, const int* bt, int max_blocks, const int* q_start, const int* positions,
                             int T, int S, void* out, int H, int r_lat, int rd, int page_size, int window, float scale, const float* sinks,
                             int ksplit, float* part_o, float* part_ml, const int* tokens, int num_tokens, cudaStream_t stream) {
     const int D = r_lat + rd;
-    constexpr int BM = SLABS * 16;
-    const size_t smem = (size_t)(BM + LxBlock<SLABS>::STAGES * LxBlock<SLABS>::BN) * (lx_row_width(R, D) + 8) * 2 + (size_t)BM * LxBlock<SLABS>::PSTR * 2 + (size_t)WARPS * 16 * sizeof(float);
+    constexpr int BM = SMALL ? LT_BM : LX_BM, THREADS = 32 * (SMALL ? LT_WARPS : LX_WARPS);
+    size_t smem;
+    if (SMALL) smem = lt_smem<R>(D);
+    else smem = (size_t)(LX_BM + LX_BN) * (lx_row_width(R, D) + 8) * 2 + (size_t)LX_BM * LX_PSTR * 2 + (size_t)LX_WARPS * 16 * sizeof(float);
     if (smem > 227 * 1024) return AIEN_E_SHAPE;
-    auto kern = latent_attention_tc_kernel<R, SLABS, WARPS>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return AIEN_E_STATE;
     // tokens: only these, each a request's one token of the step
     const long tiles = tokens != nullptr || T == S ? (long)(tokens != nullptr ? num_tokens : T) * ((H + BM - 1) / BM) : ((long)T * H) / BM + S;
-    kern<<<dim3((unsigned)tiles, ksplit), WARPS * 32, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start,
-                                                                     positions, S, (__nv_bfloat16*)out, H, r_lat, rd, page_size, window,
-                                                                     scale * 1.4426950408889634f, sinks, ksplit, part_o, part_ml, tokens != nullptr ? 1 : 0);
+    const int single_only = tokens != nullptr ? 1 : 0;
+    const dim3 grid((unsigned)tiles, ksplit);
+    const float scale2 = scale * 1.4426950408889634f;
+    if constexpr (SMALL) {
+        auto kern = latent_token_kernel<R>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return AIEN_E_STATE;
+        kern<<<grid, THREADS, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start, positions, S, (__nv_bfloat16*)out,
+                                              H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
+    } else {
+        auto kern = latent_attention_tc_kernel<R>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return AIEN_E_STATE;
+        kern<<<grid, THREADS, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start, positions, S, (__nv_bfloat16*)out,
+                                              H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
+    }
     if (ksplit > 1)
         latent_attention_merge_kernel<<<dim3((unsigned)((long)(tokens != nullptr ? num_tokens : T) * H)), 128, 0, stream>>>(
             r_lat, part_o, part_ml, ksplit, sinks, H, (__nv_bfloat16*)out, tokens);
@@ -572,7 +790,7 @@ static int lx_padded_rank(int kv_rank) { return kv_rank <= 64 ? 64 : (kv_rank <=
 
 AIEN_API int aien_latent_attention_tc_supports(int kv_rank, int rot_dim) {
     if (kv_rank <= 0 || kv_rank > 512 || (kv_rank & 7) || rot_dim < 0 || (rot_dim & 7)) return 0;
-    const size_t smem = (size_t)(LX_BM + LX_BN) * (lx_row_width(lx_padded_rank(kv_rank), kv_rank + rot_dim) + 8) * 2 + (size_t)LX_BM * LxBlock<4>::PSTR * 2 + 16 * 16 * sizeof(float);
+    const size_t smem = (size_t)(LX_BM + LX_BN) * (lx_row_width(lx_padded_rank(kv_rank), kv_rank + rot_dim) + 8) * 2 + (size_t)LX_BM * LX_PSTR * 2 + LX_WARPS * 16 * sizeof(float);
     return smem <= 227 * 1024 ? 1 : 0;
 }
 
@@ -591,14 +809,14 @@ AIEN_API int aien_latent_attention_tc(const void* q, const void* cache, const in
     if (((uintptr_t)q & 15) || ((uintptr_t)cache & 15) || ((uintptr_t)out & 3)) return AIEN_E_ALIGN;
     if (ksplit < 1 || ksplit > LX_MAX_SPLIT || num_tokens < 0 || (tokens != nullptr && num_tokens == 0) || (ksplit > 1 && (part_o == nullptr || part_ml == nullptr || ((uintptr_t)part_o & 7)))) return AIEN_E_SHAPE;
     const int padded = lx_padded_rank(kv_rank);
-#define LX_CASE(RV, SL)                                                                                                          \
+#define LX_CASE(RV, SMALL)                                                                                                       \
     if (padded == RV)                                                                                                            \
-        return launch_latent_tc<RV, SL, (SL == 4 ? 16 : 4)>(q, cache, block_table, max_blocks, q_start, positions, T, S, out, H, kv_rank, rot_dim, page_size,  \
-                                        window, scale, sinks, ksplit, part_o, part_ml, tokens, num_tokens, stream);
+        return launch_latent_tc<RV, SMALL>(q, cache, block_table, max_blocks, q_start, positions, T, S, out, H, kv_rank, rot_dim, page_size,  \
+                                           window, scale, sinks, ksplit, part_o, part_ml, tokens, num_tokens, stream);
     if (small_tiles && padded >= 128) {                    // tiles of 16 rows: a latent of 64 would leave a warp half a pair of n8 tiles
-        LX_CASE(128, 1) LX_CASE(256, 1) LX_CASE(512, 1)
+        LX_CASE(128, true) LX_CASE(256, true) LX_CASE(512, true)
     }
-    LX_CASE(64, 4) LX_CASE(128, 4) LX_CASE(256, 4) LX_CASE(512, 4)
+    LX_CASE(64, false) LX_CASE(128, false) LX_CASE(256, false) LX_CASE(512, false)
 #undef LX_CASE
     return AIEN_E_SHAPE;
 }

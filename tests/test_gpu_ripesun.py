@@ -391,6 +391,43 @@ def test_latent_attention_sees_its_window_and_the_sink(dtype, impl, window, page
     H.assert_close(out.float().cpu().numpy().reshape(len(qpos), heads, r), want, 1e-5 if dtype == torch.float32 else 1.5e-2, "weighted latents")
 
 
+@pytest.mark.parametrize("heads,r,rd,page,window,ksplit", [(16, 512, 0, 16, 0, 1), (16, 512, 64, 16, 0, 3), (33, 512, 8, 24, 100, 2), (5, 256, 0, 8, 0, 4), (16, 200, 24, 24, 0, 1),
+                                                            (16, 128, 72, 32, 40, 1), (17, 104, 0, 16, 0, 9)])
+def test_latent_attention_of_single_tokens(heads, r, rd, page, window, ksplit):
+    """Contexts from one key to more blocks of 32 than the stages hold, borders of blocks and pages (of 24 tokens too), rows
+    wider and narrower than whole vectors, more CTAs a token than it has blocks, the step's tokens and a list of them."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(heads + r + page)
+    ctx, D, scale = [1, 31, 32, 33, 97, 300, 64, 161], r + rd, 0.1
+    pages = [(n + page - 1) // page for n in ctx]
+    order = torch.randperm(sum(pages), generator=g)
+    cache = torch.zeros(sum(pages) * page, D, dtype=torch.bfloat16)
+    bt, rows, at = torch.full((len(ctx), max(pages)), -1, dtype=torch.int32), [], 0
+    for s_, n in enumerate(ctx):
+        bt[s_, :pages[s_]] = order[at:at + pages[s_]].to(torch.int32)
+        at += pages[s_]
+        rows.append((torch.randn(n, D, generator=g) * 0.7).to(torch.bfloat16))
+        for j in range(n):
+            cache[int(bt[s_, j // page]) * page + j % page] = rows[-1][j]
+    T = len(ctx)
+    q = torch.randn(T, heads * D, generator=g).to(torch.bfloat16)
+    sinks = torch.randn(heads, generator=g)
+    want = np.zeros((T, heads, r))
+    for t, n in enumerate(ctx):
+        k = rows[t].double().numpy()[max(0, n - window) if window else 0:]
+        z = q[t].double().numpy().reshape(heads, D) @ k.T * scale
+        m = np.maximum(z.max(1), sinks.double().numpy())
+        e = np.exp(z - m[:, None])
+        want[t] = (e @ k[:, :r]) / (e.sum(1) + np.exp(sinks.double().numpy() - m))[:, None]
+    scratch = torch.full((K.latent_attention_tc_scratch(T, heads, r, ksplit) + 1,), float("nan")).cuda()
+    for tokens in (None, "listed"):
+        out = torch.full((T, heads * r), 9.0, dtype=torch.bfloat16).cuda()
+        starts = list(range(T + 1))
+        K.latent_attention_tc(q.cuda(), cache.cuda(), bt.cuda(), bt.shape[1], i32(starts), i32([n - 1 for n in ctx]), out, T, heads, r, rd, page, window, scale,
+                              sinks.cuda(), ksplit, scratch, True, None if tokens is None else i32(list(range(T))), 0 if tokens is None else T)
+        H.assert_close(out.float().cpu().numpy().reshape(T, heads, r), want, 1.5e-2, "weighted latents")
+
+
 # ------------------------------------------------------------------ whole models
 @pytest.mark.parametrize("which", list(CONFIGS))
 def test_layers_of_a_short_request_float32(models, which):
