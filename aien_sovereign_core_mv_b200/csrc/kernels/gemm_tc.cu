@@ -34,12 +34,26 @@ constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64;
 // stages of W, which is what a product with few rows waits for.
 // BN rows of W per tile: 128, or 96 where that spreads a product without split-K more evenly over
 // the SMs (tc_tile_cols).  Two CTAs share an SM in every case.
-template <int AR, int BN> struct TcT {
+// Z > 1: a cluster of Z CTAs shares a tile's K.  Each keeps 128 / Z columns of the result and gets the others' parts of
+// them in PARTS bytes behind the ring (which is smaller for that; with 128 rows of A a CTA has its SM to itself).
+template <int AR, int BN, int Z = 1> struct TcT {
     static constexpr int STAGE_A = AR * TC_BK * 2, STAGE_B = BN * TC_BK * 2;
-    static constexpr int STAGES = (100 * 1024) / (STAGE_A + STAGE_B);        // BN 128: 3 / 4 / 5 for AR 128 / 64 / 32
-    static constexpr int SMEM = STAGES * (STAGE_A + STAGE_B) + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int RING = Z == 1 ? 100 : AR == 32 ? 90 : AR == 64 ? 72 : 128;
+    static constexpr int STAGES = (RING * 1024) / (STAGE_A + STAGE_B);       // BN 128: 3 / 4 / 5 for AR 128 / 64 / 32; in a cluster 4 / 3 / 4
+    static constexpr int PARTS = (Z - 1) * (BN / Z) * AR * 4;
+    static constexpr int SMEM = STAGES * (STAGE_A + STAGE_B) + PARTS + 1024 /*align*/ + 256 /*barriers*/;
     static constexpr int TMEM_COLS = BN <= 64 ? 64 : 128;
 };
+
+// address of a rank's shared memory from the address of the same place in this CTA's
+__device__ __forceinline__ uint32_t tc_map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void tc_store_remote(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 
 __device__ __forceinline__ float tc_gelu_erf(float z) { return 0.5f * z * (1.0f + erff(z * 0.7071067811865476f)); }
 __device__ __forceinline__ float tc_relu2(float z) { return z > 0.f ? z * z : 0.f; }
@@ -118,16 +132,23 @@ __device__ __forceinline__ void tc_store_chunk(const uint32_t r_in[32], TC* __re
             }
 
 // EPI 0: store; EPI 1: silu(gate)*up over columns interleaved in runs of 8 (out has N/2 columns)
-template <int EPI, typename TC, int AR, int BN>
+// Z > 1: blockIdx.z is the CTA's rank in a cluster that shares the tile's K.  A product of few rows over a long K whose consumer
+// takes no partial products is a chain of k-blocks in a few CTAs (64 x 4,384 x 2,048: 46 tiles of 96 columns, 14.7 us, of which
+// half is the 32 k-blocks; tiles of 32 columns take as long: what a CTA waits for is its ring's way through memory, block after
+// block).  In a cluster each CTA takes a quarter of them (or half), sends the others their columns of its sums through
+// distributed shared memory, adds up its own columns' parts in the order of K and stores them.
+template <int EPI, typename TC, int AR, int BN, int Z = 1>
 __global__ void __launch_bounds__(192)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                TC* __restrict__ out, long ldc, size_t part_stride, int kb_per_split, int M, int N, int K) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    constexpr int TC_STAGES = TcT<AR, BN>::STAGES, TC_STAGE_A = TcT<AR, BN>::STAGE_A, TC_STAGE_B = TcT<AR, BN>::STAGE_B;
+    using C = TcT<AR, BN, Z>;
+    constexpr int TC_STAGES = C::STAGES, TC_STAGE_A = C::STAGE_A, TC_STAGE_B = C::STAGE_B;
     constexpr int TC_BN = BN;
     const uint32_t sA = base, sB = base + TC_STAGES * TC_STAGE_A;
-    const uint32_t bars = sB + TC_STAGES * TC_STAGE_B;     // full[], empty[], tmem_full, then the tmem slot
+    const uint32_t parts = sB + TC_STAGES * TC_STAGE_B;    // Z > 1: [rank][column / 4][row][4]
+    const uint32_t bars = parts + C::PARTS;                // full[], empty[], tmem_full, then the tmem slot
     const uint32_t full0 = bars, empty0 = bars + 8 * TC_STAGES, tmem_full = bars + 16 * TC_STAGES;
     const uint32_t tmem_slot = tmem_full + 8;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -137,9 +158,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * TC_BN;
     // blockIdx.z: a range of k-blocks (split-K for small M); the partial product goes to
     // out + z * part_stride and the consumer adds the ranges in order
-    const int kb_first = blockIdx.z * kb_per_split;
-    const int num_kb = min((K + TC_BK - 1) / TC_BK - kb_first, kb_per_split);
-    out += (size_t)blockIdx.z * part_stride;
+    const int total_kb = (K + TC_BK - 1) / TC_BK, rank = blockIdx.z;
+    const int kb_first = Z > 1 ? total_kb * rank / Z : rank * kb_per_split;
+    const int num_kb = Z > 1 ? total_kb * (rank + 1) / Z - kb_first : min(total_kb - kb_first, kb_per_split);
+    if (Z == 1) out += (size_t)rank * part_stride;
 
     griddep_launch();
     if (threadIdx.x == 0) {
@@ -148,13 +170,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)TcT<AR, BN>::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)C::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_acc = *tmem_slot_ptr;
+    if (Z > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this CTA runs: its shared memory may be written
 
     if (warp == 0) {
         if (lane == 0) {
@@ -193,6 +216,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             umma_commit(tmem_full);
         }
+    } else if (Z > 1) {
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        mbar_wait(tmem_full, 0, 3);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");               // (of the arrival above; the other warps below)
+        constexpr int CW = BN / Z;
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN && m0 + quarter * 32 < M && row < AR; c0 += 32) {        // a quarter beyond M has nothing to send
+            const int owner = c0 / CW;
+            if (owner == rank) continue;
+            uint32_t r[32];
+            tmem_ld32(tmem_acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int from = rank < owner ? rank : rank - 1;
+            const uint32_t to = tc_map_rank(parts + (uint32_t)(((from * CW + c0 % CW) / 4 * AR + row) * 16), owner);
+#pragma unroll
+            for (int v = 0; v < 8; ++v) tc_store_remote(to + (uint32_t)(v * AR * 16), r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+        }
     } else {
         const int quarter = warp & 3;                    // tensor-memory lanes 32*quarter .. +31
         mbar_wait(tmem_full, 0, 3);
@@ -207,11 +249,50 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
         }
     }
+    if (Z > 1) {
+        // everyone's parts are there (the last access to another CTA's shared memory is behind this, so a CTA may leave afterwards)
+        __syncwarp();
+        if (warp < 2) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        constexpr int CW = BN / Z;
+        if (warp >= 2 && m0 + quarter * 32 < M && quarter * 32 < AR) {
+#pragma unroll 1
+            for (int c0 = 0; c0 < CW; c0 += 32) {
+                uint32_t own[32];
+                float acc[32];
+                tmem_ld32(tmem_acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(rank * CW + c0), own);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+#pragma unroll
+                for (int z = 0; z < Z; ++z) {
+                    if (z == rank) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) acc[j] += __uint_as_float(own[j]);
+                        continue;
+                    }
+                    const int from = z < rank ? z : z - 1;
+                    const uint32_t at = parts + (uint32_t)(((from * CW + c0) / 4 * AR + row) * 16);
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) {
+                        float4 p;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(at + (uint32_t)(v * AR * 16)));
+                        acc[4 * v] += p.x; acc[4 * v + 1] += p.y; acc[4 * v + 2] += p.z; acc[4 * v + 3] += p.w;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) own[j] = __float_as_uint(acc[j]);
+                if (m0 + row < M) tc_store_chunk<EPI, TC>(own, out, ldc, m0 + row, n0, rank * CW + c0, N);
+            }
+        }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)TcT<AR, BN>::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)C::TMEM_COLS) : "memory");
     }
 }
 
@@ -995,6 +1076,46 @@ static int tc_tile_cols(int M, int N, int splits) {
     return ((t96 + sms - 1) / sms) * 96 < ((t128 + sms - 1) / sms) * 128 ? 96 : 128;
 }
 
+// How many CTAs of a cluster share a tile's K (1: no cluster): four, or two, where the tiles of 128 columns leave that many CTAs
+// room at once (two on an SM; with 128 rows of A one) and each gets four k-blocks.  Only without split-K.  B200, us, one CTA a
+// tile and shared: 64 x 4,384 x 2,048 14.3 and 11.0 (the same with bfloat16 results and 4,608 columns 14.0 and 10.1), 64 x 8,192 x 2,048
+// 15.0 and 12.2, 9 x 17 x 2,048 13.2 and 7.0, 9 x 2,048 x 2,048 with silu(gate)*up 17.8 and 11.3, 40 x 1,536 x 2,048 with gelu 17.2
+// and 9.3, 2,048 x 64 x 2,048 16.0 and 9.8.  Shorter chains of sums are nearer to 64 bits too (2.1e-6 -> 0.5e-6 over K = 2,048).
+static int tc_cluster(int M, int N, int K, int splits) {
+    if (splits != 1) return 1;
+    const long tiles = (long)((M + TC_BM - 1) / TC_BM) * ((N + TC_BN - 1) / TC_BN), room = (M > 64 ? 1 : 2) * (long)tc_num_sms();
+    const int kb = (K + TC_BK - 1) / TC_BK;
+    for (const int z : {4, 2})
+        if (tiles * z <= room && kb >= 4 * z) return z;
+    return 1;
+}
+
+template <int EPI, typename TC, int AR, int Z>
+static int launch_tc_cluster(const CUtensorMap& ma, const CUtensorMap& mw, void* out, long ldc, int M, int N, int K, cudaStream_t stream) {
+    auto kern = gemm_tc_kernel<EPI, TC, AR, TC_BN, Z>;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TcT<AR, TC_BN, Z>::SMEM) != cudaSuccess) return AIEN_E_STATE;
+        configured = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((M + TC_BM - 1) / TC_BM, (N + TC_BN - 1) / TC_BN, Z);
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = TcT<AR, TC_BN, Z>::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = Z;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kern, ma, mw, (TC*)out, ldc, (size_t)0, 0, M, N, K);
+    return launch_status();
+}
+
 template <int EPI, typename TC, int AR, int BN>
 static int launch_tc_rows(const CUtensorMap& ma, const CUtensorMap& mw, void* out, long ldc, int splits, size_t part_stride,
                           int M, int N, int K, cudaStream_t stream) {
@@ -1015,11 +1136,15 @@ static int launch_tc_rows(const CUtensorMap& ma, const CUtensorMap& mw, void* ou
 template <int EPI, typename TC>
 static int launch_tc(const void* A, long lda, const void* W, long ldw, void* out, long ldc, int splits, size_t part_stride,
                      int M, int N, int K, cudaStream_t stream) {
-    const int ar = tc_a_rows(M), bn = tc_tile_cols(M, N, splits);
+    const int ar = tc_a_rows(M), z = tc_cluster(M, N, K, splits), bn = z > 1 ? TC_BN : tc_tile_cols(M, N, splits);
     CUtensorMap ma, mw;
     if (!make_map(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, TC_BK, (uint32_t)ar) ||
         !make_map(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, TC_BK, (uint32_t)bn))
         return AIEN_E_STATE;
+#define TC_CLUSTER_CASE(ARV, ZV) if (ar == ARV && z == ZV) return launch_tc_cluster<EPI, TC, ARV, ZV>(ma, mw, out, ldc, M, N, K, stream)
+    TC_CLUSTER_CASE(32, 4); TC_CLUSTER_CASE(64, 4); TC_CLUSTER_CASE(128, 4);
+    TC_CLUSTER_CASE(32, 2); TC_CLUSTER_CASE(64, 2); TC_CLUSTER_CASE(128, 2);
+#undef TC_CLUSTER_CASE
     if (bn == 96) {
         if (ar == 32) return launch_tc_rows<EPI, TC, 32, 96>(ma, mw, out, ldc, splits, part_stride, M, N, K, stream);
         return launch_tc_rows<EPI, TC, 64, 96>(ma, mw, out, ldc, splits, part_stride, M, N, K, stream);

@@ -664,6 +664,36 @@ def test_gemm_tensor_core(K, out_dtype, M, N, K_):
     assert (out_full[:, N:] == 9.0).all()                    # nothing written beyond N
 
 
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K_", [(1, 17, 1024), (31, 96, 4104), (33, 130, 1030 // 8 * 8), (64, 4384, 2048), (65, 1000, 520), (32, 9472, 1024), (64, 9488, 1024),
+                                    (128, 4640, 1024), (300, 64, 1032), (129, 33, 512), (20, 128, 511 // 8 * 8)])
+def test_gemm_tensor_core_with_k_shared_in_a_cluster(K, M, N, K_, epilogue):
+    """Few tiles over a K of eight k-blocks or more: two or four CTAs share a tile's K (and the sizes next to the rule's edges,
+    where one takes it all): rows and columns that fill no tile, k-blocks that do not divide evenly, a K that is no multiple of
+    the k-block, several row tiles, every kind of epilogue."""
+    g = torch.Generator().manual_seed(M + N + K_)
+    N = N // 16 * 16 if epilogue == 1 else N
+    a = torch.randn(M, K_, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, K_, generator=g) / math.sqrt(K_)).to(torch.bfloat16).cuda()
+    cols = N // 2 if epilogue == 1 else N
+    z = a.double().cpu() @ w.double().cpu().T
+    if epilogue == 1:
+        z = z.view(M, N // 16, 2, 8)
+        z = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, cols)
+    for dtype, tol in ((torch.float32, 5e-6), (torch.bfloat16, 1e-2)):
+        if epilogue == 2 and dtype == torch.float32:
+            continue
+        out_full = torch.full((M, cols + 5), 9.0, dtype=dtype, device="cuda")
+        for _ in range(2):
+            K.gemm_tc(a, w, out_full[:, :cols], epilogue=epilogue)
+        torch.cuda.synchronize()
+        assert K.gemm_tc_error() == 0
+        want = torch.nn.functional.gelu(z) if epilogue == 2 else z
+        # sums of 4,104 products: the tensor cores cut 2^-24 off a sum 16 times a range; silu's exponential is good to 2^-21
+        H.assert_close(out_full[:, :cols].float().cpu().numpy(), want.numpy(), tol if epilogue != 1 else max(tol, 2e-5), f"tc gemm {M}x{N}x{K_}")
+        assert (out_full[:, cols:] == 9.0).all()
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K_", [(512, 18944, 2048), (4096, 4112, 1032), (2900, 5000, 1032)])      # tiles 256, 240 and 224 wide
 def test_gemm_tensor_core_tiles_of_256_rows(K, M, N, K_, out_dtype):
