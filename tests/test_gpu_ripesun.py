@@ -317,6 +317,38 @@ def test_latents_norms_rotation_and_cache_rows(dtype, q_rank, kv_rank, rot_dim):
         assert float(qf.reshape(T, heads, -1)[:, :, :kv_rank].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("dtype,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("q_rank,kv_rank,rot_dim,rot_dims,lead", [(2048, 1024, 64, 64, 0), (2052, 64, 4, 4, 0), (1028, 1028, 0, 0, 0), (0, 512, 300, 8, 4), (4, 4, 4, 2, 0), (1536, 512, 6, 6, 0),
+                                                                  (64, 64, 8, 8, 2), (1024, 0, 0, 0, 0)])
+def test_latents_in_whole_vectors(dtype, wdt, q_rank, kv_rank, rot_dim, rot_dims, lead):
+    """Ranks at and beyond what the vector form's threads hold, rotated parts longer than its idle threads and no multiples of
+    four, rows that start off the 16-byte boundary (``lead``), no query latent, no cache; the forms agree with 64 bits."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(q_rank + kv_rank)
+    T, eps, pos = 5, 1e-5, [0, 3, 64, 1000, 70001]
+    width = q_rank + kv_rank + rot_dim
+    d = torch.randn(T, lead + width + (-(lead + width)) % 4, generator=g).cuda()[:, lead:lead + width]
+    weight = lambda n: (torch.rand(n, generator=g) * 0.4 + 0.8).to(wdt).cuda() if n else None
+    wq, wkv = weight(q_rank), weight(kv_rank)
+    ang = np.asarray(pos, dtype=np.float64)[:, None] * np.array([777.0 ** (-2.0 * i / max(rot_dims, 1)) for i in range(rot_dims // 2)])[None]
+    cos, sin = (torch.tensor(f(ang), dtype=torch.float32).cuda() if rot_dims else None for f in (np.cos, np.sin))
+    slots = i32([3, -1, 0, 6, 5])
+    cache = torch.full((7, kv_rank + rot_dim), 9.0, dtype=dtype).cuda() if kv_rank else None
+    cq = torch.empty(T, q_rank, dtype=dtype).cuda() if q_rank else None
+    K.latent_prepare(d, q_rank, wq, eps, cq, q_rank, kv_rank, rot_dim, rot_dims, wkv, cos, sin, slots if kv_rank else None, cache)
+    dn, tol = d.double().cpu().numpy(), 3e-6 if dtype == torch.float32 else 8e-3
+    if q_rank:
+        H.assert_close(cq.float().cpu().numpy(), pr.rms_norm(dn[:, :q_rank], wq.double().cpu().numpy(), eps), tol, "query latent")
+    if kv_rank:
+        c, kr = pr.rms_norm(dn[:, q_rank:q_rank + kv_rank], wkv.double().cpu().numpy(), eps), dn[:, q_rank + kv_rank:].copy()
+        if rot_dims:
+            kr[:, :rot_dims] = pr.rotate_pairs(kr[:, :rot_dims], pos, 777.0, rot_dims)
+        for t, s in enumerate(slots.tolist()):
+            if s >= 0:
+                H.assert_close(cache[s].float().cpu().numpy(), np.concatenate([c[t], kr[t]]), tol, f"cache row of token {t}")
+        assert all((cache[s] == 9.0).all() for s in range(7) if s not in slots.tolist())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,n,k", [(5, 40, 24), (17, 128, 64), (1, 7, 3)])
 def test_one_product_per_head(dtype, heads, n, k):
