@@ -794,7 +794,7 @@ static int launch_tc_grouped_persistent(const void* A, long lda, int rows_a, con
 // run under the next tile's main loop (the producer does fill the ring meanwhile), and half as many
 // tiles to deal out; tc_plan chooses by the number of waves either way.  No ranges of K.
 template <int BNV> struct TcM {
-    static constexpr int BM = 256, BN = BNV;                                       // BN 256, or 240 / 224 where that makes fewer waves
+    static constexpr int BM = 256, BN = BNV;                                       // BN 256, or 240 / 224 / 192 where that makes fewer or shorter waves
     static constexpr int STAGE_A = BM * TC_BK * 2, STAGE_B = 256 * TC_BK * 2;      // 32 KB each (a narrower W tile leaves the rest unused)
     static constexpr int STAGES = 3;
     static constexpr int SMEM = STAGES * (STAGE_A + STAGE_B) + TC_STORE_BUFS * TC_STORE_BYTES + 1024 + 256;
@@ -900,7 +900,7 @@ gemm_tc_persistent_m256_kernel(const __grid_constant__ CUtensorMap map_a, const 
             mbar_wait(tfull, i & 1, 3);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + quarter * 32 + lane;
-            const int n_end = min(N, n0 + P::BN);                      // a tile of 240 or 224 columns ends inside its last chunk of 32
+            const int n_end = min(N, n0 + P::BN);                      // a tile of 240 columns ends inside its last chunk of 32
 #pragma unroll 1
             for (int c0 = 0; c0 < P::BN; c0 += 32) {
                 uint32_t r[32];
@@ -992,10 +992,11 @@ static int launch_tc_persistent_m256_bn(const void* A, long lda, const void* W, 
 template <int EPI, typename TC>
 static int launch_tc_persistent_m256(int bn, const void* A, long lda, const void* W, long ldw, void* out, long ldc, int M, int N, int K,
                                      cudaStream_t stream) {
-    if (sizeof(TC) == 2) {                       // the narrower tiles for bfloat16 results only (fewer kernels to compile)
-        if (bn == 240) return launch_tc_persistent_m256_bn<240, EPI, __nv_bfloat16>(A, lda, W, ldw, out, ldc, M, N, K, stream);
-        if (bn == 224) return launch_tc_persistent_m256_bn<224, EPI, __nv_bfloat16>(A, lda, W, ldw, out, ldc, M, N, K, stream);
-    }
+    if constexpr (sizeof(TC) == 2)
+        if (bn == 240) return launch_tc_persistent_m256_bn<240, EPI, TC>(A, lda, W, ldw, out, ldc, M, N, K, stream);
+    if (bn == 224) return launch_tc_persistent_m256_bn<224, EPI, TC>(A, lda, W, ldw, out, ldc, M, N, K, stream);
+    if constexpr (EPI == 0)                      // the narrowest for plain results only (fewer kernels to compile)
+        if (bn == 192) return launch_tc_persistent_m256_bn<192, EPI, TC>(A, lda, W, ldw, out, ldc, M, N, K, stream);
     return launch_tc_persistent_m256_bn<256, EPI, TC>(A, lda, W, ldw, out, ldc, M, N, K, stream);
 }
 
@@ -1019,11 +1020,14 @@ static int tc_plan(int M, int N, int ranges) {
 }
 
 // Whether a product that runs on the persistent kernel takes tiles of 256 rows instead of 128 x 256, and how
-// wide (256, 240 or 224 columns; 0: no): by the time either way, in cycles: waves of tiles x (k-blocks x
+// wide (256, 240, 224 or 192 columns; 0: no): by the time either way, in cycles: waves of tiles x (k-blocks x
 // the cycles shared memory needs for one + what of a tile's epilogue stays visible).  Per k-block the
 // 128 x 256 tile moves 96 KB through shared memory, 768 cycles at 128 bytes a cycle (756 measured); the
-// 256 x BN tile (64 + 3 BN / 8) KB, 5 % more measured.  AIEN_B200_GEMM_TC=m256 | p256 pins it (m256: 256 wide).
-static int tc_m256_cols(int M, int N, int K, int ranges) {
+// 256 x BN tile (64 + 3 BN / 8) KB, 5 % more measured.  Float32 results leave in boxes of 32 columns, so not 240; 192 is built
+// for plain results (epilogue 0).  Float32, 256 columns and this rule: 2,048 x 8,192 x 2,048 54.8 and 50.3 us (224), 700 x 8,192 x
+// 2,048 30.5 and 24.7 (192); bfloat16 2,048 x 3,072 x 1,536 26.3 (128 x 256) and 20.7 (192).  208 and 176 columns measured slower
+// than either neighbour.  AIEN_B200_GEMM_TC=m256 | p256 pins it (m256: 256 wide).
+static int tc_m256_cols(int M, int N, int K, int ranges, bool f32 = false, bool plain = true) {
     static int forced = -1;
     if (forced < 0) {
         const char* e = getenv("AIEN_B200_GEMM_TC");
@@ -1033,14 +1037,15 @@ static int tc_m256_cols(int M, int N, int K, int ranges) {
     if (forced == 1) return 256;
     if (M <= TC_BM) return 0;
     const long sms = tc_num_sms(), kb = (K + TC_BK - 1) / TC_BK;
-    const long t256 = (long)((M + 127) / 128) * ((N + 255) / 256);
+    const long t256 = (long)((M + 127) / 128) * ((N + 255) / 256), wide = (long)((M + 255) / 256) * ((N + 255) / 256);
     long best = ((t256 + sms - 1) / sms) * (kb * 768 + 700) * 97 / 100;
     int cols = 0;
-    for (int bn = 256; bn >= 224; bn -= 16) {
+    for (const int bn : {256, 240, 224, 192}) {
+        if ((bn == 240 && f32) || (bn == 192 && !plain)) continue;
         const long t = (long)((M + 255) / 256) * ((N + bn - 1) / bn), w = (t + sms - 1) / sms;
         // narrower tiles pay where they shorten several waves; in a single wave more, smaller CTAs measured no faster
-        // (2,048 x 4,096 x 4,096: 144 tiles of 240 columns 51.9 us, 128 of 256 49.8 us)
-        if (bn < 256 && w == 1) continue;
+        // (2,048 x 4,096 x 4,096: 144 tiles of 240 columns 51.9 us, 128 of 256 49.8 us) unless 256 leave a third of the SMs idle
+        if (bn < 256 && w == 1 && 3 * wide > 2 * sms) continue;
         const long c = w * (kb * (512 + 3 * bn) * 105 / 100 + 4500);
         if (c < best) { best = c; cols = bn; }
     }
@@ -1189,7 +1194,7 @@ AIEN_API int aien_gemm_tc(const void* A, long lda, const void* W, long ldw, void
     if (epilogue == 2 || epilogue == 3 || epilogue == 4 || epilogue == 6) {   // gelu (erf / tanh form) or relu squared of every value, bfloat16 out, K in one range
         if (c_dt != AIEN_DT_BF16 || splits != 1) return AIEN_E_SHAPE;
         const int plan = tc_plan(M, N, 1);
-        const int wide = plan == 256 ? tc_m256_cols(M, N, K, 1) : 0;
+        const int wide = plan == 256 ? tc_m256_cols(M, N, K, 1, false, false) : 0;
         if (epilogue == 2) {
             if (wide > 0) return launch_tc_persistent_m256<2, __nv_bfloat16>(wide, A, lda, W, ldw, out, ldc, M, N, K, stream);
             if (plan == 256) return launch_tc_persistent<256, 2, __nv_bfloat16>(A, lda, W, ldw, out, ldc, M, N, K, 1, 0, stream);
@@ -1212,7 +1217,7 @@ AIEN_API int aien_gemm_tc(const void* A, long lda, const void* W, long ldw, void
     if (epilogue == 0 || epilogue == 1) {
         const int plan = tc_plan(M, N, aien_gemm_tc_ranges(K, splits));
 #define TCP_CASE(BNV, EPIV, T) return launch_tc_persistent<BNV, EPIV, T>(A, lda, W, ldw, out, ldc, M, N, K, splits, part_stride, stream)
-        const int wide = plan == 256 ? tc_m256_cols(M, N, K, aien_gemm_tc_ranges(K, splits)) : 0;
+        const int wide = plan == 256 ? tc_m256_cols(M, N, K, aien_gemm_tc_ranges(K, splits), c_dt == AIEN_DT_F32, epilogue == 0) : 0;
         if (wide > 0) {
             if (epilogue == 0 && c_dt == AIEN_DT_BF16) return launch_tc_persistent_m256<0, __nv_bfloat16>(wide, A, lda, W, ldw, out, ldc, M, N, K, stream);
             if (epilogue == 0 && c_dt == AIEN_DT_F32) return launch_tc_persistent_m256<0, float>(wide, A, lda, W, ldw, out, ldc, M, N, K, stream);

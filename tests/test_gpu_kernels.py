@@ -715,6 +715,25 @@ def test_gemm_tensor_core_tiles_of_256_rows(K, M, N, K_, out_dtype):
     assert (out_full[:, N:] == 9.0).all()
 
 
+@pytest.mark.parametrize("M,N,K_", [(2000, 8168, 1032), (700, 8188, 1544), (2048, 3050, 712)])
+def test_gemm_tensor_core_widths_of_256_rows_float32(K, M, N, K_):
+    """Float32 results in tiles of 224 and 192 columns (boxes of 32 columns by TMA, and rows that are no whole 16-byte pieces by plain
+    stores), bfloat16 results in tiles of 192; ragged last tiles either way, two waves and one."""
+    assert K.gemm_tc_takes_256_rows(M, N, K_)
+    g = torch.Generator().manual_seed(M + N)
+    a = torch.randn(M, K_, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, K_, generator=g) / math.sqrt(K_)).to(torch.bfloat16).cuda()
+    want = (a.double() @ w.double().T).cpu().numpy()
+    for pad in (4, 5):
+        for dtype, tol in ((torch.float32, 2e-5), (torch.bfloat16, 1e-2)):
+            out_full = torch.full((M, N + pad), 9.0, dtype=dtype, device="cuda")
+            K.gemm_tc(a, w, out_full[:, :N])
+            torch.cuda.synchronize()
+            assert K.gemm_tc_error() == 0
+            H.assert_close(out_full[:, :N].float().cpu().numpy(), want, tol, f"{M}x{N}x{K_}")
+            assert (out_full[:, N:] == 9.0).all()
+
+
 def test_gemm_tensor_core_tiles_of_256_rows_with_swiglu(K):
     M, I, Hd = 2900, 2504, 1032                     # tiles of 224 columns over 5,008: the last one 80 wide
     assert K.gemm_tc_takes_256_rows(M, 2 * I, Hd)
