@@ -8,6 +8,7 @@
 //                index.  One warp per token.  On request it also counts the choices per expert.
 //   plan_rows, place_rows   every expert's (token, choice) pairs in a run of rows of their own (see below)
 //   expert_rows_bf16        up and down products of a few tokens, bfloat16, a warp per four output rows
+//   expert_tiles            the same with an expert's matrix read once for all the pairs that chose it
 //   expert_up    act[t, c, :] = f(W_up[e(t,c)] h[t])             c < top, f = gelu (erf or tanh form)
 //   expert_down  part[c][t, :] = weight(t,c) * W_down[e(t,c)] act[t, c, :]   float32 parts, one per choice,
 //                which the consumer (the norm that takes the branch) adds in index order
@@ -398,6 +399,156 @@ moe_expert_rows_bf16_kernel(const __nv_bfloat16* __restrict__ x, long x_stride, 
     }
 }
 
+// The same results with every expert's matrix read once: a CTA has 16 rows of one expert's matrix and serves all pairs that chose
+// it, sixteen at a time (a token chooses an expert once, but choices without tensors of their own arrive as expert 0 with
+// weight zero), each of its four warps a quarter of the columns, on the tensor cores
+// (mma.sync.m16n8k16, rows of W on the left, pairs on the right; both sides' columns in the order in which 16-byte loads give them).
+// Sixteen products start from zero and are added to the sums by float32 additions, and the quarters are added in order: the
+// rounding of float32 multiply-adds.  A CTA finds its pairs in the list of choices and leaves where there are none; `early`: the first
+// columns of W are asked for before the kernel ahead has made the choices (where most experts are chosen).
+// What bounds moe_expert_rows_bf16_kernel is instructions: two a number of W and pair (9 tokens, 4 of 16 gated experts of 2,048 x
+// 1,024, 36 pairs: 33.6 and 31.6 us for the two products of 124 and 62 MB); 24 and 15 so.
+constexpr int ET_WARPS = 4, ET_PAIRS = 16, ET_LIST = 256;       // pairs at a time; most pairs of a step
+constexpr int ET_U = 2;                                         // k-steps of 64 whose loads are in flight together
+
+__device__ __forceinline__ void et_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] += d[e];
+}
+
+struct EtTile { uint4 w[2][2]; };                               // row g, row g + 8; columns 16 c .. 16 c + 7, .. + 15 of a k-step
+
+__device__ __forceinline__ void et_load(EtTile& t, const __nv_bfloat16* r0, const __nv_bfloat16* r1, int k, int K) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const bool in = k + 8 * p < K;
+        t.w[0][p] = in ? __ldg(reinterpret_cast<const uint4*>(r0 + k + 8 * p)) : make_uint4(0u, 0u, 0u, 0u);
+        t.w[1][p] = in ? __ldg(reinterpret_cast<const uint4*>(r1 + k + 8 * p)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+// MODE as for moe_expert_rows_bf16_kernel.  NT: eights of pairs.
+template <int NT>
+__device__ __forceinline__ void et_products(float (&acc)[NT][4], const EtTile& t, const __nv_bfloat16* const (&xr)[NT], int k, int K) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const bool in = xr[nt] != nullptr && k + 8 * p < K;
+            const uint4 x = in ? __ldcg(reinterpret_cast<const uint4*>(xr[nt] + k + 8 * p)) : make_uint4(0u, 0u, 0u, 0u);
+            et_mma(acc[nt], t.w[0][p].x, t.w[1][p].x, t.w[0][p].y, t.w[1][p].y, x.x, x.y);
+            et_mma(acc[nt], t.w[0][p].z, t.w[1][p].z, t.w[0][p].w, t.w[1][p].w, x.z, x.w);
+        }
+}
+
+template <int MODE, int NT>
+__device__ __forceinline__ void et_serve(const __nv_bfloat16* __restrict__ x, long x_stride, const __nv_bfloat16* r0, const __nv_bfloat16* r1, EtTile (&first)[ET_U],
+                                         bool early, const int* pairs, int count, const float* __restrict__ wts, void* __restrict__ out, float* red, int row0,
+                                         int T, int top, int N, int K, int act_kind, int s0, int s1) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const __nv_bfloat16* xr[NT];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const int i = nt * 8 + g;
+        xr[nt] = i < count ? x + (size_t)(MODE == 1 ? pairs[i] : pairs[i] / top) * x_stride : nullptr;
+    }
+    float acc[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+    for (int s = s0; s < s1; s += ET_U) {
+        EtTile t[ET_U];
+#pragma unroll
+        for (int u = 0; u < ET_U; ++u) {
+            if (early && s == s0) t[u] = first[u];
+            else et_load(t[u], r0, r1, s + u < s1 ? (s + u) * 64 + c * 16 : K, K);
+        }
+#pragma unroll
+        for (int u = 0; u < ET_U; ++u) et_products<NT>(acc, t[u], xr, s + u < s1 ? (s + u) * 64 + c * 16 : K, K);
+    }
+    // [quarter][nt][e][lane]: thread (warp e, lane) adds the four quarters of its value; silu(gate) * up wants e and e + 2
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) red[((warp * NT + nt) * 4 + e) * 32 + lane] = acc[nt][e];
+    __syncthreads();
+    auto total = [&](int nt, int e) {
+        float v = 0.f;
+#pragma unroll
+        for (int z = 0; z < ET_WARPS; ++z) v += red[((z * NT + nt) * 4 + e) * 32 + lane];
+        return v;
+    };
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        if (MODE == 2 && warp >= 2) break;
+        const int i = nt * 8 + 2 * c + (warp & 1);                             // the pair; rows g (e = 0, 1) and g + 8 (e = 2, 3)
+        if (i >= count) continue;
+        const int pair = pairs[i];
+        const float scale = wts != nullptr ? __ldcg(wts + pair) : 1.0f;
+        if (MODE == 2) {
+            const float gate = total(nt, warp) * scale, up = total(nt, warp + 2) * scale;
+            const int f = row0 / 2 + g;
+            if (f < N) reinterpret_cast<__nv_bfloat16*>(out)[(size_t)pair * N + f] = __float2bfloat16_rn(gate / (1.0f + expf(-gate)) * up);
+            continue;
+        }
+        const int n = row0 + g + (warp >= 2 ? 8 : 0);
+        if (n >= N) continue;
+        const float v = total(nt, warp) * scale;
+        if (MODE == 0) {
+            reinterpret_cast<__nv_bfloat16*>(out)[(size_t)pair * N + n] = __float2bfloat16_rn(act_apply(v, act_kind));
+        } else {
+            const int t = pair / top;
+            reinterpret_cast<float*>(out)[((size_t)(pair - t * top) * T + t) * N + n] = v;
+        }
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(ET_WARPS * 32)
+moe_expert_tiles_kernel(const __nv_bfloat16* __restrict__ x, long x_stride, const __nv_bfloat16* __restrict__ w, const int* __restrict__ ids,
+                        const float* __restrict__ wts, void* __restrict__ out, int T, int top, int N, int K, int act_kind, int early, int per) {
+    __shared__ int pairs[ET_LIST];
+    __shared__ int s_count;
+    __shared__ float red[2][ET_WARPS * 2 * 4 * 32];                            // of a tile and the one after it
+    griddep_launch();
+    const int e = blockIdx.y, P = T * top, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const int rows = MODE == 2 ? 2 * N : N, tiles = (rows + 15) / 16, tile0 = blockIdx.x * per, tile1 = tile0 + per < tiles ? tile0 + per : tiles;
+    const __nv_bfloat16* we = w + (size_t)e * rows * K;
+    // rows beyond the last are computed and not stored
+    auto row = [&](int tile, int r) { return we + (size_t)(tile * 16 + r < rows ? tile * 16 + r : 0) * K; };
+    const int steps = (K + 63) / 64, s0 = steps * warp / ET_WARPS, s1 = steps * (warp + 1) / ET_WARPS;
+    EtTile first[ET_U];
+    if (early) {
+#pragma unroll
+        for (int u = 0; u < ET_U; ++u) et_load(first[u], row(tile0, g), row(tile0, g + 8), s0 + u < s1 ? (s0 + u) * 64 + c * 16 : K, K);
+    }
+    griddep_wait();
+    if (warp == 0) {
+        int n = 0;
+        for (int base = 0; base < P; base += 32) {
+            const bool hit = base + lane < P && __ldcg(ids + base + lane) == e;
+            const uint32_t m = __ballot_sync(0xffffffffu, hit);
+            if (hit) pairs[n + __popc(m & ((1u << lane) - 1u))] = base + lane;
+            n += __popc(m);
+        }
+        if (lane == 0) s_count = n;
+    }
+    __syncthreads();
+    const int count = s_count;
+    if (count == 0) return;
+    int turn = 0;
+    for (int tile = tile0; tile < tile1; ++tile)
+        for (int p0 = 0; p0 < count; p0 += ET_PAIRS, turn ^= 1) {
+            const bool asked = early && tile == tile0 && p0 == 0;
+            const int n = count - p0 < ET_PAIRS ? count - p0 : ET_PAIRS;
+            if (n <= 8) et_serve<MODE, 1>(x, x_stride, row(tile, g), row(tile, g + 8), first, asked, pairs + p0, n, wts, out, red[turn], tile * 16, T, top, N, K, act_kind, s0, s1);
+            else et_serve<MODE, 2>(x, x_stride, row(tile, g), row(tile, g + 8), first, asked, pairs + p0, n, wts, out, red[turn], tile * 16, T, top, N, K, act_kind, s0, s1);
+        }
+}
+
 template <typename T>
 __global__ void act_rows_kernel(T* __restrict__ a, size_t n, int act_kind) {
     griddep_launch();
@@ -480,12 +631,36 @@ AIEN_API int aien_moe_place_rows(const void* h, long h_stride, const int* ids, c
 // same for gated experts (w [E, 2N, K], runs of `group` gate and up rows), in both wts (or null) multiplies the input; mode 1 =
 // down into float32 parts [top, T, N] (K = F) times wts (or null).  K a multiple of 8, 16-byte aligned rows.
 AIEN_API int aien_moe_expert_rows_bf16(int mode, const void* x, long x_stride, const void* w, const int* ids, const float* wts,
-                                       void* out, int T, int top, int N, int K, int act_kind, int group, cudaStream_t stream) {
+                                       void* out, int T, int top, int E, int N, int K, int act_kind, int group, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (N <= 0 || K <= 0 || (K & 7) || (x_stride & 7) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return AIEN_E_ALIGN;
     const int outs = 8 * (mode == 2 ? SV_ROWS / 2 : SV_ROWS);
     const int tiles = (N + outs - 1) / outs;
     if (tiles > 65535 || (long)T * top > 2147483647L || group < 0 || (group > 0 && N % group)) return AIEN_E_SHAPE;
+    // Every expert's matrix once for all its pairs where enough pairs share an expert, by the experts that T tokens reach on the
+    // average: 1.4 pairs an expert and more.  us, a row a pair and an expert's tile (up and down product): 16 gated experts of
+    // 2,048 x 1,024, 4 a token, 4 tokens (1.5 pairs) 21.5 and 21.2, 13.9 and 13.2; 9 (2.4) 33.0 and 24.5, 23.7 and 15.2; 16 49.7 and 26.5, 34.9
+    // and 15.7; 64 of 2,048 x 768, 6 a token, 4 tokens (1.2) 18.4 and 16.2, 16.6 and 19.7; 9 (1.4) 33.0 and 24.4, 28.2 and 28.1; 16 56.6 and
+    // 33.7, 44.4 and 38.9.  More experts than 64 (128, 8 a token, 16 tokens, 1.6 pairs: 85 and 87) cost their CTAs.
+    double missed = 1.0;
+    for (int t = 0; t < T && t <= ET_PAIRS; ++t) missed *= 1.0 - (double)(top < E ? top : E) / (E > 0 ? E : 1);
+    const double reached = (1.0 - missed) * E;
+    if (E > 0 && E <= 64 && T <= ET_PAIRS && T * top <= ET_LIST && (mode != 2 || group == 8) && (double)T * top >= 1.4 * reached) {
+        const int early = T * top >= 2 * E;          // most experts are chosen: a CTA need not wait for the choices to ask for its first rows
+        // A tile of a short K is over before its CTA has found its pairs, so a CTA takes two or four in turn while a thousand CTAs are left
+        // (64 experts, 9 tokens, K = 768: 34.9 us with one, 29.3 with two, 28.1 with four)
+        const long tiles16 = ((mode == 2 ? 2L * N : N) + 15) / 16;
+        const int per = K > 1024 || tiles16 * reached < 2048 ? 1 : tiles16 * reached < 4096 ? 2 : 4;
+        const dim3 tile_grid((unsigned)((tiles16 + per - 1) / per), E);
+#define ME_CASE(M)                                                                                                       \
+    launch_chain(moe_expert_tiles_kernel<M>, tile_grid, dim3(ET_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, x_stride, \
+                 (const __nv_bfloat16*)w, ids, wts, out, T, top, N, K, act_kind, early, per)
+        if (mode == 0) ME_CASE(0);
+        else if (mode == 2) ME_CASE(2);
+        else ME_CASE(1);
+#undef ME_CASE
+        return launch_status();
+    }
     dim3 grid(T * top, tiles);
 #define MR_CASE(M)                                                                                                       \
     launch_chain(moe_expert_rows_bf16_kernel<M>, grid, dim3(256), 0, stream, (const __nv_bfloat16*)x, x_stride,           \

@@ -500,8 +500,8 @@ def moe_experts(ctx, h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, 
     if ok and not grouped:
         act = ws.take((T * top, Fd), torch.bfloat16)
         _check(lib().aien_moe_expert_rows_bf16(2 if gated else 0, h, h.stride(0), w_up, ids, wts if on_input else None, act, T,
-                                               top, Fd, D, 0 if gated else int(act_kind), int(group), _stream()), "moe_expert_rows(up)")
-        _check(lib().aien_moe_expert_rows_bf16(1, act, Fd, w_down, ids, None if on_input else wts, parts, T, top, D, Fd,
+                                               top, E, Fd, D, 0 if gated else int(act_kind), int(group), _stream()), "moe_expert_rows(up)")
+        _check(lib().aien_moe_expert_rows_bf16(1, act, Fd, w_down, ids, None if on_input else wts, parts, T, top, E, D, Fd,
                                                0, 0, _stream()), "moe_expert_rows(down)")
         return parts
     if grouped:

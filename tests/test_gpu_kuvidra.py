@@ -375,6 +375,44 @@ def test_router_of_sigmoid_scores(E, top):
     H.assert_close(wts.cpu().numpy(), pk.sigmoid(np.take_along_axis(f64(z[:, :E]), ids.cpu().numpy().astype(np.int64), -1)), 1e-6, "weights")
 
 
+@pytest.mark.parametrize("E,top,T,D,F_", [(16, 4, 9, 2048, 1024), (5, 3, 16, 200, 24), (64, 6, 16, 512, 136), (8, 2, 5, 1032, 40), (3, 3, 16, 72, 8), (20, 16, 16, 64, 1024)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_experts_of_a_few_tokens_share_their_rows(E, top, T, D, F_, gated):
+    """Enough pairs an expert that its matrix is read once for all: rows and columns that fill no tile, one and several tiles a CTA,
+    more than sixteen pairs of one expert (choices that weigh nothing arrive as expert 0), with and without the first rows
+    asked for ahead, weights on the input and on the output."""
+    from types import SimpleNamespace
+    from aien_sovereign_core_mv_b200 import kernels as K
+    from aien_sovereign_core_mv_b200.parts import Workspace
+    g = torch.Generator().manual_seed(E + T + D)
+    bf = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)
+    h = bf(T, D)
+    up, gate, down = ((bf(E, *s).float() / s[-1] ** 0.5).to(torch.bfloat16) for s in ((F_, D), (F_, D), (D, F_)))
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    wts = torch.rand(T, top, generator=g) + 0.1
+    idle = torch.rand(T, top, generator=g) < 0.3
+    ids[idle], wts[idle] = 0, 0.0
+    w_up = torch.stack([gate.view(E, F_ // 8, 8, D), up.view(E, F_ // 8, 8, D)], dim=2).reshape(E, 2 * F_, D).contiguous() if gated else up
+    d = lambda t: t.double().numpy()
+    for on_input in (False, True):
+        ctx = SimpleNamespace(workspace=Workspace(4096, 64 << 20, torch.device("cuda")), dtype=torch.bfloat16)
+        ctx.workspace.begin_layer()
+        parts = K.moe_experts(ctx, h.cuda(), w_up.cuda(), down.cuda(), ids.cuda(), wts.cuda(), top, K.ACT_GATED if gated else 0, None, 8 if gated else 0, on_input)
+        assert tuple(parts.shape) == (top, T, D) and parts.dtype == torch.float32
+        for t in range(T):
+            for c in range(top):
+                e, w = int(ids[t, c]), float(wts[t, c])
+                x = d(h[t]) * (w if on_input else 1.0)
+                z = d(up[e]) @ x
+                if gated:
+                    y = d(gate[e]) @ x
+                    a = y / (1.0 + np.exp(-y)) * z
+                else:
+                    a = torch.nn.functional.gelu(torch.tensor(z)).numpy()
+                want = d(down[e]) @ a * (1.0 if on_input else w)
+                H.assert_close(parts[c, t].cpu().numpy(), want, 1.5e-2, f"token {t}, choice {c}")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("E,top,ff,shared", [(5, 3, 64, 72), (3, 1, 20, 0), (6, 6, 8, 40), (9, 2, 136, 24)])
 def test_gated_experts_with_the_weight_on_their_input(dtype, E, top, ff, shared):
