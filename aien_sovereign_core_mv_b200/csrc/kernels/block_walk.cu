@@ -130,6 +130,8 @@ block_coef_kernel(const BlockWalk a) {
     extern __shared__ __align__(16) float bw_smem[];
     __shared__ float dots[DELTA ? 2 : 1][BW_B * BW_B];                      // q_i . k_j and k_i . k_j
     const int slot = blockIdx.x, kvh = blockIdx.y;
+    griddep_launch();
+    griddep_wait();
     int lo = 0, hi = a.S - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) / 2;
@@ -176,8 +178,8 @@ block_coef_kernel(const BlockWalk a) {
         const int t = i / per, h = kvh * per + i - t * per;
         float g = 1.f, w = 0.f;
         if (t < n) {
-            g = a.gates != nullptr ? a.gates[(size_t)(t0 + t) * a.ldg + a.g_off + h] : a.decay[h];
-            w = a.w_off >= 0 ? a.gates[(size_t)(t0 + t) * a.ldg + a.w_off + h] : 1.f;
+            g = a.gates != nullptr ? ld_act(a.gates + (size_t)(t0 + t) * a.ldg + a.g_off + h) : a.decay[h];
+            w = a.w_off >= 0 ? ld_act(a.gates + (size_t)(t0 + t) * a.ldg + a.w_off + h) : 1.f;
         }
         sg[i] = g;
         sw[i] = w;
@@ -458,6 +460,8 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
     float* part_p = bw_smem + C::STAGES * C::STAGE;
     float* parts_r = part_p + (DELTA ? C::PART : 0);
     float* us = parts_r + C::TURNS * C::SUMS;
+    griddep_launch();
+    griddep_wait();
     const int s = bw_nth_longest(a.q_start, a.S, blockIdx.z), h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
     if (t1 <= t0 || (a.alone && t1 - t0 == 1)) return;
     const int tid = threadIdx.x & (BW_THREADS - 1), warp = tid >> 5, lane = tid & 31;
@@ -738,7 +742,7 @@ static int launch_block_walk(const BlockWalk& a, cudaStream_t stream) {
     constexpr int bytes = BwSmem<NT, MT, DELTA, HELP>::TOTAL * 4;
     auto kern = block_walk_kernel<NT, MT, DELTA, HELP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
-    kern<<<dim3((a.V + 16 * MT - 1) / (16 * MT), a.heads, a.S), (HELP ? 2 : 1) * BW_THREADS, bytes, stream>>>(a);
+    launch_chain(kern, dim3((a.V + 16 * MT - 1) / (16 * MT), a.heads, a.S), dim3((HELP ? 2 : 1) * BW_THREADS), (size_t)bytes, stream, a);
     return launch_status();
 }
 
@@ -787,7 +791,7 @@ AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, i
     const int per = heads / G, smem = 4 * (2 * BW_B * (N + 4) + 2 * BW_B * per + (delta ? 256 * per : 0));
     auto coef = delta ? block_coef_kernel<true> : block_coef_kernel<false>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(coef, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AIEN_E_STATE;
-    coef<<<dim3((unsigned)blocks, G), 256, smem, stream>>>(a);
+    launch_chain(coef, dim3((unsigned)blocks, G), dim3(256), (size_t)smem, stream, a);
     const int rc = launch_status();
     if (rc != 0) return rc;
     return N <= 64 ? dispatch_block_walk<1>(a, stream) : dispatch_block_walk<2>(a, stream);

@@ -318,6 +318,8 @@ __global__ void __launch_bounds__(256)
 grouped_gated_rmsnorm_vec_kernel(const float* __restrict__ o, long ldo, const TP* __restrict__ gate, long ldg, const void* __restrict__ w,
                                  int wdt, float eps, TO* __restrict__ out, long ldout, int T, int groups, int group, int act) {
     const size_t unit = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    griddep_launch();
+    griddep_wait();
     if (unit >= (size_t)T * groups) return;
     const int lane = threadIdx.x & 31;
     const size_t t = unit / groups;
@@ -404,8 +406,8 @@ AIEN_API int aien_grouped_gated_rmsnorm(const float* o, long ldo, const void* ga
                       reinterpret_cast<uintptr_t>(gate) % (g_dt == AIEN_DT_F32 ? 16 : 8) == 0 && reinterpret_cast<uintptr_t>(out) % (o_dt == AIEN_DT_F32 ? 16 : 8) == 0;
     if (four) {
         AIEN_DISPATCH_DTYPE(g_dt, TP, AIEN_DISPATCH_DTYPE(o_dt, TO,
-            (grouped_gated_rmsnorm_vec_kernel<TP, TO><<<blocks, 256, 0, stream>>>(o, ldo, (const TP*)gate, ldg, w, w_dt, eps, (TO*)out, ldout, T,
-                                                                                 groups, group, act))));
+            (launch_chain(grouped_gated_rmsnorm_vec_kernel<TP, TO>, dim3(blocks), dim3(256), (size_t)0, stream, o, ldo, (const TP*)gate, ldg, w, w_dt, eps, (TO*)out,
+                          ldout, T, groups, group, act))));
         return launch_status();
     }
     AIEN_DISPATCH_DTYPE(g_dt, TP, AIEN_DISPATCH_DTYPE(o_dt, TO,

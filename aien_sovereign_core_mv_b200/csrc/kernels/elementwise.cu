@@ -229,10 +229,12 @@ __global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ out, int
 __global__ void rope_table_kernel(const int* __restrict__ positions, const double* __restrict__ inv_freq,
                                   float* __restrict__ cos_t, float* __restrict__ sin_t, int T, int half, double mult) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    griddep_launch();
+    griddep_wait();
     if (idx >= T * half) return;
     const int t = idx / half, i = idx - t * half;
     double s, c;
-    sincos((double)positions[t] * inv_freq[i], &s, &c);
+    sincos((double)__ldcg(positions + t) * inv_freq[i], &s, &c);
     cos_t[idx] = (float)(c * mult);                   // mult: 1, or the factor that some frequency scalings put on both
     sin_t[idx] = (float)(s * mult);
 }
@@ -882,7 +884,7 @@ AIEN_API int aien_rope_table(const int* positions, const double* inv_freq, float
                              int T, int half, double mult, cudaStream_t stream) {
     if (T <= 0 || half <= 0) return 0;
     const int n = T * half;
-    rope_table_kernel<<<(n + 127) / 128, 128, 0, stream>>>(positions, inv_freq, cos_t, sin_t, T, half, mult);
+    launch_chain(rope_table_kernel, dim3((n + 127) / 128), dim3(128), (size_t)0, stream, positions, inv_freq, cos_t, sin_t, T, half, mult);
     return launch_status();
 }
 

@@ -23,6 +23,8 @@ __global__ void __launch_bounds__(GATED_ROWS_THREADS)
 gated_rows_kernel(const float* __restrict__ o, long ldo, const TG* __restrict__ gate, long ldg, const void* __restrict__ w, int wdt, float eps,
                   float mult, TO* __restrict__ out, long ldout, int part) {
     __shared__ float red[32];
+    griddep_launch();
+    griddep_wait();
     const size_t t = blockIdx.x;
     const int c0 = blockIdx.y * part;
     float v[NV][4], g[NV][4];
@@ -69,9 +71,9 @@ template <bool GATE_FIRST, typename TG, typename TO>
 inline void launch_gated_rows(const float* o, long ldo, const TG* gate, long ldg, const void* w, int wdt, float eps, float mult, TO* out, long ldout,
                               int rows, int parts, int part, cudaStream_t stream) {
     const dim3 grid(rows, parts);
-    if (part <= 1024) gated_rows_kernel<1, GATE_FIRST, TG, TO><<<grid, GATED_ROWS_THREADS, 0, stream>>>(o, ldo, gate, ldg, w, wdt, eps, mult, out, ldout, part);
-    else if (part <= 2048) gated_rows_kernel<2, GATE_FIRST, TG, TO><<<grid, GATED_ROWS_THREADS, 0, stream>>>(o, ldo, gate, ldg, w, wdt, eps, mult, out, ldout, part);
-    else gated_rows_kernel<4, GATE_FIRST, TG, TO><<<grid, GATED_ROWS_THREADS, 0, stream>>>(o, ldo, gate, ldg, w, wdt, eps, mult, out, ldout, part);
+    const auto kern = part <= 1024 ? gated_rows_kernel<1, GATE_FIRST, TG, TO> : part <= 2048 ? gated_rows_kernel<2, GATE_FIRST, TG, TO>
+                                                                                             : gated_rows_kernel<4, GATE_FIRST, TG, TO>;
+    launch_chain(kern, grid, dim3(GATED_ROWS_THREADS), (size_t)0, stream, o, ldo, gate, ldg, w, wdt, eps, mult, out, ldout, part);
 }
 
 }  // namespace aien

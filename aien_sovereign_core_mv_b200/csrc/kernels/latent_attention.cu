@@ -89,14 +89,16 @@ latent_prepare_vec_kernel(const float* __restrict__ d, long ld, int q_rank, LpWe
     __shared__ float red[2][8];
     const size_t t = blockIdx.x;
     const float* row = d + t * ld;
-    const int tid = threadIdx.x, at = tid * 4, slot = cache != nullptr ? slot_map[t] : -1;
+    griddep_launch();
+    griddep_wait();
+    const int tid = threadIdx.x, at = tid * 4, slot = cache != nullptr ? __ldcg(slot_map + t) : -1;
     float4 q[2], kv = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (at + 1024 * i < q_rank) q[i] = *reinterpret_cast<const float4*>(row + at + 1024 * i);
+        if (at + 1024 * i < q_rank) q[i] = ld_act4(row + at + 1024 * i);
     }
-    if (slot >= 0 && at < kv_rank) kv = *reinterpret_cast<const float4*>(row + kv_off + at);
+    if (slot >= 0 && at < kv_rank) kv = ld_act4(row + kv_off + at);
     const float sq = warp_sum(lp_square(q[0]) + lp_square(q[1])), sk = warp_sum(lp_square(kv));
     if ((tid & 31) == 0) {
         red[0][tid >> 5] = sq;
@@ -117,10 +119,10 @@ latent_prepare_vec_kernel(const float* __restrict__ d, long ld, int q_rank, LpWe
     if (at < kv_rank) lp_store(dst + at, lp_scaled(kv, 1.0f / sqrtf(sum[1] / (float)kv_rank + eps), lp_weights(wkv, at)));
     const int half = rot_dims >> 1;
     for (int i = 255 - tid; i < rot_dim; i += 256) {                           // the threads that the latent leaves idle first
-        float v = row[kv_off + kv_rank + i];
+        float v = ld_act(row + kv_off + kv_rank + i);
         if (i < rot_dims) {
             const int p = i >> 1;
-            const float c = cos_t[t * half + p], s = sin_t[t * half + p], other = row[kv_off + kv_rank + (i ^ 1)];
+            const float c = ld_act(cos_t + t * half + p), s = ld_act(sin_t + t * half + p), other = ld_act(row + kv_off + kv_rank + (i ^ 1));
             v = (i & 1) ? v * c + other * s : v * c - other * s;
         }
         dst[kv_rank + i] = from_f<TKV>(v);
@@ -136,13 +138,15 @@ __global__ void rotate_pairs_rows_kernel(const TQ* q, long ldq, long q_head, TO*
     const size_t t = blockIdx.x;
     const int half = rot_dims >> 1;
     const int pairs = (rot_dim + 1) >> 1;
+    griddep_launch();
+    griddep_wait();
     for (int idx = threadIdx.x; idx < H * pairs; idx += blockDim.x) {          // a thread owns a pair, so the rows may be turned where they lie
         const int h = idx / pairs, p = idx % pairs, i = 2 * p;
         const TQ* src = q + t * ldq + (size_t)h * q_head + i;
         TO* dst = out + t * ldo + (size_t)h * o_head + i;
         float a = to_f(src[0]), b = i + 1 < rot_dim ? to_f(src[1]) : 0.f;
         if (i < rot_dims) {
-            const float c = cos_t[t * half + p], s = sin_t[t * half + p], a0 = a;
+            const float c = ld_act(cos_t + t * half + p), s = ld_act(sin_t + t * half + p), a0 = a;
             a = a0 * c - b * s;
             b = b * c + a0 * s;
         }
@@ -394,8 +398,8 @@ AIEN_API int aien_latent_prepare(const void* d, int d_dt, long ld, int q_rank, c
         (cache == nullptr || (((kv_off | kv_rank | rot_dim) & 3) == 0 && at(cache, four_kv)))) {
         const int w4 = w_dt == AIEN_DT_F32 ? 16 : 8;
         AIEN_DISPATCH_DTYPE(cq_dt, TO, AIEN_DISPATCH_DTYPE(kv_dt, TKV,
-            (latent_prepare_vec_kernel<TO, TKV><<<T, 256, 0, stream>>>((const float*)d, ld, q_rank, LpWeights{wq, w_dt, at(wq, w4)}, eps, (TO*)cq, ldq, kv_off, kv_rank,
-                                                                      rot_dim, rot_dims, LpWeights{wkv, w_dt, at(wkv, w4)}, cos_t, sin_t, slot_map, (TKV*)cache))));
+            (launch_chain(latent_prepare_vec_kernel<TO, TKV>, dim3(T), dim3(256), (size_t)0, stream, (const float*)d, ld, q_rank, LpWeights{wq, w_dt, at(wq, w4)}, eps,
+                          (TO*)cq, ldq, kv_off, kv_rank, rot_dim, rot_dims, LpWeights{wkv, w_dt, at(wkv, w4)}, cos_t, sin_t, slot_map, (TKV*)cache))));
         return launch_status();
     }
     AIEN_DISPATCH_DTYPE(d_dt, TD, AIEN_DISPATCH_DTYPE(cq_dt, TO, AIEN_DISPATCH_DTYPE(kv_dt, TKV,
@@ -409,7 +413,8 @@ AIEN_API int aien_rotate_pairs_rows(const void* q, int q_dt, long ldq, long q_he
     if (T <= 0 || H <= 0 || rot_dim <= 0) return 0;
     if (rot_dims < 0 || rot_dims > rot_dim || (rot_dims & 1) || (rot_dims > 0 && (cos_t == nullptr || sin_t == nullptr))) return AIEN_E_SHAPE;
     AIEN_DISPATCH_DTYPE(q_dt, TQ, AIEN_DISPATCH_DTYPE(o_dt, TO,
-        (rotate_pairs_rows_kernel<TQ, TO><<<T, 128, 0, stream>>>((const TQ*)q, ldq, q_head, (TO*)out, ldo, o_head, H, rot_dim, rot_dims, cos_t, sin_t))));
+        (launch_chain(rotate_pairs_rows_kernel<TQ, TO>, dim3(T), dim3(128), (size_t)0, stream, (const TQ*)q, ldq, q_head, (TO*)out, ldo, o_head, H, rot_dim, rot_dims,
+                      cos_t, sin_t))));
     return launch_status();
 }
 

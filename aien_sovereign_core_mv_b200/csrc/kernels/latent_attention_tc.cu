@@ -71,6 +71,8 @@ latent_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
 
     // which request, which rows: the lanes count 32 requests' tiles at a time
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    griddep_launch();
+    griddep_wait();
     int s = -1, row0 = 0, unit = 0;                      // unit: how many served tokens come before a single one
     for (int base = 0, acc = 0; base < S; base += 32) {
         const int i = base + lane, n = i < S ? q_start[i + 1] - q_start[i] : 0;
@@ -345,6 +347,8 @@ latent_token_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
 
     // which request, which rows: the lanes count 32 requests' tiles at a time
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    griddep_launch();
+    griddep_wait();
     int s = -1, row0 = 0, unit = 0;                      // unit: how many served tokens come before a single one
     for (int base = 0, acc = 0; base < S; base += 32) {
         const int i = base + lane, n = i < S ? q_start[i + 1] - q_start[i] : 0;
@@ -558,18 +562,20 @@ latent_attention_merge_kernel(int R, const float* __restrict__ part_o, const flo
                               const float* __restrict__ sinks, int H, __nv_bfloat16* __restrict__ out, const int* __restrict__ tokens) {
     __shared__ float wt[LX_MAX_SPLIT];
     __shared__ float red[32];
+    griddep_launch();
+    griddep_wait();
     const int unit = blockIdx.x / H, h = blockIdx.x - unit * H;
     const size_t row = blockIdx.x, to = (size_t)(tokens != nullptr ? tokens[unit] : unit) * H + h;
     const float sk = sinks != nullptr ? sinks[h] * 1.4426950408889634f : -INFINITY;
     float M = sk;
-    for (int s = threadIdx.x; s < ksplit; s += 128) M = fmaxf(M, part_ml[(row * ksplit + s) * 2]);
+    for (int s = threadIdx.x; s < ksplit; s += 128) M = fmaxf(M, ld_act(part_ml + (row * ksplit + s) * 2));
     M = block_max(M, red);
     float den = 0.f;
     for (int s = threadIdx.x; s < ksplit; s += 128) {
-        const float m = part_ml[(row * ksplit + s) * 2];
+        const float m = ld_act(part_ml + (row * ksplit + s) * 2);
         const float w = m != -INFINITY ? exp2f(m - M) : 0.f;
         wt[s] = w;
-        den += w * part_ml[(row * ksplit + s) * 2 + 1];
+        den += w * ld_act(part_ml + (row * ksplit + s) * 2 + 1);
     }
     den = block_sum(den, red);                                             // its barriers also order the weights
     if (sinks != nullptr && M != -INFINITY) den += exp2f(sk - M);
@@ -581,7 +587,7 @@ latent_attention_merge_kernel(int R, const float* __restrict__ part_o, const flo
             float2 v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                v[u] = s0 + u < ksplit && wt[s0 + u] != 0.f ? *reinterpret_cast<const float2*>(src + (size_t)(s0 + u) * R) : make_float2(0.f, 0.f);
+                v[u] = s0 + u < ksplit && wt[s0 + u] != 0.f ? __ldcg(reinterpret_cast<const float2*>(src + (size_t)(s0 + u) * R)) : make_float2(0.f, 0.f);
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const float w = s0 + u < ksplit ? wt[s0 + u] : 0.f;
@@ -611,16 +617,16 @@ static int launch_latent_tc(const void* q, const void* cache, const int* bt, int
     if constexpr (SMALL) {
         auto kern = latent_token_kernel<R>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return AIEN_E_STATE;
-        kern<<<grid, THREADS, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start, positions, S, (__nv_bfloat16*)out,
-                                              H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
+        launch_chain(kern, grid, dim3(THREADS), smem, stream, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start, positions, S, (__nv_bfloat16*)out,
+                     H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
     } else {
         auto kern = latent_attention_tc_kernel<R>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return AIEN_E_STATE;
-        kern<<<grid, THREADS, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start, positions, S, (__nv_bfloat16*)out,
-                                              H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
+        launch_chain(kern, grid, dim3(THREADS), smem, stream, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, max_blocks, q_start, positions, S, (__nv_bfloat16*)out,
+                     H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
     }
     if (ksplit > 1)
-        latent_attention_merge_kernel<<<dim3((unsigned)((long)(tokens != nullptr ? num_tokens : T) * H)), 128, 0, stream>>>(
+        launch_chain(latent_attention_merge_kernel, dim3((unsigned)((long)(tokens != nullptr ? num_tokens : T) * H)), dim3(128), (size_t)0, stream,
             r_lat, part_o, part_ml, ksplit, sinks, H, (__nv_bfloat16*)out, tokens);
     return launch_status();
 }
@@ -646,6 +652,8 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
     __shared__ __align__(16) __nv_bfloat16 Ws[HT_STAGES][HT_BN * HT_STR];
     constexpr int NJ = HT_BN / 16;                             // n8 tiles of a warp
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    griddep_launch();
+    griddep_wait();
     const int mh = warp & 1, nh = warp >> 1, g = lane >> 2, c = lane & 3;
     const int m0 = blockIdx.y * HT_BM, n0 = blockIdx.x * HT_BN, h = blockIdx.z;
     A += (size_t)h * a_head;
@@ -682,7 +690,7 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int n = n0 + nh * (HT_BN / 2) + j * 8 + 2 * c + e;
-                    gates[mt][r][j][e] = gate_n > 0 && ml < M && n < N ? load_dyn(gate, gdt, at[mt][r] * ldg + (size_t)h * gate_n + n) : 0.f;
+                    gates[mt][r][j][e] = gate_n > 0 && ml < M && n < N ? ld_act_dyn(gate, gdt, at[mt][r] * ldg + (size_t)h * gate_n + n) : 0.f;
                 }
         }
     const int steps = (K + HT_BK - 1) / HT_BK;
@@ -724,7 +732,7 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
             const int ml = m0 + mh * 32 + mt * 16 + g + r * 8;
             if (ml >= M) continue;
             const size_t m = at[mt][r];
-            const float gs = (gate != nullptr && gate_n == 0) ? 1.0f / (1.0f + expf(-load_dyn(gate, gdt, m * ldg + h))) : 1.0f;
+            const float gs = (gate != nullptr && gate_n == 0) ? 1.0f / (1.0f + expf(-ld_act_dyn(gate, gdt, m * ldg + h))) : 1.0f;
 #pragma unroll
             for (int j = 0; j < NJ; ++j) {
                 const int n = n0 + nh * (HT_BN / 2) + j * 8 + 2 * c;
@@ -756,6 +764,8 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, int r_lat, const i
                      int* __restrict__ table) {
     __shared__ int s_req;
     const int p = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    griddep_launch();
+    griddep_wait();
     if (tid == 0) s_req = -1;
     __syncthreads();
     if (warp == 0) {
@@ -778,7 +788,7 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, int r_lat, const i
         const int page = key < n ? bt[key / page_size] : -1;
         const uint4* src = reinterpret_cast<const uint4*>(cache + ((size_t)(page >= 0 ? page : 0) * page_size + key % page_size) * r_lat);
         uint4* dst = reinterpret_cast<uint4*>(out + ((size_t)p * len + key) * r_lat);
-        for (int i = lane; i < r_lat / 8; i += 32) dst[i] = page >= 0 ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+        for (int i = lane; i < r_lat / 8; i += 32) dst[i] = page >= 0 ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -834,7 +844,7 @@ AIEN_API int aien_head_project_tc(const void* A, long lda, long a_head, const vo
     const bool narrow = rows64 * ((N + 63) / 64) * heads <= 148;           // 64 columns would give every SM one CTA at most
     const int bn = narrow ? 32 : 64;
     const dim3 grid((N + bn - 1) / bn, (unsigned)rows64, heads);
-    AIEN_DISPATCH_DTYPE(c_dt, TC, ((narrow ? head_project_tc_kernel<32, TC> : head_project_tc_kernel<64, TC>)<<<grid, 128, 0, stream>>>(
+    AIEN_DISPATCH_DTYPE(c_dt, TC, (launch_chain(narrow ? head_project_tc_kernel<32, TC> : head_project_tc_kernel<64, TC>, grid, dim3(128), (size_t)0, stream,
         (const __nv_bfloat16*)A, lda, a_head, (const __nv_bfloat16*)W, (long)N * K, (TC*)C, ldc, c_head, M, N, K, gate, gate_dt, ldg, gate_n, rows)));
     return launch_status();
 }
@@ -846,7 +856,7 @@ AIEN_API int aien_latent_gather(const void* cache, int r_lat, const int* block_t
     if (portions <= 0 || S <= 0) return 0;
     if (r_lat <= 0 || (r_lat & 7) || page_size <= 0 || len <= 0 || (len & 127) || portions > 65535) return AIEN_E_SHAPE;
     if (((uintptr_t)cache & 15) || ((uintptr_t)out & 15)) return AIEN_E_ALIGN;
-    latent_gather_kernel<<<dim3(len / 8, portions), 256, 0, stream>>>((const __nv_bfloat16*)cache, r_lat, block_table, max_blocks, page_size, q_start,
-                                                                      ctx_len, S, len, (__nv_bfloat16*)out, table);
+    launch_chain(latent_gather_kernel, dim3(len / 8, portions), dim3(256), (size_t)0, stream, (const __nv_bfloat16*)cache, r_lat, block_table, max_blocks, page_size,
+                 q_start, ctx_len, S, len, (__nv_bfloat16*)out, table);
     return launch_status();
 }

@@ -113,15 +113,17 @@ moe_route_biased_kernel(const float* __restrict__ z, long ldz, int E, int real, 
     __shared__ float ch[ROUTE_MAX_EXPERTS];
     const int t = blockIdx.x, lane = threadIdx.x;
     const float* zr = z + (size_t)t * ldz;
+    griddep_launch();
+    griddep_wait();
     if (sigmoid) {
         for (int e = lane; e < E; e += 32) {
-            const float v = zr[e];
+            const float v = ld_act(zr + e);
             s[e] = 1.0f / (1.0f + expf(-v));
             ch[e] = correction != nullptr ? s[e] + load_dyn(correction, cdt, e) : v;
         }
     } else {
         float m = -INFINITY;
-        for (int e = lane; e < E; e += 32) { const float v = zr[e]; s[e] = v; m = fmaxf(m, v); }
+        for (int e = lane; e < E; e += 32) { const float v = ld_act(zr + e); s[e] = v; m = fmaxf(m, v); }
         m = warp_max(m);
         float sum = 0.f;
         for (int e = lane; e < E; e += 32) { const float v = expf(s[e] - m); s[e] = v; sum += v; }
@@ -579,7 +581,7 @@ AIEN_API int aien_moe_route_biased(const float* z, long ldz, int T, int E, int r
                                    cudaStream_t stream) {
     if (T <= 0) return 0;
     if (E <= 0 || E > ROUTE_MAX_EXPERTS || real <= 0 || real > E || top <= 0 || top > E || (real < E && w_same == nullptr)) return AIEN_E_SHAPE;
-    moe_route_biased_kernel<<<T, 32, 0, stream>>>(z, ldz, E, real, top, renorm, renorm_eps, correction, c_dt, sigmoid, ids, wts, w_same, expert_count);
+    launch_chain(moe_route_biased_kernel, dim3(T), dim3(32), (size_t)0, stream, z, ldz, E, real, top, renorm, renorm_eps, correction, c_dt, sigmoid, ids, wts, w_same, expert_count);
     return launch_status();
 }
 

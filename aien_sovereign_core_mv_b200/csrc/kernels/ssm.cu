@@ -138,9 +138,11 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
     __shared__ __align__(16) float2 steps[C::ROWS];                    // (dt, dt * x) per token and channel
     __shared__ __align__(16) float sums[C::TOKENS * SSM_THREADS];      // a lane's part of y per token
     const int s = blockIdx.y, seg = sg.mode == 0 ? 0 : blockIdx.z;
-    int t0 = q_start[s], t1 = q_start[s + 1];
+    griddep_launch();
+    griddep_wait();
+    int t0 = __ldcg(q_start + s), t1 = __ldcg(q_start + s + 1);
     if (t1 <= t0) return;
-    const bool fresh = positions[t0] == 0;
+    const bool fresh = __ldcg(positions + t0) == 0;
     const size_t seg0 = sg.mode == 0 ? 0 : (size_t)(t0 / sg.seg_len + s);         // the request's first segment in the scratch
     if (sg.mode != 0) {
         t0 += seg * sg.seg_len;
@@ -336,6 +338,8 @@ segment_combine_kernel(float* __restrict__ state, size_t state_stride, size_t s_
                        const int* __restrict__ q_start, const int* __restrict__ positions, Segments sg, size_t lanes) {
     const int s = blockIdx.y;
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    griddep_launch();
+    griddep_wait();
     if (i >= lanes) return;
     const int t0 = q_start[s], n_tok = q_start[s + 1] - t0;
     if (n_tok <= 0) return;
@@ -358,9 +362,11 @@ __global__ void __launch_bounds__(256)
 ssd_steps_kernel(const float* __restrict__ dtr, long lddt, const float* __restrict__ A, const void* __restrict__ bias, int pdt,
                  float* __restrict__ steps, int T, int heads) {
     const int i = blockIdx.x * 256 + threadIdx.x;
+    griddep_launch();
+    griddep_wait();
     if (i >= T * heads) return;
     const int t = i / heads, h = i - t * heads;
-    const float dt = ssm_softplus(dtr[(size_t)t * lddt + h] + load_dyn(bias, pdt, h));
+    const float dt = ssm_softplus(ld_act(dtr + (size_t)t * lddt + h) + load_dyn(bias, pdt, h));
     steps[(size_t)t * 2 * heads + h] = dt;
     steps[(size_t)t * 2 * heads + heads + h] = expf(-A[h] * dt);
 }
@@ -538,14 +544,16 @@ __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, long ldx, int P, size_t part_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ rest,
                   int T, int n, int m) {
     const long i = (long)blockIdx.x * 256 + threadIdx.x;
+    griddep_launch();
+    griddep_wait();
     if (i >= (long)T * (n + m)) return;
     const int t = (int)(i / (n + m)), c = (int)(i - (long)t * (n + m));
     const float* xc = x + t * ldx + c;
-    float v = xc[0];
+    float v = ld_act(xc);
     for (int p0 = 1; p0 < P; p0 += 4) {                         // partial products in order, four loads in flight
         float w[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = p0 + j < P ? xc[(p0 + j) * part_stride] : 0.f;
+        for (int j = 0; j < 4; ++j) w[j] = p0 + j < P ? ld_act(xc + (p0 + j) * part_stride) : 0.f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) v += w[j];
     }
@@ -601,14 +609,14 @@ static void launch_selective_scan(const ScanArgs& a) {
     const dim3 grid((unsigned)((a.inner + C::CPB - 1) / C::CPB), a.S, sg.mode == 0 ? 1 : sg.nseg);
     if (sg.mode != 0) {
         const size_t lanes = (size_t)a.inner * a.N;
-        selective_scan_kernel<LANES, CH, true, TO><<<grid, SSM_THREADS, 0, a.stream>>>(
-            a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
-        segment_combine_kernel<<<dim3((unsigned)((lanes + 255) / 256), a.S), 256, 0, a.stream>>>(a.state, a.state_stride, a.s_off, a.slots, a.q_start,
-                                                                                                 a.positions, sg, lanes);
+        launch_chain(selective_scan_kernel<LANES, CH, true, TO>, grid, dim3(SSM_THREADS), (size_t)0, a.stream, a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state,
+                     a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+        launch_chain(segment_combine_kernel, dim3((unsigned)((lanes + 255) / 256), a.S), dim3(256), (size_t)0, a.stream, a.state, a.state_stride, a.s_off, a.slots,
+                     a.q_start, a.positions, sg, lanes);
         sg.mode = 2;
     }
-    selective_scan_kernel<LANES, CH, false, TO><<<grid, SSM_THREADS, 0, a.stream>>>(
-        a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+    launch_chain(selective_scan_kernel<LANES, CH, false, TO>, grid, dim3(SSM_THREADS), (size_t)0, a.stream, a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state,
+                 a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
 }
 
 template <int LANES, int CH, typename TO>
@@ -686,7 +694,7 @@ AIEN_API int aien_selective_scan(const float* x, long ldx, const float* dtz, lon
 AIEN_API int aien_ssd_steps(const float* dtr, long lddt, const float* A, const void* dt_bias, int p_dt, float* steps, int T, int heads,
                             cudaStream_t stream) {
     if (T <= 0 || heads <= 0) return T == 0 ? 0 : AIEN_E_SHAPE;
-    ssd_steps_kernel<<<(unsigned)(((long)T * heads + 255) / 256), 256, 0, stream>>>(dtr, lddt, A, dt_bias, p_dt, steps, T, heads);
+    launch_chain(ssd_steps_kernel, dim3((unsigned)(((long)T * heads + 255) / 256)), dim3(256), (size_t)0, stream, dtr, lddt, A, dt_bias, p_dt, steps, T, heads);
     return launch_status();
 }
 
@@ -767,7 +775,8 @@ AIEN_API int aien_ssd_scan(const float* xbc, long ld, int x_off, int b_off, int 
 AIEN_API int aien_split_rows(const float* x, long ldx, int P, size_t part_stride, void* out, float* rest, int T, int n, int m, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (n <= 0 || m < 0 || P < 1 || (m > 0 && rest == nullptr) || ((long)T * (n + m) + 255) / 256 > 2147483647L) return AIEN_E_SHAPE;
-    split_rows_kernel<<<(unsigned)(((long)T * (n + m) + 255) / 256), 256, 0, stream>>>(x, ldx, P, part_stride, (__nv_bfloat16*)out, rest, T, n, m);
+    launch_chain(split_rows_kernel, dim3((unsigned)(((long)T * (n + m) + 255) / 256)), dim3(256), (size_t)0, stream, x, ldx, P, part_stride, (__nv_bfloat16*)out, rest, T,
+                 n, m);
     return launch_status();
 }
 
