@@ -35,67 +35,120 @@ __device__ __forceinline__ float act_apply(float z, int kind) {
 // ---------------------------------------------------------------- router
 constexpr int ROUTE_MAX_EXPERTS = 1024;
 
-__global__ void __launch_bounds__(32)
-moe_route_kernel(const float* __restrict__ z, int E, int groups, int keep, int top, int renorm,
-                 int* __restrict__ ids, float* __restrict__ wts, int* __restrict__ expert_count) {
-    __shared__ float s[ROUTE_MAX_EXPERTS];
-    __shared__ float gs[ROUTE_MAX_EXPERTS];
-    griddep_launch();
-    griddep_wait();
-    const int t = blockIdx.x, lane = threadIdx.x;
-    const float* zr = z + (size_t)t * E;
+// One warp per token, its scores in registers: lane l holds experts l, l + 32, ...  What bounds a router is the chain of its `top` choices, one
+// after another, and a choice is two warp reductions in hardware: the largest key (unsigned, in the order of the floats), then the
+// lowest expert that has it.  Before, every choice went through shared memory and ten shuffles, the weights back through global memory.
+// B200, us, before and so: 2,048 tokens, 6 of 64 experts in 4 of 8 groups 14.7 and 7.1; 8 of 256 20.4 and 12.5; 64 tokens, 6 of 64 6.5 and 2.6;
+// 9 tokens, 4 of 16 with sigmoid scores 3.3 and 1.6; 16 tokens, 8 of 1,024 7.4 and 5.3.  Choices and weights are the same to the bit.
+constexpr int ROUTE_WARPS = 4;                                            // tokens per CTA
+constexpr uint32_t ROUTE_TAKEN = 0;                                       // below the key of every float
+
+__device__ __forceinline__ uint32_t route_key(float v) {
+    const uint32_t u = __float_as_uint(v + 0.0f);                         // -0 and 0 are one
+    return (u & 0x80000000u) != 0 ? ~u : u | 0x80000000u;
+}
+
+// The largest key's index (ties to the lower), which is then taken.
+template <int NR>
+__device__ __forceinline__ int route_pick(uint32_t (&key)[NR], int lane) {
+    uint32_t k = key[0];
+    int e = lane;
+#pragma unroll
+    for (int j = 1; j < NR; ++j)
+        if (key[j] > k) { k = key[j]; e = lane + 32 * j; }
+    const uint32_t most = __reduce_max_sync(0xffffffffu, k);
+    const int pick = __reduce_min_sync(0xffffffffu, k == most ? e : 0x7fffffff);
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+        if (pick == lane + 32 * j) key[j] = ROUTE_TAKEN;
+    return pick;
+}
+
+// The score of expert `pick` from the lane that holds it.
+template <int NR>
+__device__ __forceinline__ float route_score(const float (&s)[NR], int pick, int lane) {
+    float w = s[0];
+#pragma unroll
+    for (int j = 1; j < NR; ++j)
+        if (pick == lane + 32 * j) w = s[j];
+    return __shfl_sync(0xffffffffu, w, pick & 31);
+}
+
+// s = softmax of a row's E numbers
+template <int NR>
+__device__ __forceinline__ void route_softmax(float (&s)[NR], const float* zr, int E, int lane) {
     float m = -INFINITY;
-    for (int e = lane; e < E; e += 32) { const float v = __ldcg(zr + e); s[e] = v; m = fmaxf(m, v); }
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+        s[j] = lane + 32 * j < E ? __ldcg(zr + lane + 32 * j) : -INFINITY;
+        m = fmaxf(m, s[j]);
+    }
     m = warp_max(m);
     float sum = 0.f;
-    for (int e = lane; e < E; e += 32) { const float v = expf(s[e] - m); s[e] = v; sum += v; }
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+        if (lane + 32 * j < E) { s[j] = expf(s[j] - m); sum += s[j]; }
     sum = warp_sum(sum);
     const float inv = 1.0f / sum;
-    for (int e = lane; e < E; e += 32) s[e] *= inv;
-    __syncwarp();
-    const int per = E / groups;
-    if (groups > 1 && keep < groups) {
-        for (int g = lane; g < groups; g += 32) {
-            float best = -INFINITY;
-            for (int j = 0; j < per; ++j) best = fmaxf(best, s[g * per + j]);
-            gs[g] = best;
-        }
+#pragma unroll
+    for (int j = 0; j < NR; ++j) s[j] *= inv;
+}
+
+template <int NR>
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_kernel(const float* __restrict__ z, int T, int E, int groups, int keep, int top, int renorm,
+                 int* __restrict__ ids, float* __restrict__ wts, int* __restrict__ expert_count) {
+    __shared__ float held[ROUTE_WARPS][NR * 32];              // the groups' scores and choices, then the chosen weights
+    __shared__ int chosen[ROUTE_WARPS][NR * 32];
+    griddep_launch();
+    griddep_wait();
+    const int t = blockIdx.x * ROUTE_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= T) return;
+    float* w_at = held[threadIdx.x >> 5];
+    int* id_at = chosen[threadIdx.x >> 5];
+    float s[NR];
+    uint32_t key[NR];
+    route_softmax<NR>(s, z + (size_t)t * E, E, lane);
+#pragma unroll
+    for (int j = 0; j < NR; ++j) key[j] = lane + 32 * j < E ? route_key(s[j]) : ROUTE_TAKEN;
+    if (groups > 1 && keep < groups) {                        // only the `keep` best groups' experts may be chosen
+        const int per = E / groups;
+#pragma unroll
+        for (int j = 0; j < NR; ++j) w_at[lane + 32 * j] = s[j];
         __syncwarp();
-        // every group starts ineligible (score negated below zero); the `keep` best are restored
-        for (int r = 0; r < keep; ++r) {
-            float bv = -INFINITY; int bi = 0x7fffffff;
-            for (int g = lane; g < groups; g += 32) if (gs[g] > bv) { bv = gs[g]; bi = g; }
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+        uint32_t gkey[NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const int g = lane + 32 * i;
+            gkey[i] = ROUTE_TAKEN;
+            if (g < groups) {
+                float best = -INFINITY;
+                for (int j = 0; j < per; ++j) best = fmaxf(best, w_at[g * per + j]);
+                gkey[i] = route_key(best);
             }
-            if (lane == 0) gs[bi] = -1.0f;                 // marks a kept group (scores are >= 0)
-            __syncwarp();
         }
-        for (int e = lane; e < E; e += 32) if (gs[e / per] != -1.0f) s[e] = -1.0f;      // not eligible
+        for (int r = 0; r < keep; ++r) route_pick<NR>(gkey, lane);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < NR; ++i) id_at[lane + 32 * i] = gkey[i] == ROUTE_TAKEN;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < NR; ++j)
+            if (lane + 32 * j < E && !id_at[(lane + 32 * j) / per]) key[j] = route_key(-1.0f);      // below every score
         __syncwarp();
     }
     float wsum = 0.f;
     for (int r = 0; r < top; ++r) {
-        float bv = -INFINITY; int bi = 0x7fffffff;
-        for (int e = lane; e < E; e += 32) if (s[e] > bv) { bv = s[e]; bi = e; }
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        if (lane == 0) {
-            ids[(size_t)t * top + r] = bi;
-            wts[(size_t)t * top + r] = bv;
-            s[bi] = -2.0f;                                 // taken
-            if (expert_count != nullptr) atomicAdd(expert_count + bi, 1);     // for the plan of the grouped products
-        }
-        wsum += bv;
-        __syncwarp();
+        const int e = route_pick<NR>(key, lane);
+        const float w = route_score<NR>(s, e, lane);
+        wsum += w;
+        if (lane == 0) { id_at[r] = e; w_at[r] = w; }
     }
-    if (renorm && lane == 0) {
-        for (int r = 0; r < top; ++r) wts[(size_t)t * top + r] /= wsum;
+    __syncwarp();
+    for (int r = lane; r < top; r += 32) {
+        ids[(size_t)t * top + r] = id_at[r];
+        wts[(size_t)t * top + r] = renorm ? w_at[r] / wsum : w_at[r];
+        if (expert_count != nullptr) atomicAdd(expert_count + id_at[r], 1);     // for the plan of the grouped products
     }
 }
 
@@ -104,70 +157,71 @@ moe_route_kernel(const float* __restrict__ z, int E, int groups, int keep, int t
 // the same order and does not saturate); the `top` experts with the largest s + correction are chosen (ties to the lower index); a choice weighs s,
 // divided by the sum of the chosen s plus renorm_eps when `renorm` is set.  Experts from `real` on have no tensors:
 // their output is their input, so their weights are summed into w_same[t] and the choice is handed on as expert 0
-// with weight zero (the expert products need no case for it).  One warp per token.
-__global__ void __launch_bounds__(32)
-moe_route_biased_kernel(const float* __restrict__ z, long ldz, int E, int real, int top, int renorm, float renorm_eps,
+// with weight zero (the expert products need no case for it).
+template <int NR>
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_biased_kernel(const float* __restrict__ z, long ldz, int T, int E, int real, int top, int renorm, float renorm_eps,
                         const void* __restrict__ correction, int cdt, int sigmoid, int* __restrict__ ids, float* __restrict__ wts,
                         float* __restrict__ w_same, int* __restrict__ expert_count) {
-    __shared__ float s[ROUTE_MAX_EXPERTS];
-    __shared__ float ch[ROUTE_MAX_EXPERTS];
-    const int t = blockIdx.x, lane = threadIdx.x;
-    const float* zr = z + (size_t)t * ldz;
+    __shared__ float held[ROUTE_WARPS][NR * 32];
+    __shared__ int chosen[ROUTE_WARPS][NR * 32];
     griddep_launch();
     griddep_wait();
-    if (sigmoid) {
-        for (int e = lane; e < E; e += 32) {
-            const float v = ld_act(zr + e);
-            s[e] = 1.0f / (1.0f + expf(-v));
-            ch[e] = correction != nullptr ? s[e] + load_dyn(correction, cdt, e) : v;
-        }
-    } else {
-        float m = -INFINITY;
-        for (int e = lane; e < E; e += 32) { const float v = ld_act(zr + e); s[e] = v; m = fmaxf(m, v); }
-        m = warp_max(m);
-        float sum = 0.f;
-        for (int e = lane; e < E; e += 32) { const float v = expf(s[e] - m); s[e] = v; sum += v; }
-        sum = warp_sum(sum);
-        const float inv = 1.0f / sum;
-        for (int e = lane; e < E; e += 32) {
-            s[e] *= inv;
-            ch[e] = correction != nullptr ? s[e] + load_dyn(correction, cdt, e) : s[e];
+    const int t = blockIdx.x * ROUTE_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= T) return;
+    const float* zr = z + (size_t)t * ldz;
+    float* w_at = held[threadIdx.x >> 5];
+    int* id_at = chosen[threadIdx.x >> 5];
+    float s[NR];
+    uint32_t key[NR];
+    if (!sigmoid) route_softmax<NR>(s, zr, E, lane);
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+        const int e = lane + 32 * j;
+        key[j] = ROUTE_TAKEN;
+        if (e < E) {
+            const float v = sigmoid ? __ldcg(zr + e) : s[j];
+            if (sigmoid) s[j] = 1.0f / (1.0f + expf(-v));
+            key[j] = route_key(correction != nullptr ? s[j] + load_dyn(correction, cdt, e) : v);
         }
     }
-    __syncwarp();
     float wsum = 0.f;
     for (int r = 0; r < top; ++r) {
-        float bv = -INFINITY; int bi = 0x7fffffff;
-        for (int e = lane; e < E; e += 32) if (ch[e] > bv) { bv = ch[e]; bi = e; }
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        const float w = s[bi];
+        const int e = route_pick<NR>(key, lane);
+        const float w = route_score<NR>(s, e, lane);
         wsum += w;
-        __syncwarp();
-        if (lane == 0) {
-            ids[(size_t)t * top + r] = bi;
-            wts[(size_t)t * top + r] = w;
-            ch[bi] = -INFINITY;                            // taken
-        }
-        __syncwarp();
+        if (lane == 0) { id_at[r] = e; w_at[r] = w; }
     }
+    __syncwarp();
+    const float div = renorm ? wsum + renorm_eps : 1.0f;
+    for (int r = lane; r < top; r += 32) {
+        const float w = w_at[r] / div;
+        const int e = id_at[r], to = e < real ? e : 0;
+        w_at[r] = w;
+        ids[(size_t)t * top + r] = to;
+        wts[(size_t)t * top + r] = e < real ? w : 0.f;
+        if (expert_count != nullptr) atomicAdd(expert_count + to, 1);
+    }
+    if (w_same == nullptr) return;
+    __syncwarp();
     if (lane == 0) {
-        const float div = renorm ? wsum + renorm_eps : 1.0f;
         float same = 0.f;
-        for (int r = 0; r < top; ++r) {
-            const size_t at = (size_t)t * top + r;
-            const float w = wts[at] / div;
-            int e = ids[at];
-            if (e >= real) { same += w; e = 0; wts[at] = 0.f; } else wts[at] = w;
-            ids[at] = e;
-            if (expert_count != nullptr) atomicAdd(expert_count + e, 1);
-        }
-        if (w_same != nullptr) w_same[t] = same;
+        if (real < E)
+            for (int r = 0; r < top; ++r)
+                if (id_at[r] >= real) same += w_at[r];
+        w_same[t] = same;
     }
 }
+
+// BODY with NR bound: registers of a lane for E experts
+#define ROUTE_DISPATCH(E, BODY)                             \
+    do {                                                    \
+        if ((E) <= 32) { constexpr int NR = 1; BODY; }      \
+        else if ((E) <= 64) { constexpr int NR = 2; BODY; } \
+        else if ((E) <= 128) { constexpr int NR = 4; BODY; }\
+        else if ((E) <= 256) { constexpr int NR = 8; BODY; }\
+        else { constexpr int NR = 32; BODY; }               \
+    } while (0)
 
 // ---------------------------------------------------------------- plain expert products
 // One warp per output value; 8 warps a CTA take 8 consecutive output rows of one (token, choice).
@@ -570,7 +624,8 @@ AIEN_API int aien_moe_route(const float* z, int T, int E, int groups, int keep, 
     if (T <= 0) return 0;
     if (E <= 0 || E > ROUTE_MAX_EXPERTS || groups <= 0 || E % groups != 0 || keep <= 0 || keep > groups || top <= 0 ||
         top > keep * (E / groups)) return AIEN_E_SHAPE;
-    launch_chain(moe_route_kernel, dim3(T), dim3(32), 0, stream, z, E, groups, keep, top, renorm, ids, wts, expert_count);
+    ROUTE_DISPATCH(E, (launch_chain(moe_route_kernel<NR>, dim3((unsigned)((T + ROUTE_WARPS - 1) / ROUTE_WARPS)), dim3(ROUTE_WARPS * 32), (size_t)0, stream, z, T, E,
+                                    groups, keep, top, renorm, ids, wts, expert_count)));
     return launch_status();
 }
 
@@ -581,7 +636,8 @@ AIEN_API int aien_moe_route_biased(const float* z, long ldz, int T, int E, int r
                                    cudaStream_t stream) {
     if (T <= 0) return 0;
     if (E <= 0 || E > ROUTE_MAX_EXPERTS || real <= 0 || real > E || top <= 0 || top > E || (real < E && w_same == nullptr)) return AIEN_E_SHAPE;
-    launch_chain(moe_route_biased_kernel, dim3(T), dim3(32), (size_t)0, stream, z, ldz, E, real, top, renorm, renorm_eps, correction, c_dt, sigmoid, ids, wts, w_same, expert_count);
+    ROUTE_DISPATCH(E, (launch_chain(moe_route_biased_kernel<NR>, dim3((unsigned)((T + ROUTE_WARPS - 1) / ROUTE_WARPS)), dim3(ROUTE_WARPS * 32), (size_t)0, stream, z, ldz,
+                                    T, E, real, top, renorm, renorm_eps, correction, c_dt, sigmoid, ids, wts, w_same, expert_count)));
     return launch_status();
 }
 

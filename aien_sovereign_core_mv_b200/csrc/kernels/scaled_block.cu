@@ -102,6 +102,8 @@ routed_combine_vec_kernel(const TP* __restrict__ parts, int nparts, size_t part_
                           const float* __restrict__ w_same, const TS* __restrict__ shared, int sparts, size_t sstride,
                           const float* __restrict__ zs, long ldzs, float* __restrict__ out, int H) {
     const int t = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 4;
+    griddep_launch();
+    griddep_wait();
     if (i >= H) return;
     const size_t at = (size_t)t * H + i;
     auto sum = [&](const auto* p, int n, size_t stride) {
@@ -119,13 +121,13 @@ routed_combine_vec_kernel(const TP* __restrict__ parts, int nparts, size_t part_
     float4 v = sum(parts, nparts, part_stride);
     if (w_same != nullptr) {
         const float4 x = ld_act4(h + (size_t)t * ldh + i);
-        const float w = w_same[t];
+        const float w = ld_act(w_same + t);
         v = make_float4(fmaf(w, x.x, v.x), fmaf(w, x.y, v.y), fmaf(w, x.z, v.z), fmaf(w, x.w, v.w));
     }
     if (shared != nullptr) {
         const float4 s = sum(shared, sparts, sstride);
         if (zs != nullptr) {
-            const float g = 1.0f / (1.0f + expf(-zs[(size_t)t * ldzs]));
+            const float g = 1.0f / (1.0f + expf(-ld_act(zs + (size_t)t * ldzs)));
             v = make_float4(fmaf(g, s.x, v.x), fmaf(g, s.y, v.y), fmaf(g, s.z, v.z), fmaf(g, s.w, v.w));
         } else {
             v = make_float4(v.x + s.x, v.y + s.y, v.z + s.z, v.w + s.w);
@@ -192,7 +194,7 @@ AIEN_API int aien_routed_combine(const void* parts, int p_dt, int nparts, size_t
     if (H % 4 == 0 && part_stride % 4 == 0 && lies(parts, p_dt) && lies(out, AIEN_DT_F32) && (w_same == nullptr || (ldh % 4 == 0 && lies(h, h_dt))) &&
         (shared == nullptr || (sstride % 4 == 0 && lies(shared, s_dt)))) {
         AIEN_DISPATCH_DTYPE(p_dt, TP, AIEN_DISPATCH_DTYPE(h_dt, TH, AIEN_DISPATCH_DTYPE(s_dt, TS,
-            (routed_combine_vec_kernel<TP, TH, TS><<<dim3((H + 1023) / 1024, T), 256, 0, stream>>>(
+            (launch_chain(routed_combine_vec_kernel<TP, TH, TS>, dim3((H + 1023) / 1024, T), dim3(256), (size_t)0, stream,
                 (const TP*)parts, nparts, part_stride, (const TH*)h, ldh, w_same, (const TS*)shared, sparts, sstride, zs, ldzs, out, H)))));
         return launch_status();
     }

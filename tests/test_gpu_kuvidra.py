@@ -375,6 +375,49 @@ def test_router_of_sigmoid_scores(E, top):
     H.assert_close(wts.cpu().numpy(), pk.sigmoid(np.take_along_axis(f64(z[:, :E]), ids.cpu().numpy().astype(np.int64), -1)), 1e-6, "weights")
 
 
+@pytest.mark.parametrize("E,groups,keep,top", [(1, 1, 1, 1), (33, 1, 1, 5), (64, 8, 4, 6), (66, 33, 2, 3), (128, 128, 40, 40), (130, 2, 1, 8), (300, 3, 2, 8), (1024, 32, 3, 8)])
+def test_routers_of_every_width(E, groups, keep, top):
+    """One to thirty-two scores a lane, equal scores (the lower expert first), kept groups, more choices than lanes, weights divided by their
+    sum, experts that return their input; token counts that fill no CTA."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(E + top)
+    T = 9
+    z = torch.randint(-8, 9, (T, E + 2), generator=g).float() * 0.5
+    z[0] = -0.0                                                       # every score alike, and zeros of both signs
+    z[0, ::2] = 0.0
+    s = np.exp(f64(z[:, :E]) - f64(z[:, :E]).max(-1, keepdims=True))
+    s /= s.sum(-1, keepdims=True)
+    ids, wts = torch.zeros(T, top, dtype=torch.int32).cuda(), torch.zeros(T, top).cuda()
+    counts = torch.zeros(E, dtype=torch.int32).cuda()
+
+    def check(order, weight, may):
+        choice = np.argsort(-np.where(may, order, -1e9), axis=-1, kind="stable")[:, :top]
+        w = np.take_along_axis(weight, choice, -1)
+        return choice, w / w.sum(-1, keepdims=True)
+
+    K.moe_route(z[:, :E].contiguous().cuda(), groups, keep, top, True, ids, wts, counts)
+    best = s.reshape(T, groups, E // groups).max(-1)
+    kept = np.zeros((T, groups), bool)
+    np.put_along_axis(kept, np.argsort(-best, axis=-1, kind="stable")[:, :keep], True, -1)
+    choice, w = check(s, s, np.repeat(kept, E // groups, axis=-1))
+    assert (ids.cpu().numpy() == choice).all() and counts.cpu().tolist() == np.bincount(choice.ravel(), minlength=E).tolist()
+    H.assert_close(wts.cpu().numpy(), w, 1e-5, "weights")
+    # the correction decides the first choices; a third of the experts have no tensors
+    corr = torch.zeros(E)
+    corr[:: max(E // 3, 1)] = 1.0
+    real, same = E - E // 3, torch.full((T,), 7.0).cuda()
+    counts.zero_()
+    for sigmoid in (False, True):
+        score = pk.sigmoid(f64(z[:, :E])) if sigmoid else s
+        c = None if sigmoid else corr.cuda()
+        K.moe_route_biased(z.cuda(), E, real, top, True, 0.0, c, ids, wts, same, counts if sigmoid else None, sigmoid=sigmoid)
+        choice, w = check(f64(z[:, :E]) if sigmoid else s + f64(corr), score, True)
+        assert (ids.cpu().numpy() == np.where(choice < real, choice, 0)).all()
+        H.assert_close(wts.cpu().numpy(), np.where(choice < real, w, 0.0), 1e-5, "weights")
+        H.assert_close(same.cpu().numpy(), np.where(choice < real, 0.0, w).sum(-1), 1e-5, "weight of the input")
+    assert counts.cpu().tolist() == np.bincount(np.where(choice < real, choice, 0).ravel(), minlength=E).tolist()
+
+
 @pytest.mark.parametrize("E,top,T,D,F_", [(16, 4, 9, 2048, 1024), (5, 3, 16, 200, 24), (64, 6, 16, 512, 136), (8, 2, 5, 1032, 40), (3, 3, 16, 72, 8), (20, 16, 16, 64, 1024)])
 @pytest.mark.parametrize("gated", [True, False])
 def test_experts_of_a_few_tokens_share_their_rows(E, top, T, D, F_, gated):
