@@ -102,10 +102,13 @@ struct PtMaps {
 // stands for q and k, bit 1 for v.  v_share neighbouring key heads share a value head.  out_f32: float32 results.
 // egate (or null): bfloat16 rows of the step's tokens, ldeg numbers apart; column h * hdv + i of the result is multiplied by
 // sigmoid(egate[t][h * hdv + i]).
+// table_made: a kernel of this step wrote the block table (latent_gather_kernel), so no entry of it is read before
+// griddep_wait(): that kernel may still be waiting for its own predecessor when this one's first CTAs start.
 struct PtSizes {
     int hdv, by_head, v_share, out_f32;
     const __nv_bfloat16* egate;
     long ldeg;
+    int table_made;
 };
 
 __device__ __forceinline__ float pt_sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
@@ -216,15 +219,17 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             if (lane < pages_per_block) {
                 const int key0 = kb * PT_BN + lane * page_size;
                 const int blk = key0 / page_size;
-                if (key0 <= pos_last && key0 + page_size > first && blk < max_blocks) page = bt[blk];
+                if (key0 <= pos_last && key0 + page_size > first && blk < max_blocks) page = __ldcg(bt + blk);
             }
             return page;
         };
-        int page_next = page_of(item_block(0));          // the table is this step's metadata, not the work of the kernel ahead
+        // A table that the host copied was there before the step's first kernel, so its first entry is asked for ahead of the wait.
+        int page_next = sz.table_made ? -1 : page_of(item_block(0));
         // Queries and this step's rows of the caches come from the kernel ahead in the stream: with a
         // dependent launch everything above ran beside its tail, and no other warp touches global
         // memory before it has data from this one.
         griddep_wait();
+        if (sz.table_made) page_next = page_of(item_block(0));
         if (lane == 0) {
             mbar_expect_tx(q_full, (has_b ? 2 : 1) * S::Q_LOAD);
             for (int h = 0; h < (has_b ? 2 : 1); ++h)
@@ -709,6 +714,7 @@ AIEN_API int aien_paged_attention_prefill_tc_portions_supports(int hd, int hdv, 
 // head_scale, slopes (float32 [nq]) and gate (float32 [tokens of the step, ldg]), each of which may be null, and softcap
 // (0: none): see HeadTerms.
 // k_ld, v_ld: numbers between rows of the caches (0: the rows are contiguous); egate, ldeg: see PtSizes (bfloat16 results only).
+// table_made: 1 where a kernel of this step wrote block_table, 0 where the host copied it there (see PtSizes).
 // hdv, v_share, out_f32: values of hdv numbers, one value head for every v_share neighbouring key heads (v_cache
 // [cache_rows, nkv / v_share * hdv], out [tokens, nq * hdv]), float32 results; hd and hdv are multiples of 8,
 // hd up to 192, hdv up to 128.
@@ -717,7 +723,7 @@ AIEN_API int aien_paged_attention_prefill_tc_values(
     int max_blocks, const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_q0, int num_tiles, void* out,
     long out_stride, int nq, int nkv, int hd, int page_size, int window, float scale, void* scratch, long scratch_bytes, int max_ctx,
     int force_splits, int chunk, const float* sinks, const float* head_scale, const float* slopes, const float* gate, long ldg,
-    float softcap, int hdv, int v_share, int out_f32, long k_ld, long v_ld, const void* egate, long ldeg, cudaStream_t stream) {
+    float softcap, int hdv, int v_share, int out_f32, long k_ld, long v_ld, const void* egate, long ldeg, int table_made, cudaStream_t stream) {
     const HeadTerms ht{head_scale, slopes, gate, ldg, softcap > 0.f ? softcap : 0.f};
     if (num_tiles <= 0) return 0;
     if (chunk < 0) return AIEN_E_SHAPE;
@@ -729,7 +735,7 @@ AIEN_API int aien_paged_attention_prefill_tc_values(
         return AIEN_E_ALIGN;
     if (egate != nullptr && out_f32) return AIEN_E_SHAPE;
     if (force_splits < 0 || force_splits > PT_MAX_SPLITS) return AIEN_E_SHAPE;
-    const PtSizes sz{hdv, ((hd & 63) ? 1 : 0) | ((hdv & 63) ? 2 : 0), v_share, out_f32 ? 1 : 0, (const __nv_bfloat16*)egate, ldeg};
+    const PtSizes sz{hdv, ((hd & 63) ? 1 : 0) | ((hdv & 63) ? 2 : 0), v_share, out_f32 ? 1 : 0, (const __nv_bfloat16*)egate, ldeg, table_made};
     CUtensorMap mq;
     static PtMaps mk, mv;                      // large: kept out of the stack; filled for every launch
     static std::mutex mu;
@@ -776,7 +782,7 @@ AIEN_API int aien_paged_attention_prefill_tc_terms(
     return aien_paged_attention_prefill_tc_values(q, q_stride, q_rows, k_cache, v_cache, cache_rows, block_table, max_blocks, q_start, ctx_len,
                                                   tile_seq, tile_q0, num_tiles, out, out_stride, nq, nkv, hd, page_size, window, scale,
                                                   scratch, scratch_bytes, max_ctx, force_splits, chunk, sinks, head_scale, slopes, gate, ldg,
-                                                  softcap, hd, 1, 0, 0, 0, nullptr, 0, stream);
+                                                  softcap, hd, 1, 0, 0, 0, nullptr, 0, 0, stream);
 }
 
 AIEN_API int aien_paged_attention_prefill_tc_masked(

@@ -1534,7 +1534,7 @@ def portion_attention(ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ta
                       head_gate: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None) -> None:
     """Causal attention of the step's portions (not of its single tokens) over keys and values that lie in rows of their own:
     k [rows, heads*head_dim] and v [rows, heads*value_dim] bfloat16 with free row strides, in 128-row pages named by ``table``
-    [S, pages].  q [T, heads*head_dim] (row stride free), out bfloat16 [T, heads*value_dim].  ``head_gate`` float32 [T, heads]:
+    [S, pages], which a kernel of this step may have written (the attention reads none of it before the kernels ahead are done).  q [T, heads*head_dim] (row stride free), out bfloat16 [T, heads*value_dim].  ``head_gate`` float32 [T, heads]:
     head h's output times sigmoid(head_gate[t, h]); ``gate`` bfloat16 [T, heads*value_dim]: element by element."""
     _dev(q, k, v, table, out, sinks, head_gate, gate)
     tile_seq, tile_q0, n = ctx.prefill_tiles
@@ -1546,7 +1546,7 @@ def portion_attention(ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ta
         q, q.stride(0), q.shape[0], k, v, k.shape[0], table, table.shape[1], ctx.q_start, ctx.ctx_len, tile_seq,
         tile_q0, n, out, out.stride(0), heads, heads, head_dim, 128, window, float(scale), None, 0, int(ctx.max_ctx_len), 0, 0,
         sinks, None, None, head_gate, head_gate.stride(0) if head_gate is not None else 0, 0.0, value_dim, 1, 0, k.stride(0),
-        v.stride(0), gate, gate.stride(0) if gate is not None else 0, _stream()), "paged_attention_prefill_tc_values")
+        v.stride(0), gate, gate.stride(0) if gate is not None else 0, 1, _stream()), "paged_attention_prefill_tc_values")
 
 
 # ---------------------------------------------------------------------------- several residual streams, token shift
@@ -2215,7 +2215,7 @@ def capped_attention(ctx, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
                 ctx.ctx_len, tile_seq, tile_q0, n, out, out.stride(0), num_q_heads, num_kv_heads, head_dim,
                 group.page_size, window, float(scale), scratch, scratch.numel() * 4 if scratch is not None else 0,
                 int(ctx.max_ctx_len), 0, int(chunk), None, None, None, None, 0, float(softcap or 0.0), value_dim, int(v_share),
-                1 if out.dtype == torch.float32 else 0, 0, 0, None, 0, _stream()), "paged_attention_prefill_tc_values")
+                1 if out.dtype == torch.float32 else 0, 0, 0, None, 0, 0, _stream()), "paged_attention_prefill_tc_values")
         tokens, nd = ctx.single_tokens if ctx.single_tokens is not None else (None, 0)
         if nd > 0 and splits_ok:
             single_tokens(tokens, nd)

@@ -832,3 +832,69 @@ def test_latent_portions_with_a_rotated_part_expanded_and_absorbed(dim, rot, vdi
             H.assert_close(y, want, 3e-2, form)
     finally:
         K.LATENT_PORTIONS = saved
+
+
+@pytest.mark.parametrize("bring,held", [([300], [0]), ([130, 171], [40, 0]), ([700], [64]), ([1, 260, 40], [90, 0, 200])])
+def test_latent_portions_read_no_page_number_that_an_earlier_step_left(bring, held):
+    """The expanded form's page table is made by a kernel of the step two launches ahead of the attention.  With the table's room
+    holding zeros or other valid page numbers, and the step's launches queued behind work so that they follow one another
+    closely, the results are those of a step whose table was there before, to the bit."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    from aien_sovereign_core_mv_b200.parts import GroupView, RunBinding, StepContext, StepLimits, Workspace
+    from aien_sovereign_core_mv_b200.registry import make_part
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(sum(bring))
+    width, heads, r, rot, page, S, T = 256, 4, 64, 64, 16, len(bring), sum(bring)
+    part = make_part("mixer", "latent_attention", hidden_size=width, num_heads=heads, head_dim=128, rot_dim=rot, value_dim=128, kv_rank=r, q_rank=128, window=0,
+                     norm_eps=1e-5, position=make_part("position", "rotary", head_dim=rot, theta=10000.0, pairing="interleaved"))
+    part.bind({n: (torch.randn(shape, generator=g, device="cuda") * (shape[-1] ** -0.5 if kind == "matrix" else 1.0)).to(torch.bfloat16)
+               for n, (shape, kind) in part.param_shapes().items()})
+    h = torch.randn(T, width, generator=g, device="cuda").to(torch.bfloat16)
+    q0 = [sum(bring[:s]) for s in range(S + 1)]
+    pages = [(a + b + page - 1) // page for a, b in zip(bring, held)]
+    table = torch.full((S, max(pages)), -1, dtype=torch.int32, device="cuda")
+    for s in range(S):
+        table[s, :pages[s]] = torch.arange(sum(pages[:s]), sum(pages[:s + 1]), dtype=torch.int32, device="cuda").flip(0)
+    slots = torch.cat([table[s, p // page].long() * page + p % page for s in range(S) for p in [torch.arange(held[s], held[s] + bring[s], device="cuda")]])
+    first = torch.randn(1, sum(pages) * page, r + rot, generator=g, device="cuda").to(torch.bfloat16)
+    lim = StepLimits(max_tokens=T, max_seqs=S, max_context=max(a + b for a, b in zip(bring, held)), itemsize=2)
+    position = make_part("position", "rotary", head_dim=rot, theta=10000.0, pairing="interleaved")
+    ws = Workspace(position.step_workspace_bytes(T) + 4096, part.workspace_bytes(lim) + (1 << 16), torch.device("cuda"))
+    tiles = [(s, q) for s in range(S) for q in range(0, bring[s], K.PREFILL_TILE) if bring[s] > 1]
+    singles = [q0[s] for s in range(S) if bring[s] == 1]
+    need = part.cache_need()
+    store = first.clone()
+    fixed = dict(dtype=torch.bfloat16, num_tokens=T, num_seqs=S, token_ids=i32([0] * T), positions=i32([held[s] + i for s in range(S) for i in range(bring[s])]),
+                 seq_of_token=i32([s for s in range(S) for _ in range(bring[s])]), q_start=i32(q0), ctx_len=i32([a + b for a, b in zip(bring, held)]),
+                 groups=[GroupView(need.kind, page, need.window, table.shape[1], table, slots.to(torch.int32), {"latent": store})],
+                 workspace=ws, max_q_len=max(bring), max_ctx_len=lim.max_context, decode_only=False,
+                 prefill_tiles=(i32([s for s, _ in tiles]), i32([q for _, q in tiles]), len(tiles)), single_tokens=(i32(singles or [0]), len(singles)))
+    busy = torch.randn(4096, 4096, device="cuda").to(torch.bfloat16)
+    words = ws.buf.view(torch.int32)
+    other = torch.arange(words.numel(), dtype=torch.int32, device="cuda").flip(0) % (sum(pages) * page // 128)
+
+    def step(left):
+        store.copy_(first)
+        if left is not None:
+            words.copy_(left)
+        ws.reset()
+        ws.begin_layer()
+        torch.cuda.synchronize()
+        for _ in range(8):                                   # the step's launches wait behind this, and then start as close together as they can
+            busy @ busy
+        y = part.forward(StepContext(**fixed), h, RunBinding(0, 0, True))
+        y = (y.float().sum(0) if y.dim() == 3 else y.float()).clone()
+        torch.cuda.synchronize()
+        return y, store.clone()
+
+    saved = K.LATENT_PORTIONS
+    try:
+        K.LATENT_PORTIONS = "expand"
+        step(torch.zeros_like(words))
+        want = step(None)                                    # the table of the step before, which is this step's too
+        assert bool(torch.isfinite(want[0]).all())
+        for left in (torch.zeros_like(words), other, torch.full_like(words, 0x7fff7fff)):
+            got = step(left)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    finally:
+        K.LATENT_PORTIONS = saved
