@@ -197,7 +197,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     auto slot_addr = [&](int slot) { return slot < S::SLOTS ? sKV + slot * S::SLOT_BYTES : sQ + S::Q_BYTES; };
 
     if (nb <= 0) {
-        // an empty range: weight zero in the merge
+        // an empty range: weight zero in the merge.  It has nothing to wait for but must wait: kernels ahead may still use the scratch's memory.
+        griddep_wait();
         if (warp < 8 && (warp < 4 || has_b)) {
             const int h = warp >> 2, r = (warp & 3) * 32 + lane;
             float* ml = part_ml + ((((size_t)tile * PT_BM + r) * nq + head_a + h) * nsplit + split) * 2;

@@ -828,6 +828,39 @@ def test_paged_attention_prefill_keys_cut_into_ranges(K, nq, nkv, hd, page, wind
     _prefill_case(K, nq, nkv, hd, page, window, [130, 64, 300, 5, 200, 1000, 700], [130, 1, 77, 2, 128, 333, 700], "tc", splits=splits)
 
 
+def test_paged_attention_prefill_empty_ranges_write_nothing_before_the_kernels_ahead_are_done(K):
+    """A product whose left operand lies where the attention's scratch has the weights of its ranges (as a layer's buffers lie where
+    those of a layer before it lay), and behind it the attention with six of eight ranges empty: the product's result is the one
+    that it has alone, to the bit."""
+    nq, nkv, hd, page, splits, seq_lens = 8, 2, 128, 16, 8, [130, 128, 120, 100]
+    rng = np.random.default_rng(11)
+    kc, vc, bt, mb, _ = paged_setup(rng, seq_lens, nkv, hd, page, torch.bfloat16, sum((n + page - 1) // page for n in seq_lens) + 8)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    tiles = len(seq_lens)
+    ql = [min(n, K.PREFILL_TILE) for n in seq_lens]
+    q_start = [sum(ql[:s]) for s in range(tiles + 1)]
+    q = torch.randn(sum(ql), nq * hd, device="cuda").to(torch.bfloat16)
+    out = torch.empty_like(q)
+    rows = tiles * K.PREFILL_TILE * nq * splits
+    scratch = torch.zeros(rows * (hd + 2), device="cuda")
+    a = scratch[rows * hd:].view(torch.bfloat16).view(16, -1)                # the ranges' maxima and sums
+    fill = torch.randn(a.shape, device="cuda").to(torch.bfloat16)
+    w = torch.randn(512, a.shape[1], device="cuda").to(torch.bfloat16)
+    z, busy = torch.empty(16, 512, device="cuda"), torch.randn(4096, 4096, device="cuda").to(torch.bfloat16)
+    args = (q, kc, vc, bt, mb, i32(q_start), i32(seq_lens), i32(list(range(tiles))), i32([0] * tiles), tiles, out, nq, nkv, hd, page, 0, 0.1)
+    a.copy_(fill)
+    K.gemm_tc(a, w, z)
+    want = z.clone()
+    for _ in range(5):
+        a.copy_(fill)
+        busy @ busy                                                          # both launches wait behind this, and then start close together
+        K.gemm_tc(a, w, z)
+        K.paged_attention_prefill(*args, impl="tc", scratch=scratch, max_ctx=max(seq_lens), splits=splits)
+        torch.cuda.synchronize()
+        assert K.attention_prefill_tc_error() == 0
+        assert torch.equal(z, want)
+
+
 def test_paged_attention_prefill_chooses_ranges_for_few_tiles_over_a_long_context(K):
     """The launch's own choice: 256 tokens at the end of 4,200 are two tiles of 16 pairs each, which it
     cuts into ranges when it is given the room; the result is the same as without."""
