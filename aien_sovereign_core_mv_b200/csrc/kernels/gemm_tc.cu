@@ -1027,7 +1027,7 @@ static int tc_plan(int M, int N, int ranges) {
 // for plain results (epilogue 0).  Float32, 256 columns and this rule: 2,048 x 8,192 x 2,048 54.8 and 50.3 us (224), 700 x 8,192 x
 // 2,048 30.5 and 24.7 (192); bfloat16 2,048 x 3,072 x 1,536 26.3 (128 x 256) and 20.7 (192).  208 and 176 columns measured slower
 // than either neighbour.  AIEN_B200_GEMM_TC=m256 | p256 pins it (m256: 256 wide).
-static int tc_m256_cols(int M, int N, int K, int ranges, bool f32 = false, bool plain = true) {
+static int tc_m256_cols(int M, int N, int K, int ranges, bool f32, bool plain) {
     static int forced = -1;
     if (forced < 0) {
         const char* e = getenv("AIEN_B200_GEMM_TC");
@@ -1176,11 +1176,12 @@ AIEN_API int aien_gemm_tc_ranges(int K, int splits) {
     return (total_kb + kb_per_split - 1) / kb_per_split;
 }
 
-// Whether aien_gemm_tc runs this product on the persistent kernel with tiles of 256 x 256 (1) or not (0).
-AIEN_API int aien_gemm_tc_m256_supports(int M, int N, int K, int splits) {
+// How wide the 256-row tiles are in which aien_gemm_tc runs this product with these results (256, 240, 224 or 192 columns), 0 where it
+// takes others.
+AIEN_API int aien_gemm_tc_m256_supports(int M, int N, int K, int splits, int c_dt, int epilogue) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     const int ranges = aien_gemm_tc_ranges(K, splits);
-    return (tc_plan(M, N, ranges) == 256 && tc_m256_cols(M, N, K, ranges) > 0) ? 1 : 0;
+    return tc_plan(M, N, ranges) == 256 ? tc_m256_cols(M, N, K, ranges, c_dt == AIEN_DT_F32, epilogue == 0) : 0;
 }
 
 AIEN_API int aien_gemm_tc(const void* A, long lda, const void* W, long ldw, void* out, int c_dt, long ldc,
@@ -1194,7 +1195,7 @@ AIEN_API int aien_gemm_tc(const void* A, long lda, const void* W, long ldw, void
     if (epilogue == 2 || epilogue == 3 || epilogue == 4 || epilogue == 6) {   // gelu (erf / tanh form) or relu squared of every value, bfloat16 out, K in one range
         if (c_dt != AIEN_DT_BF16 || splits != 1) return AIEN_E_SHAPE;
         const int plan = tc_plan(M, N, 1);
-        const int wide = plan == 256 ? tc_m256_cols(M, N, K, 1, false, false) : 0;
+        const int wide = aien_gemm_tc_m256_supports(M, N, K, 1, c_dt, epilogue);
         if (epilogue == 2) {
             if (wide > 0) return launch_tc_persistent_m256<2, __nv_bfloat16>(wide, A, lda, W, ldw, out, ldc, M, N, K, stream);
             if (plan == 256) return launch_tc_persistent<256, 2, __nv_bfloat16>(A, lda, W, ldw, out, ldc, M, N, K, 1, 0, stream);
@@ -1217,7 +1218,7 @@ AIEN_API int aien_gemm_tc(const void* A, long lda, const void* W, long ldw, void
     if (epilogue == 0 || epilogue == 1) {
         const int plan = tc_plan(M, N, aien_gemm_tc_ranges(K, splits));
 #define TCP_CASE(BNV, EPIV, T) return launch_tc_persistent<BNV, EPIV, T>(A, lda, W, ldw, out, ldc, M, N, K, splits, part_stride, stream)
-        const int wide = plan == 256 ? tc_m256_cols(M, N, K, aien_gemm_tc_ranges(K, splits), c_dt == AIEN_DT_F32, epilogue == 0) : 0;
+        const int wide = aien_gemm_tc_m256_supports(M, N, K, splits, c_dt, epilogue);
         if (wide > 0) {
             if (epilogue == 0 && c_dt == AIEN_DT_BF16) return launch_tc_persistent_m256<0, __nv_bfloat16>(wide, A, lda, W, ldw, out, ldc, M, N, K, stream);
             if (epilogue == 0 && c_dt == AIEN_DT_F32) return launch_tc_persistent_m256<0, float>(wide, A, lda, W, ldw, out, ldc, M, N, K, stream);

@@ -737,9 +737,14 @@ def gemm_tc_ranges(K_: int, splits: int) -> int:
     return int(lib().aien_gemm_tc_ranges(int(K_), int(splits)))
 
 
-def gemm_tc_takes_256_rows(M: int, N: int, K_: int, splits: int = 1) -> bool:
-    """Whether gemm_tc runs this product on the persistent kernel with tiles of 256 x 256."""
-    return bool(lib().aien_gemm_tc_m256_supports(int(M), int(N), int(K_), int(splits)))
+def gemm_tc_256_rows_cols(M: int, N: int, K_: int, splits: int = 1, dtype: torch.dtype = torch.bfloat16, epilogue: int = 0) -> int:
+    """How wide the tiles of 256 rows are in which gemm_tc runs this product with results of this type and epilogue (0: other tiles)."""
+    return int(lib().aien_gemm_tc_m256_supports(int(M), int(N), int(K_), int(splits), _DT[dtype], int(epilogue)))
+
+
+def gemm_tc_takes_256_rows(M: int, N: int, K_: int, splits: int = 1, dtype: torch.dtype = torch.bfloat16, epilogue: int = 0) -> bool:
+    """Whether gemm_tc runs this product on the persistent kernel with tiles of 256 rows."""
+    return gemm_tc_256_rows_cols(M, N, K_, splits, dtype, epilogue) > 0
 
 
 def gemm_tc_splits(M: int, N: int, K_: int) -> int:

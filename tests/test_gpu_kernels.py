@@ -695,13 +695,16 @@ def test_gemm_tensor_core_with_k_shared_in_a_cluster(K, M, N, K_, epilogue):
 
 
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("M,N,K_", [(512, 18944, 2048), (4096, 4112, 1032), (2900, 5000, 1032)])      # tiles 256, 240 and 224 wide
-def test_gemm_tensor_core_tiles_of_256_rows(K, M, N, K_, out_dtype):
+@pytest.mark.parametrize("M,N,K_,cols", [(512, 18944, 2048, {torch.bfloat16: 256, torch.float32: 256}), (4096, 4112, 1032, {torch.bfloat16: 240, torch.float32: 0}),
+                                         (2900, 5000, 1032, {torch.bfloat16: 224, torch.float32: 224})])
+def test_gemm_tensor_core_tiles_of_256_rows(K, M, N, K_, cols, out_dtype):
     """Products that the persistent kernel takes with tiles of 256 x 256 (two accumulators side by side,
-    eight epilogue warps), 256, 240 or 224 columns wide as makes the shortest waves: a last row tile of 84
+    eight epilogue warps), 256, 240 or 224 columns wide as makes the shortest waves (``cols``; float32 results
+    have no 240 and take tiles of 128 rows there): a last row tile of 84
     rows, widths that are no multiple of the tile or of a chunk of 32 columns, a K that is no multiple of
     the k-block, two tiles per CTA (the accumulators handed back and forth)."""
-    assert K.gemm_tc_takes_256_rows(M, N, K_) and not K.gemm_tc_takes_256_rows(2048, 6144, 4096) and not K.gemm_tc_takes_256_rows(128, 24576, 4096)
+    assert K.gemm_tc_256_rows_cols(M, N, K_, dtype=out_dtype) == cols[out_dtype]
+    assert not K.gemm_tc_takes_256_rows(2048, 6144, 4096, dtype=out_dtype) and not K.gemm_tc_takes_256_rows(128, 24576, 4096, dtype=out_dtype)
     g = torch.Generator().manual_seed(M + N)
     a = torch.randn(M, K_, generator=g).to(torch.bfloat16).cuda()
     w = (torch.randn(N, K_, generator=g) / math.sqrt(K_)).to(torch.bfloat16).cuda()
@@ -715,11 +718,11 @@ def test_gemm_tensor_core_tiles_of_256_rows(K, M, N, K_, out_dtype):
     assert (out_full[:, N:] == 9.0).all()
 
 
-@pytest.mark.parametrize("M,N,K_", [(2000, 8168, 1032), (700, 8188, 1544), (2048, 3050, 712)])
-def test_gemm_tensor_core_widths_of_256_rows_float32(K, M, N, K_):
-    """Float32 results in tiles of 224 and 192 columns (boxes of 32 columns by TMA, and rows that are no whole 16-byte pieces by plain
-    stores), bfloat16 results in tiles of 192; ragged last tiles either way, two waves and one."""
-    assert K.gemm_tc_takes_256_rows(M, N, K_)
+@pytest.mark.parametrize("M,N,K_,cols", [(2000, 8168, 1032, 224), (700, 8188, 1544, 192), (2048, 3050, 712, 192)])
+def test_gemm_tensor_core_widths_of_256_rows_float32(K, M, N, K_, cols):
+    """Float32 and bfloat16 results in tiles of 224 and 192 columns (boxes of 32 columns by TMA, and rows that are no whole 16-byte
+    pieces by plain stores); ragged last tiles either way, two waves and one."""
+    assert K.gemm_tc_256_rows_cols(M, N, K_, dtype=torch.float32) == K.gemm_tc_256_rows_cols(M, N, K_, dtype=torch.bfloat16) == cols
     g = torch.Generator().manual_seed(M + N)
     a = torch.randn(M, K_, generator=g).to(torch.bfloat16).cuda()
     w = (torch.randn(N, K_, generator=g) / math.sqrt(K_)).to(torch.bfloat16).cuda()
@@ -736,7 +739,7 @@ def test_gemm_tensor_core_widths_of_256_rows_float32(K, M, N, K_):
 
 def test_gemm_tensor_core_tiles_of_256_rows_with_swiglu(K):
     M, I, Hd = 2900, 2504, 1032                     # tiles of 224 columns over 5,008: the last one 80 wide
-    assert K.gemm_tc_takes_256_rows(M, 2 * I, Hd)
+    assert K.gemm_tc_256_rows_cols(M, 2 * I, Hd, epilogue=1) == 224
     g = torch.Generator().manual_seed(3)
     a = torch.randn(M, Hd, generator=g).to(torch.bfloat16).cuda()
     gate = (torch.randn(I, Hd, generator=g) / math.sqrt(Hd)).to(torch.bfloat16)
