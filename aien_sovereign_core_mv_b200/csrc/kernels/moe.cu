@@ -39,13 +39,15 @@ constexpr int ROUTE_MAX_EXPERTS = 1024;
 // after another, and a choice is two warp reductions in hardware: the largest key (unsigned, in the order of the floats), then the
 // lowest expert that has it.  Before, every choice went through shared memory and ten shuffles, the weights back through global memory.
 // B200, us, before and so: 2,048 tokens, 6 of 64 experts in 4 of 8 groups 14.7 and 7.1; 8 of 256 20.4 and 12.5; 64 tokens, 6 of 64 6.5 and 2.6;
-// 9 tokens, 4 of 16 with sigmoid scores 3.3 and 1.6; 16 tokens, 8 of 1,024 7.4 and 5.3.  Choices and weights are the same to the bit.
+// 9 tokens, 4 of 16 with sigmoid scores 3.3 and 1.6; 16 tokens, 8 of 1,024 7.4 and 5.3.  Choices and weights of numbers are the same to the bit.
 constexpr int ROUTE_WARPS = 4;                                            // tokens per CTA
-constexpr uint32_t ROUTE_TAKEN = 0;                                       // below the key of every float
+constexpr uint32_t ROUTE_TAKEN = 0, ROUTE_OUT = 1, ROUTE_NAN = 2;         // chosen before, not eligible, not a number: below the key of every float
 
+// The order of the floats.  What is not a number is chosen only when no number is left, whatever its sign: one expert's NaN does not
+// reach the weights of a token that has numbers to choose from.
 __device__ __forceinline__ uint32_t route_key(float v) {
     const uint32_t u = __float_as_uint(v + 0.0f);                         // -0 and 0 are one
-    return (u & 0x80000000u) != 0 ? ~u : u | 0x80000000u;
+    return v != v ? ROUTE_NAN : (u & 0x80000000u) != 0 ? ~u : u | 0x80000000u;
 }
 
 // The largest key's index (ties to the lower), which is then taken.
@@ -134,7 +136,7 @@ moe_route_kernel(const float* __restrict__ z, int T, int E, int groups, int keep
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < NR; ++j)
-            if (lane + 32 * j < E && !id_at[(lane + 32 * j) / per]) key[j] = route_key(-1.0f);      // below every score
+            if (lane + 32 * j < E && !id_at[(lane + 32 * j) / per]) key[j] = ROUTE_OUT;
         __syncwarp();
     }
     float wsum = 0.f;

@@ -418,6 +418,38 @@ def test_routers_of_every_width(E, groups, keep, top):
     assert counts.cpu().tolist() == np.bincount(np.where(choice < real, choice, 0).ravel(), minlength=E).tolist()
 
 
+@pytest.mark.parametrize("E,top", [(5, 2), (40, 4), (300, 8)])
+def test_routers_pass_over_what_is_not_a_number(E, top):
+    """A NaN of either sign among a token's scores, or in the correction, is chosen only after every number; the other choices and the
+    weights are those of a token whose expert cannot be chosen.  A row without a number still gets experts that exist."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator().manual_seed(E)
+    T = 7
+    z = torch.randn(T, E, generator=g)
+    at = torch.randint(0, E, (T,), generator=g)
+    nan = torch.tensor([0x7fc00000, -4194304], dtype=torch.int32).view(torch.float32)          # both signs
+    low = z.clone()
+    for t in range(T - 1):
+        z[t, at[t]], low[t, at[t]] = nan[t % 2], -float("inf")
+    z[T - 1], low[T - 1] = nan[0], 0.0
+    ids, wts, same = torch.zeros(T, top, dtype=torch.int32).cuda(), torch.zeros(T, top).cuda(), torch.zeros(T).cuda()
+    for corr in (None, torch.zeros(E)):
+        K.moe_route_biased(z.cuda(), E, E, top, True, 0.0, None if corr is None else corr.cuda(), ids, wts, same, None, sigmoid=True)
+        choice = np.argsort(-f64(low), axis=-1, kind="stable")[:, :top]
+        w = np.take_along_axis(pk.sigmoid(f64(low)), choice, -1)
+        assert (ids.cpu().numpy() == choice).all()
+        H.assert_close(wts[:-1].cpu().numpy(), (w / w.sum(-1, keepdims=True))[:-1], 1e-5, "weights")
+    # the correction of one expert is no number; softmax scores, which one NaN makes NaN all of them, choose the lowest experts
+    corr = torch.zeros(E)
+    corr[int(at[0])] = nan[1]
+    K.moe_route_biased(z[1:2].nan_to_num(0.0).cuda(), E, E, top, True, 0.0, corr.cuda(), ids[:1], wts[:1], same, None, sigmoid=True)
+    score = f64(z[1:2].nan_to_num(0.0))
+    score[0, int(at[0])] = -np.inf
+    assert (ids[:1].cpu().numpy() == np.argsort(-pk.sigmoid(score), axis=-1, kind="stable")[:, :top]).all()
+    K.moe_route(z.cuda(), 1, 1, top, True, ids, wts)
+    assert (ids.cpu().numpy() == np.arange(top)).all()
+
+
 @pytest.mark.parametrize("E,top,T,D,F_", [(16, 4, 9, 2048, 1024), (5, 3, 16, 200, 24), (64, 6, 16, 512, 136), (8, 2, 5, 1032, 40), (3, 3, 16, 72, 8), (20, 16, 16, 64, 1024)])
 @pytest.mark.parametrize("gated", [True, False])
 def test_experts_of_a_few_tokens_share_their_rows(E, top, T, D, F_, gated):
