@@ -19,6 +19,7 @@ fallback path.
 from __future__ import annotations
 
 import ctypes
+import functools
 import glob
 import hashlib
 import importlib.util
@@ -28,6 +29,7 @@ import subprocess
 import sys
 import sysconfig
 import tempfile
+import threading
 import time
 from typing import List, Optional
 
@@ -89,6 +91,18 @@ def sanitizer_preload() -> Optional[str]:
 
 class BuildError(RuntimeError):
     pass
+
+
+_LOCK = threading.RLock()
+
+
+def _one_thread(fn):
+    """One thread at a time builds or loads: files on the way are named by the process, and a thread that comes later finds the artefact."""
+    @functools.wraps(fn)
+    def locked(*args, **kwargs):
+        with _LOCK:
+            return fn(*args, **kwargs)
+    return locked
 
 
 def _say(msg: str) -> None:
@@ -165,6 +179,7 @@ def _run_parallel(cmds: List[List[str]], what: str, jobs: int) -> None:
             time.sleep(0.1)
 
 
+@_one_thread
 def build_kernels(force: bool = False) -> str:
     """Compile every kernel source for sm_100a and link ``libaien_kernels.so``; returns its path."""
     out_dir = build_dir()
@@ -198,6 +213,7 @@ def _host_ext_name() -> str:
     return "_aien_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
 
 
+@_one_thread
 def build_host(force: bool = False) -> str:
     """Compile the C++ cache manager and scheduler into a pybind11 module; returns its path."""
     out_dir = build_dir()
@@ -246,6 +262,7 @@ def _launch_table() -> str:
     return "".join(rows)
 
 
+@_one_thread
 def build_launch(force: bool = False) -> str:
     """Compile the callers of the kernels' entry points into a Python module; returns its path."""
     import torch                                               # its headers, and the libraries that the module resolves against
@@ -286,6 +303,7 @@ _LAUNCH = None
 _HOST = None
 
 
+@_one_thread
 def load_kernels() -> ctypes.CDLL:
     global _KERNELS
     if _KERNELS is None:
@@ -293,6 +311,7 @@ def load_kernels() -> ctypes.CDLL:
     return _KERNELS
 
 
+@_one_thread
 def load_launch():
     global _LAUNCH
     if _LAUNCH is None:
@@ -305,6 +324,7 @@ def load_launch():
     return _LAUNCH
 
 
+@_one_thread
 def load_host():
     global _HOST
     if _HOST is None:

@@ -1,5 +1,8 @@
 """The native callers of the kernels' entry points on the CPU: a ctypes callback stands in for an entry point."""
 import ctypes
+import os
+import threading
+import time
 
 import pytest
 import torch
@@ -64,3 +67,36 @@ def test_strided_is_as_strided():
                 strided(t, shape, strides, at)
     v = strided(torch.full((8,), 3.0), (8,), (1,), 0)          # the view keeps the storage
     assert torch.equal(v, torch.full((8,), 3.0))
+
+
+def test_two_threads_build_the_callers_at_the_same_time(monkeypatch, tmp_path):
+    """Neither takes the other's work folder away; the compiler is a stand-in that reads its table at the end too, the second later than the first."""
+    monkeypatch.setenv("AIEN_B200_BUILD_DIR", str(tmp_path))
+    runs, made, errors = [], [], []
+
+    def compiler(cmds, what, jobs):
+        runs.append(what)
+        table = os.path.join(cmds[0][cmds[0].index("-I") + 1], "signatures.inc")
+        assert os.path.exists(table)
+        time.sleep(0.1 if len(runs) == 1 else 0.4)
+        assert os.path.exists(table)
+        with open(cmds[0][cmds[0].index("-o") + 1], "w") as f:
+            f.write(what)
+
+    monkeypatch.setattr(build, "_run_parallel", compiler)
+    start = threading.Barrier(2)
+
+    def thread():
+        try:
+            start.wait(10)
+            made.append(build.build_launch(force=True))
+        except BaseException as e:                             # noqa: BLE001  (told below)
+            errors.append(e)
+
+    threads = [threading.Thread(target=thread) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(30)
+    assert not errors and len(made) == 2 and made[0] == made[1] and open(made[0]).read() == "launch" and len(runs) == 2
+    assert sorted(os.path.basename(p) for p in os.listdir(tmp_path)) == sorted(os.path.basename(made[0]) + e for e in ("", ".stamp"))
