@@ -1898,8 +1898,8 @@ def selective_scan_segments(num_tokens: int, num_seqs: int, decode_only: bool, i
         6,144          45 and 56      88 and 97      171 and 179
 
     and 4,096 channels of requests of 1,500 and 500 tokens (2,048 channels each) 96 and 73.  With more than 16 states, or 8 and fewer, whose
-    forms have other lanes, only steps of few channels are cut.  It depends on the step's token and request counts and
-    the layer's sizes alone."""
+    forms have other lanes, only steps of few channels are cut, in segments of 128 tokens from an average of 1,024 on.  It depends on
+    the step's token and request counts and the layer's sizes alone."""
     average, channels = num_tokens // max(num_seqs, 1), inner * num_seqs
     if 8 < state <= 16:
         least = 256 if channels <= 512 else 512 if channels <= 3072 else 1000
@@ -1908,11 +1908,13 @@ def selective_scan_segments(num_tokens: int, num_seqs: int, decode_only: bool, i
         least, limit = 256, 1024 if average >= 1024 else 512
     if decode_only or channels > limit or average < least:
         return 0, 1
-    seg = 128 if average >= SCAN_LONG_PORTION else 64
+    seg = 128 if average >= _scan_long_portion(state) else 64
     return seg, -(-num_tokens // seg)
 
 
-SCAN_LONG_PORTION = 1500             # tokens a request on the average, from which the scan's segments are 128 tokens long instead of 64
+def _scan_long_portion(state: int) -> int:
+    """Tokens a request on the average, from which the scan's segments are 128 tokens long instead of 64."""
+    return 1500 if 8 < state <= 16 else 1024
 
 
 def selective_scan_scratch(max_tokens: int, max_seqs: int, inner: int, N: int) -> int:
@@ -1920,7 +1922,7 @@ def selective_scan_scratch(max_tokens: int, max_seqs: int, inner: int, N: int) -
     seqs = min(max_seqs, (4096 if 8 < N <= 16 else 1024) // inner)        # a step of more requests is not cut
     if seqs <= 0:
         return 0
-    segments = max(max_tokens // 128, min(max_tokens, SCAN_LONG_PORTION * seqs) // 64)
+    segments = max(max_tokens // 128, min(max_tokens, _scan_long_portion(N) * seqs) // 64)
     return 2 * (segments + seqs) * inner * N
 
 

@@ -97,3 +97,23 @@ def test_refusals(path, value, word):
     with pytest.raises(ConfigError) as e:
         model_spec_for(c)
     assert word in str(e.value)
+
+
+@pytest.mark.parametrize("state", [1, 4, 8, 9, 16, 17, 32, 128])
+def test_segments_of_the_selective_scan_and_their_scratch(state):
+    """Other state counts than 9 to 16 are cut as their own forms were measured: 128 tokens from an average of 1,024 on, 64 below, few
+    channels only.  The scratch bound covers every step up to its limits, whichever lengths were chosen."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    for inner in (24, 64, 256, 512, 1000, 1024, 2048, 4096, 5000):
+        for max_seqs in (1, 3, 40):
+            for max_tokens in (64, 300, 1023, 1024, 1500, 4096, 8192):
+                room = K.selective_scan_scratch(max_tokens, max_seqs, inner, state)
+                for S in range(1, max_seqs + 1):
+                    for T in sorted({t for t in (S, 256 * S, 256 * S + 1, 511 * S, 1000 * S, 1023 * S, 1024 * S, 1499 * S, 1500 * S - 1, 1500 * S, max_tokens) if S <= t <= max_tokens}):
+                        seg, most = K.selective_scan_segments(T, S, T == S, inner, state)
+                        if not 8 < state <= 16:
+                            average = T // S
+                            cut = T != S and inner * S <= (1024 if average >= 1024 else 512) and average >= 256
+                            assert seg == ((128 if average >= 1024 else 64) if cut else 0), (T, S, inner)
+                        if seg:
+                            assert most * seg >= T and 2 * (T // seg + S) * inner * state <= room, (T, S, inner)
