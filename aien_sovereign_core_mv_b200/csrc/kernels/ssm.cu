@@ -189,7 +189,7 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
             if (FIRST) dts += dd.x;
             if (CH % 2 == 0) {
                 float2 ys = make_float2(0.f, 0.f);
-                float bv[CH], cv[CH];
+                __align__(16) float bv[CH], cv[CH];
 #pragma unroll
                 for (int i = 0; i < CH; i += CH % 4 == 0 ? 4 : 2) {
                     if (CH % 4 == 0) {
