@@ -461,21 +461,24 @@ moe_expert_rows_bf16_kernel(const __nv_bfloat16* __restrict__ x, long x_stride, 
 // it, sixteen at a time (a token chooses an expert once, but choices without tensors of their own arrive as expert 0 with
 // weight zero), each of its four warps a quarter of the columns, on the tensor cores
 // (mma.sync.m16n8k16, rows of W on the left, pairs on the right; both sides' columns in the order in which 16-byte loads give them).
-// Sixteen products start from zero and are added to the sums by float32 additions, and the quarters are added in order: the
-// rounding of float32 multiply-adds.  A CTA finds its pairs in the list of choices and leaves where there are none; `early`: the first
+// Sixteen products start from zero, eight of their sums meet in a tree, the trees (128 columns each) are added in float32, and so are the
+// quarters, with what the tensor core cuts off a sum on the average added back.  Relative 2-norm of the down product's results against 64 bits,
+// a row a pair and so: K = 1,024 6.7e-8 and 6.7e-8, 2,048 7.5e-8 and 7.3e-8, 4,096 8.7e-8 and 8.5e-8; numbers of one sign, K = 2,048
+// 3.1e-8 and 2.9e-8 (every sum of sixteen added to one accumulator: 8.7e-8, 1.1e-7, 1.6e-7 and 5.4e-8).
+// A CTA finds its pairs in the list of choices and leaves where there are none; `early`: the first
 // columns of W are asked for before the kernel ahead has made the choices (where most experts are chosen).
 // What bounds moe_expert_rows_bf16_kernel is instructions: two a number of W and pair (9 tokens, 4 of 16 gated experts of 2,048 x
 // 1,024, 36 pairs: 33.6 and 31.6 us for the two products of 124 and 62 MB); 24 and 15 so.
 constexpr int ET_WARPS = 4, ET_PAIRS = 16, ET_LIST = 256;       // pairs at a time; most pairs of a step
 constexpr int ET_U = 2;                                         // k-steps of 64 whose loads are in flight together
+constexpr float ET_LOST = 1.6e-8f;                              // what the tensor core cuts off a sum of sixteen products, on the average of its size
 
-__device__ __forceinline__ void et_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    float d[4] = {0.f, 0.f, 0.f, 0.f};
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-#pragma unroll
-    for (int e = 0; e < 4; ++e) c[e] += d[e];
+// sixteen products, from zero
+__device__ __forceinline__ void et_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    d[0] = d[1] = d[2] = d[3] = 0.f;
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 struct EtTile { uint4 w[2][2]; };                               // row g, row g + 8; columns 16 c .. 16 c + 7, .. + 15 of a k-step
@@ -489,18 +492,29 @@ __device__ __forceinline__ void et_load(EtTile& t, const __nv_bfloat16* r0, cons
     }
 }
 
-// MODE as for moe_expert_rows_bf16_kernel.  NT: eights of pairs.
+// The sums of ET_U k-steps' products, made from zero in a tree, are added to acc.  MODE as for moe_expert_rows_bf16_kernel.  NT: eights of pairs.
 template <int NT>
-__device__ __forceinline__ void et_products(float (&acc)[NT][4], const EtTile& t, const __nv_bfloat16* const (&xr)[NT], int k, int K) {
+__device__ __forceinline__ void et_products(float (&acc)[NT][4], const EtTile (&t)[ET_U], const __nv_bfloat16* const (&xr)[NT], const int (&k)[ET_U], int K) {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int nt = 0; nt < NT; ++nt) {
+        float sum[ET_U][4];
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const bool in = xr[nt] != nullptr && k + 8 * p < K;
-            const uint4 x = in ? __ldcg(reinterpret_cast<const uint4*>(xr[nt] + k + 8 * p)) : make_uint4(0u, 0u, 0u, 0u);
-            et_mma(acc[nt], t.w[0][p].x, t.w[1][p].x, t.w[0][p].y, t.w[1][p].y, x.x, x.y);
-            et_mma(acc[nt], t.w[0][p].z, t.w[1][p].z, t.w[0][p].w, t.w[1][p].w, x.z, x.w);
+        for (int u = 0; u < ET_U; ++u) {
+            float d[2][2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const bool in = xr[nt] != nullptr && k[u] + 8 * p < K;
+                const uint4 x = in ? __ldcg(reinterpret_cast<const uint4*>(xr[nt] + k[u] + 8 * p)) : make_uint4(0u, 0u, 0u, 0u);
+                et_mma(d[p][0], t[u].w[0][p].x, t[u].w[1][p].x, t[u].w[0][p].y, t[u].w[1][p].y, x.x, x.y);
+                et_mma(d[p][1], t[u].w[0][p].z, t[u].w[1][p].z, t[u].w[0][p].w, t[u].w[1][p].w, x.z, x.w);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[u][e] = (d[0][0][e] + d[0][1][e]) + (d[1][0][e] + d[1][1][e]);
         }
+        static_assert(ET_U == 2, "two sums");
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[nt][e] += sum[0][e] + sum[1][e];
+    }
 }
 
 template <int MODE, int NT>
@@ -519,13 +533,14 @@ __device__ __forceinline__ void et_serve(const __nv_bfloat16* __restrict__ x, lo
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
     for (int s = s0; s < s1; s += ET_U) {
         EtTile t[ET_U];
+        int k[ET_U];
 #pragma unroll
         for (int u = 0; u < ET_U; ++u) {
+            k[u] = s + u < s1 ? (s + u) * 64 + c * 16 : K;
             if (early && s == s0) t[u] = first[u];
-            else et_load(t[u], r0, r1, s + u < s1 ? (s + u) * 64 + c * 16 : K, K);
+            else et_load(t[u], r0, r1, k[u], K);
         }
-#pragma unroll
-        for (int u = 0; u < ET_U; ++u) et_products<NT>(acc, t[u], xr, s + u < s1 ? (s + u) * 64 + c * 16 : K, K);
+        et_products<NT>(acc, t, xr, k, K);
     }
     // [quarter][nt][e][lane]: thread (warp e, lane) adds the four quarters of its value; silu(gate) * up wants e and e + 2
 #pragma unroll
@@ -534,10 +549,11 @@ __device__ __forceinline__ void et_serve(const __nv_bfloat16* __restrict__ x, lo
         for (int e = 0; e < 4; ++e) red[((warp * NT + nt) * 4 + e) * 32 + lane] = acc[nt][e];
     __syncthreads();
     auto total = [&](int nt, int e) {
-        float v = 0.f;
-#pragma unroll
-        for (int z = 0; z < ET_WARPS; ++z) v += red[((z * NT + nt) * 4 + e) * 32 + lane];
-        return v;
+        const float* q = red + (nt * 4 + e) * 32 + lane;
+        static_assert(ET_WARPS == 4, "four quarters");
+        const float a = q[0] + q[NT * 128], b = q[2 * NT * 128] + q[3 * NT * 128], v = a + b, held = v - a;
+        // with what a + b lost to rounding, so that less than half of a last place counts; an infinite sum stays one
+        return fabsf(v) <= 3.402823466e38f ? v + fmaf(ET_LOST, v, (a - (v - held)) + (b - held)) : v;
     };
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {

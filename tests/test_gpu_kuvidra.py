@@ -488,6 +488,42 @@ def test_experts_of_a_few_tokens_share_their_rows(E, top, T, D, F_, gated):
                 H.assert_close(parts[c, t].cpu().numpy(), want, 1.5e-2, f"token {t}, choice {c}")
 
 
+@pytest.mark.parametrize("E,top,T,D,F_", [(16, 4, 9, 2048, 1024), (64, 6, 16, 2048, 768), (16, 4, 16, 1024, 2048), (8, 4, 16, 512, 4096)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "spread"])
+def test_experts_that_share_their_rows_are_as_near_to_64_bits_as_a_row_a_pair(E, top, T, D, F_, kind):
+    """The float32 results of the down product with an expert's matrix once for its pairs, and of the same numbers a row a pair (which 65
+    experts take): a relative 2-norm no larger, and 2 % for the luck of the draw (n results of independent rounding scatter by 1 / sqrt(2 n))."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(E + F_)
+    x, w = torch.randn(T * top, F_, generator=g, device="cuda"), torch.randn(65, D, F_, generator=g, device="cuda") / F_ ** 0.5
+    if kind == "positive":
+        x, w = x.abs(), w.abs()
+    if kind == "spread":
+        x = x * torch.exp2(torch.randint(-8, 9, x.shape, generator=g, device="cuda").float())
+    x, w = x.to(torch.bfloat16), w.to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, generator=g, device="cuda")[:top] for _ in range(T)]).to(torch.int32)
+    want = torch.einsum("pnf,pf->pn", w[ids.flatten().long()].double(), x.double()).view(T, top, D).transpose(0, 1)
+    off = []
+    for experts in (E, 65):
+        parts = torch.full((top, T, D), 7.0, device="cuda")
+        K._check(K.lib().aien_moe_expert_rows_bf16(1, x, F_, w, ids, None, parts, T, top, experts, D, F_, 0, 0, K._stream()), "moe_expert_rows(down)")
+        off.append(float((parts.double() - want).norm() / want.norm()))
+    assert off[0] <= 1.02 * off[1], off
+
+
+def test_an_infinite_sum_of_experts_that_share_their_rows_stays_infinite():
+    from aien_sovereign_core_mv_b200 import kernels as K
+    T, top, E, D, F_ = 4, 2, 4, 32, 64
+    x, w = torch.zeros(T * top, F_).to(torch.bfloat16).cuda(), torch.ones(E, D, F_).to(torch.bfloat16).cuda()
+    x[0, 3], x[1, 5] = float("inf"), -float("inf")
+    x[2, 0], x[2, 63] = float("inf"), -float("inf")
+    ids = torch.tensor([[0, 1]] * T, dtype=torch.int32).cuda()
+    parts = torch.zeros(top, T, D, device="cuda")
+    K._check(K.lib().aien_moe_expert_rows_bf16(1, x, F_, w, ids, None, parts, T, top, E, D, F_, 0, 0, K._stream()), "moe_expert_rows(down)")
+    y = parts.cpu().transpose(0, 1).reshape(T * top, D)
+    assert (y[0] == float("inf")).all() and (y[1] == -float("inf")).all() and y[2].isnan().all() and (y[3:] == 0).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("E,top,ff,shared", [(5, 3, 64, 72), (3, 1, 20, 0), (6, 6, 8, 40), (9, 2, 136, 24)])
 def test_gated_experts_with_the_weight_on_their_input(dtype, E, top, ff, shared):
