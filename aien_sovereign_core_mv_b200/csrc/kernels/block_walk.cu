@@ -26,9 +26,9 @@
 //
 // Relative error (2-norm) of the results and the last states against 64 bits, 2,048 tokens, and in brackets that of the
 // float32 kernels that go token by token or, for one decay per head, by chunks of 64:
-//   one decay per head, 1 - 2^-5 .. 1 - 2^-8          0.7e-7 and 0.8e-7  (1.7e-7 and 1.3e-7)
-//   one decay per head, 1 - 1e-4                      0.8e-7 and 1.7e-7  (2.7e-7 and 3.2e-7)
-//   duality, rows of silu, drawn step sizes           0.7e-7 and 1.0e-7  (0.9e-7 and 3.0e-7)
+//   one decay per head, 1 - 2^-5 .. 1 - 2^-8          0.8e-7 and 0.8e-7  (1.7e-7 and 1.3e-7)
+//   one decay per head, 1 - 1e-4                      0.9e-7 and 1.7e-7  (2.7e-7 and 3.2e-7)
+//   duality, rows of silu, drawn step sizes           0.9e-7 and 1.0e-7  (0.9e-7 and 3.0e-7)
 //   delta rule, rows of silu, drawn decays            1.4e-7 and 1.4e-7  (2.1e-7 and 3.1e-7)
 //   delta rule, rows of either sign, decays 0.74 .. 1 1.3e-7 and 1.1e-7  (1.1e-7 and 0.8e-7)
 // With one accumulator, nothing added back and rounded products of decays the first two were 6.8e-7 and 2.3e-6.
@@ -61,14 +61,6 @@ __device__ __forceinline__ void bw_mma(float (&c)[4], const uint32_t (&a)[4], co
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// c + d += a b, the small products in d
-__device__ __forceinline__ void bw_mma3(float (&c)[4], float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[2],
-                                        const uint32_t (&bl)[2]) {
-    bw_mma(d, al, bh);
-    bw_mma(d, ah, bl);
-    bw_mma(c, ah, bh);
 }
 
 // a product of decays as the sum of two numbers
@@ -264,9 +256,8 @@ struct BwSmem {
     static constexpr int M_AT = 2 * QK + BW_B * LDV + BW_B * BW_LD, G_AT = M_AT + (DELTA ? BW_B * BW_LD : 0);
     static constexpr int STAGE = G_AT + BW_TAIL;                // q | k | v | A | M (the delta rule) | G | G_16 / G_j, what G_16 lacks
     static constexpr int PART = BW_WARPS * BW_B * LDP;
-    static constexpr int SUMS = PART + (DELTA ? 0 : 2 * BW_B * LDP);                       // without the delta rule A u too, by halves of its tokens
     static constexpr int U = DELTA ? BW_B * LDV : 0;
-    static constexpr int TOTAL = STAGES * STAGE + (DELTA ? PART : 0) + TURNS * (SUMS + U);            // partial sums of p, and of r, and u
+    static constexpr int TOTAL = STAGES * STAGE + (DELTA ? PART : 0) + TURNS * (PART + U);            // partial sums of p, and of r, and u
 };
 
 template <int NT, int MT, bool DELTA, bool HELP>
@@ -440,8 +431,9 @@ __device__ __forceinline__ int bw_nth_longest(const int* __restrict__ q_start, i
 __device__ __forceinline__ bool bw_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 // Eight warps hold the state, bring the blocks and make the results.  Without the delta rule a block's u depends on no state, so
-// A u is a product on the tensor cores too (three fragments, by three warps) and the sums over the warps' rows are added up
-// beside the next block, behind its one barrier.  With HELP eight more bring the blocks and turn a
+// a block's results (the sums over the warps' rows, and A u in float32 multiply-adds: cut in two tf32 numbers it was further from 64
+// bits where portions are short, 1.0e-7 and 0.9e-7 for 17 tokens) are made beside the next block, behind its one barrier.
+// With HELP eight more bring the blocks and turn a
 // block's partial sums into results while the state warps, which then do only what the next block waits for, are at the next
 // one.  A helper passes DONE of block i before it refills the stage of block i - 1 (whose update came before) with block
 // i + 2, makes block i's results and then reports block i + 2 FULL, so the state warps write block i + 2's sums over block
@@ -459,7 +451,7 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
     extern __shared__ __align__(16) float bw_smem[];
     float* part_p = bw_smem + C::STAGES * C::STAGE;
     float* parts_r = part_p + (DELTA ? C::PART : 0);
-    float* us = parts_r + C::TURNS * C::SUMS;
+    float* us = parts_r + C::TURNS * C::PART;
     griddep_launch();
     griddep_wait();
     const int s = bw_nth_longest(a.q_start, a.S, blockIdx.z), h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
@@ -515,19 +507,15 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
         const float* sv = bw_smem + stage * C::STAGE + 2 * C::QK;
         const float* sA = sv + BW_B * C::LDV;
         const float* gam = bw_smem + stage * C::STAGE + C::G_AT;
-        const float* u = us + turn * C::U + col;
+        const float* u = (DELTA ? us + turn * C::U : sv) + col;
         float o0[MT], o1[MT];
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-            o0[m] = gam[tok + 8 * m] * bw_sum_parts<C::LDP>(parts_r + turn * C::SUMS, tok + 8 * m, col);
+            o0[m] = gam[tok + 8 * m] * bw_sum_parts<C::LDP>(parts_r + turn * C::PART, tok + 8 * m, col);
             o1[m] = skip * sv[(tok + 8 * m) * C::LDV + col];
         }
-        if (PIPE) {                                             // A u was made on the tensor cores; the later tokens reach no earlier result
-            const float* au = parts_r + turn * C::SUMS + C::PART + tok * C::LDP + col;
-            o1[0] += tok < BW_B / 2 ? au[0] : au[0] + au[BW_B * C::LDP];
-        }
 #pragma unroll
-        for (int j = 0; j < (PIPE ? 0 : 4); ++j) {
+        for (int j = 0; j < 4; ++j) {
             const float u0 = u[(4 * j) * C::LDV], u1 = u[(4 * j + 1) * C::LDV], u2 = u[(4 * j + 2) * C::LDV], u3 = u[(4 * j + 3) * C::LDV];
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
@@ -627,7 +615,7 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
         if (DELTA) {
             float* su = us + turn * C::U;
             const float* const in[2] = {sk, sq};
-            float* const to[2] = {part_p + warp * BW_B * C::LDP, parts_r + turn * C::SUMS + warp * BW_B * C::LDP};
+            float* const to[2] = {part_p + warp * BW_B * C::LDP, parts_r + turn * C::PART + warp * BW_B * C::LDP};
             bw_read_out<NT, MT, 2>(in, sh, sl, to, row0, g, tq);
             HELP ? bw_sync(BW_BAR_STATE, BW_THREADS) : __syncthreads();
             // thread: token lane % 16 of column tid / 16 of every 16; the 16 tokens of a column meet in half a warp
@@ -652,27 +640,8 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
         }
         if (!DELTA) {
             const float* const in[1] = {sq};
-            float* const to[1] = {parts_r + turn * C::SUMS + warp * BW_B * C::LDP};
+            float* const to[1] = {parts_r + turn * C::PART + warp * BW_B * C::LDP};
             bw_read_out<NT, MT, 1>(in, sh, sl, to, row0, g, tq);
-        }
-        if (PIPE && warp < 3) {                                 // A u: tokens 8 hh .. of the earlier (ks 0) and later (ks 1) half of the u
-            const int ks = warp >> 1, hh = warp > 0, j = ks * 8 + tq;
-            const float* A = sv + BW_B * C::LDV + (hh * 8 + g) * BW_LD + j;
-            const float* uj = sv + j * C::LDV + g;
-            uint32_t ah[4], al[4], bh[2], bl[2];
-            bw_split(uj[0], ah[0], al[0]);
-            bw_split(uj[8], ah[1], al[1]);
-            bw_split(uj[4 * C::LDV], ah[2], al[2]);
-            bw_split(uj[4 * C::LDV + 8], ah[3], al[3]);
-            bw_split(A[0], bh[0], bl[0]);
-            bw_split(A[4], bh[1], bl[1]);
-            float acc[4] = {}, low[4] = {};
-            bw_mma3(acc, low, ah, al, bh, bl);
-            float* p = parts_r + turn * C::SUMS + C::PART + (ks * BW_B + hh * 8 + 2 * tq) * C::LDP + g;
-            p[0] = bw_total<1>(acc[0], low[0]);
-            p[C::LDP] = bw_total<1>(acc[1], low[1]);
-            p[8] = bw_total<1>(acc[2], low[2]);
-            p[C::LDP + 8] = bw_total<1>(acc[3], low[3]);
         }
         if (HELP) bw_sync(BW_BAR_STATE, BW_THREADS);            // u and the partial sums of r are there
         else if (!PIPE) __syncthreads();

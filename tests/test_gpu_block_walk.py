@@ -115,6 +115,28 @@ def test_long_portions_lose_no_more_than_token_by_token(form, slow):
     assert rel(out, torch.stack(want)) <= 7e-7 and rel(state, S) <= 7e-7
 
 
+def test_tokens_that_know_nothing_of_one_another_return_their_values_to_the_bit():
+    """Every token's key and query is a unit vector of its own, so its result is its own value times one: what lies inside a block is
+    multiplied and added in float32, and the state that a query reads is zero there."""
+    from aien_sovereign_core_mv_b200 import kernels as K
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    heads, N, V, lens = 3, 64, 48, [37, 16, 1]
+    T, S = sum(lens), len(lens)
+    g_ = torch.Generator().manual_seed(3)
+    rows = torch.zeros(T, 2 * N + heads * V)
+    at = torch.cat([torch.randperm(N, generator=g_)[:n] for n in lens])
+    rows[torch.arange(T), at] = 1.0
+    rows[torch.arange(T), N + at] = 1.0
+    rows[:, 2 * N:] = torch.randn(T, heads * V, generator=g_)
+    gates = torch.cat([1.0 - 0.5 * torch.rand(T, heads, generator=g_), torch.ones(T, heads)], 1)
+    state, out = torch.randn(S, heads * N * V).cuda(), torch.full((T, heads * V), 9.0).cuda()
+    q0 = [sum(lens[:s]) for s in range(S + 1)]
+    blocks = torch.empty(K.block_walk_scratch(T, S, heads, 1, N, V)).cuda()
+    assert K.block_walk(rows.cuda(), 0, N, 2 * N, gates.cuda(), 0, heads, None, state, 0, i32(list(range(S))), i32(q0),
+                        i32([p for n in lens for p in range(n)]), out, S, heads, 1, N, V, blocks, delta=False)
+    assert torch.equal(out.cpu(), rows[:, 2 * N:])
+
+
 def test_many_heads_over_one_group_walk_by_blocks():
     """The duality form needs no 16 x 16 system a head, so heads that are too many for the delta rule are not for it."""
     from aien_sovereign_core_mv_b200 import kernels as K
