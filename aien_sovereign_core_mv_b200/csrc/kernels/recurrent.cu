@@ -169,7 +169,8 @@ decay_linear_attention_token_kernel(const TP* __restrict__ proj, long ld, int q_
 
 // The same with a head's whole state in a CTA's registers, four neighbouring columns a thread and all of it requested before the
 // token's rows are made: value sizes of 64 and 128, up to 128 rows, states on 16-byte boundaries.  64 requests, 16 heads of
-// 128 x 128 (134 MB of state read and written), B200: 31 us with 4 bytes a thread and row, 24 us so (5.7 TB/s).
+// 128 x 128 (134 MB of state read and written), B200: 31 us with 4 bytes a thread and row, 24 us so (5.7 TB/s).  Results 8.5e-8 from 64
+// bits (relative 2-norm; 1.0e-7 with 4 bytes a thread and row; heads of 64 x 64 8.3e-8 and 9.0e-8).
 template <int LANES, typename TP>
 __global__ void __launch_bounds__(256, 2)
 decay_linear_attention_token_vec_kernel(const TP* __restrict__ proj, long ld, int q_off, int k_off, int v_off, const float* __restrict__ decay,
@@ -198,22 +199,28 @@ decay_linear_attention_token_vec_kernel(const TP* __restrict__ proj, long ld, in
     for (int i = 0; i < 4; ++i) v[i] = silu_f(to_f(row[v_off + (size_t)h * V + c + i]));
     const float lam = decay[h];
     __syncthreads();
+    // sums of four rows, then of the fours, then over the row groups: short chains round little
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-        const int d = rg + RG * j;
-        const float k = rows[0][d], q = rows[1][d];
-        S[j].x = fmaf(lam, S[j].x, k * v[0]); S[j].y = fmaf(lam, S[j].y, k * v[1]);
-        S[j].z = fmaf(lam, S[j].z, k * v[2]); S[j].w = fmaf(lam, S[j].w, k * v[3]);
-        o.x = fmaf(S[j].x, q, o.x); o.y = fmaf(S[j].y, q, o.y); o.z = fmaf(S[j].z, q, o.z); o.w = fmaf(S[j].w, q, o.w);
-        if (d < dim) *reinterpret_cast<float4*>(st + (size_t)d * V) = S[j];
+    for (int j0 = 0; j0 < ROWS; j0 += 4) {
+        float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = j0; j < j0 + 4; ++j) {
+            const int d = rg + RG * j;
+            const float k = rows[0][d], q = rows[1][d];
+            S[j].x = fmaf(lam, S[j].x, k * v[0]); S[j].y = fmaf(lam, S[j].y, k * v[1]);
+            S[j].z = fmaf(lam, S[j].z, k * v[2]); S[j].w = fmaf(lam, S[j].w, k * v[3]);
+            o4.x = fmaf(S[j].x, q, o4.x); o4.y = fmaf(S[j].y, q, o4.y); o4.z = fmaf(S[j].z, q, o4.z); o4.w = fmaf(S[j].w, q, o4.w);
+            if (d < dim) *reinterpret_cast<float4*>(st + (size_t)d * V) = S[j];
+        }
+        o.x += o4.x; o.y += o4.y; o.z += o4.z; o.w += o4.w;
     }
     *reinterpret_cast<float4*>(&sums[rg][c]) = o;
     __syncthreads();
     if (tid < V) {
         float y = 0.f;
 #pragma unroll
-        for (int r = 0; r < RG; ++r) y += sums[r][tid];
+        for (int r = 0; r < RG; r += 4) y += (sums[r][tid] + sums[r + 1][tid]) + (sums[r + 2][tid] + sums[r + 3][tid]);
         out[(size_t)t * ldo + (size_t)h * V + tid] = y;
     }
 }

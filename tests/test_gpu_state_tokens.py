@@ -139,7 +139,7 @@ def test_selective_scan_of_single_tokens(inner, N, s_off, b_off, lens):
             H.assert_close(dev[slots[s], s_off:s_off + inner * N].cpu().numpy().reshape(inner, N), S, 1e-5, f"state {s}")
 
 
-@pytest.mark.parametrize("form", ["delta"])
+@pytest.mark.parametrize("form", ["delta", "linear"])
 @pytest.mark.parametrize("S,heads,dim", [(9, 8, 128), (33, 32, 64), (64, 16, 128)])
 def test_single_tokens_are_as_near_to_64_bits_in_whole_vectors_as_number_by_number(form, S, heads, dim):
     """The same tokens over states on 16-byte boundaries and four bytes beside them, which the general kernels take: a relative 2-norm of
