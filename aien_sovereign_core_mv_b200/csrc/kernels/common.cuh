@@ -92,16 +92,21 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 // ---- programmatic dependent launch
-// The decode step is a chain of short kernels.  Launched with the programmatic-serialization
-// attribute, a kernel may become resident while its predecessor is still running; it must not
-// read what the predecessor writes, nor write anything, before griddep_wait() returns (which is
-// when the predecessor has completed and its writes are visible).  Weights are never written
-// during a step, so a kernel may prefetch them first.  griddep_launch() lets the successor start
-// its own prologue.  Without the launch attribute both are no-ops.
-// The recurrences by blocks, the selective scan and the latent attention are chains of this kind too, of launches of 5 to 100 us:
-// their kernels wait at the very top, so what they gain is the border itself, 1 to 2 us each.  B200, plain launches and so, one part's
-// step: latent attention of 2,048 tokens 145.4 and 137.9 us, the selective scan 286 and 278, the delta rule 273 and 267, linear
-// attention 205 and 199, the duality 187 and 185.5.
+// The decode step is a chain of short kernels, and the prompt of a recurrent or latent part one of launches of 5 to 100 us.  Launched
+// with the programmatic-serialization attribute, a kernel may become resident while its predecessor is still running; it must not
+// read what an earlier kernel of the step writes, nor write anything, before griddep_wait() returns (which is
+// when the predecessor has completed and its writes are visible).  Without the launch attribute griddep_wait() and griddep_launch() are no-ops.
+// griddep_launch() lets the successor start its own prologue, and where it stands ahead of the wait, the successor's successor too:
+// what a kernel several launches ahead writes is as little there as what the last one writes.  So ahead of a wait stand only
+//   * weights, which are never written during a step (the products' first tiles of W, norms' scales),
+//   * a step's metadata that the host copied (starts, positions, tables, tile lists: the copy is a border for the whole stream), and
+//   * in the streamed decode attention the cached keys and values of earlier positions, which earlier steps wrote.
+// A table that a kernel of the step makes is none of these: prefill_tc_kernel is told (PtSizes::table_made).
+// A kernel whose few CTAs each walk a long chain is launched plainly: started early, its CTAs are dealt to the SMs that the predecessor
+// leaves first, two or more to one, and the others stay idle for the whole walk.  B200, a layer's prompt of 2,048 tokens, the walk by
+// blocks with and without the attribute: linear attention 305 and 235 us, the duality 277 and 216, the delta rule with 32 heads 800 and
+// 609; the selective scan, 1,500 tokens of three requests, 316 and 241.  (With CTAs for every place on the GPU the border itself is
+// what counts, 1 to 3 us: the listed 2,048 tokens of latent attention 145.4 us plain and 137.9 so.)
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -134,8 +139,8 @@ inline bool pdl_enabled() {
     return v == 1;
 }
 
-// Launch `kernel` so that it may overlap the tail of the kernel before it on the stream.  Only for
-// kernels that call griddep_wait() before touching anything but weights.
+// Launch `kernel` so that it may overlap the tail of the kernel before it on the stream.  Only for kernels that keep the rule above,
+// and not for walks of few CTAs.
 template <typename... KArgs, typename... Args>
 inline void launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
