@@ -123,7 +123,6 @@ block_coef_kernel(const BlockWalk a) {
     __shared__ float dots[DELTA ? 2 : 1][BW_B * BW_B];                      // q_i . k_j and k_i . k_j
     const int slot = blockIdx.x, kvh = blockIdx.y;
     griddep_launch();
-    griddep_wait();
     int lo = 0, hi = a.S - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) / 2;
@@ -759,7 +758,7 @@ AIEN_API int aien_block_walk(const float* rows, long ld, int q_off, int k_off, i
     const int per = heads / G, smem = 4 * (2 * BW_B * (N + 4) + 2 * BW_B * per + (delta ? 256 * per : 0));
     auto coef = delta ? block_coef_kernel<true> : block_coef_kernel<false>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(coef, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return AIEN_E_STATE;
-    launch_chain(coef, dim3((unsigned)blocks, G), dim3(256), (size_t)smem, stream, a);
+    coef<<<dim3((unsigned)blocks, G), 256, smem, stream>>>(a);              // plain: see griddep_wait
     const int rc = launch_status();
     if (rc != 0) return rc;
     return N <= 64 ? dispatch_block_walk<1>(a, stream) : dispatch_block_walk<2>(a, stream);

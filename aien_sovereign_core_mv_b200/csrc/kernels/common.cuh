@@ -102,11 +102,16 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 //   * a step's metadata that the host copied (starts, positions, tables, tile lists: the copy is a border for the whole stream), and
 //   * in the streamed decode attention the cached keys and values of earlier positions, which earlier steps wrote.
 // A table that a kernel of the step makes is none of these: prefill_tc_kernel is told (PtSizes::table_made).
-// A kernel whose few CTAs each walk a long chain is launched plainly: started early, its CTAs are dealt to the SMs that the predecessor
-// leaves first, two or more to one, and the others stay idle for the whole walk.  B200, a layer's prompt of 2,048 tokens, the walk by
-// blocks with and without the attribute: linear attention 305 and 235 us, the duality 277 and 216, the delta rule with 32 heads 800 and
-// 609; the selective scan, 1,500 tokens of three requests, 316 and 241.  (With CTAs for every place on the GPU the border itself is
-// what counts, 1 to 3 us: the listed 2,048 tokens of latent attention 145.4 us plain and 137.9 so.)
+// What is launched plainly although it stands in such a chain: a kernel that is started early has its CTAs dealt to the SMs that have room
+// just then, several to one while others stay idle, and they stay where they are.  So are
+//   * the walks, whose few CTAs each walk a long chain.  B200, a layer's prompt of 2,048 tokens, with and without the attribute: linear
+//     attention 305 and 235 us, the duality 277 and 216, the delta rule with 32 heads 800 and 609; the selective scan, 1,500 tokens
+//     of three requests, 316 and 241;
+//   * the walk's coefficients, the convolutions, the scan's step sizes, the products per head, the merge and the gather of latent attention and the
+//     routers of a few tokens: 100 tokens through the duality 45.5 and 39.5 us, through linear attention 46.9 and 40.5, three tokens
+//     of latent attention with 32 heads 69.5 and 60, nine tokens through 16 gated experts 64.5 and 60.5.
+// The rest gains the border, 1 to 3 us: norms, splits, rotary tables, step sizes of the duality, the combination of segments and of experts, the
+// attention over the latent, the products (whose CTAs are one to an SM).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -563,7 +563,6 @@ latent_attention_merge_kernel(int R, const float* __restrict__ part_o, const flo
     __shared__ float wt[LX_MAX_SPLIT];
     __shared__ float red[32];
     griddep_launch();
-    griddep_wait();
     const int unit = blockIdx.x / H, h = blockIdx.x - unit * H;
     const size_t row = blockIdx.x, to = (size_t)(tokens != nullptr ? tokens[unit] : unit) * H + h;
     const float sk = sinks != nullptr ? sinks[h] * 1.4426950408889634f : -INFINITY;
@@ -626,7 +625,7 @@ static int launch_latent_tc(const void* q, const void* cache, const int* bt, int
                      H, r_lat, rd, page_size, window, scale2, sinks, ksplit, part_o, part_ml, single_only);
     }
     if (ksplit > 1)
-        launch_chain(latent_attention_merge_kernel, dim3((unsigned)((long)(tokens != nullptr ? num_tokens : T) * H)), dim3(128), (size_t)0, stream,
+        latent_attention_merge_kernel<<<dim3((unsigned)((long)(tokens != nullptr ? num_tokens : T) * H)), 128, 0, stream>>>(                // plain: see griddep_wait
             r_lat, part_o, part_ml, ksplit, sinks, H, (__nv_bfloat16*)out, tokens);
     return launch_status();
 }
@@ -653,7 +652,6 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
     constexpr int NJ = HT_BN / 16;                             // n8 tiles of a warp
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     griddep_launch();
-    griddep_wait();
     const int mh = warp & 1, nh = warp >> 1, g = lane >> 2, c = lane & 3;
     const int m0 = blockIdx.y * HT_BM, n0 = blockIdx.x * HT_BN, h = blockIdx.z;
     A += (size_t)h * a_head;
@@ -765,7 +763,6 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, int r_lat, const i
     __shared__ int s_req;
     const int p = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     griddep_launch();
-    griddep_wait();
     if (tid == 0) s_req = -1;
     __syncthreads();
     if (warp == 0) {
@@ -844,7 +841,7 @@ AIEN_API int aien_head_project_tc(const void* A, long lda, long a_head, const vo
     const bool narrow = rows64 * ((N + 63) / 64) * heads <= 148;           // 64 columns would give every SM one CTA at most
     const int bn = narrow ? 32 : 64;
     const dim3 grid((N + bn - 1) / bn, (unsigned)rows64, heads);
-    AIEN_DISPATCH_DTYPE(c_dt, TC, (launch_chain(narrow ? head_project_tc_kernel<32, TC> : head_project_tc_kernel<64, TC>, grid, dim3(128), (size_t)0, stream,
+    AIEN_DISPATCH_DTYPE(c_dt, TC, ((narrow ? head_project_tc_kernel<32, TC> : head_project_tc_kernel<64, TC>)<<<grid, 128, 0, stream>>>(         // plain: see griddep_wait
         (const __nv_bfloat16*)A, lda, a_head, (const __nv_bfloat16*)W, (long)N * K, (TC*)C, ldc, c_head, M, N, K, gate, gate_dt, ldg, gate_n, rows)));
     return launch_status();
 }
@@ -856,7 +853,7 @@ AIEN_API int aien_latent_gather(const void* cache, int r_lat, const int* block_t
     if (portions <= 0 || S <= 0) return 0;
     if (r_lat <= 0 || (r_lat & 7) || page_size <= 0 || len <= 0 || (len & 127) || portions > 65535) return AIEN_E_SHAPE;
     if (((uintptr_t)cache & 15) || ((uintptr_t)out & 15)) return AIEN_E_ALIGN;
-    launch_chain(latent_gather_kernel, dim3(len / 8, portions), dim3(256), (size_t)0, stream, (const __nv_bfloat16*)cache, r_lat, block_table, max_blocks, page_size,
-                 q_start, ctx_len, S, len, (__nv_bfloat16*)out, table);
+    latent_gather_kernel<<<dim3(len / 8, portions), 256, 0, stream>>>((const __nv_bfloat16*)cache, r_lat, block_table, max_blocks, page_size, q_start,         // plain: see griddep_wait
+                                                                      ctx_len, S, len, (__nv_bfloat16*)out, table);
     return launch_status();
 }

@@ -168,7 +168,6 @@ moe_route_biased_kernel(const float* __restrict__ z, long ldz, int T, int E, int
     __shared__ float held[ROUTE_WARPS][NR * 32];
     __shared__ int chosen[ROUTE_WARPS][NR * 32];
     griddep_launch();
-    griddep_wait();
     const int t = blockIdx.x * ROUTE_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= T) return;
     const float* zr = z + (size_t)t * ldz;
@@ -654,8 +653,8 @@ AIEN_API int aien_moe_route_biased(const float* z, long ldz, int T, int E, int r
                                    cudaStream_t stream) {
     if (T <= 0) return 0;
     if (E <= 0 || E > ROUTE_MAX_EXPERTS || real <= 0 || real > E || top <= 0 || top > E || (real < E && w_same == nullptr)) return AIEN_E_SHAPE;
-    ROUTE_DISPATCH(E, (launch_chain(moe_route_biased_kernel<NR>, dim3((unsigned)((T + ROUTE_WARPS - 1) / ROUTE_WARPS)), dim3(ROUTE_WARPS * 32), (size_t)0, stream, z, ldz,
-                                    T, E, real, top, renorm, renorm_eps, correction, c_dt, sigmoid, ids, wts, w_same, expert_count)));
+    ROUTE_DISPATCH(E, (moe_route_biased_kernel<NR><<<(unsigned)((T + ROUTE_WARPS - 1) / ROUTE_WARPS), ROUTE_WARPS * 32, 0, stream>>>(      // plain: see griddep_wait
+        z, ldz, T, E, real, top, renorm, renorm_eps, correction, c_dt, sigmoid, ids, wts, w_same, expert_count)));
     return launch_status();
 }
 

@@ -38,7 +38,6 @@ parts_product_kernel(const __nv_bfloat16* __restrict__ parts, const __nv_bfloat1
     const int m0 = blockIdx.y * PP_BM, n0 = blockIdx.x * PP_BN, steps = (K + PP_BK - 1) / PP_BK;
     const uint32_t smem = (uint32_t)__cvta_generic_to_shared(pp_smem);
     griddep_launch();
-    griddep_wait();
     // K is a multiple of 8, so a piece of 8 numbers lies inside or outside whole
     auto fetch = [&](int step) {
         if (step < steps) {
@@ -122,7 +121,7 @@ AIEN_API int aien_parts_product(const void* parts, const void* W, long ldw, floa
     constexpr int bytes = PP_STAGES * PP_STAGE * 2;
     if (cudaFuncSetAttribute(parts_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
     const int pairs = ((ldo | N) & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
-    launch_chain(parts_product_kernel, dim3((N + PP_BN - 1) / PP_BN, (M + PP_BM - 1) / PP_BM), dim3(PP_THREADS), (size_t)bytes, stream,
-                 (const __nv_bfloat16*)parts, (const __nv_bfloat16*)W, ldw, out, ldo, M, N, K, pairs);
+    parts_product_kernel<<<dim3((N + PP_BN - 1) / PP_BN, (M + PP_BM - 1) / PP_BM), PP_THREADS, bytes, stream>>>(      // plain: see griddep_wait
+        (const __nv_bfloat16*)parts, (const __nv_bfloat16*)W, ldw, out, ldo, M, N, K, pairs);
     return launch_status();
 }

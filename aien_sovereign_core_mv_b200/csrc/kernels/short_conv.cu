@@ -296,7 +296,6 @@ template <int TAPS, bool DELTA>
 __global__ void __launch_bounds__(CR_THREADS)
 conv_runs_kernel(const ConvRunArgs a) {
     griddep_launch();
-    griddep_wait();
     const int lo = blockIdx.y * a.run, hi = lo + a.run < a.T ? lo + a.run : a.T;
     if (DELTA && blockIdx.x == gridDim.x - 1) {                             // one CTA per run makes the gates
         for (int i = threadIdx.x; i < (hi - lo) * a.heads; i += CR_THREADS) {
@@ -422,8 +421,8 @@ static void launch_conv_runs(ConvRunArgs& a, int taps, cudaStream_t stream) {
     a.run = 1;
     while (a.run < 16 && (long)gx * ((a.T + 2 * a.run - 1) / (2 * a.run)) >= 4 * 148) a.run *= 2;
     const dim3 grid(gx, (a.T + a.run - 1) / a.run);
-    launch_chain(taps == 2 ? conv_runs_kernel<2, DELTA> : taps == 3 ? conv_runs_kernel<3, DELTA> : conv_runs_kernel<4, DELTA>, grid, dim3(CR_THREADS), (size_t)0,
-                 stream, a);
+    const auto kern = taps == 2 ? conv_runs_kernel<2, DELTA> : taps == 3 ? conv_runs_kernel<3, DELTA> : conv_runs_kernel<4, DELTA>;
+    kern<<<grid, CR_THREADS, 0, stream>>>(a);                               // plain: see griddep_wait
 }
 
 }  // namespace aien
