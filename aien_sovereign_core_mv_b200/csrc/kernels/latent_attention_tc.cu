@@ -637,7 +637,7 @@ static int launch_latent_tc(const void* q, const void* cache, const int* bt, int
 // (cp.async), mma.sync.m16n8k16 with float32 accumulation.
 constexpr int HT_BM = 64, HT_BK = 64, HT_STR = HT_BK + 8;
 
-// What bounds a step of few tokens is a k-step's way through memory: three stages of 32 columns, two of them on their way, and the gate's
+// What bounds a step of few tokens is a k-step's way through memory: three stages of 32 columns (two of 64), all on their way at first, and the gate's
 // values are requested with the first.  64 rows, 16 heads, 512 -> 128 columns, B200: 8.2 us with two stages of 64 columns and 13.9
 // with a gate per element read behind the products; 7.5 and 10.4 so.  rows (or null): A's and C's rows
 // are those that it lists, M of them.
@@ -692,15 +692,18 @@ head_project_tc_kernel(const __nv_bfloat16* __restrict__ A, long lda, long a_hea
                 }
         }
     const int steps = (K + HT_BK - 1) / HT_BK;
-    for (int i = 0; i < HT_STAGES - 1; ++i) {
+    for (int i = 0; i < HT_STAGES; ++i) {
         if (i < steps) fetch(i * HT_BK, i);
         else lx_cp_async_commit();
     }
     for (int i = 0, st = 0; i < steps; ++i, st = st + 1 == HT_STAGES ? 0 : st + 1) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(HT_STAGES - 2) : "memory");
+        if (i == 0) asm volatile("cp.async.wait_group %0;" ::"n"(HT_STAGES - 1) : "memory");
+        else asm volatile("cp.async.wait_group %0;" ::"n"(HT_STAGES - 2) : "memory");
         __syncthreads();                                        // the step has landed, and everyone is done with the one before it
-        if (i + HT_STAGES - 1 < steps) fetch((i + HT_STAGES - 1) * HT_BK, st == 0 ? HT_STAGES - 1 : st - 1);
-        else lx_cp_async_commit();
+        if (i > 0) {                                            // whose stage takes the next
+            if (i + HT_STAGES - 1 < steps) fetch((i + HT_STAGES - 1) * HT_BK, st == 0 ? HT_STAGES - 1 : st - 1);
+            else lx_cp_async_commit();
+        }
         const uint32_t As_u = (uint32_t)__cvta_generic_to_shared(As[st]), Ws_u = (uint32_t)__cvta_generic_to_shared(Ws[st]);
 #pragma unroll
         for (int kk = 0; kk < HT_BK / 16; ++kk) {
