@@ -111,7 +111,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 //     routers of a few tokens: 100 tokens through the duality 45.5 and 39.5 us, through linear attention 46.9 and 40.5, three tokens
 //     of latent attention with 32 heads 69.5 and 60, nine tokens through 16 gated experts 64.5 and 60.5.
 // The rest gains the border, 1 to 3 us: norms, splits, rotary tables, step sizes of the duality, the combination of segments and of experts, the
-// attention over the latent, the products (whose CTAs are one to an SM).
+// attention over the latent, the products (whose CTAs are one to an SM where they are few).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -1121,19 +1121,24 @@ static int launch_tc_cluster(const CUtensorMap& ma, const CUtensorMap& mw, void*
     return launch_status();
 }
 
+constexpr int TC_ALONE_SMEM = 120 * 1024;           // more than half of an SM's shared memory, and than any TcT's
+
 template <int EPI, typename TC, int AR, int BN>
 static int launch_tc_rows(const CUtensorMap& ma, const CUtensorMap& mw, void* out, long ldc, int splits, size_t part_stride,
                           int M, int N, int K, cudaStream_t stream) {
     auto kern = gemm_tc_kernel<EPI, TC, AR, BN>;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TcT<AR, BN>::SMEM) != cudaSuccess) return AIEN_E_STATE;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_ALONE_SMEM) != cudaSuccess) return AIEN_E_STATE;
         configured = true;
     }
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int kb_per_split = (total_kb + splits - 1) / splits;
     dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN, (total_kb + kb_per_split - 1) / kb_per_split);
-    launch_chain(kern, grid, dim3(192), (size_t)TcT<AR, BN>::SMEM, stream, ma, mw, (TC*)out, ldc, part_stride, kb_per_split, M, N, K);
+    // No more CTAs than SMs: one to an SM.  Started beside the tail of the kernel ahead, they were dealt two to the SMs that this leaves
+    // first.  A layer's prompt of 1,024 tokens, products of 128 tiles: latent attention 57 and 54.5 us, linear attention 90.5 and 88.
+    const size_t smem = (long)grid.x * grid.y * grid.z <= tc_num_sms() ? TC_ALONE_SMEM : TcT<AR, BN>::SMEM;
+    launch_chain(kern, grid, dim3(192), smem, stream, ma, mw, (TC*)out, ldc, part_stride, kb_per_split, M, N, K);
     return launch_status();
 }
 
