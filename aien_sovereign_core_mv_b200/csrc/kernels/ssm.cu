@@ -629,10 +629,11 @@ static void launch_selective_scan_token(const ScanArgs& a) {
 }
 
 // Eight lanes a channel; with fewer than 2,048 channels in the step, whose walkers would leave SM schedulers without a
-// warp, and with many state values, sixteen.  Where walkers are many, four with four states each, whose instructions per
-// state are fewer: of 16 states in segments beyond 512 channels, and whole from 12,288 channels of the step's requests on (six of
-// 300 tokens, 4,096 channels each: 88 us with eight lanes, 75 with four; six of 80 tokens 27 and 22; four of 512 tokens, 2,048
-// channels each, 54 and 64).  In segments of up to 512 channels eight from 512 tokens on (1,024 tokens: 26 us with sixteen, 23).
+// warp, and with many state values, sixteen.  In segments of 16 states beyond 512 channels four with four states each, whose
+// instructions per state are fewer: segments are of one length, so what counts is their number.  Whole portions keep eight: their longest
+// one may be all that still walks, and four lanes take half as long again a token (4,096 channels, us with eight and four: requests of
+// 900, 100, 100 and 100 tokens 83 and 113, of 700, 500 and 300 77 and 93; three of 500 88 and 76, which the step's sizes do not tell apart).
+// In segments of up to 512 channels eight from 512 tokens on (1,024 tokens: 26 us with sixteen, 23).
 template <typename TO>
 static int dispatch_selective_scan(const ScanArgs& a) {
     const int N = a.N;
@@ -651,7 +652,7 @@ static int dispatch_selective_scan(const ScanArgs& a) {
     else if (N <= 16) {
         const long channels = (long)a.inner * a.S;
         const bool few_cut = channels <= 512 && a.T >= 512L * a.S;
-        if (a.sg.mode != 0 ? channels > 512 : channels >= 12288) launch_selective_scan<4, 4, TO>(a);
+        if (a.sg.mode != 0 && channels > 512) launch_selective_scan<4, 4, TO>(a);
         else if (few && !(a.sg.mode != 0 && few_cut)) launch_selective_scan<16, 1, TO>(a);
         else launch_selective_scan<8, 2, TO>(a);
     }
