@@ -452,6 +452,7 @@ block_walk_kernel(const __grid_constant__ BlockWalk a) {
     float* parts_r = part_p + (DELTA ? C::PART : 0);
     float* us = parts_r + C::TURNS * C::PART;
     griddep_launch();
+    griddep_wait();
     const int s = bw_nth_longest(a.q_start, a.S, blockIdx.z), h = blockIdx.y, kvh = h / (a.heads / a.G), t0 = a.q_start[s], t1 = a.q_start[s + 1];
     if (t1 <= t0 || (a.alone && t1 - t0 == 1)) return;
     const int tid = threadIdx.x & (BW_THREADS - 1), warp = tid >> 5, lane = tid & 31;
@@ -709,7 +710,11 @@ static int launch_block_walk(const BlockWalk& a, cudaStream_t stream) {
     constexpr int bytes = BwSmem<NT, MT, DELTA, HELP>::TOTAL * 4;
     auto kern = block_walk_kernel<NT, MT, DELTA, HELP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return AIEN_E_STATE;
-    kern<<<dim3((a.V + 16 * MT - 1) / (16 * MT), a.heads, a.S), (HELP ? 2 : 1) * BW_THREADS, bytes, stream>>>(a);      // plain: see griddep_wait
+    constexpr int threads = (HELP ? 2 : 1) * BW_THREADS;
+    static const int resident = resident_ctas(kern, threads, bytes);
+    const dim3 grid((a.V + 16 * MT - 1) / (16 * MT), a.heads, a.S);
+    if (resident == 1) launch_chain(kern, grid, dim3(threads), (size_t)bytes, stream, a);         // see griddep_wait
+    else kern<<<grid, threads, bytes, stream>>>(a);
     return launch_status();
 }
 

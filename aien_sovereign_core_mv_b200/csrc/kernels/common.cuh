@@ -104,7 +104,9 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // A table that a kernel of the step makes is none of these: prefill_tc_kernel is told (PtSizes::table_made).
 // What is launched plainly although it stands in such a chain: a kernel that is started early has its CTAs dealt to the SMs that have room
 // just then, several to one while others stay idle, and they stay where they are.  So are
-//   * the walks, whose few CTAs each walk a long chain.  B200, a layer's prompt of 2,048 tokens, with and without the attribute: linear
+//   * the walks, whose few CTAs each walk a long chain (but for the delta rule's with helper warps, whose CTAs are one to an SM, and for the
+//     scan's segments of one length where they fill the GPU: where portions differ, the longest ones' CTAs start first and share an SM even
+//     then, 1,036 tokens of five requests through the delta rule 96 and 89 us).  B200, a layer's prompt of 2,048 tokens, with and without the attribute: linear
 //     attention 305 and 235 us, the duality 277 and 216, the delta rule with 32 heads 800 and 609; the selective scan, 1,500 tokens
 //     of three requests, 316 and 241;
 //   * the walk's coefficients, the convolutions, the scan's step sizes, the products per head, the merge and the gather of latent attention and the
@@ -159,6 +161,19 @@ inline void launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// CTAs of a kernel that an SM holds at once (0: unknown).
+template <typename Kernel>
+inline int resident_ctas(Kernel kernel, int threads, size_t smem) {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) == cudaSuccess && n > 0 ? n : 0;
+}
+// Whether a launch of so many CTAs fills every place of the GPU.
+inline bool fills_gpu(long ctas, int resident) {
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    return resident > 0 && ctas >= (long)resident * sms;
 }
 
 inline int launch_status() {

@@ -139,9 +139,10 @@ selective_scan_kernel(ScanRowsIn in, const float* __restrict__ A, const void* __
     __shared__ __align__(16) float sums[C::TOKENS * SSM_THREADS];      // a lane's part of y per token
     const int s = blockIdx.y, seg = sg.mode == 0 ? 0 : blockIdx.z;
     griddep_launch();
-    int t0 = q_start[s], t1 = q_start[s + 1];
+    griddep_wait();
+    int t0 = __ldcg(q_start + s), t1 = __ldcg(q_start + s + 1);
     if (t1 <= t0) return;
-    const bool fresh = positions[t0] == 0;
+    const bool fresh = __ldcg(positions + t0) == 0;
     const size_t seg0 = sg.mode == 0 ? 0 : (size_t)(t0 / sg.seg_len + s);         // the request's first segment in the scratch
     if (sg.mode != 0) {
         t0 += seg * sg.seg_len;
@@ -606,16 +607,25 @@ static void launch_selective_scan(const ScanArgs& a) {
     using C = ScanCfg<LANES, CH>;
     Segments sg = a.sg;
     const dim3 grid((unsigned)((a.inner + C::CPB - 1) / C::CPB), a.S, sg.mode == 0 ? 1 : sg.nseg);
+    const long ctas = (long)grid.x * grid.y * grid.z;
+    auto pass = [&](auto kern, int resident) {
+        if (sg.mode != 0 && fills_gpu(ctas, resident))                  // see griddep_wait
+            launch_chain(kern, grid, dim3(SSM_THREADS), (size_t)0, a.stream, a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start,
+                         a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+        else
+            kern<<<grid, SSM_THREADS, 0, a.stream>>>(a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out,
+                                                     a.ldo, a.inner, a.N, sg);
+    };
     if (sg.mode != 0) {
         const size_t lanes = (size_t)a.inner * a.N;
-        selective_scan_kernel<LANES, CH, true, TO><<<grid, SSM_THREADS, 0, a.stream>>>(                // plain: see griddep_wait
-            a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+        static const int resident = resident_ctas(selective_scan_kernel<LANES, CH, true, TO>, SSM_THREADS, 0);
+        pass(selective_scan_kernel<LANES, CH, true, TO>, resident);
         launch_chain(segment_combine_kernel, dim3((unsigned)((lanes + 255) / 256), a.S), dim3(256), (size_t)0, a.stream, a.state, a.state_stride, a.s_off, a.slots,
                      a.q_start, a.positions, sg, lanes);
         sg.mode = 2;
     }
-    selective_scan_kernel<LANES, CH, false, TO><<<grid, SSM_THREADS, 0, a.stream>>>(
-        a.in, a.A, a.dt_bias, a.D, a.p_dt, a.state, a.state_stride, a.s_off, a.slots, a.q_start, a.positions, (TO*)a.out, a.ldo, a.inner, a.N, sg);
+    static const int resident = resident_ctas(selective_scan_kernel<LANES, CH, false, TO>, SSM_THREADS, 0);
+    pass(selective_scan_kernel<LANES, CH, false, TO>, resident);
 }
 
 template <int LANES, int CH, typename TO>

@@ -417,8 +417,8 @@ def test_selective_scan_in_the_segments_of_few_channels(inner, N, lens, dtype):
                                           (4100, 13, [16, 1, 31]), (300, 16, [1100]), (512, 16, [511])])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_selective_scan_as_many_walkers_go(inner, N, lens, dtype):
-    """Four lanes a channel, in segments and (from 12,288 channels of the step on) whole, and the steps at the rule's edges; channels
-    that fill no CTA, tokens that fill no stage."""
+    """Four lanes a channel in segments, eight and sixteen whole, and the steps at the rule's edges; channels that fill no CTA, tokens
+    that fill no stage."""
     from aien_sovereign_core_mv_b200 import kernels as K
     cut = K.selective_scan_segments(sum(lens), len(lens), False, inner, N)
     assert 2 * (sum(lens) // max(cut[0], 1) + len(lens)) * inner * N <= K.selective_scan_scratch(sum(lens), len(lens), inner, N) or cut[0] == 0
