@@ -33,11 +33,11 @@
 //   delta rule, rows of either sign, decays 0.74 .. 1 1.3e-7 and 1.1e-7  (1.1e-7 and 0.8e-7)
 // With one accumulator, nothing added back and rounded products of decays the first two were 6.8e-7 and 2.3e-6.
 //
-// 2,048 tokens, 16 heads of 128 x 128, one request, B200: the delta rule 151 us and 16 for the coefficients (603 token by
-// token); linear attention 123 and 31.  2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality: 100 and 6 us (540;
-// 122 with the longest request's CTAs the last to start); linear attention, 1,900 tokens of two requests, 16 heads of 128 x 128: 92
-// and 29 us (237 by chunks).  What bounds the walk is a block's chain of dependent instructions (390 a warp, of which each
-// waits 4 to 5 cycles; issue slots 43 % used with one CTA on an SM, 53 % with two), not its barriers or its rows: fetched two
+// Walk and coefficients back to back, B200: 2,048 tokens, 16 heads of 128 x 128, one request, the delta rule 170 us, 16 of them the
+// coefficients (603 token by token); linear attention 159 and 31.  2,000 tokens of three requests, 32 heads of 128 x 64, state-space duality:
+// 112 and 7 us (540 token by token; 22 more with the longest request's CTAs the last to start); linear attention, 1,900 tokens of two requests, 16
+// heads of 128 x 128: 127 and 30 us (237 by chunks).  What bounds the walk is a block's chain of dependent instructions (405 a warp; issue
+// slots 55 to 58 % used with two CTAs on an SM, profiles/layer_kernels__ncu_counters.md), not its barriers or its rows: fetched two
 // blocks ahead instead of one, with one barrier a block instead of two, and with products of different sums between dependent
 // ones it gains 4 us in 128.  (The choices of a form below were measured at 148, 110 and 86 us, with one accumulator a sum.)
 #include "common.cuh"

@@ -58,8 +58,8 @@ struct Segments {
 // rows fetched into registers four tokens ahead; 147 us so, 7 of them the gate's exponential and division
 // (31 instructions a token and warp, of which half a dozen in the prologue and epilogue of a stage; 16 lanes: 180 us, 4: 216 us).
 // With few channels a portion is cut into segments (see kernels.selective_scan_segments): 126 us with four lanes a channel, of
-// which the passes take 50 and 70; there 70 % of the issue slots are used (37 and 55 instructions a token and warp of eight
-// channels, a third of them the step sizes and the gate) and 50 to 60 % of the special-function unit.
+// which the passes take 50 and 70; there 68 and 72 % of the issue slots are used (36 and 54 instructions a token and warp of eight
+// channels) and 66 and 53 % of the special-function unit (profiles/layer_kernels__ncu_counters.md).
 template <int LANES, int CH>
 struct ScanCfg {
     static constexpr int NP = LANES * CH;

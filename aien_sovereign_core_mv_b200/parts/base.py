@@ -206,7 +206,8 @@ class Workspace:
                 f"{which} workspace too small: need {end} bytes, have {self._size[region]} "
                 f"(the step brings more tokens than max_batch_tokens allows)")
         self._off[region] = end
-        # one native call on a view of the whole buffer in this type, not a slice, a change of type and a change of shape
+        # one native call on a view of the whole buffer in this type, not a slice, a change of type and a change of shape (scratch: the
+        # view has no version counter and no autograd)
         whole = self._typed.get(dtype)
         if whole is None:
             whole = self._typed[dtype] = self.buf.view(dtype)
